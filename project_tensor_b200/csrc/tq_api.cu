@@ -75,6 +75,17 @@ bool use_tensor(const tq_plan* p, int* err) {
 static std::atomic<long long> g_launches{0};
 void tq_count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 
+int tq_sm_count(int device) {
+    static std::atomic<int> known[kMaxDevices];
+    if (device < 0 || device >= kMaxDevices) return 148;
+    int sms = known[device].load(std::memory_order_relaxed);
+    if (sms == 0) {
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms <= 0) return 148;
+        known[device].store(sms, std::memory_order_relaxed);
+    }
+    return sms;
+}
+
 int tq_fail(int code, const char* fmt, ...) {
     va_list ap;
     va_start(ap, fmt);
@@ -176,11 +187,24 @@ int tq_plan_create(int d, int bits_mse, const float* rotation, const float* code
     v.codebook = reinterpret_cast<float*>(base + o_cb);
     v.boundaries = reinterpret_cast<float*>(base + o_bd);
     p->counters = reinterpret_cast<unsigned long long*>(base + o_cnt);
+    void *word = nullptr, *word_dev = nullptr;
+    e = cudaHostAlloc(&word, sizeof(unsigned long long), cudaHostAllocMapped | cudaHostAllocPortable);
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer(&word_dev, word, 0);
+    if (e != cudaSuccess) {
+        if (word) cudaFreeHost(word);
+        cudaFree(p->slab);
+        delete p;
+        return tq_fail(TQ_ERR_CUDA, "cudaHostAlloc for the status word failed: %s", cudaGetErrorString(e));
+    }
+    p->status_host = static_cast<volatile unsigned long long*>(word);
+    *p->status_host = 0ull;
+    p->status_dev = static_cast<unsigned long long*>(word_dev);
 
     p->tensor_ok = false;
     if (tq_tensor_quantize_supported(d, bits_mse, projection != nullptr)) {
         const int r = tq_tensor_plan_init(p, rotation, codebook, projection);
         if (r != TQ_OK) {
+            cudaFreeHost(word);
             cudaFree(p->slab);
             delete p;
             return r;
@@ -191,6 +215,7 @@ int tq_plan_create(int d, int bits_mse, const float* rotation, const float* code
         const int r = tq_dequant_tc_plan_init(p, rotation, projection);
         if (r != TQ_OK) {
             tq_tensor_plan_free(p);
+            cudaFreeHost(word);
             cudaFree(p->slab);
             delete p;
             return r;
@@ -210,7 +235,8 @@ void tq_plan_destroy(tq_plan* p) {
     }
     tq_tensor_plan_free(p);
     tq_dequant_tc_plan_free(p);
-    if (p->slab) cudaFree(p->slab);
+    if (p->slab) cudaFree(p->slab);     // waits for the device: no kernel can write the status word any more
+    if (p->status_host) cudaFreeHost(const_cast<unsigned long long*>(p->status_host));
     delete p;
 }
 
@@ -637,11 +663,10 @@ int tq_plan_status(const tq_plan* p, void* stream, int64_t* status) {
     if (!status) return tq_fail(TQ_ERR_INVALID_ARGUMENT, "status is null");
     DeviceScope scope(p->device);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    unsigned long long v = 0;
-    TQ_CUDA_TRY(cudaMemcpyAsync(&v, p->counters + 1, sizeof(v), cudaMemcpyDeviceToHost, st));
     TQ_CUDA_TRY(cudaStreamSynchronize(st));
+    const unsigned long long v = *p->status_host;
     *status = (int64_t)v;
-    if (v != 0) TQ_CUDA_TRY(cudaMemsetAsync(p->counters + 1, 0, sizeof(v), st));   // reported once
+    if (v != 0) *p->status_host = 0ull;   // reported once
     return TQ_OK;
 }
 
@@ -649,11 +674,12 @@ int tq_plan_last_recheck_rows(const tq_plan* p, void* stream, int64_t* rows) {
     TQ_TRY(check_plan(p, false));
     if (!rows) return tq_fail(TQ_ERR_INVALID_ARGUMENT, "rows is null");
     DeviceScope scope(p->device);
-    unsigned long long v[2] = {0, 0};
-    TQ_CUDA_TRY(cudaMemcpyAsync(v, p->counters, sizeof(v), cudaMemcpyDeviceToHost, static_cast<cudaStream_t>(stream)));
+    unsigned long long v = 0;
+    TQ_CUDA_TRY(cudaMemcpyAsync(&v, p->counters, sizeof(v), cudaMemcpyDeviceToHost, static_cast<cudaStream_t>(stream)));
     TQ_CUDA_TRY(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)));
-    *rows = (int64_t)v[0];
-    if (v[1] != 0) return tq_fail(TQ_ERR_CUDA, "a tensor-core kernel gave up on a bounded wait (status %llu)", v[1]);
+    *rows = (int64_t)v;
+    if (*p->status_host != 0)
+        return tq_fail(TQ_ERR_CUDA, "a tensor-core kernel gave up on a bounded wait (status %llu)", (unsigned long long)*p->status_host);
     return TQ_OK;
 }
 

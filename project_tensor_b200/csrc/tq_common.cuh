@@ -88,8 +88,11 @@ struct tq_plan {
     void* slab;              // one device allocation holding every constant
     TensorConsts* tensor;    // host-side bookkeeping for the tensor-core kernels (may be null)
     DequantConsts* dequant;  // operand matrices of the tensor-core dequantize kernels (may be null)
-    unsigned long long* counters;  // device: [0] rows re-done by the exact kernel in the last quantize, [1] status word
-                                   // (non-zero once a tensor-core kernel gave up on a bounded wait; sticky until read)
+    unsigned long long* counters;  // device: [0] rows re-done by the exact kernel in the last quantize
+    volatile unsigned long long* status_host;  // status word in page-locked host memory (non-zero once a tensor-core kernel
+                                               // gave up on a bounded wait; sticky until read): reading it takes a stream
+                                               // synchronisation and no copy (a copy of 8 bytes and its wait cost 17 us)
+    unsigned long long* status_dev;            // the same word as the kernels address it
     int wait_kcycles;              // limit of a bounded wait inside the tensor-core kernels, in units of 1024 cycles
     struct TqKernelTimer* timer;   // event pairs around the main kernels while tq_plan_time_kernels is on (else null)
 };
@@ -108,6 +111,21 @@ int tq_fail(int code, const char* fmt, ...);
         cudaError_t e__ = (expr);                                                           \
         if (e__ != cudaSuccess)                                                             \
             return tq_fail(TQ_ERR_CUDA, "%s failed: %s", #expr, cudaGetErrorString(e__));   \
+    } while (0)
+
+// Streaming multiprocessors of a device, asked for once (tq_api.cu).
+int tq_sm_count(int device);
+
+// Raise a kernel's limit of dynamic shared memory before its first launch on a device; the attribute stays with the
+// function, so later launches skip the call.
+#include <atomic>
+#define TQ_GRANT_SMEM(kernel, bytes, device)                                                                      \
+    do {                                                                                                          \
+        static std::atomic<int> granted__[64];                                                                    \
+        if (granted__[(device) & 63].load(std::memory_order_acquire) < (int)(bytes)) {                            \
+            TQ_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(bytes))); \
+            granted__[(device) & 63].store((int)(bytes), std::memory_order_release);                              \
+        }                                                                                                         \
     } while (0)
 
 // A named NVTX range around the launches of one step of a call (a profiler shows the library's kernels grouped by it;

@@ -494,12 +494,6 @@ int splits_for(int sms, int groups, int passes, int64_t keys_per_group) {
     return (int)best;
 }
 
-int sm_count(int device) {
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    return sms > 0 ? sms : 148;
-}
-
 template <int KB, int DR, int QP>
 int launch_partial(const tq_plan* kp, DecodeArgs a, int groups, int passes, cudaStream_t st) {
     const size_t fixed = decode_smem_floats<KB, DR, QP>() * 4, vtile = (size_t)kTile * a.vwords * 4;
@@ -507,10 +501,10 @@ int launch_partial(const tq_plan* kp, DecodeArgs a, int groups, int passes, cuda
     const size_t sm = fixed + a.vbufs * vtile;
     const dim3 grid((unsigned)a.splits, (unsigned)passes, (unsigned)groups);
     if (a.vbits == 3) {
-        TQ_CUDA_TRY(cudaFuncSetAttribute(decode_partial_kernel<KB, DR, QP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        TQ_GRANT_SMEM((decode_partial_kernel<KB, DR, QP, true>), sm, kp->device);
         decode_partial_kernel<KB, DR, QP, true><<<grid, kThreads, sm, st>>>(kp->dev, a); tq_count_launch();
     } else {
-        TQ_CUDA_TRY(cudaFuncSetAttribute(decode_partial_kernel<KB, DR, QP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        TQ_GRANT_SMEM((decode_partial_kernel<KB, DR, QP, false>), sm, kp->device);
         decode_partial_kernel<KB, DR, QP, false><<<grid, kThreads, sm, st>>>(kp->dev, a); tq_count_launch();
     }
     TQ_CUDA_TRY(cudaGetLastError());
@@ -535,7 +529,7 @@ bool tq_decode_attention_supported(const tq_plan* kp, const tq_plan* vp) {
 int64_t tq_decode_attention_scratch(const tq_plan* kp, int groups, int qpg, int64_t keys_per_group) {
     const int qp = queries_per_pass(kp->dev.bits, qpg);
     const int passes = (qpg + qp - 1) / qp;
-    const int splits = splits_for(sm_count(kp->device), groups, passes, keys_per_group);
+    const int splits = splits_for(tq_sm_count(kp->device), groups, passes, keys_per_group);
     return (int64_t)groups * qpg * splits * (kp->dev.d + 2) * (int64_t)sizeof(float);
 }
 
@@ -554,7 +548,7 @@ int tq_launch_decode_attention(const tq_plan* kp, const tq_plan* vp, const float
     a.vbits = vp->dev.bits; a.vwords = vp->dev.code_words;
     a.qpg = qpg; a.keys_per_group = keys_per_group; a.group_rows = group_rows; a.length = length;
     a.scale_log2e = scale * 1.4426950408889634f;
-    a.splits = splits_for(sm_count(kp->device), groups, passes, keys_per_group);
+    a.splits = splits_for(tq_sm_count(kp->device), groups, passes, keys_per_group);
     a.part = static_cast<float*>(scratch);
     const size_t need = (size_t)groups * qpg * a.splits * (d + 2) * sizeof(float);
     if (!scratch || scratch_bytes < need)

@@ -442,7 +442,7 @@ dequant_tc_kernel(const DequantArgs a) {
     if (*abort_flag) __nanosleep(20000);   // tensor instructions issued before the give-up may still be running
     tc_fence_before();
     __syncthreads();
-    if (threadIdx.x == 0 && *abort_flag) atomicExch(a.status, 3ull);
+    if (threadIdx.x == 0 && *abort_flag) report_status(a.status, 3ull);
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem, 512);
@@ -766,7 +766,7 @@ dequant256_kernel(const DequantArgs a) {
     if (*abort_flag) __nanosleep(20000);   // tensor instructions issued before the give-up may still be running
     tc_fence_before();
     __syncthreads();
-    if (threadIdx.x == 0 && *abort_flag) atomicExch(a.status, 3ull);
+    if (threadIdx.x == 0 && *abort_flag) report_status(a.status, 3ull);
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem, 512);
@@ -818,18 +818,18 @@ void split_transposed_chunks(const float* m, float scale, uint16_t* out) {
 }
 
 template <int BITS, bool PROD>
-int launch_256(const DequantArgs& args, int grid, cudaStream_t st) {
+int launch_256(const tq_plan* p, const DequantArgs& args, int grid, cudaStream_t st) {
     const int sm = dq256::Smem<BITS, PROD>::total;
-    TQ_CUDA_TRY(cudaFuncSetAttribute(dequant256_kernel<BITS, PROD>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+    TQ_GRANT_SMEM((dequant256_kernel<BITS, PROD>), sm, p->device);
     dequant256_kernel<BITS, PROD><<<grid, dq256::kThreads256, sm, st>>>(args); tq_count_launch();
     TQ_CUDA_TRY(cudaGetLastError());
     return TQ_OK;
 }
 
 template <int BITS, bool PROD, int DR, bool PAIR = false>
-int launch_one(const DequantArgs& args, int grid, cudaStream_t st) {
+int launch_one(const tq_plan* p, const DequantArgs& args, int grid, cudaStream_t st) {
     const int sm = DqSmem<BITS, PROD, DR>::total;
-    TQ_CUDA_TRY(cudaFuncSetAttribute(dequant_tc_kernel<BITS, PROD, DR, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+    TQ_GRANT_SMEM((dequant_tc_kernel<BITS, PROD, DR, PAIR>), sm, p->device);
     dequant_tc_kernel<BITS, PROD, DR, PAIR><<<grid, kThreads, sm, st>>>(args); tq_count_launch();
     TQ_CUDA_TRY(cudaGetLastError());
     return TQ_OK;
@@ -892,31 +892,30 @@ int tq_launch_dequant_tc(const tq_plan* p, bool prod, const uint32_t* codes, con
     a.n = n;
     a.ntiles = (n + kTileKeys - 1) / kTileKeys;
     a.out = out;
-    a.status = p->counters + 1;
+    a.status = p->status_dev;
     a.wait_kcycles = p->wait_kcycles;
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
+    const int sms = tq_sm_count(p->device);
     const int grid = (int)(a.ntiles < sms ? a.ntiles : sms);
     const int bits = p->dev.bits;
     int r = TQ_ERR_UNSUPPORTED;
 #define TQ_DQ(B, P)                                                                                  \
     case B:                                                                                          \
-        r = p->dev.d == 64 ? launch_one<B, P, 64>(a, grid, st) : launch_one<B, P, 128>(a, grid, st); \
+        r = p->dev.d == 64 ? launch_one<B, P, 64>(p, a, grid, st) : launch_one<B, P, 128>(p, a, grid, st); \
         break;
     if (p->dev.d == 256) {
         if (prod) {
             switch (bits) {
-                case 1: r = launch_256<1, true>(a, grid, st); break;
-                case 2: r = launch_256<2, true>(a, grid, st); break;
-                case 3: r = launch_256<3, true>(a, grid, st); break;
+                case 1: r = launch_256<1, true>(p, a, grid, st); break;
+                case 2: r = launch_256<2, true>(p, a, grid, st); break;
+                case 3: r = launch_256<3, true>(p, a, grid, st); break;
                 default: break;
             }
         } else {
             switch (bits) {
-                case 1: r = launch_256<1, false>(a, grid, st); break;
-                case 2: r = launch_256<2, false>(a, grid, st); break;
-                case 3: r = launch_256<3, false>(a, grid, st); break;
-                case 4: r = launch_256<4, false>(a, grid, st); break;
+                case 1: r = launch_256<1, false>(p, a, grid, st); break;
+                case 2: r = launch_256<2, false>(p, a, grid, st); break;
+                case 3: r = launch_256<3, false>(p, a, grid, st); break;
+                case 4: r = launch_256<4, false>(p, a, grid, st); break;
                 default: break;
             }
         }
@@ -945,15 +944,14 @@ int tq_launch_pairwise_tc(const tq_plan* p, const float* q, const uint32_t* code
     a.ntiles = (n + kTileKeys - 1) / kTileKeys;
     a.out = scores;
     a.pair_q = q;
-    a.status = p->counters + 1;
+    a.status = p->status_dev;
     a.wait_kcycles = p->wait_kcycles;
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
+    const int sms = tq_sm_count(p->device);
     const int grid = (int)(a.ntiles < sms ? a.ntiles : sms);
     int r = TQ_ERR_UNSUPPORTED;
 #define TQ_PW(B)                                                                                                   \
     case B:                                                                                                        \
-        r = p->dev.d == 64 ? launch_one<B, true, 64, true>(a, grid, st) : launch_one<B, true, 128, true>(a, grid, st); \
+        r = p->dev.d == 64 ? launch_one<B, true, 64, true>(p, a, grid, st) : launch_one<B, true, 128, true>(p, a, grid, st); \
         break;
     switch (p->dev.bits) { TQ_PW(1) TQ_PW(2) TQ_PW(3) default: break; }
 #undef TQ_PW

@@ -532,7 +532,7 @@ int tq_launch_exact_quantize(const tq_plan* p, bool prod, const float* x, int64_
     const int threads = (p->dev.d + 31) & ~31;
 #define TQ_LAUNCH_EXACT(P, M, T)                                                                                           \
     do {                                                                                                                  \
-        TQ_CUDA_TRY(cudaFuncSetAttribute(exact_quantize_kernel<P, M, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)); \
+        TQ_GRANT_SMEM((exact_quantize_kernel<P, M, T>), sm, p->device); \
         exact_quantize_kernel<P, M, T><<<grid, threads, sm, st>>>(p->dev, x, n, codes, signs, rnorms, norms, lists, redo_counter, map); tq_count_launch(); \
     } while (0)
 #define TQ_LAUNCH_EXACT_T(P, M)                  \
@@ -575,10 +575,10 @@ int tq_launch_exact_dequantize(const tq_plan* p, bool prod, const uint32_t* code
     const int grid = grid_for(n, kRB);
     const int threads = (d + 31) & ~31;
     if (prod) {
-        TQ_CUDA_TRY(cudaFuncSetAttribute(exact_dequantize_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        TQ_GRANT_SMEM((exact_dequantize_kernel<true>), sm, p->device);
         exact_dequantize_kernel<true><<<grid, threads, sm, st>>>(p->dev, codes, signs, rnorms, norms, n, out); tq_count_launch();
     } else {
-        TQ_CUDA_TRY(cudaFuncSetAttribute(exact_dequantize_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        TQ_GRANT_SMEM((exact_dequantize_kernel<false>), sm, p->device);
         exact_dequantize_kernel<false><<<grid, threads, sm, st>>>(p->dev, codes, signs, rnorms, norms, n, out); tq_count_launch();
     }
     TQ_CUDA_TRY(cudaGetLastError());
@@ -592,7 +592,7 @@ int tq_launch_exact_pairwise(const tq_plan* p, const float* q, const uint32_t* c
     if (n == 0) return TQ_OK;
     const int dp = (p->dev.d + 31) & ~31;
     const size_t sm = (size_t)kWarps * 3 * dp * sizeof(float);
-    TQ_CUDA_TRY(cudaFuncSetAttribute(exact_pairwise_score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    TQ_GRANT_SMEM((exact_pairwise_score_kernel), sm, p->device);
     exact_pairwise_score_kernel<<<grid_for(n, kWarps), kWarps * 32, sm, st>>>(p->dev, q, codes, signs, rnorms, norms, n, scores); tq_count_launch();
     TQ_CUDA_TRY(cudaGetLastError());
     return TQ_OK;

@@ -97,6 +97,12 @@ __device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
     }
 }
 
+// Leaves a code in the plan's status word, which lies in page-locked host memory.
+__device__ __forceinline__ void report_status(unsigned long long* status, unsigned long long code) {
+    *reinterpret_cast<volatile unsigned long long*>(status) = code;
+    __threadfence_system();
+}
+
 // The same wait executed by every lane of a converged warp; the answer is the same for all of them.
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
     const bool ok = mbar_wait(bar, parity, abort_flag);

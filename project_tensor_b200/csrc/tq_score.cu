@@ -341,7 +341,7 @@ int tq_launch_score_general(const tq_plan* p, const float* q, int groups, int qp
     const int d = p->dev.d;
     const size_t sm = (size_t)(kQT * d + kQT * 2 * d + 256) * sizeof(float) + (size_t)kQT * s.cap2 * sizeof(unsigned long long);
     if (sm > 200 * 1024) return tq_fail(TQ_ERR_UNSUPPORTED, "score kernel needs %zu bytes of shared memory", sm);
-    TQ_CUDA_TRY(cudaFuncSetAttribute(score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    TQ_GRANT_SMEM((score_kernel), sm, p->device);
     score_kernel<<<dim3(s.nblk, groups), kThreads, sm, st>>>(p->dev, q, qpg, codes, signs, rnorms, norms,
                                                              keys_per_group, group_rows, s.keys_per_block, scores, topk, s.cap2,
                                                              static_cast<unsigned long long*>(scratch)); tq_count_launch();

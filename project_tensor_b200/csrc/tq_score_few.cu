@@ -130,9 +130,8 @@ int launch_few(const tq_plan* p, const float* q, const uint32_t* codes, const ui
                const float* norms, int64_t keys_per_group, int64_t group_rows, int groups, int qpg, float* scores,
                cudaStream_t st) {
     const int sm = ((DR / 2) * (1 << (2 * BITS)) + (DR / 8) * 256) * 4;
-    TQ_CUDA_TRY(cudaFuncSetAttribute(score_few_kernel<BITS, DR>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
+    TQ_GRANT_SMEM((score_few_kernel<BITS, DR>), sm, p->device);
+    const int sms = tq_sm_count(p->device);
     int64_t blocks = (keys_per_group + kFewThreads - 1) / kFewThreads;
     const int64_t cap = (int64_t)sms * 4;   // the tables cost a few microseconds per block: a few blocks per SM, grid-stride
     if (blocks > cap) blocks = cap;

@@ -187,9 +187,8 @@ template <int KB, int DR>
 int launch_lut(const tq_plan* p, const float* q, const uint32_t* codes, const uint32_t* signs, const float* rnorms,
                const float* norms, int64_t n, int64_t group_rows, int groups, int qpg, float* scores, cudaStream_t st) {
     const size_t sm = lut_smem_floats<KB, DR>() * 4;
-    TQ_CUDA_TRY(cudaFuncSetAttribute(score_lut_kernel<KB, DR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
+    TQ_GRANT_SMEM((score_lut_kernel<KB, DR>), sm, p->device);
+    const int sms = tq_sm_count(p->device);
     int per_sm = 1;                                   // resident blocks per SM (shared memory and registers)
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, score_lut_kernel<KB, DR>, kThreads, sm);
     if (per_sm < 1) per_sm = 1;

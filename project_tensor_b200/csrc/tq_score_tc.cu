@@ -892,7 +892,7 @@ score_tc_kernel(const __grid_constant__ CUtensorMap tmap_out, const ScoreTcArgs 
     if (*abort_flag) __nanosleep(20000);   // tensor instructions issued before the give-up may still be running
     tc_fence_before();
     __syncthreads();
-    if (threadIdx.x == 0 && *abort_flag) atomicExch(a.status, 2ull);
+    if (threadIdx.x == 0 && *abort_flag) report_status(a.status, 2ull);
     TQ_PROF_CODE(if (a.prof && blockIdx.x == 0 && threadIdx.x == 0) { a.prof[16] = clock64() - prof_t0; a.prof[17] = prof_t1 - prof_t0; })
     if (warp == 1) {
         tc_fence_after();
@@ -1203,15 +1203,15 @@ int pow2_at_least(int v) {
 }
 
 template <int BITS, int QPAD, int DR>
-int launch_score(const CUtensorMap& map, const ScoreTcArgs& args, int grid, cudaStream_t st) {
+int launch_score(const tq_plan* p, const CUtensorMap& map, const ScoreTcArgs& args, int grid, cudaStream_t st) {
     const int sm = ScoreSmem<BITS, QPAD, DR>::total;
     if (args.fused) {
-        TQ_CUDA_TRY(cudaFuncSetAttribute(score_tc_kernel<BITS, QPAD, DR, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+        TQ_GRANT_SMEM((score_tc_kernel<BITS, QPAD, DR, true>), sm, p->device);
         score_tc_kernel<BITS, QPAD, DR, true><<<grid, ScoreThreads<QPAD>::kThreads, sm, st>>>(map, args); tq_count_launch();
         TQ_CUDA_TRY(cudaGetLastError());
         return TQ_OK;
     }
-    TQ_CUDA_TRY(cudaFuncSetAttribute(score_tc_kernel<BITS, QPAD, DR, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+    TQ_GRANT_SMEM((score_tc_kernel<BITS, QPAD, DR, false>), sm, p->device);
     score_tc_kernel<BITS, QPAD, DR, false><<<grid, ScoreThreads<QPAD>::kThreads, sm, st>>>(map, args); tq_count_launch();
     TQ_CUDA_TRY(cudaGetLastError());
     return TQ_OK;
@@ -1310,8 +1310,7 @@ int tq_launch_score_tc(const tq_plan* p, const float* q, int groups, int qpg, co
         return tq_fail(TQ_ERR_SCRATCH_TOO_SMALL, "score scratch: need %zu bytes, got %zu", need, scratch_bytes);
     unsigned char* sc = static_cast<unsigned char*>(scratch);
     unsigned char* prep = sc;     // both layouts start with the prepared queries
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
+    const int sms = tq_sm_count(p->device);
     const int bits = p->dev.bits;
     float* thr = reinterpret_cast<float*>(sc + cp.off_thr);
     unsigned int* cnt = reinterpret_cast<unsigned int*>(sc + cp.off_cnt);
@@ -1335,7 +1334,7 @@ int tq_launch_score_tc(const tq_plan* p, const float* q, int groups, int qpg, co
             } else if (p->dev.d == 256) {
                 score_prep256_kernel<<<dim3(qpad, groups), 1024, 0, st>>>(p->dev, q, qpg, q0, nq, qpad, prep); tq_count_launch();
             } else {
-                TQ_CUDA_TRY(cudaFuncSetAttribute(score_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrepSmemBytes));
+                TQ_GRANT_SMEM((score_prep_kernel), kPrepSmemBytes, p->device);
                 score_prep_kernel<<<dim3(qpad, groups), 128, kPrepSmemBytes, st>>>(p->dev, q, qpg, q0, nq, qpad, prep); tq_count_launch();
             }
             TQ_CUDA_TRY(cudaGetLastError());
@@ -1355,7 +1354,7 @@ int tq_launch_score_tc(const tq_plan* p, const float* q, int groups, int qpg, co
             a.fused = mat ? 0 : (tile_stride > 1 ? 2 : 1);    // 2: the sampled pass
             a.qpg_total = qpg; a.q0 = q0;
             a.thr = thr; a.cnt = cnt; a.cand = cand; a.cand_cap = cp.cand_cap;
-            a.status = p->counters + 1;
+            a.status = p->status_dev;
             a.wait_kcycles = p->wait_kcycles;
 #ifdef TQ_PROF
             a.prof = reinterpret_cast<long long*>(p->counters + 8);
@@ -1381,11 +1380,11 @@ int tq_launch_score_tc(const tq_plan* p, const float* q, int groups, int qpg, co
             tq_timer_mark(p, 1, 0, st);
 #define TQ_SC(B)                                                                                             \
     case B:                                                                                                  \
-        if (p->dev.d == 64) r = qpad == 16 ? launch_score<B, 16, 64>(map, a, grid, st) : qpad == 32 ? launch_score<B, 32, 64>(map, a, grid, st)       \
-                                                                                                   : launch_score<B, 64, 64>(map, a, grid, st);      \
-        else if (p->dev.d == 256) r = qpad == 16 ? launch_score<B, 16, 256>(map, a, grid, st) : launch_score<B, 32, 256>(map, a, grid, st);          \
-        else r = qpad == 16 ? launch_score<B, 16, 128>(map, a, grid, st) : qpad == 32 ? launch_score<B, 32, 128>(map, a, grid, st)                   \
-                                                                                      : launch_score<B, 64, 128>(map, a, grid, st);                  \
+        if (p->dev.d == 64) r = qpad == 16 ? launch_score<B, 16, 64>(p, map, a, grid, st) : qpad == 32 ? launch_score<B, 32, 64>(p, map, a, grid, st)       \
+                                                                                                   : launch_score<B, 64, 64>(p, map, a, grid, st);      \
+        else if (p->dev.d == 256) r = qpad == 16 ? launch_score<B, 16, 256>(p, map, a, grid, st) : launch_score<B, 32, 256>(p, map, a, grid, st);          \
+        else r = qpad == 16 ? launch_score<B, 16, 128>(p, map, a, grid, st) : qpad == 32 ? launch_score<B, 32, 128>(p, map, a, grid, st)                   \
+                                                                                      : launch_score<B, 64, 128>(p, map, a, grid, st);                  \
         break;
             switch (bits) { TQ_SC(1) TQ_SC(2) TQ_SC(3) TQ_SC(4) }
 #undef TQ_SC

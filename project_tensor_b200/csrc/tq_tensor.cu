@@ -793,7 +793,7 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
     if (*abort_flag) __nanosleep(20000);   // tensor instructions issued before the give-up may still be running
     tc_fence_before();
     __syncthreads();
-    if (threadIdx.x == 0 && *abort_flag) atomicExch(a.status, 1ull);
+    if (threadIdx.x == 0 && *abort_flag) report_status(a.status, 1ull);
 #ifdef TQ_PROF
     if (a.prof && blockIdx.x == 0) {
 #pragma unroll
@@ -1200,7 +1200,7 @@ tensor_quantize256_kernel(const __grid_constant__ CUtensorMap tmap_x, const Tens
     if (*abort_flag) __nanosleep(20000);   // tensor instructions issued before the give-up may still be running
     tc_fence_before();
     __syncthreads();
-    if (threadIdx.x == 0 && *abort_flag) atomicExch(a.status, 1ull);
+    if (threadIdx.x == 0 && *abort_flag) report_status(a.status, 1ull);
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem, 512);
@@ -1417,18 +1417,18 @@ void tq_tensor_plan_free(tq_plan* p) {
 #define TQ_UNI_MSE false
 #endif
 template <int D, int BITS, bool PROD>
-static int launch_one(const CUtensorMap& map, const TensorArgs& args, int grid, cudaStream_t st) {
+static int launch_one(const tq_plan* p, const CUtensorMap& map, const TensorArgs& args, int grid, cudaStream_t st) {
     constexpr bool UNI = PROD ? TQ_UNI_PROD : TQ_UNI_MSE;
     const int sm = Smem<D, PROD, UNI>::total;
-    TQ_CUDA_TRY(cudaFuncSetAttribute(tensor_quantize_kernel<D, BITS, PROD, UNI>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+    TQ_GRANT_SMEM((tensor_quantize_kernel<D, BITS, PROD, UNI>), sm, p->device);
     tensor_quantize_kernel<D, BITS, PROD, UNI><<<grid, Threads<PROD, UNI>::kThreads, sm, st>>>(map, args); tq_count_launch();
     TQ_CUDA_TRY(cudaGetLastError());
     return TQ_OK;
 }
 
 template <int BITS, bool PROD>
-static int launch_256(const CUtensorMap& map, const TensorArgs& args, int grid, cudaStream_t st) {
-    TQ_CUDA_TRY(cudaFuncSetAttribute(tensor_quantize256_kernel<BITS, PROD>, cudaFuncAttributeMaxDynamicSharedMemorySize, d256::total));
+static int launch_256(const tq_plan* p, const CUtensorMap& map, const TensorArgs& args, int grid, cudaStream_t st) {
+    TQ_GRANT_SMEM((tensor_quantize256_kernel<BITS, PROD>), d256::total, p->device);
     tensor_quantize256_kernel<BITS, PROD><<<grid, d256::kThreads, d256::total, st>>>(map, args); tq_count_launch();
     TQ_CUDA_TRY(cudaGetLastError());
     return TQ_OK;
@@ -1448,7 +1448,7 @@ int tq_launch_tensor_quantize(const tq_plan* p, bool prod, const float* x, int64
     args.norms = norms;
     args.rnorms = rnorms;
     args.lists = *lists;
-    args.status = p->counters + 1;
+    args.status = p->status_dev;
     args.wait_kcycles = p->wait_kcycles;
 #ifdef TQ_PROF
     args.prof = reinterpret_cast<long long*>(p->counters + 8);   // cycle counters per role, measurement builds only
@@ -1464,18 +1464,17 @@ int tq_launch_tensor_quantize(const tq_plan* p, bool prod, const float* x, int64
                                          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return tq_fail(TQ_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d", (int)r);
 
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
+    const int sms = tq_sm_count(p->device);
     const int grid = (int)(args.ntiles < sms ? args.ntiles : sms);
     const int bits = p->dev.bits;
     tq_timer_mark(p, 0, 0, st);
     int rc = TQ_ERR_UNSUPPORTED;
     if (d == 256) {
         switch (bits) {
-            case 1: rc = prod ? launch_256<1, true>(map, args, grid, st) : launch_256<1, false>(map, args, grid, st); break;
-            case 2: rc = prod ? launch_256<2, true>(map, args, grid, st) : launch_256<2, false>(map, args, grid, st); break;
-            case 3: rc = prod ? launch_256<3, true>(map, args, grid, st) : launch_256<3, false>(map, args, grid, st); break;
-            case 4: rc = prod ? launch_256<4, true>(map, args, grid, st) : launch_256<4, false>(map, args, grid, st); break;
+            case 1: rc = prod ? launch_256<1, true>(p, map, args, grid, st) : launch_256<1, false>(p, map, args, grid, st); break;
+            case 2: rc = prod ? launch_256<2, true>(p, map, args, grid, st) : launch_256<2, false>(p, map, args, grid, st); break;
+            case 3: rc = prod ? launch_256<3, true>(p, map, args, grid, st) : launch_256<3, false>(p, map, args, grid, st); break;
+            case 4: rc = prod ? launch_256<4, true>(p, map, args, grid, st) : launch_256<4, false>(p, map, args, grid, st); break;
         }
         tq_timer_mark(p, 0, 1, st);
         if (rc != TQ_ERR_UNSUPPORTED) return rc;
@@ -1483,8 +1482,8 @@ int tq_launch_tensor_quantize(const tq_plan* p, bool prod, const float* x, int64
     }
 #define TQ_DISPATCH(B)                                                                                     \
     case B:                                                                                                \
-        if (d == 64) rc = prod ? launch_one<64, B, true>(map, args, grid, st) : launch_one<64, B, false>(map, args, grid, st); \
-        else rc = prod ? launch_one<128, B, true>(map, args, grid, st) : launch_one<128, B, false>(map, args, grid, st);      \
+        if (d == 64) rc = prod ? launch_one<64, B, true>(p, map, args, grid, st) : launch_one<64, B, false>(p, map, args, grid, st); \
+        else rc = prod ? launch_one<128, B, true>(p, map, args, grid, st) : launch_one<128, B, false>(p, map, args, grid, st);      \
         break;
     switch (bits) {
         TQ_DISPATCH(1)

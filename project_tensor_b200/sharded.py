@@ -217,7 +217,7 @@ class ShardedKeyIndex:
         """Quantize ``keys`` (m, d) straight into the next m rows of this rank's packed buffers."""
         from .turboquant import _stage
         staged = _stage(keys, self.quantizer.dimension, device=self.device)
-        m = int(staged.tensor.shape[0])
+        m = staged.n
         if self.filled + m > self.stop - self.start:
             raise ValueError("more keys than this rank's shard holds")
         s = slice(self.filled, self.filled + m)
@@ -246,9 +246,9 @@ class ShardedKeyIndex:
         """Score this rank's keys and enqueue the all-gather of the candidates; ``.finish()`` of the returned
         exchange gives the global (scores, indices).  Work enqueued in between overlaps the collective."""
         from .turboquant import _stage
-        q = _stage(queries, self.quantizer.dimension, device=self.device).tensor
-        ex = TopkExchange(q.shape[0], k, self.device, group=group)
-        self.quantizer.attention_scores(q, self.encoding(), topk=k, index_base=self.start, out=(ex.top_scores, ex.top_idx))
+        staged = _stage(queries, self.quantizer.dimension, device=self.device)
+        ex = TopkExchange(staged.n, k, self.device, group=group)
+        self.quantizer.attention_scores(staged.tensor, self.encoding(), topk=k, index_base=self.start, out=(ex.top_scores, ex.top_idx))
         return ex.start()
 
     def search(self, queries, k: int, group=None, timeout_s: Optional[float] = None):

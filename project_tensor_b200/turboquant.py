@@ -22,6 +22,7 @@ from __future__ import annotations
 
 import ctypes
 import math
+import sys
 from dataclasses import dataclass
 from typing import Any, Dict, Optional, Tuple
 
@@ -62,10 +63,10 @@ def _is_device_array(obj: Any) -> bool:
 
 def _to_array(data: Any):
     """Unwrap a ``Tensor``-like object; leave arrays alone (_quant.py:31-34)."""
-    if isinstance(data, np.ndarray) or _is_device_array(data):
-        return data
     torch = _torch_if_loaded()
-    if torch is not None and isinstance(data, torch.Tensor):
+    if torch is not None and isinstance(data, torch.Tensor):   # before the attribute test, which builds a dict for a tensor
+        return data
+    if isinstance(data, np.ndarray) or _is_device_array(data):
         return data
     if isinstance(data, Tensor) or (hasattr(data, "data") and hasattr(data, "requires_grad")):
         return data.data
@@ -73,7 +74,6 @@ def _to_array(data: Any):
 
 
 def _torch_if_loaded():
-    import sys
     return sys.modules.get("torch")
 
 
@@ -93,13 +93,15 @@ def _quant_index_dtype(bits: int):
 
 
 class _Staged:
-    """An input brought to the GPU as a contiguous float32 (N, d) torch tensor, remembering what
-    kind of array the caller used so that results can be handed back in the same kind."""
+    """An input brought to the GPU as a contiguous float32 torch tensor of ``n`` rows (its last dimension is d; the
+    others are left as the caller had them), remembering what kind of array the caller used so that results can be
+    handed back in the same kind."""
 
-    __slots__ = ("tensor", "prefix", "kind", "device")
+    __slots__ = ("tensor", "prefix", "kind", "device", "n")
 
     def __init__(self, tensor, prefix, kind, device):
         self.tensor, self.prefix, self.kind, self.device = tensor, prefix, kind, device
+        self.n = math.prod(prefix)
 
 
 def _require_cuda():
@@ -110,39 +112,73 @@ def _require_cuda():
     return torch
 
 
-def _stage(data: Any, dim: int, device=None) -> _Staged:
+def _stage(data: Any, dim: int, device=None, halves: bool = False) -> _Staged:
+    """``halves``: the caller's kernel reads bf16 and fp16 vectors itself, so CUDA tensors of those types stay as they are
+    (see ``_dtype_code``)."""
+    torch = _torch_if_loaded()
+    if torch is not None and type(data) is torch.Tensor and data.is_cuda:
+        # the common device caller: looked at once, nothing converted, no view made (a few microseconds of every call)
+        shape = data.shape
+        if not shape or shape[-1] != dim:
+            _ensure_last_dim(data, dim)
+        dtype = data.dtype
+        if dtype is not torch.float32 and not (halves and (dtype is torch.bfloat16 or dtype is torch.float16)):
+            data = data.to(torch.float32)
+        return _Staged(data if data.is_contiguous() else data.contiguous(), tuple(shape[:-1]), "torch", data.device)
     array = _to_array(data)
     _ensure_last_dim(array, dim)
     prefix = tuple(array.shape[:-1])
     torch = _require_cuda()
     if isinstance(array, np.ndarray):
         dev = torch.device("cuda", torch.cuda.current_device()) if device is None else device
-        host = np.ascontiguousarray(array.reshape(-1, dim), dtype=np.float32)
-        t = torch.from_numpy(host)
-        return _Staged(t.to(dev, non_blocking=t.is_pinned()), prefix, "numpy", dev)
+        host = torch.from_numpy(np.ascontiguousarray(array, dtype=np.float32))
+        # The copy is enqueued and not waited for.  Pageable memory has been read when the call returns (the driver
+        # stages it); a page-locked source is the caller's to leave alone until the stream has passed the copy.
+        return _Staged(host.to(dev, non_blocking=True), prefix, "numpy", dev)
     if isinstance(array, torch.Tensor):
         if array.is_cuda:
-            t = array.reshape(-1, dim).to(torch.float32).contiguous()
-            return _Staged(t, prefix, "torch", array.device)
+            return _Staged(array.to(torch.float32).contiguous(), prefix, "torch", array.device)
         dev = torch.device("cuda", torch.cuda.current_device()) if device is None else device
-        t = array.reshape(-1, dim).to(torch.float32).contiguous()
-        return _Staged(t.to(dev), prefix, "torch_cpu", dev)
+        return _Staged(array.to(torch.float32).contiguous().to(dev), prefix, "torch_cpu", dev)
     # CuPy or any other __cuda_array_interface__ producer: zero-copy view
     t = torch.as_tensor(array, device="cuda")
     kind = "cupy" if type(array).__module__.split(".")[0] == "cupy" else "torch"
-    return _Staged(t.reshape(-1, dim).to(torch.float32).contiguous(), prefix, kind, t.device)
+    return _Staged(t.to(torch.float32).contiguous(), prefix, kind, t.device)
+
+
+def _dtype_code(tensor) -> int:
+    torch = _torch()
+    return {torch.float32: _native.TQ_F32, torch.bfloat16: _native.TQ_BF16, torch.float16: _native.TQ_F16}[tensor.dtype]
+
+
+_MAPPED_BYTES = 1 << 16
+
+
+def _stage_query(data: Any, dim: int, device) -> _Staged:
+    """Queries of a call that waits for its results before it returns.  A few NumPy queries go into a page-locked block
+    that the kernels read where it lies (one copy on the host instead of a copy through the driver, 7 us less); the
+    block is free again when the call is over."""
+    if isinstance(data, np.ndarray) and 0 < data.size * 4 <= _MAPPED_BYTES and device.type == "cuda":
+        _ensure_last_dim(data, dim)
+        block = _torch().empty(data.shape, dtype=_torch().float32, pin_memory=True)
+        block.numpy()[...] = data
+        return _Staged(block, tuple(data.shape[:-1]), "numpy", device)
+    staged = _stage(data, dim, device=device)
+    if staged.tensor.device != device:
+        staged.tensor = staged.tensor.to(device)
+    return staged
 
 
 def _deliver(tensor, kind: str, plans: "Optional[_PlanSet]" = None):
     """Hand a device tensor back in the caller's kind of array.  A result that goes to host memory synchronises
     anyway; with ``plans`` the status word of the kernels is read at that point, so that the output of a kernel
     that gave up on a bounded wait is never handed out as if it were complete."""
-    if plans is not None and kind in ("numpy", "torch_cpu"):
-        plans.check_status(tensor.device)
+    if kind == "torch":
+        return tensor
     if kind == "numpy":
-        return _to_host(tensor).numpy()
+        return _to_host(tensor, plans).numpy()
     if kind == "torch_cpu":
-        return _to_host(tensor)
+        return _to_host(tensor, plans)
     if kind == "cupy":
         try:
             import cupy
@@ -155,26 +191,37 @@ def _deliver(tensor, kind: str, plans: "Optional[_PlanSet]" = None):
 _PINNED_FROM_BYTES = 1 << 20
 
 
-def _to_host(tensor):
-    """Device tensor -> CPU tensor.  Results of a megabyte and more land in page-locked memory from torch's caching host
-    allocator (the block goes back to that cache when the array that wraps it dies): a copy into pageable memory runs at
-    a few GB/s, so that the 128 MiB score matrix of 32 queries x 1,048,576 keys took 62 ms to hand back, against 3 ms
-    at the rate of the link."""
+def _to_host(tensor, plans: "Optional[_PlanSet]" = None):
+    """Device tensor -> CPU tensor, the status of ``plans`` checked behind the copy: one synchronisation in all.
+    Every result comes down into page-locked memory from torch's caching host allocator.  From a megabyte on the caller
+    gets that block itself (it goes back to the cache when the array that wraps it dies): a copy into pageable memory
+    runs at a few GB/s, so that the 128 MiB score matrix of 32 queries x 1,048,576 keys took 62 ms to hand back, against
+    3 ms at the rate of the link.  Smaller results are copied out of the block on the host, so that arrays a caller
+    collects by the thousand do not pin memory; a device-to-host copy straight into pageable memory costs 14 us."""
     torch = _torch()
-    if tensor.device.type != "cuda" or tensor.numel() * tensor.element_size() < _PINNED_FROM_BYTES:
-        return tensor.cpu()
+    if tensor.device.type != "cuda":
+        return tensor
     host = torch.empty(tensor.shape, dtype=tensor.dtype, pin_memory=True)
     host.copy_(tensor, non_blocking=True)
-    torch.cuda.current_stream(tensor.device).synchronize()
-    return host
+    if plans is not None:
+        plans.check_status(tensor.device)      # waits for the stream
+    else:
+        torch.cuda.current_stream(tensor.device).synchronize()
+    return host if host.numel() * host.element_size() >= _PINNED_FROM_BYTES else host.clone()
 
 
 def _ptr(t) -> int:
     return 0 if t is None else t.data_ptr()
 
 
+def _device_index(device) -> int:
+    index = device.index
+    return _torch().cuda.current_device() if index is None else index
+
+
 def _stream_ptr(device) -> int:
-    return _torch().cuda.current_stream(device).cuda_stream
+    """The current stream's handle (torch.cuda.current_stream(device).cuda_stream builds an object for it: 2 us)."""
+    return _torch()._C._cuda_getCurrentRawStream(_device_index(device))
 
 
 # ------------------------------------------------------------------------------------------------
@@ -189,11 +236,11 @@ class _PlanSet:
         self._codebook = np.ascontiguousarray(codebook, dtype=np.float32)
         self._projection = None if projection is None else np.ascontiguousarray(projection, dtype=np.float32)
         self._plans: Dict[int, int] = {}
-        self._geometry: Optional[Tuple[int, int]] = None
+        self._row_bytes = (4 * ((dimension * bits_mse + 31) // 32), 4 * ((dimension + 31) // 32))
         self._path = _native.TQ_PATH_AUTO
 
     def handle(self, device) -> int:
-        idx = device.index if device.index is not None else _torch().cuda.current_device()
+        idx = _device_index(device)
         h = self._plans.get(idx)
         if h is None:
             lib = _native.load()
@@ -210,13 +257,11 @@ class _PlanSet:
     def check_status(self, device) -> None:
         """Raise if a tensor-core kernel of this quantizer gave up on a bounded wait on ``device`` since the last
         check (synchronises the current stream of that device)."""
-        idx = device.index if device.index is not None else _torch().cuda.current_device()
-        h = self._plans.get(idx)
+        h = self._plans.get(_device_index(device))
         if h is None:
             return
         status = ctypes.c_int64(0)
-        with _torch().cuda.device(idx):
-            _native.check(_native.load().tq_plan_status(h, _stream_ptr(device), ctypes.byref(status)))
+        _native.check(_native.load().tq_plan_status(h, _stream_ptr(device), ctypes.byref(status)))
         if status.value:
             what = {1: "quantize", 2: "scoring", 3: "dequantize"}.get(status.value, "tensor-core")
             raise _native.TurboQuantNativeError(
@@ -236,7 +281,7 @@ class _PlanSet:
 
     def row_bytes(self) -> Tuple[int, int]:
         """(code row bytes, sign row bytes); same formula as the library, usable without a GPU."""
-        return 4 * ((self.dimension * self.bits_mse + 31) // 32), 4 * ((self.dimension + 31) // 32)
+        return self._row_bytes
 
     def __del__(self):
         try:
@@ -280,9 +325,8 @@ def _unpack_codes(pk: _Packed):
     torch = _torch()
     out = torch.empty((pk.n, pk.plans.dimension), dtype=torch.uint8, device=pk.device)
     if pk.n:
-        with torch.cuda.device(pk.device):
-            _native.check(_native.load().tq_unpack_codes(pk.plans.handle(pk.device), _ptr(pk.codes), pk.n,
-                                                         _ptr(out), _stream_ptr(pk.device)))
+        _native.check(_native.load().tq_unpack_codes(pk.plans.handle(pk.device), _ptr(pk.codes), pk.n,
+                                                     _ptr(out), _stream_ptr(pk.device)))
     return _deliver(out, pk.kind, pk.plans)
 
 
@@ -290,9 +334,8 @@ def _unpack_signs(pk: _Packed):
     torch = _torch()
     out = torch.empty((pk.n, pk.plans.dimension), dtype=torch.int8, device=pk.device)
     if pk.n:
-        with torch.cuda.device(pk.device):
-            _native.check(_native.load().tq_unpack_signs(pk.plans.handle(pk.device), _ptr(pk.signs), pk.n,
-                                                         _ptr(out), _stream_ptr(pk.device)))
+        _native.check(_native.load().tq_unpack_signs(pk.plans.handle(pk.device), _ptr(pk.signs), pk.n,
+                                                     _ptr(out), _stream_ptr(pk.device)))
     return _deliver(out, pk.kind, pk.plans)
 
 
@@ -321,6 +364,12 @@ for _cls in (TurboQuantMSEEncoding, TurboQuantProdEncoding):
 TurboQuantProdEncoding.qjl = _lazy_field("qjl", _unpack_signs)
 TurboQuantProdEncoding.residual_norms = _lazy_field(
     "residual_norms", lambda pk: _deliver(pk.residual_norms, pk.kind, pk.plans))
+
+
+def _check_rows(out, values: int, prefix) -> None:
+    """A result allocated in the shape of ``prefix_shape`` has to hold the encoding's rows (the field can be edited)."""
+    if out.numel() != values:
+        raise ValueError(f"prefix_shape {tuple(prefix)} does not match the rows of the encoding")
 
 
 def _encoding_from_packed(cls, pk: _Packed, prefix):
@@ -527,25 +576,27 @@ class TurboQuantMSE:
         (e.g. slices of a preallocated index) instead of fresh ones."""
         torch = _torch()
         lib = _native.load()
-        x, device = staged.tensor, staged.device
-        n = x.shape[0]
+        x, device, n = staged.tensor, staged.device, staged.n
         code_bytes, sign_bytes = plans.row_bytes()
         handle = plans.handle(device)
-        with torch.cuda.device(device):
-            codes = out["codes"] if out else torch.empty((n, code_bytes), dtype=torch.uint8, device=device)
-            norms = out["norms"] if out else torch.empty((n,), dtype=torch.float32, device=device)
-            scratch = torch.empty((max(int(lib.tq_quantize_scratch_bytes(handle, n)), 16),),
-                                  dtype=torch.uint8, device=device)
-            st = _stream_ptr(device)
-            if prod:
-                signs = out["signs"] if out else torch.empty((n, sign_bytes), dtype=torch.uint8, device=device)
-                rnorms = out["residual_norms"] if out else torch.empty((n,), dtype=torch.float32, device=device)
-                _native.check(lib.tq_prod_quantize(handle, _ptr(x), n, _ptr(codes), _ptr(signs), _ptr(rnorms),
-                                                   _ptr(norms), _ptr(scratch), scratch.numel(), st))
+        if out:
+            codes, norms = out["codes"], out["norms"]
+        else:
+            codes, norms = x.new_empty((n, code_bytes), dtype=torch.uint8), x.new_empty((n,))
+        scratch_bytes = max(lib.tq_quantize_scratch_bytes(handle, n), 16)
+        scratch = x.new_empty((scratch_bytes,), dtype=torch.uint8)
+        st = _stream_ptr(device)
+        if prod:
+            if out:
+                signs, rnorms = out["signs"], out["residual_norms"]
             else:
-                signs = rnorms = None
-                _native.check(lib.tq_mse_quantize(handle, _ptr(x), n, _ptr(codes), _ptr(norms), _ptr(scratch),
-                                                  scratch.numel(), st))
+                signs, rnorms = x.new_empty((n, sign_bytes), dtype=torch.uint8), x.new_empty((n,))
+            _native.check(lib.tq_prod_quantize(handle, x.data_ptr(), n, codes.data_ptr(), signs.data_ptr(), rnorms.data_ptr(),
+                                               norms.data_ptr(), scratch.data_ptr(), scratch_bytes, st))
+        else:
+            signs = rnorms = None
+            _native.check(lib.tq_mse_quantize(handle, x.data_ptr(), n, codes.data_ptr(), norms.data_ptr(),
+                                              scratch.data_ptr(), scratch_bytes, st))
         return _Packed(codes, signs, norms, rnorms, n, staged.kind, device, plans)
 
     def quantize(self, vectors: Any) -> TurboQuantMSEEncoding:
@@ -555,13 +606,11 @@ class TurboQuantMSE:
 
     def dequantize(self, encoding: TurboQuantMSEEncoding):
         pk = _as_packed(encoding, self._plans, need_signs=False)
-        torch = _torch()
-        out = torch.empty((pk.n, self.dimension), dtype=torch.float32, device=pk.device)
-        with torch.cuda.device(pk.device):
-            _native.check(_native.load().tq_mse_dequantize(self._plans.handle(pk.device), _ptr(pk.codes),
-                                                           _ptr(pk.norms), pk.n, _ptr(out),
-                                                           _stream_ptr(pk.device)))
-        return _deliver(out, pk.kind, pk.plans).reshape(tuple(encoding.prefix_shape) + (self.dimension,))
+        out = pk.norms.new_empty(tuple(encoding.prefix_shape) + (self.dimension,))
+        _check_rows(out, pk.n * self.dimension, encoding.prefix_shape)
+        _native.check(_native.load().tq_mse_dequantize(self._plans.handle(pk.device), pk.codes.data_ptr(),
+                                                       pk.norms.data_ptr(), pk.n, out.data_ptr(), _stream_ptr(pk.device)))
+        return _deliver(out, pk.kind, pk.plans)
 
 
 class TurboQuantProd:
@@ -599,54 +648,54 @@ class TurboQuantProd:
 
     def dequantize(self, encoding: TurboQuantProdEncoding):
         pk = _as_packed(encoding, self._plans, need_signs=True)
-        torch = _torch()
-        out = torch.empty((pk.n, self.dimension), dtype=torch.float32, device=pk.device)
-        with torch.cuda.device(pk.device):
-            _native.check(_native.load().tq_prod_dequantize(
-                self._plans.handle(pk.device), _ptr(pk.codes), _ptr(pk.signs), _ptr(pk.residual_norms),
-                _ptr(pk.norms), pk.n, _ptr(out), _stream_ptr(pk.device)))
-        return _deliver(out, pk.kind, pk.plans).reshape(tuple(encoding.prefix_shape) + (self.dimension,))
+        out = pk.norms.new_empty(tuple(encoding.prefix_shape) + (self.dimension,))
+        _check_rows(out, pk.n * self.dimension, encoding.prefix_shape)
+        _native.check(_native.load().tq_prod_dequantize(
+            self._plans.handle(pk.device), pk.codes.data_ptr(), pk.signs.data_ptr(), pk.residual_norms.data_ptr(),
+            pk.norms.data_ptr(), pk.n, out.data_ptr(), _stream_ptr(pk.device)))
+        return _deliver(out, pk.kind, pk.plans)
 
     def attention_score(self, query: Any, encoding: TurboQuantProdEncoding):
         """One query row broadcast over all keys, or one query row per key (_quant.py:334-358)."""
         pk = _as_packed(encoding, self._plans, need_signs=True)
-        staged = _stage(query, self.dimension, device=pk.device)
+        staged = _stage_query(query, self.dimension, pk.device)
         q = staged.tensor
-        if q.device != pk.device:
-            q = q.to(pk.device)
         num_codes = pk.n
         q_prefix = staged.prefix
-        broadcast = q.shape[0] == 1 and num_codes > 1
-        if broadcast:
+        broadcast = staged.n == 1 and num_codes > 1
+        if staged.n == 1:
             q_prefix = tuple(encoding.prefix_shape)
-        elif q.shape[0] != num_codes:
+        if not broadcast and staged.n != num_codes:
             raise ValueError(
-                f"query batch size {q.shape[0]} does not match encoding batch size {num_codes}"
+                f"query batch size {staged.n} does not match encoding batch size {num_codes}"
             )
-        torch = _torch()
         lib = _native.load()
-        scores = torch.empty((num_codes,), dtype=torch.float32, device=pk.device)
+        # a short row of scores for a NumPy caller is written straight to page-locked memory
+        to_host = staged.kind == "numpy" and 4 * num_codes <= _MAPPED_BYTES
+        scores = _torch().empty(q_prefix, pin_memory=True) if to_host else pk.norms.new_empty(q_prefix)
+        _check_rows(scores, num_codes, q_prefix)
         handle = self._plans.handle(pk.device)
-        with torch.cuda.device(pk.device):
-            if broadcast and self._plans._path == _native.TQ_PATH_AUTO:
-                # one query against all keys: the entry point that needs no scratch buffer
-                _native.check(lib.tq_score_broadcast(handle, _ptr(q), _ptr(pk.codes), _ptr(pk.signs),
-                                                     _ptr(pk.residual_norms), _ptr(pk.norms), num_codes,
-                                                     _ptr(scores), _stream_ptr(pk.device)))
-            elif broadcast:
-                # a forced kernel path: the one-row case of the batched entry point
-                need =int(lib.tq_topk_scratch_bytes(handle, 1, 1, num_codes, 0))
-                scratch = torch.empty((max(need, 16),), dtype=torch.uint8, device=pk.device)
-                _native.check(lib.tq_score_batched(handle, _ptr(q), 1, 1, _ptr(pk.codes), _ptr(pk.signs),
-                                                   _ptr(pk.residual_norms), _ptr(pk.norms), num_codes,
-                                                   _ptr(scores), 0, None, None, 0, _ptr(scratch),
-                                                   scratch.numel(), _stream_ptr(pk.device)))
-            else:
-                _native.check(lib.tq_score_pairwise(handle, _ptr(q), _ptr(pk.codes), _ptr(pk.signs),
-                                                    _ptr(pk.residual_norms), _ptr(pk.norms), num_codes,
-                                                    _ptr(scores), _stream_ptr(pk.device)))
-        shape = q_prefix if (broadcast or q.shape[0] != 1) else tuple(encoding.prefix_shape)
-        return _deliver(scores, staged.kind, self._plans).reshape(shape)
+        st = _stream_ptr(pk.device)
+        if broadcast and self._plans._path == _native.TQ_PATH_AUTO:
+            # one query against all keys: the entry point that needs no scratch buffer
+            _native.check(lib.tq_score_broadcast(handle, q.data_ptr(), pk.codes.data_ptr(), pk.signs.data_ptr(),
+                                                 pk.residual_norms.data_ptr(), pk.norms.data_ptr(), num_codes,
+                                                 scores.data_ptr(), st))
+        elif broadcast:
+            # a forced kernel path: the one-row case of the batched entry point
+            need = max(lib.tq_topk_scratch_bytes(handle, 1, 1, num_codes, 0), 16)
+            scratch = pk.norms.new_empty((need,), dtype=_torch().uint8)
+            _native.check(lib.tq_score_batched(handle, q.data_ptr(), 1, 1, pk.codes.data_ptr(), pk.signs.data_ptr(),
+                                               pk.residual_norms.data_ptr(), pk.norms.data_ptr(), num_codes,
+                                               scores.data_ptr(), 0, None, None, 0, scratch.data_ptr(), need, st))
+        else:
+            _native.check(lib.tq_score_pairwise(handle, q.data_ptr(), pk.codes.data_ptr(), pk.signs.data_ptr(),
+                                                pk.residual_norms.data_ptr(), pk.norms.data_ptr(), num_codes,
+                                                scores.data_ptr(), st))
+        if to_host:
+            self._plans.check_status(pk.device)      # waits for the stream
+            return scores.clone().numpy()
+        return _deliver(scores, staged.kind, self._plans)
 
     def attention_scores(self, queries: Any, encoding: TurboQuantProdEncoding, *, topk: Optional[int] = None,
                          groups: int = 1, return_matrix: Optional[bool] = None, index_base: int = 0,
@@ -667,11 +716,9 @@ class TurboQuantProd:
         that the candidates need no repacking before the collective).
         """
         pk = _as_packed(encoding, self._plans, need_signs=True)
-        staged = _stage(queries, self.dimension, device=pk.device)
-        q = staged.tensor
-        if q.device != pk.device:
-            q = q.to(pk.device)
-        nq, n = q.shape[0], pk.n
+        staged = _stage_query(queries, self.dimension, pk.device)
+        q, new_empty = staged.tensor, pk.norms.new_empty
+        nq, n = staged.n, pk.n
         if groups < 1 or nq % groups or n % groups:
             raise ValueError(f"groups={groups} must divide both the query count {nq} and the key count {n}")
         qpg, kpg = nq // groups, n // groups
@@ -682,23 +729,22 @@ class TurboQuantProd:
         torch = _torch()
         lib = _native.load()
         handle = self._plans.handle(pk.device)
-        with torch.cuda.device(pk.device):
-            scores = torch.empty((nq, kpg), dtype=torch.float32, device=pk.device) if want_matrix else None
-            if out is not None and k:
-                top_s, top_i = out
-                if (tuple(top_s.shape) != (nq, k) or tuple(top_i.shape) != (nq, k) or top_s.dtype != torch.float32
-                        or top_i.dtype != torch.int64 or not top_s.is_contiguous() or not top_i.is_contiguous()
-                        or top_s.device != pk.device or top_i.device != pk.device):
-                    raise ValueError(f"out must be contiguous float32 / int64 tensors of shape ({nq}, {k}) on {pk.device}")
-            else:
-                top_s = torch.empty((nq, k), dtype=torch.float32, device=pk.device) if k else None
-                top_i = torch.empty((nq, k), dtype=torch.int64, device=pk.device) if k else None
-            need = int(lib.tq_topk_scratch_bytes(handle, groups, qpg, kpg, k))
-            scratch = torch.empty((max(need, 16),), dtype=torch.uint8, device=pk.device)
-            _native.check(lib.tq_score_batched(handle, _ptr(q), groups, qpg, _ptr(pk.codes), _ptr(pk.signs),
-                                               _ptr(pk.residual_norms), _ptr(pk.norms), kpg, _ptr(scores), k,
-                                               _ptr(top_s), _ptr(top_i), int(index_base), _ptr(scratch),
-                                               scratch.numel(), _stream_ptr(pk.device)))
+        scores = new_empty((nq, kpg)) if want_matrix else None
+        if out is not None and k:
+            top_s, top_i = out
+            if (tuple(top_s.shape) != (nq, k) or tuple(top_i.shape) != (nq, k) or top_s.dtype != torch.float32
+                    or top_i.dtype != torch.int64 or not top_s.is_contiguous() or not top_i.is_contiguous()
+                    or top_s.device != pk.device or top_i.device != pk.device):
+                raise ValueError(f"out must be contiguous float32 / int64 tensors of shape ({nq}, {k}) on {pk.device}")
+        else:
+            top_s = new_empty((nq, k)) if k else None
+            top_i = new_empty((nq, k), dtype=torch.int64) if k else None
+        need = max(lib.tq_topk_scratch_bytes(handle, groups, qpg, kpg, k), 16)
+        scratch = new_empty((need,), dtype=torch.uint8)
+        _native.check(lib.tq_score_batched(handle, q.data_ptr(), groups, qpg, pk.codes.data_ptr(), pk.signs.data_ptr(),
+                                           pk.residual_norms.data_ptr(), pk.norms.data_ptr(), kpg, _ptr(scores), k,
+                                           _ptr(top_s), _ptr(top_i), int(index_base), scratch.data_ptr(), need,
+                                           _stream_ptr(pk.device)))
         if k == 0:
             return _deliver(scores, staged.kind, self._plans)
         result = (_deliver(top_s, staged.kind, self._plans), _deliver(top_i, staged.kind))
