@@ -50,6 +50,11 @@ extern "C" {
 #define TQ_PATH_EXACT 1   /* float32 kernels that accumulate in the reference's order */
 #define TQ_PATH_TENSOR 2  /* tensor-core kernels; TQ_ERR_UNSUPPORTED if (d, bits) has none */
 
+/* Element types of vectors handed to tq_kv_append. */
+#define TQ_F32 0
+#define TQ_BF16 1
+#define TQ_F16 2
+
 typedef struct tq_plan tq_plan;
 
 int tq_version(void);
@@ -192,7 +197,8 @@ int tq_score_cache(const tq_plan* plan, const float* q, int groups, int q_per_gr
  * group g is written to row g * capacity + *length + j, with the same numbers tq_*_quantize gives
  * (the arithmetic of _quant.py:224-236, 300-308 in the reference's order of operations); rows that would
  * land beyond `capacity` are dropped.  advance != 0: afterwards *length = min(*length + tokens, capacity),
- * in stream order.  One kernel launch (two with advance), no scratch, any d and bits.
+ * in stream order.  One kernel launch, no scratch, any d and bits.  While a launch with advance != 0 runs, the
+ * word at `length` holds other values; it is right again for whatever follows on the stream.
  * No reference counterpart (TurboQuantProd.quantize, _quant.py:297-315, always builds a new encoding).
  */
 int tq_mse_append(const tq_plan* plan, const float* x, int groups, int tokens, void* codes, float* norms,
@@ -200,6 +206,16 @@ int tq_mse_append(const tq_plan* plan, const float* x, int groups, int tokens, v
 int tq_prod_append(const tq_plan* plan, const float* x, int groups, int tokens, void* codes, void* signs,
                    float* residual_norms, float* norms, int64_t capacity, int64_t* length, int advance,
                    void* stream);
+
+/*
+ * One step of a key/value cache in one launch: tq_prod_append of `keys` with `kplan` and tq_mse_append of `values` with
+ * `vplan` at the same position, vectors of element type `dtype` (TQ_F32, TQ_BF16, TQ_F16; bf16 and fp16 values are
+ * widened to float32, exactly, as they are read).  Either plan may be null (its buffers are not touched then); with both,
+ * device and d must agree.  No reference counterpart.
+ */
+int tq_kv_append(const tq_plan* kplan, const tq_plan* vplan, const void* keys, const void* values, int dtype, int groups,
+                 int tokens, void* k_codes, void* k_signs, float* k_residual_norms, float* k_norms, void* v_codes,
+                 float* v_norms, int64_t capacity, int64_t* length, int advance, void* stream);
 
 /*
  * Decode attention over a quantized key/value cache, without writing scores or dequantized values:

@@ -13,6 +13,7 @@ _PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 LIB_NAME = "libtq_sm100.so"
 
 TQ_OK = 0
+TQ_F32, TQ_BF16, TQ_F16 = 0, 1, 2
 TQ_PATH_AUTO, TQ_PATH_EXACT, TQ_PATH_TENSOR = 0, 1, 2
 
 # name -> (restype, argtypes); mirrors include/tq_b200.h one to one
@@ -49,6 +50,8 @@ SIGNATURES = {
                               c_void_p]),
     "tq_prod_append": (c_int, [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int64,
                                c_void_p, c_int, c_void_p]),
+    "tq_kv_append": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
+                             c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_int, c_void_p]),
     "tq_decode_attention_scratch_bytes": (c_int64, [c_void_p, c_int, c_int, c_int64]),
     "tq_decode_attention": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                     c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_float, c_void_p, c_void_p, c_size_t,

@@ -20,6 +20,11 @@ from . import _native
 from . import turboquant as _tq
 
 
+def _widen(staged):
+    staged.tensor = staged.tensor.float()
+    return staged
+
+
 class PackedKeyCache:
     """Packed TurboQuantProd keys of ``groups`` sequences, ``capacity`` rows each, all of one length."""
 
@@ -67,7 +72,6 @@ class PackedKeyCache:
         """Add keys of shape (groups, tokens, d), or (groups, d) for one token each, behind the present rows.
         A contiguous float32 CUDA tensor of at most ``SMALL_APPEND_ROWS`` rows is appended with no allocation
         and no host synchronisation (capturable in a CUDA graph)."""
-        torch = _tq._torch()
         d = self.quantizer.dimension
         array = _tq._to_array(keys)
         _tq._ensure_last_dim(array, d)
@@ -83,27 +87,35 @@ class PackedKeyCache:
             raise ValueError(f"cache is full: {self._length} + {tokens} rows exceed the capacity {self.capacity}")
         if tokens == 0:
             return
-        staged = _tq._stage(keys, d, device=self.device)
-        x = staged.tensor
-        lib = _native.load()
-        handle = self._plans.handle(self.device)
-        rows = self.groups * tokens
-        with torch.cuda.device(self.device):
-            if rows <= self.SMALL_APPEND_ROWS:
-                _native.check(lib.tq_prod_append(handle, x.data_ptr(), self.groups, tokens, self.codes.data_ptr(),
-                                                 self.signs.data_ptr(), self.residual_norms.data_ptr(),
-                                                 self.norms.data_ptr(), self.capacity, self.length_device.data_ptr(), 1,
-                                                 _tq._stream_ptr(self.device)))
-            else:
-                pk = self.quantizer.mse._quantize_staged(staged, self._plans, True)
-                lo, hi = self._length, self._length + tokens
-                g, c = self.groups, self.capacity
-                self.codes.view(g, c, -1)[:, lo:hi] = pk.codes.view(g, tokens, -1)
-                self.signs.view(g, c, -1)[:, lo:hi] = pk.signs.view(g, tokens, -1)
-                self.norms.view(g, c)[:, lo:hi] = pk.norms.view(g, tokens)
-                self.residual_norms.view(g, c)[:, lo:hi] = pk.residual_norms.view(g, tokens)
-                self.length_device.add_(tokens)
-        self._length += tokens
+        self._append(_tq._stage(keys, d, device=self.device, halves=True), tokens)
+
+    def _append(self, staged, tokens: int, values=None) -> None:
+        """Write ``tokens`` staged keys per group behind the present rows, and the same number of values when ``values``
+        is (staged values, their plans, their codes, their norms); the length advances once."""
+        lo, hi = self._length, self._length + tokens
+        if self.groups * tokens <= self.SMALL_APPEND_ROWS:
+            dev = self.device
+            vstaged, vplans, vcodes, vnorms = values or (None, None, None, None)
+            _native.check(_native.load().tq_kv_append(
+                self._plans.handle(dev), vplans.handle(dev) if values else None, staged.tensor.data_ptr(),
+                vstaged.tensor.data_ptr() if values else None, _tq._dtype_code(staged.tensor), self.groups, tokens,
+                self.codes.data_ptr(), self.signs.data_ptr(), self.residual_norms.data_ptr(), self.norms.data_ptr(),
+                vcodes.data_ptr() if values else None, vnorms.data_ptr() if values else None, self.capacity,
+                self.length_device.data_ptr(), 1, _tq._stream_ptr(dev)))
+        else:
+            g, c = self.groups, self.capacity
+            if values:
+                vstaged, vplans, vcodes, vnorms = values
+                pk = self.quantizer.mse._quantize_staged(_widen(vstaged), vplans, False)
+                vcodes.view(g, c, -1)[:, lo:hi] = pk.codes.view(g, tokens, -1)
+                vnorms.view(g, c)[:, lo:hi] = pk.norms.view(g, tokens)
+            pk = self.quantizer.mse._quantize_staged(_widen(staged), self._plans, True)
+            self.codes.view(g, c, -1)[:, lo:hi] = pk.codes.view(g, tokens, -1)
+            self.signs.view(g, c, -1)[:, lo:hi] = pk.signs.view(g, tokens, -1)
+            self.norms.view(g, c)[:, lo:hi] = pk.norms.view(g, tokens)
+            self.residual_norms.view(g, c)[:, lo:hi] = pk.residual_norms.view(g, tokens)
+            self.length_device.add_(tokens)
+        self._length = hi
 
     # ---- scoring --------------------------------------------------------------------------------
     def scores(self, queries: Any, *, topk: Optional[int] = None, return_matrix: Optional[bool] = None):
@@ -128,30 +140,29 @@ class PackedKeyCache:
         lib = _native.load()
         handle = self._plans.handle(self.device)
         dev = self.device
-        with torch.cuda.device(dev):
-            mat = torch.empty((self.groups, qpg, n), dtype=torch.float32, device=dev) if want_matrix else None
-            top_s = torch.empty((self.groups, qpg, k), dtype=torch.float32, device=dev) if k else None
-            top_i = torch.empty((self.groups, qpg, k), dtype=torch.int64, device=dev) if k else None
-            if n == 0:
-                # nothing to score yet: a matrix without columns, top-k slots at their fill values
-                if k:
-                    top_s.fill_(float("-inf"))
-                    top_i.fill_(-1)
-                if k == 0:
-                    return _tq._deliver(mat, staged.kind, self._plans)
-                result = (_tq._deliver(top_s, staged.kind, self._plans), _tq._deliver(top_i, staged.kind))
-                return result + (_tq._deliver(mat, staged.kind, self._plans),) if want_matrix else result
-            need = int(lib.tq_topk_scratch_bytes(handle, self.groups, qpg, n, k))
-            scratch = torch.empty((max(need, 16),), dtype=torch.uint8, device=dev)
-            _native.check(lib.tq_score_cache(handle, q.data_ptr(), self.groups, qpg, self.codes.data_ptr(),
-                                             self.signs.data_ptr(), self.residual_norms.data_ptr(),
-                                             self.norms.data_ptr(), n, self.capacity, _tq._ptr(mat), k,
-                                             _tq._ptr(top_s), _tq._ptr(top_i), 0, scratch.data_ptr(), scratch.numel(),
-                                             _tq._stream_ptr(dev)))
+        mat = torch.empty((self.groups, qpg, n), dtype=torch.float32, device=dev) if want_matrix else None
+        top_s = torch.empty((self.groups, qpg, k), dtype=torch.float32, device=dev) if k else None
+        top_i = torch.empty((self.groups, qpg, k), dtype=torch.int64, device=dev) if k else None
+        if n == 0:
+            # nothing to score yet: a matrix without columns, top-k slots at their fill values
             if k:
-                # rows of the arrays -> positions inside the group; empty slots stay -1
-                base = (torch.arange(self.groups, device=dev, dtype=torch.int64) * self.capacity).view(-1, 1, 1)
-                top_i = torch.where(top_i >= 0, top_i - base, top_i)
+                top_s.fill_(float("-inf"))
+                top_i.fill_(-1)
+            if k == 0:
+                return _tq._deliver(mat, staged.kind, self._plans)
+            result = (_tq._deliver(top_s, staged.kind, self._plans), _tq._deliver(top_i, staged.kind))
+            return result + (_tq._deliver(mat, staged.kind, self._plans),) if want_matrix else result
+        need = int(lib.tq_topk_scratch_bytes(handle, self.groups, qpg, n, k))
+        scratch = torch.empty((max(need, 16),), dtype=torch.uint8, device=dev)
+        _native.check(lib.tq_score_cache(handle, q.data_ptr(), self.groups, qpg, self.codes.data_ptr(),
+                                         self.signs.data_ptr(), self.residual_norms.data_ptr(),
+                                         self.norms.data_ptr(), n, self.capacity, _tq._ptr(mat), k,
+                                         _tq._ptr(top_s), _tq._ptr(top_i), 0, scratch.data_ptr(), scratch.numel(),
+                                         _tq._stream_ptr(dev)))
+        if k:
+            # rows of the arrays -> positions inside the group; empty slots stay -1
+            base = (torch.arange(self.groups, device=dev, dtype=torch.int64) * self.capacity).view(-1, 1, 1)
+            top_i = torch.where(top_i >= 0, top_i - base, top_i)
         if k == 0:
             return _tq._deliver(mat, staged.kind, self._plans)
         result = (_tq._deliver(top_s, staged.kind, self._plans), _tq._deliver(top_i, staged.kind))
@@ -205,7 +216,6 @@ class PackedKVCache:
     def append(self, keys: Any, values: Any) -> None:
         """Add one key and one value per token: both of shape (groups, tokens, d) or (groups, d).  The values
         are written at the position the keys take; the shared length advances once."""
-        torch = _tq._torch()
         d = self.value_quantizer.dimension
         karr, varr = _tq._to_array(keys), _tq._to_array(values)
         _tq._ensure_last_dim(varr, d)
@@ -220,27 +230,17 @@ class PackedKVCache:
             raise ValueError(f"cache is full: {lo} + {tokens} rows exceed the capacity {self.capacity}")
         if tokens == 0:
             return
-        staged = _tq._stage(values, d, device=self.device)
-        with torch.cuda.device(self.device):
-            if self.groups * tokens <= PackedKeyCache.SMALL_APPEND_ROWS:
-                # the values first, without advancing: the key append that follows reads the same length
-                _native.check(_native.load().tq_mse_append(
-                    self._vplans.handle(self.device), staged.tensor.data_ptr(), self.groups, tokens,
-                    self.value_codes.data_ptr(), self.value_norms.data_ptr(), self.capacity,
-                    self.keys.length_device.data_ptr(), 0, _tq._stream_ptr(self.device)))
-            else:
-                pk = self.value_quantizer._quantize_staged(staged, self._vplans, False)
-                g, c = self.groups, self.capacity
-                self.value_codes.view(g, c, -1)[:, lo:lo + tokens] = pk.codes.view(g, tokens, -1)
-                self.value_norms.view(g, c)[:, lo:lo + tokens] = pk.norms.view(g, tokens)
-        self.keys.append(keys)
+        vstaged = _tq._stage(values, d, device=self.device, halves=True)
+        kstaged = _tq._stage(keys, d, device=self.device, halves=True)
+        if kstaged.tensor.dtype != vstaged.tensor.dtype:
+            kstaged, vstaged = _widen(kstaged), _widen(vstaged)
+        self.keys._append(kstaged, tokens, (vstaged, self._vplans, self.value_codes, self.value_norms))
 
     def attend(self, queries: Any, *, scale: Optional[float] = None, use_device_length: bool = False):
         """``queries`` of shape (groups, q_per_group, d) or (groups, d) -> attention output of the same shape.
         ``scale`` defaults to d ** -0.5.  ``use_device_length=True`` makes the kernel read the number of keys from
         the device-side counter (up to the capacity) instead of the host's mirror, for a step that is replayed from
         a CUDA graph while the cache grows."""
-        torch = _tq._torch()
         d = self.value_quantizer.dimension
         array = _tq._to_array(queries)
         _tq._ensure_last_dim(array, d)
@@ -252,18 +252,17 @@ class PackedKVCache:
         lib = _native.load()
         kc, dev = self.keys, self.device
         kh, vh = kc._plans.handle(dev), self._vplans.handle(dev)
-        with torch.cuda.device(dev):
-            out = torch.empty((self.groups, qpg, d), dtype=torch.float32, device=dev)
-            need = int(lib.tq_decode_attention_scratch_bytes(kh, self.groups, qpg, n))
-            scratch = torch.empty((max(need, 16),), dtype=torch.uint8, device=dev)
-            _native.check(lib.tq_decode_attention(
-                kh, vh, staged.tensor.data_ptr(), self.groups, qpg, kc.codes.data_ptr(), kc.signs.data_ptr(),
-                kc.residual_norms.data_ptr(), kc.norms.data_ptr(), self.value_codes.data_ptr(),
-                self.value_norms.data_ptr(), n, self.capacity,
-                kc.length_device.data_ptr() if use_device_length else None, float(scale or 0.0), out.data_ptr(),
-                scratch.data_ptr(), scratch.numel(), _tq._stream_ptr(dev)))
-        out = _tq._deliver(out, staged.kind)
-        return out.reshape(tuple(array.shape))
+        q = staged.tensor
+        out = q.new_empty(tuple(array.shape))
+        need = max(lib.tq_decode_attention_scratch_bytes(kh, self.groups, qpg, n), 16)
+        scratch = q.new_empty((need,), dtype=_tq._torch().uint8)
+        _native.check(lib.tq_decode_attention(
+            kh, vh, q.data_ptr(), self.groups, qpg, kc.codes.data_ptr(), kc.signs.data_ptr(),
+            kc.residual_norms.data_ptr(), kc.norms.data_ptr(), self.value_codes.data_ptr(),
+            self.value_norms.data_ptr(), n, self.capacity,
+            kc.length_device.data_ptr() if use_device_length else None, float(scale or 0.0), out.data_ptr(),
+            scratch.data_ptr(), need, _tq._stream_ptr(dev)))
+        return _tq._deliver(out, staged.kind)
 
     def value_encoding(self, group: int):
         """The filled value rows of one group as a TurboQuantMSEEncoding (a view of the cache)."""

@@ -280,8 +280,12 @@ static int quantize_common(const tq_plan* p, bool prod, const float* x, int64_t 
     DeviceScope scope(p->device);
     if (!scope.ok) return tq_fail(TQ_ERR_CUDA, "cannot select device %d", p->device);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    int err;
-    if (use_tensor(p, &err)) {
+    int err = TQ_OK;
+    // Up to 32 rows per SM the reference-order kernel alone is faster than the tensor-core kernel with its second stage
+    // (four operations on the stream): TurboQuantProd, 2,048 rows: d = 64 10 against 28 us, d = 128 18 against 38, d = 256
+    // 43 against 84; 8,192 rows: 23 / 34, 44 / 45, 121 / 84.
+    const bool few = p->path == TQ_PATH_AUTO && n <= 32 * (int64_t)tq_sm_count(p->device);
+    if (!few && use_tensor(p, &err)) {
         const int64_t need = tq_quantize_scratch_bytes(p, n);
         if (!scratch || (int64_t)scratch_bytes < need)
             return tq_fail(TQ_ERR_SCRATCH_TOO_SMALL, "quantize scratch: need %lld bytes, got %zu", (long long)need, scratch_bytes);
@@ -300,13 +304,13 @@ static int quantize_common(const tq_plan* p, bool prod, const float* x, int64_t 
         TQ_TRY(tq_launch_exact_code_check(p, prod, x, n, static_cast<uint32_t*>(codes), &lists, st));
         tq_timer_mark(p, 2, 1, st);
         tq_timer_mark(p, 3, 0, st);
-        const int rc = tq_launch_exact_quantize(p, prod, x, n, static_cast<uint32_t*>(codes), static_cast<uint32_t*>(signs),
+        const int rc = tq_launch_exact_quantize(p, prod, x, TQ_F32, n, static_cast<uint32_t*>(codes), static_cast<uint32_t*>(signs),
                                                 rnorms, norms, &lists, p->counters, st);
         tq_timer_mark(p, 3, 1, st);
         return rc;
     }
     if (err != TQ_OK) return err;
-    return tq_launch_exact_quantize(p, prod, x, n, static_cast<uint32_t*>(codes), static_cast<uint32_t*>(signs), rnorms,
+    return tq_launch_exact_quantize(p, prod, x, TQ_F32, n, static_cast<uint32_t*>(codes), static_cast<uint32_t*>(signs), rnorms,
                                     norms, nullptr, nullptr, st);
 }
 
@@ -320,42 +324,64 @@ int tq_prod_quantize(const tq_plan* p, const float* x, int64_t n, void* codes, v
     return quantize_common(p, true, x, n, codes, signs, residual_norms, norms, scratch, scratch_bytes, stream);
 }
 
+static int check_encoding(const void* codes, const void* signs, const float* rn, const float* norms) {
+    TQ_TRY(check_ptr(codes, "codes"));
+    TQ_TRY(check_ptr(signs, "signs"));
+    TQ_TRY(check_ptr(rn, "residual_norms"));
+    TQ_TRY(check_ptr(norms, "norms"));
+    return TQ_OK;
+}
+
 // Append path: groups * tokens new vectors go behind the `*length` rows every group of a cache already holds.
 // One launch of the reference-order kernel (any d, any bits; the batches are small: one or a few tokens per
 // sequence and head), no scratch, no host knowledge of the length.
-static int append_common(const tq_plan* p, bool prod, const float* x, int groups, int tokens, void* codes, void* signs,
-                         float* rnorms, float* norms, int64_t capacity, int64_t* length, int advance, void* stream) {
-    TQ_TRY(check_plan(p, prod));
+static int append_common(const tq_plan* kp, const tq_plan* vp, const void* keys, const void* values, int dtype, int groups, int tokens,
+                         void* kcodes, void* ksigns, float* krnorms, float* knorms, void* vcodes, float* vnorms,
+                         int64_t capacity, int64_t* length, int advance, void* stream) {
+    if (!kp && !vp) return tq_fail(TQ_ERR_INVALID_ARGUMENT, "plan is null");
+    if (kp) TQ_TRY(check_plan(kp, true));
+    if (kp && vp && kp->device != vp->device) return tq_fail(TQ_ERR_INVALID_ARGUMENT, "key and value plans live on different devices");
+    if (kp && vp && kp->dev.d != vp->dev.d) return tq_fail(TQ_ERR_INVALID_ARGUMENT, "keys of dimension %d, values of %d", kp->dev.d, vp->dev.d);
+    if (dtype != TQ_F32 && dtype != TQ_BF16 && dtype != TQ_F16) return tq_fail(TQ_ERR_INVALID_ARGUMENT, "unknown element type %d", dtype);
     if (groups < 0 || tokens < 0 || capacity < 0) return tq_fail(TQ_ERR_INVALID_ARGUMENT, "negative size");
     if (tokens > capacity) return tq_fail(TQ_ERR_INVALID_ARGUMENT, "tokens (%d) exceed the capacity (%lld)", tokens, (long long)capacity);
     if ((double)groups * (double)capacity >= 4294967296.0)
         return tq_fail(TQ_ERR_INVALID_ARGUMENT, "groups * capacity must stay below 2^32");
     if (groups == 0 || tokens == 0) return TQ_OK;
-    TQ_TRY(check_ptr(x, "x"));
-    TQ_TRY(check_ptr(codes, "codes"));
-    TQ_TRY(check_ptr(norms, "norms"));
     TQ_TRY(check_ptr(length, "length"));
-    if (prod) {
-        TQ_TRY(check_ptr(signs, "signs"));
-        TQ_TRY(check_ptr(rnorms, "residual_norms"));
+    if (kp) {
+        TQ_TRY(check_ptr(keys, "keys"));
+        TQ_TRY(check_encoding(kcodes, ksigns, krnorms, knorms));
     }
-    DeviceScope scope(p->device);
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (vp) {
+        TQ_TRY(check_ptr(values, "values"));
+        TQ_TRY(check_ptr(vcodes, "value codes"));
+        TQ_TRY(check_ptr(vnorms, "value norms"));
+    }
+    DeviceScope scope((kp ? kp : vp)->device);
     const TqRowMap map{tokens, capacity, length};
-    TQ_TRY(tq_launch_exact_quantize(p, prod, x, (int64_t)groups * tokens, static_cast<uint32_t*>(codes),
-                                    static_cast<uint32_t*>(signs), rnorms, norms, nullptr, nullptr, st, &map));
-    if (advance) TQ_TRY(tq_launch_append_advance(length, tokens, capacity, st));
-    return TQ_OK;
+    return tq_launch_append(kp, keys, static_cast<uint32_t*>(kcodes), static_cast<uint32_t*>(ksigns), krnorms, knorms, vp, values,
+                            static_cast<uint32_t*>(vcodes), vnorms, dtype, (int64_t)groups * tokens, map, advance,
+                            static_cast<cudaStream_t>(stream));
 }
 
 int tq_mse_append(const tq_plan* p, const float* x, int groups, int tokens, void* codes, float* norms, int64_t capacity,
                   int64_t* length, int advance, void* stream) {
-    return append_common(p, false, x, groups, tokens, codes, nullptr, nullptr, norms, capacity, length, advance, stream);
+    return append_common(nullptr, p, nullptr, x, TQ_F32, groups, tokens, nullptr, nullptr, nullptr, nullptr, codes, norms, capacity,
+                         length, advance, stream);
 }
 
 int tq_prod_append(const tq_plan* p, const float* x, int groups, int tokens, void* codes, void* signs,
                    float* residual_norms, float* norms, int64_t capacity, int64_t* length, int advance, void* stream) {
-    return append_common(p, true, x, groups, tokens, codes, signs, residual_norms, norms, capacity, length, advance, stream);
+    return append_common(p, nullptr, x, nullptr, TQ_F32, groups, tokens, codes, signs, residual_norms, norms, nullptr, nullptr,
+                         capacity, length, advance, stream);
+}
+
+int tq_kv_append(const tq_plan* kplan, const tq_plan* vplan, const void* keys, const void* values, int dtype, int groups, int tokens,
+                 void* k_codes, void* k_signs, float* k_residual_norms, float* k_norms, void* v_codes, float* v_norms,
+                 int64_t capacity, int64_t* length, int advance, void* stream) {
+    return append_common(kplan, vplan, keys, values, dtype, groups, tokens, k_codes, k_signs, k_residual_norms, k_norms, v_codes,
+                         v_norms, capacity, length, advance, stream);
 }
 
 int tq_mse_quantize_noalloc(const tq_plan* p, const float* x, int64_t n, void* codes, float* norms, void* stream) {
@@ -417,14 +443,6 @@ int tq_prod_dequantize(const tq_plan* p, const void* codes, const void* signs, c
                                     residual_norms, norms, n, out, static_cast<cudaStream_t>(stream));
     return tq_launch_exact_dequantize(p, true, static_cast<const uint32_t*>(codes), static_cast<const uint32_t*>(signs),
                                       residual_norms, norms, n, out, static_cast<cudaStream_t>(stream));
-}
-
-static int check_encoding(const void* codes, const void* signs, const float* rn, const float* norms) {
-    TQ_TRY(check_ptr(codes, "codes"));
-    TQ_TRY(check_ptr(signs, "signs"));
-    TQ_TRY(check_ptr(rn, "residual_norms"));
-    TQ_TRY(check_ptr(norms, "norms"));
-    return TQ_OK;
 }
 
 int tq_score_broadcast(const tq_plan* p, const float* q, const void* codes, const void* signs,

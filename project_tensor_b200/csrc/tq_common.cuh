@@ -13,6 +13,8 @@
 #define TQ_MAX_DIM 1024
 #define TQ_MAX_BITS 8
 #define TQ_MAX_TOPK 1024
+// element types of quantizer inputs (TQ_F32 / TQ_BF16 / TQ_F16 of the C ABI)
+enum { TQ_INPUT_F32 = TQ_F32, TQ_INPUT_BF16 = TQ_BF16, TQ_INPUT_F16 = TQ_F16 };
 
 // Guard band (in units of a rotated unit-vector coordinate) inside which the tensor-core kernels
 // do not trust their own comparison against a decision boundary and hand the row to the exact
@@ -145,10 +147,12 @@ void tq_count_launch();
 // Exact (reference-order float32) kernels.  With `lists` null every row is computed; otherwise
 // first the listed coordinates are re-decided (tq_launch_exact_code_check), then the listed rows
 // are recomputed.
-int tq_launch_exact_quantize(const tq_plan* p, bool prod, const float* x, int64_t n, uint32_t* codes,
+int tq_launch_exact_quantize(const tq_plan* p, bool prod, const void* x, int xtype, int64_t n, uint32_t* codes,
                              uint32_t* signs, float* rnorms, float* norms, const TqRecheck* lists,
-                             unsigned long long* redo_counter, cudaStream_t st, const TqRowMap* map = nullptr);
-int tq_launch_append_advance(int64_t* length, int64_t tokens, int64_t capacity, cudaStream_t st);
+                             unsigned long long* redo_counter, cudaStream_t st);
+int tq_launch_append(const tq_plan* kp, const void* kx, uint32_t* kcodes, uint32_t* ksigns, float* krnorms, float* knorms,
+                     const tq_plan* vp, const void* vx, uint32_t* vcodes, float* vnorms, int xtype, int64_t rows,
+                     const TqRowMap& map, int advance, cudaStream_t st);
 int tq_launch_exact_code_check(const tq_plan* p, bool prod, const float* x, int64_t n, uint32_t* codes,
                                const TqRecheck* lists, cudaStream_t st);
 int tq_launch_exact_dequantize(const tq_plan* p, bool prod, const uint32_t* codes, const uint32_t* signs,

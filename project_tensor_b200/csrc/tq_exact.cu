@@ -11,8 +11,8 @@
 //     multiply-add per k, k ascending, starting from zero;
 //   * every other elementwise step is a separately rounded float32 operation (no contraction).
 //
-// One warp owns one row.  These kernels serve arbitrary (d <= 1024, bits <= 8); they are also the
-// second stage of the tensor-core quantizers, which hand over lists of coordinates and rows to re-decide.
+// These kernels serve arbitrary (d <= 1024, bits <= 8), single tokens appended to a cache and small batches; they are
+// also the second stage of the tensor-core quantizers, which hand over lists of coordinates and rows to re-decide.
 #include "tq_common.cuh"
 
 namespace {
@@ -47,12 +47,12 @@ __device__ float np_pairwise_sum(const float* s, int n, int lane) {
 }
 
 // np.searchsorted(boundaries, v, side="left"): boundaries strictly below v; NaN sorts last.
-__device__ __forceinline__ int count_below(const float* __restrict__ b, int nb, float v) {
+__device__ __forceinline__ int count_below(const float* b, int nb, float v) {
     if (v != v) return nb;
     int lo = 0, hi = nb;
     while (lo < hi) {
         const int mid = (lo + hi) >> 1;
-        if (__ldg(b + mid) < v) lo = mid + 1; else hi = mid;
+        if (b[mid] < v) lo = mid + 1; else hi = mid;
     }
     return lo;
 }
@@ -76,185 +76,516 @@ __device__ __forceinline__ void chain4(const float* vec, const float* __restrict
     }
 }
 
-__device__ __forceinline__ void store_packed_codes(const uint8_t* cs, int d, int bits, int words, int lane,
-                                                   uint32_t* out) {
-    for (int w = lane; w < words; w += 32) {
-        const int lo_bit = w * 32;
-        uint32_t v = 0;
-        for (int j = lo_bit / bits; j < d && j * bits < lo_bit + 32; ++j) {
-            const int sh = j * bits - lo_bit;
-            v |= sh >= 0 ? ((uint32_t)cs[j] << sh) : ((uint32_t)cs[j] >> (-sh));
+// Word w of a packed code row from the row's codes (bytes; zero behind d, eight readable bytes behind the last).  Codes are
+// fetched eight at a time, so that a word costs a few loads in flight together and not one after the other.
+__device__ __forceinline__ uint32_t packed_code_word(const uint8_t* cs, int bits, uint32_t inv_bits, int w) {
+    const int lo_bit = w * 32;
+    int j = (int)((uint32_t)lo_bit * inv_bits >> 16);        // lo_bit / bits
+    int at = j * bits - lo_bit;                              // bit position of code j in the word, <= 0 for the first
+    uint32_t v = 0;
+    while (at < 32) {
+        uint32_t c[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) c[i] = cs[j + i];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (at < 0) v |= c[i] >> -at;
+            else if (at < 32) v |= c[i] << at;
+            at += bits;
         }
-        out[w] = v;
+        j += 8;
+    }
+    return v;
+}
+// floor(x / bits) = x * inverse >> 16 for x <= 8192 and bits <= 8
+__device__ __forceinline__ uint32_t inverse_of_bits(int bits) { return (65536u + (uint32_t)bits - 1u) / (uint32_t)bits; }
+
+// Boundaries strictly below v among levels - 1 sorted ones (a power of two less one): np.searchsorted(..., side="left");
+// NaN sorts last.  N values at a time: every step of the bisection is a dependent load.
+template <int N>
+__device__ __forceinline__ void codes_of(const float* bnd, int levels, const float (&v)[N], int (&code)[N]) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) code[i] = 0;
+    for (int step = levels >> 1; step > 0; step >>= 1) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) code[i] += bnd[code[i] + step - 1] < v[i] ? step : 0;
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) code[i] = v[i] != v[i] ? levels - 1 : code[i];
+}
+
+// Sum of squares of n values of one row (v[k * stride], k ascending) in NumPy's pairwise scheme, by eight lanes.
+template <int STRIDE>
+__device__ float np_sumsq8(const float* v, int n, int l8) {
+    auto sq = [&](int i) { const float a = v[i * STRIDE]; return __fmul_rn(a, a); };
+    if (n < 8) {
+        float r = 0.f;
+        for (int i = 0; i < n; ++i) r = __fadd_rn(r, sq(i));
+        return r;
+    }
+    if (n <= 128) {
+        const int nb = n - (n & 7);
+        float r = sq(l8);
+        if (nb == 128) {
+            float a[15];
+#pragma unroll
+            for (int i = 0; i < 15; ++i) a[i] = sq(8 + 8 * i + l8);
+#pragma unroll
+            for (int i = 0; i < 15; ++i) r = __fadd_rn(r, a[i]);
+        } else {
+#pragma unroll 4
+            for (int i = 8; i < nb; i += 8) r = __fadd_rn(r, sq(i + l8));
+        }
+        r = __fadd_rn(r, __shfl_xor_sync(0xffffffffu, r, 1));
+        r = __fadd_rn(r, __shfl_xor_sync(0xffffffffu, r, 2));
+        r = __fadd_rn(r, __shfl_xor_sync(0xffffffffu, r, 4));
+        for (int i = nb; i < n; ++i) r = __fadd_rn(r, sq(i));
+        return r;
+    }
+    int h = n >> 1;
+    h -= h & 7;
+    const float a = np_sumsq8<STRIDE>(v, h, l8);
+    const float b = np_sumsq8<STRIDE>(v + h * STRIDE, n - h, l8);
+    return __fadd_rn(a, b);
+}
+
+// Values l8, l8 + 8, ... of a row (row < 0: zeros) into v[k * stride], by eight lanes; bf16 and fp16 widened to float32.
+// Sixteen loads are in flight at a time; the element type is looked at once.
+template <class Load>
+__device__ __forceinline__ void fill_row(float* v, int stride, int d, int l8, bool have, Load load) {
+    for (int k0 = l8; k0 < d; k0 += 128) {
+        float q[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) q[i] = have && k0 + 8 * i < d ? load(k0 + 8 * i) : 0.f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (k0 + 8 * i < d) v[(k0 + 8 * i) * stride] = q[i];
+    }
+}
+__device__ __forceinline__ float widen(uint16_t u, int xtype) {
+    return xtype == TQ_INPUT_BF16 ? __uint_as_float((uint32_t)u << 16) : __half2float(__ushort_as_half(u));
+}
+__device__ __forceinline__ void load_row(float* v, int stride, int d, int l8, const void* x, int xtype, int64_t row) {
+    const bool have = row >= 0;
+    const int64_t at = (have ? row : 0) * d;
+    if (xtype == TQ_INPUT_F32) {
+        const float* src = static_cast<const float*>(x) + at;
+        fill_row(v, stride, d, l8, have, [&](int k) { return __ldg(src + k); });
+    } else {
+        const uint16_t* src = static_cast<const uint16_t*>(x) + at;
+        fill_row(v, stride, d, l8, have, [&](int k) { return widen(__ldg(src + k), xtype); });
+    }
+}
+// Division of a row by its norm (zero rows stay zero); the same lanes own the same values.
+__device__ __forceinline__ void divide_row(float* v, int stride, int d, int l8, float nr) {
+    const bool ok = nr > 0.f;
+#pragma unroll 4
+    for (int k = l8; k < d; k += 8) {
+        const float q = v[k * stride];
+        v[k * stride] = ok ? __fdiv_rn(q, nr) : 0.f;
     }
 }
 
-// TurboQuantMSE.quantize / TurboQuantProd.quantize, array part (_quant.py:224-236, 300-308).
-// One block works on kRB rows at a time with one thread per output coordinate, so that every matrix
-// element fetched from L1/L2 feeds kRB chains; the vectors sit in shared memory transposed ([k][row])
-// and are read as broadcast float4s.
-constexpr int kRB = 8;
-
-struct RowsSmem {
-    float* vt;      // [d][kRB]   unit vectors, later residuals (transposed)
-    float* ct;      // [d][kRB]   centroid values (transposed)
-    float* sq;      // [kRB][dp]  squares, row-major for the pairwise sums
-    uint8_t* cs;    // [kRB][dp]  codes
-    float* nrm;     // [kRB]
+// ------------------------------------------------------------------------------------------------
+// Rows against whole matrices
+// ------------------------------------------------------------------------------------------------
+// One set of rows to quantize; a launch takes up to two (the keys and the values of a cache step).
+struct RowsJob {
+    TqDev p;
+    const void* x;          // [n][d], element type `xtype`
+    int xtype;              // TqInput
+    int prod;               // TurboQuantProd: residual norm and signs behind the codes
+    int64_t n;
+    uint32_t* codes;
+    uint32_t* signs;
+    float* rnorms;
+    float* norms;
+    TqRecheck lists;        // hdr != null: only the listed rows
+    unsigned long long* redo_counter;
+    TqRowMap map;           // tokens > 0: rows of a cache
 };
-__host__ __device__ inline size_t rows_smem_bytes(int d) {
-    const int dp = (d + 31) & ~31;
-    return (size_t)(2 * d * kRB + kRB * dp + kRB) * sizeof(float) + (size_t)kRB * dp + 64;
+
+// Where rows come from and go to.  Every thread of a block holds the same values.
+struct RowSource {
+    int64_t limit, len0;
+    bool listed, mapped;
+    __device__ __forceinline__ void open(const RowsJob& job, bool first_block) {
+        mapped = job.map.tokens > 0;
+        len0 = mapped ? (*reinterpret_cast<volatile const int64_t*>(job.map.length) & ((1ll << 40) - 1)) : 0;
+        const TqRecheckHeader* hdr = job.lists.hdr;
+        // all rows, or the rows of the list (every row again if a list overflowed)
+        listed = hdr != nullptr && hdr->overflow == 0;
+        limit = listed ? (int64_t)min(hdr->n_rows, job.lists.row_cap) : job.n;
+        if (hdr != nullptr && job.redo_counter && first_block && threadIdx.x == 0) *job.redo_counter = (unsigned long long)limit;
+    }
+    __device__ __forceinline__ int64_t src(const RowsJob& job, int64_t idx) const {
+        int64_t row = idx < limit ? (listed ? (int64_t)job.lists.row_entries[idx] : idx) : -1;
+        return row < job.n ? row : -1;
+    }
+    __device__ __forceinline__ int64_t dst(const RowsJob& job, int64_t row) const {
+        if (!mapped || row < 0) return row;
+        const int64_t grow = row / job.map.tokens, pos = len0 + (row - grow * job.map.tokens);
+        return pos < job.map.capacity ? grow * job.map.capacity + pos : -1;   // a full cache takes no more rows
+    }
+};
+
+// The last block of a launch to get here raises the cache length.  Blocks count themselves in bits 40 and up of that very
+// word, which are zero again when the kernel ends, so a step needs neither a second launch nor a counter of its own.
+// (Every block has read the length before it counts itself.)
+__device__ __forceinline__ void advance_length(const RowsJob& job, int64_t len0) {
+    unsigned long long* len = reinterpret_cast<unsigned long long*>(const_cast<int64_t*>(job.map.length));
+    const unsigned long long before = atomicAdd(len, 1ull << 40);
+    if ((before >> 40) == gridDim.x - 1) {
+        const int64_t v = len0 + job.map.tokens;
+        atomicExch(len, (unsigned long long)(v < job.map.capacity ? v : job.map.capacity));
+    }
 }
 
-// acc[r] = sum_k vt[k][r] * M[k * d + tj] for the kRB rows of a block: one FMA per k, k ascending.  The U matrix
-// elements of a batch are fetched before the first of them is used -- written out as two loops because the
-// chains wait on L2 latency, and whether the compiler hoists the loads of a single loop by itself changed the
-// kernel's time by a factor of two from one build to the next.
-template <int U>
-__device__ __forceinline__ void rows_chain(const float* __restrict__ M, int d, int tj, const float* vt, float (&acc)[kRB]) {
+// Few rows, d <= 128 (a decode step's tokens, a handful of vectors): RB rows per block, the three matrices copied whole into
+// shared memory (64 bytes a cycle and SM from L2: 1.6 us for the 192 KB of d = 128) while the rows are normalised; one thread
+// per output, so that a product is a 128-long FMA chain with its loads running ahead.  64 keys and 64 values of d = 128 with the
+// length: 10.8 us in one launch (18.6 + 10.6 + 1.2 us in three before).
+template <int RB>
+__global__ void __launch_bounds__(128 * RB)
+exact_quantize_few_kernel(const __grid_constant__ RowsJob first, const __grid_constant__ RowsJob second, int blocks0, int advance) {
+    extern __shared__ __align__(16) float smem[];
+    __shared__ __align__(16) float vt[RB][128], ct[RB][128];   // unit vector, later residual; centroids
+    __shared__ uint8_t cs[RB][128 + 8];
+    __shared__ float bnd[256], cbk[256];
+    const bool one = (int)blockIdx.x < blocks0;
+    const RowsJob& job = one ? first : second;
+    const int block = one ? blockIdx.x : blockIdx.x - blocks0, nblocks = one ? blocks0 : gridDim.x - blocks0;
+    const TqDev& p = job.p;
+    const int d = p.d, levels = p.levels, dd4 = (d * d + 3) / 4;      // 16-byte pieces of a matrix (the slab is padded)
+    const bool prod = job.prod != 0;
+    constexpr int kThreads = 128 * RB;
+    const int t = threadIdx.x, r = t >> 7, j = t & 127, lane = t & 31;
+    auto copy = [&](int which, const float* M) {
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(smem + which * dd4 * 4);
+#pragma unroll 8
+        for (int i = t; i < dd4; i += kThreads)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + i * 16), "l"(M + i * 4) : "memory");
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto product = [&](int which, const float* vec) {
+        const float* m = smem + which * dd4 * 4 + (j < d ? j : 0);
+        float acc = 0.f;
+        int k = 0;
+        for (; k + 16 <= d; k += 16) {
+            float b[16];
 #pragma unroll
-    for (int r = 0; r < kRB; ++r) acc[r] = 0.f;
-    int k0 = 0;
-    for (; k0 + U <= d; k0 += U) {
-        float m[U];
+            for (int i = 0; i < 16; ++i) b[i] = m[(k + i) * d];
 #pragma unroll
-        for (int u = 0; u < U; ++u) m[u] = __ldg(M + (size_t)(k0 + u) * d + tj);
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const float4 a = *reinterpret_cast<const float4*>(vt + (k0 + u) * kRB);
-            const float4 b = *reinterpret_cast<const float4*>(vt + (k0 + u) * kRB + 4);
-            acc[0] = __fmaf_rn(a.x, m[u], acc[0]); acc[1] = __fmaf_rn(a.y, m[u], acc[1]);
-            acc[2] = __fmaf_rn(a.z, m[u], acc[2]); acc[3] = __fmaf_rn(a.w, m[u], acc[3]);
-            acc[4] = __fmaf_rn(b.x, m[u], acc[4]); acc[5] = __fmaf_rn(b.y, m[u], acc[5]);
-            acc[6] = __fmaf_rn(b.z, m[u], acc[6]); acc[7] = __fmaf_rn(b.w, m[u], acc[7]);
+            for (int i = 0; i < 16; i += 4) {
+                const float4 v = *reinterpret_cast<const float4*>(vec + k + i);
+                acc = __fmaf_rn(v.x, b[i], acc);
+                acc = __fmaf_rn(v.y, b[i + 1], acc);
+                acc = __fmaf_rn(v.z, b[i + 2], acc);
+                acc = __fmaf_rn(v.w, b[i + 3], acc);
+            }
+        }
+        for (; k < d; ++k) acc = __fmaf_rn(vec[k], m[k * d], acc);
+        return acc;
+    };
+    copy(0, p.Rt);
+    if (prod) { copy(1, p.R); copy(2, p.St); }
+    for (int i = t; i < levels; i += kThreads) {
+        cbk[i] = __ldg(p.codebook + i);
+        if (i + 1 < levels) bnd[i] = __ldg(p.boundaries + i);
+    }
+    if (j < 8) cs[r][128 + j] = 0;
+    const uint32_t inv_bits = inverse_of_bits(p.bits);
+    RowSource rows;
+    rows.open(job, block == 0);
+    for (int64_t g0 = (int64_t)block * RB; g0 < rows.limit; g0 += (int64_t)nblocks * RB) {
+        const int64_t row = rows.src(job, g0 + r), to = rows.dst(job, row);
+        __syncthreads();
+        if (j < 8) {     // eight lanes per row: load, sum of squares, divide
+            // (the other lanes of the warp wait here; with 16 values per lane the row is in flight at once)
+            load_row(vt[r], 1, d, j, job.x, job.xtype, row);
+        }
+        if (j < 32) {
+            __syncwarp();
+            const float nr = __fsqrt_rn(np_sumsq8<1>(vt[r], d, lane & 7));
+            __syncwarp();
+            if (j < 8) divide_row(vt[r], 1, d, j, nr);
+            if (j == 0 && to >= 0) job.norms[to] = nr;
+        }
+        if (prod) asm volatile("cp.async.wait_group 2;" ::: "memory");
+        else asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        {
+            const float rotated[1] = {product(0, vt[r])};
+            int code[1];
+            codes_of<1>(bnd, levels, rotated, code);
+            cs[r][j] = j < d ? (uint8_t)code[0] : 0;
+            ct[r][j] = cbk[code[0]];
+        }
+        if (prod) asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        if (to >= 0 && j >= 128 - 32 && (int)(j - 96) < 32)     // the last warp of the row packs
+            for (int w = j - 96; w < p.code_words; w += 32) job.codes[to * p.code_words + w] = packed_code_word(cs[r], p.bits, inv_bits, w);
+        if (!prod) continue;
+        const float res = __fsub_rn(vt[r][j], product(1, ct[r]));
+        vt[r][j] = res;
+        __syncthreads();
+        if (j < 32) {
+            const float rn = __fsqrt_rn(np_sumsq8<1>(vt[r], d, lane & 7));
+            if (j == 0 && to >= 0) job.rnorms[to] = rn;
+        }
+        const float v = product(2, vt[r]);
+        const uint32_t word = __ballot_sync(0xffffffffu, j < d && v >= 0.f);
+        if (lane == 0 && j < d && to >= 0) job.signs[to * p.sign_words + (j >> 5)] = tq_sign_word_from_natural(word);
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (advance) {
+        __syncthreads();
+        if (t == 0) advance_length(job, rows.len0);
+    }
+}
+
+// Any d, any number of rows: a block takes RB = RT * TR rows through every step of a call, the matrices stream through shared
+// memory.  The vectors lie transposed ([k][row], padded to RB + 4); a thread owns TR rows x TC columns (column c of thread tx:
+// tx + CT * c), loads TR + TC values per k and multiplies TR * TC.  The shared-memory pipe delivers one 32-lane register a
+// cycle where the FMA pipes take four, so many rows want 8 x 8 sums per thread.  The matrices come in chunks of consecutive
+// k -- all d columns, so a chunk is one contiguous piece of memory -- through a ring filled by cp.async, which runs ahead
+// over the boundaries between the products and between groups of rows.
+// TurboQuantProd, 65,536 rows (one thread per column with 8 rows before): d = 96 171 us, d = 128 251 us (0.37 ms before), bound by
+// the FMA and shared-memory pipes (47 % of the FMA rate) and the phases between the products; the listed rows of 1,048,576 keys 18 us
+// (29 us before).
+template <int RT, int TR, int CT, int TC>
+struct Tile {
+    static constexpr int kRB = RT * TR, kRS = kRB + 4, kThreads = RT * CT, kCols = CT * TC;
+    static_assert(TR % 4 == 0 && kThreads % 32 == 0, "tile");
+};
+struct TileShape {
+    int kc;              // k per chunk (a multiple of 4, so that every chunk starts on a 16-byte boundary)
+    int stages;
+    int chunk_floats;    // ring stage, a multiple of 4
+    size_t bytes;
+};
+// vectors: transposed arrays of d x kRS floats; the columns behind d of a panel are read (and their sums ignored)
+template <class T>
+TileShape tile_shape(int d, int vectors, size_t extra_bytes, size_t room) {
+    TileShape s{};
+    const size_t fixed = (size_t)vectors * d * T::kRS * 4 + extra_bytes + 64 + T::kCols * 4;
+    for (int floats = 8192; floats >= 1024; floats >>= 1) {
+        s.kc = floats / d / 4 * 4;
+        if (s.kc < 4) s.kc = 4;
+        s.chunk_floats = (s.kc * d + 3) / 4 * 4;
+        for (s.stages = 4; s.stages >= (floats > 1024 ? 3 : 2); --s.stages) {
+            s.bytes = fixed + (size_t)s.stages * s.chunk_floats * 4;
+            if (s.bytes <= room) return s;
         }
     }
-    for (; k0 < d; ++k0) {
-        const float m = __ldg(M + (size_t)k0 * d + tj);
-        const float4 a = *reinterpret_cast<const float4*>(vt + k0 * kRB);
-        const float4 b = *reinterpret_cast<const float4*>(vt + k0 * kRB + 4);
-        acc[0] = __fmaf_rn(a.x, m, acc[0]); acc[1] = __fmaf_rn(a.y, m, acc[1]);
-        acc[2] = __fmaf_rn(a.z, m, acc[2]); acc[3] = __fmaf_rn(a.w, m, acc[3]);
-        acc[4] = __fmaf_rn(b.x, m, acc[4]); acc[5] = __fmaf_rn(b.y, m, acc[5]);
-        acc[6] = __fmaf_rn(b.z, m, acc[6]); acc[7] = __fmaf_rn(b.w, m, acc[7]);
-    }
+    s.stages = 0;
+    return s;
 }
 
-// MAPPED: results go to the rows the append map names (a cache) instead of the input's own row numbers; a
-// separate instantiation, so that the plain quantizer carries none of it.
-// MAXT: the largest block the instantiation is launched with (d rounded up to 32).  The small one may use up to
-// 255 registers and keeps 32 matrix elements in flight per thread (rows_chain).
-template <bool PROD, bool MAPPED, int MAXT>
-__global__ void __launch_bounds__(MAXT)
-exact_quantize_kernel(TqDev p, const float* __restrict__ x, int64_t n, uint32_t* __restrict__ codes,
-                      uint32_t* __restrict__ signs, float* __restrict__ rnorms, float* __restrict__ norms,
-                      TqRecheck lists, unsigned long long* redo_counter, TqRowMap map) {
-    extern __shared__ float smem[];
-    const int d = p.d, dp = (d + 31) & ~31;
-    const int64_t len0 = MAPPED ? *map.length : 0;
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nwarps = blockDim.x >> 5;
-    RowsSmem sm;
-    sm.vt = smem;
-    sm.ct = sm.vt + (size_t)d * kRB;
-    sm.sq = sm.ct + (size_t)d * kRB;
-    sm.nrm = sm.sq + (size_t)kRB * dp;
-    sm.cs = reinterpret_cast<uint8_t*>(sm.nrm + kRB);
-    const int tj = t < d ? t : d - 1;  // coordinate this thread computes (threads beyond d mirror the last one)
+template <int THREADS>
+struct MatrixRing {
+    float* stage;
+    const float *m0, *m1, *m2;
+    int nmat, d, kc, stages, chunk_floats;
+    int m, k0;                  // next chunk to ask for
+    int head, tail;             // stages: next to fill, next to use
+    __device__ __forceinline__ void start(float* stage_, const float* a, const float* b, const float* c, int nmat_, int d_, const TileShape& t) {
+        stage = stage_; m0 = a; m1 = b; m2 = c; nmat = nmat_; d = d_;
+        kc = t.kc; stages = t.stages; chunk_floats = t.chunk_floats;
+        m = k0 = head = tail = 0;
+        for (int i = 0; i + 1 < stages; ++i) fetch();
+    }
+    __device__ __forceinline__ void fetch() {
+        const float* src = (m == 0 ? m0 : m == 1 ? m1 : m2) + (size_t)k0 * d;
+        const int n = min(kc, d - k0);
+        const int pieces = (n * d + 3) >> 2;      // the last piece may read a few bytes past the matrix, into the slab's padding
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(stage + head * chunk_floats);
+#pragma unroll 4
+        for (int i = threadIdx.x; i < pieces; i += THREADS)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + i * 16), "l"(src + i * 4) : "memory");
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        head = head + 1 == stages ? 0 : head + 1;
+        k0 += kc;
+        if (k0 >= d) { k0 = 0; m = m + 1 == nmat ? 0 : m + 1; }
+    }
+    __device__ __forceinline__ void wait() const {
+        if (stages == 4) asm volatile("cp.async.wait_group 2;" ::: "memory");
+        else if (stages == 3) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        else asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+};
 
-    // all rows, or the rows of the list (every row again if a list overflowed)
-    const bool listed = lists.hdr != nullptr && lists.hdr->overflow == 0;
-    const int64_t limit = listed ? (int64_t)min(lists.hdr->n_rows, lists.row_cap) : n;
-    if (lists.hdr != nullptr && redo_counter && blockIdx.x == 0 && t == 0)
-        *redo_counter = (unsigned long long)limit;     // rows redone by this call (a plain store: no clearing launch needed)
-
-    for (int64_t g0 = (int64_t)blockIdx.x * kRB; g0 < limit; g0 += (int64_t)gridDim.x * kRB) {
-        int64_t rows[kRB];                    // input rows (-1: none)
-        int64_t mapped[MAPPED ? kRB : 1];     // MAPPED: the rows their results go to
+// acc[r][c] = sum_k vt[k][row r] * M[k][column c]: one FMA per k, k ascending.
+template <int RT, int TR, int CT, int TC>
+__device__ __forceinline__ void tile_product(MatrixRing<RT * CT>& ring, const float* vt, int tx, int ty, float (&acc)[TR][TC]) {
+    constexpr int kRS = Tile<RT, TR, CT, TC>::kRS;
+    float2 two[TR / 2][TC];          // pairs of rows: fma.rn.f32x2 rounds each half as fma.rn.f32 does, in half the instructions
 #pragma unroll
-        for (int r = 0; r < kRB; ++r) {
-            const int64_t idx = g0 + r;
-            int64_t row = idx < limit ? (listed ? (int64_t)lists.row_entries[idx] : idx) : -1;
-            if (row >= n) row = -1;
-            rows[r] = row;
-            if (MAPPED) {
-                mapped[r] = row;
-                if (row >= 0) {
-                    const int64_t grp = row / map.tokens, pos = len0 + (row - grp * map.tokens);
-                    mapped[r] = pos < map.capacity ? grp * map.capacity + pos : -1;   // a full cache takes no more rows
+    for (int r = 0; r < TR / 2; ++r)
+#pragma unroll
+        for (int c = 0; c < TC; ++c) two[r][c] = make_float2(0.f, 0.f);
+    const int d = ring.d;
+    for (int k0 = 0; k0 < d; k0 += ring.kc) {
+        ring.wait();
+        __syncthreads();             // this chunk has landed for every thread, and everyone is done with the one before
+        ring.fetch();
+        const float* mt = ring.stage + ring.tail * ring.chunk_floats + tx;
+        const float* v = vt + (size_t)k0 * kRS + ty * TR;
+        ring.tail = ring.tail + 1 == ring.stages ? 0 : ring.tail + 1;
+        const int n = min(ring.kc, d - k0);
+#pragma unroll 4
+        for (int k = 0; k < n; ++k) {
+            float a[TR], b[TC];
+#pragma unroll
+            for (int r = 0; r < TR; r += 4) *reinterpret_cast<float4*>(a + r) = *reinterpret_cast<const float4*>(v + k * kRS + r);
+#pragma unroll
+            for (int c = 0; c < TC; ++c) b[c] = mt[k * d + CT * c];
+#pragma unroll
+            for (int c = 0; c < TC; ++c)
+#pragma unroll
+                for (int r = 0; r < TR / 2; ++r)
+                    two[r][c] = __ffma2_rn(make_float2(a[2 * r], a[2 * r + 1]), make_float2(b[c], b[c]), two[r][c]);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < TR / 2; ++r)
+#pragma unroll
+        for (int c = 0; c < TC; ++c) {
+            acc[2 * r][c] = two[r][c].x;
+            acc[2 * r + 1][c] = two[r][c].y;
+        }
+}
+
+template <int RT, int TR, int CT, int TC>
+__global__ void __launch_bounds__(RT * CT, 384 / (RT * CT))
+exact_quantize_tile_kernel(const __grid_constant__ RowsJob first, const __grid_constant__ RowsJob second, int blocks0, int advance,
+                           const TileShape shape) {
+    using T = Tile<RT, TR, CT, TC>;
+    constexpr int RB = T::kRB, RS = T::kRS, kGroups = T::kThreads / 8, kCodeRow = T::kCols + 8;
+    extern __shared__ __align__(16) float smem[];
+    const bool one = (int)blockIdx.x < blocks0;
+    const RowsJob& job = one ? first : second;
+    const int block = one ? blockIdx.x : blockIdx.x - blocks0, nblocks = one ? blocks0 : gridDim.x - blocks0;
+    const TqDev& p = job.p;
+    const int d = p.d, levels = p.levels;
+    const bool prod = job.prod != 0;
+    float* vt = smem;                                        // [d][RS] unit vectors, later residuals
+    float* ct = vt + (size_t)d * RS;                         // [d][RS] centroid values
+    uint8_t* cs = reinterpret_cast<uint8_t*>(ct + (size_t)d * RS);   // [RB][kCodeRow] codes
+    float* stage = reinterpret_cast<float*>(cs + RB * kCodeRow);     // the ring, last: columns behind d are read past its end
+    __shared__ float bnd[256], cbk[256];
+    __shared__ int64_t src_row[RB], dst_row[RB];
+    const int t = threadIdx.x, tx = t % CT, ty = t / CT, lane = t & 31, l8 = t & 7, grp = t >> 3;
+    RowSource rows;
+    if (job.lists.hdr != nullptr && !prod) {     // the list of a TurboQuantMSE call is empty as a rule
+        rows.open(job, block == 0);
+        if (rows.limit == 0) return;
+    }
+    MatrixRing<T::kThreads> ring;
+    ring.start(stage, p.Rt, p.R, p.St, prod ? 3 : 1, d, shape);
+    for (int i = t; i < levels; i += T::kThreads) {
+        cbk[i] = __ldg(p.codebook + i);
+        if (i + 1 < levels) bnd[i] = __ldg(p.boundaries + i);
+    }
+    rows.open(job, block == 0);
+    const uint32_t inv_bits = inverse_of_bits(p.bits);
+    if (t < RB)
+        for (int i = 0; i < 8; ++i) cs[t * kCodeRow + T::kCols + i] = 0;
+    for (int64_t g0 = (int64_t)block * RB; g0 < rows.limit; g0 += (int64_t)nblocks * RB) {
+        __syncthreads();             // the previous group is written out
+        if (t < RB) {
+            src_row[t] = rows.src(job, g0 + t);
+            dst_row[t] = rows.dst(job, src_row[t]);
+        }
+        __syncthreads();
+        // eight lanes per row: load, sum of squares, divide (lanes without a row keep the warp's shuffles company)
+        for (int r0 = 0; r0 < RB; r0 += kGroups) {
+            const bool mine = r0 + grp < RB;
+            const int r = mine ? r0 + grp : RB - 1;
+            const int64_t row = src_row[r];
+            float* v = vt + r;
+            if (mine) load_row(v, RS, d, l8, job.x, job.xtype, row);
+            __syncwarp();
+            const float nr = __fsqrt_rn(np_sumsq8<RS>(v, d, l8));
+            __syncwarp();
+            if (mine) {
+                divide_row(v, RS, d, l8, nr);
+                if (l8 == 0 && dst_row[r] >= 0) job.norms[dst_row[r]] = nr;
+            }
+        }
+        // (the barrier in front of the first chunk orders the vectors)
+        float acc[TR][TC];
+        // rotated[j] = sum_k unit[k] * R[j][k] -> codes, centroids
+        tile_product<RT, TR, CT, TC>(ring, vt, tx, ty, acc);
+#pragma unroll
+        for (int c = 0; c < TC; ++c) {
+            const int j = tx + CT * c;
+            float v[TR], cent[TR];
+            int code[TR];
+#pragma unroll
+            for (int r = 0; r < TR; ++r) v[r] = acc[r][c];
+            codes_of<TR>(bnd, levels, v, code);
+#pragma unroll
+            for (int r = 0; r < TR; ++r) {
+                cs[(ty * TR + r) * kCodeRow + j] = j < d ? (uint8_t)code[r] : 0;
+                cent[r] = cbk[code[r]];
+            }
+            if (prod && j < d) {
+#pragma unroll
+                for (int r = 0; r < TR; r += 4)
+                    *reinterpret_cast<float4*>(ct + j * RS + ty * TR + r) = make_float4(cent[r], cent[r + 1], cent[r + 2], cent[r + 3]);
+            }
+        }
+        __syncthreads();
+        for (int i = t; i < RB * p.code_words; i += T::kThreads) {
+            const int r = i / p.code_words, w = i - r * p.code_words;
+            if (dst_row[r] >= 0) job.codes[dst_row[r] * p.code_words + w] = packed_code_word(cs + r * kCodeRow, p.bits, inv_bits, w);
+        }
+        if (!prod) continue;
+        // recon[j] = sum_k centroid[k] * R[k][j];  residual = unit - recon, in place (only this thread touches its elements)
+        tile_product<RT, TR, CT, TC>(ring, ct, tx, ty, acc);
+#pragma unroll
+        for (int c = 0; c < TC; ++c) {
+            const int j = tx + CT * c;
+            if (j < d) {
+#pragma unroll
+                for (int r = 0; r < TR; r += 4) {
+                    float4* at = reinterpret_cast<float4*>(vt + j * RS + ty * TR + r);
+                    const float4 u = *at;
+                    *at = make_float4(__fsub_rn(u.x, acc[r][c]), __fsub_rn(u.y, acc[r + 1][c]), __fsub_rn(u.z, acc[r + 2][c]),
+                                      __fsub_rn(u.w, acc[r + 3][c]));
                 }
             }
         }
-        const int64_t* orow = MAPPED ? mapped : rows;
-        __syncthreads();  // previous group fully written out
-#pragma unroll
-        for (int r = 0; r < kRB; ++r) {
-            const float v = (rows[r] >= 0 && t < d) ? x[rows[r] * d + t] : 0.f;
-            if (t < dp) sm.sq[r * dp + t] = __fmul_rn(v, v);
-            if (t < d) sm.vt[t * kRB + r] = v;
-        }
         __syncthreads();
-        for (int r = warp; r < kRB; r += nwarps) {
-            const float nr = __fsqrt_rn(np_pairwise_sum(sm.sq + r * dp, d, lane));
-            if (lane == 0) sm.nrm[r] = nr;
+        for (int r0 = 0; r0 < RB; r0 += kGroups) {
+            const bool mine = r0 + grp < RB;
+            const int r = mine ? r0 + grp : RB - 1;
+            const float rn = __fsqrt_rn(np_sumsq8<RS>(vt + r, d, l8));
+            if (mine && l8 == 0 && dst_row[r] >= 0) job.rnorms[dst_row[r]] = rn;
         }
-        __syncthreads();
-        if (t < d) {
+        // projected[j] = sum_k residual[k] * S[j][k] -> signs.  A ballot holds kBits consecutive columns of 32 / kBits rows.
+        tile_product<RT, TR, CT, TC>(ring, vt, tx, ty, acc);
+        constexpr int kBits = CT < 32 ? CT : 32, kPer = 32 / kBits;      // ballots per sign word
+        constexpr uint32_t kMask = kBits == 32 ? 0xffffffffu : (1u << kBits) - 1u;
+        const int shift = (lane / kBits) * kBits;
 #pragma unroll
-            for (int r = 0; r < kRB; ++r) {
-                const float nr = sm.nrm[r];
-                sm.vt[t * kRB + r] = nr > 0.f ? __fdiv_rn(sm.vt[t * kRB + r], nr) : 0.f;
-            }
-        }
-        __syncthreads();
-
-        float acc[kRB];
-        constexpr int kU = MAXT <= 256 ? 32 : 16;   // matrix elements in flight per thread (64 and 128 were slower: 50 and 62 us
-                                                    // against 33 us for the listed rows of 1,048,576 keys)
-        // rotated[j] = sum_k unit[k] * R[j][k]
-        rows_chain<kU>(p.Rt, d, tj, sm.vt, acc);
-        if (t < d) {
+        for (int r = 0; r < TR; ++r) {
+            const int64_t to = dst_row[ty * TR + r];
 #pragma unroll
-            for (int r = 0; r < kRB; ++r) {
-                const int code = count_below(p.boundaries, p.levels - 1, acc[r]);
-                sm.cs[r * dp + t] = (uint8_t)code;
-                if (PROD) sm.ct[t * kRB + r] = __ldg(p.codebook + code);
-            }
-        }
-        __syncthreads();
-        for (int r = warp; r < kRB; r += nwarps) {
-            if (orow[r] < 0) continue;
-            store_packed_codes(sm.cs + r * dp, d, p.bits, p.code_words, lane, codes + orow[r] * p.code_words);
-            if (lane == 0) norms[orow[r]] = sm.nrm[r];
-        }
-
-        if (PROD) {
-            // recon[j] = sum_k centroid[k] * R[k][j];  residual = unit - recon
-            rows_chain<kU>(p.R, d, tj, sm.ct, acc);
-            __syncthreads();  // nobody reads unit[k] of other coordinates any more
+            for (int c0 = 0; c0 < TC; c0 += kPer) {
+                uint32_t word = 0;
 #pragma unroll
-            for (int r = 0; r < kRB; ++r) {
-                const float res = t < d ? __fsub_rn(sm.vt[t * kRB + r], acc[r]) : 0.f;
-                if (t < d) sm.vt[t * kRB + r] = res;
-                if (t < dp) sm.sq[r * dp + t] = __fmul_rn(res, res);
-            }
-            __syncthreads();
-            for (int r = warp; r < kRB; r += nwarps) {
-                const float rn = __fsqrt_rn(np_pairwise_sum(sm.sq + r * dp, d, lane));
-                if (lane == 0 && orow[r] >= 0) rnorms[orow[r]] = rn;
-            }
-            // projected[j] = sum_k residual[k] * S[j][k]
-            rows_chain<kU>(p.St, d, tj, sm.vt, acc);
-#pragma unroll
-            for (int r = 0; r < kRB; ++r) {
-                const uint32_t word = __ballot_sync(0xffffffffu, t < d && acc[r] >= 0.f);
-                if (lane == 0 && orow[r] >= 0 && warp * 32 < d)
-                    signs[orow[r] * p.sign_words + warp] = tq_sign_word_from_natural(word);
+                for (int c = c0; c < c0 + kPer && c < TC; ++c)
+                    word |= ((__ballot_sync(0xffffffffu, tx + CT * c < d && acc[r][c] >= 0.f) >> shift) & kMask) << ((c - c0) * kBits);
+                const int j0 = tx / kBits * kBits + CT * c0;      // first column of the word
+                if (lane == shift && j0 < d && to >= 0) job.signs[to * p.sign_words + (j0 >> 5)] = tq_sign_word_from_natural(word);
             }
         }
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (advance && t == 0) advance_length(job, rows.len0);
 }
-
 
 // Second stage of the tensor-core quantizers, part 1: one thread per listed (row, coordinate).
 // The coordinate's rotated value is recomputed exactly as the reference does (norm by pairwise sum,
@@ -367,68 +698,55 @@ exact_code_check_kernel(TqDev p, bool prod, const float* __restrict__ x, int64_t
     }
 }
 
-// TurboQuantMSE.dequantize / TurboQuantProd.dequantize (_quant.py:238-242,251-254,317-332).
-// Same block shape as the quantizer above: kRB rows per pass, one thread per output coordinate.
-template <bool PROD>
-__global__ void __launch_bounds__(1024)
-exact_dequantize_kernel(TqDev p, const uint32_t* __restrict__ codes, const uint32_t* __restrict__ signs,
-                        const float* __restrict__ rnorms, const float* __restrict__ norms, int64_t n,
-                        float* __restrict__ out) {
-    extern __shared__ float smem[];
-    const int d = p.d, t = threadIdx.x;
-    float* ct = smem;                        // [d][kRB] centroid values (transposed)
-    float* st = ct + (size_t)d * kRB;        // [d][kRB] +-1 signs (transposed), Prod only
-    const int tj = t < d ? t : d - 1;
-    for (int64_t g0 = (int64_t)blockIdx.x * kRB; g0 < n; g0 += (int64_t)gridDim.x * kRB) {
+// TurboQuantMSE.dequantize / TurboQuantProd.dequantize (_quant.py:238-242,251-254,317-332): the block shape of
+// exact_quantize_tile_kernel.
+template <bool PROD, int RT, int TR, int CT, int TC>
+__global__ void __launch_bounds__(RT * CT, 384 / (RT * CT))
+exact_dequantize_tile_kernel(const __grid_constant__ TqDev p, const uint32_t* __restrict__ codes, const uint32_t* __restrict__ signs,
+                             const float* __restrict__ rnorms, const float* __restrict__ norms, int64_t n,
+                             float* __restrict__ out, const TileShape shape) {
+    using T = Tile<RT, TR, CT, TC>;
+    constexpr int RB = T::kRB, RS = T::kRS;
+    extern __shared__ __align__(16) float smem[];
+    const int d = p.d;
+    float* ct = smem;                                        // [d][RS] centroid values
+    float* sg = ct + (size_t)d * RS;                         // [d][RS] +-1
+    float* stage = sg + (PROD ? (size_t)d * RS : 0);
+    __shared__ float cbk[256];
+    const int t = threadIdx.x, tx = t % CT, ty = t / CT, l8 = t & 7, grp = t >> 3;
+    MatrixRing<T::kThreads> ring;
+    ring.start(stage, p.R, p.S, p.S, PROD ? 2 : 1, d, shape);
+    for (int i = t; i < p.levels; i += T::kThreads) cbk[i] = __ldg(p.codebook + i);
+    for (int64_t g0 = (int64_t)blockIdx.x * RB; g0 < n; g0 += (int64_t)gridDim.x * RB) {
         __syncthreads();
-        if (t < d) {
-#pragma unroll
-            for (int r = 0; r < kRB; ++r) {
-                const int64_t row = g0 + r;
-                float c = 0.f, sg = 0.f;
-                if (row < n) {
-                    c = __ldg(p.codebook + tq_get_code(codes + row * p.code_words, t, p.bits));
-                    if (PROD) sg = ((signs[row * p.sign_words + (t >> 5)] >> tq_sign_bitpos(t)) & 1u) ? 1.f : -1.f;
-                }
-                ct[t * kRB + r] = c;
-                if (PROD) st[t * kRB + r] = sg;
+        for (int r = grp; r < RB; r += T::kThreads / 8) {
+            const int64_t row = g0 + r < n ? g0 + r : 0;
+            const uint32_t* crow = codes + row * p.code_words;
+            const uint32_t* srow = PROD ? signs + row * p.sign_words : nullptr;
+#pragma unroll 4
+            for (int k = l8; k < d; k += 8) {
+                ct[k * RS + r] = cbk[tq_get_code(crow, k, p.bits)];
+                if (PROD) sg[k * RS + r] = ((__ldg(srow + (k >> 5)) >> tq_sign_bitpos(k)) & 1u) ? 1.f : -1.f;
             }
         }
-        __syncthreads();
-        float acc[kRB], acs[kRB];
+        float acc[TR][TC], acs[PROD ? TR : 4][TC];
+        tile_product<RT, TR, CT, TC>(ring, ct, tx, ty, acc);
+        if constexpr (PROD) tile_product<RT, TR, CT, TC>(ring, sg, tx, ty, acs);
 #pragma unroll
-        for (int r = 0; r < kRB; ++r) { acc[r] = 0.f; acs[r] = 0.f; }
-#pragma unroll 8
-        for (int k = 0; k < d; ++k) {
-            const float m = __ldg(p.R + (size_t)k * d + tj);
-            const float4 a = *reinterpret_cast<const float4*>(ct + k * kRB);
-            const float4 b = *reinterpret_cast<const float4*>(ct + k * kRB + 4);
-            acc[0] = __fmaf_rn(a.x, m, acc[0]); acc[1] = __fmaf_rn(a.y, m, acc[1]);
-            acc[2] = __fmaf_rn(a.z, m, acc[2]); acc[3] = __fmaf_rn(a.w, m, acc[3]);
-            acc[4] = __fmaf_rn(b.x, m, acc[4]); acc[5] = __fmaf_rn(b.y, m, acc[5]);
-            acc[6] = __fmaf_rn(b.z, m, acc[6]); acc[7] = __fmaf_rn(b.w, m, acc[7]);
-            if (PROD) {
-                const float ms = __ldg(p.S + (size_t)k * d + tj);
-                const float4 e = *reinterpret_cast<const float4*>(st + k * kRB);
-                const float4 f = *reinterpret_cast<const float4*>(st + k * kRB + 4);
-                acs[0] = __fmaf_rn(e.x, ms, acs[0]); acs[1] = __fmaf_rn(e.y, ms, acs[1]);
-                acs[2] = __fmaf_rn(e.z, ms, acs[2]); acs[3] = __fmaf_rn(e.w, ms, acs[3]);
-                acs[4] = __fmaf_rn(f.x, ms, acs[4]); acs[5] = __fmaf_rn(f.y, ms, acs[5]);
-                acs[6] = __fmaf_rn(f.z, ms, acs[6]); acs[7] = __fmaf_rn(f.w, ms, acs[7]);
-            }
-        }
-        if (t < d) {
+        for (int r = 0; r < TR; ++r) {
+            const int64_t row = g0 + ty * TR + r;
+            if (row >= n) continue;
+            const float nr = __ldg(norms + row), rn = PROD ? __ldg(rnorms + row) : 0.f;
 #pragma unroll
-            for (int r = 0; r < kRB; ++r) {
-                const int64_t row = g0 + r;
-                if (row < n) {
-                    float u = acc[r];
-                    if (PROD) u = __fadd_rn(u, __fmul_rn(__fmul_rn(acs[r], p.alpha), rnorms[row]));
-                    out[row * d + t] = __fmul_rn(u, norms[row]);
-                }
+            for (int c = 0; c < TC; ++c) {
+                const int j = tx + CT * c;
+                float u = acc[r][c];
+                if (PROD) u = __fadd_rn(u, __fmul_rn(__fmul_rn(acs[r][c], p.alpha), rn));
+                if (j < d) out[row * d + j] = __fmul_rn(u, nr);
             }
         }
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
 // TurboQuantProd.attention_score with one query row per key (_quant.py:342-358), in the
@@ -518,71 +836,157 @@ int tq_launch_exact_code_check(const tq_plan* p, bool prod, const float* x, int6
     return TQ_OK;
 }
 
-int tq_launch_exact_quantize(const tq_plan* p, bool prod, const float* x, int64_t n, uint32_t* codes,
-                             uint32_t* signs, float* rnorms, float* norms, const TqRecheck* lists_in,
-                             unsigned long long* redo_counter, cudaStream_t st, const TqRowMap* map_in) {
+namespace {
+// Blocks for `rows` rows of one job out of `room` that run at once.
+int job_blocks(int64_t rows, int per_block, int64_t room) {
+    const int64_t g = (rows + per_block - 1) / per_block;
+    return (int)(g < 1 ? 1 : g < room ? g : room < 1 ? 1 : room);
+}
+// Of two jobs that share a launch the first (TurboQuantProd keys, three products per row) gets two thirds of the blocks.
+void split_room(const RowsJob* b, int64_t rows, int per_block, int64_t room, int* b0, int* b1) {
+    *b0 = job_blocks(rows, per_block, b ? room * 2 / 3 : room);
+    *b1 = b ? job_blocks(rows, per_block, room - *b0) : 0;
+}
+
+template <int RB>
+int launch_few_rows(const RowsJob& a, const RowsJob* b, int64_t rows, int device, int advance, cudaStream_t st) {
+    int b0, b1;
+    split_room(b, rows, RB, tq_sm_count(device), &b0, &b1);
+    const int sm = (a.prod || (b && b->prod) ? 3 : 1) * ((a.p.d * a.p.d + 3) / 4 * 16);
+    TQ_GRANT_SMEM((exact_quantize_few_kernel<RB>), sm, device);
+    exact_quantize_few_kernel<RB><<<b0 + b1, 128 * RB, sm, st>>>(a, b ? *b : a, b0, advance); tq_count_launch();
+    TQ_CUDA_TRY(cudaGetLastError());
+    return TQ_OK;
+}
+// Blocks of a kernel that an SM's registers hold (its shared memory is a matter of the shape); asked for once per kernel.
+template <class K>
+int blocks_by_registers(K kernel, int threads) {
+    cudaFuncAttributes attr;
+    if (cudaFuncGetAttributes(&attr, kernel) != cudaSuccess || attr.numRegs <= 0) return 1;
+    const int blocks = 65536 / ((attr.numRegs + 7) / 8 * 8 * threads);
+    return blocks < 1 ? 1 : blocks > 8 ? 8 : blocks;
+}
+// Blocks per SM that shared memory leaves room for, at most `most`; the ring takes what is left.
+template <class T>
+TileShape best_shape(int d, int vectors, size_t extra, int most, int64_t groups, int sms, int* per_sm) {
+    TileShape s{};
+    if (groups < (int64_t)most * sms) most = (int)((groups + sms - 1) / sms);    // fewer blocks, longer rings
+    if (most < 1) most = 1;
+    for (int k = most; k >= 1; --k) {
+        s = tile_shape<T>(d, vectors, extra, (size_t)227 * 1024 / k - 5 * 1024);    // 5 KB: static shared memory and the system's share
+        *per_sm = k;
+        if (s.stages >= (k > 1 ? 3 : 2)) return s;
+    }
+    s.stages = 0;
+    return s;
+}
+template <int RT, int TR, int CT, int TC>
+int launch_tile_rows(const RowsJob& a, const RowsJob* b, int64_t rows, int device, int advance, cudaStream_t st) {
+    using T = Tile<RT, TR, CT, TC>;
+    int per_sm, b0, b1;
+    static const int most = blocks_by_registers(exact_quantize_tile_kernel<RT, TR, CT, TC>, T::kThreads);
+    const TileShape shape = best_shape<T>(a.p.d, 2, (size_t)T::kRB * (T::kCols + 8), most, (rows * (b ? 2 : 1) + T::kRB - 1) / T::kRB,
+                                           tq_sm_count(device), &per_sm);
+    if (shape.stages == 0) return tq_fail(TQ_ERR_UNSUPPORTED, "no tile shape for d=%d", a.p.d);
+    split_room(b, rows, T::kRB, (int64_t)tq_sm_count(device) * per_sm, &b0, &b1);
+    TQ_GRANT_SMEM((exact_quantize_tile_kernel<RT, TR, CT, TC>), shape.bytes, device);
+    exact_quantize_tile_kernel<RT, TR, CT, TC><<<b0 + b1, T::kThreads, shape.bytes, st>>>(a, b ? *b : a, b0, advance, shape); tq_count_launch();
+    TQ_CUDA_TRY(cudaGetLastError());
+    return TQ_OK;
+}
+// Rows per block: one while every row can have an SM to itself (d <= 128), then four, 16 (8 at d = 256) while larger blocks would leave
+// SMs idle, 64 or 32 from there on.
+int launch_rows(const RowsJob& a, const RowsJob* b, int64_t rows, int device, int advance, cudaStream_t st) {
+    const int d = a.p.d;
+    const int64_t sms = tq_sm_count(device), total = b ? 2 * rows : rows;
+    if (d <= 128 && total <= sms) return launch_few_rows<1>(a, b, rows, device, advance, st);
+    if (d <= 128 && total <= sms * 4) return launch_few_rows<4>(a, b, rows, device, advance, st);
+    const bool many = total > sms * 32;
+    if (d <= 64) return many ? launch_tile_rows<16, 4, 8, 8>(a, b, rows, device, advance, st) : launch_tile_rows<4, 4, 32, 2>(a, b, rows, device, advance, st);
+    if (d <= 96) return many ? launch_tile_rows<16, 4, 8, 12>(a, b, rows, device, advance, st) : launch_tile_rows<4, 4, 32, 3>(a, b, rows, device, advance, st);
+    if (d <= 128) return many ? launch_tile_rows<8, 8, 16, 8>(a, b, rows, device, advance, st) : launch_tile_rows<4, 4, 32, 4>(a, b, rows, device, advance, st);
+    if (d <= 256) {
+        if (total <= sms * 8) return launch_tile_rows<2, 4, 64, 4>(a, b, rows, device, advance, st);
+        return many ? launch_tile_rows<4, 8, 32, 8>(a, b, rows, device, advance, st) : launch_tile_rows<2, 8, 64, 4>(a, b, rows, device, advance, st);
+    }
+    if (d <= 512) return launch_tile_rows<4, 4, 64, 8>(a, b, rows, device, advance, st);
+    return launch_tile_rows<4, 4, 64, 16>(a, b, rows, device, advance, st);
+}
+RowsJob rows_job(const tq_plan* p, bool prod, const void* x, int xtype, int64_t n, uint32_t* codes, uint32_t* signs, float* rnorms,
+                 float* norms, const TqRecheck* lists, unsigned long long* redo_counter, const TqRowMap* map) {
+    RowsJob j{};
+    j.p = p->dev; j.x = x; j.xtype = xtype; j.prod = prod ? 1 : 0; j.n = n;
+    j.codes = codes; j.signs = signs; j.rnorms = rnorms; j.norms = norms;
+    if (lists) j.lists = *lists;
+    j.redo_counter = redo_counter;
+    if (map) j.map = *map;
+    return j;
+}
+}  // namespace
+
+int tq_launch_exact_quantize(const tq_plan* p, bool prod, const void* x, int xtype, int64_t n, uint32_t* codes,
+                             uint32_t* signs, float* rnorms, float* norms, const TqRecheck* lists,
+                             unsigned long long* redo_counter, cudaStream_t st) {
     TqRange range("tq.quantize.exact_rows");
     if (n == 0) return TQ_OK;
-    const size_t sm = rows_smem_bytes(p->dev.d);
-    const TqRowMap map = map_in ? *map_in : TqRowMap{0, 0, nullptr};
-    TqRecheck none{};
-    const TqRecheck lists = lists_in ? *lists_in : none;
-    // the listed pass does not know its size on the host: a fixed grid strides over the list
-    const int grid = lists_in ? 148 * 4 : grid_for(n, kRB);
-    const int threads = (p->dev.d + 31) & ~31;
-#define TQ_LAUNCH_EXACT(P, M, T)                                                                                           \
-    do {                                                                                                                  \
-        TQ_GRANT_SMEM((exact_quantize_kernel<P, M, T>), sm, p->device); \
-        exact_quantize_kernel<P, M, T><<<grid, threads, sm, st>>>(p->dev, x, n, codes, signs, rnorms, norms, lists, redo_counter, map); tq_count_launch(); \
-    } while (0)
-#define TQ_LAUNCH_EXACT_T(P, M)                  \
-    do {                                         \
-        if (threads <= 256) TQ_LAUNCH_EXACT(P, M, 256); \
-        else TQ_LAUNCH_EXACT(P, M, 1024);        \
-    } while (0)
-    const bool mapped = map.tokens > 0;
-    if (prod) {
-        if (mapped) TQ_LAUNCH_EXACT_T(true, true);
-        else TQ_LAUNCH_EXACT_T(true, false);
-    } else {
-        if (mapped) TQ_LAUNCH_EXACT_T(false, true);
-        else TQ_LAUNCH_EXACT_T(false, false);
-    }
-#undef TQ_LAUNCH_EXACT_T
-#undef TQ_LAUNCH_EXACT
+    const RowsJob job = rows_job(p, prod, x, xtype, n, codes, signs, rnorms, norms, lists, redo_counter, nullptr);
+    // A listed pass does not know its size on the host.  About one row in 450 of a TurboQuantProd call at d = 128 is listed
+    // (the coordinate re-check and the sign guard), hardly any of a TurboQuantMSE call; the blocks stride on where it is more.
+    const int64_t rows = !lists ? n : prod ? n * p->dev.d / 128 / 384 + 1 : n / 65536 + 1;
+    return launch_rows(job, nullptr, rows, p->device, 0, st);
+}
+
+// One step of a cache: the keys of `kp` (TurboQuantProd), the values of `vp` (TurboQuantMSE), or both (either plan may be
+// null), in one launch.
+int tq_launch_append(const tq_plan* kp, const void* kx, uint32_t* kcodes, uint32_t* ksigns, float* krnorms, float* knorms,
+                     const tq_plan* vp, const void* vx, uint32_t* vcodes, float* vnorms, int xtype, int64_t rows,
+                     const TqRowMap& map, int advance, cudaStream_t st) {
+    TqRange range("tq.append");
+    RowsJob k{}, v{};
+    if (kp) k = rows_job(kp, true, kx, xtype, rows, kcodes, ksigns, krnorms, knorms, nullptr, nullptr, &map);
+    if (vp) v = rows_job(vp, false, vx, xtype, rows, vcodes, nullptr, nullptr, vnorms, nullptr, nullptr, &map);
+    return launch_rows(kp ? k : v, kp && vp ? &v : nullptr, rows, (kp ? kp : vp)->device, advance, st);
+}
+
+namespace {
+template <bool PROD, int RT, int TR, int CT, int TC>
+int launch_tile_dequant(const tq_plan* p, const uint32_t* codes, const uint32_t* signs, const float* rnorms, const float* norms,
+                        int64_t n, float* out, cudaStream_t st) {
+    using T = Tile<RT, TR, CT, TC>;
+    int per_sm;
+    static const int most = blocks_by_registers(exact_dequantize_tile_kernel<PROD, RT, TR, CT, TC>, T::kThreads);
+    const TileShape shape = best_shape<T>(p->dev.d, PROD ? 2 : 1, 0, most, (n + T::kRB - 1) / T::kRB, tq_sm_count(p->device), &per_sm);
+    if (shape.stages == 0) return tq_fail(TQ_ERR_UNSUPPORTED, "no tile shape for d=%d", p->dev.d);
+    const int grid = job_blocks(n, T::kRB, (int64_t)tq_sm_count(p->device) * per_sm);
+    TQ_GRANT_SMEM((exact_dequantize_tile_kernel<PROD, RT, TR, CT, TC>), shape.bytes, p->device);
+    exact_dequantize_tile_kernel<PROD, RT, TR, CT, TC><<<grid, T::kThreads, shape.bytes, st>>>(p->dev, codes, signs, rnorms, norms, n, out, shape);
+    tq_count_launch();
     TQ_CUDA_TRY(cudaGetLastError());
     return TQ_OK;
 }
-
-__global__ void append_advance_kernel(int64_t* length, int64_t tokens, int64_t capacity) {
-    const int64_t v = *length + tokens;
-    *length = v < capacity ? v : capacity;
+template <bool PROD>
+int launch_dequant_for(const tq_plan* p, const uint32_t* codes, const uint32_t* signs, const float* rnorms, const float* norms,
+                       int64_t n, float* out, cudaStream_t st) {
+    const int d = p->dev.d;
+    const bool many = n > (int64_t)tq_sm_count(p->device) * 32;
+#define TQ_DQ(...) return launch_tile_dequant<PROD, __VA_ARGS__>(p, codes, signs, rnorms, norms, n, out, st)
+    if (d <= 64) { if (many) TQ_DQ(16, 4, 8, 8); TQ_DQ(4, 4, 32, 2); }
+    if (d <= 96) { if (many) TQ_DQ(16, 4, 8, 12); TQ_DQ(4, 4, 32, 3); }
+    if (d <= 128) { if (many) TQ_DQ(16, 4, 16, 8); TQ_DQ(4, 4, 32, 4); }
+    if (d <= 256) { if (many) TQ_DQ(8, 4, 32, 8); TQ_DQ(2, 4, 64, 4); }
+    if (d <= 512) TQ_DQ(4, 4, 64, 8);
+    TQ_DQ(4, 4, 64, 16);
+#undef TQ_DQ
 }
-
-int tq_launch_append_advance(int64_t* length, int64_t tokens, int64_t capacity, cudaStream_t st) {
-    append_advance_kernel<<<1, 1, 0, st>>>(length, tokens, capacity); tq_count_launch();
-    TQ_CUDA_TRY(cudaGetLastError());
-    return TQ_OK;
-}
+}  // namespace
 
 int tq_launch_exact_dequantize(const tq_plan* p, bool prod, const uint32_t* codes, const uint32_t* signs,
                                const float* rnorms, const float* norms, int64_t n, float* out,
                                cudaStream_t st) {
     TqRange range("tq.dequantize.exact");
     if (n == 0) return TQ_OK;
-    const int d = p->dev.d;
-    const size_t sm = (size_t)2 * d * kRB * sizeof(float);
-    const int grid = grid_for(n, kRB);
-    const int threads = (d + 31) & ~31;
-    if (prod) {
-        TQ_GRANT_SMEM((exact_dequantize_kernel<true>), sm, p->device);
-        exact_dequantize_kernel<true><<<grid, threads, sm, st>>>(p->dev, codes, signs, rnorms, norms, n, out); tq_count_launch();
-    } else {
-        TQ_GRANT_SMEM((exact_dequantize_kernel<false>), sm, p->device);
-        exact_dequantize_kernel<false><<<grid, threads, sm, st>>>(p->dev, codes, signs, rnorms, norms, n, out); tq_count_launch();
-    }
-    TQ_CUDA_TRY(cudaGetLastError());
-    return TQ_OK;
+    return prod ? launch_dequant_for<true>(p, codes, signs, rnorms, norms, n, out, st)
+                : launch_dequant_for<false>(p, codes, signs, rnorms, norms, n, out, st);
 }
 
 int tq_launch_exact_pairwise(const tq_plan* p, const float* q, const uint32_t* codes, const uint32_t* signs,

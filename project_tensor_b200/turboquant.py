@@ -447,6 +447,7 @@ def quantize_to_host(quantizer, keys, chunk_rows: int = 131072, out: Optional[Di
     if n == 0:
         return host
     chunk_rows = max(1, min(int(chunk_rows), n))
+    chunk_rows = -(-n // -(-n // chunk_rows))    # chunks of one size: no short one at the end, which would take another kernel
     with torch.cuda.device(device):
         s_in, s_run, s_out = torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.Stream()
         for s_ in (s_in, s_run, s_out):
