@@ -200,6 +200,20 @@ int tq_plan_create(int d, int bits_mse, const float* rotation, const float* code
     *p->status_host = 0ull;
     p->status_dev = static_cast<unsigned long long*>(word_dev);
 
+    for (int k = 0; k < levels; ++k) p->c_max = fmaxf(p->c_max, fabsf(codebook[k]));
+    if (projection && p->c_max > 0.f && p->c_max < 50.f) {
+        // |S q| <= longest row of S * |q| and the queries are scaled so that the largest coordinate of R q is below 2^20 / |q| *
+        // sqrt(d): this power of two keeps the rescaled S q of any query below the fp16 range
+        double longest = 0.0;
+        for (int j = 0; j < d; ++j) {
+            double sum = 0.0;
+            for (int k = 0; k < d; ++k) sum += (double)projection[(size_t)j * d + k] * projection[(size_t)j * d + k];
+            longest = fmax(longest, sqrt(sum));
+        }
+        const double need = longest * sqrt((double)d) * 1048576.0 / 60000.0;
+        if (need < 1.0e6) p->beta_scale = (float)exp2(ceil(log2(fmax(need, 1.0))));
+    }
+
     p->tensor_ok = false;
     if (tq_tensor_quantize_supported(d, bits_mse, projection != nullptr)) {
         const int r = tq_tensor_plan_init(p, rotation, codebook, projection);

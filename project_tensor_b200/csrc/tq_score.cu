@@ -149,6 +149,15 @@ merge_keys_kernel(const unsigned long long* __restrict__ part, int lists, int qp
     __shared__ int count;
     __shared__ unsigned long long thr;   // keys at or below it cannot be among the k best any more
     const int qi = blockIdx.x, g = blockIdx.y;
+    if (lists == 1) {       // a single list is sorted already
+        for (int i = threadIdx.x; i < topk; i += blockDim.x) {
+            const size_t o = ((size_t)g * qpg + qi) * topk + i;
+            const unsigned long long ck = part[o];
+            top_scores[o] = ck == 0ull ? -INFINITY : unordered_bits((uint32_t)(ck >> 32));
+            top_idx[o] = ck == 0ull ? -1 : idx_base + (int64_t)(0xffffffffu - (uint32_t)ck);
+        }
+        return;
+    }
     if (threadIdx.x == 0) { count = 0; thr = 0ull; }
     __syncthreads();
     // all slots of all lists in batches, whatever the number of lists (some callers bring hundreds of short
@@ -202,6 +211,22 @@ merge_pairs_kernel(const float* __restrict__ in_scores, const int64_t* __restric
     extern __shared__ __align__(16) unsigned char smraw[];
     unsigned long long* a = reinterpret_cast<unsigned long long*>(smraw);  // [2*k2]
     const int qi = blockIdx.x;
+    if (lists == 1) {       // one shard: its list as it is, when it is in order (scores falling, empty slots last)
+        const float* s = in_scores + (size_t)qi * topk;
+        const int64_t* x = in_idx + (size_t)qi * topk;
+        bool disorder = false;
+        for (int i = threadIdx.x; i + 1 < topk; i += blockDim.x)
+            disorder |= x[i + 1] >= 0 && (x[i] < 0 || !(s[i] >= s[i + 1]));
+        if (!__syncthreads_or(disorder)) {
+            for (int i = threadIdx.x; i < topk; i += blockDim.x) {
+                const size_t o = (size_t)qi * topk + i;
+                const bool have = x[i] >= 0;
+                out_scores[o] = have ? s[i] : -INFINITY;
+                out_idx[o] = have ? x[i] : -1;
+            }
+            return;
+        }
+    }
     for (int i = threadIdx.x; i < 2 * k2; i += blockDim.x) a[i] = 0ull;
     __syncthreads();
     for (int l = 0; l < lists; ++l) {
@@ -261,7 +286,7 @@ ScoreGeometry geometry(int groups, int64_t keys_per_group, int topk) {
 
 }  // namespace
 
-int64_t tq_score_tc_scratch(int groups, int qpg, int64_t keys_per_group, int topk);
+int64_t tq_score_tc_scratch(const tq_plan* p, int groups, int qpg, int64_t keys_per_group, int topk);
 int tq_launch_score_tc(const tq_plan* p, const float* q, int groups, int qpg, const uint32_t* codes,
                        const uint32_t* signs, const float* rnorms, const float* norms, int64_t keys_per_group,
                        float* scores, int topk, float* top_scores, int64_t* top_idx, int64_t idx_base, void* scratch,
@@ -279,7 +304,7 @@ static int64_t general_topk_scratch(int groups, int qpg, int64_t keys_per_group,
 
 int64_t tq_score_topk_scratch(const tq_plan* p, int groups, int qpg, int64_t keys_per_group, int topk) {
     const int64_t a = general_topk_scratch(groups, qpg, keys_per_group, topk);
-    const int64_t b = tq_tensor_quantize_supported(p->dev.d, p->dev.bits, true) ? tq_score_tc_scratch(groups, qpg, keys_per_group, topk) : 0;
+    const int64_t b = tq_tensor_quantize_supported(p->dev.d, p->dev.bits, true) ? tq_score_tc_scratch(p, groups, qpg, keys_per_group, topk) : 0;
     return a > b ? a : b;
 }
 

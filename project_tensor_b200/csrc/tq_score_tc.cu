@@ -24,12 +24,15 @@
 #include "tq_common.cuh"
 #include "tq_ptx.cuh"
 #include "tq_topk.cuh"
+#include "tq_filter.cuh"
 
 #include <cuda.h>
 #include <math.h>
 #include <math_constants.h>
 #include <stdlib.h>
 #include <string.h>
+
+#include <algorithm>
 
 namespace {
 
@@ -86,6 +89,8 @@ struct ScoreTcArgs {
     unsigned int* cnt;            // [groups][qpg_total] entries appended to each list
     unsigned long long* cand;     // [groups][qpg_total][cand_cap]
     int64_t cand_cap;
+    const unsigned int* dyn_keys; // keys that are really there (one group; tiles behind them are skipped); null: key_cnt
+    const unsigned int* run_if;   // the launch does nothing when this word is zero; null: always runs
     float alpha;
     unsigned long long* status;
     int wait_kcycles;             // limit of one bounded wait, in units of 1024 cycles
@@ -196,6 +201,8 @@ score_tc_kernel(const __grid_constant__ CUtensorMap tmap_out, const ScoreTcArgs 
     auto BAR = [&](int i) { return bar0 + 8u * (uint32_t)i; };
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     TQ_PROF_CODE(const long long prof_t0 = clock64();)
+    if (a.run_if && *a.run_if == 0u) return;
+    const int64_t total_tiles = a.dyn_keys ? ((int64_t)*a.dyn_keys + kTileKeys - 1) / kTileKeys : a.total_tiles;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < kStages; ++i) {
@@ -241,8 +248,8 @@ score_tc_kernel(const __grid_constant__ CUtensorMap tmap_out, const ScoreTcArgs 
     TQ_PROF_CODE(const long long prof_t1 = clock64();)
 
     // contiguous tile range of this CTA, so that it rarely changes group
-    const int64_t t0 = a.total_tiles * (int64_t)blockIdx.x / gridDim.x;
-    const int64_t t1 = a.total_tiles * (int64_t)(blockIdx.x + 1) / gridDim.x;
+    const int64_t t0 = total_tiles * (int64_t)blockIdx.x / gridDim.x;
+    const int64_t t1 = total_tiles * (int64_t)(blockIdx.x + 1) / gridDim.x;
     // Instruction descriptors for N = QPAD and N = 2*QPAD (hi and lo query halves side by side).
     constexpr uint32_t kIdesc1 = (1u << 4) | ((uint32_t)(QPAD >> 3) << 17) | ((uint32_t)(kTileKeys >> 4) << 24);
     constexpr uint32_t kIdesc2 = (1u << 4) | ((uint32_t)(2 * QPAD >> 3) << 17) | ((uint32_t)(kTileKeys >> 4) << 24);
@@ -1136,7 +1143,9 @@ topk_rows_kernel(const float* __restrict__ scores, int64_t row_stride, int64_t g
 // first threshold) leaves the best list alone: its keys will be scored again by the full pass.
 __global__ void __launch_bounds__(256)
 select_candidates_kernel(const unsigned long long* __restrict__ cand, unsigned int* __restrict__ cnt, int64_t cap,
-                         unsigned long long* __restrict__ best, float* __restrict__ thr, int qpg, int topk, int k2, int mode) {
+                         unsigned long long* __restrict__ best, float* __restrict__ thr, int qpg, int topk, int k2, int mode,
+                         const unsigned int* run_if) {
+    if (run_if && *run_if == 0u) return;
     __shared__ __align__(16) unsigned long long a[kSelCap];
     __shared__ int hist[256];
     __shared__ int scratch[4];
@@ -1190,7 +1199,8 @@ select_candidates_kernel(const unsigned long long* __restrict__ cand, unsigned i
 
 // thresholds to -inf, best lists to empty, list lengths to `first_count` (what the sampled pass will leave in them; 0 without one)
 __global__ void init_candidates_kernel(float* thr, unsigned int* cnt, unsigned long long* best, int64_t lists, int topk,
-                                       unsigned int first_count) {
+                                       unsigned int first_count, const unsigned int* run_if) {
+    if (run_if && *run_if == 0u) return;
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < lists) { thr[i] = -CUDART_INF_F; cnt[i] = first_count; }
     if (i < lists * topk) best[i] = 0ull;
@@ -1222,6 +1232,12 @@ int launch_score(const tq_plan* p, const CUtensorMap& map, const ScoreTcArgs& ar
 #ifndef TQ_SCORE_PASS
 #define TQ_SCORE_PASS 64     // queries per scoring launch at d <= 128 (32: the measurement build without passes of 64)
 #endif
+
+#define TQ_STEP(expr)                         \
+    do {                                      \
+        const int rc__ = (expr);              \
+        if (rc__ != TQ_OK) return rc__;       \
+    } while (0)
 
 // ---- host-side planning ---------------------------------------------------------------------------
 constexpr int64_t kChunkKeys = 1 << 22;     // keys per group scored into scratch at a time when only top-k is wanted
@@ -1268,7 +1284,7 @@ struct CandPlan {
 static CandPlan plan_candidates(int groups, int qpg, int64_t keys_per_group, int topk) {
     CandPlan s{};
     auto pad = [](size_t b) { return (b + 255) & ~size_t(255); };
-    s.chunk = kCandChunk;
+    s.chunk = keys_per_group < kCandChunk ? (keys_per_group < 1 ? 1 : keys_per_group) : kCandChunk;
     s.nchunks = (keys_per_group + s.chunk - 1) / s.chunk;
     s.cand_cap = s.chunk;
     s.lists = (int64_t)groups * qpg;
@@ -1287,7 +1303,44 @@ static bool use_candidates(const float* scores, int topk, int64_t keys_per_group
     return scores == nullptr && topk > 0 && keys_per_group > 2 * kCandChunk;
 }
 
-int64_t tq_score_tc_scratch(int groups, int qpg, int64_t keys_per_group, int topk) {
+// Filtered search (tq_score_filter.cu): one group of keys, no matrix, and lists short enough that a round's keys can be
+// gathered: a round whose threshold comes from 1 / r of its keys lists about r * topk keys per query.
+// Its fixed part (a sample, two rounds, the skipped fallback: some 25 launches) costs about 80 us, what it saves grows with keys
+// and queries.  Search through an index, before / with it: 1,048,576 keys, 64 queries 300 / 249 us, 32 queries 210 / 198, 8 queries
+// 160 / 160; 2,097,152 keys, 8 queries 246 / 214, 1 query 219 / 183; 8,388,608 keys, 64 queries 1502 / 622, 1 query 1004 / 424.
+constexpr int64_t kFilterFrom = 1 << 21, kFilterFromMany = 1 << 20;      // keys from which on it pays; from 32 queries on
+constexpr int64_t kFilterSample = 1 << 15;     // keys of the first sample
+constexpr int kFilterRoom = 1 << 18;           // gathered keys of a round
+static bool use_filter(const tq_plan* p, const float* scores, int groups, int qpg, int topk, int64_t keys_per_group) {
+    const int nq = qpg < 64 ? qpg : 64;
+    return scores == nullptr && topk > 0 && groups == 1 && p->beta_scale > 0.f && keys_per_group >= (qpg >= 32 ? kFilterFromMany : kFilterFrom) &&
+           keys_per_group < (int64_t)1 << 31 && (int64_t)nq * topk * 6 <= kFilterRoom;
+}
+struct FilterPlan {
+    size_t off_prep, off_bad, off_rows, off_offsets, off_codes, off_signs, off_norms, off_rnorms, off_grows, off_scores, total;
+};
+static FilterPlan plan_filter(const tq_plan* p, size_t behind) {
+    FilterPlan f{};
+    size_t at = behind;
+    auto take = [&](size_t bytes) { const size_t o = at; at += (bytes + 255) & ~size_t(255); return o; };
+    f.off_prep = take(tq_filter_prep_bytes(p->dev.d, 64));
+    f.off_bad = take(256);
+    f.off_offsets = take(64 * 4);
+    f.off_rows = take((size_t)64 * kFilterRoom * 4);
+    f.off_codes = take((size_t)kFilterRoom * p->dev.code_words * 4);
+    f.off_signs = take((size_t)kFilterRoom * p->dev.sign_words * 4);
+    f.off_norms = take((size_t)kFilterRoom * 4);
+    f.off_rnorms = take((size_t)kFilterRoom * 4);
+    f.off_grows = take((size_t)kFilterRoom * 4);
+    f.off_scores = take((size_t)64 * kFilterRoom * 4);
+    f.total = at;
+    return f;
+}
+
+int64_t tq_score_tc_scratch(const tq_plan* p, int groups, int qpg, int64_t keys_per_group, int topk) {
+    if (use_filter(p, nullptr, groups, qpg, topk, keys_per_group))       // also holds a call that wants the matrix besides
+        return (int64_t)std::max(plan_filter(p, plan_candidates(groups, qpg, keys_per_group, topk).total).total,
+                                 plan_score(groups, qpg, keys_per_group, topk, true).total);
     const size_t a = plan_score(groups, qpg, keys_per_group, topk, true).total;
     const size_t b = use_candidates(nullptr, topk, keys_per_group) ? plan_candidates(groups, qpg, keys_per_group, topk).total : 0;
     return (int64_t)(a > b ? a : b);
@@ -1302,10 +1355,12 @@ int tq_launch_score_tc(const tq_plan* p, const float* q, int groups, int qpg, co
                        size_t scratch_bytes, cudaStream_t st, int64_t group_rows) {
     TqRange range("tq.score.tensor_core");
     if (group_rows <= 0) group_rows = keys_per_group;
-    const bool candidates = use_candidates(scores, topk, keys_per_group);
+    const bool filter = p->path == TQ_PATH_AUTO && use_filter(p, scores, groups, qpg, topk, keys_per_group);
+    const bool candidates = filter || use_candidates(scores, topk, keys_per_group);
     const ScoreTcPlan sp = plan_score(groups, qpg, keys_per_group, topk, scores == nullptr);
     const CandPlan cp = plan_candidates(groups, qpg, keys_per_group, topk);
-    const size_t need = candidates ? cp.total : sp.total;
+    const FilterPlan fp = filter ? plan_filter(p, cp.total) : FilterPlan{};
+    const size_t need = filter ? fp.total : candidates ? cp.total : sp.total;
     if (!scratch || scratch_bytes < need)
         return tq_fail(TQ_ERR_SCRATCH_TOO_SMALL, "score scratch: need %zu bytes, got %zu", need, scratch_bytes);
     unsigned char* sc = static_cast<unsigned char*>(scratch);
@@ -1317,79 +1372,98 @@ int tq_launch_score_tc(const tq_plan* p, const float* q, int groups, int qpg, co
     unsigned long long* best = reinterpret_cast<unsigned long long*>(sc + cp.off_best);
     unsigned long long* cand = reinterpret_cast<unsigned long long*>(sc + cp.off_cand);
 
-    // One scoring launch per pass of at most 64 queries (32 at d = 256) over keys [key_off, key_off + key_cnt) of every group (every
+    // Which keys a launch scores: the caller's, or those gathered by a filtered search.
+    struct Keys { const uint32_t *codes, *signs; const float *rnorms, *norms; int64_t group_rows; const unsigned int* dyn_keys; };
+    const Keys all_keys{codes, signs, rnorms, norms, group_rows, nullptr};
+    const int pass = p->dev.d == 256 ? 32 : TQ_SCORE_PASS;
+    auto pad_of = [](int nq) { return nq <= 16 ? 16 : nq <= 32 ? 32 : 64; };
+    auto prepare_pass = [&](int q0, int nq) -> int {
+        const int qpad = pad_of(nq);
+        if (p->dev.d == 256) {
+            score_prep256_kernel<<<dim3(qpad, groups), 1024, 0, st>>>(p->dev, q, qpg, q0, nq, qpad, prep); tq_count_launch();
+        } else {
+            TQ_GRANT_SMEM((score_prep_kernel), kPrepSmemBytes, p->device);
+            score_prep_kernel<<<dim3(qpad, groups), 128, kPrepSmemBytes, st>>>(p->dev, q, qpg, q0, nq, qpad, prep); tq_count_launch();
+        }
+        TQ_CUDA_TRY(cudaGetLastError());
+        return TQ_OK;
+    };
+    // One scoring launch for the prepared queries [q0, q0 + nq) over keys [key_off, key_off + key_cnt) of every group (every
     // tile_stride-th tile of them), into a matrix (mat != null) or into the candidate lists.
+    auto score_pass = [&](const Keys& keys, int q0, int nq, int64_t key_off, int64_t key_cnt, int tile_stride, float* mat,
+                          int64_t row_stride, const unsigned int* run_if) -> int {
+        const int qpad = pad_of(nq);
+        const int64_t group_stride = (int64_t)qpg * row_stride;
+        ScoreTcArgs a{};
+        a.codes = keys.codes; a.signs = keys.signs; a.rnorms = keys.rnorms; a.norms = keys.norms;
+        a.dyn_keys = keys.dyn_keys; a.run_if = run_if;
+        a.prep = prep; a.codebook = p->dev.codebook;
+        a.keys_per_group = keys.group_rows; a.key_off = key_off; a.key_cnt = key_cnt;
+        a.tile_stride = tile_stride;
+        const int64_t tiles = (key_cnt + kTileKeys - 1) / kTileKeys;
+        a.tiles_per_group = (tiles + tile_stride - 1) / tile_stride;
+        a.total_tiles = a.tiles_per_group * groups;
+        a.nq = nq;
+        a.out_group_stride = group_stride; a.out_row_stride = row_stride;
+        a.scores = mat ? mat + (int64_t)q0 * row_stride : nullptr;
+        a.alpha = p->dev.alpha;
+        a.norms_bulk = (groups == 1 || keys.group_rows % 4 == 0) && key_off % 4 == 0 ? 1 : 0;   // 16-byte aligned tile starts
+        a.fused = mat ? 0 : (tile_stride > 1 ? 2 : 1);    // 2: the sampled pass
+        a.qpg_total = qpg; a.q0 = q0;
+        a.thr = thr; a.cnt = cnt; a.cand = cand; a.cand_cap = cp.cand_cap;
+        a.status = p->status_dev;
+        a.wait_kcycles = p->wait_kcycles;
+#ifdef TQ_PROF
+        a.prof = reinterpret_cast<long long*>(p->counters + 8);
+#endif
+        if (a.total_tiles == 0) return TQ_OK;
+        const int grid = (int)(a.total_tiles < sms ? a.total_tiles : sms);
+        // Score tiles leave through a bulk tensor store when the matrix allows one: 16-byte aligned base and
+        // row pitch.  Box = 128 keys x the queries of the pass x one group; extents clip ragged edges.
+        CUtensorMap map;
+        memset(&map, 0, sizeof(map));
+        a.tile_store = 0;
+        if (mat && (reinterpret_cast<uintptr_t>(a.scores) & 15u) == 0 && row_stride % 4 == 0 && key_cnt > 0 && tq_encode_tiled_fn()) {
+            const cuuint64_t gdim[3] = {(cuuint64_t)key_cnt, (cuuint64_t)nq, (cuuint64_t)groups};
+            const cuuint64_t gstride[2] = {(cuuint64_t)row_stride * 4, (cuuint64_t)group_stride * 4};
+            const cuuint32_t box[3] = {(cuuint32_t)kTileKeys, (cuuint32_t)qpad, 1};
+            const cuuint32_t estr[3] = {1, 1, 1};
+            const CUresult cr = tq_encode_tiled_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, a.scores, gdim, gstride, box, estr,
+                                                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                                                     CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+            if (cr == CUDA_SUCCESS) a.tile_store = 1;
+        }
+        int r = TQ_ERR_UNSUPPORTED;
+        tq_timer_mark(p, 1, 0, st);
+#define TQ_SC(B)                                                                                             \
+case B:                                                                                                  \
+    if (p->dev.d == 64) r = qpad == 16 ? launch_score<B, 16, 64>(p, map, a, grid, st) : qpad == 32 ? launch_score<B, 32, 64>(p, map, a, grid, st)       \
+                                                                                               : launch_score<B, 64, 64>(p, map, a, grid, st);      \
+    else if (p->dev.d == 256) r = qpad == 16 ? launch_score<B, 16, 256>(p, map, a, grid, st) : launch_score<B, 32, 256>(p, map, a, grid, st);          \
+    else r = qpad == 16 ? launch_score<B, 16, 128>(p, map, a, grid, st) : qpad == 32 ? launch_score<B, 32, 128>(p, map, a, grid, st)                   \
+                                                                                  : launch_score<B, 64, 128>(p, map, a, grid, st);                  \
+    break;
+        switch (bits) { TQ_SC(1) TQ_SC(2) TQ_SC(3) TQ_SC(4) }
+#undef TQ_SC
+        tq_timer_mark(p, 1, 1, st);
+        if (r != TQ_OK) return r == TQ_ERR_UNSUPPORTED ? tq_fail(r, "no tensor-core scoring kernel for bits=%d", bits) : r;
+        return TQ_OK;
+    };
+    // The same for every pass of at most 64 queries (32 at d = 256).  A pass of 64 expands the keys once for queries that would
+    // otherwise take two passes (64 queries x 1,048,576 keys: 171 us against 219 us in two passes of 32; 33 queries: 168
+    // against 205 us in passes of 32 and 16).
     // `prepared`: the scratch block still holds the prepared queries of the only pass (a call of several launches
     // over the same queries prepares them once).
-    auto score_passes = [&](int64_t key_off, int64_t key_cnt, int tile_stride, float* mat, int64_t row_stride, bool prepared) -> int {
-        const int64_t group_stride = (int64_t)qpg * row_stride;
-        // A pass of 64 expands the keys once for queries that would otherwise take two passes (64 queries x 1,048,576
-        // keys: 171 us against 219 us in two passes of 32; 33 queries: 168 against 205 us in passes of 32 and 16).
-        const int pass = p->dev.d == 256 ? 32 : TQ_SCORE_PASS;
+    auto score_passes = [&](int64_t key_off, int64_t key_cnt, int tile_stride, float* mat, int64_t row_stride, bool prepared,
+                            const unsigned int* run_if = nullptr) -> int {
         for (int q0 = 0; q0 < qpg; q0 += pass) {
             const int nq = qpg - q0 < pass ? qpg - q0 : pass;
-            const int qpad = nq <= 16 ? 16 : nq <= 32 ? 32 : 64;
-            if (prepared && qpg <= pass) {
-                // nothing to do
-            } else if (p->dev.d == 256) {
-                score_prep256_kernel<<<dim3(qpad, groups), 1024, 0, st>>>(p->dev, q, qpg, q0, nq, qpad, prep); tq_count_launch();
-            } else {
-                TQ_GRANT_SMEM((score_prep_kernel), kPrepSmemBytes, p->device);
-                score_prep_kernel<<<dim3(qpad, groups), 128, kPrepSmemBytes, st>>>(p->dev, q, qpg, q0, nq, qpad, prep); tq_count_launch();
+            if (!(prepared && qpg <= pass)) {
+                const int rc = prepare_pass(q0, nq);
+                if (rc != TQ_OK) return rc;
             }
-            TQ_CUDA_TRY(cudaGetLastError());
-            ScoreTcArgs a{};
-            a.codes = codes; a.signs = signs; a.rnorms = rnorms; a.norms = norms;
-            a.prep = prep; a.codebook = p->dev.codebook;
-            a.keys_per_group = group_rows; a.key_off = key_off; a.key_cnt = key_cnt;
-            a.tile_stride = tile_stride;
-            const int64_t tiles = (key_cnt + kTileKeys - 1) / kTileKeys;
-            a.tiles_per_group = (tiles + tile_stride - 1) / tile_stride;
-            a.total_tiles = a.tiles_per_group * groups;
-            a.nq = nq;
-            a.out_group_stride = group_stride; a.out_row_stride = row_stride;
-            a.scores = mat ? mat + (int64_t)q0 * row_stride : nullptr;
-            a.alpha = p->dev.alpha;
-            a.norms_bulk = (groups == 1 || group_rows % 4 == 0) && key_off % 4 == 0 ? 1 : 0;   // 16-byte aligned tile starts
-            a.fused = mat ? 0 : (tile_stride > 1 ? 2 : 1);    // 2: the sampled pass
-            a.qpg_total = qpg; a.q0 = q0;
-            a.thr = thr; a.cnt = cnt; a.cand = cand; a.cand_cap = cp.cand_cap;
-            a.status = p->status_dev;
-            a.wait_kcycles = p->wait_kcycles;
-#ifdef TQ_PROF
-            a.prof = reinterpret_cast<long long*>(p->counters + 8);
-#endif
-            if (a.total_tiles == 0) continue;
-            const int grid = (int)(a.total_tiles < sms ? a.total_tiles : sms);
-            // Score tiles leave through a bulk tensor store when the matrix allows one: 16-byte aligned base and
-            // row pitch.  Box = 128 keys x the queries of the pass x one group; extents clip ragged edges.
-            CUtensorMap map;
-            memset(&map, 0, sizeof(map));
-            a.tile_store = 0;
-            if (mat && (reinterpret_cast<uintptr_t>(a.scores) & 15u) == 0 && row_stride % 4 == 0 && key_cnt > 0 && tq_encode_tiled_fn()) {
-                const cuuint64_t gdim[3] = {(cuuint64_t)key_cnt, (cuuint64_t)nq, (cuuint64_t)groups};
-                const cuuint64_t gstride[2] = {(cuuint64_t)row_stride * 4, (cuuint64_t)group_stride * 4};
-                const cuuint32_t box[3] = {(cuuint32_t)kTileKeys, (cuuint32_t)qpad, 1};
-                const cuuint32_t estr[3] = {1, 1, 1};
-                const CUresult cr = tq_encode_tiled_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, a.scores, gdim, gstride, box, estr,
-                                                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                                         CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-                if (cr == CUDA_SUCCESS) a.tile_store = 1;
-            }
-            int r = TQ_ERR_UNSUPPORTED;
-            tq_timer_mark(p, 1, 0, st);
-#define TQ_SC(B)                                                                                             \
-    case B:                                                                                                  \
-        if (p->dev.d == 64) r = qpad == 16 ? launch_score<B, 16, 64>(p, map, a, grid, st) : qpad == 32 ? launch_score<B, 32, 64>(p, map, a, grid, st)       \
-                                                                                                   : launch_score<B, 64, 64>(p, map, a, grid, st);      \
-        else if (p->dev.d == 256) r = qpad == 16 ? launch_score<B, 16, 256>(p, map, a, grid, st) : launch_score<B, 32, 256>(p, map, a, grid, st);          \
-        else r = qpad == 16 ? launch_score<B, 16, 128>(p, map, a, grid, st) : qpad == 32 ? launch_score<B, 32, 128>(p, map, a, grid, st)                   \
-                                                                                      : launch_score<B, 64, 128>(p, map, a, grid, st);                  \
-        break;
-            switch (bits) { TQ_SC(1) TQ_SC(2) TQ_SC(3) TQ_SC(4) }
-#undef TQ_SC
-            tq_timer_mark(p, 1, 1, st);
-            if (r != TQ_OK) return r == TQ_ERR_UNSUPPORTED ? tq_fail(r, "no tensor-core scoring kernel for bits=%d", bits) : r;
+            const int rc = score_pass(all_keys, q0, nq, key_off, key_cnt, tile_stride, mat, row_stride, run_if);
+            if (rc != TQ_OK) return rc;
         }
         return TQ_OK;
     };
@@ -1431,31 +1505,94 @@ int tq_launch_score_tc(const tq_plan* p, const float* q, int groups, int qpg, co
     // and appends only about 64 k scores per query.
     const int k2 = pow2_at_least(topk);
     const int64_t cells = cp.lists * topk;
-    const int64_t tiles0 = (cp.chunk + kTileKeys - 1) / kTileKeys;
+    const int64_t tiles0 = (std::min(cp.chunk, keys_per_group) + kTileKeys - 1) / kTileKeys;
     const int64_t sample_tiles = (tiles0 + kSampleEvery - 1) / kSampleEvery;
-    init_candidates_kernel<<<(unsigned)((cells + 255) / 256), 256, 0, st>>>(thr, cnt, best, cp.lists, topk,
-                                                                            (unsigned int)(sample_tiles * kTileKeys)); tq_count_launch();
-    TQ_CUDA_TRY(cudaGetLastError());
-    auto select = [&](int mode) -> int {
-        select_candidates_kernel<<<dim3((unsigned)qpg, (unsigned)groups), 256, 0, st>>>(cand, cnt, cp.cand_cap, best, thr, qpg, topk, k2, mode);
+    auto init = [&](int64_t first_count, const unsigned int* run_if) -> int {
+        init_candidates_kernel<<<(unsigned)((cells + 255) / 256), 256, 0, st>>>(thr, cnt, best, cp.lists, topk, (unsigned int)first_count, run_if);
         tq_count_launch();
         TQ_CUDA_TRY(cudaGetLastError());
         return TQ_OK;
     };
-    for (int64_t c = 0; c < cp.nchunks; ++c) {
-        const int64_t key_off = c * cp.chunk;
-        int64_t key_cnt = keys_per_group - key_off;
-        if (key_cnt > cp.chunk) key_cnt = cp.chunk;
-        if (c == 0) {
-            int rc = score_passes(key_off, key_cnt, (int)kSampleEvery, nullptr, 0, false);
-            if (rc != TQ_OK) return rc;
-            rc = select(1);
-            if (rc != TQ_OK) return rc;
+    auto select = [&](int mode, const unsigned int* run_if) -> int {
+        select_candidates_kernel<<<dim3((unsigned)qpg, (unsigned)groups), 256, 0, st>>>(cand, cnt, cp.cand_cap, best, thr, qpg, topk, k2, mode, run_if);
+        tq_count_launch();
+        TQ_CUDA_TRY(cudaGetLastError());
+        return TQ_OK;
+    };
+    auto run_candidates = [&](const unsigned int* run_if) -> int {
+        TQ_STEP(init(sample_tiles * kTileKeys, run_if));
+        for (int64_t c = 0; c < cp.nchunks; ++c) {
+            const int64_t key_off = c * cp.chunk;
+            int64_t key_cnt = keys_per_group - key_off;
+            if (key_cnt > cp.chunk) key_cnt = cp.chunk;
+            if (c == 0) {
+                TQ_STEP(score_passes(key_off, key_cnt, (int)kSampleEvery, nullptr, 0, run_if != nullptr, run_if));
+                TQ_STEP(select(1, run_if));
+            }
+            TQ_STEP(score_passes(key_off, key_cnt, 1, nullptr, 0, true, run_if));
+            TQ_STEP(select(0, run_if));
         }
-        int rc = score_passes(key_off, key_cnt, 1, nullptr, 0, true);
-        if (rc != TQ_OK) return rc;
-        rc = select(0);
-        if (rc != TQ_OK) return rc;
+        return TQ_OK;
+    };
+    if (!filter) {
+        TQ_STEP(run_candidates(nullptr));
+        return tq_merge_keys_launch(best, 1, qpg, groups, topk, idx_base, top_scores, top_idx, st);
     }
+
+    // Filtered search over one group.  A sample of the keys, spread over all of them, is scored in full and gives every query a
+    // first threshold; each round lists the keys of a larger sample (the last round: all keys) whose single-fp16 score plus
+    // bound reaches the threshold, gathers them, scores them in full and raises the thresholds; the last round's selection is
+    // the result.  With the sizes of the samples a geometric series, every round lists about ratio * topk keys per query.
+    // Data that lists more than a round has room for (long runs of equal scores, say) sets a flag on the device, upon which
+    // the rest of the rounds does nothing and the unfiltered procedure behind them, else skipped, does the work.
+    TqFilterPass f{};
+    f.cap = kFilterRoom; f.room = kFilterRoom; f.beta_scale = p->beta_scale;
+    f.fprep = sc + fp.off_prep;
+    f.bad = reinterpret_cast<unsigned int*>(sc + fp.off_bad);
+    f.gathered = f.bad + 1;
+    f.rows = reinterpret_cast<unsigned int*>(sc + fp.off_rows);
+    f.offsets = reinterpret_cast<unsigned int*>(sc + fp.off_offsets);
+    f.g_codes = reinterpret_cast<uint32_t*>(sc + fp.off_codes);
+    f.g_signs = reinterpret_cast<uint32_t*>(sc + fp.off_signs);
+    f.g_norms = reinterpret_cast<float*>(sc + fp.off_norms);
+    f.g_rnorms = reinterpret_cast<float*>(sc + fp.off_rnorms);
+    f.g_rows = reinterpret_cast<unsigned int*>(sc + fp.off_grows);
+    f.scores = reinterpret_cast<float*>(sc + fp.off_scores);
+    const Keys gathered{f.g_codes, f.g_signs, f.g_rnorms, f.g_norms, kFilterRoom, f.gathered};
+    const int64_t tiles = (keys_per_group + kTileKeys - 1) / kTileKeys;
+    const int stride0 = (int)((tiles + kFilterSample / kTileKeys - 1) / (kFilterSample / kTileKeys));
+    const int64_t first = (tiles + stride0 - 1) / stride0 * kTileKeys;
+    TQ_CUDA_TRY(cudaMemsetAsync(f.bad, 0, 2 * sizeof(unsigned int), st));
+    TQ_STEP(init(first, nullptr));
+    for (int q0 = 0; q0 < qpg; q0 += pass) {
+        const int nq = qpg - q0 < pass ? qpg - q0 : pass;
+        f.nq = nq; f.qpad = pad_of(nq);
+        f.thr = thr + q0; f.cnt = cnt + q0; f.best = best + (int64_t)q0 * topk;
+        TQ_STEP(prepare_pass(q0, nq));
+        TQ_STEP(score_pass(all_keys, q0, nq, 0, keys_per_group, stride0, nullptr, 0, nullptr));
+        TQ_STEP(tq_launch_filter_prep(p, prep, f.qpad, nq, p->c_max, p->beta_scale, f.fprep, f.bad, st));
+    }
+    TQ_STEP(tq_launch_sample_threshold(cand, cp.cand_cap, cnt, thr, qpg, topk, st));
+    for (int q0 = 0; q0 < qpg; q0 += pass) {
+        const int nq = qpg - q0 < pass ? qpg - q0 : pass;
+        f.nq = nq; f.qpad = pad_of(nq);
+        f.thr = thr + q0; f.cnt = cnt + q0; f.best = best + (int64_t)q0 * topk;
+        if (qpg > pass) {
+            TQ_STEP(prepare_pass(q0, nq));
+            TQ_STEP(tq_launch_filter_prep(p, prep, f.qpad, nq, p->c_max, p->beta_scale, f.fprep, f.bad, st));
+        }
+        // rounds: the fewest whose ratio keeps the lists of all queries within two thirds of the room
+        const double span = (double)tiles / (double)(first / kTileKeys), most = 0.66 * kFilterRoom / ((double)nq * topk);
+        int rounds = 1;
+        while (pow(span, 1.0 / rounds) > most && rounds < 16) ++rounds;
+        for (int r = 1; r <= rounds; ++r) {
+            const int stride = r == rounds ? 1 : (int)std::max(1.0, stride0 / pow(span, (double)r / rounds));
+            TQ_STEP(tq_launch_filter(p, f, codes, signs, rnorms, norms, keys_per_group, stride, st));
+            TQ_STEP(tq_launch_filter_gather(p, f, codes, signs, rnorms, norms, st));
+            TQ_STEP(score_pass(gathered, q0, nq, 0, kFilterRoom, 1, f.scores - (int64_t)q0 * kFilterRoom, kFilterRoom, nullptr));
+            TQ_STEP(tq_launch_filter_select(f, topk, k2, r == rounds, st));
+        }
+    }
+    TQ_STEP(run_candidates(f.bad));
     return tq_merge_keys_launch(best, 1, qpg, groups, topk, idx_base, top_scores, top_idx, st);
 }

@@ -1,0 +1,63 @@
+"""Top-k search through the single-fp16 first stage (tq_score_filter.cu): the result is the stable sort of the full-accuracy
+score matrix, at the smallest key counts it serves, with ragged ends, for one and several passes of queries, for data its
+lists have no room for and for keys and queries its bound does not cover."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(prod, enc, q, k, rows=None):
+    import torch
+    prod.set_kernel_path("tensor")       # one to four queries would take a lookup-table kernel, with other last bits
+    mat = prod.attention_scores(q, enc)
+    prod.set_kernel_path("auto")
+    top_s, top_i = prod.attention_scores(q, enc, topk=k, index_base=2)
+    srt = torch.sort(mat, dim=1, descending=True, stable=True)
+    for r in range(q.shape[0]) if rows is None else rows:
+        assert torch.equal(top_s[r], srt.values[r, :k]) and torch.equal(top_i[r], srt.indices[r, :k] + 2), r
+
+
+@pytest.mark.parametrize("d,bits,n,nq,k", [
+    (128, 4, 1 << 20, 32, 100), (128, 4, (1 << 20) + 77, 64, 100), (128, 2, (1 << 21) + 1, 3, 1000), (64, 3, (1 << 20) + 129, 33, 10),
+    (64, 5, (1 << 21) + 64, 17, 64), (256, 4, (1 << 20) + 5, 40, 50), (256, 2, (1 << 21) + 3, 5, 100), (128, 5, (1 << 20) + 1, 100, 20),
+])
+def test_filtered_search_equals_the_sorted_matrix(lib_built, d, bits, n, nq, k):
+    import torch
+    import project_tensor_b200 as tg
+    gen = torch.Generator("cuda").manual_seed(n + d)
+    x = torch.randn((n, d), device="cuda", generator=gen) * (0.1 + 3.0 * torch.rand((n, 1), device="cuda", generator=gen))
+    x[n // 3] = 0.0
+    q = torch.randn((nq, d), device="cuda", generator=gen) * torch.logspace(-3, 3, nq, device="cuda")[:, None]
+    prod = tg.TurboQuantProd(d, bits, seed=2026)
+    _check(prod, prod.quantize(x), q, k)
+
+
+def test_filtered_search_falls_back_when_its_lists_are_too_short(lib_built):
+    """Half the keys are one vector: more exact ties at the threshold than a round has room for."""
+    import torch
+    import project_tensor_b200 as tg
+    d, n, nq, k = 128, (1 << 20) + 11, 32, 100
+    gen = torch.Generator("cuda").manual_seed(5)
+    x = torch.randn((n, d), device="cuda", generator=gen)
+    x[1000:1000 + n // 2] = x[7]
+    q = torch.randn((nq, d), device="cuda", generator=gen)
+    q[3] = x[7]
+    q[4] = 0.0           # every score is zero
+    prod = tg.TurboQuantProd(d, 4, seed=2026)
+    _check(prod, prod.quantize(x), q, k)
+
+
+def test_filtered_search_lists_keys_its_bound_does_not_cover(lib_built):
+    """Hand-made norms: huge residual norms (the scaled sign operand leaves the fp16 range), huge and negative norms."""
+    import torch
+    import project_tensor_b200 as tg
+    d, n, nq, k = 128, (1 << 20) + 3, 32, 100
+    gen = torch.Generator("cuda").manual_seed(6)
+    prod = tg.TurboQuantProd(d, 4, seed=2026)
+    enc = prod.quantize(torch.randn((n, d), device="cuda", generator=gen))
+    packed = tg.packed_buffers(enc)
+    packed["residual_norms"][5:4000:37] = 1.0e7
+    packed["norms"][11:9000:41] *= -50.0
+    packed["norms"][13:9000:43] = 1.0e12
+    q = torch.randn((nq, d), device="cuda", generator=gen)
+    _check(prod, enc, q, k)
