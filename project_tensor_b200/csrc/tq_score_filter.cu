@@ -146,7 +146,7 @@ score_filter_kernel(const FilterArgs a) {
     if (threadIdx.x == 0) {
         for (int i = 0; i < kStages; ++i) {
             mbar_init(BAR(FB_K_FULL + i), 1);
-            mbar_init(BAR(FB_K_EMPTY + i), L::kExpWarps / 2 + L::kEpiWarps / 2);   // one group of each takes the tile
+            mbar_init(BAR(FB_K_EMPTY + i), (kHalves == 2 ? L::kExpWarps : L::kExpWarps / 2) + L::kEpiWarps / 2);
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(BAR(FB_A_FULL + i), L::kExpWarps / 2);
@@ -237,8 +237,8 @@ score_filter_kernel(const FilterArgs a) {
             const uint32_t acc = tm + L::kColD + db * QP;
 #pragma unroll 1
             for (int h = 0; h < kHalves; ++h) {
-                const int b = (int)(i & 1);                                  // the buffer of the tile's group of expanders
-                const uint32_t use = (uint32_t)((i >> 1) * kHalves + h);     // which filling of it
+                const int b = kHalves == 2 ? h : (int)(i & 1);               // the buffer of a group of expanders, and which
+                const uint32_t use = (uint32_t)(kHalves == 2 ? i : i >> 1);  // filling of it
                 go = warp_wait(BAR(FB_A_FULL + b), use & 1u, abort_flag) &&
                      (h > 0 || warp_wait(BAR(FB_D_EMPTY + db), (uint32_t)((i / L::kDBufs) & 1) ^ 1u, abort_flag));
                 if (!go) break;
@@ -262,21 +262,21 @@ score_filter_kernel(const FilterArgs a) {
             }
         }
     } else if (warp < L::kFirstEpi) {
-        // ---- expanders: two threads per key, every second tile ----------------------------------------
+        // ---- expanders: two threads per key, every second tile (d = 256: every tile, a half of its coordinates) --------
         const int ew = warp - L::kFirstExp, group = ew >> 3, part = (ew >> 2) & 1;
         const int quarter = warp & 3;
         const int row = quarter * 32 + lane;
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
         constexpr uint32_t kPairMask = ((1u << (2 * BITS)) - 1u) << 7;     // a pair of codes, in place as a table row of 128 bytes
         const uint32_t lane4 = lane * 4;
-        for (int64_t t = t0 + group; t < t1; t += 2) {
+        for (int64_t t = t0 + (kHalves == 2 ? 0 : group); t < t1; t += kHalves == 2 ? 1 : 2) {
             const int64_t i = t - t0;
             const int s = (int)(i % kStages);
             bool fail = !mbar_wait(BAR(FB_K_FULL + s), (uint32_t)((i / kStages) & 1), abort_flag);
             const unsigned char* stage = smem + L::off_ring + s * L::kStage;
-            float rn = 0.f;
-#pragma unroll 1
-            for (int h = 0; h < kHalves; ++h) {
+            float rn;
+            {
+                const int h = kHalves == 2 ? group : 0;
                 uint32_t w[L::kSub * BITS + 1], sw[L::kSub];
                 {
                     // volatile: executed once, before the stage is released (a plain load may be repeated behind it)
@@ -293,13 +293,11 @@ score_filter_kernel(const FilterArgs a) {
                         sw[0] = sg[0];
                     }
                     w[L::kSub * BITS] = 0;
-                    if (h == 0) rn = *reinterpret_cast<const volatile float*>(stage + L::kNormOff + (kTileKeys + row) * 4);
+                    rn = *reinterpret_cast<const volatile float*>(stage + L::kNormOff + (kTileKeys + row) * 4);
                 }
-                if (h == kHalves - 1) {
-                    __threadfence_block();   // every lane's loads from the stage are performed before the stage is released
-                    __syncwarp();
-                    if (lane == 0 && !fail) mbar_arrive(BAR(FB_K_EMPTY + s));
-                }
+                __threadfence_block();   // every lane's loads from the stage are performed before the stage is released
+                __syncwarp();
+                if (lane == 0 && !fail) mbar_arrive(BAR(FB_K_EMPTY + s));
                 // +-beta: the sign bits of a pair are 16 apart; keys whose beta does not fit fp16 (or is NaN) get 0 and are
                 // listed by the epilogue without a look at their score
                 const float beta = a.alpha * rn * a.beta_scale;
@@ -315,7 +313,7 @@ score_filter_kernel(const FilterArgs a) {
                     hi[p] = *reinterpret_cast<const uint32_t*>(smem + L::off_lut + ((e & kPairMask) | lane4));
                     sg[p] = ((~sw[p >> 4] << (15 - (p & 15))) & 0x80008000u) ^ beta2;
                 }
-                const uint32_t use = (uint32_t)((i >> 1) * kHalves + h);
+                const uint32_t use = (uint32_t)(kHalves == 2 ? i : i >> 1);
                 if (!mbar_wait(BAR(FB_A_EMPTY + group), (use & 1u) ^ 1u, abort_flag)) fail = true;
                 tc_fence_after();
                 const uint32_t abase = tmem + lane_addr + group * L::kBufCols + part * L::kSub * 16;
@@ -437,7 +435,7 @@ score_filter_kernel(const FilterArgs a) {
 }
 
 // The single-fp16 operands and the constants of the bound from the prepared queries of a pass (tq_score_tc.cu): prep holds, per
-// half of the coordinates, q_hi, q_lo, p_hi, p_lo as K-major core matrices, then (1 / scale of q / 2^10, 1 / scale of p) per query.
+// half of the coordinates, q_hi, q_lo, p_hi, p_lo as K-major core matrices, then per pair of queries two 1 / (scale of q * 2^10) and two 1 / scale of p.
 // out: per half q_hi and the rescaled p, then A and the accumulator units per query, then kappa.  grid (qpad), block d.
 __global__ void __launch_bounds__(256)
 filter_prep_kernel(const unsigned char* __restrict__ prep, int qpad, int nq, int d, float beta_scale, float alpha, float c_max,
@@ -448,7 +446,8 @@ filter_prep_kernel(const unsigned char* __restrict__ prep, int qpad, int nq, int
     const size_t off = (size_t)(slot / 8) * ((kW / 8) * 128) + (size_t)(jh / 8) * 128 + (size_t)(slot % 8) * 16 + (size_t)(jh % 8) * 2;
     const unsigned char* src = prep + (size_t)half * 4 * mat + off;
     unsigned char* dst = out + (size_t)half * 2 * mat + off;
-    const float2 ds = reinterpret_cast<const float2*>(prep + (size_t)halves * 4 * mat)[slot];
+    const float* scales = reinterpret_cast<const float*>(prep + (size_t)halves * 4 * mat) + (slot >> 1) * 4 + (slot & 1);
+    const float2 ds = make_float2(scales[0], scales[2]);
     float* consts = reinterpret_cast<float*>(out + (size_t)halves * 2 * mat);
     auto H = [&](int which) { return __half2float(*reinterpret_cast<const __half*>(src + which * mat)); };
     float rq = H(0) + H(1), sq = H(2) + H(3);

@@ -5,19 +5,25 @@
 // is a small GEMM per tile of 128 keys: the keys are the M side, the (at most 32) queries the N side
 // and the 128 coordinates the K side.  Per tile:
 //
-//   bulk copy (1 thread)   packed codes and sign words of 128 keys -> smem ring (plain 1-D bulk copies)
-//   expanders (8 warps)    one thread per half key: turn packed codes into fp16 operands and store
+//   bulk copy (1 thread)   packed codes, sign words and norms of 128 keys -> smem ring (plain 1-D bulk copies)
+//   expanders (16 warps)   two threads per key: turn packed codes into fp16 operands and store
 //                          them into tensor memory with tcgen05.st (lane = key).  Two codes at a time
 //                          index a lookup table of (hi pair, lo pair) half2 values -- centroid * 2^10
 //                          split into fp16 hi + lo -- replicated per lane in smem so the lookups are
 //                          free of bank conflicts; two sign bits become one half2 of +-1 with a shift
 //                          and a logic op (the sign layout keeps them 16 bits apart for that).
-//   MMA (1 thread)         D1 = C_hi Q_hi + C_lo Q_hi + C_hi Q_lo,  D2 = Sg P_hi + Sg P_lo  (kind::f16,
-//                          fp32 accumulators in TMEM); Q = R q and P = S q are rotated / projected,
-//                          scaled by a power of two and split into fp16 hi + lo once per call by a
+//   MMA (1 thread)         D1 = C_hi Q_hi + C_hi Q_lo + C_lo Q_hi,  D2 = Sg P_hi + Sg P_lo  (kind::f16,
+//                          fp32 accumulators in TMEM, one column per query each); Q = R q and P = S q are rotated /
+//                          projected, scaled by a power of two and split into fp16 hi + lo once per call by a
 //                          small preparation kernel, and live in smem as the B operand.
-//   epilogue (4 warps)     one thread per key: tcgen05.ld both accumulators, apply the per-query
-//                          descale, alpha * rnorm and norm, store one coalesced 128-byte line per query.
+//   epilogue (8 warps)     one thread per key: tcgen05.ld both accumulators, apply the per-query
+//                          descale, alpha * rnorm and norm (fma.rn.f32x2), stage the tile for a bulk tensor store.
+//
+// Expanders and epilogue warps come in two groups that take tiles in turn (a pass of 64 queries: the epilogue groups
+// take halves of the queries instead): what a warp does for a tile is a chain of waits, loads and a round trip to tensor
+// memory that is longer than a tile may take.  Before -- every warp at every tile, hi and lo products in columns of their own,
+// which the epilogue had to fetch and add and which left room for one accumulator at 32 queries -- a tile of 32 queries took
+// 3,600 cycles (106 us per 32 x 1,048,576 scores).
 //
 // A second kernel selects the per-query top-k from a score matrix with a rising threshold and a
 // bitonic prune (the same scheme as the general kernel in tq_score.cu), one block per row segment.
@@ -41,23 +47,15 @@ using namespace tqtopk;
 
 constexpr int D = 128;
 constexpr int kTileKeys = 128;
-// Warps: bulk copy, MMA, 16 expanders (one thread per quarter key), then 4 epilogue warps per 16 queries of the pass.
-// A pass of 64 queries has 16 epilogue warps and, a block being limited to 32 warps, 8 expanders (one thread per
-// half key): what its tile waits for is the way of the single accumulator through the epilogue, which is as short with
-// one block of 16 queries per thread as in the smaller passes.
-template <int QPAD> struct ScoreThreads {
-    static constexpr int kExpWarps = QPAD == 64 ? 8 : 16;
-    static constexpr int kEpiPerRow = QPAD / 16;
-    static constexpr int kEpiThreads = 4 * kEpiPerRow * 32;
-    static constexpr int kThreads = (2 + kExpWarps) * 32 + kEpiThreads;
-    static constexpr int kFirstEpiWarp = 2 + kExpWarps;
-};
-constexpr int kFirstExpWarp = 2;
+constexpr int kExpWarps = 16, kEpiWarps = 8;      // behind the bulk-copy and the MMA warp; two groups each
+constexpr int kFirstExpWarp = 2, kFirstEpiWarp = kFirstExpWarp + kExpWarps;
+constexpr int kThreads = (2 + kExpWarps + kEpiWarps) * 32;
+constexpr int kPendKeys = 64;                     // survivors a warp stages in candidate mode
 constexpr int kMaxStages = 8;
 constexpr float kCentScale = 1024.f;
 constexpr int kRowBytesB = D * 2;  // one query row of one fp16 operand matrix
 constexpr int kPrepSmemBytes = 2 * D * D * 4;  // rotation and projection matrices staged by the preparation kernel
-constexpr int kEpiBarrier = 1;     // named barrier of the epilogue warps
+constexpr int kEpiBarrier = 1;     // named barriers of the epilogue groups: this one and the next
 
 // Prepared queries of one group: per half of the coordinates (two halves of 128 for d = 256, one otherwise) the four
 // fp16 operand matrices q_hi, q_lo, p_hi, p_lo, then one (1 / scale) pair per query.
@@ -94,18 +92,15 @@ struct ScoreTcArgs {
     float alpha;
     unsigned long long* status;
     int wait_kcycles;             // limit of one bounded wait, in units of 1024 cycles
-#ifdef TQ_PROF
-    long long* prof;              // per-role cycle counters (measurement builds only)
-#endif
 };
 
 enum {
     SB_K_FULL = 0,      // [8]
     SB_K_EMPTY = 8,     // [8]
-    SB_A_FULL = 16,     // [4]: per A buffer; in a pass of 64 queries per chunk of 32 coordinates of the single buffer
-    SB_A_EMPTY = 20,    // [4]
-    SB_D_FULL = 24,     // [2]
-    SB_D_EMPTY = 26,    // [2]
+    SB_A_FULL = 16,     // [2]: one operand buffer per group of expanders
+    SB_A_EMPTY = 18,    // [2]
+    SB_D_FULL = 20,     // [4]
+    SB_D_EMPTY = 24,    // [4]
     SB_B_FULL = 28,     // [2]
     SB_B_EMPTY = 30,    // [2]
     SB_COUNT = 32
@@ -147,7 +142,11 @@ template <int BITS, int QPAD, int DR>
 struct ScoreSmem {
     static_assert(QPAD <= 32 || DR <= 128, "a pass of 64 queries exists for d <= 128");
     static constexpr int kHalves = DR == 256 ? 2 : 1;
+    static constexpr int kSub = DR / kHalves / 64;        // chunks of 32 coordinates per expander thread and half
     static constexpr int kBBufs = (DR == 256 || QPAD == 64) ? 1 : 2;     // 64 KB of prepared queries: one group resident
+    static constexpr int kDBufs = 64 / QPAD;              // accumulators: 2 * QPAD of the 128 columns behind the operand buffers
+    static constexpr int kQT = QPAD < 32 ? QPAD : 32;     // queries of an epilogue thread
+    static constexpr bool kSplitQ = QPAD == 64;           // the epilogue groups split the queries (else they take tiles in turn)
     static constexpr int kPrepBytes = prep_group_bytes(QPAD, kHalves);
     static constexpr int kLutEntries = 1 << (2 * BITS);
     static constexpr int kLutBytes = kLutEntries * 32 * 8;
@@ -156,43 +155,39 @@ struct ScoreSmem {
     static constexpr int kNormOff = kTileKeys * (kCodeRowBytes + kSignRowBytes);   // norms, then residual norms, of the tile's keys
     static constexpr int kStageBytes = kNormOff + 2 * kTileKeys * 4;
     static constexpr int kBBytes = (kPrepBytes + 127) & ~127;
-    static constexpr int kOutBytes = QPAD * kTileKeys * 4;          // one staged tile of scores [query][key]
-    static constexpr int kFixed = kLutBytes + kBBufs * kBBytes + 2 * kOutBytes + 640 + 128 + 128;
-    static constexpr int kFit = (227 * 1024 - kFixed) / kStageBytes;
+    static constexpr int kOutBytes = kQT * kTileKeys * 4;           // one staged box of scores [query][key] per epilogue group
+    // candidate mode, in place of the boxes: per epilogue warp 16 x 32 parked scores and the staged survivors
+    static constexpr int kCandBytes = kEpiWarps * (16 * 32 * 4 + kPendKeys * 12);
+    static constexpr int kOutArea = 2 * kOutBytes > kCandBytes ? 2 * kOutBytes : kCandBytes;
+    static constexpr int kMisc = 512;
+    static constexpr int kFixed = kLutBytes + kBBufs * kBBytes + kOutArea + kMisc;
+    static constexpr int kFit = (226 * 1024 - kFixed) / kStageBytes;
     static constexpr int kStages = kFit < kMaxStages ? kFit : kMaxStages;
     static_assert(kStages >= 3, "key ring too short");
     static constexpr int off_lut = 0;
     static constexpr int off_b = off_lut + kLutBytes;
     static constexpr int off_out = off_b + kBBufs * kBBytes;
-    static constexpr int off_ring = off_out + 2 * kOutBytes;
+    static constexpr int off_ring = off_out + kOutArea;
     static constexpr int off_misc = off_ring + kStages * kStageBytes;
-    static constexpr int total = off_misc + 640 + 128;
+    static constexpr int total = off_misc + kMisc;
+    static_assert(off_ring % 128 == 0 && off_misc % 16 == 0 && off_out % 128 == 0, "alignment");
 };
+
+// two words of a ring stage, read exactly once
+__device__ __forceinline__ void lds_once_u2(uint32_t& x, uint32_t& y, const volatile uint32_t* p) {
+    asm volatile("ld.volatile.shared.v2.u32 {%0, %1}, [%2];" : "=r"(x), "=r"(y) : "r"(smem_u32(const_cast<const uint32_t*>(p))));
+}
 
 // CAND: candidate mode (top-k without a score matrix) is a kernel of its own, so that the matrix kernel carries none
 // of its registers and code.
 template <int BITS, int QPAD, int DR, bool CAND>
-__global__ void __launch_bounds__(ScoreThreads<QPAD>::kThreads, 1)
-score_tc_kernel(const __grid_constant__ CUtensorMap tmap_out, const ScoreTcArgs a) {
+__global__ void __launch_bounds__(kThreads, 1)
+score_tc_kernel(const __grid_constant__ CUtensorMap tmap_out, const __grid_constant__ ScoreTcArgs a) {
     static_assert(DR == 256 || DR == 128 || DR == 64, "written for d = 256, 128 and 64");
     using L = ScoreSmem<BITS, QPAD, DR>;
-    constexpr int kHalves = L::kHalves;          // passes of a key tile through the operand buffers
-    constexpr int kBBufs = L::kBBufs;
-    constexpr int kDH = DR / kHalves;            // coordinates per pass
-    constexpr int kChunks = kDH / 32;            // chunks of 32 coordinates per pass of a key through the buffers
-    constexpr int kSub = kChunks * 4 > ScoreThreads<QPAD>::kExpWarps ? kChunks * 4 / ScoreThreads<QPAD>::kExpWarps : 1;   // chunks per expander thread (2 in a pass of 64 queries at d = 128)
-    constexpr int kParts = kChunks / kSub;       // expander warps per lane quarter that have data
-    constexpr int kFirstEpiWarp = ScoreThreads<QPAD>::kFirstEpiWarp;
-    // A pass of 64 queries runs its single A buffer as a ring of chunks: the contractions of a tile take the chunks in
-    // order (two k-blocks each) and hand every chunk back as soon as they are through with it, so the expanders fill
-    // chunk c of the next tile while the contractions of this one are at chunk c + 1.
-    constexpr bool kChunkRing = QPAD == 64;
-    constexpr int kStages = L::kStages;
-    constexpr int kThreads = ScoreThreads<QPAD>::kThreads;
-    constexpr int kEpiPerRow = ScoreThreads<QPAD>::kEpiPerRow;
-    constexpr int kEpiThreads = ScoreThreads<QPAD>::kEpiThreads;
-    extern __shared__ unsigned char smem_raw[];
-    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+    constexpr int kHalves = L::kHalves, kBBufs = L::kBBufs, kDBufs = L::kDBufs, kStages = L::kStages, kQT = L::kQT;
+    constexpr int kDH = DR / kHalves;            // coordinates per pass through the operand buffers
+    extern __shared__ __align__(128) unsigned char smem[];     // (an address the compiler knows: the table lookups fold it in)
     const uint32_t smem_base = smem_u32(smem);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::off_misc);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + SB_COUNT);
@@ -200,30 +195,31 @@ score_tc_kernel(const __grid_constant__ CUtensorMap tmap_out, const ScoreTcArgs 
     const uint32_t bar0 = smem_u32(bars);
     auto BAR = [&](int i) { return bar0 + 8u * (uint32_t)i; };
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    TQ_PROF_CODE(const long long prof_t0 = clock64();)
     if (a.run_if && *a.run_if == 0u) return;
-    const int64_t total_tiles = a.dyn_keys ? ((int64_t)*a.dyn_keys + kTileKeys - 1) / kTileKeys : a.total_tiles;
+    const uint32_t total_tiles = (uint32_t)(a.dyn_keys ? ((int64_t)*a.dyn_keys + kTileKeys - 1) / kTileKeys : a.total_tiles);
+    const uint32_t tiles_per_group = (uint32_t)a.tiles_per_group;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < kStages; ++i) {
             mbar_init(BAR(SB_K_FULL + i), 1);
-            mbar_init(BAR(SB_K_EMPTY + i), 4 * kParts + (a.norms_bulk ? 4 * kEpiPerRow : 0));   // expanders (+ epilogue warps)
-        }
-        for (int i = 0; i < 4; ++i) {
-            mbar_init(BAR(SB_A_FULL + i), kChunkRing ? 4 : 4 * kParts);
-            mbar_init(BAR(SB_A_EMPTY + i), 1);
+            // one group of expanders (d = 256: both) and the epilogue warps that work on the tile read a stage
+            mbar_init(BAR(SB_K_EMPTY + i), (kHalves == 2 ? kExpWarps : kExpWarps / 2) + (a.norms_bulk ? (L::kSplitQ ? kEpiWarps : kEpiWarps / 2) : 0));
         }
         for (int i = 0; i < 2; ++i) {
-            mbar_init(BAR(SB_D_FULL + i), 1);
-            mbar_init(BAR(SB_D_EMPTY + i), 4 * kEpiPerRow);
+            mbar_init(BAR(SB_A_FULL + i), kExpWarps / 2);
+            mbar_init(BAR(SB_A_EMPTY + i), 1);
             mbar_init(BAR(SB_B_FULL + i), 1);
-            mbar_init(BAR(SB_B_EMPTY + i), 1 + 4 * kEpiPerRow);  // last MMA of the group + every epilogue warp
+            mbar_init(BAR(SB_B_EMPTY + i), 1 + kEpiWarps);      // last MMA of the group + every epilogue warp
+        }
+        for (int i = 0; i < kDBufs; ++i) {
+            mbar_init(BAR(SB_D_FULL + i), 1);
+            mbar_init(BAR(SB_D_EMPTY + i), L::kSplitQ ? kEpiWarps : kEpiWarps / 2);
         }
         abort_flag[0] = 0;
         abort_flag[1] = a.wait_kcycles;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    {   // pair lookup table: entry e = (code0 | code1 << BITS) -> (half2 hi(c0), hi(c1)), (half2 lo(c0), lo(c1))
+    {   // pair lookup table: entry e = (code0 | code1 << BITS) -> (half2 hi(c0), hi(c1)), (half2 lo(c0), lo(c1)), a copy per lane
         uint2* lut = reinterpret_cast<uint2*>(smem + L::off_lut);
         for (int i = threadIdx.x; i < L::kLutEntries * 32; i += kThreads) {
             const int e = i >> 5;
@@ -245,49 +241,36 @@ score_tc_kernel(const __grid_constant__ CUtensorMap tmap_out, const ScoreTcArgs 
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    TQ_PROF_CODE(const long long prof_t1 = clock64();)
 
     // contiguous tile range of this CTA, so that it rarely changes group
-    const int64_t t0 = total_tiles * (int64_t)blockIdx.x / gridDim.x;
-    const int64_t t1 = total_tiles * (int64_t)(blockIdx.x + 1) / gridDim.x;
-    // Instruction descriptors for N = QPAD and N = 2*QPAD (hi and lo query halves side by side).
-    constexpr uint32_t kIdesc1 = (1u << 4) | ((uint32_t)(QPAD >> 3) << 17) | ((uint32_t)(kTileKeys >> 4) << 24);
-    constexpr uint32_t kIdesc2 = (1u << 4) | ((uint32_t)(2 * QPAD >> 3) << 17) | ((uint32_t)(kTileKeys >> 4) << 24);
-    // TMEM: two A buffers of 192 columns (C_hi | C_lo | Sg), then the accumulators D1 = [C q_hi | C_hi q_lo]
-    // and D2 = [Sg p_hi | Sg p_lo], 2*QPAD columns each; double-buffered when they fit (QPAD = 16).
-    constexpr uint32_t kBufCols = 192;
-    constexpr uint32_t kColHi = 0, kColLo = 64, kColSg = 128;
-    // A pass of 64 queries has 256 accumulator columns and room for one A buffer only (run as a ring of chunks, below).
-    // Measured alternatives per 64 x 1,048,576 scores / per 1,048,576 keys in candidate mode: 16 expander and 8 epilogue
-    // warps with two blocks of 16 queries per epilogue thread 176 / 258 us (the accumulator stays with the epilogue twice
-    // as long); the same with both A buffers and the hi and lo products added inside 128 accumulator columns (40
-    // instructions of N = 64 per tile) 173 / 245 us; 8 expander and 16 epilogue warps with the A buffer handed over
-    // whole 174 / 175 us; as a ring of chunks 171 / 178 us.
-    constexpr int kABufs = QPAD == 64 ? 1 : 2;
-    constexpr int kDBufs = QPAD == 16 ? 2 : 1;
-    constexpr uint32_t kColD = kABufs * kBufCols, kDCols = 4 * QPAD;
+    const uint32_t t0 = (uint32_t)((uint64_t)total_tiles * blockIdx.x / gridDim.x);
+    const uint32_t t1 = (uint32_t)((uint64_t)total_tiles * (blockIdx.x + 1) / gridDim.x);
+    const uint32_t g_first = t0 / tiles_per_group;
+    // TMEM: two operand buffers of 192 columns (C_hi | C_lo | Sg), then the accumulators (D1 | D2), QPAD columns each
+    constexpr uint32_t kBufCols = 192, kColHi = 0, kColLo = 64, kColSg = 128;
+    constexpr uint32_t kColD = 2 * kBufCols, kDCols = 2 * QPAD;
+    static_assert(kColD + kDBufs * kDCols <= 512, "tensor memory plan");
 
     if (warp == 0) {
         if (lane == 0) {
-            int64_t prev_g = -1, gcount = 0, issued = 0;
-            int64_t g = t0 / a.tiles_per_group, kt = t0 - g * a.tiles_per_group;
-            for (int64_t t = t0; t < t1; ++t, ++kt) {
-                if (kt == a.tiles_per_group) { kt = 0; ++g; }
-                if (g != prev_g) {
-                    const int bb = (kBBufs == 2 ? (int)(gcount & 1) : 0);
-                    if (!mbar_wait(BAR(SB_B_EMPTY + bb), (uint32_t)((kBBufs == 2 ? gcount >> 1 : gcount) & 1) ^ 1u, abort_flag)) break;
+            uint32_t issued = 0, gcount = 0;
+            uint32_t g = g_first, kt = t0 - g * tiles_per_group;
+            for (uint32_t t = t0; t < t1; ++t, ++kt) {
+                if (kt == tiles_per_group) { kt = 0; ++g; }
+                if (g - g_first == gcount) {
+                    const int bb = kBBufs == 2 ? (int)(gcount & 1) : 0;
+                    if (!mbar_wait(BAR(SB_B_EMPTY + bb), ((kBBufs == 2 ? gcount >> 1 : gcount) & 1) ^ 1u, abort_flag)) break;
                     mbar_arrive_expect_tx(BAR(SB_B_FULL + bb), L::kPrepBytes);
-                    bulk_load(smem_base + L::off_b + bb * L::kBBytes, a.prep + g * L::kPrepBytes, L::kPrepBytes, BAR(SB_B_FULL + bb));
-                    prev_g = g;
+                    bulk_load(smem_base + L::off_b + bb * L::kBBytes, a.prep + (size_t)g * L::kPrepBytes, L::kPrepBytes, BAR(SB_B_FULL + bb));
                     ++gcount;
                 }
-                const int64_t i = t - t0;
+                const uint32_t i = t - t0;
                 const int s = (int)(i % kStages);
-                if (!mbar_wait(BAR(SB_K_EMPTY + s), (uint32_t)((i / kStages) & 1) ^ 1u, abort_flag)) break;
-                const int64_t k0 = kt * a.tile_stride * kTileKeys;      // first key of the tile within this launch's range
+                if (!mbar_wait(BAR(SB_K_EMPTY + s), ((i / kStages) & 1) ^ 1u, abort_flag)) break;
+                const int64_t k0 = (int64_t)kt * a.tile_stride * kTileKeys;      // first key of the tile within this launch's range
                 int64_t valid = a.key_cnt - k0;
                 if (valid > kTileKeys) valid = kTileKeys;
-                const int64_t row0 = g * a.keys_per_group + a.key_off + k0;
+                const int64_t row0 = (int64_t)g * a.keys_per_group + a.key_off + k0;
                 const uint32_t cb = (uint32_t)valid * L::kCodeRowBytes, sb = (uint32_t)valid * L::kSignRowBytes;
                 const unsigned char* csrc = reinterpret_cast<const unsigned char*>(a.codes) + row0 * L::kCodeRowBytes;
                 const unsigned char* ssrc = reinterpret_cast<const unsigned char*>(a.signs) + row0 * L::kSignRowBytes;
@@ -313,420 +296,199 @@ score_tc_kernel(const __grid_constant__ CUtensorMap tmap_out, const ScoreTcArgs 
             }
             if (*abort_flag) {
                 // copies armed above may still be on their way into this block's shared memory
-                for (int64_t ii = issued > kStages ? issued - kStages : 0; ii < issued; ++ii)
-                    mbar_drain(BAR(SB_K_FULL + (int)(ii % kStages)), (uint32_t)((ii / kStages) & 1));
-                for (int64_t gg = gcount > kBBufs ? gcount - kBBufs : 0; gg < gcount; ++gg)
-                    mbar_drain(BAR(SB_B_FULL + (kBBufs == 2 ? (int)(gg & 1) : 0)), (uint32_t)((kBBufs == 2 ? gg >> 1 : gg) & 1));
+                for (uint32_t ii = issued > kStages ? issued - kStages : 0; ii < issued; ++ii)
+                    mbar_drain(BAR(SB_K_FULL + (int)(ii % kStages)), (ii / kStages) & 1);
+                for (uint32_t gg = gcount > kBBufs ? gcount - kBBufs : 0; gg < gcount; ++gg)
+                    mbar_drain(BAR(SB_B_FULL + (kBBufs == 2 ? (int)(gg & 1) : 0)), (kBBufs == 2 ? gg >> 1 : gg) & 1);
             }
         }
     } else if (warp == 1) {
         // The whole warp walks the tiles and waits; one elected lane issues, with every operand computed from
         // warp-uniform values (a single lane of a diverged warp pays about 64 cycles per instruction).
-        {
-            const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
-            const uint32_t lbo = 128, sbo = (D / 8) * 128;
-            int64_t prev_g = -1, gcount = 0;
-            int bb = 0;
-            int64_t g = t0 / a.tiles_per_group, kt = t0 - g * a.tiles_per_group;
-            uint64_t dq_hi = 0, dp_hi = 0;
-            if constexpr (kChunkRing) {
-                bool gave_up = false;
-                for (int64_t t = t0; t < t1 && !gave_up; ++t, ++kt) {
-                    if (kt == a.tiles_per_group) { kt = 0; ++g; }
-                    const int64_t i = t - t0;
-                    const uint32_t par = (uint32_t)(i & 1);
-                    if (g != prev_g) {
-                        bb = 0;
-                        if (!warp_wait(BAR(SB_B_FULL), (uint32_t)(gcount & 1), abort_flag)) break;
-                        prev_g = g;
-                        ++gcount;
-                        const uint32_t bq = smem_base + L::off_b;
-                        dq_hi = make_smem_desc(bq + 0 * QPAD * kRowBytesB, lbo, sbo);
-                        dp_hi = make_smem_desc(bq + 2 * QPAD * kRowBytesB, lbo, sbo);
-                    }
-                    const uint32_t d1 = tm + kColD, d2 = d1 + 2 * QPAD;
-                    const bool last_of_group = (t + 1 == t1) || (kt + 1 == a.tiles_per_group);
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+        constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(QPAD >> 3) << 17) | ((uint32_t)(kTileKeys >> 4) << 24);
+        const uint32_t lbo = 128, sbo = (D / 8) * 128;
+        uint32_t g = g_first, kt = t0 - g * tiles_per_group, gcount = 0;
+        int bb = 0;
+        uint64_t dq = 0;                // descriptor of q_hi; q_lo, p_hi and p_lo follow, QPAD rows each
+        constexpr uint64_t kMat = (uint64_t)(QPAD * kRowBytesB >> 4);
+        bool go = true;
+        for (uint32_t t = t0; t < t1 && go; ++t, ++kt) {
+            if (kt == tiles_per_group) { kt = 0; ++g; }
+            const uint32_t i = t - t0;
+            if (g - g_first == gcount) {
+                bb = kBBufs == 2 ? (int)(gcount & 1) : 0;
+                if (!warp_wait(BAR(SB_B_FULL + bb), (kBBufs == 2 ? gcount >> 1 : gcount) & 1, abort_flag)) break;
+                ++gcount;
+                dq = make_smem_desc(smem_base + L::off_b + bb * L::kBBytes, lbo, sbo);
+            }
+            const int db = (int)(i % kDBufs);
+            const uint32_t d1 = tm + kColD + db * kDCols, d2 = d1 + QPAD;
+            const bool last_of_group = t + 1 == t1 || kt + 1 == tiles_per_group;
 #pragma unroll 1
-                    for (int c = 0; c < kChunks; ++c) {
-                        if (!warp_wait(BAR(SB_A_FULL + c), par, abort_flag)) { gave_up = true; break; }
-                        if (c == 0 && !warp_wait(BAR(SB_D_EMPTY), par ^ 1u, abort_flag)) { gave_up = true; break; }
-                        tc_fence_after();
-                        if (elect_one()) {
+            for (int h = 0; h < kHalves; ++h) {
+                const int b = kHalves == 2 ? h : (int)(i & 1);               // the operand buffer, and which filling of it
+                const uint32_t use = kHalves == 2 ? i : i >> 1, base = tm + b * kBufCols;
+                go = warp_wait(BAR(SB_A_FULL + b), use & 1u, abort_flag) &&
+                     (h > 0 || warp_wait(BAR(SB_D_EMPTY + db), ((i / kDBufs) & 1) ^ 1u, abort_flag));
+                if (!go) break;
+                tc_fence_after();
+                if (elect_one()) {
 #pragma unroll 1
-                            for (int kb = 2 * c; kb < 2 * c + 2; ++kb) {
-                                const uint64_t step = (uint64_t)(kb * 2 * lbo >> 4);
-                                const uint64_t qh = dq_hi + step, ph = dp_hi + step;
-                                if (kb == 0) {
-                                    mma_ts_first(d1, tm + kColHi, qh, kIdesc2);
-                                    mma_ts_acc(d1, tm + kColLo, qh, kIdesc1);
-                                    mma_ts_first(d2, tm + kColSg, ph, kIdesc2);
-                                } else {
-                                    mma_ts_acc(d1, tm + kColHi + kb * 8, qh, kIdesc2);
-                                    mma_ts_acc(d1, tm + kColLo + kb * 8, qh, kIdesc1);
-                                    mma_ts_acc(d2, tm + kColSg + kb * 8, ph, kIdesc2);
-                                }
-                            }
-                            mma_commit(BAR(SB_A_EMPTY + c));     // this chunk's slot may be filled for the next tile
-                            if (c == kChunks - 1) {
-                                mma_commit(BAR(SB_D_FULL));
-                                if (last_of_group) mma_commit(BAR(SB_B_EMPTY));
-                            }
+                    for (int kb = 0; kb < kDH / 16; ++kb) {
+                        // the start-address field counts 16-byte units: one k-block is two core matrices further, the
+                        // operand matrices of the second half of the coordinates follow those of the first
+                        const uint64_t qh = dq + (uint64_t)h * 4 * kMat + (uint64_t)(kb * 2 * lbo >> 4);
+                        const uint32_t hi = base + kColHi + kb * 8, lo = base + kColLo + kb * 8, sg = base + kColSg + kb * 8;
+                        if (h == 0 && kb == 0) {
+                            mma_ts_first(d1, hi, qh, kIdesc);
+                            mma_ts_first(d2, sg, qh + 2 * kMat, kIdesc);
+                        } else {
+                            mma_ts_acc(d1, hi, qh, kIdesc);
+                            mma_ts_acc(d2, sg, qh + 2 * kMat, kIdesc);
                         }
-                        __syncwarp();
+                        mma_ts_acc(d1, hi, qh + kMat, kIdesc);
+                        mma_ts_acc(d2, sg, qh + 3 * kMat, kIdesc);
+                        mma_ts_acc(d1, lo, qh, kIdesc);
                     }
+                    if (h == kHalves - 1) mma_commit(BAR(SB_D_FULL + db));
+                    mma_commit(BAR(SB_A_EMPTY + b));
+                    if (h == kHalves - 1 && last_of_group) mma_commit(BAR(SB_B_EMPTY + bb));
                 }
-            } else if constexpr (kHalves == 1) {
-                for (int64_t t = t0; t < t1; ++t, ++kt) {
-                    if (kt == a.tiles_per_group) { kt = 0; ++g; }
-                    const int64_t i = t - t0;
-                    const int b = kABufs == 2 ? (int)(i & 1) : 0;
-                    const uint32_t par2 = (uint32_t)((kABufs == 2 ? i >> 1 : i) & 1);
-                    if (g != prev_g) {
-                        bb = (kBBufs == 2 ? (int)(gcount & 1) : 0);
-                        if (!warp_wait(BAR(SB_B_FULL + bb), (uint32_t)((kBBufs == 2 ? gcount >> 1 : gcount) & 1), abort_flag)) break;
-                        prev_g = g;
-                        ++gcount;
-                        const uint32_t bq = smem_base + L::off_b + bb * L::kBBytes;
-                        dq_hi = make_smem_desc(bq + 0 * QPAD * kRowBytesB, lbo, sbo);
-                        dp_hi = make_smem_desc(bq + 2 * QPAD * kRowBytesB, lbo, sbo);
-                    }
-                    TQ_PROF_CODE(long long c0 = clock64();)
-                    if (!warp_wait(BAR(SB_A_FULL + b), par2, abort_flag)) break;
-                    TQ_PROF_CODE(long long c1 = clock64();)
-                    const int db = kDBufs == 2 ? (int)(i & 1) : 0;
-                    const uint32_t dpar = (uint32_t)((kDBufs == 2 ? i >> 1 : i) & 1);
-                    if (!warp_wait(BAR(SB_D_EMPTY + db), dpar ^ 1u, abort_flag)) break;
-                    tc_fence_after();
-                    TQ_PROF_CODE(long long c2 = clock64(); if (a.prof && blockIdx.x == 0 && lane == 0) { a.prof[8] += c1 - c0; a.prof[9] += c2 - c1; })
-                    const uint32_t base = tm + b * kBufCols;
-                    const uint32_t d1 = tm + kColD + db * kDCols, d2 = d1 + 2 * QPAD;
-                    const bool last_of_group = (t + 1 == t1) || (kt + 1 == a.tiles_per_group);
-                    if (elect_one()) {
-                        // q_hi and q_lo (p_hi and p_lo) are adjacent row blocks of one operand: N = 2*QPAD
-                        mma_ts_first(d1, base + kColHi, dq_hi, kIdesc2);
-                        mma_ts_acc(d1, base + kColLo, dq_hi, kIdesc1);
-                        mma_ts_first(d2, base + kColSg, dp_hi, kIdesc2);
-#pragma unroll 1
-                        for (int kb = 1; kb < DR / 16; ++kb) {
-                            // the start-address field counts 16-byte units: one k-block (two core matrices) further
-                            const uint64_t step = (uint64_t)(kb * 2 * lbo >> 4);
-                            const uint64_t qh = dq_hi + step, ph = dp_hi + step;
-                            mma_ts_acc(d1, base + kColHi + kb * 8, qh, kIdesc2);
-                            mma_ts_acc(d1, base + kColLo + kb * 8, qh, kIdesc1);
-                            mma_ts_acc(d2, base + kColSg + kb * 8, ph, kIdesc2);
-                        }
-                        mma_commit(BAR(SB_D_FULL + db));
-                        mma_commit(BAR(SB_A_EMPTY + b));
-                        if (last_of_group) mma_commit(BAR(SB_B_EMPTY + bb));
-                    }
-                    __syncwarp();
-                    TQ_PROF_CODE(if (a.prof && blockIdx.x == 0 && lane == 0) a.prof[10] += clock64() - c2;)
-                }
-            } else {
-                // d = 256: every tile passes through the operand buffers twice (coordinates 0..127, then 128..255)
-                bool gave_up = false;
-                for (int64_t t = t0; t < t1 && !gave_up; ++t, ++kt) {
-                    if (kt == a.tiles_per_group) { kt = 0; ++g; }
-                    const int64_t i = t - t0;
-                    if (g != prev_g) {
-                        bb = (kBBufs == 2 ? (int)(gcount & 1) : 0);
-                        if (!warp_wait(BAR(SB_B_FULL + bb), (uint32_t)((kBBufs == 2 ? gcount >> 1 : gcount) & 1), abort_flag)) break;
-                        prev_g = g;
-                        ++gcount;
-                        const uint32_t bq = smem_base + L::off_b + bb * L::kBBytes;
-                        dq_hi = make_smem_desc(bq + 0 * QPAD * kRowBytesB, lbo, sbo);
-                        dp_hi = make_smem_desc(bq + 2 * QPAD * kRowBytesB, lbo, sbo);
-                    }
-                    const int db = kDBufs == 2 ? (int)(i & 1) : 0;
-                    const uint32_t dpar = kDBufs == 2 ? (uint32_t)((i >> 1) & 1) : (uint32_t)(i & 1);
-                    const uint32_t d1 = tm + kColD + db * kDCols, d2 = d1 + 2 * QPAD;
-                    const bool last_of_group = (t + 1 == t1) || (kt + 1 == a.tiles_per_group);
-#pragma unroll 1
-                    for (int h = 0; h < kHalves; ++h) {
-                        const int64_t j = i * kHalves + h;       // passes through the operand buffers since the start
-                        const int b = (int)(j & 1);
-                        const uint32_t par2 = (uint32_t)((j >> 1) & 1);
-                        TQ_PROF_CODE(long long c0 = clock64();)
-                        if (!warp_wait(BAR(SB_A_FULL + b), par2, abort_flag)) { gave_up = true; break; }
-                        TQ_PROF_CODE(long long c1 = clock64();)
-                        if (h == 0 && !warp_wait(BAR(SB_D_EMPTY + db), dpar ^ 1u, abort_flag)) { gave_up = true; break; }
-                        tc_fence_after();
-                        TQ_PROF_CODE(long long c2 = clock64(); if (a.prof && blockIdx.x == 0 && lane == 0) { a.prof[8] += c1 - c0; a.prof[9] += c2 - c1; })
-                        const uint32_t base = tm + b * kBufCols;
-                        if (elect_one()) {
-                            // the operand matrices of the second half of the coordinates follow those of the first
-                            const uint64_t half_step = (uint64_t)((uint32_t)h * 4u * QPAD * kRowBytesB >> 4);
-                            const uint64_t q0d = dq_hi + half_step, p0d = dp_hi + half_step;
-                            // q_hi and q_lo (p_hi and p_lo) are adjacent row blocks of one operand: N = 2*QPAD
-                            if (h == 0) {
-                                mma_ts_first(d1, base + kColHi, q0d, kIdesc2);
-                                mma_ts_acc(d1, base + kColLo, q0d, kIdesc1);
-                                mma_ts_first(d2, base + kColSg, p0d, kIdesc2);
-                            } else {
-                                mma_ts_acc(d1, base + kColHi, q0d, kIdesc2);
-                                mma_ts_acc(d1, base + kColLo, q0d, kIdesc1);
-                                mma_ts_acc(d2, base + kColSg, p0d, kIdesc2);
-                            }
-#pragma unroll 1
-                            for (int kb = 1; kb < kDH / 16; ++kb) {
-                                // the start-address field counts 16-byte units: one k-block (two core matrices) further
-                                const uint64_t step = (uint64_t)(kb * 2 * lbo >> 4);
-                                const uint64_t qh = q0d + step, ph = p0d + step;
-                                mma_ts_acc(d1, base + kColHi + kb * 8, qh, kIdesc2);
-                                mma_ts_acc(d1, base + kColLo + kb * 8, qh, kIdesc1);
-                                mma_ts_acc(d2, base + kColSg + kb * 8, ph, kIdesc2);
-                            }
-                            if (h == kHalves - 1) mma_commit(BAR(SB_D_FULL + db));
-                            mma_commit(BAR(SB_A_EMPTY + b));
-                            if (h == kHalves - 1 && last_of_group) mma_commit(BAR(SB_B_EMPTY + bb));
-                        }
-                        __syncwarp();
-                        TQ_PROF_CODE(if (a.prof && blockIdx.x == 0 && lane == 0) a.prof[10] += clock64() - c2;)
-                    }
-                }
+                __syncwarp();
             }
         }
     } else if (warp < kFirstEpiWarp) {
-        // ---- expanders: one thread per quarter key (32 coordinates) ---------------------------------
-        const int part = (warp - kFirstExpWarp) >> 2;
+        // ---- expanders: two threads per key, every second tile (d = 256: every tile, a half of its coordinates) --------
+        const int ew = warp - kFirstExpWarp, group = ew >> 3, part = (ew >> 2) & 1;
         const int quarter = warp & 3;
         const int row = quarter * 32 + lane;
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
-        const uint2* lut_lane = reinterpret_cast<const uint2*>(smem + L::off_lut) + lane;
-        constexpr uint32_t kPairMask = (1u << (2 * BITS)) - 1u;
-        TQ_PROF_CODE(long long pc[5] = {0, 0, 0, 0, 0};)
-        if constexpr (kChunkRing) {
-            // a pass of 64 queries: the thread's chunks one after the other, each into its slot of the single A buffer
-            for (int64_t t = t0; t < (part < kParts ? t1 : t0); ++t) {
-                const int64_t i = t - t0;
-                const int s = (int)(i % kStages);
-                const uint32_t par = (uint32_t)(i & 1);
-                bool fail = !mbar_wait(BAR(SB_K_FULL + s), (uint32_t)((i / kStages) & 1), abort_flag);
-#pragma unroll 1
-                for (int sp = 0; sp < kSub; ++sp) {
-                    const int chunk = part * kSub + sp;
-                    uint32_t w[BITS + 1], sw;
-                    {
-                        const unsigned char* stage = smem + L::off_ring + s * L::kStageBytes;
-                        const volatile uint32_t* cw = reinterpret_cast<const volatile uint32_t*>(stage + row * L::kCodeRowBytes) + chunk * BITS;
-                        const volatile uint32_t* sg = reinterpret_cast<const volatile uint32_t*>(stage + kTileKeys * L::kCodeRowBytes + row * L::kSignRowBytes) + chunk;
-#pragma unroll
-                        for (int k = 0; k < BITS; ++k) w[k] = fail ? 0u : cw[k];
-                        w[BITS] = 0;
-                        sw = fail ? 0u : ~sg[0];
-                    }
-                    __threadfence_block();   // every lane's loads from the stage are performed before the stage is released
-                    __syncwarp();
-                    if (sp == kSub - 1 && lane == 0 && !fail) mbar_arrive(BAR(SB_K_EMPTY + s));
-                    uint32_t hi[16], lo[16], sg[16];
-#pragma unroll
-                    for (int p = 0; p < 16; ++p) {
-                        const int bit = p * 2 * BITS, wi = bit >> 5, sh = bit & 31;
-                        uint32_t e;
-                        if (sh + 2 * BITS <= 32) e = (w[wi] >> sh) & kPairMask;
-                        else e = __funnelshift_r(w[wi], w[wi + 1], sh) & kPairMask;
-                        const uint2 v = lut_lane[e * 32];
-                        hi[p] = v.x;
-                        lo[p] = v.y;
-                        sg[p] = ((sw << (15 - p)) & 0x80008000u) | 0x3c003c00u;
-                    }
-                    if (!mbar_wait(BAR(SB_A_EMPTY + chunk), par ^ 1u, abort_flag)) fail = true;
-                    tc_fence_after();
-                    const uint32_t abase = tmem + lane_addr + chunk * 16;
-                    tmem_st16(abase + kColHi, hi);
-                    tmem_st16(abase + kColLo, lo);
-                    tmem_st16(abase + kColSg, sg);
-                    tmem_wait_st();
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(BAR(SB_A_FULL + chunk));
-                }
-            }
-        } else if constexpr (kHalves == 1) {
-            for (int64_t t = t0; t < (part < kParts ? t1 : t0); ++t) {
-                const int64_t i = t - t0;
-                const int s = (int)(i % kStages);
-                const int b = kABufs == 2 ? (int)(i & 1) : 0;
-                const uint32_t par2 = (uint32_t)((kABufs == 2 ? i >> 1 : i) & 1);
-                TQ_PROF_CODE(long long c0 = clock64();)
-                bool fail = !mbar_wait(BAR(SB_K_FULL + s), (uint32_t)((i / kStages) & 1), abort_flag);
-                TQ_PROF_CODE(long long c1 = clock64(); pc[0] += c1 - c0;)
-                uint32_t w[BITS + 1], sw;
+        constexpr uint32_t kPairMask = ((1u << (2 * BITS)) - 1u) << 8;     // a pair of codes, in place as a table row of 256 bytes
+        const uint32_t lane8 = lane * 8;
+        constexpr uint32_t t_step = kHalves == 2 ? 1u : 2u;
+        for (uint32_t t = t0 + (kHalves == 2 ? 0 : group); t < t1; t += t_step) {
+            const uint32_t i = t - t0;
+            const int s = (int)(i % kStages);
+            bool fail = !mbar_wait(BAR(SB_K_FULL + s), (i / kStages) & 1, abort_flag);
+            const unsigned char* stage = smem + L::off_ring + s * L::kStageBytes;
+            {
+                const int h = kHalves == 2 ? group : 0;
+                uint32_t w[L::kSub * BITS + 1], sw[L::kSub];
                 {
-                    const unsigned char* stage = smem + L::off_ring + s * L::kStageBytes;
-                    const volatile uint32_t* cw = reinterpret_cast<const volatile uint32_t*>(stage + row * L::kCodeRowBytes) + part * BITS;
-                    const volatile uint32_t* sg = reinterpret_cast<const volatile uint32_t*>(stage + kTileKeys * L::kCodeRowBytes + row * L::kSignRowBytes) + part;
+                    // volatile: executed once, before the stage is released (a plain load may be repeated behind it)
+                    const int chunk = (h * 2 + part) * L::kSub;
+                    const volatile uint32_t* cw = reinterpret_cast<const volatile uint32_t*>(stage + row * L::kCodeRowBytes) + chunk * BITS;
+                    const volatile uint32_t* sg = reinterpret_cast<const volatile uint32_t*>(stage + kTileKeys * L::kCodeRowBytes + row * L::kSignRowBytes) + chunk;
+                    if constexpr (L::kSub == 2) {
 #pragma unroll
-                    for (int k = 0; k < BITS; ++k) w[k] = fail ? 0u : cw[k];
-                    w[BITS] = 0;
-                    sw = fail ? 0u : ~sg[0];
+                        for (int k = 0; k < 2 * BITS; k += 2) lds_once_u2(w[k], w[k + 1], cw + k);
+                        lds_once_u2(sw[0], sw[1], sg);
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < BITS; ++k) w[k] = cw[k];
+                        sw[0] = sg[0];
+                    }
+                    w[L::kSub * BITS] = 0;
                 }
                 __threadfence_block();   // every lane's loads from the stage are performed before the stage is released
                 __syncwarp();
                 if (lane == 0 && !fail) mbar_arrive(BAR(SB_K_EMPTY + s));
-                TQ_PROF_CODE(c0 = clock64(); pc[1] += c0 - c1;)
-                // expand while the A buffer may still be in use; only the stores wait for it
-                uint32_t hi[16], lo[16], sg[16];
+                const uint32_t use = kHalves == 2 ? i : i >> 1;
+                const uint32_t abase = tmem + lane_addr + group * kBufCols + part * L::kSub * 16;
 #pragma unroll
-                for (int p = 0; p < 16; ++p) {
-                    const int bit = p * 2 * BITS, wi = bit >> 5, sh = bit & 31;
-                    uint32_t e;
-                    if (sh + 2 * BITS <= 32) e = (w[wi] >> sh) & kPairMask;
-                    else e = __funnelshift_r(w[wi], w[wi + 1], sh) & kPairMask;
-                    const uint2 v = lut_lane[e * 32];
-                    hi[p] = v.x;
-                    lo[p] = v.y;
-                    // the sign word covers the 32 coordinates of this part; pair p: bits p, 16+p
-                    sg[p] = ((sw << (15 - p)) & 0x80008000u) | 0x3c003c00u;
-                }
-                TQ_PROF_CODE(c1 = clock64(); pc[4] += c1 - c0;)
-                if (!mbar_wait(BAR(SB_A_EMPTY + b), par2 ^ 1u, abort_flag)) fail = true;
-                TQ_PROF_CODE(c0 = clock64(); pc[2] += c0 - c1;)
-                tc_fence_after();
-                const uint32_t abase = tmem + lane_addr + b * kBufCols + part * 16;
-                tmem_st16(abase + kColHi, hi);
-                tmem_st16(abase + kColLo, lo);
-                tmem_st16(abase + kColSg, sg);
-                tmem_wait_st();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(BAR(SB_A_FULL + b));
-                TQ_PROF_CODE(c1 = clock64(); pc[3] += c1 - c0;)
-#ifdef TQ_PROF
-                if (a.prof && blockIdx.x == 0 && threadIdx.x == kFirstExpWarp * 32 && t + 1 == t1) {
-                    for (int k = 0; k < 5; ++k) a.prof[k] = pc[k];
-                    a.prof[6] = t1 - t0;
-                }
-#endif
-            }
-        } else {
-            for (int64_t t = t0; t < (part < kParts ? t1 : t0); ++t) {
-                const int64_t i = t - t0;
-                const int s = (int)(i % kStages);
-                TQ_PROF_CODE(long long c0 = clock64();)
-                bool fail = !mbar_wait(BAR(SB_K_FULL + s), (uint32_t)((i / kStages) & 1), abort_flag);
-                TQ_PROF_CODE(long long c1 = clock64(); pc[0] += c1 - c0;)
-#pragma unroll 1
-                for (int h = 0; h < kHalves; ++h) {
-                    const int64_t j = i * kHalves + h;       // passes through the operand buffers since the start
-                    const int b = (int)(j & 1);
-                    const uint32_t par2 = (uint32_t)((j >> 1) & 1);
-                    TQ_PROF_CODE(if (h) c1 = clock64();)
-                    uint32_t w[BITS + 1], sw;
-                    {
-                        const int chunk = h * 4 + part;      // this thread's 32 coordinates of the key
-                        const unsigned char* stage = smem + L::off_ring + s * L::kStageBytes;
-                        const volatile uint32_t* cw = reinterpret_cast<const volatile uint32_t*>(stage + row * L::kCodeRowBytes) + chunk * BITS;
-                        const volatile uint32_t* sg = reinterpret_cast<const volatile uint32_t*>(stage + kTileKeys * L::kCodeRowBytes + row * L::kSignRowBytes) + chunk;
-#pragma unroll
-                        for (int k = 0; k < BITS; ++k) w[k] = fail ? 0u : cw[k];
-                        w[BITS] = 0;
-                        sw = fail ? 0u : ~sg[0];
-                    }
-                    __threadfence_block();   // every lane's loads from the stage are performed before the stage is released
-                    __syncwarp();
-                    if (h == kHalves - 1 && lane == 0 && !fail) mbar_arrive(BAR(SB_K_EMPTY + s));
-                    TQ_PROF_CODE(c0 = clock64(); pc[1] += c0 - c1;)
-                    // expand while the A buffer may still be in use; only the stores wait for it
+                for (int c = 0; c < L::kSub; ++c) {
                     uint32_t hi[16], lo[16], sg[16];
 #pragma unroll
                     for (int p = 0; p < 16; ++p) {
-                        const int bit = p * 2 * BITS, wi = bit >> 5, sh = bit & 31;
-                        uint32_t e;
-                        if (sh + 2 * BITS <= 32) e = (w[wi] >> sh) & kPairMask;
-                        else e = __funnelshift_r(w[wi], w[wi + 1], sh) & kPairMask;
-                        const uint2 v = lut_lane[e * 32];
+                        const int bit = (c * 16 + p) * 2 * BITS, wi = bit >> 5, sh = bit & 31;
+                        uint32_t e;      // the pair's bits moved to bit 8
+                        if (sh + 2 * BITS > 32) e = __funnelshift_r(w[wi], w[wi + 1], sh) << 8;
+                        else if (sh >= 8) e = w[wi] >> (sh - 8);
+                        else e = w[wi] << (8 - sh);
+                        const uint2 v = *reinterpret_cast<const uint2*>(smem + L::off_lut + ((e & kPairMask) | lane8));
                         hi[p] = v.x;
                         lo[p] = v.y;
-                        // the sign word covers the 32 coordinates of this part; pair p: bits p, 16+p
-                        sg[p] = ((sw << (15 - p)) & 0x80008000u) | 0x3c003c00u;
+                        // the sign word covers the 32 coordinates of the chunk; pair p: bits p, 16+p
+                        sg[p] = ((~sw[c] << (15 - p)) & 0x80008000u) | 0x3c003c00u;
                     }
-                    TQ_PROF_CODE(c1 = clock64(); pc[4] += c1 - c0;)
-                    if (!mbar_wait(BAR(SB_A_EMPTY + b), par2 ^ 1u, abort_flag)) fail = true;
-                    TQ_PROF_CODE(c0 = clock64(); pc[2] += c0 - c1;)
-                    tc_fence_after();
-                    const uint32_t abase = tmem + lane_addr + b * kBufCols + part * 16;
-                    tmem_st16(abase + kColHi, hi);
-                    tmem_st16(abase + kColLo, lo);
-                    tmem_st16(abase + kColSg, sg);
-                    tmem_wait_st();
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(BAR(SB_A_FULL + b));
-                    TQ_PROF_CODE(c1 = clock64(); pc[3] += c1 - c0;)
+                    if (c == 0) {        // the first chunk is expanded while the buffer may still be in use
+                        if (!mbar_wait(BAR(SB_A_EMPTY + group), (use & 1u) ^ 1u, abort_flag)) fail = true;
+                        tc_fence_after();
+                    }
+                    tmem_st16(abase + kColHi + c * 16, hi);
+                    tmem_st16(abase + kColLo + c * 16, lo);
+                    tmem_st16(abase + kColSg + c * 16, sg);
                 }
-#ifdef TQ_PROF
-                if (a.prof && blockIdx.x == 0 && threadIdx.x == kFirstExpWarp * 32 && t + 1 == t1) {
-                    for (int k = 0; k < 5; ++k) a.prof[k] = pc[k];
-                    a.prof[6] = t1 - t0;
-                }
-#endif
+                tmem_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(BAR(SB_A_FULL + group));
             }
         }
     } else {
-        // ---- epilogue -----------------------------------------------------------------------------
+        // ---- epilogue: one thread per key ---------------------------------------------------------------
+        const int ew = warp - kFirstEpiWarp, group = ew >> 2;
         const int quarter = warp & 3;
         const int row = quarter * 32 + lane;
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
-        const int q16 = ((warp - kFirstEpiWarp) >> 2) * 16;   // this thread's 16 queries of the pass
-        const bool store_leader = threadIdx.x == kFirstEpiWarp * 32;
-        int64_t prev_g = -1, gcount = 0;
-        int bb = 0;
-        int64_t g = t0 / a.tiles_per_group, kt = t0 - g * a.tiles_per_group;
-        // norm and residual norm of this thread's key, fetched one tile ahead of their use (a load issued
-        // in the tile that needs it would stall the stores for a full trip to memory)
-        auto fetch_norms = [&](int64_t gg, int64_t kk, float& n_out, float& r_out) {
-            const int64_t key_n = kk * a.tile_stride * kTileKeys + row;
-            const bool live_n = key_n < a.key_cnt;
-            const int64_t grow_n = gg * a.keys_per_group + a.key_off + key_n;
+        const int q_mine = L::kSplitQ ? group * kQT : 0;       // first query of this thread
+        const uint32_t t_step = L::kSplitQ ? 1u : 2u;
+        const bool leader = quarter == (kFirstEpiWarp & 3) && lane == 0;     // issues the group's tensor stores
+        float* box = reinterpret_cast<float*>(smem + L::off_out + group * L::kOutBytes);
+        // norm and residual norm of this thread's key when they do not ride in the key ring: fetched one tile of this
+        // warp ahead of their use (a load issued in the tile that needs it would stall the stores for a full trip to memory)
+        auto fetch_norms = [&](uint32_t t, float& n_out, float& r_out) {
+            const uint32_t gg = t / tiles_per_group;
+            const int64_t key_n = (int64_t)(t - gg * tiles_per_group) * a.tile_stride * kTileKeys + row;
+            const bool live_n = t < t1 && key_n < a.key_cnt;
+            const int64_t grow_n = (int64_t)gg * a.keys_per_group + a.key_off + key_n;
             n_out = live_n ? __ldg(a.norms + grow_n) : 0.f;
             r_out = live_n ? __ldg(a.rnorms + grow_n) : 0.f;
         };
-        // candidate mode: thresholds of the current group, and in place of the score tile buffers a staging list of
-        // survivors (keys, then the numbers of their lists) and 16 x 32 parked scores per warp
-        int64_t thr_g = -1;
-        float* thr_s = reinterpret_cast<float*>(bars + SB_COUNT + 2);   // [QPAD]
-        int* st_count = reinterpret_cast<int*>(thr_s + QPAD);
-        constexpr int kStageCap = (2 * L::kOutBytes - 4 * kEpiPerRow * 16 * 32 * 4) / 12 / 128 * 128;    // 1,280 entries (32 queries), 640 (16), 2,688 (64)
-        static_assert(kStageCap >= 512, "candidate staging must fit the score tile buffers");
-        unsigned long long* st_keys = reinterpret_cast<unsigned long long*>(smem + L::off_out);
-        uint32_t* st_list = reinterpret_cast<uint32_t*>(smem + L::off_out + kStageCap * 8);
-        float* warp_scores = reinterpret_cast<float*>(smem + L::off_out + kStageCap * 12) + (warp - kFirstEpiWarp) * 16 * 32;
-        const int epi_t = threadIdx.x - kFirstEpiWarp * 32;
-        auto flush_staging = [&]() {      // all epilogue threads, after a barrier that made every append visible
-            int n = *st_count;
-            if (n > kStageCap) n = kStageCap;
-            for (int i = epi_t; i < n; i += kEpiThreads) {
-                const int64_t l = st_list[i];
+        // candidate mode: 16 x 32 parked scores and the staged survivors (keys, then the numbers of their lists) of this warp
+        float* parked = reinterpret_cast<float*>(smem + L::off_out) + ew * 16 * 32 + lane;
+        unsigned long long* pend = reinterpret_cast<unsigned long long*>(smem + L::off_out + kEpiWarps * 16 * 32 * 4) + ew * kPendKeys;
+        uint32_t* pend_list = reinterpret_cast<uint32_t*>(smem + L::off_out + kEpiWarps * (16 * 32 * 4 + kPendKeys * 8)) + ew * kPendKeys;
+        int n_pend = 0;
+        auto flush = [&]() {
+            __syncwarp();
+            for (int e = lane; e < n_pend; e += 32) {
+                const int64_t l = pend_list[e];
                 const int64_t gp = (int64_t)atomicAdd(a.cnt + l, 1u);
-                if (gp < a.cand_cap) a.cand[l * a.cand_cap + gp] = st_keys[i];
+                if (gp < a.cand_cap) a.cand[l * a.cand_cap + gp] = pend[e];
             }
-            bar_sync(kEpiBarrier, kEpiThreads);
-            if (epi_t == 0) *st_count = 0;
-            bar_sync(kEpiBarrier, kEpiThreads);
+            __syncwarp();
+            n_pend = 0;
         };
-        if (CAND) {
-            if (epi_t == 0) *st_count = 0;
-            bar_sync(kEpiBarrier, kEpiThreads);
-        }
+        const uint32_t t_begin = t0 + (L::kSplitQ ? 0u : (uint32_t)group);
         float nrm_next = 0.f, rn_next = 0.f;
-        if (t0 < t1 && !a.norms_bulk) fetch_norms(g, kt, nrm_next, rn_next);
-        TQ_PROF_CODE(long long ep[8] = {0, 0, 0, 0, 0, 0, 0, 0};)
-        for (int64_t t = t0; t < t1; ++t, ++kt) {
-            TQ_PROF_CODE(const long long ctop = clock64();)
-            if (kt == a.tiles_per_group) { kt = 0; ++g; }
-            const int64_t i = t - t0;
-            const int b = (int)(i & 1);        // staging buffer and accumulators of this tile
-            const uint32_t par2 = (uint32_t)((i >> 1) & 1);
-            if (g != prev_g) { bb = (kBBufs == 2 ? (int)(gcount & 1) : 0); prev_g = g; ++gcount; }
-            const int64_t key = kt * a.tile_stride * kTileKeys + row;          // within this launch's key range
+        if (t_begin < t1 && !a.norms_bulk) fetch_norms(t_begin, nrm_next, rn_next);
+        // Key groups whose prepared queries this warp is done with: it says so once for each, in order, after it has seen
+        // that they were there at all (a warp may have no tile of a short group).
+        uint32_t g_done = g_first;
+        auto release_groups = [&](uint32_t up_to) {
+            for (; g_done < up_to; ++g_done) {
+                const uint32_t c = g_done - g_first;
+                const int bb = kBBufs == 2 ? (int)(c & 1) : 0;
+                mbar_wait(BAR(SB_B_FULL + bb), (kBBufs == 2 ? c >> 1 : c) & 1, abort_flag);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(BAR(SB_B_EMPTY + bb));
+            }
+        };
+        for (uint32_t t = t_begin; t < t1; t += t_step) {
+            const uint32_t i = t - t0;
+            const uint32_t g = t / tiles_per_group, kt = t - g * tiles_per_group;
+            release_groups(g);
+            const int bb = kBBufs == 2 ? (int)((g - g_first) & 1) : 0;
+            const int64_t key = (int64_t)kt * a.tile_stride * kTileKeys + row;          // within this launch's key range
             const bool live = key < a.key_cnt;
             float nrm, arn;
             if (a.norms_bulk) {
                 // norms ride in the key ring (a load from global memory here costs a full trip to HBM per tile,
                 // which one tile of lookahead does not hide once a tile takes less than a microsecond)
                 const int s = (int)(i % kStages);
-                mbar_wait(BAR(SB_K_FULL + s), (uint32_t)((i / kStages) & 1), abort_flag);
+                mbar_wait(BAR(SB_K_FULL + s), (i / kStages) & 1, abort_flag);
                 // volatile: the values stay in registers through the whole tile, and a plain load may be executed again where
                 // the value is used (cheaper than keeping or spilling a register) -- after the arrival below, when the
                 // stage may already hold another tile.  That happened: in candidate mode, where warps that lag behind
@@ -740,167 +502,121 @@ score_tc_kernel(const __grid_constant__ CUtensorMap tmap_out, const ScoreTcArgs 
             } else {
                 nrm = nrm_next;
                 arn = a.alpha * rn_next;
-                if (t + 1 < t1) {
-                    const bool wrap = kt + 1 == a.tiles_per_group;
-                    fetch_norms(wrap ? g + 1 : g, wrap ? 0 : kt + 1, nrm_next, rn_next);
-                }
+                if (t + t_step < t1) fetch_norms(t + t_step, nrm_next, rn_next);
             }
-            TQ_PROF_CODE(long long c0 = clock64();)
-            const int db = kDBufs == 2 ? b : 0;
-            const uint32_t dpar = kDBufs == 2 ? par2 : (uint32_t)(i & 1);
-            const bool got = mbar_wait(BAR(SB_D_FULL + db), dpar, abort_flag);   // false: some role gave up
+            const int db = (int)(i % kDBufs);
+            const bool got = mbar_wait(BAR(SB_D_FULL + db), (i / kDBufs) & 1, abort_flag);   // false: some role gave up
             tc_fence_after();
-            TQ_PROF_CODE(long long c1 = clock64();)
-            TQ_PROF_CODE(long long c2 = c1;)
-            const uint32_t rowid = (uint32_t)(g * a.keys_per_group + a.key_off + key);   // row of the key arrays (candidate mode)
-            uint32_t pm = 0;      // candidate mode: bit k = this key's score for query q16 + k reaches the query's threshold
-            const uint32_t dbase = tmem + lane_addr + kColD + db * kDCols + q16;
-            const float2* ds = reinterpret_cast<const float2*>(smem + L::off_b + bb * L::kBBytes + kHalves * 4 * QPAD * kRowBytesB) + q16;
-            float sc[16];
-            {
-                uint32_t ua[16], ub[16];
-                tmem_ld16(dbase, ua);                  // C q_hi   (+ C_lo q_hi)
-                tmem_ld16(dbase + QPAD, ub);           // C_hi q_lo
-                tmem_wait_ld();
-#pragma unroll
-                for (int k = 0; k < 16; ++k) sc[k] = (__uint_as_float(ua[k]) + __uint_as_float(ub[k])) * ds[k].x;
-                tmem_ld16(dbase + 2 * QPAD, ua);       // Sg p_hi
-                tmem_ld16(dbase + 3 * QPAD, ub);       // Sg p_lo
-                tmem_wait_ld();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(BAR(SB_D_EMPTY + db));   // the accumulators are free again
-#pragma unroll
-                for (int k = 0; k < 16; ++k) {
-                    const float s2 = (__uint_as_float(ua[k]) + __uint_as_float(ub[k])) * ds[k].y;
-                    sc[k] = nrm * fmaf(arn, s2, sc[k]);
-                }
+            const uint32_t rowid = (uint32_t)((int64_t)g * a.keys_per_group + a.key_off + key);   // row of the key arrays (candidate mode)
+            const uint32_t dbase = tmem + lane_addr + kColD + db * kDCols + q_mine;
+            const float4* ds = reinterpret_cast<const float4*>(smem + L::off_b + bb * L::kBBytes + kHalves * 4 * QPAD * kRowBytesB) + q_mine / 2;
+            const float2 n2 = make_float2(nrm, nrm), r2 = make_float2(arn, arn);
+            // A give-up (`got` false) writes nothing for the tile, but every epilogue warp still walks through the named
+            // barriers: the warps learn of it at different tiles, and a barrier that some of them skipped would never complete.
+            if (!CAND && a.tile_store) {
+                // the store of this group's previous tile must have read the box before this tile overwrites it
+                if (leader) bulk_wait_read<0>();
+                bar_sync(kEpiBarrier + group, 128);
             }
-            TQ_PROF_CODE(c2 = clock64();)
-            // After a give-up (`got` false) nothing is written for the tile, but every epilogue warp still walks through the
-            // named barriers below: the warps learn of the give-up at different tiles, and a barrier that some of them
-            // skipped would never complete.
-            if (CAND) {
-                if (g != thr_g) {      // thresholds of this group's queries (constant during the launch) into shared memory
-                    thr_g = g;
-                    bar_sync(kEpiBarrier, kEpiThreads);      // everybody is done with the previous group's
-                    if (epi_t < QPAD) thr_s[epi_t] = epi_t < a.nq ? __ldg(a.thr + g * a.qpg_total + a.q0 + epi_t) : CUDART_INF_F;
-                    bar_sync(kEpiBarrier, kEpiThreads);
-                }
-                const int64_t q_first = g * a.qpg_total + a.q0 + q16;
-                if (a.fused == 2) {
-                    // The sampled pass (thresholds at -inf, every score is a candidate): the slot of a score is known
-                    // without a counter (tile of the sample x 128 + row); the host presets the lists' lengths.
-                    // A key beyond the end of the group leaves an empty slot.
 #pragma unroll
-                    for (int k = 0; k < 16; ++k)
-                        if (q16 + k < a.nq)
-                            a.cand[(q_first + k) * a.cand_cap + kt * kTileKeys + row] = live && got ? make_key(sc[k], rowid) : 0ull;
-                } else {
-                    // This thread's scores against their thresholds: a mask, and -- when any of the warp's 32 keys has
-                    // a survivor -- the scores parked in shared memory, so that the loop below can pick them by a
-                    // run-time index.
-                    float* mine = warp_scores + lane;
-                    uint32_t m = 0;
-#pragma unroll
-                    for (int k = 0; k < 16; ++k) m |= (live && got && sc[k] >= thr_s[q16 + k]) ? (1u << k) : 0u;
-                    if (__any_sync(0xffffffffu, m != 0u)) {
-#pragma unroll
-                        for (int k = 0; k < 16; ++k) mine[k * 32] = sc[k];
+            for (int q16 = 0; q16 < kQT; q16 += 16) {
+                float sc[16];
+                {
+                    uint32_t ua[16], ub[16];
+                    tmem_ld16(dbase + q16, ua);               // (C_hi + C_lo) q
+                    tmem_ld16(dbase + QPAD + q16, ub);        // Sg p
+                    tmem_wait_ld();
+                    if (q16 + 16 == kQT) {
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(BAR(SB_D_EMPTY + db));   // the accumulators are free again
                     }
-                    pm = m;
-                }
-            } else if (a.tile_store) {
-                // The tile leaves as one box [queries of the pass][128 keys]: staged in shared memory (lanes hold
-                // consecutive keys, so the stores are free of bank conflicts) and written by one bulk tensor store,
-                // which clips the keys and queries beyond the matrix.  Two staging buffers: the store of tile
-                // i - 2 must have read its buffer before tile i overwrites it.  (A box per warp -- 32 keys x 16 queries from
-                // a slice of its own, no barrier between the epilogue warps -- was slower: 115 against 109 us.)
-                float* stage = reinterpret_cast<float*>(smem + L::off_out + b * L::kOutBytes);
-                TQ_PROF_CODE(const long long s0 = clock64();)
-                if (store_leader) bulk_wait_read<1>();
-                bar_sync(kEpiBarrier, kEpiThreads);
-                TQ_PROF_CODE(const long long s1 = clock64();)
 #pragma unroll
-                for (int k = 0; k < 16; ++k) stage[(q16 + k) * kTileKeys + row] = sc[k];
-                fence_async_smem();
-                TQ_PROF_CODE(const long long s2 = clock64();)
-                bar_sync(kEpiBarrier, kEpiThreads);
-                TQ_PROF_CODE(const long long s3 = clock64();)
-                if (store_leader && got) {
-                    tensor_store_3d(&tmap_out, smem_base + L::off_out + b * L::kOutBytes, (int)(kt * kTileKeys), 0, (int)g);
-                    bulk_commit();
-                }
-                TQ_PROF_CODE(ep[4] += s1 - s0; ep[5] += s2 - s1; ep[6] += s3 - s2; ep[7] += clock64() - s3;)
-            } else if (live && got) {
-                float* out = a.scores + g * a.out_group_stride + key + (int64_t)q16 * a.out_row_stride;
-#pragma unroll
-                for (int k = 0; k < 16; ++k) {
-                    if (q16 + k < a.nq) {
-                        __stcs(out, sc[k]);
-                        out += a.out_row_stride;
+                    for (int k = 0; k < 16; k += 2) {
+                        const float4 e = ds[(q16 + k) / 2];           // 1 / scales: two of q, two of p
+                        const float2 s1 = __fmul2_rn(make_float2(__uint_as_float(ua[k]), __uint_as_float(ua[k + 1])), make_float2(e.x, e.y));
+                        const float2 s2 = __fmul2_rn(make_float2(__uint_as_float(ub[k]), __uint_as_float(ub[k + 1])), make_float2(e.z, e.w));
+                        const float2 v = __fmul2_rn(n2, __ffma2_rn(r2, s2, s1));
+                        sc[k] = v.x;
+                        sc[k + 1] = v.y;
                     }
                 }
-            }
-            if (CAND && a.fused != 2) {
-                // The loop runs once per query that has a survivor among the warp's 32 keys and is kept rolled: the candidate
-                // path must stay small, this kernel lives on its instruction cache (the same logic unrolled over the
-                // queries doubled the kernel's time without a single survivor).
-                // Survivors go to a staging list in shared memory (a global counter update per survivor would put a
-                // trip to L2 on this warp's path every tile); the list is emptied into the global lists, all its
-                // entries at once, when it is half full (looked at every eighth tile: the barrier couples the warps).
-                const float* mine = warp_scores + lane;
-                const int64_t q_first = g * a.qpg_total + a.q0 + q16;
-                if ((i & 7) == 0 && bar_or(kEpiBarrier, kEpiThreads, *st_count > kStageCap / 2)) flush_staging();
-                uint32_t wm = __reduce_or_sync(0xffffffffu, pm);
+                const int q0 = q_mine + q16;
+                if (CAND) {
+                    const int64_t list0 = (int64_t)g * a.qpg_total + a.q0 + q0;
+                    if (a.fused == 2) {
+                        // The sampled pass (thresholds at -inf, every score is a candidate): the slot of a score is known
+                        // without a counter (tile of the sample x 128 + row); the host presets the lists' lengths.
+                        // A key beyond the end of the group leaves an empty slot.
+#pragma unroll
+                        for (int k = 0; k < 16; ++k)
+                            if (q0 + k < a.nq)
+                                a.cand[(list0 + k) * a.cand_cap + (int64_t)kt * kTileKeys + row] = live && got ? make_key(sc[k], rowid) : 0ull;
+                    } else {
+                        // This thread's scores against their thresholds: a mask, and -- when any of the warp's 32 keys has
+                        // a survivor -- the scores parked in shared memory, so that the loop below, once per query with
+                        // a survivor and kept rolled (this kernel lives on its instruction cache), can pick them by
+                        // a run-time index.  Survivors are staged per warp: a global counter update per survivor would put a trip
+                        // to L2 on this warp's path every time.
+                        uint32_t m = 0;
+#pragma unroll
+                        for (int k = 0; k < 16; ++k)
+                            m |= (live && got && q0 + k < a.nq && sc[k] >= __ldg(a.thr + (q0 + k < a.nq ? list0 + k : 0))) ? (1u << k) : 0u;
+                        uint32_t wm = __reduce_or_sync(0xffffffffu, m);
+                        if (wm != 0u) {
+#pragma unroll
+                            for (int k = 0; k < 16; ++k) parked[k * 32] = sc[k];
 #pragma unroll 1
-                while (wm != 0u) {
-                    const int k = __ffs(wm) - 1;
-                    wm &= wm - 1u;
-                    const bool pass = (pm >> k) & 1u;
-                    const uint32_t votes = __ballot_sync(0xffffffffu, pass);
-                    const int leader = __ffs(votes) - 1;
-                    uint32_t base = 0;
-                    if (lane == leader) base = (uint32_t)atomicAdd(st_count, (int)__popc(votes));
-                    base = __shfl_sync(0xffffffffu, base, leader);
-                    if (pass) {
-                        const uint32_t pos = base + __popc(votes & ((1u << lane) - 1u));
-                        const unsigned long long ck = make_key(mine[k * 32], rowid);
-                        if (pos < (uint32_t)kStageCap) {
-                            st_keys[pos] = ck;
-                            st_list[pos] = (uint32_t)(q_first + k);
-                        } else {      // the staging list is full (nearly every score passes): straight to the global list
-                            const int64_t gp = (int64_t)atomicAdd(a.cnt + q_first + k, 1u);
-                            if (gp < a.cand_cap) a.cand[(q_first + k) * a.cand_cap + gp] = ck;
+                            while (wm != 0u) {
+                                const int k = __ffs(wm) - 1;
+                                wm &= wm - 1u;
+                                const bool pass = (m >> k) & 1u;
+                                const uint32_t votes = __ballot_sync(0xffffffffu, pass);
+                                if (n_pend + __popc(votes) > kPendKeys) flush();
+                                if (pass) {
+                                    const int pos = n_pend + __popc(votes & ((1u << lane) - 1u));
+                                    pend[pos] = make_key(parked[k * 32], rowid);
+                                    pend_list[pos] = (uint32_t)(list0 + k);
+                                }
+                                n_pend += __popc(votes);
+                            }
+                        }
+                    }
+                } else if (a.tile_store) {
+                    // The tile leaves as one box [queries of the group][128 keys]: staged in shared memory (lanes hold
+                    // consecutive keys, so the stores are free of bank conflicts) and written by one bulk tensor store,
+                    // which clips the keys and queries beyond the matrix.
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) box[(q16 + k) * kTileKeys + row] = sc[k];
+                } else if (live && got) {
+                    float* out = a.scores + (int64_t)g * a.out_group_stride + key + (int64_t)q0 * a.out_row_stride;
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) {
+                        if (q0 + k < a.nq) {
+                            __stcs(out, sc[k]);
+                            out += a.out_row_stride;
                         }
                     }
                 }
             }
-            TQ_PROF_CODE(ep[0] += c0 - ctop; ep[1] += c1 - c0; ep[2] += c2 - c1; ep[3] += clock64() - c2;)
-            const bool last_of_group = (t + 1 == t1) || (kt + 1 == a.tiles_per_group);
-            if (last_of_group) {
-                __syncwarp();
-                if (lane == 0) mbar_arrive(BAR(SB_B_EMPTY + bb));
+            if (!CAND && a.tile_store) {
+                fence_async_smem();
+                bar_sync(kEpiBarrier + group, 128);
+                if (leader && got) {
+                    tensor_store_3d(&tmap_out, smem_u32(box), (int)(kt * kTileKeys), q_mine, (int)g);
+                    bulk_commit();
+                }
             }
         }
-        if (CAND) {
-            bar_sync(kEpiBarrier, kEpiThreads);
-            flush_staging();
-        }
-#ifdef TQ_PROF
-        if (a.prof && blockIdx.x == 0 && threadIdx.x == kFirstEpiWarp * 32 + 32) {      // a thread that is not the store leader's warp
-            a.prof[18] = ep[0]; a.prof[12] = ep[1]; a.prof[13] = ep[2]; a.prof[14] = ep[3];
-            a.prof[19] = ep[4]; a.prof[20] = ep[5]; a.prof[21] = ep[6]; a.prof[22] = ep[7];
-        }
-#endif
-        if (store_leader) bulk_wait_all();   // the staged tiles must have left before the block's shared memory goes away
+        if (t0 < t1) release_groups((t1 - 1) / tiles_per_group + 1);
+        if (CAND) flush();
+        if (leader) bulk_wait_all();   // the staged tiles must have left before the block's shared memory goes away
     }
 
     if (*abort_flag) __nanosleep(20000);   // tensor instructions issued before the give-up may still be running
     tc_fence_before();
     __syncthreads();
     if (threadIdx.x == 0 && *abort_flag) report_status(a.status, 2ull);
-    TQ_PROF_CODE(if (a.prof && blockIdx.x == 0 && threadIdx.x == 0) { a.prof[16] = clock64() - prof_t0; a.prof[17] = prof_t1 - prof_t0; })
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem, 512);
@@ -920,10 +636,10 @@ score_prep_kernel(TqDev p, const float* __restrict__ q, int qpg, int q0, int nq,
     __half* m1 = reinterpret_cast<__half*>(base + 1 * (size_t)qpad * kRowBytesB + off);
     __half* m2 = reinterpret_cast<__half*>(base + 2 * (size_t)qpad * kRowBytesB + off);
     __half* m3 = reinterpret_cast<__half*>(base + 3 * (size_t)qpad * kRowBytesB + off);
-    float2* ds = reinterpret_cast<float2*>(base + 4 * (size_t)qpad * kRowBytesB);
+    float* ds = reinterpret_cast<float*>(base + 4 * (size_t)qpad * kRowBytesB) + (slot >> 1) * 4 + (slot & 1);   // pairs of queries: two 1 / scales of q, two of p
     if (slot >= nq) {
         *m0 = *m1 = *m2 = *m3 = __float2half_rn(0.f);
-        if (j == 0) ds[slot] = make_float2(0.f, 0.f);
+        if (j == 0) ds[0] = ds[2] = 0.f;
         return;
     }
     const int d = p.d;   // 128, or 64 with the upper half of every operand row left unused
@@ -973,7 +689,7 @@ score_prep_kernel(TqDev p, const float* __restrict__ q, int qpg, int q0, int nq,
     *m1 = __float2half_rn(rs - __half2float(rh));
     *m2 = sh;
     *m3 = __float2half_rn(ss - __half2float(sh));
-    if (j == 0) ds[slot] = make_float2(1.f / (e1 * kCentScale), 1.f / e2);
+    if (j == 0) { ds[0] = 1.f / (e1 * kCentScale); ds[2] = 1.f / e2; }
 }
 
 // The same for d = 256: the matrices do not fit shared memory and are read from global memory (usually cold), so the
@@ -995,11 +711,11 @@ score_prep256_kernel(TqDev p, const float* __restrict__ q, int qpg, int q0, int 
     __half* m1 = reinterpret_cast<__half*>(base + 1 * (size_t)qpad * kRowBytesB + off);
     __half* m2 = reinterpret_cast<__half*>(base + 2 * (size_t)qpad * kRowBytesB + off);
     __half* m3 = reinterpret_cast<__half*>(base + 3 * (size_t)qpad * kRowBytesB + off);
-    float2* ds = reinterpret_cast<float2*>(base + 8 * (size_t)qpad * kRowBytesB);
+    float* ds = reinterpret_cast<float*>(base + 8 * (size_t)qpad * kRowBytesB) + (slot >> 1) * 4 + (slot & 1);
     if (slot >= nq) {
         if (kq == 0) {
             *m0 = *m1 = *m2 = *m3 = __float2half_rn(0.f);
-            if (j == 0) ds[slot] = make_float2(0.f, 0.f);
+            if (j == 0) ds[0] = ds[2] = 0.f;
         }
         return;
     }
@@ -1040,7 +756,7 @@ score_prep256_kernel(TqDev p, const float* __restrict__ q, int qpg, int q0, int 
     *m1 = __float2half_rn(rs - __half2float(rh));
     *m2 = sh;
     *m3 = __float2half_rn(ss - __half2float(sh));
-    if (j == 0) ds[slot] = make_float2(1.f / (e1 * kCentScale), 1.f / e2);
+    if (j == 0) { ds[0] = 1.f / (e1 * kCentScale); ds[2] = 1.f / e2; }
 }
 
 // grid (segments, rows): block scans scores[row][seg*seg_len ...) and writes its k best as sortable keys
@@ -1217,12 +933,12 @@ int launch_score(const tq_plan* p, const CUtensorMap& map, const ScoreTcArgs& ar
     const int sm = ScoreSmem<BITS, QPAD, DR>::total;
     if (args.fused) {
         TQ_GRANT_SMEM((score_tc_kernel<BITS, QPAD, DR, true>), sm, p->device);
-        score_tc_kernel<BITS, QPAD, DR, true><<<grid, ScoreThreads<QPAD>::kThreads, sm, st>>>(map, args); tq_count_launch();
+        score_tc_kernel<BITS, QPAD, DR, true><<<grid, kThreads, sm, st>>>(map, args); tq_count_launch();
         TQ_CUDA_TRY(cudaGetLastError());
         return TQ_OK;
     }
     TQ_GRANT_SMEM((score_tc_kernel<BITS, QPAD, DR, false>), sm, p->device);
-    score_tc_kernel<BITS, QPAD, DR, false><<<grid, ScoreThreads<QPAD>::kThreads, sm, st>>>(map, args); tq_count_launch();
+    score_tc_kernel<BITS, QPAD, DR, false><<<grid, kThreads, sm, st>>>(map, args); tq_count_launch();
     TQ_CUDA_TRY(cudaGetLastError());
     return TQ_OK;
 }
@@ -1413,9 +1129,6 @@ int tq_launch_score_tc(const tq_plan* p, const float* q, int groups, int qpg, co
         a.thr = thr; a.cnt = cnt; a.cand = cand; a.cand_cap = cp.cand_cap;
         a.status = p->status_dev;
         a.wait_kcycles = p->wait_kcycles;
-#ifdef TQ_PROF
-        a.prof = reinterpret_cast<long long*>(p->counters + 8);
-#endif
         if (a.total_tiles == 0) return TQ_OK;
         const int grid = (int)(a.total_tiles < sms ? a.total_tiles : sms);
         // Score tiles leave through a bulk tensor store when the matrix allows one: 16-byte aligned base and
@@ -1426,7 +1139,7 @@ int tq_launch_score_tc(const tq_plan* p, const float* q, int groups, int qpg, co
         if (mat && (reinterpret_cast<uintptr_t>(a.scores) & 15u) == 0 && row_stride % 4 == 0 && key_cnt > 0 && tq_encode_tiled_fn()) {
             const cuuint64_t gdim[3] = {(cuuint64_t)key_cnt, (cuuint64_t)nq, (cuuint64_t)groups};
             const cuuint64_t gstride[2] = {(cuuint64_t)row_stride * 4, (cuuint64_t)group_stride * 4};
-            const cuuint32_t box[3] = {(cuuint32_t)kTileKeys, (cuuint32_t)qpad, 1};
+            const cuuint32_t box[3] = {(cuuint32_t)kTileKeys, (cuuint32_t)(qpad < 32 ? qpad : 32), 1};
             const cuuint32_t estr[3] = {1, 1, 1};
             const CUresult cr = tq_encode_tiled_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, a.scores, gdim, gstride, box, estr,
                                                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
