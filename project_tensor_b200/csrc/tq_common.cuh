@@ -145,6 +145,21 @@ struct TqRange {
 // Every kernel launch of the library is counted (tq_kernel_launches reports the total).
 void tq_count_launch();
 
+// Launch `kernel` so that its blocks may start while the kernel before it in the stream drains: it has to call
+// tq_grid_wait() before it touches anything that kernel writes or reads.  The kernel before allows it with tq_grid_release().
+template <class... P, class... A>
+inline cudaError_t tq_launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st; cfg.attrs = &attr; cfg.numAttrs = 1;
+    tq_count_launch();
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+__device__ __forceinline__ void tq_grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void tq_grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- launchers implemented in the kernel files -----------------------------------------------
 // Exact (reference-order float32) kernels.  With `lists` null every row is computed; otherwise
 // first the listed coordinates are re-decided (tq_launch_exact_code_check), then the listed rows

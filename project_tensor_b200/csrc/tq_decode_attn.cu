@@ -8,31 +8,56 @@
 // _core.py:1606-1683 -- done without ever writing the scores or the dequantized values to memory: per key
 // the kernel reads the packed key (d*b/8 + d/8 + 8 bytes) and the packed value (d*b/8 + 4 bytes) once.
 //
-// Two facts shape it:
-//   * scores for a few queries per group come from lookup tables (as in tq_score_few.cu): per query a pair
-//     table [d/2][4^bits] and a byte table [d/8][256], here interleaved by query so that one vector load
-//     serves all queries of a pass;
-//   * dequantize is linear after the centroid gather: sum_i p_i * norm_i * (c[idx_i] R) = (sum_i p_i norm_i
-//     c[idx_i]) R, so the block accumulates in the rotated domain (one multiply-add per coordinate, key and
-//     query) and the d x d rotation is applied once per query in the combine kernel.
+// dequantize is linear after the centroid gather: sum_i p_i * norm_i * (c[idx_i] R) = (sum_i p_i norm_i
+// c[idx_i]) R, so the kernel accumulates in the rotated domain and the d x d rotation is applied once per query
+// in the combine kernel.
 //
-// A block of 512 threads walks tiles of 512 keys of one group: thread t scores key t of the tile for the QP
-// queries of the pass, the block agrees on the running maximum (online softmax), then the same threads
-// regroup as (8 consecutive coordinates, key t / (d/8) of every batch of 512 / (d/8) keys) and add the tile's
-// values, staged in shared memory by cp.async, into their 8 x QP accumulators: one load of packed codes, one
-// of the weights and eight codebook lookups feed 8 x QP multiply-adds.  Key ranges are split over blocks; every block leaves (max, sum,
-// accumulator) per query in scratch and decode_combine_kernel merges the splits and rotates.
+// Both contractions -- keys times queries, weights times values -- run on the tensor cores with warp-level matrix
+// instructions (m16n8k16, fp16 operands, fp32 sums): the packed codes are expanded in the registers of the lane that
+// feeds them to the instruction, which tcgen05 does not offer (its operands go through tensor or shared memory, and the
+// expansion, not the arithmetic, is what costs).  To keep 32-bit accuracy every factor is split into fp16 hi + lo:
+//
+//   scores   B = queries; up to 4 queries: columns 0..3 are q_hi, columns 4..7 q_lo of the same queries; up to 8: one
+//            instruction for q_hi and one for q_lo.  A = keys x 16 coordinates; the order of the rows and of the coordinates inside
+//            a contraction is free, so lane t of a quad takes d/4 consecutive coordinates of its key -- whole 32-bit words
+//            of the packed row (d = 128) -- and the two halves of the instruction's rows are hi and lo of the same 8 keys:
+//            one table row is the operand's registers as they are.  Sign bits are used where they stand in the word, as
+//            subnormal fp16 numbers 2^(b - 24) that the scale of the projected query makes up for (a sign is 2 bit - 1).
+//   values   A = 16 coordinates x 16 keys (transposed: a register holds one coordinate of two keys), B = weights p * norm, hi
+//            and lo, which reach their lanes from the scores' layout by one 8 x 8 transposition (movmatrix).
+//
+// The tables sit in shared memory: two codes (four up to 2 bits) select a row of 256 bytes, replicated so that no two lanes of
+// a load meet in a bank; a byte permutation makes the address.  The value codes of neighbouring keys are interleaved
+// with a shift and a bit-select first.  What bounds it at d = 128, 2-bit keys, 4-bit values: shared-memory lookups (62 % of the
+// pipe's cycles; tensor pipe 24 %, integer 38 %) and the latencies of a chain that 12 warps an SM, which is what the registers
+// allow, do not fill (47 % of the issue slots).
+//
+// Every warp walks its own tiles of 16 keys with its own running softmax; there is no barrier inside the loop, and the
+// words of the next tile are fetched while a tile is computed.  A score that exceeds the warp's reference by more than
+// 2^8 moves the reference (exact softmax: the reference cancels); weights are scaled by a power of two that follows the
+// largest weight x norm seen, so that their fp16 hi parts neither overflow nor lose their lo parts.  Key ranges are split
+// over blocks; every block leaves (max, sum, accumulator) per query in scratch and decode_combine_kernel merges.
+//
+// The kernel this replaced scored from per-query lookup tables and accumulated values with one multiply-add per key,
+// coordinate and query: 64 groups x 4 queries x 32,768 keys (d = 128, 2 + 1 bit keys, 4-bit values) took 254 us, now 138; 8 queries
+// 476 and 160.
 #include "tq_common.cuh"
 
 #include <math_constants.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 namespace {
 
-constexpr int kThreads = 512;
-constexpr int kTile = 512;
-constexpr int kMaxSplits = 64;
+constexpr int kThreads = 384;
 constexpr int kWarps = kThreads / 32;
+constexpr int kTile = 16;           // keys a warp takes at a time
+constexpr int kMaxSplits = 64;
+constexpr float kCentScale = 1024.f;   // centroids (at most 1 in magnitude) before their split into fp16 hi + lo
+constexpr float kSlack = 8.f;          // a score may exceed the reference of its softmax by 2^kSlack
+constexpr float kWeightMax = 32768.f;  // largest scaled weight (fp16 reaches 65,504)
+constexpr int kRowBytes = 256;         // a table row (keys use the first half)
 
 struct DecodeArgs {
     const float* q;              // [groups][qpg][d]
@@ -43,479 +68,692 @@ struct DecodeArgs {
     const uint32_t* vcodes;
     const float* vnorms;
     const float* vcodebook;      // codebook of the value quantizer
-    int vbits, vwords;           // bits per value code, 32-bit words per packed value row
     int qpg;
     int64_t keys_per_group, group_rows;
     const int64_t* length;       // optional device-side number of keys per group (capped by keys_per_group)
     float scale_log2e;           // scale * log2(e): the softmax runs in base 2
     int splits;
-    int vbufs;                   // value tiles in shared memory: 2 = the next tile is copied while this one is used
     float* part;                 // [groups][qpg][splits][d + 2]: accumulator, running max, running sum
 };
 
-template <int QP>
-__device__ __forceinline__ void ld_vec(const float* p, float (&v)[QP]) {
-    if constexpr (QP == 4) {
-        const float4 t = *reinterpret_cast<const float4*>(p);
-        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
-    } else if constexpr (QP == 2) {
-        const float2 t = *reinterpret_cast<const float2*>(p);
-        v[0] = t.x; v[1] = t.y;
-    } else {
-        v[0] = *p;
+__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t transpose8x8(uint32_t v) {
+    uint32_t r;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+    return r;
+}
+__device__ __forceinline__ uint32_t half2_bits(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
+// (a, b) -> fp16 pairs hi and lo with hi + lo = value to about 22 bits
+__device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint32_t& lo) {
+    const __half2 h = __floats2half2_rn(a, b);
+    const float2 f = __half22float2(h);
+    hi = half2_bits(h);
+    lo = half2_bits(__floats2half2_rn(a - f.x, b - f.y));
+}
+// Shift left by s (negative: right) with s known at compile time.
+template <int S> __device__ __forceinline__ uint32_t shl(uint32_t v) {
+    if constexpr (S >= 0) return v << S;
+    else return v >> -S;
+}
+// 2^e as a float, e clamped to the normal range
+__device__ __forceinline__ float pow2i(int e) { return __int_as_float((min(max(e, -126), 127) + 127) << 23); }
+// power of two that brings a magnitude into [2^13, 2^14)
+__device__ __forceinline__ int scale_exp(float m) {
+    if (!(m > 0.f) || !(m < 3.0e38f)) return 0;
+    return min(max(13 - (int)((__float_as_uint(m) >> 23) - 127), -100), 100);
+}
+
+// f(0), f(1), ... f(N - 1) with compile-time arguments
+template <int N, class F, int I = 0>
+__device__ __forceinline__ void for_steps(F&& f) {
+    if constexpr (I < N) {
+        f(std::integral_constant<int, I>{});
+        for_steps<N, F, I + 1>(static_cast<F&&>(f));
     }
 }
-template <int QP>
-__device__ __forceinline__ void st_vec(float* p, const float (&v)[QP]) {
-    if constexpr (QP == 4) *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
-    else if constexpr (QP == 2) *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
-    else *p = v[0];
-}
 
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+// Rows of the key table: four codes at a time up to 2 bits, two at a time above.
+__host__ __device__ constexpr int codes_per_row(int bits) { return bits <= 2 ? 4 : 2; }
+__host__ __device__ constexpr int table_rows(int bits) { return 1 << (bits * codes_per_row(bits)); }
 
-template <int DR, int QP>
-__host__ __device__ constexpr int pbuf_floats() { return kTile * QP > kWarps * DR ? kTile * QP : kWarps * DR; }
+template <int KB, int VB, int DR, int NQ>
+struct Plan {
+    static constexpr int kSteps = DR / 16;            // contraction steps of the scores
+    static constexpr int kMTiles = DR / 16;           // 16-coordinate tiles of the output
+    static constexpr int kChunkCodes = VB >= 3 ? 8 : DR / 8;   // value codes that are interleaved as one word ...
+    static constexpr int kChunks = DR / 8 / kChunkCodes;       // ... and such words per lane and key
+    static constexpr int kKeyBits = DR / 4 * KB, kValBits = DR / 8 * VB;      // bits of a packed row that a lane uses
+    static constexpr int kKeyRowWords = DR * KB / 32, kValRowWords = DR * VB / 32, kSignRowWords = DR / 32;
+    // words a lane loads per row: its bits may start in the middle of a word
+    static constexpr int kKW = kKeyBits % 32 == 0 ? kKeyBits / 32 : kKeyBits / 32 + 1;
+    static constexpr int kVW = kValBits % 32 == 0 ? kValBits / 32 : (32 % kValBits == 0 ? 1 : 2);
+    static constexpr int off_val = table_rows(KB) * kRowBytes;           // value table behind the key table
+    static constexpr int kTables = off_val + (1 << (2 * VB)) * kRowBytes;
+    static constexpr int kFragBytes = kSteps * 32 * 16;      // one query operand (NQ = 8): hi and lo registers per lane
+    static constexpr int kMerge = kWarps * kMTiles * 4 * 32 * 4;      // accumulators of the warps, over the tables at the end
+    // The queries are rotated and projected by all threads at once: four consecutive outputs of one matrix and a slice
+    // of the sum per thread, so that both matrices are on their way from the L2 cache in one go.
+    static constexpr int kSlices = kThreads / (DR / 2), kSliceLen = (DR + kSlices - 1) / kSlices;
+    static constexpr int kLuts = kTables > kMerge ? kTables : kMerge;
+    static constexpr int off_frag = kLuts;                               // two query operands
+    static constexpr int off_slice = off_frag + (NQ == 8 ? 2 * kFragBytes : 0);   // [kSlices][2][NQ][DR] partial sums
+    static constexpr int off_vec = off_slice + kSlices * 2 * NQ * DR * 4;         // [2][NQ][DR] rotated, projected queries
+    static constexpr int off_qin = off_vec + 2 * NQ * DR * 4;            // [DR][NQ]
+    static constexpr int off_small = off_qin + NQ * DR * 4;              // [2][NQ] scales, [NQ] sums of the projected queries, [kWarps][NQ] max, sum, factor
+    static constexpr int total = off_small + (3 * NQ + 3 * kWarps * NQ) * 4;
+};
 
-// floats of shared memory in front of the value tiles
-template <int KB, int DR, int QP>
-constexpr size_t decode_smem_floats() {
-    return (size_t)((DR / 2) * (1 << (2 * KB)) + (DR / 8) * 256) * QP + pbuf_floats<DR, QP>() + kTile * QP + 3 * QP * DR +
-           kWarps * QP + 8 + 16;
-}
+// Packed words of one tile of 16 keys, as the lanes of a warp hold them.
+template <class P>
+struct TileWords {
+    uint32_t kc[2][P::kKW], sg[2], vc[4][P::kVW];
+    float kn[2], rn[2], vn[2];
+};
 
 // grid (splits, passes over the queries of a group, groups)
-// VSTRADDLE: the 8 codes of a thread may lie across two 32-bit words (3-bit values only)
-template <int KB, int DR, int QP, bool VSTRADDLE>
+template <int KB, int VB, int DR, int NQ>
 __global__ void __launch_bounds__(kThreads, 1)
 decode_partial_kernel(TqDev kp, DecodeArgs a) {
-    constexpr int kPairs = DR / 2, kEntries = 1 << (2 * KB), kBytes = DR / 8;
-    constexpr int kCodeWords = DR * KB / 32, kSignWords = DR / 32;
-    constexpr uint32_t kMask = kEntries - 1;
-    // scoring: 8 lanes share a key; lane l walks pairs PPL*l .. PPL*l + PPL-1 and sign bytes BPL*l .. of the row
-    constexpr int PPL = kPairs / 8, BPL = kBytes / 8;
-    constexpr int kLaneBits = PPL * 2 * KB;             // bits of the code row one lane looks at (<= 64)
-    constexpr int kSteps = kTile / (kWarps * 4);        // a warp takes 4 keys per step
-    // value phase: 8 coordinates per thread
-    constexpr int kCT = DR / 8;                         // threads that share a key
-    constexpr int kIterKeys = kThreads / kCT;           // keys the block takes per step
-    extern __shared__ __align__(16) unsigned char smraw[];
-    float* pair_t = reinterpret_cast<float*>(smraw);   // [PPL][kEntries][8 lanes][QP]
-    float* byte_t = pair_t + kPairs * kEntries * QP;    // [BPL][256][8 lanes][QP]
-    float* pbuf = byte_t + kBytes * 256 * QP;           // [kTile][QP] weight * value norm; at the end [kWarps][DR]
-    float* sbuf = pbuf + pbuf_floats<DR, QP>();         // [kTile][QP] scaled scores of the tile
-    float* qin = sbuf + kTile * QP;                     // [QP][DR]
-    float* qr = qin + QP * DR;                          // rotated queries
-    float* ps = qr + QP * DR;                           // projected queries
-    float* red = ps + QP * DR;                          // [kWarps][QP]
-    float* sm_m = red + kWarps * QP;                    // [4] running maximum per query
-    float* sm_f = sm_m + 4;                             // [4] factor that brings older sums to the new maximum
-    float* vcb = sm_f + 4;                              // [16] value codebook
-    uint32_t* vt = reinterpret_cast<uint32_t*>(vcb + 16);   // [vbufs][kTile][vwords] packed value rows
+    using P = Plan<KB, VB, DR, NQ>;
+    extern __shared__ __align__(128) unsigned char smem[];
+    float* vec = reinterpret_cast<float*>(smem + P::off_vec);
+    float* qin = reinterpret_cast<float*>(smem + P::off_qin);
+    int* scl = reinterpret_cast<int*>(smem + P::off_small);                   // exponents of the queries' scales
+    float* psum = reinterpret_cast<float*>(smem + P::off_small) + 2 * NQ;     // [NQ]
+    float* wm = psum + NQ;                                                    // [kWarps][NQ]
+    float* wl = wm + kWarps * NQ;
+    float* wf = wl + kWarps * NQ;
 
-    const int g = blockIdx.z, q0 = blockIdx.y * QP, split = blockIdx.x;
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int g = blockIdx.z, q0 = blockIdx.y * NQ, split = blockIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int t = lane & 3, r = lane >> 2;      // position in the quad, row of the fragments
     int64_t n = a.keys_per_group;
     if (a.length) {
         const int64_t len = *a.length;
         n = len < n ? len : n;
         if (n < 0) n = 0;
     }
+    const uint32_t keys = (uint32_t)n;           // rows of all groups together stay below 2^32
+    const uint32_t tiles_total = (uint32_t)((n + kTile - 1) / kTile), tps = (tiles_total + a.splits - 1) / a.splits;
+    const uint32_t tile1 = min((uint32_t)(split + 1) * tps, tiles_total);
+    uint32_t tile = (uint32_t)split * tps + warp;
 
-    for (int i = t; i < QP * DR; i += kThreads) {
-        const int qq = i / DR, k = i - qq * DR;
-        qin[i] = q0 + qq < a.qpg ? __ldg(a.q + ((size_t)g * a.qpg + q0 + qq) * DR + k) : 0.f;
-    }
-    if (t < 16) vcb[t] = t < (1 << a.vbits) ? __ldg(a.vcodebook + t) : 0.f;
-    if (t < 4) sm_m[t] = -CUDART_INF_F;
-    __syncthreads();
-    // rotated[j] = sum_k q[k] R[j][k], projected[j] = sum_k q[k] S[j][k]: one FMA per k, k ascending, as in
-    // the reference's matrix products
-    for (int i = t; i < QP * DR; i += kThreads) {
-        const int qq = i / DR, j = i - qq * DR;
-        const float* qv = qin + qq * DR;
-        float r = 0.f, sacc = 0.f;
-        for (int k0 = 0; k0 < DR; k0 += 16) {
-            float mr[16], ms[16];
+    // ---- packed words of a tile -----------------------------------------------------------------
+    // Row r of the score fragments is key (r >> 1) + 4 (r & 1) (+ 8) of the tile, so that the keys 2t, 2t + 1, 2t + 8,
+    // 2t + 9 of the value fragments are t, t + 4, t + 8, t + 12: every load of a warp covers consecutive rows.
+    const int64_t row_base = (int64_t)g * a.group_rows;
+    const int kbit = P::kKeyBits * t, kword = kbit >> 5, kshift = kbit & 31;
+    const int vbit = P::kValBits * r, vword = vbit >> 5, vshift = vbit & 31;
+    const uint32_t key_r = (uint32_t)((r >> 1) + 4 * (r & 1));
+    const uint32_t* kc_base = a.kcodes + row_base * P::kKeyRowWords + kword;
+    const uint32_t* sg_base = a.ksigns + row_base * P::kSignRowWords + (DR == 128 ? t : t >> 1);
+    const uint32_t* vc_base = a.vcodes + row_base * P::kValRowWords + vword;
+    const int vnext = vword + 1 < P::kValRowWords ? 1 : 0;
+    const float* kn_base = a.knorms + row_base;
+    const float* rn_base = a.krnorms + row_base;
+    const float* vn_base = a.vnorms + row_base;
+    auto fetch = [&](uint32_t tl, TileWords<P>& w) {
+        const uint32_t k0 = tl * kTile, last = keys - 1;       // rows behind the last one: read that one, its weight will be zero
 #pragma unroll
-            for (int u = 0; u < 16; ++u) {
-                mr[u] = __ldg(kp.Rt + (size_t)(k0 + u) * DR + j);
-                ms[u] = __ldg(kp.St + (size_t)(k0 + u) * DR + j);
-            }
-#pragma unroll
-            for (int u = 0; u < 16; ++u) {
-                r = fmaf(qv[k0 + u], mr[u], r);
-                sacc = fmaf(qv[k0 + u], ms[u], sacc);
-            }
-        }
-        qr[i] = r;
-        ps[i] = sacc;
-    }
-    __syncthreads();
-    // Tables.  Entry (i, e) of lane l sits at ((i * entries + e) * 8 + l) * QP floats: with QP = 4 the eight
-    // lanes of a key read eight different 16-byte bank groups whatever their codes are.
-    for (int idx = t; idx < kPairs * kEntries; idx += kThreads) {
-        const int l = idx & 7, e = (idx >> 3) & (kEntries - 1), i = idx / (8 * kEntries);
-        const int pp = PPL * l + i;
-        const float c0 = __ldg(kp.codebook + (e & ((1 << KB) - 1))), c1 = __ldg(kp.codebook + (e >> KB));
-#pragma unroll
-        for (int qq = 0; qq < QP; ++qq) pair_t[idx * QP + qq] = fmaf(c1, qr[qq * DR + 2 * pp + 1], c0 * qr[qq * DR + 2 * pp]);
-    }
-    for (int idx = t; idx < kBytes * 256; idx += kThreads) {
-        const int l = idx & 7, v = (idx >> 3) & 255, i = idx >> 11;
-        const int pos = BPL * l + i, w = pos >> 2, b = pos & 3;
-#pragma unroll
-        for (int qq = 0; qq < QP; ++qq) {
-            float acc = 0.f;
-#pragma unroll
-            for (int bit = 0; bit < 8; ++bit) {
-                // stored order of the sign words: even coordinates in bits 0..15, odd ones in bits 16..31
-                const int bp = 8 * b + bit;
-                const int coord = 32 * w + (bp < 16 ? 2 * bp : 2 * (bp - 16) + 1);
-                const float x = ps[qq * DR + coord];
-                acc += (v >> bit) & 1 ? x : -x;
-            }
-            byte_t[idx * QP + qq] = acc;
-        }
-    }
-
-    const int64_t tiles_total = (n + kTile - 1) / kTile;
-    const int64_t tps = (tiles_total + a.splits - 1) / a.splits;
-    const int64_t tile0 = (int64_t)split * tps;
-    int64_t tile1 = tile0 + tps;
-    if (tile1 > tiles_total) tile1 = tiles_total;
-
-    // scoring role: lane l8 of the 8 that share key (warp * 32 + step * 4 + lane / 8) of the tile
-    const int l8 = lane & 7, ksc = warp * 32 + (lane >> 3);
-    constexpr int kLastWord = kCodeWords - 1;
-    const int cw_i = (kLaneBits * l8) >> 5, cw_sh = (kLaneBits * l8) & 31;
-    const int cw_i2 = cw_i + 1 < kLastWord ? cw_i + 1 : kLastWord;
-    const int sw_i = (BPL * l8) >> 2, sw_sh = ((BPL * l8) & 3) * 8;
-    const bool b0 = l8 & 1, b1 = l8 & 2;
-    // the query whose sum the lane holds after the exchange among the eight lanes of a key
-    const int qsel = QP == 4 ? 2 * (l8 & 1) + ((l8 >> 1) & 1) : QP == 2 ? (l8 & 1) : 0;
-    const float* pair_l = pair_t + l8 * QP;
-    const float* byte_l = byte_t + l8 * QP;
-    // value role: coordinates 8c .. 8c+7 of key `ksub` of every batch of kIterKeys keys; their codes are the
-    // 8 * vbits bits that start at byte vbits * c of the packed row
-    const int c = t & (kCT - 1), ksub = t / kCT;
-    const int vbyte = a.vbits * c, vw = vbyte >> 2, vsh = (vbyte & 3) * 8;
-    const int vw2 = vw + 1 < a.vwords ? vw + 1 : vw;
-    const int vbits = a.vbits;
-    const uint32_t vmask = (1u << a.vbits) - 1u;
-    const int vwords = a.vwords;
-    const float alpha = kp.alpha;
-    const int vstride = a.vbufs > 1 ? kTile * vwords : 0;   // words between the two value buffers
-
-    float l_part[QP], acc[QP][8];
-#pragma unroll
-    for (int qq = 0; qq < QP; ++qq) {
-        l_part[qq] = 0.f;
-#pragma unroll
-        for (int u = 0; u < 8; ++u) acc[qq][u] = 0.f;
-    }
-    // packed key words and norms of the next tile, fetched one tile ahead
-    uint32_t pw0[kSteps], pw1[kSteps], psg[kSteps];
-    float pnr[kSteps], prn[kSteps], vn = 0.f;
-    auto fetch_keys = [&](int64_t tile) {
-        const int64_t k0 = tile * kTile;
-#pragma unroll
-        for (int st = 0; st < kSteps; ++st) {
-            const int64_t key = k0 + ksc + st * 4;
-            pw0[st] = 0u; pw1[st] = 0u; psg[st] = 0u; pnr[st] = 0.f; prn[st] = 0.f;
-            if (key < n) {
-                const int64_t row = (int64_t)g * a.group_rows + key;
-                const uint32_t* crow = a.kcodes + row * kCodeWords;
-                pw0[st] = __ldg(crow + cw_i);
-                pw1[st] = __ldg(crow + cw_i2);
-                psg[st] = __ldg(a.ksigns + row * kSignWords + sw_i);
-                pnr[st] = __ldg(a.knorms + row);
-                prn[st] = __ldg(a.krnorms + row);
-            }
-        }
-        vn = k0 + t < n ? __ldg(a.vnorms + (int64_t)g * a.group_rows + k0 + t) : 0.f;
-    };
-    // packed value rows of a tile -> shared memory (rows beyond n are not read from memory; what shared memory
-    // holds for them meets a weight of zero)
-    auto fetch_values = [&](int64_t tile, uint32_t* dst) {
-        const int64_t k0 = tile * kTile;
-        int64_t rows = n - k0;
-        if (rows > kTile) rows = kTile;
-        const int nwords = (int)rows * vwords;
-        const uint32_t* src = a.vcodes + ((int64_t)g * a.group_rows + k0) * vwords;
-        if ((reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
-            const int n16 = nwords >> 2;
-            for (int i = t; i < n16; i += kThreads) cp_async16(dst + 4 * i, src + 4 * i);
-            for (int i = 4 * n16 + t; i < nwords; i += kThreads) cp_async4(dst + i, src + i);
-        } else {
-            for (int i = t; i < nwords; i += kThreads) cp_async4(dst + i, src + i);
-        }
-        cp_async_commit();
-    };
-    if (tile0 < tile1) {
-        fetch_keys(tile0);
-        if (a.vbufs > 1) fetch_values(tile0, vt);
-    }
-    __syncthreads();   // tables complete
-
-    // scoring phase of a tile: its scaled scores go to sbuf, the warp's maximum per query to red
-    auto score_tile = [&](int64_t tile) {
-        const int64_t k0 = tile * kTile;
-        float mrun = -CUDART_INF_F;    // running maximum of this lane's query (qsel) over its keys of the tile
-#pragma unroll
-        for (int st = 0; st < kSteps; ++st) {
-            float v[QP];
-            const uint32_t lo = __funnelshift_r(pw0[st], pw1[st], cw_sh);
-            const uint64_t z = kLaneBits > 32 ? ((uint64_t)(pw1[st] >> cw_sh) << 32) | lo : (uint64_t)lo;
-            const uint32_t sg = psg[st] >> sw_sh;
-            float a1[QP], a2[QP];
-#pragma unroll
-            for (int qq = 0; qq < QP; ++qq) { a1[qq] = 0.f; a2[qq] = 0.f; }
-#pragma unroll
-            for (int i = 0; i < PPL; ++i) {
-                const uint32_t e = (uint32_t)(z >> (i * 2 * KB)) & kMask;
-                float x[QP];
-                ld_vec<QP>(pair_l + (i * kEntries + e) * 8 * QP, x);
-#pragma unroll
-                for (int qq = 0; qq < QP; ++qq) a1[qq] += x[qq];
-            }
-#pragma unroll
-            for (int i = 0; i < BPL; ++i) {
-                float x[QP];
-                ld_vec<QP>(byte_l + (i * 256 + ((sg >> (8 * i)) & 255u)) * 8 * QP, x);
-#pragma unroll
-                for (int qq = 0; qq < QP; ++qq) a2[qq] += x[qq];
-            }
-            const float ar = alpha * prn[st];
-#pragma unroll
-            for (int qq = 0; qq < QP; ++qq) v[qq] = fmaf(ar, a2[qq], a1[qq]);
-            // The eight partial sums of every query meet in a reduce-scatter: lanes trade the values their partner
-            // keeps, so QP = 4 takes 2 + 1 + 1 shuffles instead of the 12 of four butterflies (shuffles share the
-            // pipe of the lookups).  The lane ends with the sum of query qsel.
-            float s;
-            if constexpr (QP == 4) {
-                const float rx = __shfl_xor_sync(0xffffffffu, b0 ? v[0] : v[2], 1);
-                const float ry = __shfl_xor_sync(0xffffffffu, b0 ? v[1] : v[3], 1);
-                const float ax = (b0 ? v[2] : v[0]) + rx, ay = (b0 ? v[3] : v[1]) + ry;
-                s = (b1 ? ay : ax) + __shfl_xor_sync(0xffffffffu, b1 ? ax : ay, 2);
-            } else if constexpr (QP == 2) {
-                s = (b0 ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, b0 ? v[0] : v[1], 1);
-                s += __shfl_xor_sync(0xffffffffu, s, 2);
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t key = min(k0 + key_r + 8 * h, last);
+            const uint32_t* src = kc_base + (size_t)key * P::kKeyRowWords;
+            if constexpr (P::kKW == 4) {
+                const uint4 v = __ldg(reinterpret_cast<const uint4*>(src));
+                w.kc[h][0] = v.x; w.kc[h][1] = v.y; w.kc[h][2] = v.z; w.kc[h][3] = v.w;
+            } else if constexpr (P::kKeyBits == 64) {
+                const uint2 v = __ldg(reinterpret_cast<const uint2*>(src));
+                w.kc[h][0] = v.x; w.kc[h][1] = v.y;
             } else {
-                s = v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
-                s += __shfl_xor_sync(0xffffffffu, s, 2);
+#pragma unroll
+                for (int i = 0; i < P::kKW; ++i) w.kc[h][i] = __ldg(src + i);
             }
-            s += __shfl_xor_sync(0xffffffffu, s, 4);
-            const bool valid = k0 + ksc + st * 4 < n;
-            s = valid ? s * (pnr[st] * a.scale_log2e) : -CUDART_INF_F;
-            mrun = fmaxf(mrun, s);
-            if (l8 < QP) sbuf[(ksc + st * 4) * QP + qsel] = s;
+            w.sg[h] = __ldg(sg_base + (size_t)key * P::kSignRowWords);
+            w.kn[h] = __ldg(kn_base + key);
+            w.rn[h] = __ldg(rn_base + key);
+            w.vn[h] = __ldg(vn_base + key);
         }
-        {
-            // lanes 0..QP-1 of the warp end with the maximum of their query over the warp's 32 keys
-            float m = mrun;
-            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
-            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
-            if (lane < QP) red[warp * QP + qsel] = m;
-        }
-    };
-    // value phase of a tile: weights (pbuf) times centroid values, added to the accumulators
-    auto value_tile = [&](const uint32_t* vcur) {
-#pragma unroll 4
-        for (int it = 0; it < kTile / kIterKeys; ++it) {
-            const int kk = it * kIterKeys + ksub;
-            uint32_t cbits = vcur[kk * vwords + vw];
-            if (VSTRADDLE) cbits = __funnelshift_r(cbits, vcur[kk * vwords + vw2], vsh);
-            else cbits >>= vsh;
-            float pq[QP];
-            ld_vec<QP>(pbuf + kk * QP, pq);
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const float cv = vcb[cbits & vmask];
-                cbits >>= vbits;
-#pragma unroll
-                for (int qq = 0; qq < QP; ++qq) acc[qq][u] = fmaf(pq[qq], cv, acc[qq][u]);
+        for (int h = 0; h < 4; ++h) {
+            const uint32_t* src = vc_base + (size_t)min(k0 + t + 4 * h, last) * P::kValRowWords;
+            if constexpr (P::kValBits == 64) {
+                const uint2 v = __ldg(reinterpret_cast<const uint2*>(src));
+                w.vc[h][0] = v.x; w.vc[h][1] = v.y;
+            } else {
+                w.vc[h][0] = __ldg(src);
+                if constexpr (P::kVW == 2) w.vc[h][1] = __ldg(src + vnext);
             }
         }
     };
-    if (tile0 < tile1) score_tile(tile0);
+    TileWords<P> cur;
+    if (tile < tile1) fetch(tile, cur);        // on its way while the block prepares
 
-    int buf = 0;
-    for (int64_t tile = tile0; tile < tile1; ++tile) {
-        const float vn_tile = vn;
-        __syncthreads();   // scores and tile maxima visible; the value phase of the previous tile is over
-        if (a.vbufs == 1) fetch_values(tile, vt);
-        if (t < ((kWarps * QP + 31) & ~31)) {   // whole warps, so that the shuffles have all their lanes
-            // 16 lanes per query: each takes one warp's maximum, a butterfly leaves the tile maximum in all of them
-            const int qq = t / kWarps, w = t & (kWarps - 1);
-            float mt = qq < QP ? red[w * QP + qq] : -CUDART_INF_F;
+    // ---- tables and queries -----------------------------------------------------------------------
+    for (int i = tid; i < NQ * DR; i += kThreads) {
+        const int qq = i / DR, k = i - qq * DR;
+        qin[k * NQ + qq] = q0 + qq < a.qpg ? __ldg(a.q + ((size_t)g * a.qpg + q0 + qq) * DR + k) : 0.f;
+    }
+    const int xm = tid / (DR / 4) & 1, xj = tid % (DR / 4) * 4, xs = tid / (DR / 2), xk = xs * P::kSliceLen;    // matrix, first output, slice
+    float4 mat[P::kSliceLen];
+    {
+        const float* src = (xm ? kp.St : kp.Rt) + xj;
 #pragma unroll
-            for (int o = kWarps / 2; o > 0; o >>= 1) mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, o));
-            if (w == 0 && qq < QP) {
-                const float mo = sm_m[qq], mn = fmaxf(mo, mt);
-                sm_f[qq] = mn == -CUDART_INF_F ? 1.f : exp2f(mo - mn);
-                sm_m[qq] = mn;
+        for (int u = 0; u < P::kSliceLen; ++u)
+            mat[u] = xk + u < DR ? __ldg(reinterpret_cast<const float4*>(src + (size_t)(xk + u) * DR)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    // Key table, row e: 128 bytes of copies of (hi, lo) of a pair of codes, or (hi, lo, hi, lo) of four codes: the registers
+    // of an A operand.  Value table: 32 copies of hi, 32 copies of lo of the same coordinate of two keys.  A thread fills whole
+    // rows, starting at a copy of its own (stores to rows 256 bytes apart would all hit the same banks).
+    auto value = [](const float* codebook, int code) { return __ldg(codebook + code) * kCentScale; };
+    for (int e = tid; e < table_rows(KB); e += kThreads) {
+        constexpr int m = (1 << KB) - 1;
+        uint4 v;
+        split_pair(value(kp.codebook, e & m), value(kp.codebook, (e >> KB) & m), v.x, v.y);
+        if constexpr (codes_per_row(KB) == 4) split_pair(value(kp.codebook, (e >> 2 * KB) & m), value(kp.codebook, e >> 3 * KB), v.z, v.w);
+        else { v.z = v.x; v.w = v.y; }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(smem + e * kRowBytes + ((i + tid) & 7) * 16) = v;
+    }
+    for (int e = kThreads - 1 - tid; e < 1 << (2 * VB); e += kThreads) {
+        uint32_t hi, lo;
+        split_pair(value(a.vcodebook, e & ((1 << VB) - 1)), value(a.vcodebook, e >> VB), hi, lo);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            *reinterpret_cast<uint4*>(smem + P::off_val + e * kRowBytes + ((i + tid) & 7) * 16) = make_uint4(hi, hi, hi, hi);
+            *reinterpret_cast<uint4*>(smem + P::off_val + e * kRowBytes + 128 + ((i + tid) & 7) * 16) = make_uint4(lo, lo, lo, lo);
+        }
+    }
+    __syncthreads();
+    // rotated[j] = sum_k q[k] R[j][k], projected[j] = sum_k q[k] S[j][k] in 32-bit arithmetic
+    float* slice = reinterpret_cast<float*>(smem + P::off_slice);
+    {
+        float4 sum[NQ];
+#pragma unroll
+        for (int qq = 0; qq < NQ; ++qq) sum[qq] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < P::kSliceLen; ++u) {
+            const float* qk = qin + min(xk + u, DR - 1) * NQ;       // (meets a matrix element of zero behind the end)
+#pragma unroll
+            for (int qq = 0; qq < NQ; ++qq) {
+                const float v = qk[qq];
+                sum[qq].x = fmaf(v, mat[u].x, sum[qq].x);
+                sum[qq].y = fmaf(v, mat[u].y, sum[qq].y);
+                sum[qq].z = fmaf(v, mat[u].z, sum[qq].z);
+                sum[qq].w = fmaf(v, mat[u].w, sum[qq].w);
             }
         }
-        __syncthreads();
-        {
-            float s[QP], pv[QP];
-            ld_vec<QP>(sbuf + t * QP, s);
 #pragma unroll
-            for (int qq = 0; qq < QP; ++qq) {
-                const float mn = sm_m[qq], f = sm_f[qq];
-                const float p = exp2f(s[qq] - (mn == -CUDART_INF_F ? 0.f : mn));   // masked keys: exp2(-inf) = 0
-                l_part[qq] = fmaf(l_part[qq], f, p);
+        for (int qq = 0; qq < NQ; ++qq) *reinterpret_cast<float4*>(slice + ((xs * 2 + xm) * NQ + qq) * DR + xj) = sum[qq];
+    }
+    __syncthreads();
+    for (int i = tid; i < 2 * NQ * DR; i += kThreads) {
+        float v = slice[i];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) acc[qq][u] *= f;
-                pv[qq] = p * vn_tile;
+        for (int u = 1; u < P::kSlices; ++u) v += slice[u * 2 * NQ * DR + i];
+        vec[i] = v;
+    }
+    __syncthreads();
+    for (int v = warp; v < 2 * NQ; v += kWarps) {
+        float m = 0.f, sum = 0.f;
+        for (int k = lane; k < DR; k += 32) {
+            m = fmaxf(m, fabsf(vec[v * DR + k]));
+            sum += vec[v * DR + k];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+            sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        }
+        if (lane == 0) {
+            scl[v] = scale_exp(m);
+            if (v >= NQ) psum[v - NQ] = sum;
+        }
+    }
+    __syncthreads();
+    // Query operands.  Up to 4 queries: in registers, column r is hi (r < 4) or lo (r >= 4) of query r & 3.  Up to 8: in
+    // shared memory, (hi b0, hi b1, lo b0, lo b1) of query r per lane and step.  The sign bits of a pair of coordinates are
+    // used where they stand, as the fp16 numbers 0 or 2^(b - 24) (b = 0..7, see below): the projected query is scaled by 2^-b.
+    constexpr int kRegSteps = NQ == 4 ? P::kSteps : 1;
+    uint32_t qf[2][kRegSteps][2];
+    {
+        const int qq = NQ == 4 ? r & 3 : r;
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+            const float* x = vec + (m * NQ + qq) * DR + t * (DR / 4);
+            const float sc = pow2i(scl[m * NQ + qq]);
+#pragma unroll
+            for (int s = 0; s < P::kSteps; ++s) {
+                if (NQ == 8 && s % kWarps != warp) continue;      // (each warp stores some of the steps)
+                uint32_t h0, l0, h1, l1;
+                const float s0 = m == 0 ? sc : sc * (1.f / (1 << ((2 * s) & 7))), s1 = m == 0 ? sc : sc * (1.f / (1 << ((2 * s + 1) & 7)));
+                split_pair(x[4 * s] * s0, x[4 * s + 1] * s0, h0, l0);
+                split_pair(x[4 * s + 2] * s1, x[4 * s + 3] * s1, h1, l1);
+                if constexpr (NQ == 4) {
+                    qf[m][s][0] = r < 4 ? h0 : l0;
+                    qf[m][s][1] = r < 4 ? h1 : l1;
+                } else {
+                    *reinterpret_cast<uint4*>(smem + P::off_frag + m * P::kFragBytes + (s * 32 + lane) * 16) = make_uint4(h0, h1, l0, l1);
+                }
             }
-            st_vec<QP>(pbuf + t * QP, pv);
         }
-        cp_async_wait_all();
-        __syncthreads();
-        const uint32_t* vcur = vt + buf * vstride;
-        if (tile + 1 < tile1) {
-            fetch_keys(tile + 1);
-            if (a.vbufs > 1) fetch_values(tile + 1, vt + (buf ^ 1) * vstride);
+    }
+    if constexpr (NQ == 8) __syncthreads();
+    // The two queries of this lane's score columns: descaling factors, softmax state.  A sign is 2 bit - 1: the contraction
+    // with the bits, doubled, less the sum of the projected query.
+    float ds1[2], ds2[2], dsum[2], mref[2], lsum[2];
+    float wsc[2];                     // power of two that scales the weights
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        const int qq = (2 * t + c) & (NQ - 1);
+        ds1[c] = pow2i(-scl[qq]) * (1.f / kCentScale);
+        ds2[c] = pow2i(25 - scl[NQ + qq]) * kp.alpha;
+        dsum[c] = 2 * t < NQ ? -kp.alpha * psum[qq] : 0.f;     // (once: hi and lo columns are added)
+        mref[c] = -CUDART_INF_F;
+        lsum[c] = 0.f;
+        wsc[c] = pow2i(126);
+    }
+    float acc[P::kMTiles][4];
+#pragma unroll
+    for (int i = 0; i < P::kMTiles; ++i)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[i][c] = 0.f;
+
+    // Table lookups.  A byte of a word selects a row with one byte permutation: (lane's copy, byte, 0, 0) is its address.
+    const uint32_t lane4 = (uint32_t)lane * 4u, lane8 = (uint32_t)(lane & 15) * 8u, lane16 = (uint32_t)(lane & 7) * 16u;
+    auto pick = [&](uint32_t word, int byte, uint32_t copy) { return __byte_perm(word, copy, 0x5504u | (uint32_t)byte << 4); };
+    auto row8 = [&](uint32_t at) { return *reinterpret_cast<const uint2*>(smem + at); };
+    auto row16 = [&](uint32_t at) { return *reinterpret_cast<const uint4*>(smem + at); };
+
+    // ---- tiles ----------------------------------------------------------------------------------------
+    tq_grid_release();      // (the blocks that merge may take an SM when its last block here has ended)
+    for (; tile < tile1; tile += kWarps) {
+        TileWords<P> nxt;
+        if (tile + kWarps < tile1) fetch(tile + kWarps, nxt);
+        const uint32_t left = keys - tile * kTile;      // keys of this tile and behind it
+        // -- scores
+        float c1[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, c2[4] = {0.f, 0.f, 0.f, 0.f};
+        uint32_t kw[2][P::kKW], kw1[2], sw[2][2];
+        (void)kw1;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if constexpr (P::kKeyBits % 32 == 0) {
+#pragma unroll
+                for (int i = 0; i < P::kKW; ++i) kw[h][i] = cur.kc[h][i];
+            } else {
+                // half words (d = 64, odd bits): shift them to the front
+                if constexpr (P::kKW == 2) {
+                    kw[h][0] = __funnelshift_r(cur.kc[h][0], cur.kc[h][1], kshift);
+                    kw[h][1] = cur.kc[h][1] >> kshift;
+                } else {
+                    kw[h][0] = cur.kc[h][0] >> kshift;
+                }
+            }
+            sw[h][0] = DR == 128 ? cur.sg[h] : cur.sg[h] >> (8 * (t & 1));
+            sw[h][1] = sw[h][0] >> 8;
+            if constexpr (KB == 1) {         // four codes: a nibble; even ones and odd ones in words of their own
+                kw1[h] = (kw[h][0] >> 4) & 0x0f0f0f0fu;
+                kw[h][0] &= 0x0f0f0f0fu;
+            }
         }
-        // Between here and the next barrier every warp owes the value phase of this tile and the scoring phase of
-        // the next one.  Even warps take them in that order, odd warps in the other, so that at any time half of
-        // the SM's warps walk the tables (16-byte shared-memory loads) while the other half multiply and add.
-        const bool more = tile + 1 < tile1;
-        for (int ph = 0; ph < 2; ++ph) {
-            if (((ph ^ warp) & 1) == 0) value_tile(vcur);
-            else if (more) score_tile(tile + 1);
+        auto key_step = [&](auto sc) {
+            constexpr int s = decltype(sc)::value;
+            uint32_t ak[2][4], as[4];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                // coordinates 4s .. 4s + 3 of the lane
+                if constexpr (KB >= 3) {
+                    uint2 v0, v1;
+                    if constexpr (KB == 4) {
+                        v0 = row8(pick(kw[h][s >> 1], 2 * (s & 1), lane8));
+                        v1 = row8(pick(kw[h][s >> 1], 2 * (s & 1) + 1, lane8));
+                    } else {
+                        auto pair = [&](auto pc) {
+                            constexpr int bit = decltype(pc)::value * 6, w0 = bit >> 5, sh = bit & 31;
+                            uint32_t x;                   // the pair at bit 8
+                            if constexpr (sh + 6 > 32) x = __funnelshift_r(kw[h][w0], kw[h][w0 + 1 < P::kKW ? w0 + 1 : w0], sh - 8);
+                            else x = shl<8 - sh>(kw[h][w0]);
+                            return row8((x & 0x3f00u) | lane8);
+                        };
+                        v0 = pair(std::integral_constant<int, 2 * s>{});
+                        v1 = pair(std::integral_constant<int, 2 * s + 1>{});
+                    }
+                    ak[h][0] = v0.x; ak[h][1] = v0.y; ak[h][2] = v1.x; ak[h][3] = v1.y;
+                } else {
+                    const uint4 v = row16(KB == 2 ? pick(kw[h][s >> 2], s & 3, lane16) : pick(s & 1 ? kw1[h] : kw[h][0], s >> 1, lane16));
+                    ak[h][0] = v.x; ak[h][1] = v.y; ak[h][2] = v.z; ak[h][3] = v.w;
+                }
+                // signs of two coordinates: bit b = (pair & 7) of both halves of the word (or of the word moved by 8), where it
+                // stands -- a subnormal number 2^(b - 24), which the operand of the query makes up for
+                as[h] = sw[h][s >> 2] & (0x00010001u << ((2 * s) & 7));
+                as[2 + h] = sw[h][s >> 2] & (0x00010001u << ((2 * s + 1) & 7));
+            }
+            if constexpr (NQ == 4) {
+                mma16816(c1[0], ak[0], qf[0][s][0], qf[0][s][1]);
+                mma16816(c1[1], ak[1], qf[0][s][0], qf[0][s][1]);
+                mma16816(c2, as, qf[1][s][0], qf[1][s][1]);
+            } else {
+                const uint4 b = *reinterpret_cast<const uint4*>(smem + P::off_frag + (s * 32 + lane) * 16);
+                const uint4 p = *reinterpret_cast<const uint4*>(smem + P::off_frag + P::kFragBytes + (s * 32 + lane) * 16);
+                mma16816(c1[0], ak[0], b.x, b.y);
+                mma16816(c1[1], ak[1], b.x, b.y);
+                mma16816(c2, as, p.x, p.y);
+                mma16816(c1[0], ak[0], b.z, b.w);
+                mma16816(c1[1], ak[1], b.z, b.w);
+                mma16816(c2, as, p.z, p.w);
+            }
+        };
+        for_steps<P::kSteps>(key_step);
+        float s[2][2];                 // [key r + 8 h][query column c]
+        bool above = false;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                float v = fmaf(fmaf(c2[2 * h + c], ds2[c], dsum[c]), cur.rn[h], (c1[h][c] + c1[h][2 + c]) * ds1[c]);
+                if constexpr (NQ == 4) v += __shfl_xor_sync(0xffffffffu, v, 2);     // hi and lo columns
+                v *= cur.kn[h] * a.scale_log2e;
+                s[h][c] = key_r + 8 * h < left ? v : -CUDART_INF_F;
+                above = above || s[h][c] > mref[c] + kSlack;
+            }
         }
-        if (a.vbufs > 1) buf ^= 1;
+        // -- softmax reference and weights
+        if (__any_sync(0xffffffffu, above)) {
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                float m = fmaxf(s[0][c], s[1][c]);
+#pragma unroll
+                for (int o = 4; o < 32; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+                m = fmaxf(m, mref[c]);
+                if (m > mref[c]) {
+                    const float step = m - mref[c];      // +inf the first time: nothing to carry over
+                    const int e0 = (int)(__float_as_uint(wsc[c]) >> 23) - 127, up = step < 252.f ? (int)step : 252;
+                    const int e = min(126, e0 + up);          // older weights shrink by 2^-step: their scale may grow
+                    const float f = exp2f(-step), fw = exp2f((float)(e - e0) - step);
+                    lsum[c] *= f;
+                    wsc[c] = pow2i(e);
+                    mref[c] = m;
+#pragma unroll
+                    for (int i = 0; i < P::kMTiles; ++i) { acc[i][c] *= fw; acc[i][2 + c] *= fw; }
+                }
+            }
+        }
+        float u[2][2];
+        bool big = false;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float vn = key_r + 8 * h < left ? cur.vn[h] : 0.f;
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const float p = exp2f(s[h][c] - (mref[c] == -CUDART_INF_F ? 0.f : mref[c]));   // masked keys: exp2(-inf) = 0
+                lsum[c] += p;
+                u[h][c] = p * vn;
+                big = big || u[h][c] * wsc[c] > kWeightMax;
+            }
+        }
+        if (__any_sync(0xffffffffu, big)) {
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                float m = fmaxf(u[0][c], u[1][c]);
+#pragma unroll
+                for (int o = 4; o < 32; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+                if (m * wsc[c] > kWeightMax) {
+                    const int e0 = (int)(__float_as_uint(wsc[c]) >> 23) - 127;
+                    const int e = max(13 - (int)((__float_as_uint(m) >> 23) - 127), -126);     // the largest becomes 2^13 .. 2^14
+                    const float fw = pow2i(e - e0) * (e - e0 < -126 ? 0.f : 1.f);
+                    wsc[c] = pow2i(e);
+#pragma unroll
+                    for (int i = 0; i < P::kMTiles; ++i) { acc[i][c] *= fw; acc[i][2 + c] *= fw; }
+                }
+            }
+        }
+        uint32_t bh[2], bl[2];          // weights as the B operand: keys 2t, 2t + 1 (+ 8 h) of column r
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            uint32_t hi, lo;
+            split_pair(u[h][0] * wsc[0], u[h][1] * wsc[1], hi, lo);
+            if constexpr (NQ == 4) {
+                bh[h] = transpose8x8(t < 2 ? hi : lo);
+            } else {
+                bh[h] = transpose8x8(hi);
+                bl[h] = transpose8x8(lo);
+            }
+        }
+        // -- values
+        uint32_t ve[2][P::kChunks], vo[2][P::kChunks], ve1[2], vo1[2];     // per pair of keys: even and odd coordinates, codes of both keys side by side
+        (void)ve1; (void)vo1;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+#pragma unroll
+            for (int ch = 0; ch < P::kChunks; ++ch) {
+                uint32_t x[2];
+#pragma unroll
+                for (int y = 0; y < 2; ++y) {
+                    const uint32_t w0 = cur.vc[2 * h + y][0], w1 = cur.vc[2 * h + y][P::kVW - 1];
+                    constexpr int kAt = P::kChunkCodes * VB;            // bits of a chunk
+                    if constexpr (P::kValBits == 64) x[y] = ch == 0 ? w0 : w1;
+                    else if constexpr (P::kVW == 2) x[y] = ch == 0 ? __funnelshift_r(w0, w1, vshift) : (uint32_t)((((uint64_t)w1 << 32) | w0) >> (vshift + kAt));
+                    else x[y] = P::kValBits % 32 == 0 ? w0 : w0 >> vshift;
+                }
+                constexpr uint32_t kEven = VB == 4 ? 0x0f0f0f0fu : VB == 3 ? 0x001c71c7u : VB == 2 ? 0x33333333u : 0x55555555u;
+                ve[h][ch] = (x[0] & kEven) | ((x[1] << VB) & (kEven << VB));
+                vo[h][ch] = ((x[0] >> VB) & kEven) | (x[1] & (kEven << VB));
+            }
+        }
+        if constexpr (VB == 2) {            // a field is a nibble: even ones and odd ones in words of their own
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                ve1[h] = (ve[h][0] >> 4) & 0x0f0f0f0fu; ve[h][0] &= 0x0f0f0f0fu;
+                vo1[h] = (vo[h][0] >> 4) & 0x0f0f0f0fu; vo[h][0] &= 0x0f0f0f0fu;
+            }
+        }
+        auto value_tile = [&](auto mc) {
+            constexpr int mt = decltype(mc)::value;
+            uint32_t ah[4], al[4];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                auto row = [&](const uint32_t (&w)[P::kChunks], uint32_t w1) {
+                    if constexpr (VB == 4) return pick(w[mt >> 2], mt & 3, lane4);
+                    else if constexpr (VB == 3) return (shl<8 - 6 * (mt & 3)>(w[mt >> 2]) & 0x3f00u) | lane4;
+                    else if constexpr (VB == 2) return pick(mt & 1 ? w1 : w[0], mt >> 1, lane4);
+                    else return (shl<8 - 2 * mt>(w[0]) & 0x300u) | lane4;
+                };
+                const uint32_t e = row(ve[h], ve1[h]), o = row(vo[h], vo1[h]);
+                ah[2 * h] = *reinterpret_cast<const uint32_t*>(smem + P::off_val + e);
+                al[2 * h] = *reinterpret_cast<const uint32_t*>(smem + P::off_val + 128 + e);
+                ah[2 * h + 1] = *reinterpret_cast<const uint32_t*>(smem + P::off_val + o);
+                al[2 * h + 1] = *reinterpret_cast<const uint32_t*>(smem + P::off_val + 128 + o);
+            }
+            mma16816(acc[mt], ah, bh[0], bh[1]);
+            mma16816(acc[mt], al, bh[0], bh[1]);
+            if constexpr (NQ == 8) mma16816(acc[mt], ah, bl[0], bl[1]);
+        };
+        for_steps<P::kMTiles>(value_tile);
+        cur = nxt;
     }
 
-    __syncthreads();   // last value phase over: pbuf and red are free
+    // ---- merge the warps -----------------------------------------------------------------------------------
 #pragma unroll
-    for (int qq = 0; qq < QP; ++qq) {
-        float v = l_part[qq];
+    for (int c = 0; c < 2; ++c) {
+        float v = lsum[c];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0) red[warp * QP + qq] = v;
-    }
-    // accumulators: lanes c, c + kCT, ... of a warp hold the same coordinates; warps are added through pbuf
-    float res[QP];
-#pragma unroll
-    for (int qq = 0; qq < QP; ++qq) {
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            float v = acc[qq][u];
-#pragma unroll
-            for (int o = kCT; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane < kCT) pbuf[warp * DR + lane * 8 + u] = v;
+        for (int o = 4; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (r == 0 && 2 * t < NQ) {
+            wm[warp * NQ + 2 * t + c] = mref[c];
+            wl[warp * NQ + 2 * t + c] = v;
         }
-        __syncthreads();
-        float sum = 0.f;
-        if (t < DR) {
-#pragma unroll
-            for (int w = 0; w < kWarps; ++w) sum += pbuf[w * DR + t];
-        }
-        res[qq] = sum;
-        __syncthreads();
     }
-    if (t < DR) {
-#pragma unroll
-        for (int qq = 0; qq < QP; ++qq) {
-            if (q0 + qq >= a.qpg) continue;
+    __syncthreads();          // maxima in place; the tables are no longer needed
+    for (int qq = tid; qq < NQ; qq += kThreads) {
+        float m = -CUDART_INF_F, l = 0.f;
+        for (int w = 0; w < kWarps; ++w) m = fmaxf(m, wm[w * NQ + qq]);
+        for (int w = 0; w < kWarps; ++w) {
+            const float f = wm[w * NQ + qq] == -CUDART_INF_F ? 0.f : exp2f(wm[w * NQ + qq] - m);
+            wf[w * NQ + qq] = f;
+            l = fmaf(f, wl[w * NQ + qq], l);
+        }
+        if (q0 + qq < a.qpg) {
             float* dst = a.part + (((size_t)g * a.qpg + q0 + qq) * a.splits + split) * (DR + 2);
-            dst[t] = res[qq];
-            if (t == 0) {
-                float l = 0.f;
-#pragma unroll
-                for (int w = 0; w < kWarps; ++w) l += red[w * QP + qq];
-                dst[DR] = sm_m[qq];
-                dst[DR + 1] = l;
-            }
+            dst[DR] = m;
+            dst[DR + 1] = l;
         }
+    }
+    // accumulators as the lanes hold them, [warp][tile][register][lane]
+    float* wacc = reinterpret_cast<float*>(smem);
+    constexpr int kAcc = P::kMTiles * 4 * 32;
+#pragma unroll
+    for (int i = 0; i < P::kMTiles; ++i)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) wacc[warp * kAcc + (i * 4 + c) * 32 + lane] = acc[i][c] * (1.f / wsc[c & 1]) * (1.f / kCentScale);
+    __syncthreads();
+    for (int i = tid; i < NQ * DR; i += kThreads) {
+        const int qq = i / DR, j = i - qq * DR;
+        if (q0 + qq >= a.qpg) continue;
+        // coordinate j is 2 i + (c >> 1) of row j / (DR / 8), query qq in register c & 1 of lane qq / 2 (lo columns: two lanes further)
+        const int jr = j / (DR / 8), jc = j % (DR / 8);
+        const float* src = wacc + ((jc >> 1) * 4 + (jc & 1) * 2 + (qq & 1)) * 32 + jr * 4 + (qq >> 1);
+        float v = 0.f;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+            const float f = wf[w * NQ + qq];
+            const float x = NQ == 4 ? src[w * kAcc] + src[w * kAcc + 2] : src[w * kAcc];
+            v = fmaf(f, f == 0.f ? 0.f : x, v);
+        }
+        a.part[(((size_t)g * a.qpg + q0 + qq) * a.splits + split) * (DR + 2) + j] = v;
     }
 }
 
 // One block per (group, query): merge the splits (weights 2^(m_s - M)), divide by the sum, and apply the value
-// quantizer's rotation: out[j] = sum_k a[k] R[k][j] (the `@ self.rotation` of _quant.py:241).
-__global__ void decode_combine_kernel(const float* __restrict__ part, int splits, int d, const float* __restrict__ Rv,
-                                      float* __restrict__ out) {
-    extern __shared__ float avec[];
-    const int t = threadIdx.x;
-    const float* pr = part + (size_t)blockIdx.x * splits * (d + 2);
-    float M = -CUDART_INF_F;
-    for (int s = 0; s < splits; ++s) M = fmaxf(M, pr[(size_t)s * (d + 2) + d]);
-    float L = 0.f, av = 0.f;
-    for (int s = 0; s < splits; ++s) {
-        const float m = pr[(size_t)s * (d + 2) + d];
-        const float w = m == -CUDART_INF_F ? 0.f : exp2f(m - M);
-        L = fmaf(w, pr[(size_t)s * (d + 2) + d + 1], L);
-        if (t < d) av = fmaf(w, pr[(size_t)s * (d + 2) + t], av);
-    }
-    if (t < d) avec[t] = L > 0.f ? av / L : 0.f;   // no keys at all: zeros
-    __syncthreads();
-    if (t < d) {
-        float o = 0.f;
-        for (int k0 = 0; k0 < d; k0 += 32) {   // d is 64 or 128; 32 matrix elements in flight
-            float m[32];
+// quantizer's rotation: out[j] = sum_k a[k] R[k][j] (the `@ self.rotation` of _quant.py:241).  Latency is all there is to
+// it (it took 7.6 us with one thread per coordinate walking the splits): the matrix is fetched before the wait for the splits,
+// the splits and the sum over k are shared out among the threads.
+constexpr int kCombineThreads = 256;
+
+template <int DR>
+__global__ void __launch_bounds__(kCombineThreads)
+decode_combine_kernel(const float* __restrict__ part, int splits, const float* __restrict__ Rv, float* __restrict__ out) {
+    constexpr int kParts = kCombineThreads / DR, kSlices = kCombineThreads / (DR / 4), kLen = DR / kSlices;
+    __shared__ float weight[kMaxSplits], vec[kParts][DR], total[kSlices][DR];
+    __shared__ float inverse;
+    const int t = threadIdx.x, lane = t & 31;
+    const int j4 = t % (DR / 4) * 4, k0 = t / (DR / 4) * kLen;
+    float4 m[kLen];
 #pragma unroll
-            for (int u = 0; u < 32; ++u) m[u] = __ldg(Rv + (size_t)(k0 + u) * d + t);
+    for (int u = 0; u < kLen; ++u) m[u] = __ldg(reinterpret_cast<const float4*>(Rv + (size_t)(k0 + u) * DR + j4));
+    tq_grid_wait();
+    const float* pr = part + (size_t)blockIdx.x * splits * (DR + 2);
+    const int c = t % DR, slice = t / DR;
+    constexpr int kAhead = 8;       // accumulators in flight, fetched before the weights are known
+    float x[kAhead];
 #pragma unroll
-            for (int u = 0; u < 32; ++u) o = fmaf(avec[k0 + u], m[u], o);
+    for (int u = 0; u < kAhead; ++u) x[u] = slice + u * kParts < splits ? pr[(size_t)(slice + u * kParts) * (DR + 2) + c] : 0.f;
+    if (t < 32) {
+        float ms[kMaxSplits / 32], ls[kMaxSplits / 32], top = -CUDART_INF_F, sum = 0.f;
+#pragma unroll
+        for (int u = 0; u < kMaxSplits / 32; ++u) {
+            const int s = lane + 32 * u;
+            ms[u] = s < splits ? pr[(size_t)s * (DR + 2) + DR] : -CUDART_INF_F;
+            ls[u] = s < splits ? pr[(size_t)s * (DR + 2) + DR + 1] : 0.f;
+            top = fmaxf(top, ms[u]);
         }
-        out[(size_t)blockIdx.x * d + t] = o;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+#pragma unroll
+        for (int u = 0; u < kMaxSplits / 32; ++u) {
+            const float w = ms[u] == -CUDART_INF_F ? 0.f : exp2f(ms[u] - top);
+            weight[lane + 32 * u] = w;
+            sum = fmaf(w, ls[u], sum);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (lane == 0) inverse = sum > 0.f ? 1.f / sum : 0.f;     // no keys at all: zeros
+    }
+    __syncthreads();
+    float v = 0.f;
+    for (int s0 = slice; s0 < splits; s0 += kAhead * kParts) {
+        float next[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int s = s0 + (u + kAhead) * kParts;
+            next[u] = s < splits ? pr[(size_t)s * (DR + 2) + c] : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int s = s0 + u * kParts;
+            if (s < splits && weight[s] != 0.f) v = fmaf(weight[s], x[u], v);
+            x[u] = next[u];
+        }
+    }
+    vec[slice][c] = v;
+    __syncthreads();
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < kLen; ++u) {
+        float a = vec[0][k0 + u];
+#pragma unroll
+        for (int i = 1; i < kParts; ++i) a += vec[i][k0 + u];
+        a *= inverse;
+        o.x = fmaf(a, m[u].x, o.x); o.y = fmaf(a, m[u].y, o.y); o.z = fmaf(a, m[u].z, o.z); o.w = fmaf(a, m[u].w, o.w);
+    }
+    *reinterpret_cast<float4*>(&total[t / (DR / 4)][j4]) = o;
+    __syncthreads();
+    if (t < DR) {
+        float r = 0.f;
+#pragma unroll
+        for (int i = 0; i < kSlices; ++i) r += total[i][t];
+        out[(size_t)blockIdx.x * DR + t] = r;
     }
 }
 
-int queries_per_pass(int kbits, int qpg) { return qpg == 1 ? 1 : (kbits <= 3 ? 4 : 2); }
+// Up to four queries share a pass with their hi and lo parts as the eight columns of the operand; more take eight per pass.
+int queries_per_pass(int qpg) { return qpg <= 4 ? 4 : 8; }
 
-// One block is resident per SM, so blocks run in waves of `sms`.  Among the split counts that fill 1..4 waves,
-// take the one with the fewest tile times per SM (a block's set-up counted as one tile).
+// One block is resident per SM (its registers), so blocks run in waves of `sms`.  Among the split counts that fill 1..4 waves,
+// take the one with the fewest rounds of its warps per SM (a block's set-up counted as four rounds).
 int splits_for(int sms, int groups, int passes, int64_t keys_per_group) {
     const int64_t tiles = (keys_per_group + kTile - 1) / kTile;
     const int64_t gq = (int64_t)groups * passes;
-    if (tiles <= 1 || gq <= 0) return 1;
+    if (tiles <= kWarps || gq <= 0) return 1;
     int64_t best = 1, best_cost = -1;
     for (int w = 1; w <= 4; ++w) {
         int64_t s = (int64_t)sms * w / gq;
         if (s < 1) s = 1;
-        if (s > tiles) s = tiles;
+        if (s > (tiles + kWarps - 1) / kWarps) s = (tiles + kWarps - 1) / kWarps;
         if (s > kMaxSplits) s = kMaxSplits;
         const int64_t waves = (gq * s + sms - 1) / sms;
-        const int64_t cost = waves * ((tiles + s - 1) / s + 1);
+        const int64_t cost = waves * (((tiles + s - 1) / s + kWarps - 1) / kWarps + 4);
         if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = s; }
     }
     return (int)best;
 }
 
-template <int KB, int DR, int QP>
-int launch_partial(const tq_plan* kp, DecodeArgs a, int groups, int passes, cudaStream_t st) {
-    const size_t fixed = decode_smem_floats<KB, DR, QP>() * 4, vtile = (size_t)kTile * a.vwords * 4;
-    a.vbufs = fixed + 2 * vtile <= 227 * 1024 ? 2 : 1;
-    const size_t sm = fixed + a.vbufs * vtile;
-    const dim3 grid((unsigned)a.splits, (unsigned)passes, (unsigned)groups);
-    if (a.vbits == 3) {
-        TQ_GRANT_SMEM((decode_partial_kernel<KB, DR, QP, true>), sm, kp->device);
-        decode_partial_kernel<KB, DR, QP, true><<<grid, kThreads, sm, st>>>(kp->dev, a); tq_count_launch();
-    } else {
-        TQ_GRANT_SMEM((decode_partial_kernel<KB, DR, QP, false>), sm, kp->device);
-        decode_partial_kernel<KB, DR, QP, false><<<grid, kThreads, sm, st>>>(kp->dev, a); tq_count_launch();
-    }
+template <int KB, int VB, int DR, int NQ>
+int launch_partial(const tq_plan* kp, const DecodeArgs& a, int groups, int passes, cudaStream_t st) {
+    using P = Plan<KB, VB, DR, NQ>;
+    TQ_GRANT_SMEM((decode_partial_kernel<KB, VB, DR, NQ>), P::total, kp->device);
+    decode_partial_kernel<KB, VB, DR, NQ><<<dim3((unsigned)a.splits, (unsigned)passes, (unsigned)groups), kThreads, P::total, st>>>(kp->dev, a);
+    tq_count_launch();
     TQ_CUDA_TRY(cudaGetLastError());
     return TQ_OK;
 }
 
-template <int KB, int DR>
-int launch_partial_qp(const tq_plan* kp, const DecodeArgs& a, int groups, int passes, int qp, cudaStream_t st) {
-    if (qp == 1) return launch_partial<KB, DR, 1>(kp, a, groups, passes, st);
-    if constexpr (KB <= 3) return launch_partial<KB, DR, 4>(kp, a, groups, passes, st);
-    else return launch_partial<KB, DR, 2>(kp, a, groups, passes, st);
+template <int KB, int VB>
+int launch_partial_dq(const tq_plan* kp, const DecodeArgs& a, int groups, int passes, int qp, cudaStream_t st) {
+    if (kp->dev.d == 64) return qp == 4 ? launch_partial<KB, VB, 64, 4>(kp, a, groups, passes, st) : launch_partial<KB, VB, 64, 8>(kp, a, groups, passes, st);
+    return qp == 4 ? launch_partial<KB, VB, 128, 4>(kp, a, groups, passes, st) : launch_partial<KB, VB, 128, 8>(kp, a, groups, passes, st);
+}
+
+template <int KB>
+int launch_partial_v(const tq_plan* kp, int vbits, const DecodeArgs& a, int groups, int passes, int qp, cudaStream_t st) {
+    switch (vbits) {
+        case 1: return launch_partial_dq<KB, 1>(kp, a, groups, passes, qp, st);
+        case 2: return launch_partial_dq<KB, 2>(kp, a, groups, passes, qp, st);
+        case 3: return launch_partial_dq<KB, 3>(kp, a, groups, passes, qp, st);
+        default: return launch_partial_dq<KB, 4>(kp, a, groups, passes, qp, st);
+    }
 }
 
 }  // namespace
@@ -527,7 +765,7 @@ bool tq_decode_attention_supported(const tq_plan* kp, const tq_plan* vp) {
 }
 
 int64_t tq_decode_attention_scratch(const tq_plan* kp, int groups, int qpg, int64_t keys_per_group) {
-    const int qp = queries_per_pass(kp->dev.bits, qpg);
+    const int qp = queries_per_pass(qpg);
     const int passes = (qpg + qp - 1) / qp;
     const int splits = splits_for(tq_sm_count(kp->device), groups, passes, keys_per_group);
     return (int64_t)groups * qpg * splits * (kp->dev.d + 2) * (int64_t)sizeof(float);
@@ -540,12 +778,11 @@ int tq_launch_decode_attention(const tq_plan* kp, const tq_plan* vp, const float
                                cudaStream_t st) {
     TqRange range("tq.decode_attention");
     const int d = kp->dev.d, kb = kp->dev.bits;
-    const int qp = queries_per_pass(kb, qpg);
+    const int qp = queries_per_pass(qpg);
     const int passes = (qpg + qp - 1) / qp;
     DecodeArgs a{};
     a.q = q; a.kcodes = kcodes; a.ksigns = ksigns; a.krnorms = krnorms; a.knorms = knorms;
     a.vcodes = vcodes; a.vnorms = vnorms; a.vcodebook = vp->dev.codebook;
-    a.vbits = vp->dev.bits; a.vwords = vp->dev.code_words;
     a.qpg = qpg; a.keys_per_group = keys_per_group; a.group_rows = group_rows; a.length = length;
     a.scale_log2e = scale * 1.4426950408889634f;
     a.splits = splits_for(tq_sm_count(kp->device), groups, passes, keys_per_group);
@@ -554,15 +791,18 @@ int tq_launch_decode_attention(const tq_plan* kp, const tq_plan* vp, const float
     if (!scratch || scratch_bytes < need)
         return tq_fail(TQ_ERR_SCRATCH_TOO_SMALL, "decode attention scratch: need %zu bytes, got %zu", need, scratch_bytes);
     int r = TQ_ERR_UNSUPPORTED;
-#define TQ_DEC(B)                                                                                     \
-    case B:                                                                                           \
-        r = d == 64 ? launch_partial_qp<B, 64>(kp, a, groups, passes, qp, st)                          \
-                    : launch_partial_qp<B, 128>(kp, a, groups, passes, qp, st);                        \
-        break;
-    switch (kb) { TQ_DEC(1) TQ_DEC(2) TQ_DEC(3) TQ_DEC(4) }
-#undef TQ_DEC
+    switch (kb) {
+        case 1: r = launch_partial_v<1>(kp, vp->dev.bits, a, groups, passes, qp, st); break;
+        case 2: r = launch_partial_v<2>(kp, vp->dev.bits, a, groups, passes, qp, st); break;
+        case 3: r = launch_partial_v<3>(kp, vp->dev.bits, a, groups, passes, qp, st); break;
+        case 4: r = launch_partial_v<4>(kp, vp->dev.bits, a, groups, passes, qp, st); break;
+    }
     if (r != TQ_OK) return r;
-    decode_combine_kernel<<<(unsigned)(groups * qpg), (d + 31) & ~31, d * sizeof(float), st>>>(a.part, a.splits, d, vp->dev.R, out); tq_count_launch();
-    TQ_CUDA_TRY(cudaGetLastError());
+    if (d == 64)
+        TQ_CUDA_TRY(tq_launch_dependent(decode_combine_kernel<64>, dim3((unsigned)(groups * qpg)), dim3(kCombineThreads), 0, st,
+                                        (const float*)a.part, a.splits, vp->dev.R, out));
+    else
+        TQ_CUDA_TRY(tq_launch_dependent(decode_combine_kernel<128>, dim3((unsigned)(groups * qpg)), dim3(kCombineThreads), 0, st,
+                                        (const float*)a.part, a.splits, vp->dev.R, out));
     return TQ_OK;
 }
