@@ -50,7 +50,7 @@ extern "C" {
 #define TQ_PATH_EXACT 1   /* float32 kernels that accumulate in the reference's order */
 #define TQ_PATH_TENSOR 2  /* tensor-core kernels; TQ_ERR_UNSUPPORTED if (d, bits) has none */
 
-/* Element types of vectors handed to tq_kv_append. */
+/* Element types of vectors handed to tq_kv_append and tq_kv_prefill. */
 #define TQ_F32 0
 #define TQ_BF16 1
 #define TQ_F16 2
@@ -216,6 +216,16 @@ int tq_prod_append(const tq_plan* plan, const float* x, int groups, int tokens, 
 int tq_kv_append(const tq_plan* kplan, const tq_plan* vplan, const void* keys, const void* values, int dtype, int groups,
                  int tokens, void* k_codes, void* k_signs, float* k_residual_norms, float* k_norms, void* v_codes,
                  float* v_norms, int64_t capacity, int64_t* length, int advance, void* stream);
+
+/*
+ * Many tokens of a key/value cache: as tq_kv_append, through the bulk quantizers (scratch as for tq_*_quantize).  The rows go
+ * behind the `offset` rows that the host knows of; `*length` (device memory) is raised by `tokens` on the stream and not read.
+ */
+int64_t tq_kv_prefill_scratch_bytes(const tq_plan* kplan, const tq_plan* vplan, int64_t rows);
+int tq_kv_prefill(const tq_plan* kplan, const tq_plan* vplan, const void* keys, const void* values, int dtype, int groups,
+                  int tokens, void* k_codes, void* k_signs, float* k_residual_norms, float* k_norms, void* v_codes,
+                  float* v_norms, int64_t capacity, int64_t offset, int64_t* length, void* scratch, size_t scratch_bytes,
+                  void* stream);
 
 /*
  * Decode attention over a quantized key/value cache, without writing scores or dequantized values:

@@ -52,6 +52,9 @@ SIGNATURES = {
                                c_void_p, c_int, c_void_p]),
     "tq_kv_append": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
                              c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_int, c_void_p]),
+    "tq_kv_prefill_scratch_bytes": (c_int64, [c_void_p, c_void_p, c_int64]),
+    "tq_kv_prefill": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
+                              c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_size_t, c_void_p]),
     "tq_decode_attention_scratch_bytes": (c_int64, [c_void_p, c_int, c_int, c_int64]),
     "tq_decode_attention": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                     c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_float, c_void_p, c_void_p, c_size_t,

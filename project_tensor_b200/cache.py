@@ -29,7 +29,7 @@ class PackedKeyCache:
     """Packed TurboQuantProd keys of ``groups`` sequences, ``capacity`` rows each, all of one length."""
 
     #: appends of at most this many rows go through the one-launch append kernel; larger ones (prefill) through
-    #: the bulk quantizer and a copy of the packed rows into place
+    #: the bulk quantizers, which write the packed rows into place
     SMALL_APPEND_ROWS = 4096
 
     def __init__(self, quantizer: "_tq.TurboQuantProd", groups: int, capacity: int, device: Any = None):
@@ -93,28 +93,24 @@ class PackedKeyCache:
         """Write ``tokens`` staged keys per group behind the present rows, and the same number of values when ``values``
         is (staged values, their plans, their codes, their norms); the length advances once."""
         lo, hi = self._length, self._length + tokens
-        if self.groups * tokens <= self.SMALL_APPEND_ROWS:
-            dev = self.device
-            vstaged, vplans, vcodes, vnorms = values or (None, None, None, None)
-            _native.check(_native.load().tq_kv_append(
-                self._plans.handle(dev), vplans.handle(dev) if values else None, staged.tensor.data_ptr(),
-                vstaged.tensor.data_ptr() if values else None, _tq._dtype_code(staged.tensor), self.groups, tokens,
-                self.codes.data_ptr(), self.signs.data_ptr(), self.residual_norms.data_ptr(), self.norms.data_ptr(),
-                vcodes.data_ptr() if values else None, vnorms.data_ptr() if values else None, self.capacity,
-                self.length_device.data_ptr(), 1, _tq._stream_ptr(dev)))
+        dev, lib = self.device, _native.load()
+        vstaged, vplans, vcodes, vnorms = values or (None, None, None, None)
+        rows = self.groups * tokens
+        bulk = rows > self.SMALL_APPEND_ROWS
+        if bulk and self.quantizer.dimension == 256:      # (its bulk kernel reads float32 only)
+            staged, vstaged = _widen(staged), _widen(vstaged) if values else None
+        kh, vh = self._plans.handle(dev), vplans.handle(dev) if values else None
+        args = (kh, vh, staged.tensor.data_ptr(), vstaged.tensor.data_ptr() if values else None,
+                _tq._dtype_code(staged.tensor), self.groups, tokens, self.codes.data_ptr(), self.signs.data_ptr(),
+                self.residual_norms.data_ptr(), self.norms.data_ptr(), vcodes.data_ptr() if values else None,
+                vnorms.data_ptr() if values else None, self.capacity)
+        if bulk:
+            need = lib.tq_kv_prefill_scratch_bytes(kh, vh, rows)
+            scratch = self.codes.new_empty((need,))
+            _native.check(lib.tq_kv_prefill(*args, lo, self.length_device.data_ptr(), scratch.data_ptr(), need,
+                                            _tq._stream_ptr(dev)))
         else:
-            g, c = self.groups, self.capacity
-            if values:
-                vstaged, vplans, vcodes, vnorms = values
-                pk = self.quantizer.mse._quantize_staged(_widen(vstaged), vplans, False)
-                vcodes.view(g, c, -1)[:, lo:hi] = pk.codes.view(g, tokens, -1)
-                vnorms.view(g, c)[:, lo:hi] = pk.norms.view(g, tokens)
-            pk = self.quantizer.mse._quantize_staged(_widen(staged), self._plans, True)
-            self.codes.view(g, c, -1)[:, lo:hi] = pk.codes.view(g, tokens, -1)
-            self.signs.view(g, c, -1)[:, lo:hi] = pk.signs.view(g, tokens, -1)
-            self.norms.view(g, c)[:, lo:hi] = pk.norms.view(g, tokens)
-            self.residual_norms.view(g, c)[:, lo:hi] = pk.residual_norms.view(g, tokens)
-            self.length_device.add_(tokens)
+            _native.check(lib.tq_kv_append(*args, self.length_device.data_ptr(), 1, _tq._stream_ptr(dev)))
         self._length = hi
 
     # ---- scoring --------------------------------------------------------------------------------

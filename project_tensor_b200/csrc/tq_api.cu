@@ -279,6 +279,21 @@ int64_t tq_topk_scratch_bytes(const tq_plan* p, int groups, int q_per_group, int
     return tq_score_topk_scratch(p, groups, q_per_group, keys_per_group, topk);
 }
 
+// Up to 32 rows per SM the reference-order kernel alone is faster than the tensor-core kernel with its second stage
+// (four operations on the stream): TurboQuantProd, 2,048 rows: d = 64 10 against 28 us, d = 128 18 against 38, d = 256
+// 43 against 84; 8,192 rows: 23 / 34, 44 / 45, 121 / 84.
+static bool few_rows(const tq_plan* p, int64_t n) { return p->path == TQ_PATH_AUTO && n <= 32 * (int64_t)tq_sm_count(p->device); }
+
+// The lists of one call in the caller's scratch, behind its header.
+static unsigned char* place_lists(TqRecheck* l, TqRecheckHeader* hdr, unsigned char* at, int64_t n) {
+    l->hdr = hdr;
+    l->code_cap = tq_recheck_code_cap(n);
+    l->row_cap = tq_recheck_row_cap(n);
+    l->code_entries = reinterpret_cast<unsigned long long*>(at);
+    l->row_entries = reinterpret_cast<unsigned int*>(at + 8 * (size_t)l->code_cap);
+    return at + 8 * (size_t)l->code_cap + (4 * (size_t)l->row_cap + 15) / 16 * 16;
+}
+
 static int quantize_common(const tq_plan* p, bool prod, const float* x, int64_t n, void* codes, void* signs,
                            float* rnorms, float* norms, void* scratch, size_t scratch_bytes, void* stream) {
     TQ_TRY(check_plan(p, prod));
@@ -295,37 +310,27 @@ static int quantize_common(const tq_plan* p, bool prod, const float* x, int64_t 
     if (!scope.ok) return tq_fail(TQ_ERR_CUDA, "cannot select device %d", p->device);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int err = TQ_OK;
-    // Up to 32 rows per SM the reference-order kernel alone is faster than the tensor-core kernel with its second stage
-    // (four operations on the stream): TurboQuantProd, 2,048 rows: d = 64 10 against 28 us, d = 128 18 against 38, d = 256
-    // 43 against 84; 8,192 rows: 23 / 34, 44 / 45, 121 / 84.
-    const bool few = p->path == TQ_PATH_AUTO && n <= 32 * (int64_t)tq_sm_count(p->device);
-    if (!few && use_tensor(p, &err)) {
+    const TqQuantOut out{static_cast<uint32_t*>(codes), static_cast<uint32_t*>(signs), rnorms, norms, TqRowMap{}};
+    if (!few_rows(p, n) && use_tensor(p, &err)) {
         const int64_t need = tq_quantize_scratch_bytes(p, n);
         if (!scratch || (int64_t)scratch_bytes < need)
             return tq_fail(TQ_ERR_SCRATCH_TOO_SMALL, "quantize scratch: need %lld bytes, got %zu", (long long)need, scratch_bytes);
         TQ_TRY(check_ptr(scratch, "scratch"));
-        TqRecheck lists;
         unsigned char* sc = static_cast<unsigned char*>(scratch);
-        lists.hdr = reinterpret_cast<TqRecheckHeader*>(sc);
-        lists.code_cap = tq_recheck_code_cap(n);
-        lists.row_cap = tq_recheck_row_cap(n);
-        lists.code_entries = reinterpret_cast<unsigned long long*>(sc + sizeof(TqRecheckHeader));
-        lists.row_entries = reinterpret_cast<unsigned int*>(sc + sizeof(TqRecheckHeader) + 8 * (size_t)lists.code_cap);
-        TQ_CUDA_TRY(cudaMemsetAsync(lists.hdr, 0, sizeof(TqRecheckHeader), st));
-        TQ_TRY(tq_launch_tensor_quantize(p, prod, x, n, static_cast<uint32_t*>(codes), static_cast<uint32_t*>(signs),
-                                         rnorms, norms, &lists, st));
+        TqSecondStage second{p, prod, x, TQ_F32, n, out, {}};
+        place_lists(&second.lists, reinterpret_cast<TqRecheckHeader*>(sc), sc + sizeof(TqRecheckHeader), n);
+        TQ_CUDA_TRY(cudaMemsetAsync(second.lists.hdr, 0, sizeof(TqRecheckHeader), st));
+        TQ_TRY(tq_launch_tensor_quantize(p, prod, x, TQ_F32, n, out, &second.lists, st));
         tq_timer_mark(p, 2, 0, st);
-        TQ_TRY(tq_launch_exact_code_check(p, prod, x, n, static_cast<uint32_t*>(codes), &lists, st));
+        TQ_TRY(tq_launch_exact_code_check(&second, nullptr, st));
         tq_timer_mark(p, 2, 1, st);
         tq_timer_mark(p, 3, 0, st);
-        const int rc = tq_launch_exact_quantize(p, prod, x, TQ_F32, n, static_cast<uint32_t*>(codes), static_cast<uint32_t*>(signs),
-                                                rnorms, norms, &lists, p->counters, st);
+        const int rc = tq_launch_exact_listed(&second, nullptr, 0, st);
         tq_timer_mark(p, 3, 1, st);
         return rc;
     }
     if (err != TQ_OK) return err;
-    return tq_launch_exact_quantize(p, prod, x, TQ_F32, n, static_cast<uint32_t*>(codes), static_cast<uint32_t*>(signs), rnorms,
-                                    norms, nullptr, nullptr, st);
+    return tq_launch_exact_quantize(p, prod, x, TQ_F32, n, out.codes, out.signs, rnorms, norms, st);
 }
 
 int tq_mse_quantize(const tq_plan* p, const float* x, int64_t n, void* codes, float* norms, void* scratch,
@@ -346,12 +351,9 @@ static int check_encoding(const void* codes, const void* signs, const float* rn,
     return TQ_OK;
 }
 
-// Append path: groups * tokens new vectors go behind the `*length` rows every group of a cache already holds.
-// One launch of the reference-order kernel (any d, any bits; the batches are small: one or a few tokens per
-// sequence and head), no scratch, no host knowledge of the length.
-static int append_common(const tq_plan* kp, const tq_plan* vp, const void* keys, const void* values, int dtype, int groups, int tokens,
-                         void* kcodes, void* ksigns, float* krnorms, float* knorms, void* vcodes, float* vnorms,
-                         int64_t capacity, int64_t* length, int advance, void* stream) {
+static int check_append(const tq_plan* kp, const tq_plan* vp, const void* keys, const void* values, int dtype, int groups, int tokens,
+                        const void* kcodes, const void* ksigns, const float* krnorms, const float* knorms, const void* vcodes,
+                        const float* vnorms, int64_t capacity, const int64_t* length) {
     if (!kp && !vp) return tq_fail(TQ_ERR_INVALID_ARGUMENT, "plan is null");
     if (kp) TQ_TRY(check_plan(kp, true));
     if (kp && vp && kp->device != vp->device) return tq_fail(TQ_ERR_INVALID_ARGUMENT, "key and value plans live on different devices");
@@ -372,8 +374,19 @@ static int append_common(const tq_plan* kp, const tq_plan* vp, const void* keys,
         TQ_TRY(check_ptr(vcodes, "value codes"));
         TQ_TRY(check_ptr(vnorms, "value norms"));
     }
+    return TQ_OK;
+}
+
+// Append path: groups * tokens new vectors go behind the `*length` rows every group of a cache already holds.
+// One launch of the reference-order kernel (any d, any bits; the batches are small: one or a few tokens per
+// sequence and head), no scratch, no host knowledge of the length.
+static int append_common(const tq_plan* kp, const tq_plan* vp, const void* keys, const void* values, int dtype, int groups, int tokens,
+                         void* kcodes, void* ksigns, float* krnorms, float* knorms, void* vcodes, float* vnorms,
+                         int64_t capacity, int64_t* length, int advance, void* stream) {
+    TQ_TRY(check_append(kp, vp, keys, values, dtype, groups, tokens, kcodes, ksigns, krnorms, knorms, vcodes, vnorms, capacity, length));
+    if (groups == 0 || tokens == 0) return TQ_OK;
     DeviceScope scope((kp ? kp : vp)->device);
-    const TqRowMap map{tokens, capacity, length};
+    const TqRowMap map{tokens, capacity, length, 0, nullptr};
     return tq_launch_append(kp, keys, static_cast<uint32_t*>(kcodes), static_cast<uint32_t*>(ksigns), krnorms, knorms, vp, values,
                             static_cast<uint32_t*>(vcodes), vnorms, dtype, (int64_t)groups * tokens, map, advance,
                             static_cast<cudaStream_t>(stream));
@@ -396,6 +409,62 @@ int tq_kv_append(const tq_plan* kplan, const tq_plan* vplan, const void* keys, c
                  int64_t capacity, int64_t* length, int advance, void* stream) {
     return append_common(kplan, vplan, keys, values, dtype, groups, tokens, k_codes, k_signs, k_residual_norms, k_norms, v_codes,
                          v_norms, capacity, length, advance, stream);
+}
+
+int64_t tq_kv_prefill_scratch_bytes(const tq_plan* kp, const tq_plan* vp, int64_t rows) {
+    if ((!kp && !vp) || rows < 0) return 0;
+    return tq_quantize_scratch_bytes(kp ? kp : vp, rows) * (kp && vp ? 2 : 1) + 64;
+}
+
+// Many tokens per sequence: the bulk quantizers, reading rows of any element type and writing straight into the cache; the
+// keys' and the values' second stages share their launches.
+int tq_kv_prefill(const tq_plan* kp, const tq_plan* vp, const void* keys, const void* values, int dtype, int groups, int tokens,
+                  void* k_codes, void* k_signs, float* k_residual_norms, float* k_norms, void* v_codes, float* v_norms,
+                  int64_t capacity, int64_t offset, int64_t* length, void* scratch, size_t scratch_bytes, void* stream) {
+    TQ_TRY(check_append(kp, vp, keys, values, dtype, groups, tokens, k_codes, k_signs, k_residual_norms, k_norms, v_codes, v_norms,
+                        capacity, length));
+    if (offset < 0 || offset + tokens > capacity)
+        return tq_fail(TQ_ERR_INVALID_ARGUMENT, "rows %lld + %d outside the capacity %lld", (long long)offset, tokens, (long long)capacity);
+    if (groups == 0 || tokens == 0) return TQ_OK;
+    const int64_t rows = (int64_t)groups * tokens;
+    DeviceScope scope((kp ? kp : vp)->device);
+    if (!scope.ok) return tq_fail(TQ_ERR_CUDA, "cannot select device %d", (kp ? kp : vp)->device);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const TqRowMap map{tokens, capacity, nullptr, offset, length};
+    TqSecondStage jobs[2], tensor[2];
+    int njobs = 0, ntensor = 0;
+    if (kp) jobs[njobs++] = TqSecondStage{kp, true, keys, dtype, rows, {static_cast<uint32_t*>(k_codes), static_cast<uint32_t*>(k_signs), k_residual_norms, k_norms, map}, {}};
+    if (vp) jobs[njobs++] = TqSecondStage{vp, false, values, dtype, rows, {static_cast<uint32_t*>(v_codes), nullptr, nullptr, v_norms, map}, {}};
+    bool whole[2] = {false, false};      // jobs for the reference-order kernel alone
+    for (int i = 0; i < njobs; ++i) {
+        int err = TQ_OK;
+        const tq_plan* p = jobs[i].plan;
+        whole[i] = few_rows(p, rows) || !use_tensor(p, &err) || !tq_tensor_input_supported(p->dev.d, dtype);
+        if (err != TQ_OK) return err;
+        if (!whole[i]) tensor[ntensor++] = jobs[i];
+    }
+    if (ntensor) {
+        const int64_t need = tq_kv_prefill_scratch_bytes(kp, vp, rows);
+        if (!scratch || (int64_t)scratch_bytes < need)
+            return tq_fail(TQ_ERR_SCRATCH_TOO_SMALL, "prefill scratch: need %lld bytes, got %zu", (long long)need, scratch_bytes);
+        TQ_TRY(check_ptr(scratch, "scratch"));
+        TqRecheckHeader* hdr = static_cast<TqRecheckHeader*>(scratch);
+        unsigned char* at = reinterpret_cast<unsigned char*>(hdr + ntensor);
+        for (int i = 0; i < ntensor; ++i) at = place_lists(&tensor[i].lists, hdr + i, at, rows);
+        TQ_CUDA_TRY(cudaMemsetAsync(hdr, 0, ntensor * sizeof(TqRecheckHeader), st));
+    }
+    for (int i = 0; i < ntensor; ++i)
+        TQ_TRY(tq_launch_tensor_quantize(tensor[i].plan, tensor[i].prod, tensor[i].x, dtype, rows, tensor[i].out, &tensor[i].lists, st));
+    // the last launch raises the length
+    for (int i = 0, left = njobs - ntensor; i < njobs; ++i)
+        if (whole[i])
+            TQ_TRY(tq_launch_exact_mapped(jobs[i].plan, jobs[i].prod, jobs[i].x, dtype, rows, jobs[i].out, --left == 0 && !ntensor ? 2 : 0, st));
+    if (ntensor) {
+        const TqSecondStage* second = ntensor == 2 ? &tensor[1] : nullptr;
+        TQ_TRY(tq_launch_exact_code_check(&tensor[0], second, st));
+        TQ_TRY(tq_launch_exact_listed(&tensor[0], second, 2, st));
+    }
+    return TQ_OK;
 }
 
 int tq_mse_quantize_noalloc(const tq_plan* p, const float* x, int64_t n, void* codes, float* norms, void* stream) {

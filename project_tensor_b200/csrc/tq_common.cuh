@@ -43,10 +43,21 @@ struct TqRecheck {
 // Where the rows of a quantize call land when they are appended to a cache of `capacity` rows per group:
 // input row r is token r % tokens of group r / tokens and goes to row group * capacity + *length + token.
 // `length` lives on the device (one value for all groups), so a captured launch stays valid while the cache
-// grows.  tokens == 0: output row = input row.
+// grows; where it is null the rows go behind `base` instead, and `counter` is what a launch that is told to raises by `tokens`.
+// tokens == 0: output row = input row.
 struct TqRowMap {
     int64_t tokens, capacity;
     const int64_t* length;
+    int64_t base;
+    int64_t* counter;
+};
+// What a quantize call writes, and where.
+struct TqQuantOut {
+    uint32_t* codes;
+    uint32_t* signs;
+    float* rnorms;
+    float* norms;
+    TqRowMap map;
 };
 __host__ __device__ __forceinline__ unsigned int tq_recheck_code_cap(int64_t n) { return (unsigned int)(n / 2 + 4096); }
 __host__ __device__ __forceinline__ unsigned int tq_recheck_row_cap(int64_t n) { return (unsigned int)(n / 8 + 4096); }
@@ -161,17 +172,28 @@ __device__ __forceinline__ void tq_grid_wait() { asm volatile("griddepcontrol.wa
 __device__ __forceinline__ void tq_grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---- launchers implemented in the kernel files -----------------------------------------------
-// Exact (reference-order float32) kernels.  With `lists` null every row is computed; otherwise
-// first the listed coordinates are re-decided (tq_launch_exact_code_check), then the listed rows
-// are recomputed.
+// Exact (reference-order float32) kernels.
 int tq_launch_exact_quantize(const tq_plan* p, bool prod, const void* x, int xtype, int64_t n, uint32_t* codes,
-                             uint32_t* signs, float* rnorms, float* norms, const TqRecheck* lists,
-                             unsigned long long* redo_counter, cudaStream_t st);
+                             uint32_t* signs, float* rnorms, float* norms, cudaStream_t st);
 int tq_launch_append(const tq_plan* kp, const void* kx, uint32_t* kcodes, uint32_t* ksigns, float* krnorms, float* knorms,
                      const tq_plan* vp, const void* vx, uint32_t* vcodes, float* vnorms, int xtype, int64_t rows,
                      const TqRowMap& map, int advance, cudaStream_t st);
-int tq_launch_exact_code_check(const tq_plan* p, bool prod, const float* x, int64_t n, uint32_t* codes,
-                               const TqRecheck* lists, cudaStream_t st);
+// Second stage of the tensor-core quantizers for one call, or for the keys and the values of a cache: first the listed coordinates,
+// then the listed rows.
+struct TqSecondStage {
+    const tq_plan* plan;
+    bool prod;
+    const void* x;
+    int xtype;
+    int64_t n;
+    TqQuantOut out;
+    TqRecheck lists;
+};
+int tq_launch_exact_code_check(const TqSecondStage* a, const TqSecondStage* b, cudaStream_t st);
+int tq_launch_exact_listed(const TqSecondStage* a, const TqSecondStage* b, int advance, cudaStream_t st);
+// All rows of one call into the rows of a cache.
+int tq_launch_exact_mapped(const tq_plan* p, bool prod, const void* x, int xtype, int64_t n, const TqQuantOut& out, int advance,
+                           cudaStream_t st);
 int tq_launch_exact_dequantize(const tq_plan* p, bool prod, const uint32_t* codes, const uint32_t* signs,
                                const float* rnorms, const float* norms, int64_t n, float* out,
                                cudaStream_t st);
@@ -184,9 +206,9 @@ bool tq_tensor_supported(int d, int bits);
 bool tq_tensor_quantize_supported(int d, int bits, bool has_projection);
 int tq_tensor_plan_init(tq_plan* p, const float* rotation, const float* codebook, const float* projection);
 void tq_tensor_plan_free(tq_plan* p);
-int tq_launch_tensor_quantize(const tq_plan* p, bool prod, const float* x, int64_t n, uint32_t* codes,
-                              uint32_t* signs, float* rnorms, float* norms, const TqRecheck* lists,
-                              cudaStream_t st);
+bool tq_tensor_input_supported(int d, int xtype);
+int tq_launch_tensor_quantize(const tq_plan* p, bool prod, const void* x, int xtype, int64_t n, const TqQuantOut& out,
+                              const TqRecheck* lists, cudaStream_t st);
 
 // Tensor-core dequantize (d = 128): operand matrices per plan, then one launch per call.
 bool tq_dequant_tc_supported(int d, int bits_mse, bool prod);

@@ -211,7 +211,7 @@ struct RowSource {
     bool listed, mapped;
     __device__ __forceinline__ void open(const RowsJob& job, bool first_block) {
         mapped = job.map.tokens > 0;
-        len0 = mapped ? (*reinterpret_cast<volatile const int64_t*>(job.map.length) & ((1ll << 40) - 1)) : 0;
+        len0 = !mapped ? 0 : !job.map.length ? job.map.base : (*reinterpret_cast<volatile const int64_t*>(job.map.length) & ((1ll << 40) - 1));
         const TqRecheckHeader* hdr = job.lists.hdr;
         // all rows, or the rows of the list (every row again if a list overflowed)
         listed = hdr != nullptr && hdr->overflow == 0;
@@ -231,8 +231,12 @@ struct RowSource {
 
 // The last block of a launch to get here raises the cache length.  Blocks count themselves in bits 40 and up of that very
 // word, which are zero again when the kernel ends, so a step needs neither a second launch nor a counter of its own.
-// (Every block has read the length before it counts itself.)
-__device__ __forceinline__ void advance_length(const RowsJob& job, int64_t len0) {
+// (Every block has read the length before it counts itself.)  advance == 2: nothing in the launch reads it; one block adds.
+__device__ __forceinline__ void advance_length(const RowsJob& job, int64_t len0, int advance) {
+    if (advance == 2) {
+        if (blockIdx.x == 0) *job.map.counter += job.map.tokens;
+        return;
+    }
     unsigned long long* len = reinterpret_cast<unsigned long long*>(const_cast<int64_t*>(job.map.length));
     const unsigned long long before = atomicAdd(len, 1ull << 40);
     if ((before >> 40) == gridDim.x - 1) {
@@ -340,7 +344,7 @@ exact_quantize_few_kernel(const __grid_constant__ RowsJob first, const __grid_co
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     if (advance) {
         __syncthreads();
-        if (t == 0) advance_length(job, rows.len0);
+        if (t == 0) advance_length(job, rows.len0, advance);
     }
 }
 
@@ -584,117 +588,105 @@ exact_quantize_tile_kernel(const __grid_constant__ RowsJob first, const __grid_c
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    if (advance && t == 0) advance_length(job, rows.len0);
+    if (advance && t == 0) advance_length(job, rows.len0, advance);
 }
 
-// Second stage of the tensor-core quantizers, part 1: one thread per listed (row, coordinate).
-// The coordinate's rotated value is recomputed exactly as the reference does (norm by pairwise sum,
-// IEEE division, one FMA per k, k ascending) and its code re-decided.  If the stored code differs it is
-// patched in place (MSE); for TurboQuantProd the residual of the whole row depends on it, so the
-// row goes to the row list instead.  A list holds some ten thousand entries per million rows and a dependent access
-// to global memory costs about a microsecond, so the kernel is as long as its chain of such accesses: header, entry,
-// then the whole row into registers (D / 4 loads of 16 bytes in flight at once) together with the first half of the
-// matrix row.  D is 64, 128 or 256 (the tensor-core geometries): the row sum is one block of NumPy's pairwise scheme
-// (eight interleaved sums) per 128 values.
-// Sum of squares of Q * 4 consecutive values as NumPy sums a block of its pairwise scheme (eight interleaved sums);
-// the values stay in xv.
-template <int Q>
-__device__ __forceinline__ float block_sumsq(const float4* __restrict__ xr, float4 (&xv)[Q]) {
-#pragma unroll
-    for (int i = 0; i < Q; ++i) xv[i] = xr[i];
-    float r8[8] = {__fmul_rn(xv[0].x, xv[0].x), __fmul_rn(xv[0].y, xv[0].y), __fmul_rn(xv[0].z, xv[0].z), __fmul_rn(xv[0].w, xv[0].w),
-                   __fmul_rn(xv[1].x, xv[1].x), __fmul_rn(xv[1].y, xv[1].y), __fmul_rn(xv[1].z, xv[1].z), __fmul_rn(xv[1].w, xv[1].w)};
-#pragma unroll
-    for (int i = 2; i < Q; i += 2) {
-        const float4 a = xv[i], b = xv[i + 1];
-        r8[0] = __fadd_rn(r8[0], __fmul_rn(a.x, a.x)); r8[1] = __fadd_rn(r8[1], __fmul_rn(a.y, a.y));
-        r8[2] = __fadd_rn(r8[2], __fmul_rn(a.z, a.z)); r8[3] = __fadd_rn(r8[3], __fmul_rn(a.w, a.w));
-        r8[4] = __fadd_rn(r8[4], __fmul_rn(b.x, b.x)); r8[5] = __fadd_rn(r8[5], __fmul_rn(b.y, b.y));
-        r8[6] = __fadd_rn(r8[6], __fmul_rn(b.z, b.z)); r8[7] = __fadd_rn(r8[7], __fmul_rn(b.w, b.w));
-    }
-    return __fadd_rn(__fadd_rn(__fadd_rn(r8[0], r8[1]), __fadd_rn(r8[2], r8[3])),
-                     __fadd_rn(__fadd_rn(r8[4], r8[5]), __fadd_rn(r8[6], r8[7])));
-}
-// acc += sum over the Q * 4 values in xv of (value / nrm) * matrix value, one FMA per value, in order; the matrix row
-// part comes in two batches of loads.
-template <int Q>
-__device__ __forceinline__ float block_chain(const float4 (&xv)[Q], const float4* __restrict__ rj, float nrm, bool ok, float acc) {
-    float4 rv[Q / 2];
-#pragma unroll
-    for (int i = 0; i < Q / 2; ++i) rv[i] = __ldg(rj + i);
-#pragma unroll
-    for (int i = 0; i < Q; ++i) {
-        if (i == Q / 2) {
-#pragma unroll
-            for (int u = 0; u < Q / 2; ++u) rv[u] = __ldg(rj + Q / 2 + u);
-        }
-        const float4 v = xv[i], m = rv[i % (Q / 2)];
-        acc = __fmaf_rn(ok ? __fdiv_rn(v.x, nrm) : 0.f, m.x, acc);
-        acc = __fmaf_rn(ok ? __fdiv_rn(v.y, nrm) : 0.f, m.y, acc);
-        acc = __fmaf_rn(ok ? __fdiv_rn(v.z, nrm) : 0.f, m.z, acc);
-        acc = __fmaf_rn(ok ? __fdiv_rn(v.w, nrm) : 0.f, m.w, acc);
-    }
-    return acc;
-}
+// Listed coordinates (those inside the guard band of the tensor-core kernel) re-decided in the reference's order: norm, division and
+// the rotated coordinate as one FMA chain.  A wrong code is corrected in place (TurboQuantMSE) or puts its row on the row list
+// (TurboQuantProd).  Work is small -- 20,000 entries of 1,048,576 rows -- and every dependent access to global memory costs
+// about a microsecond, so the kernel is as long as its chain of such accesses: header and entry, then row, matrix row and
+// boundaries together.  Eight lanes fetch an entry's rows, normalise and leave both in shared memory; then a
+// lane per entry runs the chain, 32 entries side by side.  (One lane per entry for everything, 128 divisions in a row:
+// 18 us for the entries of 1,048,576 rows, now 8.7; 12.6 and 5.7 for 65,536.)
+struct CheckJob {
+    TqDev p;
+    const void* x;
+    int xtype, prod;
+    int64_t n;
+    uint32_t* codes;
+    TqRecheck lists;
+    TqRowMap map;
+};
 
 template <int D>
-__global__ void __launch_bounds__(128)
-exact_code_check_kernel(TqDev p, bool prod, const float* __restrict__ x, int64_t n, uint32_t* __restrict__ codes,
-                        TqRecheck lists) {
-    // D = 256: two neighbouring lanes share an entry, each with one half of the row in its registers (the halves are
-    // also the two blocks of NumPy's pairwise sum for n = 256).  The chain runs over the first half in the even lane,
-    // then over the second half in the odd lane, which decides.
-    constexpr int LANES = D > 128 ? 2 : 1;                 // lanes per entry
-    constexpr int H = D / LANES, Q = H / 4;
-    const unsigned int t0 = blockIdx.x * blockDim.x + threadIdx.x;
-    const unsigned int e0 = t0 / LANES;
-    const int half = LANES == 2 ? (int)(threadIdx.x & 1u) : 0;
+__global__ void __launch_bounds__(256)
+exact_code_check_kernel(const __grid_constant__ CheckJob first, const __grid_constant__ CheckJob second, int blocks0) {
+    constexpr int E = D > 128 ? 16 : 32, kLanes = 256 / E, kStep = E / (32 / kLanes);      // entries per block; lanes per entry
+    constexpr int kStride = D + 1;                                                      // odd: a column is free of bank conflicts
+    __shared__ float vt[E * kStride], mt[E * kStride];
+    __shared__ float bnd[16];
+    __shared__ unsigned long long entry[E];      // ~0: none
+    __shared__ uint32_t stored[E];               // the code that stands in the packed row
+    const bool one = (int)blockIdx.x < blocks0;
+    const CheckJob& job = one ? first : second;
+    const TqDev& p = job.p;
+    const unsigned int block = one ? blockIdx.x : blockIdx.x - blocks0, nblocks = one ? blocks0 : gridDim.x - blocks0;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    // entries warp, warp + kStep, ... of the block: the lanes of different entries meet in different banks
+    const int e = warp + kStep * (lane / kLanes), l = lane & (kLanes - 1);
+    const TqRecheck& lists = job.lists;
     // asked for before the header is known to allow it (the list's capacity bounds the index)
-    unsigned long long ent = e0 < lists.code_cap ? lists.code_entries[e0] : 0ull;
+    unsigned int at = block * E + e;
+    unsigned long long ent = at < lists.code_cap ? lists.code_entries[at] : 0ull;
+    if (t < p.levels - 1) bnd[t] = __ldg(p.boundaries + t);      // (at most 15: the tensor-core kernels take up to 4 bits)
     if (lists.hdr->overflow) return;  // the row pass will redo everything
     const unsigned int count = min(lists.hdr->n_codes, lists.code_cap);
-    const unsigned int stride = gridDim.x * blockDim.x / LANES;
-    // both lanes of a pair run the same number of passes (their e is the same), so the shuffles below are whole-warp
-    for (unsigned int e = e0; e < ((count + 31u) & ~31u) + stride; e += stride) {
-        if (__all_sync(0xffffffffu, e >= count)) break;
-        const bool have = e < count;
-        if (e != e0 && have) ent = lists.code_entries[e];
+    for (unsigned int at0 = block * E; at0 < count; at0 += nblocks * E) {
+        const unsigned int mine = at0 + e;
+        if (mine != at && mine < count) ent = lists.code_entries[mine];
+        at = mine;
         const int64_t row = (int64_t)(ent >> 8);
         const int j = (int)(ent & 255u);
-        const bool valid = have && row < n && j < D;
-        const float4* xr = reinterpret_cast<const float4*>(x + (valid ? row : 0) * D) + half * Q;
-        const float4* rj = reinterpret_cast<const float4*>(p.R + (size_t)(valid ? j : 0) * D) + half * Q;
-        uint32_t* crow = codes + (valid ? row : 0) * p.code_words;
-        const uint32_t old = tq_get_code(crow, valid ? j : 0, p.bits);
-        float4 xv[Q];
-        float acc;
-        const float mine = block_sumsq<Q>(xr, xv);
-        if (LANES == 1) {
-            const float nrm = __fsqrt_rn(mine);
-            acc = block_chain<Q>(xv, rj, nrm, nrm > 0.f, 0.f);
-        } else {
-            const float other = __shfl_xor_sync(0xffffffffu, mine, 1);
-            const float nrm = __fsqrt_rn(half == 0 ? __fadd_rn(mine, other) : __fadd_rn(other, mine));   // first half + second half
-            const bool ok = nrm > 0.f;
-            const float first = block_chain<Q>(xv, rj, nrm, ok, 0.f);                 // meaningful in the even lane
-            const float carry = __shfl_xor_sync(0xffffffffu, first, 1);               // odd lane: the first half's sum
-            acc = block_chain<Q>(xv, rj, nrm, ok, carry);                             // meaningful in the odd lane
-            if (half == 0) continue;                                                  // the odd lane decides
+        const bool valid = mine < count && row < job.n && j < D;
+        float* v = vt + e * kStride;
+        float* m = mt + e * kStride;
+        auto packed_row = [&](int64_t r) {
+            return job.codes + (job.map.tokens > 0 ? r / job.map.tokens * job.map.capacity + job.map.base + r % job.map.tokens : r) * p.code_words;
+        };
+        if (l == 0) {
+            entry[e] = valid ? ent : ~0ull;
+            if (valid) stored[e] = tq_get_code(packed_row(row), j, p.bits);
         }
-        if (!valid) continue;
-        const uint32_t code = (uint32_t)count_below(p.boundaries, p.levels - 1, acc);
-        if (old == code) continue;
-        if (prod) {
-            const unsigned int pos = atomicAdd(&lists.hdr->n_rows, 1u);
-            if (pos < lists.row_cap) lists.row_entries[pos] = (unsigned int)row;
-            else lists.hdr->overflow = 1u;
+        if (l < 8) {
+            load_row(v, 1, D, l, job.x, job.xtype, valid ? row : -1);
+            if (kLanes == 8) load_row(m, 1, D, l, p.R, TQ_INPUT_F32, valid ? j : -1);
         } else {
-            const uint32_t delta = old ^ code;
-            const int bit = j * p.bits, w = bit >> 5, sh = bit & 31;
-            atomicXor(crow + w, delta << sh);
-            if (sh + p.bits > 32) atomicXor(crow + w + 1, delta >> (32 - sh));
+            load_row(m, 1, D, l - 8, p.R, TQ_INPUT_F32, valid ? j : -1);
         }
-        atomicAdd(&lists.hdr->pad[0], 1u);  // diagnostic: codes the exact arithmetic decided differently
+        __syncwarp();
+        const float nr = __fsqrt_rn(np_sumsq8<1>(v, D, l & 7));
+        __syncwarp();
+        if (l < 8) divide_row(v, 1, D, l, nr);
+        __syncthreads();
+        // lane i of the first warp takes the chain of entry i
+        if (warp == 0) {
+            if (lane < E && entry[lane] != ~0ull) {
+                const int64_t r = (int64_t)(entry[lane] >> 8);
+                const int c = (int)(entry[lane] & 255u);
+                const uint32_t old = stored[lane];
+                const float* ve = vt + lane * kStride;
+                const float* me = mt + lane * kStride;
+                float acc = 0.f;
+#pragma unroll 32
+                for (int k = 0; k < D; ++k) acc = __fmaf_rn(ve[k], me[k], acc);
+                const uint32_t code = (uint32_t)count_below(bnd, p.levels - 1, acc);
+                if (old != code) {
+                    if (job.prod) {
+                        const unsigned int pos = atomicAdd(&lists.hdr->n_rows, 1u);
+                        if (pos < lists.row_cap) lists.row_entries[pos] = (unsigned int)r;
+                        else lists.hdr->overflow = 1u;
+                    } else {
+                        uint32_t* crow = packed_row(r);
+                        const uint32_t delta = old ^ code;
+                        const int bit = c * p.bits, w = bit >> 5, sh = bit & 31;
+                        atomicXor(crow + w, delta << sh);
+                        if (sh + p.bits > 32) atomicXor(crow + w + 1, delta >> (32 - sh));
+                    }
+                    atomicAdd(&lists.hdr->pad[0], 1u);  // diagnostic: codes the exact arithmetic decided differently
+                }
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -819,17 +811,27 @@ int grid_for(int64_t work_items, int per_block) {
 
 }  // namespace
 
-int tq_launch_exact_code_check(const tq_plan* p, bool prod, const float* x, int64_t n, uint32_t* codes,
-                               const TqRecheck* lists, cudaStream_t st) {
+int tq_launch_exact_code_check(const TqSecondStage* a, const TqSecondStage* b, cudaStream_t st) {
     TqRange range("tq.quantize.recheck_coordinates");
-    if (n == 0) return TQ_OK;
-    // as many threads as a list of typical length has entries (about 1 in 50 rows of 128 coordinates at 4 bits, in
+    const int d = a->plan->dev.d;
+    const int64_t per_block = d > 128 ? 16 : 32, most = tq_sm_count(a->plan->device) * (int64_t)(b ? 3 : 6);
+    // as many blocks as a list of typical length has entries for (about 1 in 48 rows of 128 coordinates at 4 bits, in
     // proportion to the coordinates); longer lists take more passes
-    int64_t blocks = (n * p->dev.d / 128 / 48 * (p->dev.d > 128 ? 2 : 1) + 127) / 128;   // d = 256: two lanes per entry
-    blocks = blocks < 8 ? 8 : (blocks > 148 * 8 ? 148 * 8 : blocks);
-    if (p->dev.d == 128) exact_code_check_kernel<128><<<(int)blocks, 128, 0, st>>>(p->dev, prod, x, n, codes, *lists);
-    else if (p->dev.d == 64) exact_code_check_kernel<64><<<(int)blocks, 128, 0, st>>>(p->dev, prod, x, n, codes, *lists);
-    else if (p->dev.d == 256) exact_code_check_kernel<256><<<(int)blocks, 128, 0, st>>>(p->dev, prod, x, n, codes, *lists);
+    auto blocks = [&](const TqSecondStage* s) {
+        const int64_t w = (s->n * d / 128 / 48 + per_block - 1) / per_block;
+        return (int)(w < 4 ? 4 : w > most ? most : w);
+    };
+    auto job = [](const TqSecondStage* s) {
+        CheckJob j{};
+        j.p = s->plan->dev; j.x = s->x; j.xtype = s->xtype; j.prod = s->prod ? 1 : 0; j.n = s->n;
+        j.codes = s->out.codes; j.lists = s->lists; j.map = s->out.map;
+        return j;
+    };
+    const CheckJob first = job(a), second = b ? job(b) : first;
+    const int b0 = blocks(a), grid = b0 + (b ? blocks(b) : 0);
+    if (d == 128) exact_code_check_kernel<128><<<grid, 256, 0, st>>>(first, second, b0);
+    else if (d == 64) exact_code_check_kernel<64><<<grid, 256, 0, st>>>(first, second, b0);
+    else if (d == 256) exact_code_check_kernel<256><<<grid, 256, 0, st>>>(first, second, b0);
     else return tq_fail(TQ_ERR_UNSUPPORTED, "the coordinate re-check is written for d = 64, 128 and 256");
     tq_count_launch();
     TQ_CUDA_TRY(cudaGetLastError());
@@ -925,15 +927,32 @@ RowsJob rows_job(const tq_plan* p, bool prod, const void* x, int xtype, int64_t 
 }  // namespace
 
 int tq_launch_exact_quantize(const tq_plan* p, bool prod, const void* x, int xtype, int64_t n, uint32_t* codes,
-                             uint32_t* signs, float* rnorms, float* norms, const TqRecheck* lists,
-                             unsigned long long* redo_counter, cudaStream_t st) {
+                             uint32_t* signs, float* rnorms, float* norms, cudaStream_t st) {
     TqRange range("tq.quantize.exact_rows");
     if (n == 0) return TQ_OK;
-    const RowsJob job = rows_job(p, prod, x, xtype, n, codes, signs, rnorms, norms, lists, redo_counter, nullptr);
+    const RowsJob job = rows_job(p, prod, x, xtype, n, codes, signs, rnorms, norms, nullptr, nullptr, nullptr);
+    return launch_rows(job, nullptr, n, p->device, 0, st);
+}
+
+int tq_launch_exact_mapped(const tq_plan* p, bool prod, const void* x, int xtype, int64_t n, const TqQuantOut& out, int advance,
+                           cudaStream_t st) {
+    TqRange range("tq.quantize.exact_rows");
+    const RowsJob job = rows_job(p, prod, x, xtype, n, out.codes, out.signs, out.rnorms, out.norms, nullptr, nullptr, &out.map);
+    return launch_rows(job, nullptr, n, p->device, advance, st);
+}
+
+int tq_launch_exact_listed(const TqSecondStage* a, const TqSecondStage* b, int advance, cudaStream_t st) {
+    TqRange range("tq.quantize.exact_rows");
+    auto job = [](const TqSecondStage* s) {
+        return rows_job(s->plan, s->prod, s->x, s->xtype, s->n, s->out.codes, s->out.signs, s->out.rnorms, s->out.norms, &s->lists,
+                        s->plan->counters, &s->out.map);
+    };
     // A listed pass does not know its size on the host.  About one row in 450 of a TurboQuantProd call at d = 128 is listed
     // (the coordinate re-check and the sign guard), hardly any of a TurboQuantMSE call; the blocks stride on where it is more.
-    const int64_t rows = !lists ? n : prod ? n * p->dev.d / 128 / 384 + 1 : n / 65536 + 1;
-    return launch_rows(job, nullptr, rows, p->device, 0, st);
+    auto rows = [](const TqSecondStage* s) { return s->prod ? s->n * s->plan->dev.d / 128 / 384 + 1 : s->n / 65536 + 1; };
+    const RowsJob first = job(a), second = b ? job(b) : first;
+    const int64_t ra = rows(a), rb = b ? rows(b) : 0;
+    return launch_rows(first, b ? &second : nullptr, ra > rb ? ra : rb, a->plan->device, advance, st);
 }
 
 // One step of a cache: the keys of `kp` (TurboQuantProd), the values of `vp` (TurboQuantMSE), or both (either plan may be

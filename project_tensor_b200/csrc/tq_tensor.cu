@@ -73,6 +73,8 @@ struct TensorArgs {
     uint32_t* signs;
     float* norms;
     float* rnorms;
+    int bf16;                    // 16-bit rows: 1 bf16, 0 fp16
+    uint32_t tokens, capacity, base;   // tokens > 0: rows of a cache (TqRowMap)
     TqRecheck lists;
     unsigned long long* status;  // [0]: set to a non-zero code when a wait timed out
     int wait_kcycles;            // limit of one bounded wait, in units of 1024 cycles
@@ -81,13 +83,24 @@ struct TensorArgs {
 #endif
 };
 
+// Row of the output arrays that takes input row `row` (< 2^31).
+__device__ __forceinline__ int64_t output_row(const TensorArgs& a, int64_t row) {
+    if (a.tokens == 0) return row;
+    const uint32_t group = (uint32_t)row / a.tokens;
+    return (int64_t)group * a.capacity + a.base + ((uint32_t)row - group * a.tokens);
+}
+// two 16-bit values of a row as floats
+__device__ __forceinline__ float2 widen_pair(uint32_t u, bool bf16) {
+    if (bf16) return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
+    return __half22float2(*reinterpret_cast<const __half2*>(&u));
+}
+
 // ---------------------------------------------------------------------------------------------
 // Shared-memory plan
 // ---------------------------------------------------------------------------------------------
 constexpr int kW = 128;   // width of the operand layouts in tensor and shared memory; d = 64 is zero-padded to it
 template <int D, bool PROD, bool UNI>
 struct Smem {
-    static constexpr int kBoxesPerTile = D / 32;
     static constexpr int kBBytes = kW * kW * 2;                     // one fp16 operand matrix (padded)
     static constexpr int kNumB = PROD ? 4 : 2;
     static constexpr int kRingBoxes = PROD ? 5 : 8;
@@ -252,7 +265,8 @@ __device__ __noinline__ void pend_codes(const TqRecheck& l, WarpPending& w, uint
     }
 }
 
-template <int D, int BITS, bool PROD, bool UNI>
+// HALF: rows of bf16 or fp16, widened (exactly) by the converters; a TMA box then holds 64 columns.
+template <int D, int BITS, bool PROD, bool UNI, bool HALF>
 __global__ void __launch_bounds__(Threads<PROD, UNI>::kThreads, 1)
 tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorArgs a) {
     static_assert(D == 128 || D == 64, "this kernel is written for d = 128 and d = 64");
@@ -268,6 +282,11 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
     constexpr int kEpiChunks = UNI ? 1 : 2;                     // 32-column chunks a thread owns in the first epilogue
     constexpr int kEpiParts = D / (32 * kEpiChunks);            // first-epilogue threads per row that have data
     constexpr int kSignChunks = kXs / 32;                       // chunks a thread owns in the sign epilogue
+    constexpr int kBoxCols = HALF ? 64 : 32;                    // columns of a TMA box (128 bytes a row)
+    constexpr int kBoxes = D / kBoxCols;                        // boxes of a tile
+    constexpr int kBoxReaders = kXs < kBoxCols ? kBoxCols / kXs : 1;   // converter threads that share a row of a box
+    const bool bf16 = HALF && a.bf16 != 0;
+    (void)bf16;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const uint32_t smem_base = smem_u32(smem);
@@ -288,7 +307,7 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
 
     // ---- one-time set-up ------------------------------------------------------------------------
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 8; ++i) { mbar_init(BAR(BAR_FULL + i), 1); mbar_init(BAR(BAR_EMPTY + i), 4); }
+        for (int i = 0; i < 8; ++i) { mbar_init(BAR(BAR_FULL + i), 1); mbar_init(BAR(BAR_EMPTY + i), 4 * kBoxReaders); }
         for (int i = 0; i < 2; ++i) {
             mbar_init(BAR(BAR_A_FULL + i), 4 * kActiveParts);              // the converter warps that have data
             mbar_init(BAR(BAR_A_EMPTY + i), PROD ? 4 * kActiveParts : 1);  // Prod: freed by the sign epilogue
@@ -335,12 +354,12 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
             for (int64_t i = 0; i < my_tiles; ++i) {
                 const int64_t tile = blockIdx.x + i * gridDim.x;
                 bool ok = true;
-                for (int bx = 0; bx < L::kBoxesPerTile; ++bx, ++g) {
+                for (int bx = 0; bx < kBoxes; ++bx, ++g) {
                     const int slot = (int)(g % L::kRingBoxes);
                     const uint32_t par = (uint32_t)((g / L::kRingBoxes) & 1);
                     if (!mbar_wait(BAR(BAR_EMPTY + slot), par ^ 1u, abort_flag)) { ok = false; break; }
                     mbar_arrive_expect_tx(BAR(BAR_FULL + slot), kBoxBytes);
-                    tma_load_box(smem_base + L::off_ring + slot * kBoxBytes, &tmap_x, bx * 32, (int)(tile * kTileRows),
+                    tma_load_box(smem_base + L::off_ring + slot * kBoxBytes, &tmap_x, bx * kBoxCols, (int)(tile * kTileRows),
                                  BAR(BAR_FULL + slot));
                 }
                 if (!ok) break;
@@ -474,7 +493,7 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
             const int64_t tile = blockIdx.x + j * gridDim.x;
             const int b = (int)(j & 1);
             const uint32_t par2 = (uint32_t)((j >> 1) & 1);
-            const int64_t grow = tile * kTileRows + row;
+            const int64_t grow = tile * kTileRows + row, orow = output_row(a, grow);
             TQ_PROF_CODE(const bool pr = a.prof && blockIdx.x == 0 && threadIdx.x == kFirstConvWarp * 32; long long c0 = clock64(), c1;)
             bool redo_row = sc0 == 0 && force[(j & 3) * kTileRows + row] != 0;
             const bool live = mbar_wait(BAR(BAR_ACC2_FULL + b), par2, abort_flag) && grow < a.n;   // no stores after a give-up
@@ -486,7 +505,7 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
                 float rs_all = rp[0];
 #pragma unroll
                 for (int pt = 1; pt < kEpiParts; ++pt) rs_all += rp[pt * kTileRows];
-                a.rnorms[grow] = sqrtf(rs_all) * kScaleRho;
+                a.rnorms[orow] = sqrtf(rs_all) * kScaleRho;
             }
             uint32_t va[32];
             uint32_t sw0 = 0, sw1 = 0;
@@ -526,8 +545,8 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
             __syncwarp();
             if (lane == 0) mbar_arrive(BAR(BAR_A_EMPTY + (b ^ 1)));  // that A block may be refilled
             if (live) {
-                if (kSignChunks == 2) *reinterpret_cast<uint2*>(a.signs + grow * (D / 32) + sc0) = make_uint2(sw0, sw1);
-                else a.signs[grow * (D / 32) + sc0] = sw0;
+                if (kSignChunks == 2) *reinterpret_cast<uint2*>(a.signs + orow * (D / 32) + sc0) = make_uint2(sw0, sw1);
+                else a.signs[orow * (D / 32) + sc0] = sw0;
             }
             pend_rows(a.lists, pend, redo_row && live, grow, lane);
             TQ_PROF_CODE(if (pr) prof_acc[19] += clock64() - c1;)
@@ -542,26 +561,41 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
             bool fail = false;
             TQ_PROF_CODE(const bool pr = a.prof && blockIdx.x == 0 && threadIdx.x == kFirstConvWarp * 32; long long c0 = clock64(), c1;)
 #pragma unroll
-            for (int bb = 0; bb < kXs / 32; ++bb) {
-                const int64_t g = g_base + half * (kXs / 32) + bb;
+            for (int bb = 0; bb < (HALF ? 1 : kXs / 32); ++bb) {
+                const int64_t g = g_base + (HALF ? half / kBoxReaders : half * (kXs / 32) + bb);
                 const int slot = (int)(g % L::kRingBoxes);
                 const uint32_t par = (uint32_t)((g / L::kRingBoxes) & 1);
                 TQ_PROF_CODE(long long cw0 = clock64();)
                 if (!fail && !mbar_wait(BAR(BAR_FULL + slot), par, abort_flag)) fail = true;
                 TQ_PROF_CODE(if (pr) prof_acc[6] += clock64() - cw0;)
                 const unsigned char* box = smem + L::off_ring + slot * kBoxBytes + row * 128;
+                constexpr int kPieces = HALF ? kXs / 8 : 8;      // 16-byte pieces of the row in this box
+                const int piece0 = HALF ? (half % kBoxReaders) * kPieces : 0;
+                uint32_t raw[kPieces * 4];
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {
+                for (int c = 0; c < kPieces; ++c) {
                     const float4 v = fail ? make_float4(0.f, 0.f, 0.f, 0.f)
-                                          : lds_once_f4(box + ((c ^ (row & 7)) << 4));
-                    x[bb * 32 + c * 4 + 0] = v.x;
-                    x[bb * 32 + c * 4 + 1] = v.y;
-                    x[bb * 32 + c * 4 + 2] = v.z;
-                    x[bb * 32 + c * 4 + 3] = v.w;
+                                          : lds_once_f4(box + (((piece0 + c) ^ (row & 7)) << 4));
+                    raw[c * 4 + 0] = __float_as_uint(v.x);
+                    raw[c * 4 + 1] = __float_as_uint(v.y);
+                    raw[c * 4 + 2] = __float_as_uint(v.z);
+                    raw[c * 4 + 3] = __float_as_uint(v.w);
                 }
                 __threadfence_block();   // every lane's loads from the stage are performed before the stage is released
                 __syncwarp();
                 if (lane == 0 && !fail) mbar_arrive(BAR(BAR_EMPTY + slot));
+                if constexpr (HALF) {
+                    if (bf16) {          // (looked at once)
+#pragma unroll
+                        for (int c = 0; c < kXs / 2; ++c) { const float2 f = widen_pair(raw[c], true); x[2 * c] = f.x; x[2 * c + 1] = f.y; }
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < kXs / 2; ++c) { const float2 f = widen_pair(raw[c], false); x[2 * c] = f.x; x[2 * c + 1] = f.y; }
+                    }
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 32; ++c) x[bb * 32 + c] = __uint_as_float(raw[c]);
+                }
             }
             // 32 values per thread: two values per instruction (fma / mul / add .f32x2), 3 % faster; 64 values per
             // thread: scalar, the packed form is 7 % slower there (register pairs)
@@ -602,7 +636,7 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
             const float sc = (ok && !odd) ? kScaleA / nrm : 0.f;
             if (half == 0) {
                 const int64_t grow = tile * kTileRows + row;
-                if (grow < a.n && !fail) a.norms[grow] = nrm;
+                if (grow < a.n && !fail) a.norms[output_row(a, grow)] = nrm;
                 force[(i & 3) * kTileRows + row] = odd ? 1 : 0;
             }
             if (!mbar_wait(BAR(BAR_A_EMPTY + b), par2 ^ 1u, abort_flag)) fail = true;
@@ -641,7 +675,7 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
             __syncwarp();
             if (lane == 0) mbar_arrive(BAR(BAR_A_FULL + b));
             TQ_PROF_CODE(if (pr) { prof_acc[4] += clock64() - c0; prof_acc[5] += 1; })
-            g_base += L::kBoxesPerTile;
+            g_base += kBoxes;
         };
 
         // -- first-accumulator epilogue of tile i: codes (+ rho for TurboQuantProd)
@@ -649,7 +683,7 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
             const int64_t tile = blockIdx.x + i * gridDim.x;
             const int b = (int)(i & 1);
             const uint32_t par2 = (uint32_t)((i >> 1) & 1);
-            const int64_t grow = tile * kTileRows + row;
+            const int64_t grow = tile * kTileRows + row, orow = output_row(a, grow);
             const bool live_row = grow < a.n;
             TQ_PROF_CODE(const bool pr = a.prof && blockIdx.x == 0 && threadIdx.x == (UNI ? kFirstConvWarp : kFirstEpiWarp) * 32; long long c0 = clock64(), c1;)
             const bool got = mbar_wait(BAR(BAR_ACC_FULL + b), par2, abort_flag);   // false: some role gave up, the
@@ -662,7 +696,7 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
             uint32_t nm[kEpiChunks];
             auto store_codes = [&](int ch, const uint32_t (&w)[BITS + 1]) {
                 if (live) {  // this chunk's packed codes: BITS words at a BITS*4-byte aligned offset of the row
-                    uint32_t* dst = a.codes + grow * kCodeWords + (chunk0 + ch) * BITS;
+                    uint32_t* dst = a.codes + orow * kCodeWords + (chunk0 + ch) * BITS;
                     if (BITS == 4) *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
                     else if (BITS == 2) *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
                     else {
@@ -1052,7 +1086,7 @@ tensor_quantize256_kernel(const __grid_constant__ CUtensorMap tmap_x, const Tens
             const float sc = (okn && !odd) ? kScaleA / nrm : 0.f;
             if (part == 0) {
                 const int64_t grow = tile * kTileRows + row;
-                if (grow < a.n && !fail) a.norms[grow] = nrm;
+                if (grow < a.n && !fail) a.norms[output_row(a, grow)] = nrm;
                 force[(i & 3) * kTileRows + row] = odd ? 1 : 0;
             }
             // TurboQuantProd: this thread itself was the last reader of its cells (sign epilogue of the previous tile, below)
@@ -1089,7 +1123,7 @@ tensor_quantize256_kernel(const __grid_constant__ CUtensorMap tmap_x, const Tens
                 tc_fence_after();
                 if (part == 0 && live) {      // |rho|^2 in 2^10 units: the four partial sums of the first epilogue
                     const float rs_all = (rs_part[row] + rs_part[kTileRows + row]) + (rs_part[2 * kTileRows + row] + rs_part[3 * kTileRows + row]);
-                    a.rnorms[grow] = sqrtf(rs_all) * kScaleRho;
+                    a.rnorms[output_row(a, grow)] = sqrtf(rs_all) * kScaleRho;
                 }
                 const uint32_t acc2 = tmem + lane_addr + A_COL(j);
                 uint32_t sw[2] = {0u, 0u};
@@ -1117,8 +1151,9 @@ tensor_quantize256_kernel(const __grid_constant__ CUtensorMap tmap_x, const Tens
                 }
                 tc_fence_before();
                 if (live) {
-                    a.signs[grow * (kD / 32) + j * 4 + hcol] = sw[0];
-                    a.signs[grow * (kD / 32) + j * 4 + 2 + hcol] = sw[1];
+                    const int64_t orow = output_row(a, grow);
+                    a.signs[orow * (kD / 32) + j * 4 + hcol] = sw[0];
+                    a.signs[orow * (kD / 32) + j * 4 + 2 + hcol] = sw[1];
                 }
                 pend_rows(a.lists, cpend, redo_row && live, grow, lane);
             }
@@ -1143,7 +1178,7 @@ tensor_quantize256_kernel(const __grid_constant__ CUtensorMap tmap_x, const Tens
         for (int64_t i = 0; i < my_tiles; ++i) {
             const int64_t tile = blockIdx.x + i * gridDim.x;
             const uint32_t par = (uint32_t)(i & 1);
-            const int64_t grow = tile * kTileRows + row;
+            const int64_t grow = tile * kTileRows + row, orow = output_row(a, grow);
 #pragma unroll 1
             for (int j = 0; j < 2; ++j) {
                 const bool got = mbar_wait(BAR(ACC_FULL + j), par, abort_flag);
@@ -1167,7 +1202,7 @@ tensor_quantize256_kernel(const __grid_constant__ CUtensorMap tmap_x, const Tens
                         tmem_st16(acc + chunk * 32 + 16, rlo);
                     }
                     if (live) {
-                        uint32_t* dst = a.codes + grow * kCodeWords + (j * 4 + chunk) * BITS;
+                        uint32_t* dst = a.codes + orow * kCodeWords + (j * 4 + chunk) * BITS;
                         if (BITS == 4) *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
                         else if (BITS == 2) *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
                         else {
@@ -1416,14 +1451,19 @@ void tq_tensor_plan_free(tq_plan* p) {
 #ifndef TQ_UNI_MSE
 #define TQ_UNI_MSE false
 #endif
-template <int D, int BITS, bool PROD>
-static int launch_one(const tq_plan* p, const CUtensorMap& map, const TensorArgs& args, int grid, cudaStream_t st) {
+template <int D, int BITS, bool PROD, bool HALF>
+static int launch_type(const tq_plan* p, const CUtensorMap& map, const TensorArgs& args, int grid, cudaStream_t st) {
     constexpr bool UNI = PROD ? TQ_UNI_PROD : TQ_UNI_MSE;
     const int sm = Smem<D, PROD, UNI>::total;
-    TQ_GRANT_SMEM((tensor_quantize_kernel<D, BITS, PROD, UNI>), sm, p->device);
-    tensor_quantize_kernel<D, BITS, PROD, UNI><<<grid, Threads<PROD, UNI>::kThreads, sm, st>>>(map, args); tq_count_launch();
+    TQ_GRANT_SMEM((tensor_quantize_kernel<D, BITS, PROD, UNI, HALF>), sm, p->device);
+    tensor_quantize_kernel<D, BITS, PROD, UNI, HALF><<<grid, Threads<PROD, UNI>::kThreads, sm, st>>>(map, args); tq_count_launch();
     TQ_CUDA_TRY(cudaGetLastError());
     return TQ_OK;
+}
+
+template <int D, int BITS, bool PROD>
+static int launch_one(const tq_plan* p, const CUtensorMap& map, const TensorArgs& args, bool half, int grid, cudaStream_t st) {
+    return half ? launch_type<D, BITS, PROD, true>(p, map, args, grid, st) : launch_type<D, BITS, PROD, false>(p, map, args, grid, st);
 }
 
 template <int BITS, bool PROD>
@@ -1434,19 +1474,27 @@ static int launch_256(const tq_plan* p, const CUtensorMap& map, const TensorArgs
     return TQ_OK;
 }
 
-int tq_launch_tensor_quantize(const tq_plan* p, bool prod, const float* x, int64_t n, uint32_t* codes,
-                              uint32_t* signs, float* rnorms, float* norms, const TqRecheck* lists, cudaStream_t st) {
+// The kernels that read 16-bit rows are those for d = 64 and 128.
+bool tq_tensor_input_supported(int d, int xtype) { return xtype == TQ_INPUT_F32 || d != 256; }
+
+int tq_launch_tensor_quantize(const tq_plan* p, bool prod, const void* x, int xtype, int64_t n, const TqQuantOut& out,
+                              const TqRecheck* lists, cudaStream_t st) {
     TqRange range("tq.quantize.tensor_core");
     if (!p->tensor) return tq_fail(TQ_ERR_UNSUPPORTED, "no tensor-core kernel for this plan");
     const int d = p->dev.d;
+    const bool half = xtype != TQ_INPUT_F32;
     if (n > (int64_t)0x7fffff00) return tq_fail(TQ_ERR_UNSUPPORTED, "n above 2^31 rows per call");
     TensorArgs args = p->tensor->args;
     args.n = n;
     args.ntiles = (n + kTileRows - 1) / kTileRows;
-    args.codes = codes;
-    args.signs = signs;
-    args.norms = norms;
-    args.rnorms = rnorms;
+    args.codes = out.codes;
+    args.signs = out.signs;
+    args.norms = out.norms;
+    args.rnorms = out.rnorms;
+    args.bf16 = xtype == TQ_INPUT_BF16;
+    args.tokens = (uint32_t)out.map.tokens;
+    args.capacity = (uint32_t)out.map.capacity;
+    args.base = (uint32_t)out.map.base;
     args.lists = *lists;
     args.status = p->status_dev;
     args.wait_kcycles = p->wait_kcycles;
@@ -1456,10 +1504,10 @@ int tq_launch_tensor_quantize(const tq_plan* p, bool prod, const float* x, int64
 
     CUtensorMap map;
     const cuuint64_t gdim[2] = {(cuuint64_t)d, (cuuint64_t)n};
-    const cuuint64_t gstride[1] = {(cuuint64_t)d * 4};
-    const cuuint32_t box[2] = {32, (cuuint32_t)kTileRows};
+    const cuuint64_t gstride[1] = {(cuuint64_t)d * (half ? 2 : 4)};
+    const cuuint32_t box[2] = {half ? 64u : 32u, (cuuint32_t)kTileRows};
     const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = tq_encode_tiled_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(x), gdim, gstride,
+    const CUresult r = tq_encode_tiled_fn()(&map, half ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(x), gdim, gstride,
                                          box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return tq_fail(TQ_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d", (int)r);
@@ -1482,8 +1530,8 @@ int tq_launch_tensor_quantize(const tq_plan* p, bool prod, const float* x, int64
     }
 #define TQ_DISPATCH(B)                                                                                     \
     case B:                                                                                                \
-        if (d == 64) rc = prod ? launch_one<64, B, true>(p, map, args, grid, st) : launch_one<64, B, false>(p, map, args, grid, st); \
-        else rc = prod ? launch_one<128, B, true>(p, map, args, grid, st) : launch_one<128, B, false>(p, map, args, grid, st);      \
+        if (d == 64) rc = prod ? launch_one<64, B, true>(p, map, args, half, grid, st) : launch_one<64, B, false>(p, map, args, half, grid, st); \
+        else rc = prod ? launch_one<128, B, true>(p, map, args, half, grid, st) : launch_one<128, B, false>(p, map, args, half, grid, st);      \
         break;
     switch (bits) {
         TQ_DISPATCH(1)

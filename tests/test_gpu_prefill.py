@@ -1,0 +1,42 @@
+"""Bulk appends to a key/value cache: rows of every element type go straight into place, and are what the quantizers give
+for the widened rows -- tile remainders, a cache that is partly filled, bit widths without a tensor-core kernel."""
+import pytest
+
+import project_tensor_b200 as tg
+from project_tensor_b200.cache import PackedKVCache
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16", "float16"])
+@pytest.mark.parametrize("d,kbits,vbits,groups,lengths", [
+    (128, 3, 4, 3, (5, 4001)),           # 12,003 rows: a tile with 99 of them
+    (64, 4, 3, 4, (1500, 1190, 7)),      # the second call has 4,760 rows, just above what one launch takes
+    (128, 6, 2, 2, (2500,)),             # 5-bit keys have no tensor-core kernel, the values do
+    (96, 4, 4, 1, (4200,)), (256, 4, 4, 2, (3000,)),
+])
+def test_bulk_append_equals_quantize(dtype, d, kbits, vbits, groups, lengths):
+    import torch
+    kq = tg.TurboQuantProd(d, kbits, seed=2026, grid_size=4097, max_iter=64)
+    vq = tg.TurboQuantMSE(d, vbits, seed=77, grid_size=4097, max_iter=64)
+    cap = sum(lengths) + 3
+    cache = PackedKVCache(kq, vq, groups, cap)
+    gen = torch.Generator("cuda").manual_seed(d + kbits)
+    keys, values = (torch.randn(groups, sum(lengths), d, device="cuda", generator=gen).to(getattr(torch, dtype)) for _ in range(2))
+    keys[0, 1] = 0
+    keys[0, 2] *= 1e-4
+    at = 0
+    for n in lengths:
+        cache.append(keys[:, at:at + n].contiguous(), values[:, at:at + n].contiguous())
+        at += n
+        assert len(cache) == at and int(cache.keys.length_device.item()) == at
+    want = tg.packed_buffers(kq.quantize(keys.float().reshape(-1, d)))
+    kc = cache.keys
+    for name, have in (("codes", kc.codes), ("signs", kc.signs), ("norms", kc.norms), ("residual_norms", kc.residual_norms)):
+        have = have.view(groups, cap, -1)
+        assert torch.equal(have[:, :at].reshape(groups * at, -1), want[name].reshape(groups * at, -1)) or (
+            "norms" in name and float((have[:, :at].reshape(-1) / want[name].reshape(-1) - 1).nan_to_num().abs().max()) <= 1e-6), name
+        assert not bool(have[:, at:].any()), name
+    want = tg.packed_buffers(vq.quantize(values.float().reshape(-1, d)))
+    assert torch.equal(cache.value_codes.view(groups, cap, -1)[:, :at].reshape(groups * at, -1), want["codes"].reshape(groups * at, -1))
+    assert float((cache.value_norms.view(groups, cap)[:, :at].reshape(-1) / want["norms"] - 1).abs().max()) <= 1e-6
