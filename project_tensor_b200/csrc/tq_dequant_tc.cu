@@ -458,17 +458,21 @@ dequant_tc_kernel(const DequantArgs a) {
 // coordinates, hi then lo, K-major core matrices) through a ring, three tensor instructions per chunk.  TurboQuantProd
 // runs a second phase on the same tile: the expanders overwrite the operand blocks with +-beta (beta = alpha * rnorm
 // * 2^16, hi / lo), 32 chunks of the transposed projection follow, and the products add into the same accumulators.
+// Operand block I is multiplied into both output halves before block 1 - I is, so that the expanders fill one block while
+// the other one is read, and the halves finish one after the other, so that the epilogue of the first runs beside the second
+// (output half by output half, with both blocks held to the end, 524,309 keys took 414 us; now @D@).
 // Warps: bulk copies of the packed keys, MMA, bulk copies of the chunks, 16 expanders (64 coordinates per thread),
 // 8 epilogue warps (two threads per key and output half).
 namespace dq256 {
 constexpr int kD = 256;
 constexpr int kChunkBytes = 8192;
-constexpr int kBRing = 8;
+constexpr int kStep = 2, kStepBytes = kStep * kChunkBytes;   // chunks per copy and stage of the ring
+constexpr int kBRing = 4;
 constexpr int kKStages = 2;
 constexpr int kExpWarps = 16, kEpiWarps = 8;
 constexpr int kFirstExp = 3, kFirstEpi = kFirstExp + kExpWarps;
 constexpr int kThreads256 = (3 + kExpWarps + kEpiWarps) * 32;
-enum { K_FULL = 0, K_EMPTY = 2, B_FULL = 4, B_EMPTY = 12, A_FULL = 20, A_EMPTY = 21, D_FULL = 22, D_EMPTY = 24, N_BARS = 26 };
+enum { K_FULL = 0, K_EMPTY = 2, B_FULL = 4, B_EMPTY = 12, A_FULL = 20, A_EMPTY = 22, D_FULL = 24, D_EMPTY = 26, N_BARS = 28 };
 template <int BITS, bool PROD>
 struct Smem {
     static constexpr int kLutBytes = (1 << (2 * BITS)) * 32 * 8;
@@ -479,7 +483,7 @@ struct Smem {
     static constexpr int kOutWarpBytes = 32 * kOutRowBytes;
     static constexpr int off_lut = 0;
     static constexpr int off_b = off_lut + kLutBytes;
-    static constexpr int off_ring = off_b + kBRing * kChunkBytes;
+    static constexpr int off_ring = off_b + kBRing * kStepBytes;
     static constexpr int off_out = off_ring + kKStages * kStageBytes;
     static constexpr int off_misc = off_out + kEpiWarps * kOutWarpBytes;
     static constexpr int total = off_misc + 512 + 128 + 128;    // + slack to align the base
@@ -506,8 +510,7 @@ dequant256_kernel(const DequantArgs a) {
     if (threadIdx.x == 0) {
         for (int i = 0; i < kKStages; ++i) { mbar_init(BAR(K_FULL + i), 1); mbar_init(BAR(K_EMPTY + i), kExpWarps); }
         for (int i = 0; i < kBRing; ++i) { mbar_init(BAR(B_FULL + i), 1); mbar_init(BAR(B_EMPTY + i), 1); }
-        mbar_init(BAR(A_FULL), kExpWarps);
-        mbar_init(BAR(A_EMPTY), 1);
+        for (int h = 0; h < 2; ++h) { mbar_init(BAR(A_FULL + h), kExpWarps / 2); mbar_init(BAR(A_EMPTY + h), 1); }
         for (int j = 0; j < 2; ++j) { mbar_init(BAR(D_FULL + j), 1); mbar_init(BAR(D_EMPTY + j), kEpiWarps); }
         abort_flag[0] = 0;
         abort_flag[1] = a.wait_kcycles;
@@ -572,16 +575,17 @@ dequant256_kernel(const DequantArgs a) {
                     mbar_drain(BAR(K_FULL + (int)(ii % kKStages)), (uint32_t)((ii / kKStages) & 1));
         }
     } else if (warp == 2) {
-        // ---- operand chunks: the same 32 (64) chunks for every tile -------------------------------------
+        // ---- operand chunks: the same 32 (64) chunks for every tile, in the order of the instructions: (phase, I, J, kb) ----
         if (lane == 0) {
             int64_t g = 0;
             bool ok = true;
             for (int64_t i = 0; i < my_tiles && ok; ++i) {
-                for (int c = 0; c < kPhases * 32; ++c, ++g) {
+                for (int c = 0; c < kPhases * 32; c += kStep, ++g) {
                     const int slot = (int)(g % kBRing);
+                    const int chunk = (c & 32) + ((c & 8) << 1) + ((c & 16) >> 1) + (c & 7);
                     if (!mbar_wait(BAR(B_EMPTY + slot), (uint32_t)(((g / kBRing) & 1) ^ 1), abort_flag)) { ok = false; break; }
-                    mbar_arrive_expect_tx(BAR(B_FULL + slot), kChunkBytes);
-                    bulk_load(smem_base + L::off_b + slot * kChunkBytes, a.bmat + (size_t)c * kChunkBytes, kChunkBytes, BAR(B_FULL + slot));
+                    mbar_arrive_expect_tx(BAR(B_FULL + slot), kStepBytes);
+                    bulk_load(smem_base + L::off_b + slot * kStepBytes, a.bmat + (size_t)chunk * kChunkBytes, kStepBytes, BAR(B_FULL + slot));
                 }
             }
             if (*abort_flag)
@@ -596,32 +600,37 @@ dequant256_kernel(const DequantArgs a) {
         for (int64_t i = 0; i < my_tiles && ok; ++i) {
             const uint32_t par = (uint32_t)(i & 1);
             for (int ph = 0; ph < kPhases && ok; ++ph, ++phase_n) {
-                if (!warp_wait(BAR(A_FULL), (uint32_t)(phase_n & 1), abort_flag)) { ok = false; break; }
-                for (int j = 0; j < 2 && ok; ++j) {
-                    if (ph == 0 && !warp_wait(BAR(D_EMPTY + j), par ^ 1u, abort_flag)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint32_t acc = tm + ACC_COL(j);
-                    for (int c = 0; c < 16; ++c, ++g) {          // c = I * 8 + kb
-                        const int slot = (int)(g % kBRing);
-                        if (!warp_wait(BAR(B_FULL + slot), (uint32_t)((g / kBRing) & 1), abort_flag)) { ok = false; break; }
+                for (int h = 0; h < 2 && ok; ++h) {              // K half
+                    if (!warp_wait(BAR(A_FULL + h), (uint32_t)(phase_n & 1), abort_flag)) { ok = false; break; }
+                    for (int j = 0; j < 2 && ok; ++j) {
+                        if (ph == 0 && h == 0 && !warp_wait(BAR(D_EMPTY + j), par ^ 1u, abort_flag)) { ok = false; break; }
                         tc_fence_after();
-                        const uint32_t chunk = smem_base + L::off_b + slot * kChunkBytes;
-                        const uint64_t d_hi = make_smem_desc(chunk, 128, 256), d_lo = make_smem_desc(chunk + kChunkBytes / 2, 128, 256);
-                        const uint32_t a_hi = tm + A_COL(c >> 3) + (uint32_t)(c & 7) * 8, a_lo = a_hi + kABlock;
-                        if (elect_one()) {
-                            if (ph == 0 && c == 0) mma_ts_first(acc, a_hi, d_hi, kIdesc);
-                            else mma_ts_acc(acc, a_hi, d_hi, kIdesc);
-                            mma_ts_acc(acc, a_hi, d_lo, kIdesc);
-                            mma_ts_acc(acc, a_lo, d_hi, kIdesc);
-                            mma_commit(BAR(B_EMPTY + slot));
-                            if (c == 15 && ph == kPhases - 1) mma_commit(BAR(D_FULL + j));
+                        const uint32_t acc = tm + ACC_COL(j);
+                        for (int c = 0; c < 8; c += kStep, ++g) {
+                            const int slot = (int)(g % kBRing);
+                            if (!warp_wait(BAR(B_FULL + slot), (uint32_t)((g / kBRing) & 1), abort_flag)) { ok = false; break; }
+                            tc_fence_after();
+                            const uint64_t d0 = make_smem_desc(smem_base + L::off_b + slot * kStepBytes, 128, 256);
+                            if (elect_one()) {
+#pragma unroll
+                                for (int u = 0; u < kStep; ++u) {
+                                    const uint64_t d_hi = d0 + (uint64_t)(u * kChunkBytes >> 4), d_lo = d_hi + (uint64_t)(kChunkBytes / 2 >> 4);
+                                    const uint32_t a_hi = tm + A_COL(h) + (uint32_t)(c + u) * 8, a_lo = a_hi + kABlock;
+                                    if (ph == 0 && h == 0 && c + u == 0) mma_ts_first(acc, a_hi, d_hi, kIdesc);
+                                    else mma_ts_acc(acc, a_hi, d_hi, kIdesc);
+                                    mma_ts_acc(acc, a_hi, d_lo, kIdesc);
+                                    mma_ts_acc(acc, a_lo, d_hi, kIdesc);
+                                }
+                                mma_commit(BAR(B_EMPTY + slot));
+                                if (c + kStep == 8 && h == 1 && ph == kPhases - 1) mma_commit(BAR(D_FULL + j));
+                            }
+                            __syncwarp();
                         }
-                        __syncwarp();
                     }
+                    if (!ok) break;
+                    if (elect_one()) mma_commit(BAR(A_EMPTY + h));       // the operand block has been read
+                    __syncwarp();
                 }
-                if (!ok) break;
-                if (elect_one()) mma_commit(BAR(A_EMPTY));       // the operand blocks have been read
-                __syncwarp();
             }
         }
     } else if (warp < kFirstEpi) {
@@ -675,7 +684,7 @@ dequant256_kernel(const DequantArgs a) {
                         hi[sb][p] = v.x;
                         lo[sb][p] = v.y;
                     }
-                if (!mbar_wait(BAR(A_EMPTY), (uint32_t)(phase_n & 1) ^ 1u, abort_flag)) fail = true;
+                if (!mbar_wait(BAR(A_EMPTY + (part >> 1)), (uint32_t)(phase_n & 1) ^ 1u, abort_flag)) fail = true;
                 tc_fence_after();
 #pragma unroll
                 for (int sb = 0; sb < 2; ++sb) {
@@ -685,7 +694,7 @@ dequant256_kernel(const DequantArgs a) {
                 tmem_wait_st();
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(BAR(A_FULL));
+                if (lane == 0) mbar_arrive(BAR(A_FULL + (part >> 1)));
                 ++phase_n;
             }
             if (PROD) {   // phase 1: +-beta, both halves of a pair alike; the signs flip bit 15 / 31
@@ -694,7 +703,7 @@ dequant256_kernel(const DequantArgs a) {
                 const __half bl = __float2half_rn(beta - __half2float(bh));
                 const uint32_t bhu = (uint32_t)__half_as_ushort(bh), blu = (uint32_t)__half_as_ushort(bl);
                 const uint32_t bh2 = bhu | (bhu << 16), bl2 = blu | (blu << 16);
-                if (!mbar_wait(BAR(A_EMPTY), (uint32_t)(phase_n & 1) ^ 1u, abort_flag)) fail = true;
+                if (!mbar_wait(BAR(A_EMPTY + (part >> 1)), (uint32_t)(phase_n & 1) ^ 1u, abort_flag)) fail = true;
                 tc_fence_after();
 #pragma unroll
                 for (int sb = 0; sb < 2; ++sb) {
@@ -711,7 +720,7 @@ dequant256_kernel(const DequantArgs a) {
                 tmem_wait_st();
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(BAR(A_FULL));
+                if (lane == 0) mbar_arrive(BAR(A_FULL + (part >> 1)));
                 ++phase_n;
             }
         }

@@ -83,9 +83,11 @@ struct TensorArgs {
 #endif
 };
 
-// Row of the output arrays that takes input row `row` (< 2^31).
+// Row of the output arrays that takes input row `row` (< 2^31).  (Kernels of their own for rows of a cache: the divisions
+// cost the plain ones a tenth of their time, through the instruction cache.)
+template <bool MAPPED>
 __device__ __forceinline__ int64_t output_row(const TensorArgs& a, int64_t row) {
-    if (a.tokens == 0) return row;
+    if constexpr (!MAPPED) return row;
     const uint32_t group = (uint32_t)row / a.tokens;
     return (int64_t)group * a.capacity + a.base + ((uint32_t)row - group * a.tokens);
 }
@@ -266,7 +268,7 @@ __device__ __noinline__ void pend_codes(const TqRecheck& l, WarpPending& w, uint
 }
 
 // HALF: rows of bf16 or fp16, widened (exactly) by the converters; a TMA box then holds 64 columns.
-template <int D, int BITS, bool PROD, bool UNI, bool HALF>
+template <int D, int BITS, bool PROD, bool UNI, bool HALF, bool MAPPED>
 __global__ void __launch_bounds__(Threads<PROD, UNI>::kThreads, 1)
 tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorArgs a) {
     static_assert(D == 128 || D == 64, "this kernel is written for d = 128 and d = 64");
@@ -493,7 +495,7 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
             const int64_t tile = blockIdx.x + j * gridDim.x;
             const int b = (int)(j & 1);
             const uint32_t par2 = (uint32_t)((j >> 1) & 1);
-            const int64_t grow = tile * kTileRows + row, orow = output_row(a, grow);
+            const int64_t grow = tile * kTileRows + row, orow = output_row<MAPPED>(a, grow);
             TQ_PROF_CODE(const bool pr = a.prof && blockIdx.x == 0 && threadIdx.x == kFirstConvWarp * 32; long long c0 = clock64(), c1;)
             bool redo_row = sc0 == 0 && force[(j & 3) * kTileRows + row] != 0;
             const bool live = mbar_wait(BAR(BAR_ACC2_FULL + b), par2, abort_flag) && grow < a.n;   // no stores after a give-up
@@ -636,7 +638,7 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
             const float sc = (ok && !odd) ? kScaleA / nrm : 0.f;
             if (half == 0) {
                 const int64_t grow = tile * kTileRows + row;
-                if (grow < a.n && !fail) a.norms[output_row(a, grow)] = nrm;
+                if (grow < a.n && !fail) a.norms[output_row<MAPPED>(a, grow)] = nrm;
                 force[(i & 3) * kTileRows + row] = odd ? 1 : 0;
             }
             if (!mbar_wait(BAR(BAR_A_EMPTY + b), par2 ^ 1u, abort_flag)) fail = true;
@@ -683,7 +685,7 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
             const int64_t tile = blockIdx.x + i * gridDim.x;
             const int b = (int)(i & 1);
             const uint32_t par2 = (uint32_t)((i >> 1) & 1);
-            const int64_t grow = tile * kTileRows + row, orow = output_row(a, grow);
+            const int64_t grow = tile * kTileRows + row, orow = output_row<MAPPED>(a, grow);
             const bool live_row = grow < a.n;
             TQ_PROF_CODE(const bool pr = a.prof && blockIdx.x == 0 && threadIdx.x == (UNI ? kFirstConvWarp : kFirstEpiWarp) * 32; long long c0 = clock64(), c1;)
             const bool got = mbar_wait(BAR(BAR_ACC_FULL + b), par2, abort_flag);   // false: some role gave up, the
@@ -848,43 +850,50 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
 }
 
 // ---------------------------------------------------------------------------------------------
-// d = 256 (TurboQuantMSE): the split rotation is 2 x 128 KB and cannot stay in shared memory, so it streams
+// d = 256: the split rotation is 2 x 128 KB and cannot stay in shared memory, so it streams
 // ---------------------------------------------------------------------------------------------
 // A tile is 128 rows x 256 columns.  The unit rows, split into fp16 hi / lo, fill both A blocks of tensor memory
 // (K half I in block I); the two accumulator blocks take the two halves J of the output columns.  The rotation is
 // stored as 32 chunks of 8 KB -- chunk ((J * 2 + I) * 8 + kb) holds R_hi and R_lo for output columns [128 J, 128 J + 128)
 // and input coordinates [128 I + 16 kb, + 16) as K-major 8 x 8 core matrices -- and every CTA pulls the 256 KB through a
-// ring of 8 chunks once per tile (from L2), three tensor instructions per chunk.  Tensor memory is full with one tile
-// (A 256 + accumulators 256 columns), so the conversion of a tile cannot overlap the contractions of its predecessor;
-// the epilogue of output half 0 runs beside the contractions of half 1.  96 tensor instructions (6.1 K cycles) per tile
-// stand against 6.4 K cycles of HBM time for its 148 KB.
-// Warps: TMA for the rows, MMA, bulk copies of the rotation, 16 converters (64 values per thread), 8 epilogue warps.
+// ring of 8 chunks once per tile (from L2), three tensor instructions per chunk.  For TurboQuantProd rho (split, in place of
+// the accumulators) is multiplied with 16 (R S^T), 32 more chunks, into the A blocks.
+//
+// Tensor memory is full with one tile (A 256 + accumulators 256 columns), so the phases of a tile form a chain and what counts is
+// how short the chain is beside its 96 (TurboQuantProd 192) tensor instructions of 64 cycles.  Sixteen worker warps, four per
+// row, take every phase together, each on its own columns; the work splits into halves so that tensor instructions run beside it:
+//   TurboQuantProd   first contraction J = 0 | J = 1 beside the epilogue of J = 0 | second contraction over rho half 0 beside the
+//                    epilogue of J = 1 | over rho half 1 beside the norms of the next rows | signs and conversion of the next rows
+//   TurboQuantMSE    J = 0 beside the epilogue of J = 1 of the tile before | J = 1 beside the next norms and the epilogue of J = 0
+// The rows stay in shared memory between the norm and the conversion (64 registers a thread otherwise).
+// Before -- 16 converter warps that idled through the epilogues of 8 other warps, the second contraction behind both
+// epilogues -- 524,309 rows, TurboQuantProd at 4 bits took 542 us, now @P@ (TurboQuantMSE @M0@, now @M1@).
+// Warps: TMA for the rows, MMA, bulk copies of the rotation, 16 workers.
 namespace d256 {
 constexpr int kD = 256;
 constexpr int kBoxesPerTile = kD / 32;           // 8
-constexpr int kXRing = 8;                    // one tile: a converter must not meet a slot's second use before its first
+constexpr int kXRing = 8;                    // one tile: a worker must not meet a slot's second use before its first
                                             // (its wait on the later parity would pass at once while the first copy is still on its way)
 constexpr int kChunkBytes = 8192;                // R_hi and R_lo of one (J, I, kb): 128 x 16 halves each
-constexpr int kChunksPerMatrix = 32;          // per tile: the rotation, and for TurboQuantProd 16 (R S^T) behind it
-constexpr int kBRing = 8;                    // (10 chunks, which is what shared memory leaves room for, were slower: 582 against 542 us)
-constexpr int kConvWarps = 16, kEpiWarps = 8;
-constexpr int kFirstConv = 3, kFirstEpi = kFirstConv + kConvWarps;
-constexpr int kThreads = (3 + kConvWarps + kEpiWarps) * 32;      // 864
+constexpr int kStep = 2;                         // chunks per copy and stage of the ring
+constexpr int kStepBytes = kStep * kChunkBytes;
+constexpr int kBRing = 4;
+constexpr int kWorkers = 16, kFirstWorker = 3;
+constexpr int kThreads = (kFirstWorker + kWorkers) * 32;         // 608
 constexpr int off_b = 0;
-constexpr int off_x = off_b + kBRing * kChunkBytes;              // 128 KB
+constexpr int off_x = off_b + kBRing * kStepBytes;               // 128 KB
 constexpr int off_ssq = off_x + kXRing * kBoxBytes;              // [2 tiles][4 parts][128] floats
 constexpr int off_force = off_ssq + 2 * 4 * kTileRows * 4;       // [4][128] bytes
 constexpr int off_bars = off_force + 4 * kTileRows;
 enum { X_FULL = 0, X_EMPTY = 8, B_FULL = 16, B_EMPTY = 24, A_FULL = 32, A_EMPTY = 33, ACC_FULL = 34, ACC_EMPTY = 36, RHO_FULL = 38, ACC2_FULL = 40, N_BARS = 42 };
 constexpr int off_lut = off_bars + 512;                          // barriers, tensor-memory slot, give-up flag; then the cell table
-constexpr int off_rs = off_lut + 512;                            // |rho|^2 partial sums [4 column groups][128] (TurboQuantProd)
+constexpr int off_rs = off_lut + 512;                            // |rho|^2 partial sums [4 parts][128] (TurboQuantProd)
 constexpr int off_pend = off_rs + 4 * kTileRows * 4;
-constexpr int kPendBytes = kEpiWarps * kPendCap * (8 + 4) + kConvWarps * kPendCap * 4;   // epilogue warps: both lists; converters: rows
-constexpr int total = off_pend + kPendBytes + 1024;
+constexpr int total = off_pend + kWorkers * kPendCap * (8 + 4) + 1024;
 static_assert(total <= 227 * 1024, "shared memory plan");
 }  // namespace d256
 
-template <int BITS, bool PROD>
+template <int BITS, bool PROD, bool MAPPED>
 __global__ void __launch_bounds__(d256::kThreads, 1)
 tensor_quantize256_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorArgs a) {
     using namespace d256;
@@ -906,12 +915,12 @@ tensor_quantize256_kernel(const __grid_constant__ CUtensorMap tmap_x, const Tens
     if (threadIdx.x == 0) {
         for (int i = 0; i < kXRing; ++i) { mbar_init(BAR(X_FULL + i), 1); mbar_init(BAR(X_EMPTY + i), 4); }
         for (int i = 0; i < kBRing; ++i) { mbar_init(BAR(B_FULL + i), 1); mbar_init(BAR(B_EMPTY + i), 1); }
-        mbar_init(BAR(A_FULL), kConvWarps);
+        mbar_init(BAR(A_FULL), kWorkers);
         mbar_init(BAR(A_EMPTY), 1);
         for (int j = 0; j < 2; ++j) {
             mbar_init(BAR(ACC_FULL + j), 1);
-            mbar_init(BAR(ACC_EMPTY + j), PROD ? 1 : kEpiWarps);      // Prod: freed when the second contraction has read rho
-            mbar_init(BAR(RHO_FULL + j), kEpiWarps);
+            mbar_init(BAR(ACC_EMPTY + j), kWorkers);             // TurboQuantMSE (Prod: the next A_FULL says as much)
+            mbar_init(BAR(RHO_FULL + j), kWorkers);
             mbar_init(BAR(ACC2_FULL + j), 1);
         }
         abort_flag[0] = 0;
@@ -952,18 +961,20 @@ tensor_quantize256_kernel(const __grid_constant__ CUtensorMap tmap_x, const Tens
                     mbar_drain(BAR(X_FULL + (int)(gg % kXRing)), (uint32_t)((gg / kXRing) & 1));
         }
     } else if (warp == 2) {
-        // ---- rotation: one bulk copy per chunk, the same 32 chunks for every tile ------------------------
+        // ---- matrices: one bulk copy per chunk, the same chunks for every tile, in the order of the instructions ----
         if (lane == 0) {
             int64_t g = 0;
             bool ok = true;
             const unsigned char* src = reinterpret_cast<const unsigned char*>(a.bmat);
             for (int64_t i = 0; i < my_tiles && ok; ++i) {
-                for (int c = 0; c < (PROD ? 2 : 1) * kChunksPerMatrix; ++c, ++g) {
+                for (int c = 0; c < (PROD ? 64 : 32); c += kStep, ++g) {
                     const int slot = (int)(g % kBRing);
+                    // first contraction: (J, I, kb); second: (I, J, kb) of the 32 chunks behind
+                    const int chunk = c < 32 ? c : 32 + ((c & 8) << 1) + ((c & 16) >> 1) + (c & 7);
                     if (!mbar_wait(BAR(B_EMPTY + slot), (uint32_t)(((g / kBRing) & 1) ^ 1), abort_flag)) { ok = false; break; }
-                    mbar_arrive_expect_tx(BAR(B_FULL + slot), kChunkBytes);
+                    mbar_arrive_expect_tx(BAR(B_FULL + slot), kStepBytes);
                     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                                 ::"r"(smem_base + off_b + slot * kChunkBytes), "l"(src + (size_t)c * kChunkBytes), "r"(kChunkBytes),
+                                 ::"r"(smem_base + off_b + slot * kStepBytes), "l"(src + (size_t)chunk * kChunkBytes), "r"(kStepBytes),
                                    "r"(BAR(B_FULL + slot))
                                  : "memory");
                 }
@@ -976,31 +987,44 @@ tensor_quantize256_kernel(const __grid_constant__ CUtensorMap tmap_x, const Tens
         // ---- MMA issuer: the whole warp walks the loop, one elected lane issues -------------------------
         const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
         int64_t g = 0;
-        bool ok = true;
-        for (int64_t i = 0; i < my_tiles && ok; ++i) {
-            const uint32_t par = (uint32_t)(i & 1);
-            if (!warp_wait(BAR(A_FULL), par, abort_flag)) break;
-            for (int j = 0; j < 2 && ok; ++j) {
-                if (!warp_wait(BAR(ACC_EMPTY + j), par ^ 1u, abort_flag)) { ok = false; break; }
+        // eight chunks: acc (+)= A (hi | lo at lo_off, k-blocks of 16 values at k_col(kb)) * chunk; `done`: barrier to commit to, or -1
+        auto contract = [&](uint32_t acc, bool first, uint32_t a0, uint32_t lo_off, auto k_col, int done) {
+            for (int k0 = 0; k0 < 8; k0 += kStep, ++g) {
+                const int slot = (int)(g % kBRing);
+                if (!warp_wait(BAR(B_FULL + slot), (uint32_t)((g / kBRing) & 1), abort_flag)) return false;
                 tc_fence_after();
-                const uint32_t acc = tm + ACC_COL(j);
-                for (int c = 0; c < 16; ++c, ++g) {          // c = I * 8 + kb
-                    const int slot = (int)(g % kBRing);
-                    if (!warp_wait(BAR(B_FULL + slot), (uint32_t)((g / kBRing) & 1), abort_flag)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint32_t chunk = smem_base + off_b + slot * kChunkBytes;
-                    const uint64_t d_hi = make_smem_desc(chunk, 128, 256), d_lo = make_smem_desc(chunk + kChunkBytes / 2, 128, 256);
-                    const uint32_t a_hi = tm + A_COL(c >> 3) + (uint32_t)(c & 7) * 8, a_lo = a_hi + kABlock;
-                    if (elect_one()) {
-                        if (c == 0) mma_ts_first(acc, a_hi, d_hi, kIdesc);
+                const uint32_t stage = smem_base + off_b + slot * kStepBytes;
+                const uint64_t d0 = make_smem_desc(stage, 128, 256);
+                if (elect_one()) {
+#pragma unroll
+                    for (int u = 0; u < kStep; ++u) {
+                        // (the descriptor's address counts 16-byte units)
+                        const uint64_t d_hi = d0 + (uint64_t)(u * kChunkBytes >> 4), d_lo = d_hi + (uint64_t)(kChunkBytes / 2 >> 4);
+                        const uint32_t a_hi = a0 + k_col(k0 + u), a_lo = a_hi + lo_off;
+                        if (first && k0 + u == 0) mma_ts_first(acc, a_hi, d_hi, kIdesc);
                         else mma_ts_acc(acc, a_hi, d_hi, kIdesc);
                         mma_ts_acc(acc, a_hi, d_lo, kIdesc);
                         mma_ts_acc(acc, a_lo, d_hi, kIdesc);
-                        mma_commit(BAR(B_EMPTY + slot));
-                        if (c == 15) mma_commit(BAR(ACC_FULL + j));
                     }
-                    __syncwarp();
+                    mma_commit(BAR(B_EMPTY + slot));
+                    if (k0 + kStep == 8 && done >= 0) mma_commit(BAR(done));
                 }
+                __syncwarp();
+            }
+            return true;
+        };
+        auto unit_col = [](int kb) { return (uint32_t)kb * 8u; };
+        // rho of 32 coordinates: 16 columns of hi pairs, then 16 of lo pairs
+        auto rho_col = [](int kb) { return (uint32_t)(kb >> 1) * 32u + (uint32_t)(kb & 1) * 8u; };
+        for (int64_t i = 0; i < my_tiles; ++i) {
+            const uint32_t par = (uint32_t)(i & 1);
+            if (!warp_wait(BAR(A_FULL), par, abort_flag)) break;
+            bool ok = true;
+            for (int j = 0; j < 2 && ok; ++j) {
+                if (!PROD && !warp_wait(BAR(ACC_EMPTY + j), par ^ 1u, abort_flag)) { ok = false; break; }
+                tc_fence_after();
+                ok = contract(tm + ACC_COL(j), true, tm + A_COL(0), kABlock, unit_col, -1) &&
+                     contract(tm + ACC_COL(j), false, tm + A_COL(1), kABlock, unit_col, ACC_FULL + j);
             }
             if (!ok) break;
             if (!PROD) {
@@ -1008,162 +1032,21 @@ tensor_quantize256_kernel(const __grid_constant__ CUtensorMap tmap_x, const Tens
                 __syncwarp();
                 continue;
             }
-            // TurboQuantProd: rho (split, in place of the accumulators: K half I in accumulator block I) times the chunks of
-            // 16 (R S^T); output half J goes to operand block J, which the first contraction has finished reading.
-            if (!warp_wait(BAR(RHO_FULL + 0), par, abort_flag) || !warp_wait(BAR(RHO_FULL + 1), par, abort_flag)) break;
-            tc_fence_after();
-            for (int j = 0; j < 2 && ok; ++j) {
-                const uint32_t acc2 = tm + A_COL(j);
-                for (int c = 0; c < 16; ++c, ++g) {
-                    const int slot = (int)(g % kBRing);
-                    if (!warp_wait(BAR(B_FULL + slot), (uint32_t)((g / kBRing) & 1), abort_flag)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint32_t chunk = smem_base + off_b + slot * kChunkBytes;
-                    const uint64_t d_hi = make_smem_desc(chunk, 128, 256), d_lo = make_smem_desc(chunk + kChunkBytes / 2, 128, 256);
-                    const int kb = c & 7;
-                    // rho of 32 coordinates: 16 columns of hi pairs, then 16 of lo pairs
-                    const uint32_t r_hi = tm + ACC_COL(c >> 3) + (uint32_t)(kb >> 1) * 32 + (uint32_t)(kb & 1) * 8, r_lo = r_hi + 16;
-                    if (elect_one()) {
-                        if (c == 0) mma_ts_first(acc2, r_hi, d_hi, kIdesc);
-                        else mma_ts_acc(acc2, r_hi, d_hi, kIdesc);
-                        mma_ts_acc(acc2, r_hi, d_lo, kIdesc);
-                        mma_ts_acc(acc2, r_lo, d_hi, kIdesc);
-                        mma_commit(BAR(B_EMPTY + slot));
-                        if (c == 15) mma_commit(BAR(ACC2_FULL + j));
-                    }
-                    __syncwarp();
-                }
+            // the second accumulators go to the operand blocks, once the first contraction has read them
+            if (!warp_wait(BAR(ACC_FULL + 1), par, abort_flag)) break;
+            for (int h = 0; h < 2 && ok; ++h) {
+                if (!warp_wait(BAR(RHO_FULL + h), par, abort_flag)) { ok = false; break; }
+                tc_fence_after();
+                for (int j = 0; j < 2 && ok; ++j)
+                    ok = contract(tm + A_COL(j), h == 0, tm + ACC_COL(h), 16, rho_col, h == 1 ? ACC2_FULL + j : -1);
             }
             if (!ok) break;
-            if (elect_one()) { mma_commit(BAR(ACC_EMPTY + 0)); mma_commit(BAR(ACC_EMPTY + 1)); }   // rho has been read
-            __syncwarp();
         }
-    } else if (warp < kFirstEpi) {
-        // ---- converters: one thread per quarter row (64 values, two boxes) -------------------------------
-        const int cw = warp - kFirstConv;
+    } else {
+        // ---- workers: four threads per row, one per quarter of the columns ---------------------------------
+        const int cw = warp - kFirstWorker;
         const int part = cw >> 2;
         const int quarter = warp & 3;
-        const int row = quarter * 32 + lane;
-        const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
-        WarpPending cpend;           // rows for the exact stage found by the sign epilogue
-        cpend.codes = nullptr;
-        cpend.rows = reinterpret_cast<unsigned int*>(pend_base + kEpiWarps * kPendCap * 12) + cw * kPendCap;
-        cpend.n_codes = 0;
-        cpend.n_rows = 0;
-        for (int64_t i = 0; i < my_tiles; ++i) {
-            const int64_t tile = blockIdx.x + i * gridDim.x;
-            const uint32_t par = (uint32_t)(i & 1);
-            float x[64];
-            bool fail = false;
-#pragma unroll
-            for (int bb = 0; bb < 2; ++bb) {
-                const int64_t g = i * kBoxesPerTile + part * 2 + bb;
-                const int slot = (int)(g % kXRing);
-                if (!fail && !mbar_wait(BAR(X_FULL + slot), (uint32_t)((g / kXRing) & 1), abort_flag)) fail = true;
-                const unsigned char* box = smem + off_x + slot * kBoxBytes + row * 128;
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    const float4 v = fail ? make_float4(0.f, 0.f, 0.f, 0.f) : lds_once_f4(box + ((c ^ (row & 7)) << 4));
-                    x[bb * 32 + c * 4 + 0] = v.x;
-                    x[bb * 32 + c * 4 + 1] = v.y;
-                    x[bb * 32 + c * 4 + 2] = v.z;
-                    x[bb * 32 + c * 4 + 3] = v.w;
-                }
-                __threadfence_block();   // every lane's loads from the stage are performed before the stage is released
-                __syncwarp();
-                if (lane == 0 && !fail) mbar_arrive(BAR(X_EMPTY + slot));
-            }
-            float s4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int k = 0; k < 64; ++k) s4[k & 3] = fmaf(x[k], x[k], s4[k & 3]);
-            float* ssq = ssq_all + (int)par * 4 * kTileRows;     // by tile parity: a fast warp may write the next tile's sums early
-            ssq[part * kTileRows + row] = (s4[0] + s4[1]) + (s4[2] + s4[3]);
-            bar_sync(1 + quarter, 128);                           // the four warps that share these 32 rows
-            const float tot = (ssq[row] + ssq[kTileRows + row]) + (ssq[2 * kTileRows + row] + ssq[3 * kTileRows + row]);
-            const float nrm = sqrtf(tot);
-            const bool okn = nrm > 0.f;
-            const bool odd = !(tot < 3.0e38f) || (okn && tot < 1.0e-30f);   // rows for the exact kernel: overflowed or denormal-range norms
-            const float sc = (okn && !odd) ? kScaleA / nrm : 0.f;
-            if (part == 0) {
-                const int64_t grow = tile * kTileRows + row;
-                if (grow < a.n && !fail) a.norms[output_row(a, grow)] = nrm;
-                force[(i & 3) * kTileRows + row] = odd ? 1 : 0;
-            }
-            // TurboQuantProd: this thread itself was the last reader of its cells (sign epilogue of the previous tile, below)
-            if (!PROD && !mbar_wait(BAR(A_EMPTY), par ^ 1u, abort_flag)) fail = true;
-            tc_fence_after();
-            const uint32_t a_hi = tmem + lane_addr + A_COL(part >> 1) + (uint32_t)(part & 1) * 32;
-#pragma unroll
-            for (int s = 0; s < 2; ++s) {
-                uint32_t hi[16], lo[16];
-#pragma unroll
-                for (int p = 0; p < 16; ++p) {
-                    const float u0 = x[s * 32 + 2 * p] * sc, u1 = x[s * 32 + 2 * p + 1] * sc;
-                    const __half2 h = __floats2half2_rn(u0, u1);
-                    const float2 hf = __half22float2(h);
-                    hi[p] = *reinterpret_cast<const uint32_t*>(&h);
-                    lo[p] = pack_half2(u0 - hf.x, u1 - hf.y);
-                }
-                tmem_st16(a_hi + s * 16, hi);
-                tmem_st16(a_hi + kABlock + s * 16, lo);
-            }
-            tmem_wait_st();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(BAR(A_FULL));
-            if (PROD) {
-                // ---- sign epilogue of the same tile: the second accumulator of output half J sits in operand block J.  A
-                // thread reads exactly the cells it fills again for the next tile (columns [32 h, 32 h + 32) and
-                // [64 + 32 h, 64 + 32 h + 32) with h = part & 1: two sign words of the row), so no other warp's
-                // progress matters to it.
-                const int j = part >> 1, hcol = part & 1;
-                const int64_t grow = tile * kTileRows + row;
-                bool redo_row = part == 0 && force[(i & 3) * kTileRows + row] != 0;
-                const bool live = mbar_wait(BAR(ACC2_FULL + j), par, abort_flag) && grow < a.n;   // no stores after a give-up
-                tc_fence_after();
-                if (part == 0 && live) {      // |rho|^2 in 2^10 units: the four partial sums of the first epilogue
-                    const float rs_all = (rs_part[row] + rs_part[kTileRows + row]) + (rs_part[2 * kTileRows + row] + rs_part[3 * kTileRows + row]);
-                    a.rnorms[output_row(a, grow)] = sqrtf(rs_all) * kScaleRho;
-                }
-                const uint32_t acc2 = tmem + lane_addr + A_COL(j);
-                uint32_t sw[2] = {0u, 0u};
-#pragma unroll 1
-                for (int ch = 0; ch < 2; ++ch) {
-                    uint32_t va[32];
-                    tmem_ld32(acc2 + (hcol + 2 * ch) * 32, va);
-                    tmem_wait_ld();
-                    uint32_t wd[4] = {0u, 0u, 0u, 0u};
-                    float am[4] = {3.0e38f, 3.0e38f, 3.0e38f, 3.0e38f};
-#pragma unroll
-                    for (int k = 7; k >= 0; --k) {
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) wd[c] = __funnelshift_l(va[(c >> 1) * 16 + 2 * k + (c & 1)], wd[c], 1);
-                    }
-#pragma unroll
-                    for (int e = 0; e < 32; e += 8) {
-#pragma unroll
-                        for (int c = 0; c < 4; ++c)
-                            am[c] = min3_abs(am[c], __uint_as_float(va[e + 2 * c]), __uint_as_float(va[e + 2 * c + 1]));
-                    }
-                    const uint32_t word = ~((wd[0] | (wd[2] << 8)) | ((wd[1] | (wd[3] << 8)) << 16));
-                    if (ch == 0) sw[0] = word; else sw[1] = word;
-                    redo_row = redo_row || (fminf(fminf(am[0], am[1]), fminf(am[2], am[3])) < a.sign_guard);
-                }
-                tc_fence_before();
-                if (live) {
-                    const int64_t orow = output_row(a, grow);
-                    a.signs[orow * (kD / 32) + j * 4 + hcol] = sw[0];
-                    a.signs[orow * (kD / 32) + j * 4 + 2 + hcol] = sw[1];
-                }
-                pend_rows(a.lists, cpend, redo_row && live, grow, lane);
-            }
-        }
-        if (PROD && cpend.n_rows > 0) flush_pending_rows(a.lists, cpend, lane);
-    } else {
-        // ---- epilogue: two threads per row, 64 columns of each output half -------------------------------
-        const int ew = warp - kFirstEpi;
-        const int quarter = warp & 3;
-        const int colgroup = ew >> 2;
         const int row = quarter * 32 + lane;
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
         constexpr int kCodeWords = kD * BITS / 32;
@@ -1171,61 +1054,175 @@ tensor_quantize256_kernel(const __grid_constant__ CUtensorMap tmap_x, const Tens
         const int lut_base1 = __float_as_int(cell_lut[lane].y);
         const float lut_ncent = PROD ? a.code_ncent[lane] : 0.f;
         WarpPending pend;
-        pend.codes = reinterpret_cast<unsigned long long*>(pend_base) + ew * kPendCap;
-        pend.rows = reinterpret_cast<unsigned int*>(pend_base + kEpiWarps * kPendCap * 8) + ew * kPendCap;
+        pend.codes = reinterpret_cast<unsigned long long*>(pend_base) + cw * kPendCap;
+        pend.rows = reinterpret_cast<unsigned int*>(pend_base + kWorkers * kPendCap * 8) + cw * kPendCap;
         pend.n_codes = 0;
         pend.n_rows = 0;
-        for (int64_t i = 0; i < my_tiles; ++i) {
-            const int64_t tile = blockIdx.x + i * gridDim.x;
-            const uint32_t par = (uint32_t)(i & 1);
-            const int64_t grow = tile * kTileRows + row, orow = output_row(a, grow);
-#pragma unroll 1
-            for (int j = 0; j < 2; ++j) {
-                const bool got = mbar_wait(BAR(ACC_FULL + j), par, abort_flag);
-                const bool live = got && grow < a.n;
-                const bool redo_row = force[(i & 3) * kTileRows + row] != 0;   // written before this tile's A_FULL, which precedes ACC_FULL
-                tc_fence_after();
-                const uint32_t acc = tmem + lane_addr + ACC_COL(j);
-                uint32_t nm0 = 0, nm1 = 0;
-                float rs = 0.f;
-#pragma unroll 1
-                for (int ch = 0; ch < 2; ++ch) {
-                    const int chunk = colgroup * 2 + ch;                 // 32-column chunk of this output half
-                    uint32_t va[32];
-                    tmem_ld32(acc + chunk * 32, va);
-                    tmem_wait_ld();
-                    uint32_t w[BITS + 1], rhi[16], rlo[16];
-                    const uint32_t m = process_chunk<BITS, PROD>(va, lut_bnd, lut_base1, lut_ncent, a.cell_scale, a.cell_offset, a.code_guard, w, rhi, rlo, rs);
-                    if (ch == 0) nm0 = m; else nm1 = m;
-                    if (PROD) {      // rho replaces the chunk it was computed from: 16 columns of hi pairs, 16 of lo pairs
-                        tmem_st16(acc + chunk * 32, rhi);
-                        tmem_st16(acc + chunk * 32 + 16, rlo);
-                    }
-                    if (live) {
-                        uint32_t* dst = a.codes + orow * kCodeWords + (j * 4 + chunk) * BITS;
-                        if (BITS == 4) *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
-                        else if (BITS == 2) *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
-                        else {
+        bool fail = false;
+        float scale = 0.f;          // of the tile whose norm was computed last
+        // 64 columns [64 part, + 64) of the row: boxes 2 part and 2 part + 1, in the slots of the same numbers
+        const unsigned char* x0 = smem + off_x + part * 2 * kBoxBytes + row * 128;
+        static_assert(kXRing == kBoxesPerTile, "a box has the slot of its number");
+
+        // -- norm of the rows of tile i, which stay in shared memory
+        auto norm = [&](int64_t i) {
+            float s4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                            for (int k = 0; k < BITS; ++k) dst[k] = w[k];
-                        }
-                    }
+            for (int bb = 0; bb < 2; ++bb) {
+                if (!fail && !mbar_wait(BAR(X_FULL + part * 2 + bb), (uint32_t)(i & 1), abort_flag)) fail = true;
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    const float4 v = fail ? make_float4(0.f, 0.f, 0.f, 0.f) : lds_once_f4(x0 + bb * kBoxBytes + ((c ^ (row & 7)) << 4));
+                    s4[0] = fmaf(v.x, v.x, s4[0]);
+                    s4[1] = fmaf(v.y, v.y, s4[1]);
+                    s4[2] = fmaf(v.z, v.z, s4[2]);
+                    s4[3] = fmaf(v.w, v.w, s4[3]);
                 }
-                if (PROD) {
-                    tmem_wait_st();
-                    // this thread's share of |rho|^2; one tile is in flight per block, and the sign epilogue that reads the
-                    // sums comes after the second contraction, which waits for every epilogue warp's arrival below
-                    rs_part[(j * 2 + colgroup) * kTileRows + row] = rs;
+            }
+            float* ssq = ssq_all + (int)(i & 1) * 4 * kTileRows;     // by tile parity: a fast warp may write the next tile's sums early
+            ssq[part * kTileRows + row] = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+            bar_sync(1 + quarter, 128);                           // the four warps that share these 32 rows
+            const float tot = (ssq[row] + ssq[kTileRows + row]) + (ssq[2 * kTileRows + row] + ssq[3 * kTileRows + row]);
+            const float nrm = sqrtf(tot);
+            const bool okn = nrm > 0.f;
+            const bool odd = !(tot < 3.0e38f) || (okn && tot < 1.0e-30f);   // rows for the exact kernel: overflowed or denormal-range norms
+            scale = (okn && !odd) ? kScaleA / nrm : 0.f;
+            if (part == 0) {
+                const int64_t grow = (blockIdx.x + i * gridDim.x) * kTileRows + row;
+                if (grow < a.n && !fail) a.norms[output_row<MAPPED>(a, grow)] = nrm;
+                force[(i & 3) * kTileRows + row] = odd ? 1 : 0;
+            }
+        };
+        // -- tile i into the operand blocks.  TurboQuantProd: the cells a thread fills are those it read as sign epilogue of
+        // the tile before, so no other warp's progress matters to it.
+        auto convert = [&](int64_t i) {
+            if (!PROD && !mbar_wait(BAR(A_EMPTY), (uint32_t)(i & 1) ^ 1u, abort_flag)) fail = true;
+            tc_fence_after();
+            const uint32_t a_hi = tmem + lane_addr + A_COL(part >> 1) + (uint32_t)(part & 1) * 32;
+#pragma unroll 1
+            for (int bb = 0; bb < 2; ++bb) {
+                uint32_t hi[16], lo[16];
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    const float4 v = fail ? make_float4(0.f, 0.f, 0.f, 0.f) : lds_once_f4(x0 + bb * kBoxBytes + ((c ^ (row & 7)) << 4));
+                    const float u0 = v.x * scale, u1 = v.y * scale, u2 = v.z * scale, u3 = v.w * scale;
+                    const __half2 h0 = __floats2half2_rn(u0, u1), h1 = __floats2half2_rn(u2, u3);
+                    const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
+                    hi[2 * c] = *reinterpret_cast<const uint32_t*>(&h0);
+                    hi[2 * c + 1] = *reinterpret_cast<const uint32_t*>(&h1);
+                    lo[2 * c] = pack_half2(u0 - f0.x, u1 - f0.y);
+                    lo[2 * c + 1] = pack_half2(u2 - f1.x, u3 - f1.y);
                 }
+                tmem_st16(a_hi + bb * 16, hi);
+                tmem_st16(a_hi + kABlock + bb * 16, lo);
+            }
+            tmem_wait_st();
+            tc_fence_before();
+            __threadfence_block();   // every lane's loads from the stages are performed before the stages are released
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(BAR(A_FULL));
+                if (!fail) { mbar_arrive(BAR(X_EMPTY + part * 2)); mbar_arrive(BAR(X_EMPTY + part * 2 + 1)); }
+            }
+        };
+        float rs = 0.f;
+        // -- columns [32 part, + 32) of output half j of tile i: codes, for TurboQuantProd rho in their place
+        auto epilogue = [&](int64_t i, int j) {
+            const int64_t grow = (blockIdx.x + i * gridDim.x) * kTileRows + row;
+            const bool live = mbar_wait(BAR(ACC_FULL + j), (uint32_t)(i & 1), abort_flag) && grow < a.n;
+            const bool redo_row = force[(i & 3) * kTileRows + row] != 0;   // written before this tile's A_FULL, which precedes ACC_FULL
+            tc_fence_after();
+            const uint32_t acc = tmem + lane_addr + ACC_COL(j) + part * 32;
+            uint32_t va[32], w[BITS + 1], rhi[16], rlo[16];
+            tmem_ld32(acc, va);
+            tmem_wait_ld();
+            if (!PROD) {
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(BAR(PROD ? RHO_FULL + j : ACC_EMPTY + j));
-                if (!live || redo_row) { nm0 = 0; nm1 = 0; }
-                if (__any_sync(0xffffffffu, (nm0 | nm1) != 0u)) {
-                    pend_codes(a.lists, pend, nm0, grow, j * 128 + (colgroup * 2) * 32, lane);
-                    pend_codes(a.lists, pend, nm1, grow, j * 128 + (colgroup * 2 + 1) * 32, lane);
+                if (lane == 0) mbar_arrive(BAR(ACC_EMPTY + j));
+            }
+            uint32_t nm = process_chunk<BITS, PROD>(va, lut_bnd, lut_base1, lut_ncent, a.cell_scale, a.cell_offset, a.code_guard, w, rhi, rlo, rs);
+            if (PROD) {      // rho replaces the chunk it was computed from: 16 columns of hi pairs, 16 of lo pairs
+                tmem_st16(acc, rhi);
+                tmem_st16(acc + 16, rlo);
+                tmem_wait_st();
+                // this thread's share of |rho|^2: read by the sign epilogue, which the second contraction, and so every
+                // warp's arrival below, comes before; written again after the next A_FULL, which the sign epilogue comes before
+                if (j == 1) rs_part[part * kTileRows + row] = rs;
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(BAR(RHO_FULL + j));
+            }
+            if (live) {
+                uint32_t* dst = a.codes + output_row<MAPPED>(a, grow) * kCodeWords + (j * 4 + part) * BITS;
+                if (BITS == 4) *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+                else if (BITS == 2) *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
+                else {
+#pragma unroll
+                    for (int k = 0; k < BITS; ++k) dst[k] = w[k];
                 }
-                if (!PROD && j == 0) pend_rows(a.lists, pend, redo_row && live && colgroup == 0, grow, lane);
+            }
+            if (!live || redo_row) nm = 0;
+            if (__any_sync(0xffffffffu, nm != 0u)) pend_codes(a.lists, pend, nm, grow, j * 128 + part * 32, lane);
+            if (!PROD && j == 0) pend_rows(a.lists, pend, redo_row && live && part == 0, grow, lane);
+        };
+        // -- TurboQuantProd: second accumulator of output half part >> 1 -> two sign words of the row, from the cells that this
+        // thread fills again for the next tile (columns [32 h, + 32) and [64 + 32 h, + 32) with h = part & 1)
+        auto sign_epilogue = [&](int64_t i) {
+            const int j = part >> 1, hcol = part & 1;
+            const int64_t grow = (blockIdx.x + i * gridDim.x) * kTileRows + row, orow = output_row<MAPPED>(a, grow);
+            bool redo_row = part == 0 && force[(i & 3) * kTileRows + row] != 0;
+            const bool live = mbar_wait(BAR(ACC2_FULL + j), (uint32_t)(i & 1), abort_flag) && grow < a.n;   // no stores after a give-up
+            tc_fence_after();
+            if (part == 0 && live) {      // |rho|^2 in 2^10 units
+                const float rs_all = (rs_part[row] + rs_part[kTileRows + row]) + (rs_part[2 * kTileRows + row] + rs_part[3 * kTileRows + row]);
+                a.rnorms[orow] = sqrtf(rs_all) * kScaleRho;
+            }
+            const uint32_t acc2 = tmem + lane_addr + A_COL(j);
+#pragma unroll 1
+            for (int ch = 0; ch < 2; ++ch) {
+                uint32_t va[32];
+                tmem_ld32(acc2 + (hcol + 2 * ch) * 32, va);
+                tmem_wait_ld();
+                uint32_t wd[4] = {0u, 0u, 0u, 0u};
+                float am[4] = {3.0e38f, 3.0e38f, 3.0e38f, 3.0e38f};
+#pragma unroll
+                for (int k = 7; k >= 0; --k) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) wd[c] = __funnelshift_l(va[(c >> 1) * 16 + 2 * k + (c & 1)], wd[c], 1);
+                }
+#pragma unroll
+                for (int e = 0; e < 32; e += 8) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        am[c] = min3_abs(am[c], __uint_as_float(va[e + 2 * c]), __uint_as_float(va[e + 2 * c + 1]));
+                }
+                const uint32_t word = ~((wd[0] | (wd[2] << 8)) | ((wd[1] | (wd[3] << 8)) << 16));
+                redo_row = redo_row || (fminf(fminf(am[0], am[1]), fminf(am[2], am[3])) < a.sign_guard);
+                if (live) a.signs[orow * (kD / 32) + j * 4 + 2 * ch + hcol] = word;
+            }
+            tc_fence_before();
+            pend_rows(a.lists, pend, redo_row && live, grow, lane);
+        };
+
+        if (my_tiles > 0) norm(0);
+        if (PROD) {
+            for (int64_t i = 0; i < my_tiles; ++i) {
+                convert(i);
+                rs = 0.f;
+#pragma unroll 1
+                for (int j = 0; j < 2; ++j) epilogue(i, j);
+                if (i + 1 < my_tiles) norm(i + 1);
+                sign_epilogue(i);
+            }
+        } else {
+            for (int64_t i = 0; i <= my_tiles && my_tiles > 0; ++i) {
+                if (i < my_tiles) convert(i);
+#pragma unroll 1
+                for (int s = 0; s < 2; ++s) {          // J = 1 of the tile before, then J = 0 of this one
+                    if (s == 1 && i + 1 < my_tiles) norm(i + 1);
+                    if (s == 0 ? i > 0 : i < my_tiles) epilogue(i - 1 + s, 1 - s);
+                }
             }
         }
         if (pend.n_codes > 0) flush_pending_codes(a.lists, pend, lane);
@@ -1451,27 +1448,34 @@ void tq_tensor_plan_free(tq_plan* p) {
 #ifndef TQ_UNI_MSE
 #define TQ_UNI_MSE false
 #endif
-template <int D, int BITS, bool PROD, bool HALF>
+template <int D, int BITS, bool PROD, bool HALF, bool MAPPED>
 static int launch_type(const tq_plan* p, const CUtensorMap& map, const TensorArgs& args, int grid, cudaStream_t st) {
     constexpr bool UNI = PROD ? TQ_UNI_PROD : TQ_UNI_MSE;
     const int sm = Smem<D, PROD, UNI>::total;
-    TQ_GRANT_SMEM((tensor_quantize_kernel<D, BITS, PROD, UNI, HALF>), sm, p->device);
-    tensor_quantize_kernel<D, BITS, PROD, UNI, HALF><<<grid, Threads<PROD, UNI>::kThreads, sm, st>>>(map, args); tq_count_launch();
+    TQ_GRANT_SMEM((tensor_quantize_kernel<D, BITS, PROD, UNI, HALF, MAPPED>), sm, p->device);
+    tensor_quantize_kernel<D, BITS, PROD, UNI, HALF, MAPPED><<<grid, Threads<PROD, UNI>::kThreads, sm, st>>>(map, args); tq_count_launch();
     TQ_CUDA_TRY(cudaGetLastError());
     return TQ_OK;
 }
 
 template <int D, int BITS, bool PROD>
 static int launch_one(const tq_plan* p, const CUtensorMap& map, const TensorArgs& args, bool half, int grid, cudaStream_t st) {
-    return half ? launch_type<D, BITS, PROD, true>(p, map, args, grid, st) : launch_type<D, BITS, PROD, false>(p, map, args, grid, st);
+    // (16-bit rows come from caches only)
+    if (half) return launch_type<D, BITS, PROD, true, true>(p, map, args, grid, st);
+    return args.tokens ? launch_type<D, BITS, PROD, false, true>(p, map, args, grid, st) : launch_type<D, BITS, PROD, false, false>(p, map, args, grid, st);
+}
+
+template <int BITS, bool PROD, bool MAPPED>
+static int launch_256_rows(const tq_plan* p, const CUtensorMap& map, const TensorArgs& args, int grid, cudaStream_t st) {
+    TQ_GRANT_SMEM((tensor_quantize256_kernel<BITS, PROD, MAPPED>), d256::total, p->device);
+    tensor_quantize256_kernel<BITS, PROD, MAPPED><<<grid, d256::kThreads, d256::total, st>>>(map, args); tq_count_launch();
+    TQ_CUDA_TRY(cudaGetLastError());
+    return TQ_OK;
 }
 
 template <int BITS, bool PROD>
 static int launch_256(const tq_plan* p, const CUtensorMap& map, const TensorArgs& args, int grid, cudaStream_t st) {
-    TQ_GRANT_SMEM((tensor_quantize256_kernel<BITS, PROD>), d256::total, p->device);
-    tensor_quantize256_kernel<BITS, PROD><<<grid, d256::kThreads, d256::total, st>>>(map, args); tq_count_launch();
-    TQ_CUDA_TRY(cudaGetLastError());
-    return TQ_OK;
+    return args.tokens ? launch_256_rows<BITS, PROD, true>(p, map, args, grid, st) : launch_256_rows<BITS, PROD, false>(p, map, args, grid, st);
 }
 
 // The kernels that read 16-bit rows are those for d = 64 and 128.
@@ -1483,6 +1487,7 @@ int tq_launch_tensor_quantize(const tq_plan* p, bool prod, const void* x, int xt
     if (!p->tensor) return tq_fail(TQ_ERR_UNSUPPORTED, "no tensor-core kernel for this plan");
     const int d = p->dev.d;
     const bool half = xtype != TQ_INPUT_F32;
+    if (half && out.map.tokens == 0) return tq_fail(TQ_ERR_UNSUPPORTED, "16-bit rows are quantized into caches only");
     if (n > (int64_t)0x7fffff00) return tq_fail(TQ_ERR_UNSUPPORTED, "n above 2^31 rows per call");
     TensorArgs args = p->tensor->args;
     args.n = n;
