@@ -17,8 +17,7 @@
 //                          successive tiles)
 //   MMA (1 thread)         operand by operand: C_hi x (Rt_hi, Rt_lo), C_lo x Rt_hi [, B_hi x (St_hi, St_lo),
 //                          B_lo x St_hi], N = 128, accumulators double-buffered
-//   epilogue (8 warps)     two threads per key: tcgen05.ld, times norm * 2^-20, then through a staging block in
-//                          shared memory so that every global store instruction writes whole 128-byte lines
+//   epilogue (8 warps)     two threads per key: tcgen05.ld, times norm * 2^-20, then through shared memory and tensor stores
 //
 // Every wait is bounded; a wait that runs out sets the plan's status word and the kernel drains.
 #include "tq_common.cuh"
@@ -77,6 +76,46 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
                  : "memory");
 }
 
+// Reconstructed rows leave through shared memory: an epilogue warp writes 32 x 32 floats (row = lane, 16-byte pieces swizzled by
+// the row as the tensor map says, so that no two lanes of a store meet in a bank) and one lane starts a tensor store, which
+// clips the rows behind the last.  (Loading the block back and storing it with the warp's own instructions made the epilogue the
+// longest role: 3,200 cycles a block.)
+constexpr int kBlockBytes = 32 * 128;
+template <int BUFS>
+struct BlockStore {
+    unsigned char* stage;
+    int next;          // buffer of the next block
+    __device__ __forceinline__ unsigned char* open(int lane) {
+        // all but the newest BUFS - 1 stores have left their buffers
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(BUFS - 1) : "memory");
+        __syncwarp();
+        return stage + next * kBlockBytes;
+    }
+    __device__ __forceinline__ void write(const uint32_t (&v)[32], float sc, int lane) {
+        unsigned char* mine = open(lane) + lane * 128;
+#pragma unroll
+        for (int m = 0; m < 8; ++m)
+            *reinterpret_cast<float4*>(mine + ((m ^ (lane & 7)) << 4)) =
+                make_float4(__uint_as_float(v[4 * m]) * sc, __uint_as_float(v[4 * m + 1]) * sc, __uint_as_float(v[4 * m + 2]) * sc,
+                            __uint_as_float(v[4 * m + 3]) * sc);
+        fence_async_smem();
+        __syncwarp();
+    }
+    __device__ __forceinline__ void send(const CUtensorMap* map, int col, int64_t row, bool live, int lane) {
+        if (lane == 0) {
+            if (live)
+                asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
+                             ::"l"(map), "r"(smem_u32(stage + next * kBlockBytes)), "r"(col), "r"((int)row)
+                             : "memory");
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+        next = next + 1 == BUFS ? 0 : next + 1;
+    }
+    __device__ __forceinline__ void close(int lane) {
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    }
+};
+
 __device__ __forceinline__ void tmem_ld32_(uint32_t taddr, uint32_t (&v)[32]) { tmem_ld32(taddr, v); }
 
 template <int BITS, bool PROD, int DR>
@@ -88,16 +127,20 @@ struct DqSmem {
     static constexpr int kRowExtra = PROD ? kSignRowBytes : 0;   // sign words
     static constexpr int kStageBytes = kTileKeys * (kCodeRowBytes + kRowExtra);
     static constexpr int kNumB = PROD ? 4 : 2;
-    static constexpr int kStages = PROD ? 4 : 6;
-    static constexpr int kOutRowBytes = 36 * 4;                   // 32 floats of a row + padding against bank conflicts
-    static constexpr int kOutWarpBytes = 32 * kOutRowBytes;       // staging block of one epilogue warp
-    static constexpr int off_lut = 0;
+    static constexpr int kOutBufs = 2;                            // 4 KB blocks per epilogue warp
+    static constexpr int kOutRowBytes = 36 * 4;                   // pair mode: 32 floats of a row + padding against bank conflicts
+    static constexpr int kOutWarpBytes = kOutBufs * kBlockBytes;  // staging of one epilogue warp (a pair-mode block fits)
+    static constexpr int off_out = 0;                             // (the swizzle wants blocks on 1 KB boundaries)
+    static constexpr int off_lut = off_out + 8 * kOutWarpBytes;
     static constexpr int off_b = off_lut + kLutBytes;
     static constexpr int off_ring = off_b + kNumB * kMatBytes;
-    static constexpr int off_out = off_ring + kStages * kStageBytes;
-    static constexpr int off_misc = off_out + 8 * kOutWarpBytes;
-    static constexpr int off_pair = off_misc + 512 + 128;           // pair mode: partial dot products [2 tiles][128]
-    static constexpr int total = off_pair + 2 * kTileKeys * 4;
+    static constexpr int kMisc = 512 + 128 + 2 * kTileKeys * 4;   // barriers; pair mode: partial dot products [2 tiles][128]
+    static constexpr int kStageRoom = (227 * 1024 - 1024 - off_ring - kMisc) / kStageBytes;
+    static constexpr int kStages = kStageRoom < 6 ? kStageRoom : 6;
+    static_assert(kStages >= 2, "shared memory plan");
+    static constexpr int off_misc = off_ring + kStages * kStageBytes;
+    static constexpr int off_pair = off_misc + 512 + 128;
+    static constexpr int total = off_misc + kMisc + 1024;         // + slack to align the base
     static_assert(total <= 227 * 1024, "shared memory plan");
 };
 
@@ -105,7 +148,7 @@ struct DqSmem {
 // index and summed: attention_score with one query per key (_quant.py:342-358), which equals q . dequantize(key).
 template <int BITS, bool PROD, int DR, bool PAIR>
 __global__ void __launch_bounds__(kThreads, 1)
-dequant_tc_kernel(const DequantArgs a) {
+dequant_tc_kernel(const __grid_constant__ CUtensorMap tmap_out, const DequantArgs a) {
     static_assert(DR == 128 || DR == 64, "written for d = 128 and d = 64");
     // d = 64: the expander warps and the epilogue warps of the upper half idle, the contractions stop after
     // DR / 16 k-blocks and cover N = DR output coordinates
@@ -114,7 +157,7 @@ dequant_tc_kernel(const DequantArgs a) {
     constexpr int kStages = L::kStages;
     constexpr int kOps = PROD ? 4 : 2;   // operands per tile: C_hi, C_lo [, B_hi, B_lo]
     extern __shared__ unsigned char smem_raw[];
-    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const uint32_t smem_base = smem_u32(smem);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::off_misc);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + DB_COUNT);
@@ -341,6 +384,7 @@ dequant_tc_kernel(const DequantArgs a) {
         const int row = quarter * 32 + lane;
         const int colhalf = (warp - kFirstEpiWarp) >> 2;
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
+        BlockStore<L::kOutBufs> store{smem + L::off_out + (warp - kFirstEpiWarp) * L::kOutWarpBytes, 0};
         float nrm_next = 0.f;
         if (my_tiles > 0) {
             const int64_t r0 = (int64_t)blockIdx.x * kTileKeys + row;
@@ -414,28 +458,12 @@ dequant_tc_kernel(const DequantArgs a) {
                 if (colhalf == 0 && grow < n_live) a.out[grow] = dot * sc;
                 continue;
             }
-            // Through a per-warp staging block in shared memory, so that the global stores of a warp cover
-            // whole 128-byte lines (four rows x 32 floats per instruction) instead of 16 bytes of 32 rows.
-#pragma unroll
-            for (int ch = 0; ch < 2; ++ch) {
-                float4* mine = reinterpret_cast<float4*>(stg + lane * L::kOutRowBytes);
-#pragma unroll
-                for (int m = 0; m < 8; ++m) {
-                    const uint32_t* v = ch == 0 ? va : vb;
-                    mine[m] = make_float4(__uint_as_float(v[4 * m]) * sc, __uint_as_float(v[4 * m + 1]) * sc,
-                                          __uint_as_float(v[4 * m + 2]) * sc, __uint_as_float(v[4 * m + 3]) * sc);
-                }
-                __syncwarp();
-#pragma unroll
-                for (int it = 0; it < 8; ++it) {
-                    const int r = it * 4 + (lane >> 3), c4 = lane & 7;
-                    const float4 val = *reinterpret_cast<const float4*>(stg + r * L::kOutRowBytes + c4 * 16);
-                    if (row0 + r < n_live)
-                        __stcs(reinterpret_cast<float4*>(a.out + (row0 + r) * DR + colhalf * 64 + ch * 32) + c4, val);
-                }
-                __syncwarp();
-            }
+            store.write(va, sc, lane);
+            store.send(&tmap_out, colhalf * 64, row0, row0 < n_live, lane);
+            store.write(vb, sc, lane);
+            store.send(&tmap_out, colhalf * 64 + 32, row0, row0 < n_live, lane);
         }
+        if (!PAIR) store.close(lane);
     }
 
     // ---- teardown ---------------------------------------------------------------------------------
@@ -467,38 +495,44 @@ namespace dq256 {
 constexpr int kD = 256;
 constexpr int kChunkBytes = 8192;
 constexpr int kStep = 2, kStepBytes = kStep * kChunkBytes;   // chunks per copy and stage of the ring
-constexpr int kBRing = 4;
+constexpr int kMaxBRing = 8;
 constexpr int kKStages = 2;
 constexpr int kExpWarps = 16, kEpiWarps = 8;
 constexpr int kFirstExp = 3, kFirstEpi = kFirstExp + kExpWarps;
 constexpr int kThreads256 = (3 + kExpWarps + kEpiWarps) * 32;
-enum { K_FULL = 0, K_EMPTY = 2, B_FULL = 4, B_EMPTY = 12, A_FULL = 20, A_EMPTY = 22, D_FULL = 24, D_EMPTY = 26, N_BARS = 28 };
+enum { K_FULL = 0, K_EMPTY = 2, B_FULL = 4, B_EMPTY = 4 + kMaxBRing, A_FULL = 20, A_EMPTY = 22, D_FULL = 24, D_EMPTY = 26, N_BARS = 28 };
 template <int BITS, bool PROD>
 struct Smem {
     static constexpr int kLutBytes = (1 << (2 * BITS)) * 32 * 8;
     static constexpr int kCodeRowBytes = kD * BITS / 8;
     static constexpr int kSignRowBytes = kD / 8;
     static constexpr int kStageBytes = kTileKeys * (kCodeRowBytes + (PROD ? kSignRowBytes : 0));
-    static constexpr int kOutRowBytes = 36 * 4;
-    static constexpr int kOutWarpBytes = 32 * kOutRowBytes;
-    static constexpr int off_lut = 0;
+    static constexpr int kOutBufs = 2;
+    static constexpr int kOutWarpBytes = kOutBufs * kBlockBytes;
+    static constexpr int off_out = 0;                                   // (the swizzle wants blocks on 1 KB boundaries)
+    static constexpr int off_lut = off_out + kEpiWarps * kOutWarpBytes;
     static constexpr int off_b = off_lut + kLutBytes;
+    // The ring takes what is left: a step is 350 cycles of tensor work, and its way round -- release, producer, L2, arrival -- takes some
+    // 2,400 under load.
+    static constexpr int kMisc = 512 + 128 + 1024;                      // + slack to align the base
+    static constexpr int kBRoom = (227 * 1024 - kMisc - off_b - kKStages * kStageBytes) / kStepBytes;
+    static constexpr int kBRing = kBRoom < kMaxBRing ? kBRoom : kMaxBRing;
     static constexpr int off_ring = off_b + kBRing * kStepBytes;
-    static constexpr int off_out = off_ring + kKStages * kStageBytes;
-    static constexpr int off_misc = off_out + kEpiWarps * kOutWarpBytes;
-    static constexpr int total = off_misc + 512 + 128 + 128;    // + slack to align the base
+    static constexpr int off_misc = off_ring + kKStages * kStageBytes;
+    static constexpr int total = off_misc + kMisc;
     static_assert(total <= 227 * 1024, "shared memory plan");
 };
 }  // namespace dq256
 
 template <int BITS, bool PROD>
 __global__ void __launch_bounds__(dq256::kThreads256, 1)
-dequant256_kernel(const DequantArgs a) {
+dequant256_kernel(const __grid_constant__ CUtensorMap tmap_out, const DequantArgs a) {
     using namespace dq256;
     using L = dq256::Smem<BITS, PROD>;
     constexpr int kPhases = PROD ? 2 : 1;
+    constexpr int kBRing = L::kBRing;
     extern __shared__ unsigned char smem_raw[];
-    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const uint32_t smem_base = smem_u32(smem);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::off_misc);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + N_BARS);
@@ -576,22 +610,24 @@ dequant256_kernel(const DequantArgs a) {
         }
     } else if (warp == 2) {
         // ---- operand chunks: the same 32 (64) chunks for every tile, in the order of the instructions: (phase, I, J, kb) ----
-        if (lane == 0) {
-            int64_t g = 0;
-            bool ok = true;
-            for (int64_t i = 0; i < my_tiles && ok; ++i) {
-                for (int c = 0; c < kPhases * 32; c += kStep, ++g) {
-                    const int slot = (int)(g % kBRing);
-                    const int chunk = (c & 32) + ((c & 8) << 1) + ((c & 16) >> 1) + (c & 7);
-                    if (!mbar_wait(BAR(B_EMPTY + slot), (uint32_t)(((g / kBRing) & 1) ^ 1), abort_flag)) { ok = false; break; }
+        // (the whole warp walks the loop, as for the tensor instructions: a copy issued by a lane on its own costs several times as much)
+        int64_t g = 0;
+        bool ok = true;
+        for (int64_t i = 0; i < my_tiles && ok; ++i) {
+            for (int c = 0; c < kPhases * 32; c += kStep, ++g) {
+                const int slot = (int)(g % kBRing);
+                const int chunk = (c & 32) + ((c & 8) << 1) + ((c & 16) >> 1) + (c & 7);
+                if (!warp_wait(BAR(B_EMPTY + slot), (uint32_t)(((g / kBRing) & 1) ^ 1), abort_flag)) { ok = false; break; }
+                if (elect_one()) {
                     mbar_arrive_expect_tx(BAR(B_FULL + slot), kStepBytes);
                     bulk_load(smem_base + L::off_b + slot * kStepBytes, a.bmat + (size_t)chunk * kChunkBytes, kStepBytes, BAR(B_FULL + slot));
                 }
+                __syncwarp();
             }
-            if (*abort_flag)
-                for (int64_t gg = g > kBRing ? g - kBRing : 0; gg < g; ++gg)
-                    mbar_drain(BAR(B_FULL + (int)(gg % kBRing)), (uint32_t)((gg / kBRing) & 1));
         }
+        if (lane == 0 && *abort_flag)
+            for (int64_t gg = g > kBRing ? g - kBRing : 0; gg < g; ++gg)
+                mbar_drain(BAR(B_FULL + (int)(gg % kBRing)), (uint32_t)((gg / kBRing) & 1));
     } else if (warp == 1) {
         // ---- MMA issuer ---------------------------------------------------------------------------------
         const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
@@ -730,12 +766,18 @@ dequant256_kernel(const DequantArgs a) {
         const int quarter = warp & 3;
         const int colgroup = ew >> 2;
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
-        unsigned char* stg = smem + L::off_out + ew * L::kOutWarpBytes;
+        BlockStore<L::kOutBufs> store{smem + L::off_out + ew * L::kOutWarpBytes, 0};
+        const int row = quarter * 32 + lane;
+        float nrm_next = my_tiles > 0 && (int64_t)blockIdx.x * kTileKeys + row < a.n ? __ldg(a.norms + (int64_t)blockIdx.x * kTileKeys + row) : 0.f;
         for (int64_t i = 0; i < my_tiles; ++i) {
             const int64_t tile = blockIdx.x + i * gridDim.x;
             const uint32_t par = (uint32_t)(i & 1);
             const int64_t row0 = tile * kTileKeys + quarter * 32;
-            const float sc = (row0 + lane < a.n ? __ldg(a.norms + row0 + lane) : 0.f) * kOutScale;
+            const float sc = nrm_next * kOutScale;
+            if (i + 1 < my_tiles) {   // the norm of the next tile's key is fetched a tile ahead of its use
+                const int64_t rn = (tile + gridDim.x) * kTileKeys + row;
+                nrm_next = rn < a.n ? __ldg(a.norms + rn) : 0.f;
+            }
 #pragma unroll 1
             for (int j = 0; j < 2; ++j) {
                 const int64_t n_live = mbar_wait(BAR(D_FULL + j), par, abort_flag) ? a.n : 0;   // after a give-up nothing is written
@@ -748,28 +790,14 @@ dequant256_kernel(const DequantArgs a) {
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(BAR(D_EMPTY + j));   // the accumulator is free again
-                // through the warp's staging block, so that its global stores cover whole 128-byte lines
-#pragma unroll
-                for (int ch = 0; ch < 2; ++ch) {
-                    float4* mine = reinterpret_cast<float4*>(stg + lane * L::kOutRowBytes);
-#pragma unroll
-                    for (int m = 0; m < 8; ++m) {
-                        const uint32_t* v = ch == 0 ? va : vb;
-                        mine[m] = make_float4(__uint_as_float(v[4 * m]) * sc, __uint_as_float(v[4 * m + 1]) * sc,
-                                              __uint_as_float(v[4 * m + 2]) * sc, __uint_as_float(v[4 * m + 3]) * sc);
-                    }
-                    __syncwarp();
-#pragma unroll
-                    for (int it = 0; it < 8; ++it) {
-                        const int r = it * 4 + (lane >> 3), c4 = lane & 7;
-                        const float4 val = *reinterpret_cast<const float4*>(stg + r * L::kOutRowBytes + c4 * 16);
-                        if (row0 + r < n_live)
-                            __stcs(reinterpret_cast<float4*>(a.out + (row0 + r) * kD + j * 128 + colgroup * 64 + ch * 32) + c4, val);
-                    }
-                    __syncwarp();
-                }
+                const int col = j * 128 + colgroup * 64;
+                store.write(va, sc, lane);
+                store.send(&tmap_out, col, row0, row0 < n_live, lane);
+                store.write(vb, sc, lane);
+                store.send(&tmap_out, col + 32, row0, row0 < n_live, lane);
             }
         }
+        store.close(lane);
     }
 
     if (*abort_flag) __nanosleep(20000);   // tensor instructions issued before the give-up may still be running
@@ -826,20 +854,38 @@ void split_transposed_chunks(const float* m, float scale, uint16_t* out) {
         }
 }
 
+// The reconstructions [n][d] as boxes of 32 rows x 32 floats.
+int output_map(float* out, int64_t n, int d, CUtensorMap* map) {
+    const cuuint64_t gdim[2] = {(cuuint64_t)d, (cuuint64_t)n};
+    const cuuint64_t gstride[1] = {(cuuint64_t)d * 4};
+    const cuuint32_t box[2] = {32, 32}, estr[2] = {1, 1};
+    const CUresult r = tq_encode_tiled_fn()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, out, gdim, gstride, box, estr,
+                                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return tq_fail(TQ_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d", (int)r);
+    return TQ_OK;
+}
+
 template <int BITS, bool PROD>
 int launch_256(const tq_plan* p, const DequantArgs& args, int grid, cudaStream_t st) {
+    CUtensorMap map;
+    const int rc = output_map(args.out, args.n, 256, &map);
+    if (rc != TQ_OK) return rc;
     const int sm = dq256::Smem<BITS, PROD>::total;
     TQ_GRANT_SMEM((dequant256_kernel<BITS, PROD>), sm, p->device);
-    dequant256_kernel<BITS, PROD><<<grid, dq256::kThreads256, sm, st>>>(args); tq_count_launch();
+    dequant256_kernel<BITS, PROD><<<grid, dq256::kThreads256, sm, st>>>(map, args); tq_count_launch();
     TQ_CUDA_TRY(cudaGetLastError());
     return TQ_OK;
 }
 
 template <int BITS, bool PROD, int DR, bool PAIR = false>
 int launch_one(const tq_plan* p, const DequantArgs& args, int grid, cudaStream_t st) {
+    CUtensorMap map{};
+    const int rc = PAIR ? TQ_OK : output_map(args.out, args.n, DR, &map);
+    if (rc != TQ_OK) return rc;
     const int sm = DqSmem<BITS, PROD, DR>::total;
     TQ_GRANT_SMEM((dequant_tc_kernel<BITS, PROD, DR, PAIR>), sm, p->device);
-    dequant_tc_kernel<BITS, PROD, DR, PAIR><<<grid, kThreads, sm, st>>>(args); tq_count_launch();
+    dequant_tc_kernel<BITS, PROD, DR, PAIR><<<grid, kThreads, sm, st>>>(map, args); tq_count_launch();
     TQ_CUDA_TRY(cudaGetLastError());
     return TQ_OK;
 }

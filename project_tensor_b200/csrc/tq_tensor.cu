@@ -856,7 +856,7 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
 // (K half I in block I); the two accumulator blocks take the two halves J of the output columns.  The rotation is
 // stored as 32 chunks of 8 KB -- chunk ((J * 2 + I) * 8 + kb) holds R_hi and R_lo for output columns [128 J, 128 J + 128)
 // and input coordinates [128 I + 16 kb, + 16) as K-major 8 x 8 core matrices -- and every CTA pulls the 256 KB through a
-// ring of 8 chunks once per tile (from L2), three tensor instructions per chunk.  For TurboQuantProd rho (split, in place of
+// ring of 10 chunks once per tile (from L2), three tensor instructions per chunk.  For TurboQuantProd rho (split, in place of
 // the accumulators) is multiplied with 16 (R S^T), 32 more chunks, into the A blocks.
 //
 // Tensor memory is full with one tile (A 256 + accumulators 256 columns), so the phases of a tile form a chain and what counts is
@@ -877,7 +877,7 @@ constexpr int kXRing = 8;                    // one tile: a worker must not meet
 constexpr int kChunkBytes = 8192;                // R_hi and R_lo of one (J, I, kb): 128 x 16 halves each
 constexpr int kStep = 2;                         // chunks per copy and stage of the ring
 constexpr int kStepBytes = kStep * kChunkBytes;
-constexpr int kBRing = 4;
+constexpr int kBRing = 5;
 constexpr int kWorkers = 16, kFirstWorker = 3;
 constexpr int kThreads = (kFirstWorker + kWorkers) * 32;         // 608
 constexpr int off_b = 0;
@@ -885,7 +885,7 @@ constexpr int off_x = off_b + kBRing * kStepBytes;               // 128 KB
 constexpr int off_ssq = off_x + kXRing * kBoxBytes;              // [2 tiles][4 parts][128] floats
 constexpr int off_force = off_ssq + 2 * 4 * kTileRows * 4;       // [4][128] bytes
 constexpr int off_bars = off_force + 4 * kTileRows;
-enum { X_FULL = 0, X_EMPTY = 8, B_FULL = 16, B_EMPTY = 24, A_FULL = 32, A_EMPTY = 33, ACC_FULL = 34, ACC_EMPTY = 36, RHO_FULL = 38, ACC2_FULL = 40, N_BARS = 42 };
+enum { X_FULL = 0, X_EMPTY = 8, B_FULL = 16, B_EMPTY = 24, A_FULL = 32, A_EMPTY = 34, ACC_FULL = 35, ACC_EMPTY = 37, RHO_FULL = 39, ACC2_FULL = 41, N_BARS = 43 };
 constexpr int off_lut = off_bars + 512;                          // barriers, tensor-memory slot, give-up flag; then the cell table
 constexpr int off_rs = off_lut + 512;                            // |rho|^2 partial sums [4 parts][128] (TurboQuantProd)
 constexpr int off_pend = off_rs + 4 * kTileRows * 4;
@@ -915,7 +915,7 @@ tensor_quantize256_kernel(const __grid_constant__ CUtensorMap tmap_x, const Tens
     if (threadIdx.x == 0) {
         for (int i = 0; i < kXRing; ++i) { mbar_init(BAR(X_FULL + i), 1); mbar_init(BAR(X_EMPTY + i), 4); }
         for (int i = 0; i < kBRing; ++i) { mbar_init(BAR(B_FULL + i), 1); mbar_init(BAR(B_EMPTY + i), 1); }
-        mbar_init(BAR(A_FULL), kWorkers);
+        for (int h = 0; h < 2; ++h) mbar_init(BAR(A_FULL + h), kWorkers / 2);
         mbar_init(BAR(A_EMPTY), 1);
         for (int j = 0; j < 2; ++j) {
             mbar_init(BAR(ACC_FULL + j), 1);
@@ -961,28 +961,30 @@ tensor_quantize256_kernel(const __grid_constant__ CUtensorMap tmap_x, const Tens
                     mbar_drain(BAR(X_FULL + (int)(gg % kXRing)), (uint32_t)((gg / kXRing) & 1));
         }
     } else if (warp == 2) {
-        // ---- matrices: one bulk copy per chunk, the same chunks for every tile, in the order of the instructions ----
-        if (lane == 0) {
-            int64_t g = 0;
-            bool ok = true;
-            const unsigned char* src = reinterpret_cast<const unsigned char*>(a.bmat);
-            for (int64_t i = 0; i < my_tiles && ok; ++i) {
-                for (int c = 0; c < (PROD ? 64 : 32); c += kStep, ++g) {
-                    const int slot = (int)(g % kBRing);
-                    // first contraction: (J, I, kb); second: (I, J, kb) of the 32 chunks behind
-                    const int chunk = c < 32 ? c : 32 + ((c & 8) << 1) + ((c & 16) >> 1) + (c & 7);
-                    if (!mbar_wait(BAR(B_EMPTY + slot), (uint32_t)(((g / kBRing) & 1) ^ 1), abort_flag)) { ok = false; break; }
+        // ---- matrices: the same chunks for every tile, in the order of the instructions -------------------
+        // (the whole warp walks the loop, as for the tensor instructions: a copy issued by a lane on its own costs several times as much)
+        int64_t g = 0;
+        bool ok = true;
+        const unsigned char* src = reinterpret_cast<const unsigned char*>(a.bmat);
+        for (int64_t i = 0; i < my_tiles && ok; ++i) {
+            for (int c = 0; c < (PROD ? 64 : 32); c += kStep, ++g) {
+                const int slot = (int)(g % kBRing);
+                // first contraction: (J, I, kb); second: (I, J, kb) of the 32 chunks behind
+                const int chunk = c < 32 ? c : 32 + ((c & 8) << 1) + ((c & 16) >> 1) + (c & 7);
+                if (!warp_wait(BAR(B_EMPTY + slot), (uint32_t)(((g / kBRing) & 1) ^ 1), abort_flag)) { ok = false; break; }
+                if (elect_one()) {
                     mbar_arrive_expect_tx(BAR(B_FULL + slot), kStepBytes);
                     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                                  ::"r"(smem_base + off_b + slot * kStepBytes), "l"(src + (size_t)chunk * kChunkBytes), "r"(kStepBytes),
                                    "r"(BAR(B_FULL + slot))
                                  : "memory");
                 }
+                __syncwarp();
             }
-            if (*abort_flag)
-                for (int64_t gg = g > kBRing ? g - kBRing : 0; gg < g; ++gg)
-                    mbar_drain(BAR(B_FULL + (int)(gg % kBRing)), (uint32_t)((gg / kBRing) & 1));
         }
+        if (lane == 0 && *abort_flag)
+            for (int64_t gg = g > kBRing ? g - kBRing : 0; gg < g; ++gg)
+                mbar_drain(BAR(B_FULL + (int)(gg % kBRing)), (uint32_t)((gg / kBRing) & 1));
     } else if (warp == 1) {
         // ---- MMA issuer: the whole warp walks the loop, one elected lane issues -------------------------
         const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
@@ -1024,6 +1026,7 @@ tensor_quantize256_kernel(const __grid_constant__ CUtensorMap tmap_x, const Tens
                 if (!PROD && !warp_wait(BAR(ACC_EMPTY + j), par ^ 1u, abort_flag)) { ok = false; break; }
                 tc_fence_after();
                 ok = contract(tm + ACC_COL(j), true, tm + A_COL(0), kABlock, unit_col, -1) &&
+                     (j == 1 || warp_wait(BAR(A_FULL + 1), par, abort_flag)) &&      // (a signed-off half starts without the other)
                      contract(tm + ACC_COL(j), false, tm + A_COL(1), kABlock, unit_col, ACC_FULL + j);
             }
             if (!ok) break;
@@ -1105,13 +1108,15 @@ tensor_quantize256_kernel(const __grid_constant__ CUtensorMap tmap_x, const Tens
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {
                     const float4 v = fail ? make_float4(0.f, 0.f, 0.f, 0.f) : lds_once_f4(x0 + bb * kBoxBytes + ((c ^ (row & 7)) << 4));
-                    const float u0 = v.x * scale, u1 = v.y * scale, u2 = v.z * scale, u3 = v.w * scale;
-                    const __half2 h0 = __floats2half2_rn(u0, u1), h1 = __floats2half2_rn(u2, u3);
+                    const float2 sc2 = make_float2(scale, scale);
+                    const float2 u0 = __fmul2_rn(make_float2(v.x, v.y), sc2), u1 = __fmul2_rn(make_float2(v.z, v.w), sc2);
+                    const __half2 h0 = __floats2half2_rn(u0.x, u0.y), h1 = __floats2half2_rn(u1.x, u1.y);
                     const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
+                    const float2 l0 = __fadd2_rn(u0, make_float2(-f0.x, -f0.y)), l1 = __fadd2_rn(u1, make_float2(-f1.x, -f1.y));
                     hi[2 * c] = *reinterpret_cast<const uint32_t*>(&h0);
                     hi[2 * c + 1] = *reinterpret_cast<const uint32_t*>(&h1);
-                    lo[2 * c] = pack_half2(u0 - f0.x, u1 - f0.y);
-                    lo[2 * c + 1] = pack_half2(u2 - f1.x, u3 - f1.y);
+                    lo[2 * c] = pack_half2(l0.x, l0.y);
+                    lo[2 * c + 1] = pack_half2(l1.x, l1.y);
                 }
                 tmem_st16(a_hi + bb * 16, hi);
                 tmem_st16(a_hi + kABlock + bb * 16, lo);
@@ -1121,7 +1126,7 @@ tensor_quantize256_kernel(const __grid_constant__ CUtensorMap tmap_x, const Tens
             __threadfence_block();   // every lane's loads from the stages are performed before the stages are released
             __syncwarp();
             if (lane == 0) {
-                mbar_arrive(BAR(A_FULL));
+                mbar_arrive(BAR(A_FULL + (part >> 1)));
                 if (!fail) { mbar_arrive(BAR(X_EMPTY + part * 2)); mbar_arrive(BAR(X_EMPTY + part * 2 + 1)); }
             }
         };
