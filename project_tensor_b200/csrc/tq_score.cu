@@ -1,4 +1,5 @@
-// Scoring kernels for TurboQuantProd encodings (any d <= 1024, bits <= 8).
+// Scoring kernels for TurboQuantProd encodings (any d <= 1024, bits <= 8): score_matrix_kernel where the matrix alone is wanted,
+// score_kernel for the best keys of every query (with the matrix or without).
 //
 // score(q, key i) = norms[i] * ( (R q) . codebook[codes_i]  +  alpha * residual_norms[i] * ((S q) . qjl_i) )
 //
@@ -19,6 +20,14 @@ namespace {
 
 constexpr int kThreads = 128;
 constexpr int kQT = 8;  // queries scored together per pass over a block's keys
+constexpr int kMatThreads = 256;   // threads of score_matrix_kernel
+
+// Both kernels give a score the same bits: the sums of the rotated and projected queries come in slices of k, added up in order;
+// a score is one chain over the coordinates, centroid and sign in turn.
+__host__ __device__ inline int query_slices(int d) {
+    const int quarter = ((d + 31) & ~31) / 2;
+    return quarter < kMatThreads ? kMatThreads / quarter : 1;
+}
 
 using namespace tqtopk;
 
@@ -60,38 +69,40 @@ score_kernel(TqDev p, const float* __restrict__ q, int qpg, const uint32_t* __re
             const int t = i / (2 * d), r = i - t * 2 * d, which = r / d, j = r - which * d;
             const float* M = which ? p.St : p.Rt;
             const float* qv = qraw + t * d;
-            float acc = 0.f;
-            for (int k = 0; k < d; ++k) acc = fmaf(qv[k], __ldg(M + (size_t)k * d + j), acc);
-            qs[i] = acc;
+            float sum = 0.f;
+            const int slices = query_slices(d), len = (d + slices - 1) / slices;
+            for (int k0 = 0; k0 < d; k0 += len) {
+                float acc = 0.f;
+                for (int k = k0; k < min(k0 + len, d); ++k) acc = fmaf(qv[k], __ldg(M + (size_t)k * d + j), acc);
+                sum += acc;
+            }
+            qs[i] = sum;
         }
         __syncthreads();
 
         for (int64_t kb = k0; kb < k1; kb += kThreads) {
             const int64_t key = kb + threadIdx.x;
             const bool live = key < k1;
-            float a1[kQT], a2[kQT];
+            float acc[kQT];
 #pragma unroll
-            for (int t = 0; t < kQT; ++t) { a1[t] = 0.f; a2[t] = 0.f; }
+            for (int t = 0; t < kQT; ++t) acc[t] = 0.f;
             if (live) {
+                const float arn = p.alpha * rnorms[gbase + key];
                 const uint32_t* crow = codes + (gbase + key) * p.code_words;
                 const uint32_t* srow = signs + (gbase + key) * p.sign_words;
                 uint32_t sw = 0;
                 for (int j = 0; j < d; ++j) {
                     if ((j & 31) == 0) sw = srow[j >> 5];
                     const float c = cb[tq_get_code(crow, j, p.bits)];
-                    const float s = (sw >> tq_sign_bitpos(j)) & 1u ? 1.f : -1.f;
+                    const float s = (sw >> tq_sign_bitpos(j)) & 1u ? arn : -arn;
 #pragma unroll
-                    for (int t = 0; t < kQT; ++t) {
-                        a1[t] = fmaf(c, qs[(t * 2) * d + j], a1[t]);
-                        a2[t] = fmaf(s, qs[(t * 2 + 1) * d + j], a2[t]);
-                    }
+                    for (int t = 0; t < kQT; ++t) acc[t] = fmaf(s, qs[(t * 2 + 1) * d + j], fmaf(c, qs[(t * 2) * d + j], acc[t]));
                 }
                 const float nrm = norms[gbase + key];
-                const float arn = p.alpha * rnorms[gbase + key];
 #pragma unroll
                 for (int t = 0; t < kQT; ++t) {
                     if (t < nq) {
-                        const float s = nrm * (a1[t] + arn * a2[t]);
+                        const float s = nrm * acc[t];
                         if (scores) scores[((int64_t)g * qpg + q0 + t) * keys_per_group + key] = s;
                         if (topk > 0) {
                             const unsigned long long ck = make_key(s, (uint32_t)(gbase + key));
@@ -133,6 +144,158 @@ score_kernel(TqDev p, const float* __restrict__ q, int qpg, const uint32_t* __re
                 unsigned long long* dst = part + (((size_t)g * gridDim.x + blockIdx.x) * qpg + q0 + t) * topk;
                 for (int i = threadIdx.x; i < topk; i += kThreads) dst[i] = b[i];
             }
+        }
+    }
+}
+
+// A score matrix without top-k, any d and bits: the case that repeats (validation runs and sweeps at dimensions or bit widths without
+// a tensor-core kernel).  A thread scores KT keys for QT queries, 32 coordinates at a time -- BITS words of codes, taken apart with
+// compile-time shifts, and one sign word; c * (R q)[j] and +-(alpha * rnorm) * (S q)[j] add up in one accumulator.  The shared-memory
+// pipe returns 16 bytes a lane in four cycles, so one pair of query vectors has to feed several keys: four keys x eight queries
+// balance it with the FMA pipe.  The queries are rotated and projected by the whole block, four outputs and a slice of the sum
+// per thread with 32 or 64 matrix elements in flight.  50,021 keys, d = 96, 5-bit codes, 16 queries: 96 us in the kernel above
+// (one key and eight queries a thread, four-byte loads, generic bit arithmetic), now 25; one query against 256 keys,
+// d = 128: 79 us, now 14.
+template <int BITS, int QT, int KT>
+__global__ void __launch_bounds__(kMatThreads)
+score_matrix_kernel(TqDev p, const float* __restrict__ q, int qpg, const uint32_t* __restrict__ codes,
+                    const uint32_t* __restrict__ signs, const float* __restrict__ rnorms, const float* __restrict__ norms,
+                    int64_t keys_per_group, int64_t group_rows, int slices, int pass0, float* __restrict__ scores) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    const int d = p.d, dp = (d + 31) & ~31, t = threadIdx.x;
+    float* qs = reinterpret_cast<float*>(smraw);         // [dp][2][QT] rotated | projected, zeros behind d
+    float* qraw = qs + dp * 2 * QT;                       // [d][QT]
+    __shared__ float cb[1 << BITS];
+    const int g = blockIdx.z, q0 = (pass0 + (int)blockIdx.y) * QT, nq = min(QT, qpg - q0);
+    const int64_t gbase = (int64_t)g * group_rows;
+    for (int i = t; i < (1 << BITS); i += kMatThreads) cb[i] = __ldg(p.codebook + i);
+    for (int i = t; i < QT * d; i += kMatThreads) {
+        const int u = i / d, k = i - u * d;
+        qraw[k * QT + u] = u < nq ? __ldg(q + ((int64_t)g * qpg + q0 + u) * d + k) : 0.f;
+    }
+    __syncthreads();
+    // outputs 0 .. 2 dp: rotated, then projected; a thread takes o, o + quarter, ... and one slice of the sum
+    const int quarter = dp / 2;
+    constexpr int kAhead = QT > 2 ? 8 : 16;
+    for (int pass = 0; pass < (quarter + kMatThreads - 1) / kMatThreads; ++pass) {
+        const int o = slices > 1 ? t % quarter : t + pass * kMatThreads, slice = slices > 1 ? t / quarter : 0;
+        const bool mine = o < quarter && slice < slices;
+        const int len = (d + slices - 1) / slices, k0 = slice * len, k1 = min(k0 + len, d);
+        float acc[4][QT];
+        const float* src[4];
+        bool have[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int out = o + c * quarter, j = out < dp ? out : out - dp;
+            have[c] = mine && j < d;
+            src[c] = (out < dp ? p.Rt : p.St) + (have[c] ? j : 0);
+#pragma unroll
+            for (int u = 0; u < QT; ++u) acc[c][u] = 0.f;
+        }
+        if (mine) {
+            for (int k = k0; k < k1; k += kAhead) {
+                float m[kAhead][4];
+#pragma unroll
+                for (int a = 0; a < kAhead; ++a)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) m[a][c] = __ldg(src[c] + (size_t)min(k + a, d - 1) * d);
+#pragma unroll
+                for (int a = 0; a < kAhead; ++a) {
+                    if (k + a >= k1) break;
+                    const float* v = qraw + (k + a) * QT;
+#pragma unroll
+                    for (int u = 0; u < QT; ++u)
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) acc[c][u] = fmaf(v[u], m[a][c], acc[c][u]);
+                }
+            }
+        }
+        for (int s = 0; s < slices; ++s) {       // the slices add up one after the other
+            if (s == slice && mine) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const int out = o + c * quarter, j = out < dp ? out : out - dp;
+                    float* dst = qs + (j * 2 + (out < dp ? 0 : 1)) * QT;
+#pragma unroll
+                    for (int u = 0; u < QT; ++u) dst[u] = (s > 0 ? dst[u] : 0.f) + (have[c] ? acc[c][u] : 0.f);
+                }
+            }
+            __syncthreads();
+        }
+    }
+    for (int64_t kb = (int64_t)blockIdx.x * kMatThreads * KT; kb < keys_per_group; kb += (int64_t)gridDim.x * kMatThreads * KT) {
+        float2 acc[KT][QT / 2];
+        float arn[KT];
+        const uint32_t *crow[KT], *srow[KT];
+#pragma unroll
+        for (int e = 0; e < KT; ++e) {
+            const int64_t key = kb + t + e * kMatThreads, row = gbase + (key < keys_per_group ? key : keys_per_group - 1);
+            crow[e] = codes + row * p.code_words;
+            srow[e] = signs + row * p.sign_words;
+            arn[e] = p.alpha * __ldg(rnorms + row);
+#pragma unroll
+            for (int u = 0; u < QT / 2; ++u) acc[e][u] = make_float2(0.f, 0.f);
+        }
+        uint32_t wn[KT][BITS], sn[KT];               // words of the next 32 coordinates
+        auto fetch = [&](int j0) {
+            const int w0 = j0 / 32 * BITS, last = p.code_words - 1;
+#pragma unroll
+            for (int e = 0; e < KT; ++e) {
+#pragma unroll
+                for (int i = 0; i < BITS; ++i) wn[e][i] = __ldg(crow[e] + min(w0 + i, last));   // (codes behind d meet zeros)
+                sn[e] = ~__ldg(srow[e] + j0 / 32);           // a set bit now means a negative sign
+            }
+        };
+        fetch(0);
+        for (int j0 = 0; j0 < dp; j0 += 32) {
+            uint32_t w[KT][BITS], sw[KT];
+#pragma unroll
+            for (int e = 0; e < KT; ++e) {
+#pragma unroll
+                for (int i = 0; i < BITS; ++i) w[e][i] = wn[e][i];
+                sw[e] = sn[e];
+            }
+            if (j0 + 32 < dp) fetch(j0 + 32);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+                constexpr uint32_t kMask = (1u << BITS) - 1u;
+                const int bit = i * BITS, at = bit >> 5, sh = bit & 31;
+                float2 x[2][QT / 2];
+                const float2* v = reinterpret_cast<const float2*>(qs + (j0 + i) * 2 * QT);
+                if constexpr (QT % 4 == 0) {
+#pragma unroll
+                    for (int u = 0; u < QT; u += 2) {
+                        const float4 f = reinterpret_cast<const float4*>(v)[u / 2];
+                        x[u / (QT / 2)][u % (QT / 2)] = make_float2(f.x, f.y);
+                        x[u / (QT / 2)][u % (QT / 2) + 1] = make_float2(f.z, f.w);
+                    }
+                } else {
+                    x[0][0] = v[0];
+                    x[1][0] = v[1];
+                }
+#pragma unroll
+                for (int e = 0; e < KT; ++e) {
+                    uint32_t code = w[e][at] >> sh;
+                    if (sh + BITS > 32) code |= w[e][at + 1 < BITS ? at + 1 : at] << (32 - sh);
+                    const float c = cb[code & kMask];
+                    const float s = __uint_as_float(__float_as_uint(arn[e]) ^ ((sw[e] << (31 - tq_sign_bitpos(i))) & 0x80000000u));
+#pragma unroll
+                    for (int u = 0; u < QT / 2; ++u) {
+                        acc[e][u] = __ffma2_rn(make_float2(c, c), x[0][u], acc[e][u]);
+                        acc[e][u] = __ffma2_rn(make_float2(s, s), x[1][u], acc[e][u]);
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < KT; ++e) {
+            const int64_t key = kb + t + e * kMatThreads;
+            if (key >= keys_per_group) break;
+            const float nrm = __ldg(norms + gbase + key);
+            float* dst = scores + ((int64_t)g * qpg + q0) * keys_per_group + key;
+#pragma unroll
+            for (int u = 0; u < QT; ++u)
+                if (u < nq) dst[u * keys_per_group] = nrm * (u & 1 ? acc[e][u / 2].y : acc[e][u / 2].x);
         }
     }
 }
@@ -284,6 +447,33 @@ ScoreGeometry geometry(int groups, int64_t keys_per_group, int topk) {
     return s;
 }
 
+template <int BITS, int QT, int KT>
+int launch_matrix(const tq_plan* p, const float* q, int groups, int qpg, const uint32_t* codes, const uint32_t* signs, const float* rnorms,
+                  const float* norms, int64_t keys_per_group, int64_t group_rows, float* scores, cudaStream_t st) {
+    const int d = p->dev.d, dp = (d + 31) & ~31, slices = query_slices(d);
+    const size_t sm = (size_t)(dp * 2 + d) * QT * sizeof(float);
+    const int passes = (qpg + QT - 1) / QT;
+    // every block transforms the queries: no more of them than run at once
+    int64_t blocks = (keys_per_group + kMatThreads * KT - 1) / (kMatThreads * KT);
+    const int64_t room = (tq_sm_count(p->device) * (int64_t)4 + (int64_t)passes * groups - 1) / ((int64_t)passes * groups);
+    if (blocks > room) blocks = room < 1 ? 1 : room;
+    TQ_GRANT_SMEM((score_matrix_kernel<BITS, QT, KT>), sm, p->device);
+    for (int pass0 = 0; pass0 < passes; pass0 += 65535) {        // (rows of a grid)
+        const unsigned rows = (unsigned)(passes - pass0 < 65535 ? passes - pass0 : 65535);
+        score_matrix_kernel<BITS, QT, KT><<<dim3((unsigned)blocks, rows, (unsigned)groups), kMatThreads, sm, st>>>(
+            p->dev, q, qpg, codes, signs, rnorms, norms, keys_per_group, group_rows, slices, pass0, scores); tq_count_launch();
+        TQ_CUDA_TRY(cudaGetLastError());
+    }
+    return TQ_OK;
+}
+template <int BITS>
+int launch_matrix_bits(const tq_plan* p, const float* q, int groups, int qpg, const uint32_t* codes, const uint32_t* signs, const float* rnorms,
+                       const float* norms, int64_t keys_per_group, int64_t group_rows, float* scores, cudaStream_t st) {
+    // one or two queries: a thread per key keeps more SMs busy, and there is little to share
+    if (qpg <= 2) return launch_matrix<BITS, 2, 1>(p, q, groups, qpg, codes, signs, rnorms, norms, keys_per_group, group_rows, scores, st);
+    return launch_matrix<BITS, 8, 4>(p, q, groups, qpg, codes, signs, rnorms, norms, keys_per_group, group_rows, scores, st);
+}
+
 }  // namespace
 
 int64_t tq_score_tc_scratch(const tq_plan* p, int groups, int qpg, int64_t keys_per_group, int topk);
@@ -362,6 +552,14 @@ int tq_launch_score_general(const tq_plan* p, const float* q, int groups, int qp
             TQ_CUDA_TRY(cudaGetLastError());
         }
         return TQ_OK;
+    }
+    if (topk <= 0) {
+        switch (p->dev.bits) {
+#define TQ_MATRIX(B) case B: return launch_matrix_bits<B>(p, q, groups, qpg, codes, signs, rnorms, norms, keys_per_group, group_rows, scores, st);
+            TQ_MATRIX(1) TQ_MATRIX(2) TQ_MATRIX(3) TQ_MATRIX(4) TQ_MATRIX(5) TQ_MATRIX(6) TQ_MATRIX(7) TQ_MATRIX(8)
+#undef TQ_MATRIX
+        }
+        return tq_fail(TQ_ERR_UNSUPPORTED, "bits=%d", p->dev.bits);
     }
     const int d = p->dev.d;
     const size_t sm = (size_t)(kQT * d + kQT * 2 * d + 256) * sizeof(float) + (size_t)kQT * s.cap2 * sizeof(unsigned long long);
