@@ -220,15 +220,9 @@ int tq_launch_dequant_tc(const tq_plan* p, bool prod, const uint32_t* codes, con
 int tq_launch_pairwise_tc(const tq_plan* p, const float* q, const uint32_t* codes, const uint32_t* signs, const float* rnorms,
                           const float* norms, int64_t n, float* scores, cudaStream_t st);
 
-// Streaming scoring kernel for one or two queries per group (d = 128 / 64, 1..4 code bits).
+// Scoring kernel for at most four queries per group (d = 64, 128, 256, 1..4 code bits), tq_score_few.cu.
 bool tq_score_few_supported(const tq_plan* p, int qpg);
 int tq_launch_score_few(const tq_plan* p, const float* q, int groups, int qpg, const uint32_t* codes, const uint32_t* signs,
-                        const float* rnorms, const float* norms, int64_t keys_per_group, float* scores, cudaStream_t st,
-                        int64_t group_rows = 0);
-
-// Lookup-table scoring kernel for three or four queries per group (d = 128 / 64, 1..3 code bits), tq_score_lut.cu.
-bool tq_score_lut_supported(const tq_plan* p, int qpg);
-int tq_launch_score_lut(const tq_plan* p, const float* q, int groups, int qpg, const uint32_t* codes, const uint32_t* signs,
                         const float* rnorms, const float* norms, int64_t keys_per_group, float* scores, cudaStream_t st,
                         int64_t group_rows = 0);
 

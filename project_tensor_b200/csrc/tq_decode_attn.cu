@@ -42,6 +42,7 @@
 // coordinate and query: 64 groups x 4 queries x 32,768 keys (d = 128, 2 + 1 bit keys, 4-bit values) took 254 us, now 138; 8 queries
 // 476 and 160.
 #include "tq_common.cuh"
+#include "tq_mma.cuh"
 
 #include <math_constants.h>
 #include <stdint.h>
@@ -50,14 +51,14 @@
 
 namespace {
 
+using namespace tqmma;
+
 constexpr int kThreads = 384;
 constexpr int kWarps = kThreads / 32;
 constexpr int kTile = 16;           // keys a warp takes at a time
 constexpr int kMaxSplits = 64;
-constexpr float kCentScale = 1024.f;   // centroids (at most 1 in magnitude) before their split into fp16 hi + lo
 constexpr float kSlack = 8.f;          // a score may exceed the reference of its softmax by 2^kSlack
 constexpr float kWeightMax = 32768.f;  // largest scaled weight (fp16 reaches 65,504)
-constexpr int kRowBytes = 256;         // a table row (keys use the first half)
 
 struct DecodeArgs {
     const float* q;              // [groups][qpg][d]
@@ -75,50 +76,6 @@ struct DecodeArgs {
     int splits;
     float* part;                 // [groups][qpg][splits][d + 2]: accumulator, running max, running sum
 };
-
-__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ uint32_t transpose8x8(uint32_t v) {
-    uint32_t r;
-    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
-    return r;
-}
-__device__ __forceinline__ uint32_t half2_bits(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
-// (a, b) -> fp16 pairs hi and lo with hi + lo = value to about 22 bits
-__device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint32_t& lo) {
-    const __half2 h = __floats2half2_rn(a, b);
-    const float2 f = __half22float2(h);
-    hi = half2_bits(h);
-    lo = half2_bits(__floats2half2_rn(a - f.x, b - f.y));
-}
-// Shift left by s (negative: right) with s known at compile time.
-template <int S> __device__ __forceinline__ uint32_t shl(uint32_t v) {
-    if constexpr (S >= 0) return v << S;
-    else return v >> -S;
-}
-// 2^e as a float, e clamped to the normal range
-__device__ __forceinline__ float pow2i(int e) { return __int_as_float((min(max(e, -126), 127) + 127) << 23); }
-// power of two that brings a magnitude into [2^13, 2^14)
-__device__ __forceinline__ int scale_exp(float m) {
-    if (!(m > 0.f) || !(m < 3.0e38f)) return 0;
-    return min(max(13 - (int)((__float_as_uint(m) >> 23) - 127), -100), 100);
-}
-
-// f(0), f(1), ... f(N - 1) with compile-time arguments
-template <int N, class F, int I = 0>
-__device__ __forceinline__ void for_steps(F&& f) {
-    if constexpr (I < N) {
-        f(std::integral_constant<int, I>{});
-        for_steps<N, F, I + 1>(static_cast<F&&>(f));
-    }
-}
-
-// Rows of the key table: four codes at a time up to 2 bits, two at a time above.
-__host__ __device__ constexpr int codes_per_row(int bits) { return bits <= 2 ? 4 : 2; }
-__host__ __device__ constexpr int table_rows(int bits) { return 1 << (bits * codes_per_row(bits)); }
 
 template <int KB, int VB, int DR, int NQ>
 struct Plan {
@@ -150,7 +107,7 @@ struct Plan {
 // Packed words of one tile of 16 keys, as the lanes of a warp hold them.
 template <class P>
 struct TileWords {
-    uint32_t kc[2][P::kKW], sg[2], vc[4][P::kVW];
+    uint32_t kc[2][P::kKW], sg[2][1], vc[4][P::kVW];
     float kn[2], rn[2], vn[2];
 };
 
@@ -212,7 +169,7 @@ decode_partial_kernel(TqDev kp, DecodeArgs a) {
 #pragma unroll
                 for (int i = 0; i < P::kKW; ++i) w.kc[h][i] = __ldg(src + i);
             }
-            w.sg[h] = __ldg(sg_base + (size_t)key * P::kSignRowWords);
+            w.sg[h][0] = __ldg(sg_base + (size_t)key * P::kSignRowWords);
             w.kn[h] = __ldg(kn_base + key);
             w.rn[h] = __ldg(rn_base + key);
             w.vn[h] = __ldg(vn_base + key);
@@ -249,15 +206,7 @@ decode_partial_kernel(TqDev kp, DecodeArgs a) {
     // of an A operand.  Value table: 32 copies of hi, 32 copies of lo of the same coordinate of two keys.  A thread fills whole
     // rows, starting at a copy of its own (stores to rows 256 bytes apart would all hit the same banks).
     auto value = [](const float* codebook, int code) { return __ldg(codebook + code) * kCentScale; };
-    for (int e = tid; e < table_rows(KB); e += kThreads) {
-        constexpr int m = (1 << KB) - 1;
-        uint4 v;
-        split_pair(value(kp.codebook, e & m), value(kp.codebook, (e >> KB) & m), v.x, v.y);
-        if constexpr (codes_per_row(KB) == 4) split_pair(value(kp.codebook, (e >> 2 * KB) & m), value(kp.codebook, e >> 3 * KB), v.z, v.w);
-        else { v.z = v.x; v.w = v.y; }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(smem + e * kRowBytes + ((i + tid) & 7) * 16) = v;
-    }
+    build_key_table<KB>(smem, kp.codebook, tid, kThreads);
     for (int e = kThreads - 1 - tid; e < 1 << (2 * VB); e += kThreads) {
         uint32_t hi, lo;
         split_pair(value(a.vcodebook, e & ((1 << VB) - 1)), value(a.vcodebook, e >> VB), hi, lo);
@@ -365,8 +314,6 @@ decode_partial_kernel(TqDev kp, DecodeArgs a) {
     // Table lookups.  A byte of a word selects a row with one byte permutation: (lane's copy, byte, 0, 0) is its address.
     const uint32_t lane4 = (uint32_t)lane * 4u, lane8 = (uint32_t)(lane & 15) * 8u, lane16 = (uint32_t)(lane & 7) * 16u;
     auto pick = [&](uint32_t word, int byte, uint32_t copy) { return __byte_perm(word, copy, 0x5504u | (uint32_t)byte << 4); };
-    auto row8 = [&](uint32_t at) { return *reinterpret_cast<const uint2*>(smem + at); };
-    auto row16 = [&](uint32_t at) { return *reinterpret_cast<const uint4*>(smem + at); };
 
     // ---- tiles ----------------------------------------------------------------------------------------
     tq_grid_release();      // (the blocks that merge may take an SM when its last block here has ended)
@@ -376,61 +323,12 @@ decode_partial_kernel(TqDev kp, DecodeArgs a) {
         const uint32_t left = keys - tile * kTile;      // keys of this tile and behind it
         // -- scores
         float c1[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, c2[4] = {0.f, 0.f, 0.f, 0.f};
-        uint32_t kw[2][P::kKW], kw1[2], sw[2][2];
-        (void)kw1;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            if constexpr (P::kKeyBits % 32 == 0) {
-#pragma unroll
-                for (int i = 0; i < P::kKW; ++i) kw[h][i] = cur.kc[h][i];
-            } else {
-                // half words (d = 64, odd bits): shift them to the front
-                if constexpr (P::kKW == 2) {
-                    kw[h][0] = __funnelshift_r(cur.kc[h][0], cur.kc[h][1], kshift);
-                    kw[h][1] = cur.kc[h][1] >> kshift;
-                } else {
-                    kw[h][0] = cur.kc[h][0] >> kshift;
-                }
-            }
-            sw[h][0] = DR == 128 ? cur.sg[h] : cur.sg[h] >> (8 * (t & 1));
-            sw[h][1] = sw[h][0] >> 8;
-            if constexpr (KB == 1) {         // four codes: a nibble; even ones and odd ones in words of their own
-                kw1[h] = (kw[h][0] >> 4) & 0x0f0f0f0fu;
-                kw[h][0] &= 0x0f0f0f0fu;
-            }
-        }
+        KeyWords<KB, DR> key;
+        key.unpack(cur.kc, cur.sg, kshift, t);
         auto key_step = [&](auto sc) {
             constexpr int s = decltype(sc)::value;
             uint32_t ak[2][4], as[4];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                // coordinates 4s .. 4s + 3 of the lane
-                if constexpr (KB >= 3) {
-                    uint2 v0, v1;
-                    if constexpr (KB == 4) {
-                        v0 = row8(pick(kw[h][s >> 1], 2 * (s & 1), lane8));
-                        v1 = row8(pick(kw[h][s >> 1], 2 * (s & 1) + 1, lane8));
-                    } else {
-                        auto pair = [&](auto pc) {
-                            constexpr int bit = decltype(pc)::value * 6, w0 = bit >> 5, sh = bit & 31;
-                            uint32_t x;                   // the pair at bit 8
-                            if constexpr (sh + 6 > 32) x = __funnelshift_r(kw[h][w0], kw[h][w0 + 1 < P::kKW ? w0 + 1 : w0], sh - 8);
-                            else x = shl<8 - sh>(kw[h][w0]);
-                            return row8((x & 0x3f00u) | lane8);
-                        };
-                        v0 = pair(std::integral_constant<int, 2 * s>{});
-                        v1 = pair(std::integral_constant<int, 2 * s + 1>{});
-                    }
-                    ak[h][0] = v0.x; ak[h][1] = v0.y; ak[h][2] = v1.x; ak[h][3] = v1.y;
-                } else {
-                    const uint4 v = row16(KB == 2 ? pick(kw[h][s >> 2], s & 3, lane16) : pick(s & 1 ? kw1[h] : kw[h][0], s >> 1, lane16));
-                    ak[h][0] = v.x; ak[h][1] = v.y; ak[h][2] = v.z; ak[h][3] = v.w;
-                }
-                // signs of two coordinates: bit b = (pair & 7) of both halves of the word (or of the word moved by 8), where it
-                // stands -- a subnormal number 2^(b - 24), which the operand of the query makes up for
-                as[h] = sw[h][s >> 2] & (0x00010001u << ((2 * s) & 7));
-                as[2 + h] = sw[h][s >> 2] & (0x00010001u << ((2 * s + 1) & 7));
-            }
+            key.template operands<s>(smem, lane8, lane16, ak, as);
             if constexpr (NQ == 4) {
                 mma16816(c1[0], ak[0], qf[0][s][0], qf[0][s][1]);
                 mma16816(c1[1], ak[1], qf[0][s][0], qf[0][s][1]);

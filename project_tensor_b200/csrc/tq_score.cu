@@ -216,8 +216,17 @@ score_matrix_kernel(TqDev p, const float* __restrict__ q, int qpg, const uint32_
                 for (int c = 0; c < 4; ++c) {
                     const int out = o + c * quarter, j = out < dp ? out : out - dp;
                     float* dst = qs + (j * 2 + (out < dp ? 0 : 1)) * QT;
+                    if constexpr (QT % 4 == 0) {
 #pragma unroll
-                    for (int u = 0; u < QT; ++u) dst[u] = (s > 0 ? dst[u] : 0.f) + (have[c] ? acc[c][u] : 0.f);
+                        for (int u = 0; u < QT; u += 4) {
+                            float4 f = s > 0 ? *reinterpret_cast<float4*>(dst + u) : make_float4(0.f, 0.f, 0.f, 0.f);
+                            if (have[c]) { f.x += acc[c][u]; f.y += acc[c][u + 1]; f.z += acc[c][u + 2]; f.w += acc[c][u + 3]; }
+                            *reinterpret_cast<float4*>(dst + u) = f;
+                        }
+                    } else {
+#pragma unroll
+                        for (int u = 0; u < QT; ++u) dst[u] = (s > 0 ? dst[u] : 0.f) + (have[c] ? acc[c][u] : 0.f);
+                    }
                 }
             }
             __syncthreads();
@@ -513,12 +522,9 @@ int tq_launch_score_batched(const tq_plan* p, const float* q, int groups, int qp
                             int64_t* top_idx, int64_t idx_base, void* scratch, size_t scratch_bytes,
                             cudaStream_t st, int64_t group_rows) {
     if (group_rows <= 0) group_rows = keys_per_group;
-    // One or two queries per group and the matrix wanted (the reference's own call): the streaming kernel.
+    // At most four queries per group and the matrix wanted: the warp-level kernel.
     if (p->path == TQ_PATH_AUTO && topk == 0 && scores && tq_score_few_supported(p, qpg) && keys_per_group > 0 && groups > 0)
         return tq_launch_score_few(p, q, groups, qpg, codes, signs, rnorms, norms, keys_per_group, scores, st, group_rows);
-    // Three or four queries per group (grouped-query decode): the lane-interleaved lookup-table kernel.
-    if (p->path == TQ_PATH_AUTO && topk == 0 && scores && tq_score_lut_supported(p, qpg) && keys_per_group > 0 && groups > 0)
-        return tq_launch_score_lut(p, q, groups, qpg, codes, signs, rnorms, norms, keys_per_group, scores, st, group_rows);
     // d = 64 has 8-byte sign rows (and 8- or 24-byte code rows): a group must start on a 16-byte boundary
     // for the bulk copies of the tensor-core kernel
     const bool aligned_groups = p->dev.d >= 128 || groups == 1 || group_rows % 2 == 0;

@@ -1,173 +1,277 @@
-// attention_score for one or two queries per group of keys (the reference's own call pattern: one query broadcast
-// over all keys, _quant.py:334-358), d = 128, 64 or 256, 1..4 code bits.
+// Scores of at most four queries per group of keys (one query against every key is the reference's own call pattern,
+// _quant.py:334-358; four are a grouped-query decode step), d = 128, 64 or 256, 1..4 code bits.
 //
 //   score(q, key) = norm * ( (R q) . codebook[codes]  +  alpha * rnorm * ((S q) . signs) )
 //
-// With so few queries the tensor-core kernel would idle most of each instruction (its cost does not shrink
-// with the number of queries below 16), and the arithmetic is tiny: the call is bound by reading 72 bytes per
-// key.  So this is a plain streaming kernel: per (group, query) the rotated and projected query are turned
-// into two lookup tables in shared memory,
+// The tcgen05 kernel costs the same below 16 queries; here the expansion of the packed keys in the registers of the lane that
+// feeds them to a warp-level matrix instruction is all there is to pay, once for up to four queries (their hi and lo parts side
+// by side are the eight columns).  A warp takes 16 keys at a time, the words of the next tile in
+// flight, no barriers; the tables (tq_mma.cuh) do not depend on the queries, so they are built while the matrices are on
+// their way, and the matrices while the queries are (page-locked host memory in a NumPy call).
 //
-//   pair table   [d/2 positions][4^bits entries]   c[code0] * (R q)[2p] + c[code1] * (R q)[2p+1]
-//   byte table   [d/8 positions][256 entries]      sum over the 8 sign bits of the byte of +-(S q)[coordinate]
-//
-// and every thread walks the packed codes and sign words of one key: d/2 + d/8 lookups and additions, no
-// unpacking.  The sums run in another order than the reference's (table entries are pairs / octets of
-// products), which keeps the scores within about 1e-6 relative of the float32 reference, inside the 1e-4 bound.
+// Bound: shared-memory lookups, 64 8-byte loads a key at d = 128 and 3-bit codes (2 cycles a warp and load, four lanes a key), and for
+// few keys the prologue.  Before -- one thread per key through tables of the query's own products, whose random rows met
+// in banks (another kernel for three or four queries) -- 1,048,576 keys of d = 128, 3-bit codes took 40 us for one query, 69 for
+// two, 84 for four, now 35 to 36; 262,147 keys and one query 19.7, now 15.2.
 #include "tq_common.cuh"
+#include "tq_mma.cuh"
 
 #include <stdint.h>
 
 namespace {
 
-constexpr int kFewThreads = 256;
+using namespace tqmma;
 
-// grid (blocks over keys, queries per group, groups)
-template <int BITS, int DR>
-__global__ void __launch_bounds__(kFewThreads)
-score_few_kernel(TqDev p, const float* __restrict__ q, const uint32_t* __restrict__ codes,
-                 const uint32_t* __restrict__ signs, const float* __restrict__ rnorms, const float* __restrict__ norms,
-                 int64_t keys_per_group, int64_t group_rows, int qpg, float* __restrict__ scores) {
-    constexpr int kPairs = DR / 2, kEntries = 1 << (2 * BITS), kBytes = DR / 8;
-    constexpr int kCodeWords = DR * BITS / 32, kSignWords = DR / 32;
-    constexpr uint32_t kMask = kEntries - 1;
-    extern __shared__ float tables[];
-    float* pair_t = tables;                       // [kPairs][kEntries]
-    float* byte_t = tables + kPairs * kEntries;   // [kBytes][256]
-    const int g = blockIdx.z, qi = blockIdx.y;
-    // Every block rotates and projects its query itself (2 d^2 FMAs, the matrices come from L2): rotated[j] =
-    // sum_k q[k] R[j][k], projected[j] = sum_k q[k] S[j][k], one FMA per k, k ascending as in the reference's
-    // matrix products.  That costs a few microseconds per block and saves a launch and a scratch buffer.
-    __shared__ float qs[DR], qr[DR], ps[DR];
-    if (threadIdx.x < DR) qs[threadIdx.x] = __ldg(q + ((size_t)g * qpg + qi) * DR + threadIdx.x);
-    __syncthreads();
-    if (threadIdx.x < DR) {
-        const int j = threadIdx.x;
-        float r = 0.f, sacc = 0.f;
-        for (int k0 = 0; k0 < DR; k0 += 16) {
-            float mr[16], ms[16];
-#pragma unroll
-            for (int u = 0; u < 16; ++u) {
-                mr[u] = __ldg(p.Rt + (size_t)(k0 + u) * DR + j);
-                ms[u] = __ldg(p.St + (size_t)(k0 + u) * DR + j);
-            }
-#pragma unroll
-            for (int u = 0; u < 16; ++u) {
-                r = fmaf(qs[k0 + u], mr[u], r);
-                sacc = fmaf(qs[k0 + u], ms[u], sacc);
-            }
-        }
-        qr[j] = r;
-        ps[j] = sacc;
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < kPairs * kEntries; i += kFewThreads) {
-        const int pp = i / kEntries, e = i - pp * kEntries;
-        const float c0 = __ldg(p.codebook + (e & ((1 << BITS) - 1))), c1 = __ldg(p.codebook + (e >> BITS));
-        pair_t[i] = fmaf(c1, qr[2 * pp + 1], c0 * qr[2 * pp]);
-    }
-    for (int i = threadIdx.x; i < kBytes * 256; i += kFewThreads) {
-        const int pos = i >> 8, v = i & 255, w = pos >> 2, b = pos & 3;
-        float acc = 0.f;
-#pragma unroll
-        for (int bit = 0; bit < 8; ++bit) {
-            // stored order of the sign words: even coordinates in bits 0..15, odd ones in bits 16..31
-            const int bp = 8 * b + bit;
-            const int coord = 32 * w + (bp < 16 ? 2 * bp : 2 * (bp - 16) + 1);
-            const float x = ps[coord];
-            acc += (v >> bit) & 1 ? x : -x;
-        }
-        byte_t[i] = acc;
-    }
-    __syncthreads();
+constexpr int kFewThreads = 512;
+constexpr int kFewWarps = kFewThreads / 32;
+constexpr int kTile = 16;           // keys a warp takes at a time
+constexpr int NQ = 4;               // queries of a pass
 
-    const float alpha = p.alpha;
-    float* out = scores + ((size_t)g * qpg + qi) * keys_per_group;
-    for (int64_t key = (int64_t)blockIdx.x * kFewThreads + threadIdx.x; key < keys_per_group;
-         key += (int64_t)gridDim.x * kFewThreads) {
-        const int64_t row = (int64_t)g * group_rows + key;
-        uint32_t cw[kCodeWords + 1], sw[kSignWords];
-        const uint32_t* crow = codes + row * kCodeWords;
-        const uint32_t* srow = signs + row * kSignWords;
-        if (kCodeWords % 4 == 0) {
+struct FewArgs {
+    const float* q;              // [groups][qpg][d]
+    const uint32_t* codes;
+    const uint32_t* signs;
+    const float* rnorms;
+    const float* norms;
+    int qpg;
+    int64_t keys_per_group, group_rows;
+    float* scores;               // [groups][qpg][keys_per_group]
+};
+
+template <int KB, int DR>
+struct FewPlan {
+    static constexpr int kSteps = DR / 16;
+    static constexpr int kSlices = kFewThreads / (DR / 2), kSliceLen = DR / kSlices;   // four outputs of one matrix and a slice of the sum per thread
+    static constexpr int off_slice = table_rows(KB) * kRowBytes;                     // [kSlices][2][NQ][DR] partial sums
+    static constexpr int off_vec = off_slice + kSlices * 2 * NQ * DR * 4;            // [2][NQ][DR] rotated, projected queries
+    static constexpr int off_qin = off_vec + 2 * NQ * DR * 4;                        // [DR][NQ]
+    static constexpr int off_small = off_qin + NQ * DR * 4;                          // [2][NQ] scales, [NQ] sums of the projected queries
+    static constexpr int total = off_small + 3 * NQ * 4;
+    static_assert(total <= 227 * 1024, "shared memory plan");
+};
+
+// grid (blocks over the keys, passes over the queries of a group, groups)
+template <int KB, int DR>
+__global__ void __launch_bounds__(kFewThreads, 1)
+score_few_kernel(const TqDev p, const FewArgs a) {
+    using P = FewPlan<KB, DR>;
+    using W = KeyWords<KB, DR>;
+    extern __shared__ __align__(128) unsigned char smem[];
+    float* vec = reinterpret_cast<float*>(smem + P::off_vec);
+    float* qin = reinterpret_cast<float*>(smem + P::off_qin);
+    float* slice = reinterpret_cast<float*>(smem + P::off_slice);
+    int* scl = reinterpret_cast<int*>(smem + P::off_small);                   // exponents of the queries' scales
+    float* psum = reinterpret_cast<float*>(smem + P::off_small) + 2 * NQ;
+
+    const int g = blockIdx.z, q0 = blockIdx.y * NQ;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int t = lane & 3, r = lane >> 2;      // position in the quad, row of the fragments
+    const uint32_t keys = (uint32_t)a.keys_per_group;            // rows of all groups together stay below 2^32
+    const uint32_t tiles = (uint32_t)((a.keys_per_group + kTile - 1) / kTile), stride = gridDim.x * kFewWarps;
+    // neighbouring tiles go to different blocks: with fewer tiles than warps every SM has some
+    uint32_t tile = (uint32_t)warp * gridDim.x + blockIdx.x;
+
+    // the matrices: in flight before anything else is waited for
+    const int xm = tid / (DR / 4) & 1, xj = tid % (DR / 4) * 4, xk = tid / (DR / 2) * P::kSliceLen;    // matrix, first output, slice
+    constexpr int kBatch = P::kSliceLen < 16 ? P::kSliceLen : 16;
+    static_assert(P::kSliceLen % kBatch == 0, "slices");
+    const float* msrc = (xm ? p.St : p.Rt) + (size_t)xk * DR + xj;
+    float4 mat[kBatch];
 #pragma unroll
-            for (int k = 0; k < kCodeWords; k += 4) {
-                const uint4 v = __ldg(reinterpret_cast<const uint4*>(crow + k));
-                cw[k] = v.x; cw[k + 1] = v.y; cw[k + 2] = v.z; cw[k + 3] = v.w;
+    for (int u = 0; u < kBatch; ++u) mat[u] = __ldg(reinterpret_cast<const float4*>(msrc + (size_t)u * DR));
+
+    const int64_t row_base = (int64_t)g * a.group_rows;
+    const int kbit = W::kBits * t, kshift = kbit & 31;
+    const uint32_t* kc_base = a.codes + row_base * (DR * KB / 32) + (kbit >> 5);
+    const uint32_t* sg_base = a.signs + row_base * (DR / 32) + (DR == 256 ? 2 * t : DR == 128 ? t : t >> 1);
+    const float* kn_base = a.norms + row_base;
+    const float* rn_base = a.rnorms + row_base;
+    struct Words { uint32_t kc[2][W::kWords], sg[2][W::kSigns]; float kn[2], rn[2]; };
+    auto fetch = [&](uint32_t tl, Words& w) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t key = min(tl * kTile + r + 8 * h, keys - 1);       // rows behind the last one: read that one
+            const uint32_t* src = kc_base + (size_t)key * (DR * KB / 32);
+            if constexpr (W::kBits % 128 == 0) {
+#pragma unroll
+                for (int i = 0; i < W::kWords; i += 4) {
+                    const uint4 v = __ldg(reinterpret_cast<const uint4*>(src + i));
+                    w.kc[h][i] = v.x; w.kc[h][i + 1] = v.y; w.kc[h][i + 2] = v.z; w.kc[h][i + 3] = v.w;
+                }
+            } else if constexpr (W::kBits % 64 == 0) {
+#pragma unroll
+                for (int i = 0; i < W::kWords; i += 2) {
+                    const uint2 v = __ldg(reinterpret_cast<const uint2*>(src + i));
+                    w.kc[h][i] = v.x; w.kc[h][i + 1] = v.y;
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < W::kWords; ++i) w.kc[h][i] = __ldg(src + i);
             }
-        } else {
 #pragma unroll
-            for (int k = 0; k < kCodeWords; k += 2) {
-                const uint2 v = __ldg(reinterpret_cast<const uint2*>(crow + k));
-                cw[k] = v.x; cw[k + 1] = v.y;
+            for (int i = 0; i < W::kSigns; ++i) w.sg[h][i] = __ldg(sg_base + (size_t)key * (DR / 32) + i);
+            w.kn[h] = __ldg(kn_base + key);
+            w.rn[h] = __ldg(rn_base + key);
+        }
+    };
+    Words cur;
+    if (tile < tiles) fetch(tile, cur);
+    for (int i = tid; i < NQ * DR; i += kFewThreads) {
+        const int qq = i / DR, k = i - qq * DR;
+        qin[k * NQ + qq] = q0 + qq < a.qpg ? __ldg(a.q + ((size_t)g * a.qpg + q0 + qq) * DR + k) : 0.f;
+    }
+    build_key_table<KB>(smem, p.codebook, tid, kFewThreads);
+    __syncthreads();
+    {   // rotated[j] = sum_k q[k] R[j][k], projected[j] = sum_k q[k] S[j][k] in 32-bit arithmetic
+        float4 sum[NQ];
+#pragma unroll
+        for (int qq = 0; qq < NQ; ++qq) sum[qq] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int b = 0; b < P::kSliceLen; b += kBatch) {
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) {
+                const float* qk = qin + (xk + b + u) * NQ;
+#pragma unroll
+                for (int qq = 0; qq < NQ; ++qq) {
+                    const float v = qk[qq];
+                    sum[qq].x = fmaf(v, mat[u].x, sum[qq].x);
+                    sum[qq].y = fmaf(v, mat[u].y, sum[qq].y);
+                    sum[qq].z = fmaf(v, mat[u].z, sum[qq].z);
+                    sum[qq].w = fmaf(v, mat[u].w, sum[qq].w);
+                }
+            }
+            if (b + kBatch < P::kSliceLen) {
+#pragma unroll
+                for (int u = 0; u < kBatch; ++u) mat[u] = __ldg(reinterpret_cast<const float4*>(msrc + (size_t)(b + kBatch + u) * DR));
             }
         }
-        cw[kCodeWords] = 0u;
 #pragma unroll
-        for (int k = 0; k < kSignWords; k += 2) {
-            const uint2 v = __ldg(reinterpret_cast<const uint2*>(srow + k));
-            sw[k] = v.x; sw[k + 1] = v.y;
+        for (int qq = 0; qq < NQ; ++qq) *reinterpret_cast<float4*>(slice + ((tid / (DR / 2) * 2 + xm) * NQ + qq) * DR + xj) = sum[qq];
+    }
+    __syncthreads();
+    for (int v = warp; v < 2 * NQ; v += kFewWarps) {      // a warp per vector: slices added up, largest value, sum
+        float m = 0.f, sum = 0.f;
+#pragma unroll
+        for (int k = lane; k < DR; k += 32) {
+            float x = slice[v * DR + k];
+#pragma unroll
+            for (int u = 1; u < P::kSlices; ++u) x += slice[(u * 2 * NQ + v) * DR + k];
+            vec[v * DR + k] = x;
+            m = fmaxf(m, fabsf(x));
+            sum += x;
         }
-        const float nrm = __ldg(norms + row), rn = __ldg(rnorms + row);
-        float s1[4] = {0.f, 0.f, 0.f, 0.f}, s2[2] = {0.f, 0.f};
 #pragma unroll
-        for (int pp = 0; pp < kPairs; ++pp) {
-            const int bit = pp * 2 * BITS, wi = bit >> 5, sh = bit & 31;
-            uint32_t e;
-            if (sh + 2 * BITS <= 32) e = (cw[wi] >> sh) & kMask;
-            else e = __funnelshift_r(cw[wi], cw[wi + 1], sh) & kMask;
-            s1[pp & 3] += pair_t[pp * kEntries + e];
+        for (int o = 16; o > 0; o >>= 1) {
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+            sum += __shfl_xor_sync(0xffffffffu, sum, o);
         }
+        if (lane == 0) {
+            scl[v] = scale_exp(m);
+            if (v >= NQ) psum[v - NQ] = sum;
+        }
+    }
+    __syncthreads();
+    // Query operands: column r is hi (r < 4) or lo (r >= 4) of query r & 3.  The projected query makes up for the place 2^(b - 24) of
+    // the sign bits.
+    uint32_t qf[2][P::kSteps][2];
 #pragma unroll
-        for (int pos = 0; pos < kBytes; ++pos) s2[pos & 1] += byte_t[pos * 256 + ((sw[pos >> 2] >> (8 * (pos & 3))) & 255u)];
-        const float a1 = (s1[0] + s1[1]) + (s1[2] + s1[3]);
-        out[key] = nrm * fmaf(alpha * rn, s2[0] + s2[1], a1);
+    for (int m = 0; m < 2; ++m) {
+        const float* x = vec + (m * NQ + (r & 3)) * DR + t * (DR / 4);
+        const float sc = pow2i(scl[m * NQ + (r & 3)]);
+#pragma unroll
+        for (int s = 0; s < P::kSteps; ++s) {
+            uint32_t h0, l0, h1, l1;
+            const float s0 = m == 0 ? sc : sc * (1.f / (1 << ((2 * s) & 7))), s1 = m == 0 ? sc : sc * (1.f / (1 << ((2 * s + 1) & 7)));
+            const float4 f = *reinterpret_cast<const float4*>(x + 4 * s);
+            split_pair(f.x * s0, f.y * s0, h0, l0);
+            split_pair(f.z * s1, f.w * s1, h1, l1);
+            qf[m][s][0] = r < 4 ? h0 : l0;
+            qf[m][s][1] = r < 4 ? h1 : l1;
+        }
+    }
+    // the two queries of this lane's score columns; a sign is 2 bit - 1
+    float ds1[2], ds2[2], dsum[2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        const int qq = (2 * t + c) & (NQ - 1);
+        ds1[c] = pow2i(-scl[qq]) * (1.f / kCentScale);
+        ds2[c] = pow2i(25 - scl[NQ + qq]) * p.alpha;
+        dsum[c] = 2 * t < NQ ? -p.alpha * psum[qq] : 0.f;     // (once: hi and lo columns are added)
+    }
+    const uint32_t lane8 = (uint32_t)(lane & 15) * 8u, lane16 = (uint32_t)(lane & 7) * 16u;
+    // The lane's scores: queries 2 (t & 1) + c of key r + 8 (t >> 1) -- adding hi and lo columns leaves both lanes with the sum.
+    const int qs0 = q0 + 2 * (t & 1);
+    float* out = a.scores + ((int64_t)g * a.qpg + qs0) * a.keys_per_group;
+
+    for (; tile < tiles; tile += stride) {
+        Words nxt;
+        if (tile + stride < tiles) fetch(tile + stride, nxt);
+        W key;
+        key.unpack(cur.kc, cur.sg, kshift, t);
+        float c1[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, c2[4] = {0.f, 0.f, 0.f, 0.f};
+        for_steps<P::kSteps>([&](auto sc) {
+            constexpr int s = decltype(sc)::value;
+            uint32_t ak[2][4], as[4];
+            key.template operands<s>(smem, lane8, lane16, ak, as);
+            mma16816(c1[0], ak[0], qf[0][s][0], qf[0][s][1]);
+            mma16816(c1[1], ak[1], qf[0][s][0], qf[0][s][1]);
+            mma16816(c2, as, qf[1][s][0], qf[1][s][1]);
+        });
+        float v[2][2];                 // [key r + 8 h][query column c]
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                float s = fmaf(fmaf(c2[2 * h + c], ds2[c], dsum[c]), cur.rn[h], (c1[h][c] + c1[h][2 + c]) * ds1[c]);
+                s += __shfl_xor_sync(0xffffffffu, s, 2);     // hi and lo columns
+                v[h][c] = s * cur.kn[h];
+            }
+        const uint32_t k0 = tile * kTile + r + 8 * (t >> 1);
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+            if (qs0 + c < a.qpg && k0 < keys) out[c * a.keys_per_group + k0] = t < 2 ? v[0][c] : v[1][c];
+        cur = nxt;
     }
 }
 
-template <int BITS, int DR>
-int launch_few(const tq_plan* p, const float* q, const uint32_t* codes, const uint32_t* signs, const float* rnorms,
-               const float* norms, int64_t keys_per_group, int64_t group_rows, int groups, int qpg, float* scores,
-               cudaStream_t st) {
-    const int sm = ((DR / 2) * (1 << (2 * BITS)) + (DR / 8) * 256) * 4;
-    TQ_GRANT_SMEM((score_few_kernel<BITS, DR>), sm, p->device);
-    const int sms = tq_sm_count(p->device);
-    int64_t blocks = (keys_per_group + kFewThreads - 1) / kFewThreads;
-    const int64_t cap = (int64_t)sms * 4;   // the tables cost a few microseconds per block: a few blocks per SM, grid-stride
-    if (blocks > cap) blocks = cap;
-    score_few_kernel<BITS, DR><<<dim3((unsigned)blocks, (unsigned)qpg, (unsigned)groups), kFewThreads, sm, st>>>(
-        p->dev, q, codes, signs, rnorms, norms, keys_per_group, group_rows, qpg, scores); tq_count_launch();
+template <int KB, int DR>
+int launch_few(const tq_plan* p, const FewArgs& a, int groups, cudaStream_t st) {
+    using P = FewPlan<KB, DR>;
+    TQ_GRANT_SMEM((score_few_kernel<KB, DR>), P::total, p->device);
+    const int passes = (a.qpg + NQ - 1) / NQ;
+    // a block per SM over all groups (its prologue costs some 4 us): every block of a group gets at least a tile per warp
+    int64_t blocks = (tq_sm_count(p->device) + (int64_t)passes * groups - 1) / ((int64_t)passes * groups);
+    const int64_t tiles = (a.keys_per_group + kTile - 1) / kTile, most = (tiles + 3) / 4;
+    if (blocks > most) blocks = most;
+    score_few_kernel<KB, DR><<<dim3((unsigned)blocks, (unsigned)passes, (unsigned)groups), kFewThreads, P::total, st>>>(p->dev, a); tq_count_launch();
     TQ_CUDA_TRY(cudaGetLastError());
     return TQ_OK;
 }
-
 }  // namespace
 
-// d = 128 and 64: one or two queries (from three on, the lookup-table kernel for four and the tensor-core kernel are
-// faster).  d = 256: one query (a pass over the packed keys per query; against 1,048,576 keys one query takes 145 us here
-// and 201 us on the tensor-core kernel, two 228 and 200, four 394 and 194).
+// Beyond these counts (d = 128 with up to 3 code bits: four queries; d = 64 and 4 bits: two; d = 256: one) a matrix has the very
+// bits of the top-k search, whose kernel is the tcgen05 one, and keeps them.
 bool tq_score_few_supported(const tq_plan* p, int qpg) {
-    if (!p->has_projection || p->dev.bits < 1 || p->dev.bits > 4 || qpg < 1) return false;
-    if (p->dev.d == 256) return qpg == 1;
-    return (p->dev.d == 128 || p->dev.d == 64) && qpg <= 2;
+    const int d = p->dev.d, bits = p->dev.bits;
+    if (!p->has_projection || bits < 1 || bits > 4 || qpg < 1) return false;
+    return d == 128 ? qpg <= (bits <= 3 ? 4 : 2) : d == 64 ? qpg <= 2 : d == 256 && qpg == 1;
 }
 
 // scores: [groups][qpg][keys_per_group]
 int tq_launch_score_few(const tq_plan* p, const float* q, int groups, int qpg, const uint32_t* codes, const uint32_t* signs,
                         const float* rnorms, const float* norms, int64_t keys_per_group, float* scores, cudaStream_t st,
                         int64_t group_rows) {
-    TqRange range("tq.score.one_or_two_queries");
+    TqRange range("tq.score.few_queries");
     if (group_rows <= 0) group_rows = keys_per_group;
-    const int d = p->dev.d, bits = p->dev.bits;
-    int r = TQ_ERR_UNSUPPORTED;
-#define TQ_FEW(B)                                                                                                        \
-    case B:                                                                                                             \
-        r = d == 64 ? launch_few<B, 64>(p, q, codes, signs, rnorms, norms, keys_per_group, group_rows, groups, qpg, scores, st)     \
-            : d == 256 ? launch_few<B, 256>(p, q, codes, signs, rnorms, norms, keys_per_group, group_rows, groups, qpg, scores, st) \
-                       : launch_few<B, 128>(p, q, codes, signs, rnorms, norms, keys_per_group, group_rows, groups, qpg, scores, st); \
-        break;
-    switch (bits) { TQ_FEW(1) TQ_FEW(2) TQ_FEW(3) TQ_FEW(4) }
+    const FewArgs a{q, codes, signs, rnorms, norms, qpg, keys_per_group, group_rows, scores};
+    const int d = p->dev.d;
+    switch (p->dev.bits) {
+#define TQ_FEW(B)                                                                                                    \
+    case B:                                                                                                         \
+        return d == 64 ? launch_few<B, 64>(p, a, groups, st) : d == 256 ? launch_few<B, 256>(p, a, groups, st) \
+                                                                                : launch_few<B, 128>(p, a, groups, st);
+        TQ_FEW(1) TQ_FEW(2) TQ_FEW(3) TQ_FEW(4)
 #undef TQ_FEW
-    if (r == TQ_ERR_UNSUPPORTED) return tq_fail(r, "no few-query scoring kernel for d=%d bits=%d", d, bits);
-    return r;
+    }
+    return tq_fail(TQ_ERR_UNSUPPORTED, "no few-query scoring kernel for d=%d bits=%d", d, p->dev.bits);
 }

@@ -1,0 +1,29 @@
+"""Scores of one to four queries per group: tiles of 16 keys with a remainder, fewer tiles than warps, every code width, groups --
+against q . dequantize(key) in 64-bit."""
+import pytest
+
+import project_tensor_b200 as tg
+import parity
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("d", [64, 128, 256])
+@pytest.mark.parametrize("bits", [2, 3, 4, 5])
+def test_few_queries(d, bits):
+    import torch
+    quant = tg.TurboQuantProd(d, bits, seed=2026)
+    gen = torch.Generator("cuda").manual_seed(d + bits)
+    for groups, qpg, n in ((1, 1, 1), (1, 1, 15), (3, 1, 4097), (1, 2, 17), (2, 2, 2368), (1, 3, 37889), (4, 4, 530), (1, 1, 300001)):
+        keys = torch.randn(groups * n, d, device="cuda", generator=gen)
+        keys[n // 2] = 0
+        queries = torch.randn(groups * qpg, d, device="cuda", generator=gen) * 100
+        queries[0] *= 1e-4
+        enc = quant.quantize(keys)
+        got = quant.attention_scores(queries, enc, groups=groups)
+        want = torch.einsum("gqd,gnd->gqn", queries.view(groups, qpg, d).double(),
+                            quant.dequantize(enc).double().view(groups, n, d)).reshape(groups * qpg, n)
+        knorm = keys.norm(dim=1).view(groups, 1, n).expand(groups, qpg, n).reshape(groups * qpg, n)
+        err = parity.max_score_err(got.cpu().numpy(), want.cpu().numpy(), queries.norm(dim=1)[:, None].cpu().numpy(),
+                                   knorm.cpu().numpy(), d)
+        assert err <= 2e-5, (groups, qpg, n, err)
