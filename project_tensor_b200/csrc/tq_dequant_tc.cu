@@ -17,7 +17,8 @@
 //                          successive tiles)
 //   MMA (1 thread)         operand by operand: C_hi x (Rt_hi, Rt_lo), C_lo x Rt_hi [, B_hi x (St_hi, St_lo),
 //                          B_lo x St_hi], N = 128, accumulators double-buffered
-//   epilogue (8 warps)     two threads per key: tcgen05.ld, times norm * 2^-20, then through shared memory and tensor stores
+//   epilogue (8 warps)     two threads per key: tcgen05.ld, times norm * 2^-20, then through a staging block in
+//                          shared memory so that every global store instruction writes whole 128-byte lines
 //
 // Every wait is bounded; a wait that runs out sets the plan's status word and the kernel drains.
 #include "tq_common.cuh"
@@ -78,8 +79,9 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
 
 // Reconstructed rows leave through shared memory: an epilogue warp writes 32 x 32 floats (row = lane, 16-byte pieces swizzled by
 // the row as the tensor map says, so that no two lanes of a store meet in a bank) and one lane starts a tensor store, which
-// clips the rows behind the last.  (Loading the block back and storing it with the warp's own instructions made the epilogue the
-// longest role: 3,200 cycles a block.)
+// clips the rows behind the last.  d = 256, where the accumulators are not double-buffered: loading the block back and storing it
+// with the warp's own instructions made the epilogue the longest role, 3,200 cycles a block.  (At d = 128 the two are
+// equal, at d = 64 the own stores are the faster ones, 76 against 86 us for 1,048,576 vectors.)
 constexpr int kBlockBytes = 32 * 128;
 template <int BUFS>
 struct BlockStore {
@@ -127,20 +129,16 @@ struct DqSmem {
     static constexpr int kRowExtra = PROD ? kSignRowBytes : 0;   // sign words
     static constexpr int kStageBytes = kTileKeys * (kCodeRowBytes + kRowExtra);
     static constexpr int kNumB = PROD ? 4 : 2;
-    static constexpr int kOutBufs = 2;                            // 4 KB blocks per epilogue warp
-    static constexpr int kOutRowBytes = 36 * 4;                   // pair mode: 32 floats of a row + padding against bank conflicts
-    static constexpr int kOutWarpBytes = kOutBufs * kBlockBytes;  // staging of one epilogue warp (a pair-mode block fits)
-    static constexpr int off_out = 0;                             // (the swizzle wants blocks on 1 KB boundaries)
-    static constexpr int off_lut = off_out + 8 * kOutWarpBytes;
+    static constexpr int kStages = PROD ? 4 : 6;
+    static constexpr int kOutRowBytes = 36 * 4;                   // 32 floats of a row + padding against bank conflicts
+    static constexpr int kOutWarpBytes = 32 * kOutRowBytes;       // staging block of one epilogue warp
+    static constexpr int off_lut = 0;
     static constexpr int off_b = off_lut + kLutBytes;
     static constexpr int off_ring = off_b + kNumB * kMatBytes;
-    static constexpr int kMisc = 512 + 128 + 2 * kTileKeys * 4;   // barriers; pair mode: partial dot products [2 tiles][128]
-    static constexpr int kStageRoom = (227 * 1024 - 1024 - off_ring - kMisc) / kStageBytes;
-    static constexpr int kStages = kStageRoom < 6 ? kStageRoom : 6;
-    static_assert(kStages >= 2, "shared memory plan");
-    static constexpr int off_misc = off_ring + kStages * kStageBytes;
-    static constexpr int off_pair = off_misc + 512 + 128;
-    static constexpr int total = off_misc + kMisc + 1024;         // + slack to align the base
+    static constexpr int off_out = off_ring + kStages * kStageBytes;
+    static constexpr int off_misc = off_out + 8 * kOutWarpBytes;
+    static constexpr int off_pair = off_misc + 512 + 128;           // pair mode: partial dot products [2 tiles][128]
+    static constexpr int total = off_pair + 2 * kTileKeys * 4;
     static_assert(total <= 227 * 1024, "shared memory plan");
 };
 
@@ -148,7 +146,7 @@ struct DqSmem {
 // index and summed: attention_score with one query per key (_quant.py:342-358), which equals q . dequantize(key).
 template <int BITS, bool PROD, int DR, bool PAIR>
 __global__ void __launch_bounds__(kThreads, 1)
-dequant_tc_kernel(const __grid_constant__ CUtensorMap tmap_out, const DequantArgs a) {
+dequant_tc_kernel(const DequantArgs a) {
     static_assert(DR == 128 || DR == 64, "written for d = 128 and d = 64");
     // d = 64: the expander warps and the epilogue warps of the upper half idle, the contractions stop after
     // DR / 16 k-blocks and cover N = DR output coordinates
@@ -157,7 +155,7 @@ dequant_tc_kernel(const __grid_constant__ CUtensorMap tmap_out, const DequantArg
     constexpr int kStages = L::kStages;
     constexpr int kOps = PROD ? 4 : 2;   // operands per tile: C_hi, C_lo [, B_hi, B_lo]
     extern __shared__ unsigned char smem_raw[];
-    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
     const uint32_t smem_base = smem_u32(smem);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::off_misc);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + DB_COUNT);
@@ -384,7 +382,6 @@ dequant_tc_kernel(const __grid_constant__ CUtensorMap tmap_out, const DequantArg
         const int row = quarter * 32 + lane;
         const int colhalf = (warp - kFirstEpiWarp) >> 2;
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
-        BlockStore<L::kOutBufs> store{smem + L::off_out + (warp - kFirstEpiWarp) * L::kOutWarpBytes, 0};
         float nrm_next = 0.f;
         if (my_tiles > 0) {
             const int64_t r0 = (int64_t)blockIdx.x * kTileKeys + row;
@@ -458,12 +455,28 @@ dequant_tc_kernel(const __grid_constant__ CUtensorMap tmap_out, const DequantArg
                 if (colhalf == 0 && grow < n_live) a.out[grow] = dot * sc;
                 continue;
             }
-            store.write(va, sc, lane);
-            store.send(&tmap_out, colhalf * 64, row0, row0 < n_live, lane);
-            store.write(vb, sc, lane);
-            store.send(&tmap_out, colhalf * 64 + 32, row0, row0 < n_live, lane);
+            // Through a per-warp staging block in shared memory, so that the global stores of a warp cover
+            // whole 128-byte lines (four rows x 32 floats per instruction) instead of 16 bytes of 32 rows.
+#pragma unroll
+            for (int ch = 0; ch < 2; ++ch) {
+                float4* mine = reinterpret_cast<float4*>(stg + lane * L::kOutRowBytes);
+#pragma unroll
+                for (int m = 0; m < 8; ++m) {
+                    const uint32_t* v = ch == 0 ? va : vb;
+                    mine[m] = make_float4(__uint_as_float(v[4 * m]) * sc, __uint_as_float(v[4 * m + 1]) * sc,
+                                          __uint_as_float(v[4 * m + 2]) * sc, __uint_as_float(v[4 * m + 3]) * sc);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int it = 0; it < 8; ++it) {
+                    const int r = it * 4 + (lane >> 3), c4 = lane & 7;
+                    const float4 val = *reinterpret_cast<const float4*>(stg + r * L::kOutRowBytes + c4 * 16);
+                    if (row0 + r < n_live)
+                        __stcs(reinterpret_cast<float4*>(a.out + (row0 + r) * DR + colhalf * 64 + ch * 32) + c4, val);
+                }
+                __syncwarp();
+            }
         }
-        if (!PAIR) store.close(lane);
     }
 
     // ---- teardown ---------------------------------------------------------------------------------
@@ -880,12 +893,9 @@ int launch_256(const tq_plan* p, const DequantArgs& args, int grid, cudaStream_t
 
 template <int BITS, bool PROD, int DR, bool PAIR = false>
 int launch_one(const tq_plan* p, const DequantArgs& args, int grid, cudaStream_t st) {
-    CUtensorMap map{};
-    const int rc = PAIR ? TQ_OK : output_map(args.out, args.n, DR, &map);
-    if (rc != TQ_OK) return rc;
     const int sm = DqSmem<BITS, PROD, DR>::total;
     TQ_GRANT_SMEM((dequant_tc_kernel<BITS, PROD, DR, PAIR>), sm, p->device);
-    dequant_tc_kernel<BITS, PROD, DR, PAIR><<<grid, kThreads, sm, st>>>(map, args); tq_count_launch();
+    dequant_tc_kernel<BITS, PROD, DR, PAIR><<<grid, kThreads, sm, st>>>(args); tq_count_launch();
     TQ_CUDA_TRY(cudaGetLastError());
     return TQ_OK;
 }
