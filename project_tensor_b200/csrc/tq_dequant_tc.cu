@@ -198,6 +198,7 @@ dequant_tc_kernel(const DequantArgs a) {
         tmem_relinquish();
     }
     tc_fence_before();
+    tq_grid_wait();         // (only constants of the plan have been read so far)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
@@ -582,6 +583,7 @@ dequant256_kernel(const __grid_constant__ CUtensorMap tmap_out, const DequantArg
         tmem_relinquish();
     }
     tc_fence_before();
+    tq_grid_wait();         // (only constants of the plan have been read so far)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
@@ -886,8 +888,7 @@ int launch_256(const tq_plan* p, const DequantArgs& args, int grid, cudaStream_t
     if (rc != TQ_OK) return rc;
     const int sm = dq256::Smem<BITS, PROD>::total;
     TQ_GRANT_SMEM((dequant256_kernel<BITS, PROD>), sm, p->device);
-    dequant256_kernel<BITS, PROD><<<grid, dq256::kThreads256, sm, st>>>(map, args); tq_count_launch();
-    TQ_CUDA_TRY(cudaGetLastError());
+    TQ_CUDA_TRY(tq_launch_dependent(dequant256_kernel<BITS, PROD>, dim3(grid), dim3(dq256::kThreads256), (size_t)sm, st, map, args));
     return TQ_OK;
 }
 
@@ -895,8 +896,7 @@ template <int BITS, bool PROD, int DR, bool PAIR = false>
 int launch_one(const tq_plan* p, const DequantArgs& args, int grid, cudaStream_t st) {
     const int sm = DqSmem<BITS, PROD, DR>::total;
     TQ_GRANT_SMEM((dequant_tc_kernel<BITS, PROD, DR, PAIR>), sm, p->device);
-    dequant_tc_kernel<BITS, PROD, DR, PAIR><<<grid, kThreads, sm, st>>>(args); tq_count_launch();
-    TQ_CUDA_TRY(cudaGetLastError());
+    TQ_CUDA_TRY(tq_launch_dependent(dequant_tc_kernel<BITS, PROD, DR, PAIR>, dim3(grid), dim3(kThreads), (size_t)sm, st, args));
     return TQ_OK;
 }
 

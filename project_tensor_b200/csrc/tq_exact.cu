@@ -299,6 +299,8 @@ exact_quantize_few_kernel(const __grid_constant__ RowsJob first, const __grid_co
     }
     if (j < 8) cs[r][128 + j] = 0;
     const uint32_t inv_bits = inverse_of_bits(p.bits);
+    tq_grid_release();
+    tq_grid_wait();         // (only constants of the plan have been read so far)
     RowSource rows;
     rows.open(job, block == 0);
     for (int64_t g0 = (int64_t)block * RB; g0 < rows.limit; g0 += (int64_t)nblocks * RB) {
@@ -481,7 +483,9 @@ exact_quantize_tile_kernel(const __grid_constant__ RowsJob first, const __grid_c
     __shared__ int64_t src_row[RB], dst_row[RB];
     const int t = threadIdx.x, tx = t % CT, ty = t / CT, lane = t & 31, l8 = t & 7, grp = t >> 3;
     RowSource rows;
+    tq_grid_release();
     if (job.lists.hdr != nullptr && !prod) {     // the list of a TurboQuantMSE call is empty as a rule
+        tq_grid_wait();
         rows.open(job, block == 0);
         if (rows.limit == 0) return;
     }
@@ -491,6 +495,7 @@ exact_quantize_tile_kernel(const __grid_constant__ RowsJob first, const __grid_c
         cbk[i] = __ldg(p.codebook + i);
         if (i + 1 < levels) bnd[i] = __ldg(p.boundaries + i);
     }
+    tq_grid_wait();         // (only constants of the plan have been read so far)
     rows.open(job, block == 0);
     const uint32_t inv_bits = inverse_of_bits(p.bits);
     if (t < RB)
@@ -625,10 +630,12 @@ exact_code_check_kernel(const __grid_constant__ CheckJob first, const __grid_con
     // entries warp, warp + kStep, ... of the block: the lanes of different entries meet in different banks
     const int e = warp + kStep * (lane / kLanes), l = lane & (kLanes - 1);
     const TqRecheck& lists = job.lists;
+    if (t < p.levels - 1) bnd[t] = __ldg(p.boundaries + t);      // (at most 15: the tensor-core kernels take up to 4 bits)
+    tq_grid_release();
+    tq_grid_wait();
     // asked for before the header is known to allow it (the list's capacity bounds the index)
     unsigned int at = block * E + e;
     unsigned long long ent = at < lists.code_cap ? lists.code_entries[at] : 0ull;
-    if (t < p.levels - 1) bnd[t] = __ldg(p.boundaries + t);      // (at most 15: the tensor-core kernels take up to 4 bits)
     if (lists.hdr->overflow) return;  // the row pass will redo everything
     const unsigned int count = min(lists.hdr->n_codes, lists.code_cap);
     for (unsigned int at0 = block * E; at0 < count; at0 += nblocks * E) {
@@ -829,12 +836,10 @@ int tq_launch_exact_code_check(const TqSecondStage* a, const TqSecondStage* b, c
     };
     const CheckJob first = job(a), second = b ? job(b) : first;
     const int b0 = blocks(a), grid = b0 + (b ? blocks(b) : 0);
-    if (d == 128) exact_code_check_kernel<128><<<grid, 256, 0, st>>>(first, second, b0);
-    else if (d == 64) exact_code_check_kernel<64><<<grid, 256, 0, st>>>(first, second, b0);
-    else if (d == 256) exact_code_check_kernel<256><<<grid, 256, 0, st>>>(first, second, b0);
+    if (d == 128) TQ_CUDA_TRY(tq_launch_dependent(exact_code_check_kernel<128>, dim3(grid), dim3(256), 0, st, first, second, b0));
+    else if (d == 64) TQ_CUDA_TRY(tq_launch_dependent(exact_code_check_kernel<64>, dim3(grid), dim3(256), 0, st, first, second, b0));
+    else if (d == 256) TQ_CUDA_TRY(tq_launch_dependent(exact_code_check_kernel<256>, dim3(grid), dim3(256), 0, st, first, second, b0));
     else return tq_fail(TQ_ERR_UNSUPPORTED, "the coordinate re-check is written for d = 64, 128 and 256");
-    tq_count_launch();
-    TQ_CUDA_TRY(cudaGetLastError());
     return TQ_OK;
 }
 
@@ -856,8 +861,7 @@ int launch_few_rows(const RowsJob& a, const RowsJob* b, int64_t rows, int device
     split_room(b, rows, RB, tq_sm_count(device), &b0, &b1);
     const int sm = (a.prod || (b && b->prod) ? 3 : 1) * ((a.p.d * a.p.d + 3) / 4 * 16);
     TQ_GRANT_SMEM((exact_quantize_few_kernel<RB>), sm, device);
-    exact_quantize_few_kernel<RB><<<b0 + b1, 128 * RB, sm, st>>>(a, b ? *b : a, b0, advance); tq_count_launch();
-    TQ_CUDA_TRY(cudaGetLastError());
+    TQ_CUDA_TRY(tq_launch_dependent(exact_quantize_few_kernel<RB>, dim3(b0 + b1), dim3(128 * RB), (size_t)sm, st, a, b ? *b : a, b0, advance));
     return TQ_OK;
 }
 // Blocks of a kernel that an SM's registers hold (its shared memory is a matter of the shape); asked for once per kernel.
@@ -892,8 +896,8 @@ int launch_tile_rows(const RowsJob& a, const RowsJob* b, int64_t rows, int devic
     if (shape.stages == 0) return tq_fail(TQ_ERR_UNSUPPORTED, "no tile shape for d=%d", a.p.d);
     split_room(b, rows, T::kRB, (int64_t)tq_sm_count(device) * per_sm, &b0, &b1);
     TQ_GRANT_SMEM((exact_quantize_tile_kernel<RT, TR, CT, TC>), shape.bytes, device);
-    exact_quantize_tile_kernel<RT, TR, CT, TC><<<b0 + b1, T::kThreads, shape.bytes, st>>>(a, b ? *b : a, b0, advance, shape); tq_count_launch();
-    TQ_CUDA_TRY(cudaGetLastError());
+    TQ_CUDA_TRY(tq_launch_dependent(exact_quantize_tile_kernel<RT, TR, CT, TC>, dim3(b0 + b1), dim3(T::kThreads), shape.bytes, st, a, b ? *b : a, b0,
+                                    advance, shape));
     return TQ_OK;
 }
 // Rows per block: one while every row can have an SM to itself (d <= 128), then four, 16 (8 at d = 256) while larger blocks would leave

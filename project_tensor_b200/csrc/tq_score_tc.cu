@@ -195,6 +195,7 @@ score_tc_kernel(const __grid_constant__ CUtensorMap tmap_out, const __grid_const
     const uint32_t bar0 = smem_u32(bars);
     auto BAR = [&](int i) { return bar0 + 8u * (uint32_t)i; };
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (a.run_if || a.dyn_keys) tq_grid_wait();      // words of kernels before
     if (a.run_if && *a.run_if == 0u) return;
     const uint32_t total_tiles = (uint32_t)(a.dyn_keys ? ((int64_t)*a.dyn_keys + kTileKeys - 1) / kTileKeys : a.total_tiles);
     const uint32_t tiles_per_group = (uint32_t)a.tiles_per_group;
@@ -238,6 +239,7 @@ score_tc_kernel(const __grid_constant__ CUtensorMap tmap_out, const __grid_const
         tmem_relinquish();
     }
     tc_fence_before();
+    tq_grid_wait();         // the prepared queries; so far only constants of the plan have been read
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
@@ -627,6 +629,7 @@ score_tc_kernel(const __grid_constant__ CUtensorMap tmap_out, const __grid_const
 // grid (QPAD, groups), block 128 (thread = coordinate).
 __global__ void __launch_bounds__(128)
 score_prep_kernel(TqDev p, const float* __restrict__ q, int qpg, int q0, int nq, int qpad, unsigned char* __restrict__ prep) {
+    tq_grid_release();      // the scoring kernel sets itself up meanwhile
     __shared__ float qs[D];
     __shared__ float red[2][4];
     const int slot = blockIdx.x, g = blockIdx.y, j = threadIdx.x;
@@ -712,6 +715,7 @@ score_prep256_kernel(TqDev p, const float* __restrict__ q, int qpg, int q0, int 
     __half* m2 = reinterpret_cast<__half*>(base + 2 * (size_t)qpad * kRowBytesB + off);
     __half* m3 = reinterpret_cast<__half*>(base + 3 * (size_t)qpad * kRowBytesB + off);
     float* ds = reinterpret_cast<float*>(base + 8 * (size_t)qpad * kRowBytesB) + (slot >> 1) * 4 + (slot & 1);
+    tq_grid_release();      // the scoring kernel sets itself up meanwhile
     if (slot >= nq) {
         if (kq == 0) {
             *m0 = *m1 = *m2 = *m3 = __float2half_rn(0.f);
@@ -933,12 +937,12 @@ int launch_score(const tq_plan* p, const CUtensorMap& map, const ScoreTcArgs& ar
     const int sm = ScoreSmem<BITS, QPAD, DR>::total;
     if (args.fused) {
         TQ_GRANT_SMEM((score_tc_kernel<BITS, QPAD, DR, true>), sm, p->device);
-        score_tc_kernel<BITS, QPAD, DR, true><<<grid, kThreads, sm, st>>>(map, args); tq_count_launch();
+        TQ_CUDA_TRY(tq_launch_dependent(score_tc_kernel<BITS, QPAD, DR, true>, dim3(grid), dim3(kThreads), (size_t)sm, st, map, args));
         TQ_CUDA_TRY(cudaGetLastError());
         return TQ_OK;
     }
     TQ_GRANT_SMEM((score_tc_kernel<BITS, QPAD, DR, false>), sm, p->device);
-    score_tc_kernel<BITS, QPAD, DR, false><<<grid, kThreads, sm, st>>>(map, args); tq_count_launch();
+    TQ_CUDA_TRY(tq_launch_dependent(score_tc_kernel<BITS, QPAD, DR, false>, dim3(grid), dim3(kThreads), (size_t)sm, st, map, args));
     TQ_CUDA_TRY(cudaGetLastError());
     return TQ_OK;
 }

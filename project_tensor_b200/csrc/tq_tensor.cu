@@ -334,6 +334,7 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
         tmem_alloc(smem_u32(tmem_slot), 512);
         tmem_relinquish();
     }
+    tq_grid_release();      // the second stage may be set up while this kernel runs
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -932,6 +933,7 @@ tensor_quantize256_kernel(const __grid_constant__ CUtensorMap tmap_x, const Tens
         tmem_alloc(smem_u32(tmem_slot), 512);
         tmem_relinquish();
     }
+    tq_grid_release();      // the second stage may be set up while this kernel runs
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
