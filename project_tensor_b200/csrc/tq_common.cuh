@@ -32,7 +32,9 @@ struct TqRecheckHeader {
     unsigned int n_codes;    // entries appended to the coordinate list (may exceed code_cap)
     unsigned int n_rows;     // entries appended to the row list (may exceed row_cap)
     unsigned int overflow;
-    unsigned int pad[13];
+    unsigned int changed;    // diagnostic: codes the exact arithmetic decided differently
+    unsigned int whole_rows; // non-zero: some listed rows have no codes yet (norms outside the tensor-core kernel's range)
+    unsigned int pad[11];
 };
 struct TqRecheck {
     TqRecheckHeader* hdr;

@@ -489,14 +489,25 @@ exact_quantize_tile_kernel(const __grid_constant__ RowsJob first, const __grid_c
         rows.open(job, block == 0);
         if (rows.limit == 0) return;
     }
+    // The listed rows of a TurboQuantProd call have their codes as a rule, settled by the coordinate check: what is left are the
+    // residual and its signs, two products of three.  (d > 128: below, fetching the codes costs what the product does.  524,309
+    // rows, d = 256, with the listed rows' pass at 66 us: 15 us less.)
+    const bool expected = prod && d > 128 && job.lists.hdr != nullptr;
     MatrixRing<T::kThreads> ring;
-    ring.start(stage, p.Rt, p.R, p.St, prod ? 3 : 1, d, shape);
+    if (expected) ring.start(stage, p.R, p.St, p.St, 2, d, shape);
+    else ring.start(stage, p.Rt, p.R, p.St, prod ? 3 : 1, d, shape);
     for (int i = t; i < levels; i += T::kThreads) {
         cbk[i] = __ldg(p.codebook + i);
         if (i + 1 < levels) bnd[i] = __ldg(p.boundaries + i);
     }
     tq_grid_wait();         // (only constants of the plan have been read so far)
     rows.open(job, block == 0);
+    const bool known = expected && rows.listed && job.lists.hdr->whole_rows == 0;
+    if (expected && !known) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        ring.start(stage, p.Rt, p.R, p.St, 3, d, shape);
+    }
     const uint32_t inv_bits = inverse_of_bits(p.bits);
     if (t < RB)
         for (int i = 0; i < 8; ++i) cs[t * kCodeRow + T::kCols + i] = 0;
@@ -524,31 +535,49 @@ exact_quantize_tile_kernel(const __grid_constant__ RowsJob first, const __grid_c
         }
         // (the barrier in front of the first chunk orders the vectors)
         float acc[TR][TC];
-        // rotated[j] = sum_k unit[k] * R[j][k] -> codes, centroids
-        tile_product<RT, TR, CT, TC>(ring, vt, tx, ty, acc);
+        if (known) {
+            constexpr int kAhead = 8;
+            for (int i0 = t; i0 < RB * d; i0 += kAhead * T::kThreads) {
+                uint32_t code[kAhead];
 #pragma unroll
-        for (int c = 0; c < TC; ++c) {
-            const int j = tx + CT * c;
-            float v[TR], cent[TR];
-            int code[TR];
+                for (int u = 0; u < kAhead; ++u) {
+                    const int i = i0 + u * T::kThreads, r = i % RB, j = min(i / RB, d - 1);
+                    const int64_t to = dst_row[r];
+                    code[u] = tq_get_code(job.codes + (to < 0 ? 0 : to) * p.code_words, j, p.bits);
+                }
 #pragma unroll
-            for (int r = 0; r < TR; ++r) v[r] = acc[r][c];
-            codes_of<TR>(bnd, levels, v, code);
-#pragma unroll
-            for (int r = 0; r < TR; ++r) {
-                cs[(ty * TR + r) * kCodeRow + j] = j < d ? (uint8_t)code[r] : 0;
-                cent[r] = cbk[code[r]];
+                for (int u = 0; u < kAhead; ++u) {
+                    const int i = i0 + u * T::kThreads;
+                    if (i < RB * d) ct[i / RB * RS + i % RB] = cbk[code[u]];
+                }
             }
-            if (prod && j < d) {
+        } else {
+            // rotated[j] = sum_k unit[k] * R[j][k] -> codes, centroids
+            tile_product<RT, TR, CT, TC>(ring, vt, tx, ty, acc);
 #pragma unroll
-                for (int r = 0; r < TR; r += 4)
-                    *reinterpret_cast<float4*>(ct + j * RS + ty * TR + r) = make_float4(cent[r], cent[r + 1], cent[r + 2], cent[r + 3]);
+            for (int c = 0; c < TC; ++c) {
+                const int j = tx + CT * c;
+                float v[TR], cent[TR];
+                int code[TR];
+#pragma unroll
+                for (int r = 0; r < TR; ++r) v[r] = acc[r][c];
+                codes_of<TR>(bnd, levels, v, code);
+#pragma unroll
+                for (int r = 0; r < TR; ++r) {
+                    cs[(ty * TR + r) * kCodeRow + j] = j < d ? (uint8_t)code[r] : 0;
+                    cent[r] = cbk[code[r]];
+                }
+                if (prod && j < d) {
+#pragma unroll
+                    for (int r = 0; r < TR; r += 4)
+                        *reinterpret_cast<float4*>(ct + j * RS + ty * TR + r) = make_float4(cent[r], cent[r + 1], cent[r + 2], cent[r + 3]);
+                }
             }
-        }
-        __syncthreads();
-        for (int i = t; i < RB * p.code_words; i += T::kThreads) {
-            const int r = i / p.code_words, w = i - r * p.code_words;
-            if (dst_row[r] >= 0) job.codes[dst_row[r] * p.code_words + w] = packed_code_word(cs + r * kCodeRow, p.bits, inv_bits, w);
+            __syncthreads();
+            for (int i = t; i < RB * p.code_words; i += T::kThreads) {
+                const int r = i / p.code_words, w = i - r * p.code_words;
+                if (dst_row[r] >= 0) job.codes[dst_row[r] * p.code_words + w] = packed_code_word(cs + r * kCodeRow, p.bits, inv_bits, w);
+            }
         }
         if (!prod) continue;
         // recon[j] = sum_k centroid[k] * R[k][j];  residual = unit - recon, in place (only this thread touches its elements)
@@ -597,8 +626,8 @@ exact_quantize_tile_kernel(const __grid_constant__ RowsJob first, const __grid_c
 }
 
 // Listed coordinates (those inside the guard band of the tensor-core kernel) re-decided in the reference's order: norm, division and
-// the rotated coordinate as one FMA chain.  A wrong code is corrected in place (TurboQuantMSE) or puts its row on the row list
-// (TurboQuantProd).  Work is small -- 20,000 entries of 1,048,576 rows -- and every dependent access to global memory costs
+// the rotated coordinate as one FMA chain.  A wrong code is corrected in place and (TurboQuantProd) puts its row on the row
+// list.  Work is small -- 20,000 entries of 1,048,576 rows -- and every dependent access to global memory costs
 // about a microsecond, so the kernel is as long as its chain of such accesses: header and entry, then row, matrix row and
 // boundaries together.  Eight lanes fetch an entry's rows, normalise and leave both in shared memory; then a
 // lane per entry runs the chain, 32 entries side by side.  (One lane per entry for everything, 128 divisions in a row:
@@ -678,18 +707,17 @@ exact_code_check_kernel(const __grid_constant__ CheckJob first, const __grid_con
                 for (int k = 0; k < D; ++k) acc = __fmaf_rn(ve[k], me[k], acc);
                 const uint32_t code = (uint32_t)count_below(bnd, p.levels - 1, acc);
                 if (old != code) {
-                    if (job.prod) {
+                    if (job.prod) {        // the row's residual is another one
                         const unsigned int pos = atomicAdd(&lists.hdr->n_rows, 1u);
                         if (pos < lists.row_cap) lists.row_entries[pos] = (unsigned int)r;
                         else lists.hdr->overflow = 1u;
-                    } else {
-                        uint32_t* crow = packed_row(r);
-                        const uint32_t delta = old ^ code;
-                        const int bit = c * p.bits, w = bit >> 5, sh = bit & 31;
-                        atomicXor(crow + w, delta << sh);
-                        if (sh + p.bits > 32) atomicXor(crow + w + 1, delta >> (32 - sh));
                     }
-                    atomicAdd(&lists.hdr->pad[0], 1u);  // diagnostic: codes the exact arithmetic decided differently
+                    uint32_t* crow = packed_row(r);
+                    const uint32_t delta = old ^ code;
+                    const int bit = c * p.bits, w = bit >> 5, sh = bit & 31;
+                    atomicXor(crow + w, delta << sh);
+                    if (sh + p.bits > 32) atomicXor(crow + w + 1, delta >> (32 - sh));
+                    atomicAdd(&lists.hdr->changed, 1u);
                 }
             }
         }

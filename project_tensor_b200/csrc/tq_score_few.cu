@@ -114,13 +114,15 @@ score_few_kernel(const TqDev p, const FewArgs a) {
             w.rn[h] = __ldg(rn_base + key);
         }
     };
+    build_key_table<KB>(smem, p.codebook, tid, kFewThreads);
+    tq_grid_release();
+    tq_grid_wait();         // (only constants of the plan have been read so far)
     Words cur;
     if (tile < tiles) fetch(tile, cur);
     for (int i = tid; i < NQ * DR; i += kFewThreads) {
         const int qq = i / DR, k = i - qq * DR;
         qin[k * NQ + qq] = q0 + qq < a.qpg ? __ldg(a.q + ((size_t)g * a.qpg + q0 + qq) * DR + k) : 0.f;
     }
-    build_key_table<KB>(smem, p.codebook, tid, kFewThreads);
     __syncthreads();
     {   // rotated[j] = sum_k q[k] R[j][k], projected[j] = sum_k q[k] S[j][k] in 32-bit arithmetic
         float4 sum[NQ];
@@ -243,8 +245,8 @@ int launch_few(const tq_plan* p, const FewArgs& a, int groups, cudaStream_t st) 
     int64_t blocks = (tq_sm_count(p->device) + (int64_t)passes * groups - 1) / ((int64_t)passes * groups);
     const int64_t tiles = (a.keys_per_group + kTile - 1) / kTile, most = (tiles + 3) / 4;
     if (blocks > most) blocks = most;
-    score_few_kernel<KB, DR><<<dim3((unsigned)blocks, (unsigned)passes, (unsigned)groups), kFewThreads, P::total, st>>>(p->dev, a); tq_count_launch();
-    TQ_CUDA_TRY(cudaGetLastError());
+    TQ_CUDA_TRY(tq_launch_dependent(score_few_kernel<KB, DR>, dim3((unsigned)blocks, (unsigned)passes, (unsigned)groups), dim3(kFewThreads),
+                                    (size_t)P::total, st, p->dev, a));
     return TQ_OK;
 }
 }  // namespace

@@ -1096,6 +1096,7 @@ tensor_quantize256_kernel(const __grid_constant__ CUtensorMap tmap_x, const Tens
                 const int64_t grow = (blockIdx.x + i * gridDim.x) * kTileRows + row;
                 if (grow < a.n && !fail) a.norms[output_row<MAPPED>(a, grow)] = nrm;
                 force[(i & 3) * kTileRows + row] = odd ? 1 : 0;
+                if (PROD && odd && grow < a.n) a.lists.hdr->whole_rows = 1u;      // (d = 64, 128: nobody asks)
             }
         };
         // -- tile i into the operand blocks.  TurboQuantProd: the cells a thread fills are those it read as sign epilogue of
