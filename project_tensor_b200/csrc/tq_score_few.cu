@@ -9,6 +9,8 @@
 // flight, no barriers; the tables (tq_mma.cuh) do not depend on the queries, so they are built while the matrices are on
 // their way, and the matrices while the queries are (page-locked host memory in a NumPy call).
 //
+// 1-bit codes need no table: a centroid is c0 + bit (c1 - c0), so their bits are an operand where they stand, as the signs are.
+//
 // Bound: shared-memory lookups, 64 8-byte loads a key at d = 128 and 3-bit codes (2 cycles a warp and load, four lanes a key), and for
 // few keys the prologue.  Before -- one thread per key through tables of the query's own products, whose random rows met
 // in banks (another kernel for three or four queries) -- 1,048,576 keys of d = 128, 3-bit codes took 40 us for one query, 69 for
@@ -45,8 +47,8 @@ struct FewPlan {
     static constexpr int off_slice = table_rows(KB) * kRowBytes;                     // [kSlices][2][NQ][DR] partial sums
     static constexpr int off_vec = off_slice + kSlices * 2 * NQ * DR * 4;            // [2][NQ][DR] rotated, projected queries
     static constexpr int off_qin = off_vec + 2 * NQ * DR * 4;                        // [DR][NQ]
-    static constexpr int off_small = off_qin + NQ * DR * 4;                          // [2][NQ] scales, [NQ] sums of the projected queries
-    static constexpr int total = off_small + 3 * NQ * 4;
+    static constexpr int off_small = off_qin + NQ * DR * 4;                          // [2][NQ] scales, [2][NQ] sums of the vectors
+    static constexpr int total = off_small + 4 * NQ * 4;
     static_assert(total <= 227 * 1024, "shared memory plan");
 };
 
@@ -114,7 +116,7 @@ score_few_kernel(const TqDev p, const FewArgs a) {
             w.rn[h] = __ldg(rn_base + key);
         }
     };
-    build_key_table<KB>(smem, p.codebook, tid, kFewThreads);
+    if (KB > 1) build_key_table<KB>(smem, p.codebook, tid, kFewThreads);
     tq_grid_release();
     tq_grid_wait();         // (only constants of the plan have been read so far)
     Words cur;
@@ -169,7 +171,7 @@ score_few_kernel(const TqDev p, const FewArgs a) {
         }
         if (lane == 0) {
             scl[v] = scale_exp(m);
-            if (v >= NQ) psum[v - NQ] = sum;
+            psum[v] = sum;
         }
     }
     __syncthreads();
@@ -183,8 +185,17 @@ score_few_kernel(const TqDev p, const FewArgs a) {
 #pragma unroll
         for (int s = 0; s < P::kSteps; ++s) {
             uint32_t h0, l0, h1, l1;
-            const float s0 = m == 0 ? sc : sc * (1.f / (1 << ((2 * s) & 7))), s1 = m == 0 ? sc : sc * (1.f / (1 << ((2 * s + 1) & 7)));
-            const float4 f = *reinterpret_cast<const float4*>(x + 4 * s);
+            const bool bits = m == 1 || KB == 1;         // an operand of bits where they stand
+            const float s0 = bits ? sc * (1.f / (1 << ((2 * s) & 7))) : sc, s1 = bits ? sc * (1.f / (1 << ((2 * s + 1) & 7))) : sc;
+            float4 f;
+            if (KB == 1 && m == 0) {
+                // 1-bit codes: coordinates that lie half a word apart make a pair
+                constexpr int kHalf = DR == 64 ? 8 : 16;
+                const int at = 2 * s / kHalf * 32 + 2 * s % kHalf;
+                f = make_float4(x[at], x[at + kHalf], x[at + 1], x[at + 1 + kHalf]);
+            } else {
+                f = *reinterpret_cast<const float4*>(x + 4 * s);
+            }
             split_pair(f.x * s0, f.y * s0, h0, l0);
             split_pair(f.z * s1, f.w * s1, h1, l1);
             qf[m][s][0] = r < 4 ? h0 : l0;
@@ -192,13 +203,18 @@ score_few_kernel(const TqDev p, const FewArgs a) {
         }
     }
     // the two queries of this lane's score columns; a sign is 2 bit - 1
-    float ds1[2], ds2[2], dsum[2];
+    float ds1[2], ds2[2], dsum[2], dbase[2] = {0.f, 0.f};
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
         const int qq = (2 * t + c) & (NQ - 1);
         ds1[c] = pow2i(-scl[qq]) * (1.f / kCentScale);
+        if constexpr (KB == 1) {                  // a centroid is c0 + bit (c1 - c0)
+            const float c0 = __ldg(p.codebook);
+            ds1[c] = pow2i(24 - scl[qq]) * (__ldg(p.codebook + 1) - c0);
+            dbase[c] = 2 * t < NQ ? c0 * psum[qq] : 0.f;
+        }
         ds2[c] = pow2i(25 - scl[NQ + qq]) * p.alpha;
-        dsum[c] = 2 * t < NQ ? -p.alpha * psum[qq] : 0.f;     // (once: hi and lo columns are added)
+        dsum[c] = 2 * t < NQ ? -p.alpha * psum[NQ + qq] : 0.f;     // (once: hi and lo columns are added)
     }
     const uint32_t lane8 = (uint32_t)(lane & 15) * 8u, lane16 = (uint32_t)(lane & 7) * 16u;
     // The lane's scores: queries 2 (t & 1) + c of key r + 8 (t >> 1) -- adding hi and lo columns leaves both lanes with the sum.
@@ -211,9 +227,34 @@ score_few_kernel(const TqDev p, const FewArgs a) {
         W key;
         key.unpack(cur.kc, cur.sg, kshift, t);
         float c1[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, c2[4] = {0.f, 0.f, 0.f, 0.f};
+        uint32_t cbits[2][2 * W::kWords];        // 1-bit codes, as the sign words
+        if constexpr (KB == 1) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int i = 0; i < W::kWords; ++i) {
+                    uint32_t w = cur.kc[h][i];
+                    if (DR == 64) { w >>= kshift; w = (w & 0xffu) | ((w & 0xff00u) << 8); }
+                    cbits[h][2 * i] = w;
+                    cbits[h][2 * i + 1] = w >> 8;
+                }
+        }
         for_steps<P::kSteps>([&](auto sc) {
             constexpr int s = decltype(sc)::value;
             uint32_t ak[2][4], as[4];
+            if constexpr (KB == 1) {
+                uint32_t ab[4];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    ab[h] = cbits[h][s >> 2] & (0x00010001u << ((2 * s) & 7));
+                    ab[2 + h] = cbits[h][s >> 2] & (0x00010001u << ((2 * s + 1) & 7));
+                    as[h] = key.sw[h][s >> 2] & (0x00010001u << ((2 * s) & 7));
+                    as[2 + h] = key.sw[h][s >> 2] & (0x00010001u << ((2 * s + 1) & 7));
+                }
+                mma16816(c1[0], ab, qf[0][s][0], qf[0][s][1]);
+                mma16816(c2, as, qf[1][s][0], qf[1][s][1]);
+                return;
+            }
             key.template operands<s>(smem, lane8, lane16, ak, as);
             mma16816(c1[0], ak[0], qf[0][s][0], qf[0][s][1]);
             mma16816(c1[1], ak[1], qf[0][s][0], qf[0][s][1]);
@@ -224,7 +265,8 @@ score_few_kernel(const TqDev p, const FewArgs a) {
         for (int h = 0; h < 2; ++h)
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
-                float s = fmaf(fmaf(c2[2 * h + c], ds2[c], dsum[c]), cur.rn[h], (c1[h][c] + c1[h][2 + c]) * ds1[c]);
+                const float centroids = KB == 1 ? fmaf(c1[0][2 * h + c], ds1[c], dbase[c]) : (c1[h][c] + c1[h][2 + c]) * ds1[c];
+                float s = fmaf(fmaf(c2[2 * h + c], ds2[c], dsum[c]), cur.rn[h], centroids);
                 s += __shfl_xor_sync(0xffffffffu, s, 2);     // hi and lo columns
                 v[h][c] = s * cur.kn[h];
             }
@@ -265,6 +307,8 @@ int tq_launch_score_few(const tq_plan* p, const float* q, int groups, int qpg, c
                         int64_t group_rows) {
     TqRange range("tq.score.few_queries");
     if (group_rows <= 0) group_rows = keys_per_group;
+    if (tq_score_table_better(p, groups, qpg, keys_per_group))
+        return tq_launch_score_table(p, q, groups, codes, signs, rnorms, norms, keys_per_group, scores, st, group_rows);
     const FewArgs a{q, codes, signs, rnorms, norms, qpg, keys_per_group, group_rows, scores};
     const int d = p->dev.d;
     switch (p->dev.bits) {
