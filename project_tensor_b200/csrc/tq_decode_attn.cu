@@ -21,8 +21,7 @@
 //            instruction for q_hi and one for q_lo.  A = keys x 16 coordinates; the order of the rows and of the coordinates inside
 //            a contraction is free, so lane t of a quad takes d/4 consecutive coordinates of its key -- whole 32-bit words
 //            of the packed row (d = 128) -- and the two halves of the instruction's rows are hi and lo of the same 8 keys:
-//            one table row is the operand's registers as they are.  Sign bits are used where they stand in the word, as
-//            subnormal fp16 numbers 2^(b - 24) that the scale of the projected query makes up for (a sign is 2 bit - 1).
+//            one table row is the operand's registers as they are; signs become +-1 by a shift and a logic operation.
 //   values   A = 16 coordinates x 16 keys (transposed: a register holds one coordinate of two keys), B = weights p * norm, hi
 //            and lo, which reach their lanes from the scores' layout by one 8 x 8 transposition (movmatrix).
 //
@@ -100,8 +99,8 @@ struct Plan {
     static constexpr int off_slice = off_frag + (NQ == 8 ? 2 * kFragBytes : 0);   // [kSlices][2][NQ][DR] partial sums
     static constexpr int off_vec = off_slice + kSlices * 2 * NQ * DR * 4;         // [2][NQ][DR] rotated, projected queries
     static constexpr int off_qin = off_vec + 2 * NQ * DR * 4;            // [DR][NQ]
-    static constexpr int off_small = off_qin + NQ * DR * 4;              // [2][NQ] scales, [NQ] sums of the projected queries, [kWarps][NQ] max, sum, factor
-    static constexpr int total = off_small + (3 * NQ + 3 * kWarps * NQ) * 4;
+    static constexpr int off_small = off_qin + NQ * DR * 4;              // [2][NQ] scales, [kWarps][NQ] max, sum, factor
+    static constexpr int total = off_small + (2 * NQ + 3 * kWarps * NQ) * 4;
 };
 
 // Packed words of one tile of 16 keys, as the lanes of a warp hold them.
@@ -120,8 +119,7 @@ decode_partial_kernel(TqDev kp, DecodeArgs a) {
     float* vec = reinterpret_cast<float*>(smem + P::off_vec);
     float* qin = reinterpret_cast<float*>(smem + P::off_qin);
     int* scl = reinterpret_cast<int*>(smem + P::off_small);                   // exponents of the queries' scales
-    float* psum = reinterpret_cast<float*>(smem + P::off_small) + 2 * NQ;     // [NQ]
-    float* wm = psum + NQ;                                                    // [kWarps][NQ]
+    float* wm = reinterpret_cast<float*>(smem + P::off_small) + 2 * NQ;                                                    // [kWarps][NQ]
     float* wl = wm + kWarps * NQ;
     float* wf = wl + kWarps * NQ;
 
@@ -247,25 +245,21 @@ decode_partial_kernel(TqDev kp, DecodeArgs a) {
     }
     __syncthreads();
     for (int v = warp; v < 2 * NQ; v += kWarps) {
-        float m = 0.f, sum = 0.f;
+        float m = 0.f;
         for (int k = lane; k < DR; k += 32) {
             m = fmaxf(m, fabsf(vec[v * DR + k]));
-            sum += vec[v * DR + k];
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-            sum += __shfl_xor_sync(0xffffffffu, sum, o);
         }
         if (lane == 0) {
             scl[v] = scale_exp(m);
-            if (v >= NQ) psum[v - NQ] = sum;
         }
     }
     __syncthreads();
     // Query operands.  Up to 4 queries: in registers, column r is hi (r < 4) or lo (r >= 4) of query r & 3.  Up to 8: in
-    // shared memory, (hi b0, hi b1, lo b0, lo b1) of query r per lane and step.  The sign bits of a pair of coordinates are
-    // used where they stand, as the fp16 numbers 0 or 2^(b - 24) (b = 0..7, see below): the projected query is scaled by 2^-b.
+    // shared memory, (hi b0, hi b1, lo b0, lo b1) of query r per lane and step.
     constexpr int kRegSteps = NQ == 4 ? P::kSteps : 1;
     uint32_t qf[2][kRegSteps][2];
     {
@@ -278,9 +272,8 @@ decode_partial_kernel(TqDev kp, DecodeArgs a) {
             for (int s = 0; s < P::kSteps; ++s) {
                 if (NQ == 8 && s % kWarps != warp) continue;      // (each warp stores some of the steps)
                 uint32_t h0, l0, h1, l1;
-                const float s0 = m == 0 ? sc : sc * (1.f / (1 << ((2 * s) & 7))), s1 = m == 0 ? sc : sc * (1.f / (1 << ((2 * s + 1) & 7)));
-                split_pair(x[4 * s] * s0, x[4 * s + 1] * s0, h0, l0);
-                split_pair(x[4 * s + 2] * s1, x[4 * s + 3] * s1, h1, l1);
+                split_pair(x[4 * s] * sc, x[4 * s + 1] * sc, h0, l0);
+                split_pair(x[4 * s + 2] * sc, x[4 * s + 3] * sc, h1, l1);
                 if constexpr (NQ == 4) {
                     qf[m][s][0] = r < 4 ? h0 : l0;
                     qf[m][s][1] = r < 4 ? h1 : l1;
@@ -291,16 +284,14 @@ decode_partial_kernel(TqDev kp, DecodeArgs a) {
         }
     }
     if constexpr (NQ == 8) __syncthreads();
-    // The two queries of this lane's score columns: descaling factors, softmax state.  A sign is 2 bit - 1: the contraction
-    // with the bits, doubled, less the sum of the projected query.
-    float ds1[2], ds2[2], dsum[2], mref[2], lsum[2];
+    // The two queries of this lane's score columns: descaling factors, softmax state.
+    float ds1[2], ds2[2], mref[2], lsum[2];
     float wsc[2];                     // power of two that scales the weights
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
         const int qq = (2 * t + c) & (NQ - 1);
         ds1[c] = pow2i(-scl[qq]) * (1.f / kCentScale);
-        ds2[c] = pow2i(25 - scl[NQ + qq]) * kp.alpha;
-        dsum[c] = 2 * t < NQ ? -kp.alpha * psum[qq] : 0.f;     // (once: hi and lo columns are added)
+        ds2[c] = pow2i(-scl[NQ + qq]) * kp.alpha;
         mref[c] = -CUDART_INF_F;
         lsum[c] = 0.f;
         wsc[c] = pow2i(126);
@@ -351,7 +342,7 @@ decode_partial_kernel(TqDev kp, DecodeArgs a) {
         for (int h = 0; h < 2; ++h) {
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
-                float v = fmaf(fmaf(c2[2 * h + c], ds2[c], dsum[c]), cur.rn[h], (c1[h][c] + c1[h][2 + c]) * ds1[c]);
+                float v = fmaf(c2[2 * h + c] * ds2[c], cur.rn[h], (c1[h][c] + c1[h][2 + c]) * ds1[c]);
                 if constexpr (NQ == 4) v += __shfl_xor_sync(0xffffffffu, v, 2);     // hi and lo columns
                 v *= cur.kn[h] * a.scale_log2e;
                 s[h][c] = key_r + 8 * h < left ? v : -CUDART_INF_F;

@@ -84,7 +84,7 @@ struct KeyWords {
     static constexpr int kBits = DR / 4 * KB;                                    // bits of a packed row that a lane uses
     static constexpr int kWords = kBits % 32 == 0 ? kBits / 32 : kBits / 32 + 1; // words it loads: they may start inside a word
     static constexpr int kSigns = DR == 256 ? 2 : 1;                             // sign words it loads
-    uint32_t kw[2][kWords], kw1[2][kWords], sw[2][2 * kSigns];
+    uint32_t kw[2][kWords], kw1[2][kWords], sw[2][kSigns];
     __device__ __forceinline__ void unpack(const uint32_t (&kc)[2][kWords], const uint32_t (&sg)[2][kSigns], int shift, int t) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -102,8 +102,7 @@ struct KeyWords {
             }
 #pragma unroll
             for (int i = 0; i < kSigns; ++i) {
-                sw[h][2 * i] = DR >= 128 ? sg[h][i] : sg[h][i] >> (8 * (t & 1));
-                sw[h][2 * i + 1] = sw[h][2 * i] >> 8;
+                sw[h][i] = DR >= 128 ? sg[h][i] : sg[h][i] >> (8 * (t & 1));
             }
             if constexpr (KB == 1) {         // four codes: a nibble; even ones and odd ones in words of their own
 #pragma unroll
@@ -142,10 +141,17 @@ struct KeyWords {
                 const uint4 v = row16(KB == 2 ? pick(kw[h][S >> 2], S & 3, lane16) : pick(S & 1 ? kw1[h][S >> 3] : kw[h][S >> 3], (S >> 1) & 3, lane16));
                 ak[h][0] = v.x; ak[h][1] = v.y; ak[h][2] = v.z; ak[h][3] = v.w;
             }
-            // signs of two coordinates: bit b = (pair & 7) of both halves of the word (or of the word moved by 8), where it
-            // stands -- a subnormal number 2^(b - 24), which the operand of the query makes up for
-            as[h] = sw[h][S >> 2] & (0x00010001u << ((2 * S) & 7));
-            as[2 + h] = sw[h][S >> 2] & (0x00010001u << ((2 * S + 1) & 7));
+        }
+        signs<S>(as);
+    }
+    // Signs of coordinates 4s .. 4s + 3 as +-1.  (Bits used where they stand, as subnormal numbers, save an instruction each, but
+    // their sums are several times the signed ones, and the rounding of the accumulators with them.)
+    template <int S>
+    __device__ __forceinline__ void signs(uint32_t (&as)[4]) const {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            as[h] = ((sw[h][S >> 3] << (15 - (2 * S & 15))) & 0x80008000u) ^ 0xbc00bc00u;
+            as[2 + h] = ((sw[h][S >> 3] << (14 - (2 * S & 15))) & 0x80008000u) ^ 0xbc00bc00u;
         }
     }
 };

@@ -9,7 +9,8 @@
 // flight, no barriers; the tables (tq_mma.cuh) do not depend on the queries, so they are built while the matrices are on
 // their way, and the matrices while the queries are (page-locked host memory in a NumPy call).
 //
-// 1-bit codes need no table: a centroid is c0 + bit (c1 - c0), so their bits are an operand where they stand, as the signs are.
+// 1-bit codes need no table: a centroid is c0 + bit (c1 - c0), so their bits are an operand where they stand, as subnormal
+// fp16 numbers that the scale of the rotated query makes up for.
 //
 // Bound: shared-memory lookups, 64 8-byte loads a key at d = 128 and 3-bit codes (2 cycles a warp and load, four lanes a key), and for
 // few keys the prologue.  Before -- one thread per key through tables of the query's own products, whose random rows met
@@ -175,8 +176,7 @@ score_few_kernel(const TqDev p, const FewArgs a) {
         }
     }
     __syncthreads();
-    // Query operands: column r is hi (r < 4) or lo (r >= 4) of query r & 3.  The projected query makes up for the place 2^(b - 24) of
-    // the sign bits.
+    // Query operands: column r is hi (r < 4) or lo (r >= 4) of query r & 3.
     uint32_t qf[2][P::kSteps][2];
 #pragma unroll
     for (int m = 0; m < 2; ++m) {
@@ -185,7 +185,7 @@ score_few_kernel(const TqDev p, const FewArgs a) {
 #pragma unroll
         for (int s = 0; s < P::kSteps; ++s) {
             uint32_t h0, l0, h1, l1;
-            const bool bits = m == 1 || KB == 1;         // an operand of bits where they stand
+            const bool bits = m == 0 && KB == 1;         // an operand of bits where they stand, 2^(b - 24)
             const float s0 = bits ? sc * (1.f / (1 << ((2 * s) & 7))) : sc, s1 = bits ? sc * (1.f / (1 << ((2 * s + 1) & 7))) : sc;
             float4 f;
             if (KB == 1 && m == 0) {
@@ -202,8 +202,8 @@ score_few_kernel(const TqDev p, const FewArgs a) {
             qf[m][s][1] = r < 4 ? h1 : l1;
         }
     }
-    // the two queries of this lane's score columns; a sign is 2 bit - 1
-    float ds1[2], ds2[2], dsum[2], dbase[2] = {0.f, 0.f};
+    // the two queries of this lane's score columns
+    float ds1[2], ds2[2], dbase[2] = {0.f, 0.f};
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
         const int qq = (2 * t + c) & (NQ - 1);
@@ -213,8 +213,7 @@ score_few_kernel(const TqDev p, const FewArgs a) {
             ds1[c] = pow2i(24 - scl[qq]) * (__ldg(p.codebook + 1) - c0);
             dbase[c] = 2 * t < NQ ? c0 * psum[qq] : 0.f;
         }
-        ds2[c] = pow2i(25 - scl[NQ + qq]) * p.alpha;
-        dsum[c] = 2 * t < NQ ? -p.alpha * psum[NQ + qq] : 0.f;     // (once: hi and lo columns are added)
+        ds2[c] = pow2i(-scl[NQ + qq]) * p.alpha;
     }
     const uint32_t lane8 = (uint32_t)(lane & 15) * 8u, lane16 = (uint32_t)(lane & 7) * 16u;
     // The lane's scores: queries 2 (t & 1) + c of key r + 8 (t >> 1) -- adding hi and lo columns leaves both lanes with the sum.
@@ -227,7 +226,7 @@ score_few_kernel(const TqDev p, const FewArgs a) {
         W key;
         key.unpack(cur.kc, cur.sg, kshift, t);
         float c1[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, c2[4] = {0.f, 0.f, 0.f, 0.f};
-        uint32_t cbits[2][2 * W::kWords];        // 1-bit codes, as the sign words
+        uint32_t cbits[2][2 * W::kWords];        // 1-bit codes: the word, and the word moved by 8
         if constexpr (KB == 1) {
 #pragma unroll
             for (int h = 0; h < 2; ++h)
@@ -248,9 +247,8 @@ score_few_kernel(const TqDev p, const FewArgs a) {
                 for (int h = 0; h < 2; ++h) {
                     ab[h] = cbits[h][s >> 2] & (0x00010001u << ((2 * s) & 7));
                     ab[2 + h] = cbits[h][s >> 2] & (0x00010001u << ((2 * s + 1) & 7));
-                    as[h] = key.sw[h][s >> 2] & (0x00010001u << ((2 * s) & 7));
-                    as[2 + h] = key.sw[h][s >> 2] & (0x00010001u << ((2 * s + 1) & 7));
                 }
+                key.template signs<s>(as);
                 mma16816(c1[0], ab, qf[0][s][0], qf[0][s][1]);
                 mma16816(c2, as, qf[1][s][0], qf[1][s][1]);
                 return;
@@ -266,7 +264,7 @@ score_few_kernel(const TqDev p, const FewArgs a) {
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
                 const float centroids = KB == 1 ? fmaf(c1[0][2 * h + c], ds1[c], dbase[c]) : (c1[h][c] + c1[h][2 + c]) * ds1[c];
-                float s = fmaf(fmaf(c2[2 * h + c], ds2[c], dsum[c]), cur.rn[h], centroids);
+                float s = fmaf(c2[2 * h + c] * ds2[c], cur.rn[h], centroids);
                 s += __shfl_xor_sync(0xffffffffu, s, 2);     // hi and lo columns
                 v[h][c] = s * cur.kn[h];
             }

@@ -1,4 +1,4 @@
-// attention_score for one query against many keys at d = 64, and at d = 256 with 2-bit codes (_quant.py:334-358).
+// attention_score for one query against many keys (_quant.py:334-358).
 //
 //   score(q, key) = norm * ( (R q) . codebook[codes]  +  alpha * rnorm * ((S q) . signs) )
 //
@@ -9,8 +9,8 @@
 //
 // and every thread walks the packed codes and sign words of one key: d/2 + d/8 lookups and additions, no unpacking.
 // score_few_kernel expands the keys for up to four queries at once; for one it pays its per-tile overhead at d = 64 (4,068,313
-// keys, 1 / 2 / 3 code bits: 76 / 79 / 83 us there, 54 / 58 / 66 here) and, at d = 256 with 2-bit codes, twice the 16-byte
-// lookups (225 and 197 us).  Its prologue is the shorter one, so few keys are its own in either case.
+// keys, 1 / 2 / 3 code bits: 76 / 79 / 83 us there, 54 / 58 / 66 here) and the expansion at d = 256 (2 / 3 bits: 225 / 316 us there, 197 /
+// 275 here).  Its prologue is the shorter one, so few keys are its own in either case.
 #include "tq_common.cuh"
 
 #include <stdint.h>
@@ -140,13 +140,14 @@ int launch_table(const tq_plan* p, const float* q, const uint32_t* codes, const 
 
 }  // namespace
 
-// The lines lie where the two kernels meet: prologues of 5 and 4 us and 0.013 against 0.019 ns a key at d = 64, 0.046 against 0.053 at
-// d = 256.
+// The lines lie where the two kernels meet: the prologue is 1 to 6 us longer here, a thousand keys cost 13 against 19 ns at d = 64,
+// 30 against 31 at d = 128 (3-bit codes), 48 to 68 against 54 to 78 at d = 256 (2 and 3 bits).
 bool tq_score_table_better(const tq_plan* p, int groups, int qpg, int64_t keys_per_group) {
     const int64_t keys = (int64_t)groups * keys_per_group;
+    const int d = p->dev.d, bits = p->dev.bits;
     if (!p->has_projection || qpg != 1) return false;
-    return (p->dev.d == 64 && p->dev.bits >= 1 && p->dev.bits <= 4 && keys >= 1 << 18) ||
-           (p->dev.d == 256 && p->dev.bits == 2 && keys >= 1 << 20);
+    return (d == 64 && bits >= 1 && bits <= 4 && keys >= 1 << 18) || (d == 128 && (bits == 2 || bits == 3) && keys >= 3 << 20) ||
+           (d == 256 && (bits == 2 || bits == 3) && keys >= 1 << 20);
 }
 
 // scores: [groups][keys_per_group]
@@ -154,7 +155,10 @@ int tq_launch_score_table(const tq_plan* p, const float* q, int groups, const ui
                           const float* norms, int64_t keys_per_group, float* scores, cudaStream_t st, int64_t group_rows) {
     TqRange range("tq.score.one_query");
     if (group_rows <= 0) group_rows = keys_per_group;
-    if (p->dev.d == 256) return launch_table<2, 256>(p, q, codes, signs, rnorms, norms, keys_per_group, group_rows, groups, 1, scores, st);
+#define TQ_TABLE_ARGS p, q, codes, signs, rnorms, norms, keys_per_group, group_rows, groups, 1, scores, st
+    if (p->dev.d == 256) return p->dev.bits == 2 ? launch_table<2, 256>(TQ_TABLE_ARGS) : launch_table<3, 256>(TQ_TABLE_ARGS);
+    if (p->dev.d == 128) return p->dev.bits == 2 ? launch_table<2, 128>(TQ_TABLE_ARGS) : launch_table<3, 128>(TQ_TABLE_ARGS);
+#undef TQ_TABLE_ARGS
     switch (p->dev.bits) {
 #define TQ_TABLE(B) case B: return launch_table<B, 64>(p, q, codes, signs, rnorms, norms, keys_per_group, group_rows, groups, 1, scores, st);
         TQ_TABLE(1) TQ_TABLE(2) TQ_TABLE(3) TQ_TABLE(4)
