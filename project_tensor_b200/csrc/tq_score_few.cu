@@ -14,8 +14,9 @@
 //
 // Bound: shared-memory lookups, 64 8-byte loads a key at d = 128 and 3-bit codes (2 cycles a warp and load, four lanes a key), and for
 // few keys the prologue.  Before -- one thread per key through tables of the query's own products, whose random rows met
-// in banks (another kernel for three or four queries) -- 1,048,576 keys of d = 128, 3-bit codes took 40 us for one query, 69 for
-// two, 84 for four, now 35 to 36; 262,147 keys and one query 19.7, now 15.2.
+// in banks (another kernel for three or four queries) -- 2,000,000 keys of d = 128, 3-bit codes and one query took 71 us, now 66;
+// 262,147 keys 23, now 15.5.  (With signs as bits where they stand 1,048,576 keys took 35 us for one query and 36 for four, 40
+// and 84 before; +-1 costs some 8 % of that and gives a four times smaller error.)
 #include "tq_common.cuh"
 #include "tq_mma.cuh"
 
