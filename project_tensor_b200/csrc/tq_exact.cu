@@ -487,7 +487,10 @@ exact_quantize_tile_kernel(const __grid_constant__ RowsJob first, const __grid_c
     if (job.lists.hdr != nullptr && !prod) {     // the list of a TurboQuantMSE call is empty as a rule
         tq_grid_wait();
         rows.open(job, block == 0);
-        if (rows.limit == 0) return;
+        if (rows.limit == 0) {
+            if (advance && t == 0) advance_length(job, rows.len0, advance);      // (block 0 raises the length, work or not)
+            return;
+        }
     }
     // The listed rows of a TurboQuantProd call have their codes as a rule, settled by the coordinate check: what is left are the
     // residual and its signs, two products of three.  (d > 128: below, fetching the codes costs what the product does.  524,309

@@ -14,6 +14,7 @@ pytestmark = pytest.mark.gpu
     (64, 4, 3, 4, (1500, 1190, 7)),      # the second call has 4,760 rows, just above what one launch takes
     (128, 6, 2, 2, (2500,)),             # 5-bit keys have no tensor-core kernel, the values do
     (96, 4, 4, 1, (4200,)), (256, 4, 4, 2, (3000,)),
+    (256, 6, 4, 2, (3000, 7)),           # the same at d = 256; the second call reads the length the first one raised
 ])
 def test_bulk_append_equals_quantize(dtype, d, kbits, vbits, groups, lengths):
     import torch
@@ -40,3 +41,23 @@ def test_bulk_append_equals_quantize(dtype, d, kbits, vbits, groups, lengths):
     want = tg.packed_buffers(vq.quantize(values.float().reshape(-1, d)))
     assert torch.equal(cache.value_codes.view(groups, cap, -1)[:, :at].reshape(groups * at, -1), want["codes"].reshape(groups * at, -1))
     assert float((cache.value_norms.view(groups, cap)[:, :at].reshape(-1) / want["norms"] - 1).abs().max()) <= 1e-6
+
+
+@pytest.mark.parametrize("d", [128, 256])
+def test_bulk_append_of_values_alone_raises_the_length(d):
+    import torch
+    from project_tensor_b200 import _native
+    lib = _native.load()
+    vq = tg.TurboQuantMSE(d, 4, seed=77, grid_size=4097, max_iter=64)
+    n, cap, dev = 6000, 6400, torch.device("cuda", 0)
+    values = torch.randn(1, n, d, device=dev, generator=torch.Generator("cuda").manual_seed(d))
+    plan, stream = vq._plans.handle(dev), torch.cuda.current_stream().cuda_stream
+    codes = torch.zeros((cap, d // 2), dtype=torch.uint8, device=dev)
+    norms, length = torch.zeros(cap, device=dev), torch.full((1,), 100, dtype=torch.int64, device=dev)
+    need = lib.tq_kv_prefill_scratch_bytes(None, plan, n)
+    scratch = torch.empty(need, dtype=torch.uint8, device=dev)
+    _native.check(lib.tq_kv_prefill(None, plan, None, values.data_ptr(), _native.TQ_F32, 1, n, None, None, None, None,
+                                    codes.data_ptr(), norms.data_ptr(), cap, 100, length.data_ptr(), scratch.data_ptr(), need, stream))
+    assert int(length.item()) == 100 + n
+    want = tg.packed_buffers(vq.quantize(values[0]))
+    assert torch.equal(codes[100:100 + n], want["codes"]) and torch.equal(norms[100:100 + n], want["norms"])
