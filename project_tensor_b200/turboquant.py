@@ -256,9 +256,11 @@ class _PlanSet:
 
     def check_status(self, device) -> None:
         """Raise if a tensor-core kernel of this quantizer gave up on a bounded wait on ``device`` since the last
-        check (synchronises the current stream of that device)."""
+        check.  Synchronises the current stream of that device in any case: callers rely on it to have waited for the copies they
+        enqueued, also for an encoding whose quantizer has not been used on the device yet (one read from a file)."""
         h = self._plans.get(_device_index(device))
         if h is None:
+            _torch().cuda.current_stream(device).synchronize()
             return
         status = ctypes.c_int64(0)
         _native.check(_native.load().tq_plan_status(h, _stream_ptr(device), ctypes.byref(status)))

@@ -210,3 +210,19 @@ def test_gpu_save_load_round_trip(tmp_path):
     again = pf.load_encoding(cpu_file, quant)
     for name in a:
         assert torch.equal(a[name], tg.packed_buffers(again)[name])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["prod", "mse"])
+def test_saving_with_a_quantizer_that_has_not_run_waits_for_the_copies(tmp_path, lib_built, kind):
+    """No kernel of the quantizer has run on the device (it only read a file), and the stream is busy."""
+    import torch
+    import project_tensor_b200 as tg
+    make = {"prod": tg.TurboQuantProd, "mse": tg.TurboQuantMSE}[kind]
+    first, path = make(64, 4, seed=5), tmp_path / "first.tqp"
+    pf.save_encoding(path, first, first.quantize(torch.randn(3000, 64, device="cuda")))
+    fresh = make(64, 4, seed=5)
+    back = pf.load_encoding(path, fresh)
+    torch.cuda._sleep(100_000_000)       # some 50 ms
+    pf.save_encoding(tmp_path / "second.tqp", fresh, back)
+    assert path.read_bytes() == (tmp_path / "second.tqp").read_bytes()
