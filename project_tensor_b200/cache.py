@@ -25,6 +25,10 @@ def _widen(staged):
     return staged
 
 
+def _off_boundary(staged) -> bool:
+    return staged is not None and staged.tensor.element_size() == 2 and staged.tensor.data_ptr() % 16 != 0
+
+
 class PackedKeyCache:
     """Packed TurboQuantProd keys of ``groups`` sequences, ``capacity`` rows each, all of one length."""
 
@@ -97,7 +101,9 @@ class PackedKeyCache:
         vstaged, vplans, vcodes, vnorms = values or (None, None, None, None)
         rows = self.groups * tokens
         bulk = rows > self.SMALL_APPEND_ROWS
-        if bulk and self.quantizer.dimension == 256:      # (its bulk kernel reads float32 only)
+        # 16-bit rows are widened first where the kernels do not take them as they are: the bulk kernel of d = 256 reads float32 only,
+        # and the rows have to start on a 16-byte boundary (a view of a larger tensor need not)
+        if bulk and self.quantizer.dimension == 256 or any(_off_boundary(s) for s in (staged, vstaged)):
             staged, vstaged = _widen(staged), _widen(vstaged) if values else None
         kh, vh = self._plans.handle(dev), vplans.handle(dev) if values else None
         args = (kh, vh, staged.tensor.data_ptr(), vstaged.tensor.data_ptr() if values else None,

@@ -61,3 +61,23 @@ def test_bulk_append_of_values_alone_raises_the_length(d):
     assert int(length.item()) == 100 + n
     want = tg.packed_buffers(vq.quantize(values[0]))
     assert torch.equal(codes[100:100 + n], want["codes"]) and torch.equal(norms[100:100 + n], want["norms"])
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float16"])
+@pytest.mark.parametrize("d,tokens,offset", [(100, 1, 100), (20, 7, 20), (64, 1, 3), (128, 2500, 1), (256, 2500, 5)])
+def test_append_takes_16_bit_rows_off_a_16_byte_boundary(dtype, d, tokens, offset):
+    import torch
+    kq, vq = tg.TurboQuantProd(d, 3, seed=2026, grid_size=4097, max_iter=64), tg.TurboQuantMSE(d, 4, seed=77, grid_size=4097, max_iter=64)
+    groups = 2
+    gen = torch.Generator("cuda").manual_seed(d)
+    flat = torch.randn(groups * tokens * d + offset, device="cuda", generator=gen).to(getattr(torch, dtype))
+    rows = flat[offset:].view(groups, tokens, d)
+    assert rows.data_ptr() % 16 != 0 and rows.is_contiguous()
+    for keys, values in ((rows, rows), (rows, rows.clone()), (rows.clone(), rows)):
+        cache = PackedKVCache(kq, vq, groups, tokens + 1)
+        cache.append(keys, values)
+        want = PackedKVCache(kq, vq, groups, tokens + 1)
+        want.append(rows.float(), rows.float())
+        for have, other in ((cache.keys, want.keys), (cache, want)):
+            for name in ("codes", "signs", "norms", "residual_norms", "length_device") if have is cache.keys else ("value_codes", "value_norms"):
+                assert torch.equal(getattr(have, name), getattr(other, name)), name
