@@ -160,7 +160,7 @@ def _stage_query(data: Any, dim: int, device) -> _Staged:
     block is free again when the call is over."""
     if isinstance(data, np.ndarray) and 0 < data.size * 4 <= _MAPPED_BYTES and device.type == "cuda":
         _ensure_last_dim(data, dim)
-        block = _torch().empty(data.shape, dtype=_torch().float32, pin_memory=True)
+        block = _torch().empty(data.shape, dtype=_torch().float32, device="cpu", pin_memory=True)
         block.numpy()[...] = data
         return _Staged(block, tuple(data.shape[:-1]), "numpy", device)
     staged = _stage(data, dim, device=device)
@@ -201,7 +201,7 @@ def _to_host(tensor, plans: "Optional[_PlanSet]" = None):
     torch = _torch()
     if tensor.device.type != "cuda":
         return tensor
-    host = torch.empty(tensor.shape, dtype=tensor.dtype, pin_memory=True)
+    host = torch.empty(tensor.shape, dtype=tensor.dtype, device="cpu", pin_memory=True)
     host.copy_(tensor, non_blocking=True)
     if plans is not None:
         plans.check_status(tensor.device)      # waits for the stream
@@ -406,7 +406,7 @@ def packed_to_host(encoding, out: Optional[Dict[str, Any]] = None, wait: bool = 
             continue
         dst = host.get(name)
         if dst is None or dst.shape != dev_t.shape or dst.dtype != dev_t.dtype or not dst.is_pinned():
-            dst = torch.empty(dev_t.shape, dtype=dev_t.dtype, pin_memory=True)
+            dst = torch.empty(dev_t.shape, dtype=dev_t.dtype, device="cpu", pin_memory=True)
             host[name] = dst
         dst.copy_(dev_t, non_blocking=True)
     if wait:
@@ -443,7 +443,7 @@ def quantize_to_host(quantizer, keys, chunk_rows: int = 131072, out: Optional[Di
     for name, (shape, dtype) in shapes.items():
         t = host.get(name)
         if t is None or tuple(t.shape) != shape or t.dtype != dtype or not t.is_pinned():
-            host[name] = torch.empty(shape, dtype=dtype, pin_memory=True)
+            host[name] = torch.empty(shape, dtype=dtype, device="cpu", pin_memory=True)
     if not prod:
         host["signs"] = host["residual_norms"] = None
     if n == 0:
@@ -675,7 +675,7 @@ class TurboQuantProd:
         lib = _native.load()
         # a short row of scores for a NumPy caller is written straight to page-locked memory
         to_host = staged.kind == "numpy" and 4 * num_codes <= _MAPPED_BYTES
-        scores = _torch().empty(q_prefix, pin_memory=True) if to_host else pk.norms.new_empty(q_prefix)
+        scores = _torch().empty(q_prefix, dtype=_torch().float32, device="cpu", pin_memory=True) if to_host else pk.norms.new_empty(q_prefix)
         _check_rows(scores, num_codes, q_prefix)
         handle = self._plans.handle(pk.device)
         st = _stream_ptr(pk.device)
