@@ -327,38 +327,50 @@ score_tc_kernel(const __grid_constant__ CUtensorMap tmap_out, const __grid_const
             const int db = (int)(i % kDBufs);
             const uint32_t d1 = tm + kColD + db * kDCols, d2 = d1 + QPAD;
             const bool last_of_group = t + 1 == t1 || kt + 1 == tiles_per_group;
-#pragma unroll 1
-            for (int h = 0; h < kHalves; ++h) {
-                const int b = kHalves == 2 ? h : (int)(i & 1);               // the operand buffer, and which filling of it
-                const uint32_t use = kHalves == 2 ? i : i >> 1, base = tm + b * kBufCols;
-                go = warp_wait(BAR(SB_A_FULL + b), use & 1u, abort_flag) &&
-                     (h > 0 || warp_wait(BAR(SB_D_EMPTY + db), ((i / kDBufs) & 1) ^ 1u, abort_flag));
-                if (!go) break;
-                tc_fence_after();
-                if (elect_one()) {
-#pragma unroll 1
-                    for (int kb = 0; kb < kDH / 16; ++kb) {
-                        // the start-address field counts 16-byte units: one k-block is two core matrices further, the
-                        // operand matrices of the second half of the coordinates follow those of the first
-                        const uint64_t qh = dq + (uint64_t)h * 4 * kMat + (uint64_t)(kb * 2 * lbo >> 4);
-                        const uint32_t hi = base + kColHi + kb * 8, lo = base + kColLo + kb * 8, sg = base + kColSg + kb * 8;
-                        if (h == 0 && kb == 0) {
-                            mma_ts_first(d1, hi, qh, kIdesc);
-                            mma_ts_first(d2, sg, qh + 2 * kMat, kIdesc);
-                        } else {
-                            mma_ts_acc(d1, hi, qh, kIdesc);
-                            mma_ts_acc(d2, sg, qh + 2 * kMat, kIdesc);
-                        }
-                        mma_ts_acc(d1, hi, qh + kMat, kIdesc);
-                        mma_ts_acc(d2, sg, qh + 3 * kMat, kIdesc);
-                        mma_ts_acc(d1, lo, qh, kIdesc);
+            // operand buffers of the tile: the one of its group of expanders, or both, and which filling of them
+            const int b0 = kHalves == 2 ? 0 : (int)(i & 1);
+            const uint32_t use = kHalves == 2 ? i : i >> 1;
+            go = warp_wait(BAR(SB_A_FULL + b0), use & 1u, abort_flag) &&
+                 (kHalves == 1 || warp_wait(BAR(SB_A_FULL + 1), use & 1u, abort_flag)) &&
+                 warp_wait(BAR(SB_D_EMPTY + db), ((i / kDBufs) & 1) ^ 1u, abort_flag);
+            if (!go) break;
+            tc_fence_after();
+            if (elect_one()) {
+                // The products with a lo part come first: the tensor pipe truncates its sums at every instruction, by a share of
+                // what they have grown to, and so the small products cost nothing (all three products of a k-block in turn:
+                // 1.3 to 1.5 times the error of sums of their own for the lo parts; so 0.7 to 0.9 times).  Rolled up, the loops
+                // issue too slowly (32 x 1,048,576 scores at d = 128: 80 us, unrolled by eight 66).
+                // The start-address field of a descriptor counts 16-byte units: one k-block is two core matrices further, the
+                // operand matrices of the second half of the coordinates follow those of the first.
+                constexpr uint64_t kBlock = 2 * 128 >> 4;
+#pragma unroll 8
+                for (int kb = 0; kb < DR / 16; ++kb) {
+                    const int h = kb / (kDH / 16), k = kb % (kDH / 16);
+                    const uint32_t buf = tm + (b0 + h) * kBufCols + k * 8;
+                    const uint64_t qh = dq + (uint64_t)h * 4 * kMat + k * kBlock;
+                    if (kb == 0) {
+                        mma_ts_first(d1, buf + kColHi, qh + kMat, kIdesc);
+                        mma_ts_first(d2, buf + kColSg, qh + 3 * kMat, kIdesc);
+                    } else {
+                        mma_ts_acc(d1, buf + kColHi, qh + kMat, kIdesc);
+                        mma_ts_acc(d2, buf + kColSg, qh + 3 * kMat, kIdesc);
                     }
-                    if (h == kHalves - 1) mma_commit(BAR(SB_D_FULL + db));
-                    mma_commit(BAR(SB_A_EMPTY + b));
-                    if (h == kHalves - 1 && last_of_group) mma_commit(BAR(SB_B_EMPTY + bb));
+                    mma_ts_acc(d1, buf + kColLo, qh, kIdesc);
                 }
-                __syncwarp();
+#pragma unroll 8
+                for (int kb = 0; kb < DR / 16; ++kb) {
+                    const int h = kb / (kDH / 16), k = kb % (kDH / 16);
+                    const uint32_t buf = tm + (b0 + h) * kBufCols + k * 8;
+                    const uint64_t qh = dq + (uint64_t)h * 4 * kMat + k * kBlock;
+                    mma_ts_acc(d1, buf + kColHi, qh, kIdesc);
+                    mma_ts_acc(d2, buf + kColSg, qh + 2 * kMat, kIdesc);
+                    if (kHalves == 2 && k + 1 == kDH / 16) mma_commit(BAR(SB_A_EMPTY + h));
+                }
+                mma_commit(BAR(SB_D_FULL + db));
+                if (kHalves == 1) mma_commit(BAR(SB_A_EMPTY + b0));
+                if (last_of_group) mma_commit(BAR(SB_B_EMPTY + bb));
             }
+            __syncwarp();
         }
     } else if (warp < kFirstEpiWarp) {
         // ---- expanders: two threads per key, every second tile (d = 256: every tile, a half of its coordinates) --------
