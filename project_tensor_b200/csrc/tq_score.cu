@@ -23,7 +23,8 @@ constexpr int kQT = 8;  // queries scored together per pass over a block's keys
 constexpr int kMatThreads = 256;   // threads of score_matrix_kernel
 
 // Both kernels give a score the same bits: the sums of the rotated and projected queries come in slices of k, added up in order;
-// a score is one chain over the coordinates, centroid and sign in turn.
+// a score has a chain of its own for the centroids and one for the signs (one chain for both, centroid and sign in turn, took eight registers
+// less a key and gave 6 to 20 % more error).
 __host__ __device__ inline int query_slices(int d) {
     const int quarter = ((d + 31) & ~31) / 2;
     return quarter < kMatThreads ? kMatThreads / quarter : 1;
@@ -83,9 +84,9 @@ score_kernel(TqDev p, const float* __restrict__ q, int qpg, const uint32_t* __re
         for (int64_t kb = k0; kb < k1; kb += kThreads) {
             const int64_t key = kb + threadIdx.x;
             const bool live = key < k1;
-            float acc[kQT];
+            float a1[kQT], a2[kQT];
 #pragma unroll
-            for (int t = 0; t < kQT; ++t) acc[t] = 0.f;
+            for (int t = 0; t < kQT; ++t) { a1[t] = 0.f; a2[t] = 0.f; }
             if (live) {
                 const float arn = p.alpha * rnorms[gbase + key];
                 const uint32_t* crow = codes + (gbase + key) * p.code_words;
@@ -94,15 +95,18 @@ score_kernel(TqDev p, const float* __restrict__ q, int qpg, const uint32_t* __re
                 for (int j = 0; j < d; ++j) {
                     if ((j & 31) == 0) sw = srow[j >> 5];
                     const float c = cb[tq_get_code(crow, j, p.bits)];
-                    const float s = (sw >> tq_sign_bitpos(j)) & 1u ? arn : -arn;
+                    const float s = (sw >> tq_sign_bitpos(j)) & 1u ? 1.f : -1.f;
 #pragma unroll
-                    for (int t = 0; t < kQT; ++t) acc[t] = fmaf(s, qs[(t * 2 + 1) * d + j], fmaf(c, qs[(t * 2) * d + j], acc[t]));
+                    for (int t = 0; t < kQT; ++t) {
+                        a1[t] = fmaf(c, qs[(t * 2) * d + j], a1[t]);
+                        a2[t] = fmaf(s, qs[(t * 2 + 1) * d + j], a2[t]);
+                    }
                 }
                 const float nrm = norms[gbase + key];
 #pragma unroll
                 for (int t = 0; t < kQT; ++t) {
                     if (t < nq) {
-                        const float s = nrm * acc[t];
+                        const float s = nrm * fmaf(arn, a2[t], a1[t]);
                         if (scores) scores[((int64_t)g * qpg + q0 + t) * keys_per_group + key] = s;
                         if (topk > 0) {
                             const unsigned long long ck = make_key(s, (uint32_t)(gbase + key));
@@ -150,7 +154,7 @@ score_kernel(TqDev p, const float* __restrict__ q, int qpg, const uint32_t* __re
 
 // A score matrix without top-k, any d and bits: the case that repeats (validation runs and sweeps at dimensions or bit widths without
 // a tensor-core kernel).  A thread scores KT keys for QT queries, 32 coordinates at a time -- BITS words of codes, taken apart with
-// compile-time shifts, and one sign word; c * (R q)[j] and +-(alpha * rnorm) * (S q)[j] add up in one accumulator.  The shared-memory
+// compile-time shifts, and one sign word; c * (R q)[j] and +-(S q)[j] add up in two.  The shared-memory
 // pipe returns 16 bytes a lane in four cycles, so one pair of query vectors has to feed several keys: four keys x eight queries
 // balance it with the FMA pipe.  The queries are rotated and projected by the whole block, four outputs and a slice of the sum
 // per thread with 32 or 64 matrix elements in flight.  50,021 keys, d = 96, 5-bit codes, 16 queries: 96 us in the kernel above
@@ -233,17 +237,15 @@ score_matrix_kernel(TqDev p, const float* __restrict__ q, int qpg, const uint32_
         }
     }
     for (int64_t kb = (int64_t)blockIdx.x * kMatThreads * KT; kb < keys_per_group; kb += (int64_t)gridDim.x * kMatThreads * KT) {
-        float2 acc[KT][QT / 2];
-        float arn[KT];
+        float2 a1[KT][QT / 2], a2[KT][QT / 2];
         const uint32_t *crow[KT], *srow[KT];
 #pragma unroll
         for (int e = 0; e < KT; ++e) {
             const int64_t key = kb + t + e * kMatThreads, row = gbase + (key < keys_per_group ? key : keys_per_group - 1);
             crow[e] = codes + row * p.code_words;
             srow[e] = signs + row * p.sign_words;
-            arn[e] = p.alpha * __ldg(rnorms + row);
 #pragma unroll
-            for (int u = 0; u < QT / 2; ++u) acc[e][u] = make_float2(0.f, 0.f);
+            for (int u = 0; u < QT / 2; ++u) a1[e][u] = a2[e][u] = make_float2(0.f, 0.f);
         }
         uint32_t wn[KT][BITS], sn[KT];               // words of the next 32 coordinates
         auto fetch = [&](int j0) {
@@ -287,11 +289,11 @@ score_matrix_kernel(TqDev p, const float* __restrict__ q, int qpg, const uint32_
                     uint32_t code = w[e][at] >> sh;
                     if (sh + BITS > 32) code |= w[e][at + 1 < BITS ? at + 1 : at] << (32 - sh);
                     const float c = cb[code & kMask];
-                    const float s = __uint_as_float(__float_as_uint(arn[e]) ^ ((sw[e] << (31 - tq_sign_bitpos(i))) & 0x80000000u));
+                    const float s = __uint_as_float(0x3f800000u ^ ((sw[e] << (31 - tq_sign_bitpos(i))) & 0x80000000u));
 #pragma unroll
                     for (int u = 0; u < QT / 2; ++u) {
-                        acc[e][u] = __ffma2_rn(make_float2(c, c), x[0][u], acc[e][u]);
-                        acc[e][u] = __ffma2_rn(make_float2(s, s), x[1][u], acc[e][u]);
+                        a1[e][u] = __ffma2_rn(make_float2(c, c), x[0][u], a1[e][u]);
+                        a2[e][u] = __ffma2_rn(make_float2(s, s), x[1][u], a2[e][u]);
                     }
                 }
             }
@@ -300,11 +302,11 @@ score_matrix_kernel(TqDev p, const float* __restrict__ q, int qpg, const uint32_
         for (int e = 0; e < KT; ++e) {
             const int64_t key = kb + t + e * kMatThreads;
             if (key >= keys_per_group) break;
-            const float nrm = __ldg(norms + gbase + key);
+            const float nrm = __ldg(norms + gbase + key), arn = p.alpha * __ldg(rnorms + gbase + key);
             float* dst = scores + ((int64_t)g * qpg + q0) * keys_per_group + key;
 #pragma unroll
             for (int u = 0; u < QT; ++u)
-                if (u < nq) dst[u * keys_per_group] = nrm * (u & 1 ? acc[e][u / 2].y : acc[e][u / 2].x);
+                if (u < nq) dst[u * keys_per_group] = nrm * (u & 1 ? fmaf(arn, a2[e][u / 2].y, a1[e][u / 2].y) : fmaf(arn, a2[e][u / 2].x, a1[e][u / 2].x));
         }
     }
 }

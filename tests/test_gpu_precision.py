@@ -28,7 +28,7 @@ def _keys64(quant, enc):
 _MANY = {64: 2.95e-7, 128: 4.4e-7, 256: 6.3e-7, 96: 2.75e-7}
 
 
-@pytest.mark.parametrize("d", [64, 128, 256])
+@pytest.mark.parametrize("d", [64, 96, 128, 256])
 @pytest.mark.parametrize("bits", [2, 3, 4, 5])
 def test_scores(d, bits):
     n = 20011
