@@ -66,18 +66,36 @@ score_kernel(TqDev p, const float* __restrict__ q, int qpg, const uint32_t* __re
         if (threadIdx.x == 0) need_prune = 0;
         __syncthreads();
         // rotated / projected queries: qs[t][0][j] = sum_k R[j][k] q[k],  qs[t][1][j] = sum_k S[j][k] q[k]
-        for (int i = threadIdx.x; i < kQT * 2 * d; i += kThreads) {
-            const int t = i / (2 * d), r = i - t * 2 * d, which = r / d, j = r - which * d;
-            const float* M = which ? p.St : p.Rt;
-            const float* qv = qraw + t * d;
-            float sum = 0.f;
-            const int slices = query_slices(d), len = (d + slices - 1) / slices;
-            for (int k0 = 0; k0 < d; k0 += len) {
-                float acc = 0.f;
-                for (int k = k0; k < min(k0 + len, d); ++k) acc = fmaf(qv[k], __ldg(M + (size_t)k * d + j), acc);
-                sum += acc;
+        // (a thread takes a column of a matrix for all queries: its elements are loaded once, eight at a time)
+        const int slices = query_slices(d), len = (d + slices - 1) / slices;
+        for (int i = threadIdx.x; i < 2 * d; i += kThreads) {
+            const int which = i >= d ? 1 : 0, j = i - which * d;
+            const float* M = (which ? p.St : p.Rt) + j;
+            float sum[kQT];
+#pragma unroll
+            for (int t = 0; t < kQT; ++t) sum[t] = 0.f;
+            for (int s0 = 0; s0 < d; s0 += len) {
+                const int s1 = min(s0 + len, d);
+                float acc[kQT];
+#pragma unroll
+                for (int t = 0; t < kQT; ++t) acc[t] = 0.f;
+                for (int k = s0; k < s1; k += 8) {
+                    float m[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) m[u] = k + u < s1 ? __ldg(M + (size_t)(k + u) * d) : 0.f;
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        if (k + u < s1) {
+#pragma unroll
+                            for (int t = 0; t < kQT; ++t) acc[t] = fmaf(qraw[t * d + k + u], m[u], acc[t]);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int t = 0; t < kQT; ++t) sum[t] += acc[t];
             }
-            qs[i] = sum;
+#pragma unroll
+            for (int t = 0; t < kQT; ++t) qs[(t * 2 + which) * d + j] = sum[t];
         }
         __syncthreads();
 
