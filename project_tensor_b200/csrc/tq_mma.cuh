@@ -78,6 +78,18 @@ __device__ __forceinline__ uint32_t pick(uint32_t word, int byte, uint32_t copy)
     return __byte_perm(word, copy, 0x5504u | (uint32_t)byte << 4);
 }
 
+// Bits of two keys as +-1 (set: +1): step S takes bits 2S and 2S + 1 of the halves of the keys' words.  (Bits used where they stand, as
+// subnormal numbers, save an instruction each, but their sums are several times the signed ones, and the rounding of the
+// accumulators with them.)
+template <int S, int WORDS>
+__device__ __forceinline__ void plus_minus(const uint32_t (&w)[2][WORDS], uint32_t (&a)[4]) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        a[h] = ((w[h][S >> 3] << (15 - (2 * S & 15))) & 0x80008000u) ^ 0xbc00bc00u;
+        a[2 + h] = ((w[h][S >> 3] << (14 - (2 * S & 15))) & 0x80008000u) ^ 0xbc00bc00u;
+    }
+}
+
 // The words of two keys that lane t of a quad turns into operands: DR / 4 consecutive coordinates of each.
 template <int KB, int DR>
 struct KeyWords {
@@ -144,16 +156,8 @@ struct KeyWords {
         }
         signs<S>(as);
     }
-    // Signs of coordinates 4s .. 4s + 3 as +-1.  (Bits used where they stand, as subnormal numbers, save an instruction each, but
-    // their sums are several times the signed ones, and the rounding of the accumulators with them.)
     template <int S>
-    __device__ __forceinline__ void signs(uint32_t (&as)[4]) const {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            as[h] = ((sw[h][S >> 3] << (15 - (2 * S & 15))) & 0x80008000u) ^ 0xbc00bc00u;
-            as[2 + h] = ((sw[h][S >> 3] << (14 - (2 * S & 15))) & 0x80008000u) ^ 0xbc00bc00u;
-        }
-    }
+    __device__ __forceinline__ void signs(uint32_t (&as)[4]) const { plus_minus<S>(sw, as); }
 };
 
 }  // namespace tqmma

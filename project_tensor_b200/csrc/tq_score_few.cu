@@ -9,8 +9,11 @@
 // flight, no barriers; the tables (tq_mma.cuh) do not depend on the queries, so they are built while the matrices are on
 // their way, and the matrices while the queries are (page-locked host memory in a NumPy call).
 //
-// 1-bit codes need no table: a centroid is c0 + bit (c1 - c0), so their bits are an operand where they stand, as subnormal
-// fp16 numbers that the scale of the rotated query makes up for.
+// 1-bit codes need no table: a centroid is (c0 + c1) / 2 +- (c1 - c0) / 2, so their bits become +-1 as the signs do.  (c0 + bit (c1 - c0),
+// the bits used where they stand, saved an instruction a register and gave ten times the error: the two terms cancel.)
+//
+// The tensor pipe truncates a sum at every instruction, so a score is added up from two chains of half the coordinates each (one
+// chain: 3 to 12 % more error than the multiply-adds of the table kernel, two: 10 to 40 % less).
 //
 // Bound: shared-memory lookups, 64 8-byte loads a key at d = 128 and 3-bit codes (2 cycles a warp and load, four lanes a key), and for
 // few keys the prologue.  Before -- one thread per key through tables of the query's own products, whose random rows met
@@ -186,8 +189,6 @@ score_few_kernel(const TqDev p, const FewArgs a) {
 #pragma unroll
         for (int s = 0; s < P::kSteps; ++s) {
             uint32_t h0, l0, h1, l1;
-            const bool bits = m == 0 && KB == 1;         // an operand of bits where they stand, 2^(b - 24)
-            const float s0 = bits ? sc * (1.f / (1 << ((2 * s) & 7))) : sc, s1 = bits ? sc * (1.f / (1 << ((2 * s + 1) & 7))) : sc;
             float4 f;
             if (KB == 1 && m == 0) {
                 // 1-bit codes: coordinates that lie half a word apart make a pair
@@ -197,8 +198,8 @@ score_few_kernel(const TqDev p, const FewArgs a) {
             } else {
                 f = *reinterpret_cast<const float4*>(x + 4 * s);
             }
-            split_pair(f.x * s0, f.y * s0, h0, l0);
-            split_pair(f.z * s1, f.w * s1, h1, l1);
+            split_pair(f.x * sc, f.y * sc, h0, l0);
+            split_pair(f.z * sc, f.w * sc, h1, l1);
             qf[m][s][0] = r < 4 ? h0 : l0;
             qf[m][s][1] = r < 4 ? h1 : l1;
         }
@@ -209,10 +210,10 @@ score_few_kernel(const TqDev p, const FewArgs a) {
     for (int c = 0; c < 2; ++c) {
         const int qq = (2 * t + c) & (NQ - 1);
         ds1[c] = pow2i(-scl[qq]) * (1.f / kCentScale);
-        if constexpr (KB == 1) {                  // a centroid is c0 + bit (c1 - c0)
-            const float c0 = __ldg(p.codebook);
-            ds1[c] = pow2i(24 - scl[qq]) * (__ldg(p.codebook + 1) - c0);
-            dbase[c] = 2 * t < NQ ? c0 * psum[qq] : 0.f;
+        if constexpr (KB == 1) {
+            const float c0 = __ldg(p.codebook), c1 = __ldg(p.codebook + 1);
+            ds1[c] = pow2i(-scl[qq]) * (0.5f * (c1 - c0));
+            dbase[c] = 2 * t < NQ ? 0.5f * (c0 + c1) * psum[qq] : 0.f;
         }
         ds2[c] = pow2i(-scl[NQ + qq]) * p.alpha;
     }
@@ -226,8 +227,7 @@ score_few_kernel(const TqDev p, const FewArgs a) {
         if (tile + stride < tiles) fetch(tile + stride, nxt);
         W key;
         key.unpack(cur.kc, cur.sg, kshift, t);
-        float c1[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, c2[4] = {0.f, 0.f, 0.f, 0.f};
-        uint32_t cbits[2][2 * W::kWords];        // 1-bit codes: the word, and the word moved by 8
+        uint32_t cbits[2][W::kWords];
         if constexpr (KB == 1) {
 #pragma unroll
             for (int h = 0; h < 2; ++h)
@@ -235,39 +235,44 @@ score_few_kernel(const TqDev p, const FewArgs a) {
                 for (int i = 0; i < W::kWords; ++i) {
                     uint32_t w = cur.kc[h][i];
                     if (DR == 64) { w >>= kshift; w = (w & 0xffu) | ((w & 0xff00u) << 8); }
-                    cbits[h][2 * i] = w;
-                    cbits[h][2 * i + 1] = w >> 8;
+                    cbits[h][i] = w;
                 }
         }
-        for_steps<P::kSteps>([&](auto sc) {
-            constexpr int s = decltype(sc)::value;
-            uint32_t ak[2][4], as[4];
-            if constexpr (KB == 1) {
-                uint32_t ab[4];
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    ab[h] = cbits[h][s >> 2] & (0x00010001u << ((2 * s) & 7));
-                    ab[2 + h] = cbits[h][s >> 2] & (0x00010001u << ((2 * s + 1) & 7));
-                }
-                key.template signs<s>(as);
-                mma16816(c1[0], ab, qf[0][s][0], qf[0][s][1]);
-                mma16816(c2, as, qf[1][s][0], qf[1][s][1]);
-                return;
-            }
-            key.template operands<s>(smem, lane8, lane16, ak, as);
-            mma16816(c1[0], ak[0], qf[0][s][0], qf[0][s][1]);
-            mma16816(c1[1], ak[1], qf[0][s][0], qf[0][s][1]);
-            mma16816(c2, as, qf[1][s][0], qf[1][s][1]);
-        });
         float v[2][2];                 // [key r + 8 h][query column c]
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
+            for (int c = 0; c < 2; ++c) v[h][c] = dbase[c];
+        auto half = [&](auto first) {
+            float c1[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, c2[4] = {0.f, 0.f, 0.f, 0.f};
+            for_steps<P::kSteps / 2>([&](auto sc) {
+                constexpr int s = decltype(first)::value + decltype(sc)::value;
+                uint32_t ak[2][4], as[4];
+                if constexpr (KB == 1) {
+                    plus_minus<s>(cbits, ak[0]);
+                    key.template signs<s>(as);
+                    mma16816(c1[0], ak[0], qf[0][s][0], qf[0][s][1]);
+                } else {
+                    key.template operands<s>(smem, lane8, lane16, ak, as);
+                    mma16816(c1[0], ak[0], qf[0][s][0], qf[0][s][1]);
+                    mma16816(c1[1], ak[1], qf[0][s][0], qf[0][s][1]);
+                }
+                mma16816(c2, as, qf[1][s][0], qf[1][s][1]);
+            });
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+                    v[h][c] += fmaf(c2[2 * h + c] * ds2[c], cur.rn[h], (KB == 1 ? c1[0][2 * h + c] : c1[h][c] + c1[h][2 + c]) * ds1[c]);
+        };
+        half(std::integral_constant<int, 0>{});
+        half(std::integral_constant<int, P::kSteps / 2>{});
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
             for (int c = 0; c < 2; ++c) {
-                const float centroids = KB == 1 ? fmaf(c1[0][2 * h + c], ds1[c], dbase[c]) : (c1[h][c] + c1[h][2 + c]) * ds1[c];
-                float s = fmaf(c2[2 * h + c] * ds2[c], cur.rn[h], centroids);
-                s += __shfl_xor_sync(0xffffffffu, s, 2);     // hi and lo columns
-                v[h][c] = s * cur.kn[h];
+                v[h][c] += __shfl_xor_sync(0xffffffffu, v[h][c], 2);     // hi and lo columns
+                v[h][c] *= cur.kn[h];
             }
         const uint32_t k0 = tile * kTile + r + 8 * (t >> 1);
 #pragma unroll

@@ -25,6 +25,7 @@ def _keys64(quant, enc):
     return rows * enc.norms.double()[:, None]
 
 
+_FEW = {64: 1.75e-7, 128: 2.6e-7, 256: 3.6e-7, 96: 2.75e-7}
 _MANY = {64: 2.95e-7, 128: 4.4e-7, 256: 6.3e-7, 96: 2.75e-7}
 
 
@@ -35,8 +36,9 @@ def test_scores(d, bits):
     quant = tg.TurboQuantProd(d, bits, seed=2026)
     enc = quant.quantize(_randn((n, d), d + bits))
     keys = _keys64(quant, enc)
-    for nq in (5, 16, 40):
+    few = {64: 2, 128: 4 if bits <= 4 else 2, 256: 1, 96: 1}[d]       # queries that the warp-level kernel takes
+    for nq in (1, 2, 3, 4, 5, 16, 40):
         q = _randn((nq, d), nq)
         want = q.double() @ keys.T
         err = float((quant.attention_scores(q, enc).double() - want).norm() / want.norm())
-        assert err <= _MANY[d], (nq, err)
+        assert err <= (_FEW if nq <= few else _MANY)[d], (nq, err)
