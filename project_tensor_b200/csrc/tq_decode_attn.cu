@@ -312,47 +312,56 @@ decode_partial_kernel(TqDev kp, DecodeArgs a) {
         if (tile + kWarps < tile1) fetch(tile + kWarps, nxt);
         const uint32_t left = keys - tile * kTile;      // keys of this tile and behind it
         // -- scores
-        float c1[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, c2[4] = {0.f, 0.f, 0.f, 0.f};
         KeyWords<KB, DR> key;
         key.unpack(cur.kc, cur.sg, kshift, t);
-        auto key_step = [&](auto sc) {
-            constexpr int s = decltype(sc)::value;
-            uint32_t ak[2][4], as[4];
-            key.template operands<s>(smem, lane8, lane16, ak, as);
-            if constexpr (NQ == 4) {
-                mma16816(c1[0], ak[0], qf[0][s][0], qf[0][s][1]);
-                mma16816(c1[1], ak[1], qf[0][s][0], qf[0][s][1]);
-                mma16816(c2, as, qf[1][s][0], qf[1][s][1]);
-            } else {
-                const uint4 b = *reinterpret_cast<const uint4*>(smem + P::off_frag + (s * 32 + lane) * 16);
-                const uint4 p = *reinterpret_cast<const uint4*>(smem + P::off_frag + P::kFragBytes + (s * 32 + lane) * 16);
-                mma16816(c1[0], ak[0], b.x, b.y);
-                mma16816(c1[1], ak[1], b.x, b.y);
-                mma16816(c2, as, p.x, p.y);
-                mma16816(c1[0], ak[0], b.z, b.w);
-                mma16816(c1[1], ak[1], b.z, b.w);
-                mma16816(c2, as, p.z, p.w);
-            }
+        float s[2][2] = {{0.f, 0.f}, {0.f, 0.f}};                 // [key r + 8 h][query column c]
+        auto half = [&](auto first) {       // (a chain of half the coordinates: the tensor pipe truncates its sums at every instruction)
+            float c1[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, c2[4] = {0.f, 0.f, 0.f, 0.f};
+            for_steps<P::kSteps / 2>([&](auto sc) {
+                constexpr int s = decltype(first)::value + decltype(sc)::value;
+                uint32_t ak[2][4], as[4];
+                key.template operands<s>(smem, lane8, lane16, ak, as);
+                if constexpr (NQ == 4) {
+                    mma16816(c1[0], ak[0], qf[0][s][0], qf[0][s][1]);
+                    mma16816(c1[1], ak[1], qf[0][s][0], qf[0][s][1]);
+                    mma16816(c2, as, qf[1][s][0], qf[1][s][1]);
+                } else {
+                    const uint4 b = *reinterpret_cast<const uint4*>(smem + P::off_frag + (s * 32 + lane) * 16);
+                    const uint4 p = *reinterpret_cast<const uint4*>(smem + P::off_frag + P::kFragBytes + (s * 32 + lane) * 16);
+                    mma16816(c1[0], ak[0], b.z, b.w);
+                    mma16816(c1[1], ak[1], b.z, b.w);
+                    mma16816(c2, as, p.z, p.w);
+                    mma16816(c1[0], ak[0], b.x, b.y);
+                    mma16816(c1[1], ak[1], b.x, b.y);
+                    mma16816(c2, as, p.x, p.y);
+                }
+            });
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int c = 0; c < 2; ++c) s[h][c] += fmaf(c2[2 * h + c] * ds2[c], cur.rn[h], (c1[h][c] + c1[h][2 + c]) * ds1[c]);
         };
-        for_steps<P::kSteps>(key_step);
-        float s[2][2];                 // [key r + 8 h][query column c]
+        half(std::integral_constant<int, 0>{});
+        half(std::integral_constant<int, P::kSteps / 2>{});
+        // the exponent of key r + 8 h is s * f[h]; keys behind the last: -inf
+        float f[2];
         bool above = false;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
+            const bool have = key_r + 8 * h < left;
+            f[h] = have ? cur.kn[h] * a.scale_log2e : 1.f;
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
-                float v = fmaf(c2[2 * h + c] * ds2[c], cur.rn[h], (c1[h][c] + c1[h][2 + c]) * ds1[c]);
-                if constexpr (NQ == 4) v += __shfl_xor_sync(0xffffffffu, v, 2);     // hi and lo columns
-                v *= cur.kn[h] * a.scale_log2e;
-                s[h][c] = key_r + 8 * h < left ? v : -CUDART_INF_F;
-                above = above || s[h][c] > mref[c] + kSlack;
+                if constexpr (NQ == 4) s[h][c] += __shfl_xor_sync(0xffffffffu, s[h][c], 2);     // hi and lo columns
+                if (!have) s[h][c] = -CUDART_INF_F;
+                above = above || s[h][c] * f[h] > mref[c] + kSlack;
             }
         }
         // -- softmax reference and weights
         if (__any_sync(0xffffffffu, above)) {
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
-                float m = fmaxf(s[0][c], s[1][c]);
+                float m = fmaxf(s[0][c] * f[0], s[1][c] * f[1]);
 #pragma unroll
                 for (int o = 4; o < 32; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
                 m = fmaxf(m, mref[c]);
@@ -360,8 +369,8 @@ decode_partial_kernel(TqDev kp, DecodeArgs a) {
                     const float step = m - mref[c];      // +inf the first time: nothing to carry over
                     const int e0 = (int)(__float_as_uint(wsc[c]) >> 23) - 127, up = step < 252.f ? (int)step : 252;
                     const int e = min(126, e0 + up);          // older weights shrink by 2^-step: their scale may grow
-                    const float f = exp2f(-step), fw = exp2f((float)(e - e0) - step);
-                    lsum[c] *= f;
+                    const float fl = exp2f(-step), fw = exp2f((float)(e - e0) - step);
+                    lsum[c] *= fl;
                     wsc[c] = pow2i(e);
                     mref[c] = m;
 #pragma unroll
@@ -376,7 +385,8 @@ decode_partial_kernel(TqDev kp, DecodeArgs a) {
             const float vn = key_r + 8 * h < left ? cur.vn[h] : 0.f;
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
-                const float p = exp2f(s[h][c] - (mref[c] == -CUDART_INF_F ? 0.f : mref[c]));   // masked keys: exp2(-inf) = 0
+                // (one rounding, of the difference: the exponents near the reference are the ones that count)
+                const float p = exp2f(fmaf(s[h][c], f[h], mref[c] == -CUDART_INF_F ? 0.f : -mref[c]));
                 lsum[c] += p;
                 u[h][c] = p * vn;
                 big = big || u[h][c] * wsc[c] > kWeightMax;
@@ -455,9 +465,18 @@ decode_partial_kernel(TqDev kp, DecodeArgs a) {
                 ah[2 * h + 1] = *reinterpret_cast<const uint32_t*>(smem + P::off_val + o);
                 al[2 * h + 1] = *reinterpret_cast<const uint32_t*>(smem + P::off_val + 128 + o);
             }
-            mma16816(acc[mt], ah, bh[0], bh[1]);
-            mma16816(acc[mt], al, bh[0], bh[1]);
-            if constexpr (NQ == 8) mma16816(acc[mt], ah, bl[0], bl[1]);
+            // A tile's products, small ones first, in sums of their own that are rounded onto the accumulator: the tensor pipe
+            // truncates, which over a long context (32,768 keys: seven times the error) is a bias.
+            float c[4] = {0.f, 0.f, 0.f, 0.f};
+            mma16816(c, al, bh[0], bh[1]);
+            if constexpr (NQ == 8) mma16816(c, ah, bl[0], bl[1]);
+            mma16816(c, ah, bh[0], bh[1]);
+#pragma unroll
+            for (int i = 0; i < 4; i += 2) {
+                const float2 v = __fadd2_rn(make_float2(acc[mt][i], acc[mt][i + 1]), make_float2(c[i], c[i + 1]));
+                acc[mt][i] = v.x;
+                acc[mt][i + 1] = v.y;
+            }
         };
         for_steps<P::kMTiles>(value_tile);
         cur = nxt;

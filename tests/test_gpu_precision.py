@@ -8,6 +8,7 @@ import math
 import pytest
 
 import project_tensor_b200 as tg
+from project_tensor_b200.cache import PackedKVCache
 
 pytestmark = pytest.mark.gpu
 
@@ -23,6 +24,12 @@ def _keys64(quant, enc):
     rows = to64(quant.mse.codebook)[enc.indices.long()] @ to64(quant.mse.rotation)
     rows += math.sqrt(math.pi / 2) / quant.dimension * enc.residual_norms.double()[:, None] * (enc.qjl.double() @ to64(quant.projection))
     return rows * enc.norms.double()[:, None]
+
+
+def _values64(quant, enc):
+    import torch
+    to64 = lambda a: torch.as_tensor(a, device="cuda").double()
+    return to64(quant.codebook)[enc.indices.long()] @ to64(quant.rotation) * enc.norms.double()[:, None]
 
 
 _FEW = {64: 1.75e-7, 128: 2.6e-7, 256: 3.6e-7, 96: 2.75e-7}
@@ -42,3 +49,23 @@ def test_scores(d, bits):
         want = q.double() @ keys.T
         err = float((quant.attention_scores(q, enc).double() - want).norm() / want.norm())
         assert err <= (_FEW if nq <= few else _MANY)[d], (nq, err)
+
+
+@pytest.mark.parametrize("d,kbits,vbits,groups,n", [(64, 4, 3, 16, 129), (64, 4, 4, 4, 30011), (128, 4, 4, 4, 30011), (128, 2, 2, 16, 1531),
+                                                    (128, 5, 1, 4, 30011)])
+def test_attention(d, kbits, vbits, groups, n):
+    """Exponents of about 10 rounded to float32 alone give some 5e-7; the weighted sums must not add a bias to it."""
+    import torch
+    kq, vq = tg.TurboQuantProd(d, kbits, seed=2026), tg.TurboQuantMSE(d, vbits, seed=77)
+    cache = PackedKVCache(kq, vq, groups, (n + 15) // 16 * 16)
+    loud = torch.ones(d, device="cuda")
+    loud[3::d // 4] = 10.0
+    cache.append(_randn((groups, n, d), 1) * loud, _randn((groups, n, d), 2) * loud)
+    for qpg in (1, 4, 8):
+        q = _randn((groups, qpg, d), qpg)
+        got, square = cache.attend(q).double(), []
+        for g in range(groups):
+            s = (q[g].double() @ _keys64(kq, cache.keys.encoding(g)).T) * d ** -0.5
+            want = torch.softmax(s, dim=-1) @ _values64(vq, cache.value_encoding(g))
+            square.append(((got[g] - want).norm(dim=1) / want.norm(dim=1)).square())
+        assert float(torch.cat(square).mean().sqrt()) <= 1.5e-6, qpg
