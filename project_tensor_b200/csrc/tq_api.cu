@@ -108,6 +108,32 @@ int tq_device_count(void) {
     return n;
 }
 
+// The centroids as fp16 hi + lo parts of a common unit (the return value) that brings the largest to between 512 and 1024.  Two
+// fp16 numbers hold 22 bits, so every centroid has an error of its own, which all its occurrences share; among 1,024 units take the one
+// with the smallest (8 levels of d = 64 in powers of two: 6e-8 of the largest centroid, now below 1e-8).
+static float split_centroids(const float* codebook, int levels, uint32_t* parts) {
+    float top = 0.f;
+    for (int k = 0; k < levels; ++k) top = fmaxf(top, fabsf(codebook[k]));
+    if (levels > 16 || !(top > 0.f) || !(top < 1.0e30f)) return 1.f;
+    auto split = [&](float unit, int k, uint32_t* out) {
+        const double v = (double)codebook[k] / unit;
+        const __half hi = __float2half_rn((float)v);
+        const __half lo = __float2half_rn((float)(v - (double)__half2float(hi)));
+        if (out) *out = (uint32_t)__half_as_ushort(hi) | (uint32_t)__half_as_ushort(lo) << 16;
+        return v - (double)__half2float(hi) - (double)__half2float(lo);
+    };
+    float best = 0.f;
+    double least = -1.0;
+    for (int i = 0; i < 1024; ++i) {
+        const float unit = top / (float)(1023.5 - 0.5 * i);
+        double sum = 0.0;
+        for (int k = 0; k < levels; ++k) { const double e = split(unit, k, nullptr) * unit; sum += e * e; }
+        if (least < 0.0 || sum < least) { least = sum; best = unit; }
+    }
+    for (int k = 0; k < levels; ++k) split(best, k, parts + k);
+    return best;
+}
+
 int tq_plan_create(int d, int bits_mse, const float* rotation, const float* codebook, const float* projection,
                    int device, tq_plan** out) {
     if (!out) return tq_fail(TQ_ERR_INVALID_ARGUMENT, "out is null");
@@ -138,7 +164,7 @@ int tq_plan_create(int d, int bits_mse, const float* rotation, const float* code
     // host staging: R, Rt, S, St, codebook, boundaries, counters (padded to 256 B each)
     auto pad = [](size_t bytes) { return (bytes + 255) & ~size_t(255); };
     const size_t o_R = 0, o_Rt = o_R + pad(dd * 4), o_S = o_Rt + pad(dd * 4), o_St = o_S + pad(dd * 4),
-                 o_cb = o_St + pad(dd * 4), o_bd = o_cb + pad(levels * 4), o_cnt = o_bd + pad(levels * 4),
+                 o_cb = o_St + pad(dd * 4), o_bd = o_cb + pad(levels * 4), o_parts = o_bd + pad(levels * 4), o_cnt = o_parts + pad(levels * 4),
                  total = o_cnt + 256;
     std::vector<unsigned char> host(total, 0);
     float* hR = reinterpret_cast<float*>(host.data() + o_R);
@@ -160,6 +186,7 @@ int tq_plan_create(int d, int bits_mse, const float* rotation, const float* code
         volatile float s = codebook[k] + codebook[k + 1];  // float32 sum, then float32 product
         hbd[k] = 0.5f * s;
     }
+    p->dev.cent_unit = split_centroids(codebook, levels, reinterpret_cast<uint32_t*>(host.data() + o_parts));
 
     cudaError_t e = cudaMalloc(&p->slab, total);
     if (e != cudaSuccess) {
@@ -186,6 +213,7 @@ int tq_plan_create(int d, int bits_mse, const float* rotation, const float* code
     v.St = projection ? reinterpret_cast<float*>(base + o_St) : nullptr;
     v.codebook = reinterpret_cast<float*>(base + o_cb);
     v.boundaries = reinterpret_cast<float*>(base + o_bd);
+    v.cent_parts = reinterpret_cast<uint32_t*>(base + o_parts);
     p->counters = reinterpret_cast<unsigned long long*>(base + o_cnt);
     void *word = nullptr, *word_dev = nullptr;
     e = cudaHostAlloc(&word, sizeof(unsigned long long), cudaHostAllocMapped | cudaHostAllocPortable);

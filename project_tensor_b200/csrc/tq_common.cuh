@@ -78,6 +78,8 @@ struct TqDev {
     const float* St;   // its transpose
     const float* codebook;    // [levels]
     const float* boundaries;  // [levels-1]
+    const uint32_t* cent_parts;  // [levels] codebook / cent_unit as fp16 hi (low half) + lo; plans of up to 4 bits
+    float cent_unit;
 };
 
 // Optional timing of the main kernel of a quantize (kind 0) or batched scoring (kind 1) call: a ring of event pairs,

@@ -66,7 +66,8 @@ struct DecodeArgs {
     const float* knorms;
     const uint32_t* vcodes;
     const float* vnorms;
-    const float* vcodebook;      // codebook of the value quantizer
+    const uint32_t* vparts;      // centroids of the value quantizer, in parts of vunit
+    float vunit;
     int qpg;
     int64_t keys_per_group, group_rows;
     const int64_t* length;       // optional device-side number of keys per group (capped by keys_per_group)
@@ -202,11 +203,10 @@ decode_partial_kernel(TqDev kp, DecodeArgs a) {
     // Key table, row e: 128 bytes of copies of (hi, lo) of a pair of codes, or (hi, lo, hi, lo) of four codes: the registers
     // of an A operand.  Value table: 32 copies of hi, 32 copies of lo of the same coordinate of two keys.  A thread fills whole
     // rows, starting at a copy of its own (stores to rows 256 bytes apart would all hit the same banks).
-    auto value = [](const float* codebook, int code) { return __ldg(codebook + code) * kCentScale; };
-    build_key_table<KB>(smem, kp.codebook, tid, kThreads);
+    build_key_table<KB>(smem, kp.cent_parts, tid, kThreads);
     for (int e = kThreads - 1 - tid; e < 1 << (2 * VB); e += kThreads) {
         uint32_t hi, lo;
-        split_pair(value(a.vcodebook, e & ((1 << VB) - 1)), value(a.vcodebook, e >> VB), hi, lo);
+        pair_parts(__ldg(a.vparts + (e & ((1 << VB) - 1))), __ldg(a.vparts + (e >> VB)), hi, lo);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             *reinterpret_cast<uint4*>(smem + P::off_val + e * kRowBytes + ((i + tid) & 7) * 16) = make_uint4(hi, hi, hi, hi);
@@ -289,7 +289,7 @@ decode_partial_kernel(TqDev kp, DecodeArgs a) {
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
         const int qq = (2 * t + c) & (NQ - 1);
-        ds1[c] = pow2i(-scl[qq]) * (1.f / kCentScale);
+        ds1[c] = pow2i(-scl[qq]) * kp.cent_unit;
         ds2[c] = pow2i(-scl[NQ + qq]) * kp.alpha;
         mref[c] = -CUDART_INF_F;
         lsum[c] = 0.f;
@@ -514,7 +514,7 @@ decode_partial_kernel(TqDev kp, DecodeArgs a) {
 #pragma unroll
     for (int i = 0; i < P::kMTiles; ++i)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) wacc[warp * kAcc + (i * 4 + c) * 32 + lane] = acc[i][c] * (1.f / wsc[c & 1]) * (1.f / kCentScale);
+        for (int c = 0; c < 4; ++c) wacc[warp * kAcc + (i * 4 + c) * 32 + lane] = acc[i][c] * (1.f / wsc[c & 1]) * a.vunit;
     __syncthreads();
     for (int i = tid; i < NQ * DR; i += kThreads) {
         const int qq = i / DR, j = i - qq * DR;
@@ -689,7 +689,7 @@ int tq_launch_decode_attention(const tq_plan* kp, const tq_plan* vp, const float
     const int passes = (qpg + qp - 1) / qp;
     DecodeArgs a{};
     a.q = q; a.kcodes = kcodes; a.ksigns = ksigns; a.krnorms = krnorms; a.knorms = knorms;
-    a.vcodes = vcodes; a.vnorms = vnorms; a.vcodebook = vp->dev.codebook;
+    a.vcodes = vcodes; a.vnorms = vnorms; a.vparts = vp->dev.cent_parts; a.vunit = vp->dev.cent_unit;
     a.qpg = qpg; a.keys_per_group = keys_per_group; a.group_rows = group_rows; a.length = length;
     a.scale_log2e = scale * 1.4426950408889634f;
     a.splits = splits_for(tq_sm_count(kp->device), groups, passes, keys_per_group);

@@ -8,7 +8,6 @@
 
 namespace tqmma {
 
-constexpr float kCentScale = 1024.f;   // centroids (at most 1 in magnitude) before their split into fp16 hi + lo
 constexpr int kRowBytes = 256;         // a table row (keys use the first half)
 
 __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -28,6 +27,11 @@ __device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint3
     const float2 f = __half22float2(h);
     hi = half2_bits(h);
     lo = half2_bits(__floats2half2_rn(a - f.x, b - f.y));
+}
+// Parts (hi, lo) of two centroids -> hi pair, lo pair.
+__device__ __forceinline__ void pair_parts(uint32_t a, uint32_t b, uint32_t& hi, uint32_t& lo) {
+    hi = __byte_perm(a, b, 0x5410);
+    lo = __byte_perm(a, b, 0x7632);
 }
 // Shift left by s (negative: right) with s known at compile time.
 template <int S> __device__ __forceinline__ uint32_t shl(uint32_t v) {
@@ -60,13 +64,13 @@ __host__ __device__ constexpr int table_rows(int bits) { return bits == 1 ? 16 :
 // operand.  A thread fills whole rows, starting at a copy of its own (stores to rows 256 bytes apart would all hit the same
 // banks).
 template <int KB>
-__device__ __forceinline__ void build_key_table(unsigned char* table, const float* __restrict__ codebook, int tid, int threads) {
-    auto value = [&](int code) { return __ldg(codebook + code) * kCentScale; };
+__device__ __forceinline__ void build_key_table(unsigned char* table, const uint32_t* __restrict__ parts, int tid, int threads) {
+    auto pair = [&](int c0, int c1, uint32_t& hi, uint32_t& lo) { pair_parts(__ldg(parts + c0), __ldg(parts + c1), hi, lo); };
     for (int e = tid; e < table_rows(KB); e += threads) {
         constexpr int m = (1 << KB) - 1;
         uint4 v;
-        split_pair(value(e & m), value((e >> KB) & m), v.x, v.y);
-        if constexpr (codes_per_row(KB) == 4) split_pair(value((e >> 2 * KB) & m), value(e >> 3 * KB), v.z, v.w);
+        pair(e & m, (e >> KB) & m, v.x, v.y);
+        if constexpr (codes_per_row(KB) == 4) pair((e >> 2 * KB) & m, e >> 3 * KB, v.z, v.w);
         else { v.z = v.x; v.w = v.y; }
 #pragma unroll
         for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(table + e * kRowBytes + ((i + tid) & 7) * 16) = v;

@@ -121,7 +121,7 @@ score_few_kernel(const TqDev p, const FewArgs a) {
             w.rn[h] = __ldg(rn_base + key);
         }
     };
-    if (KB > 1) build_key_table<KB>(smem, p.codebook, tid, kFewThreads);
+    if (KB > 1) build_key_table<KB>(smem, p.cent_parts, tid, kFewThreads);
     tq_grid_release();
     tq_grid_wait();         // (only constants of the plan have been read so far)
     Words cur;
@@ -209,7 +209,7 @@ score_few_kernel(const TqDev p, const FewArgs a) {
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
         const int qq = (2 * t + c) & (NQ - 1);
-        ds1[c] = pow2i(-scl[qq]) * (1.f / kCentScale);
+        ds1[c] = pow2i(-scl[qq]) * p.cent_unit;
         if constexpr (KB == 1) {
             const float c0 = __ldg(p.codebook), c1 = __ldg(p.codebook + 1);
             ds1[c] = pow2i(-scl[qq]) * (0.5f * (c1 - c0));

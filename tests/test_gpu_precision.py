@@ -69,3 +69,28 @@ def test_attention(d, kbits, vbits, groups, n):
             want = torch.softmax(s, dim=-1) @ _values64(vq, cache.value_encoding(g))
             square.append(((got[g] - want).norm(dim=1) / want.norm(dim=1)).square())
         assert float(torch.cat(square).mean().sqrt()) <= 1.5e-6, qpg
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("scale", [300.0, 1e-4])
+def test_codebooks_of_any_size(d, scale):
+    """The parts of a centroid have a unit of their own, so that a plan's codebook may lie outside [-1, 1]."""
+    import torch
+    from project_tensor_b200.turboquant import _PlanSet
+    n, kq, vq = 3001, tg.TurboQuantProd(d, 4, seed=2026), tg.TurboQuantMSE(d, 4, seed=77)
+    cache = PackedKVCache(kq, vq, 1, 3008)
+    cache.append(_randn((1, n, d), 1), _randn((1, n, d), 2))
+    for quant in (kq.mse, vq):
+        quant.codebook = quant.codebook * scale
+    kq._plans = cache.keys._plans = _PlanSet(d, 3, kq.mse.rotation, kq.mse.codebook, kq.projection)
+    vq._plans = cache._vplans = _PlanSet(d, 4, vq.rotation, vq.codebook, None)
+    keys, q = _keys64(kq, cache.keys.encoding(0)), _randn((1, 2, d), 3)
+    want = q[0].double() @ keys.T
+    err = float((kq.attention_scores(q[0], cache.keys.encoding(0)).double() - want).norm() / want.norm())
+    assert err <= _FEW[d], err
+    for qpg in (2, 5):
+        q = _randn((1, qpg, d), qpg)
+        small = min(1.0, 1.0 / scale)
+        w = torch.softmax((q[0].double() @ keys.T) * small * d ** -0.5, dim=-1) @ _values64(vq, cache.value_encoding(0))
+        got = cache.attend(q, scale=small * d ** -0.5)[0].double()
+        assert float((got - w).norm() / w.norm()) <= 1.5e-6, qpg
