@@ -43,7 +43,7 @@ __device__ __forceinline__ float pow2i(int e) { return __int_as_float((min(max(e
 // power of two that brings a magnitude into [2^13, 2^14)
 __device__ __forceinline__ int scale_exp(float m) {
     if (!(m > 0.f) || !(m < 3.0e38f)) return 0;
-    return min(max(13 - (int)((__float_as_uint(m) >> 23) - 127), -100), 100);
+    return min(max(13 - (int)((__float_as_uint(m) >> 23) - 127), -115), 100);      // (the largest float needs -114)
 }
 
 // f(0), f(1), ... f(N - 1) with compile-time arguments

@@ -28,3 +28,17 @@ def test_few_queries(d, bits):
         err = parity.max_score_err(got.cpu().numpy(), want.cpu().numpy(), queries.norm(dim=1)[:, None].cpu().numpy(),
                                    knorm.cpu().numpy(), d)
         assert err <= 2e-5, (groups, qpg, n, err)
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("bits", [2, 4])
+def test_queries_near_the_largest_float(d, bits):
+    import torch
+    quant = tg.TurboQuantProd(d, bits, seed=2026)
+    gen = torch.Generator("cuda").manual_seed(d + bits)
+    enc = quant.quantize(torch.randn(300, d, device="cuda", generator=gen) * 1e-3)
+    queries = torch.randn(2, d, device="cuda", generator=gen)
+    want = quant.attention_scores(queries, enc)
+    for scale in (2.0 ** 116, 2.0 ** 121):       # (S q itself is near the largest float)
+        got = quant.attention_scores(queries * scale, enc) * (1.0 / scale)
+        assert float((got - want).abs().max()) <= 1e-6 * float(want.abs().max()), scale
