@@ -135,16 +135,16 @@ int tq_fail(int code, const char* fmt, ...);
 // Streaming multiprocessors of a device, asked for once (tq_api.cu).
 int tq_sm_count(int device);
 
-// Raise a kernel's limit of dynamic shared memory before its first launch on a device; the attribute stays with the
-// function, so later launches skip the call.
-#include <atomic>
-#define TQ_GRANT_SMEM(kernel, bytes, device)                                                                      \
-    do {                                                                                                          \
-        static std::atomic<int> granted__[64];                                                                    \
-        if (granted__[(device) & 63].load(std::memory_order_acquire) < (int)(bytes)) {                            \
-            TQ_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(bytes))); \
-            granted__[(device) & 63].store((int)(bytes), std::memory_order_release);                              \
-        }                                                                                                         \
+// Raise a kernel's limit of dynamic shared memory to what a launch needs, where it is lower.
+#include "tq_grant.h"
+#define TQ_GRANT_SMEM(kernel, bytes, device)                                                                          \
+    do {                                                                                                              \
+        static TqSmemGrant grant__;                                                                                   \
+        const cudaError_t set_shared_memory_limit =                                                                   \
+            static_cast<cudaError_t>(grant__.raise(device, (int)(bytes), [&](int limit__) {                           \
+                return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit__);       \
+            }));                                                                                                      \
+        TQ_CUDA_TRY(set_shared_memory_limit);                                                                         \
     } while (0)
 
 // A named NVTX range around the launches of one step of a call (a profiler shows the library's kernels grouped by it;
