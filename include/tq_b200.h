@@ -197,8 +197,9 @@ int tq_score_cache(const tq_plan* plan, const float* q, int groups, int q_per_gr
  * group g is written to row g * capacity + *length + j, with the same numbers tq_*_quantize gives
  * (the arithmetic of _quant.py:224-236, 300-308 in the reference's order of operations); rows that would
  * land beyond `capacity` are dropped.  advance != 0: afterwards *length = min(*length + tokens, capacity),
- * in stream order.  One kernel launch, no scratch, any d and bits.  While a launch with advance != 0 runs, the
- * word at `length` holds other values; it is right again for whatever follows on the stream.
+ * in stream order.  One kernel launch, no scratch, any d and bits.  While a launch with advance != 0 runs, bits 40 and up
+ * of the word at `length` count its blocks; they are zero again for whatever follows on the stream, and a reader on another
+ * stream that masks them off, as tq_decode_attention does, sees the old length or the new one.
  * No reference counterpart (TurboQuantProd.quantize, _quant.py:297-315, always builds a new encoding).
  */
 int tq_mse_append(const tq_plan* plan, const float* x, int groups, int tokens, void* codes, float* norms,

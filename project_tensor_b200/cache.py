@@ -20,6 +20,10 @@ from . import _native
 from . import turboquant as _tq
 
 
+#: the length's bits of its device word; an append that runs on another stream counts its blocks in those above
+_LENGTH_MASK = (1 << 40) - 1
+
+
 def _widen(staged):
     staged.tensor = staged.tensor.float()
     return staged
@@ -63,7 +67,7 @@ class PackedKeyCache:
 
     def sync_length(self) -> int:
         """Read the length back from the device (needed after replaying a CUDA graph that appends)."""
-        self._length = int(self.length_device.item())
+        self._length = int(self.length_device.item()) & _LENGTH_MASK
         self._plans.check_status(self.device)
         return self._length
 

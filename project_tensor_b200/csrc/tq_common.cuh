@@ -47,6 +47,12 @@ struct TqRecheck {
 // `length` lives on the device (one value for all groups), so a captured launch stays valid while the cache
 // grows; where it is null the rows go behind `base` instead, and `counter` is what a launch that is told to raises by `tokens`.
 // tokens == 0: output row = input row.
+// The length is in the low kLengthBits bits of its word; an append that raises it counts its blocks in the bits above while it runs.
+constexpr int kLengthBits = 40;
+__device__ __forceinline__ int64_t tq_cache_length(const int64_t* word) {
+    const int64_t v = *reinterpret_cast<const volatile int64_t*>(word);
+    return v < 0 ? 0 : v & ((1ll << kLengthBits) - 1);
+}
 struct TqRowMap {
     int64_t tokens, capacity;
     const int64_t* length;

@@ -128,9 +128,8 @@ decode_partial_kernel(TqDev kp, DecodeArgs a) {
     const int t = lane & 3, r = lane >> 2;      // position in the quad, row of the fragments
     int64_t n = a.keys_per_group;
     if (a.length) {
-        const int64_t len = *a.length;
+        const int64_t len = tq_cache_length(a.length);      // (an append on another stream may be at work on the word)
         n = len < n ? len : n;
-        if (n < 0) n = 0;
     }
     const uint32_t keys = (uint32_t)n;           // rows of all groups together stay below 2^32
     const uint32_t tiles_total = (uint32_t)((n + kTile - 1) / kTile), tps = (tiles_total + a.splits - 1) / a.splits;

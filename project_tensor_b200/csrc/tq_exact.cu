@@ -211,7 +211,7 @@ struct RowSource {
     bool listed, mapped;
     __device__ __forceinline__ void open(const RowsJob& job, bool first_block) {
         mapped = job.map.tokens > 0;
-        len0 = !mapped ? 0 : !job.map.length ? job.map.base : (*reinterpret_cast<volatile const int64_t*>(job.map.length) & ((1ll << 40) - 1));
+        len0 = !mapped ? 0 : !job.map.length ? job.map.base : tq_cache_length(job.map.length);
         const TqRecheckHeader* hdr = job.lists.hdr;
         // all rows, or the rows of the list (every row again if a list overflowed)
         listed = hdr != nullptr && hdr->overflow == 0;
@@ -229,8 +229,9 @@ struct RowSource {
     }
 };
 
-// The last block of a launch to get here raises the cache length.  Blocks count themselves in bits 40 and up of that very
-// word, which are zero again when the kernel ends, so a step needs neither a second launch nor a counter of its own.
+// The last block of a launch to get here raises the cache length.  Blocks count themselves in the upper bits of that very
+// word, which are zero again when the kernel ends, so a step needs neither a second launch nor a counter of its own; readers
+// on other streams mask them off (tq_cache_length) and see the old length or the new one.
 // (Every block has read the length before it counts itself.)  advance == 2: nothing in the launch reads it; one block adds.
 __device__ __forceinline__ void advance_length(const RowsJob& job, int64_t len0, int advance) {
     if (advance == 2) {
@@ -238,8 +239,8 @@ __device__ __forceinline__ void advance_length(const RowsJob& job, int64_t len0,
         return;
     }
     unsigned long long* len = reinterpret_cast<unsigned long long*>(const_cast<int64_t*>(job.map.length));
-    const unsigned long long before = atomicAdd(len, 1ull << 40);
-    if ((before >> 40) == gridDim.x - 1) {
+    const unsigned long long before = atomicAdd(len, 1ull << kLengthBits);
+    if ((before >> kLengthBits) == gridDim.x - 1) {
         const int64_t v = len0 + job.map.tokens;
         atomicExch(len, (unsigned long long)(v < job.map.capacity ? v : job.map.capacity));
     }

@@ -50,3 +50,20 @@ def test_tile_and_block_edges(qpg):
 def test_value_norms_far_apart(grow):
     _check(128, 4, 4, 4, (700, 5000), grow)
     _check(64, 3, 2, 6, (700,), grow)
+
+
+@pytest.mark.parametrize("d", [64, 128])
+def test_length_word_of_an_append_at_work(d):
+    """While an append runs on another stream, the bits above the length count its blocks: they are not part of the length."""
+    import torch
+    groups, n, cap = 2, 300, 512
+    cache = PackedKVCache(tg.TurboQuantProd(d, 4, seed=2026), tg.TurboQuantMSE(d, 4, seed=77), groups, cap)
+    cache.append(_randn((groups, n, d), 6), _randn((groups, n, d), 7))
+    queries = _randn((groups, 3, d), 5)
+    want = cache.attend(queries)
+    cache.keys.length_device += 37 << 40
+    assert cache.sync_length() == n
+    for got in (cache.attend(queries), cache.attend(queries, use_device_length=True)):
+        assert float((got - want).abs().max()) <= 1e-5 * float(want.abs().max())
+    cache.keys.length_device.fill_(-1)
+    assert not bool(cache.attend(queries, use_device_length=True).any())
