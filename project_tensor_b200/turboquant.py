@@ -368,10 +368,15 @@ TurboQuantProdEncoding.residual_norms = _lazy_field(
     "residual_norms", lambda pk: _deliver(pk.residual_norms, pk.kind, pk.plans))
 
 
-def _check_rows(out, values: int, prefix) -> None:
-    """A result allocated in the shape of ``prefix_shape`` has to hold the encoding's rows (the field can be edited)."""
-    if out.numel() != values:
-        raise ValueError(f"prefix_shape {tuple(prefix)} does not match the rows of the encoding")
+def _row_shape(rows: int, prefix) -> Tuple[int, ...]:
+    """Shape to allocate the results of ``rows`` rows in: ``prefix`` when it holds them as it stands, else flat -- the field
+    ``prefix_shape`` can be edited, and ``reshape`` then says what it makes of it (a -1 in it, or no such shape)."""
+    prefix = tuple(prefix)
+    return prefix if math.prod(prefix) == rows and min(prefix, default=0) >= 0 else (rows,)
+
+
+def _in_shape(result, shape):
+    return result if tuple(result.shape) == shape else result.reshape(shape)
 
 
 def _encoding_from_packed(cls, pk: _Packed, prefix):
@@ -609,11 +614,10 @@ class TurboQuantMSE:
 
     def dequantize(self, encoding: TurboQuantMSEEncoding):
         pk = _as_packed(encoding, self._plans, need_signs=False)
-        out = pk.norms.new_empty(tuple(encoding.prefix_shape) + (self.dimension,))
-        _check_rows(out, pk.n * self.dimension, encoding.prefix_shape)
+        out = pk.norms.new_empty(_row_shape(pk.n, encoding.prefix_shape) + (self.dimension,))
         _native.check(_native.load().tq_mse_dequantize(self._plans.handle(pk.device), pk.codes.data_ptr(),
                                                        pk.norms.data_ptr(), pk.n, out.data_ptr(), _stream_ptr(pk.device)))
-        return _deliver(out, pk.kind, pk.plans)
+        return _in_shape(_deliver(out, pk.kind, pk.plans), tuple(encoding.prefix_shape) + (self.dimension,))
 
 
 class TurboQuantProd:
@@ -651,12 +655,11 @@ class TurboQuantProd:
 
     def dequantize(self, encoding: TurboQuantProdEncoding):
         pk = _as_packed(encoding, self._plans, need_signs=True)
-        out = pk.norms.new_empty(tuple(encoding.prefix_shape) + (self.dimension,))
-        _check_rows(out, pk.n * self.dimension, encoding.prefix_shape)
+        out = pk.norms.new_empty(_row_shape(pk.n, encoding.prefix_shape) + (self.dimension,))
         _native.check(_native.load().tq_prod_dequantize(
             self._plans.handle(pk.device), pk.codes.data_ptr(), pk.signs.data_ptr(), pk.residual_norms.data_ptr(),
             pk.norms.data_ptr(), pk.n, out.data_ptr(), _stream_ptr(pk.device)))
-        return _deliver(out, pk.kind, pk.plans)
+        return _in_shape(_deliver(out, pk.kind, pk.plans), tuple(encoding.prefix_shape) + (self.dimension,))
 
     def attention_score(self, query: Any, encoding: TurboQuantProdEncoding):
         """One query row broadcast over all keys, or one query row per key (_quant.py:334-358)."""
@@ -675,8 +678,8 @@ class TurboQuantProd:
         lib = _native.load()
         # a short row of scores for a NumPy caller is written straight to page-locked memory
         to_host = staged.kind == "numpy" and 4 * num_codes <= _MAPPED_BYTES
-        scores = _torch().empty(q_prefix, dtype=_torch().float32, device="cpu", pin_memory=True) if to_host else pk.norms.new_empty(q_prefix)
-        _check_rows(scores, num_codes, q_prefix)
+        rows = _row_shape(num_codes, q_prefix)
+        scores = _torch().empty(rows, dtype=_torch().float32, device="cpu", pin_memory=True) if to_host else pk.norms.new_empty(rows)
         handle = self._plans.handle(pk.device)
         st = _stream_ptr(pk.device)
         if broadcast and self._plans._path == _native.TQ_PATH_AUTO:
@@ -697,8 +700,8 @@ class TurboQuantProd:
                                                 scores.data_ptr(), st))
         if to_host:
             self._plans.check_status(pk.device)      # waits for the stream
-            return scores.clone().numpy()
-        return _deliver(scores, staged.kind, self._plans)
+            return _in_shape(scores.clone().numpy(), q_prefix)
+        return _in_shape(_deliver(scores, staged.kind, self._plans), q_prefix)
 
     def attention_scores(self, queries: Any, encoding: TurboQuantProdEncoding, *, topk: Optional[int] = None,
                          groups: int = 1, return_matrix: Optional[bool] = None, index_base: int = 0,
