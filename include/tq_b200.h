@@ -285,7 +285,8 @@ int tq_pack_signs(const tq_plan* plan, const int8_t* qjl, int64_t n, void* signs
 /*
  * Counters of the last tq_*_quantize call on this plan, read back from the device (synchronises
  * `stream`): rows the tensor-core kernel handed to the exact kernel because a coordinate fell
- * within the guard band of a decision boundary.  Diagnostic only.
+ * within the guard band of a decision boundary; all rows of a batch so small that the exact kernel alone
+ * is the faster one.  Diagnostic only.
  */
 int tq_plan_last_recheck_rows(const tq_plan* plan, void* stream, int64_t* rows);
 

@@ -358,7 +358,9 @@ static int quantize_common(const tq_plan* p, bool prod, const float* x, int64_t 
         return rc;
     }
     if (err != TQ_OK) return err;
-    return tq_launch_exact_quantize(p, prod, x, TQ_F32, n, out.codes, out.signs, rnorms, norms, st);
+    // (a plan with tensor-core kernels counts the rows of this kernel, all of them here)
+    return tq_launch_exact_quantize(p, prod, x, TQ_F32, n, out.codes, out.signs, rnorms, norms,
+                                    p->path == TQ_PATH_AUTO && p->tensor_ok ? p->counters : nullptr, st);
 }
 
 int tq_mse_quantize(const tq_plan* p, const float* x, int64_t n, void* codes, float* norms, void* scratch,

@@ -184,7 +184,7 @@ __device__ __forceinline__ void tq_grid_release() { asm volatile("griddepcontrol
 // ---- launchers implemented in the kernel files -----------------------------------------------
 // Exact (reference-order float32) kernels.
 int tq_launch_exact_quantize(const tq_plan* p, bool prod, const void* x, int xtype, int64_t n, uint32_t* codes,
-                             uint32_t* signs, float* rnorms, float* norms, cudaStream_t st);
+                             uint32_t* signs, float* rnorms, float* norms, unsigned long long* redo_counter, cudaStream_t st);
 int tq_launch_append(const tq_plan* kp, const void* kx, uint32_t* kcodes, uint32_t* ksigns, float* krnorms, float* knorms,
                      const tq_plan* vp, const void* vx, uint32_t* vcodes, float* vnorms, int xtype, int64_t rows,
                      const TqRowMap& map, int advance, cudaStream_t st);

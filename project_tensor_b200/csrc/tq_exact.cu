@@ -216,7 +216,7 @@ struct RowSource {
         // all rows, or the rows of the list (every row again if a list overflowed)
         listed = hdr != nullptr && hdr->overflow == 0;
         limit = listed ? (int64_t)min(hdr->n_rows, job.lists.row_cap) : job.n;
-        if (hdr != nullptr && job.redo_counter && first_block && threadIdx.x == 0) *job.redo_counter = (unsigned long long)limit;
+        if (job.redo_counter && first_block && threadIdx.x == 0) *job.redo_counter = (unsigned long long)limit;
     }
     __device__ __forceinline__ int64_t src(const RowsJob& job, int64_t idx) const {
         int64_t row = idx < limit ? (listed ? (int64_t)job.lists.row_entries[idx] : idx) : -1;
@@ -963,10 +963,10 @@ RowsJob rows_job(const tq_plan* p, bool prod, const void* x, int xtype, int64_t 
 }  // namespace
 
 int tq_launch_exact_quantize(const tq_plan* p, bool prod, const void* x, int xtype, int64_t n, uint32_t* codes,
-                             uint32_t* signs, float* rnorms, float* norms, cudaStream_t st) {
+                             uint32_t* signs, float* rnorms, float* norms, unsigned long long* redo_counter, cudaStream_t st) {
     TqRange range("tq.quantize.exact_rows");
     if (n == 0) return TQ_OK;
-    const RowsJob job = rows_job(p, prod, x, xtype, n, codes, signs, rnorms, norms, nullptr, nullptr, nullptr);
+    const RowsJob job = rows_job(p, prod, x, xtype, n, codes, signs, rnorms, norms, nullptr, redo_counter, nullptr);
     return launch_rows(job, nullptr, n, p->device, 0, st);
 }
 

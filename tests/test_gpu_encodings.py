@@ -1,9 +1,12 @@
-"""Encodings whose ``prefix_shape`` was edited."""
+"""What a call leaves behind besides its result: encodings whose ``prefix_shape`` was edited, the counter of rows done in the reference's
+order."""
+import ctypes
 
 import numpy as np
 import pytest
 
 import project_tensor_b200 as tg
+from project_tensor_b200 import _native
 
 pytestmark = pytest.mark.gpu
 
@@ -28,3 +31,12 @@ def test_edited_prefix_shape(lib_built, kind):
             enc.prefix_shape = prefix
             with pytest.raises((ValueError, RuntimeError)):
                 quant.dequantize(enc)
+
+
+def test_rows_done_in_reference_order_are_those_of_the_last_call(lib_built):
+    import torch
+    prod, rows, dev = tg.TurboQuantProd(128, 4, seed=5), ctypes.c_int64(-1), torch.device("cuda", 0)
+    for n in (200_000, 300, 5):
+        prod.quantize(torch.randn(n, 128, device=dev, generator=torch.Generator(dev).manual_seed(n)))
+        _native.check(_native.load().tq_plan_last_recheck_rows(prod._plans.handle(dev), torch.cuda.current_stream().cuda_stream, ctypes.byref(rows)))
+        assert rows.value == n if n < 1000 else 0 < rows.value < n // 50
