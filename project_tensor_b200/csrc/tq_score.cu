@@ -334,7 +334,8 @@ score_matrix_kernel(TqDev p, const float* __restrict__ q, int qpg, const uint32_
 // shared buffer that is cut back to the k best by radix select whenever it fills; one final sort.
 __global__ void __launch_bounds__(256)
 merge_keys_kernel(const unsigned long long* __restrict__ part, int lists, int qpg, int topk, int k2,
-                  int64_t idx_base, float* __restrict__ top_scores, int64_t* __restrict__ top_idx) {
+                  int64_t idx_base, float* __restrict__ top_scores, int64_t* __restrict__ top_idx, const unsigned int* run_if) {
+    if (run_if && *run_if == 0u) return;
     __shared__ __align__(16) unsigned long long a[kSelCap];
     __shared__ int hist[256];
     __shared__ int scratch[4];
@@ -528,10 +529,9 @@ int64_t tq_score_topk_scratch(const tq_plan* p, int groups, int qpg, int64_t key
 }
 
 int tq_merge_keys_launch(const unsigned long long* part, int lists, int qpg, int groups, int topk, int64_t idx_base,
-                         float* top_scores, int64_t* top_idx, cudaStream_t st) {
+                         float* top_scores, int64_t* top_idx, cudaStream_t st, const unsigned int* run_if) {
     const int k2 = pow2_at_least(topk);
-    merge_keys_kernel<<<dim3(qpg, groups), 256, 0, st>>>(part, lists, qpg, topk, k2,
-                                                                                           idx_base, top_scores, top_idx); tq_count_launch();
+    merge_keys_kernel<<<dim3(qpg, groups), 256, 0, st>>>(part, lists, qpg, topk, k2, idx_base, top_scores, top_idx, run_if); tq_count_launch();
     TQ_CUDA_TRY(cudaGetLastError());
     return TQ_OK;
 }
@@ -574,7 +574,7 @@ int tq_launch_score_general(const tq_plan* p, const float* q, int groups, int qp
             const size_t cnt = (size_t)groups * qpg * topk;
             TQ_CUDA_TRY(cudaMemsetAsync(scratch, 0, cnt * sizeof(unsigned long long), st));
             merge_keys_kernel<<<dim3(qpg, groups), 256, 0, st>>>(
-                static_cast<unsigned long long*>(scratch), 1, qpg, topk, pow2_at_least(topk), idx_base, top_scores, top_idx); tq_count_launch();
+                static_cast<unsigned long long*>(scratch), 1, qpg, topk, pow2_at_least(topk), idx_base, top_scores, top_idx, nullptr); tq_count_launch();
             TQ_CUDA_TRY(cudaGetLastError());
         }
         return TQ_OK;
@@ -598,7 +598,7 @@ int tq_launch_score_general(const tq_plan* p, const float* q, int groups, int qp
     if (topk > 0) {
         const int k2 = pow2_at_least(topk);
         merge_keys_kernel<<<dim3(qpg, groups), 256, 0, st>>>(
-            static_cast<unsigned long long*>(scratch), s.nblk, qpg, topk, k2, idx_base, top_scores, top_idx); tq_count_launch();
+            static_cast<unsigned long long*>(scratch), s.nblk, qpg, topk, k2, idx_base, top_scores, top_idx, nullptr); tq_count_launch();
         TQ_CUDA_TRY(cudaGetLastError());
     }
     return TQ_OK;

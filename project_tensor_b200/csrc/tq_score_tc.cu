@@ -782,7 +782,8 @@ score_prep256_kernel(TqDev p, const float* __restrict__ q, int qpg, int q0, int 
 __global__ void __launch_bounds__(kSelThreads)
 topk_rows_kernel(const float* __restrict__ scores, int64_t row_stride, int64_t group_stride, int qpg, int64_t n,
                  int64_t seg_len, int64_t first_row_of_group_stride, int64_t key_off, int topk, int k2,
-                 int lists_per_group, int list_base, unsigned long long* __restrict__ part) {
+                 int lists_per_group, int list_base, unsigned long long* __restrict__ part, const unsigned int* run_if) {
+    if (run_if && *run_if == 0u) return;
     __shared__ __align__(16) unsigned long long buf[kSelCap];
     __shared__ int hist[256];
     __shared__ int scratch[4];
@@ -1048,38 +1049,67 @@ static bool use_filter(const tq_plan* p, const float* scores, int groups, int qp
     return scores == nullptr && topk > 0 && groups == 1 && p->beta_scale > 0.f && keys_per_group >= (qpg >= 32 ? kFilterFromMany : kFilterFrom) &&
            keys_per_group < (int64_t)1 << 31 && (int64_t)nq * topk * 6 <= kFilterRoom;
 }
+// The procedure that a filtered search falls back to takes the same passes of queries, one after the other, and works in the
+// memory that the pass's lists, scores and gathered keys have left: the whole is no larger than one pass of that procedure (64 queries x
+// 1,048,576 keys 0.27 GB, from 4,194,304 keys on 1.07 GB, whatever the number of queries), or about 25 MB for a handful of
+// queries.  (What a call asks for is still what the unfiltered path would take, which a plan can be switched to.)
 struct FilterPlan {
-    size_t off_prep, off_bad, off_rows, off_offsets, off_codes, off_signs, off_norms, off_rnorms, off_grows, off_scores, total;
+    int pass;                    // queries of the largest pass
+    int64_t stride0, first;      // tiles between the sampled ones; keys of the sample, a multiple of 128
+    bool matrix;                 // the fallback scores into a matrix (else candidate mode)
+    int64_t segs;
+    size_t off_thr, off_cnt, off_best, off_prep, off_words;
+    size_t off_sample, off_rows, off_offsets, off_codes, off_signs, off_norms, off_rnorms, off_grows, off_scores;
+    size_t off_matrix, off_part, off_cand, total;
 };
-static FilterPlan plan_filter(const tq_plan* p, size_t behind) {
+static FilterPlan plan_filter(const tq_plan* p, int qpg, int64_t keys, int topk) {
     FilterPlan f{};
-    size_t at = behind;
-    auto take = [&](size_t bytes) { const size_t o = at; at += (bytes + 255) & ~size_t(255); return o; };
+    auto pad = [](size_t bytes) { return (bytes + 255) & ~size_t(255); };
+    const int most = p->dev.d == 256 ? 32 : TQ_SCORE_PASS;
+    f.pass = qpg < most ? qpg : most;
+    const int64_t tiles = (keys + kTileKeys - 1) / kTileKeys;
+    f.stride0 = (tiles + kFilterSample / kTileKeys - 1) / (kFilterSample / kTileKeys);
+    f.first = (tiles + f.stride0 - 1) / f.stride0 * kTileKeys;
+    f.matrix = keys <= 2 * kCandChunk;
+    f.segs = (keys + kSegLen - 1) / kSegLen;
+    size_t at = pad(kPrepGroupMax);      // the prepared queries come first in every layout
+    auto take = [&](size_t bytes) { const size_t o = at; at += pad(bytes); return o; };
+    f.off_thr = take((size_t)qpg * 4);
+    f.off_cnt = take((size_t)qpg * 4);
+    f.off_best = take((size_t)qpg * topk * 8);
     f.off_prep = take(tq_filter_prep_bytes(p->dev.d, 64));
-    f.off_bad = take(256);
+    f.off_words = take(256);
+    const size_t shared = at;
+    f.off_sample = take((size_t)f.pass * f.first * 8);
     f.off_offsets = take(64 * 4);
-    f.off_rows = take((size_t)64 * kFilterRoom * 4);
+    f.off_rows = take((size_t)f.pass * kFilterRoom * 4);
     f.off_codes = take((size_t)kFilterRoom * p->dev.code_words * 4);
     f.off_signs = take((size_t)kFilterRoom * p->dev.sign_words * 4);
     f.off_norms = take((size_t)kFilterRoom * 4);
     f.off_rnorms = take((size_t)kFilterRoom * 4);
     f.off_grows = take((size_t)kFilterRoom * 4);
-    f.off_scores = take((size_t)64 * kFilterRoom * 4);
+    f.off_scores = take((size_t)f.pass * kFilterRoom * 4);
     f.total = at;
+    at = shared;                          // the fallback, in the same place
+    if (f.matrix) {
+        f.off_matrix = take((size_t)f.pass * keys * 4);
+        f.off_part = take((size_t)f.segs * f.pass * topk * 8);
+    } else {
+        f.off_cand = take((size_t)f.pass * kCandChunk * 8);
+    }
+    if (at > f.total) f.total = at;
     return f;
 }
 
 int64_t tq_score_tc_scratch(const tq_plan* p, int groups, int qpg, int64_t keys_per_group, int topk) {
-    if (use_filter(p, nullptr, groups, qpg, topk, keys_per_group))       // also holds a call that wants the matrix besides
-        return (int64_t)std::max(plan_filter(p, plan_candidates(groups, qpg, keys_per_group, topk).total).total,
-                                 plan_score(groups, qpg, keys_per_group, topk, true).total);
     const size_t a = plan_score(groups, qpg, keys_per_group, topk, true).total;
     const size_t b = use_candidates(nullptr, topk, keys_per_group) ? plan_candidates(groups, qpg, keys_per_group, topk).total : 0;
-    return (int64_t)(a > b ? a : b);
+    const size_t c = use_filter(p, nullptr, groups, qpg, topk, keys_per_group) ? plan_filter(p, qpg, keys_per_group, topk).total : 0;
+    return (int64_t)std::max(std::max(a, b), c);
 }
 
 int tq_merge_keys_launch(const unsigned long long* part, int lists, int qpg, int groups, int topk, int64_t idx_base,
-                         float* top_scores, int64_t* top_idx, cudaStream_t st);
+                         float* top_scores, int64_t* top_idx, cudaStream_t st, const unsigned int* run_if = nullptr);
 
 int tq_launch_score_tc(const tq_plan* p, const float* q, int groups, int qpg, const uint32_t* codes,
                        const uint32_t* signs, const float* rnorms, const float* norms, int64_t keys_per_group,
@@ -1088,21 +1118,23 @@ int tq_launch_score_tc(const tq_plan* p, const float* q, int groups, int qpg, co
     TqRange range("tq.score.tensor_core");
     if (group_rows <= 0) group_rows = keys_per_group;
     const bool filter = p->path == TQ_PATH_AUTO && use_filter(p, scores, groups, qpg, topk, keys_per_group);
-    const bool candidates = filter || use_candidates(scores, topk, keys_per_group);
+    const bool candidates = !filter && use_candidates(scores, topk, keys_per_group);
     const ScoreTcPlan sp = plan_score(groups, qpg, keys_per_group, topk, scores == nullptr);
     const CandPlan cp = plan_candidates(groups, qpg, keys_per_group, topk);
-    const FilterPlan fp = filter ? plan_filter(p, cp.total) : FilterPlan{};
+    const FilterPlan fp = filter ? plan_filter(p, qpg, keys_per_group, topk) : FilterPlan{};
     const size_t need = filter ? fp.total : candidates ? cp.total : sp.total;
     if (!scratch || scratch_bytes < need)
         return tq_fail(TQ_ERR_SCRATCH_TOO_SMALL, "score scratch: need %zu bytes, got %zu", need, scratch_bytes);
     unsigned char* sc = static_cast<unsigned char*>(scratch);
-    unsigned char* prep = sc;     // both layouts start with the prepared queries
+    unsigned char* prep = sc;     // every layout starts with the prepared queries
     const int sms = tq_sm_count(p->device);
     const int bits = p->dev.bits;
-    float* thr = reinterpret_cast<float*>(sc + cp.off_thr);
-    unsigned int* cnt = reinterpret_cast<unsigned int*>(sc + cp.off_cnt);
-    unsigned long long* best = reinterpret_cast<unsigned long long*>(sc + cp.off_best);
-    unsigned long long* cand = reinterpret_cast<unsigned long long*>(sc + cp.off_cand);
+    float* thr = reinterpret_cast<float*>(sc + (filter ? fp.off_thr : cp.off_thr));
+    unsigned int* cnt = reinterpret_cast<unsigned int*>(sc + (filter ? fp.off_cnt : cp.off_cnt));
+    unsigned long long* best = reinterpret_cast<unsigned long long*>(sc + (filter ? fp.off_best : cp.off_best));
+    // candidate lists: of every query, or (filtered search) of the queries of the pass at work
+    struct Lists { unsigned long long* at; int64_t cap; };
+    const Lists all_lists{reinterpret_cast<unsigned long long*>(sc + cp.off_cand), cp.cand_cap};
 
     // Which keys a launch scores: the caller's, or those gathered by a filtered search.
     struct Keys { const uint32_t *codes, *signs; const float *rnorms, *norms; int64_t group_rows; const unsigned int* dyn_keys; };
@@ -1123,7 +1155,7 @@ int tq_launch_score_tc(const tq_plan* p, const float* q, int groups, int qpg, co
     // One scoring launch for the prepared queries [q0, q0 + nq) over keys [key_off, key_off + key_cnt) of every group (every
     // tile_stride-th tile of them), into a matrix (mat != null) or into the candidate lists.
     auto score_pass = [&](const Keys& keys, int q0, int nq, int64_t key_off, int64_t key_cnt, int tile_stride, float* mat,
-                          int64_t row_stride, const unsigned int* run_if) -> int {
+                          int64_t row_stride, const Lists& lists, const unsigned int* run_if) -> int {
         const int qpad = pad_of(nq);
         const int64_t group_stride = (int64_t)qpg * row_stride;
         ScoreTcArgs a{};
@@ -1142,7 +1174,7 @@ int tq_launch_score_tc(const tq_plan* p, const float* q, int groups, int qpg, co
         a.norms_bulk = (groups == 1 || keys.group_rows % 4 == 0) && key_off % 4 == 0 ? 1 : 0;   // 16-byte aligned tile starts
         a.fused = mat ? 0 : (tile_stride > 1 ? 2 : 1);    // 2: the sampled pass
         a.qpg_total = qpg; a.q0 = q0;
-        a.thr = thr; a.cnt = cnt; a.cand = cand; a.cand_cap = cp.cand_cap;
+        a.thr = thr; a.cnt = cnt; a.cand = lists.at; a.cand_cap = lists.cap;
         a.status = p->status_dev;
         a.wait_kcycles = p->wait_kcycles;
         if (a.total_tiles == 0) return TQ_OK;
@@ -1183,21 +1215,20 @@ case B:                                                                         
     // against 205 us in passes of 32 and 16).
     // `prepared`: the scratch block still holds the prepared queries of the only pass (a call of several launches
     // over the same queries prepares them once).
-    auto score_passes = [&](int64_t key_off, int64_t key_cnt, int tile_stride, float* mat, int64_t row_stride, bool prepared,
-                            const unsigned int* run_if = nullptr) -> int {
+    auto score_passes = [&](int64_t key_off, int64_t key_cnt, int tile_stride, float* mat, int64_t row_stride, bool prepared) -> int {
         for (int q0 = 0; q0 < qpg; q0 += pass) {
             const int nq = qpg - q0 < pass ? qpg - q0 : pass;
             if (!(prepared && qpg <= pass)) {
                 const int rc = prepare_pass(q0, nq);
                 if (rc != TQ_OK) return rc;
             }
-            const int rc = score_pass(all_keys, q0, nq, key_off, key_cnt, tile_stride, mat, row_stride, run_if);
+            const int rc = score_pass(all_keys, q0, nq, key_off, key_cnt, tile_stride, mat, row_stride, all_lists, nullptr);
             if (rc != TQ_OK) return rc;
         }
         return TQ_OK;
     };
 
-    if (!candidates) {
+    if (!candidates && !filter) {
         // A score matrix exists: the caller's (everything scored in one go) or, when only the top-k is wanted, a scratch
         // matrix per chunk of keys; the top-k is selected from it segment by segment and the lists are merged at the end.
         unsigned long long* part = reinterpret_cast<unsigned long long*>(sc + sp.off_part);
@@ -1217,7 +1248,7 @@ case B:                                                                         
                 // lists of chunk c occupy slots [c*segs_per_chunk, ...); unused slots stay zero (= empty)
                 topk_rows_kernel<<<dim3((unsigned)segs, (unsigned)(groups * qpg)), kSelThreads, 0, st>>>(
                     mat, row_stride, (int64_t)qpg * row_stride, qpg, key_cnt, kSegLen, group_rows, key_off, topk, pow2_at_least(topk),
-                    (int)sp.lists_per_group, (int)(c * sp.segs_per_chunk), part); tq_count_launch();
+                    (int)sp.lists_per_group, (int)(c * sp.segs_per_chunk), part, nullptr); tq_count_launch();
                 TQ_CUDA_TRY(cudaGetLastError());
             }
         }
@@ -1233,51 +1264,60 @@ case B:                                                                         
     // k-th best of a subset is a lower bound of the k-th best of the whole, so the full pass that follows loses nothing
     // and appends only about 64 k scores per query.
     const int k2 = pow2_at_least(topk);
-    const int64_t cells = cp.lists * topk;
     const int64_t tiles0 = (std::min(cp.chunk, keys_per_group) + kTileKeys - 1) / kTileKeys;
     const int64_t sample_tiles = (tiles0 + kSampleEvery - 1) / kSampleEvery;
-    auto init = [&](int64_t first_count, const unsigned int* run_if) -> int {
-        init_candidates_kernel<<<(unsigned)((cells + 255) / 256), 256, 0, st>>>(thr, cnt, best, cp.lists, topk, (unsigned int)first_count, run_if);
+    // (of the queries from q0 on, `queries` per group)
+    auto init = [&](int q0, int64_t queries, int64_t first_count, const unsigned int* run_if) -> int {
+        init_candidates_kernel<<<(unsigned)((queries * topk + 255) / 256), 256, 0, st>>>(thr + q0, cnt + q0, best + (int64_t)q0 * topk, queries, topk,
+                                                                                         (unsigned int)first_count, run_if);
         tq_count_launch();
         TQ_CUDA_TRY(cudaGetLastError());
         return TQ_OK;
     };
-    auto select = [&](int mode, const unsigned int* run_if) -> int {
-        select_candidates_kernel<<<dim3((unsigned)qpg, (unsigned)groups), 256, 0, st>>>(cand, cnt, cp.cand_cap, best, thr, qpg, topk, k2, mode, run_if);
+    auto select = [&](const Lists& lists, int q0, int queries, int mode, const unsigned int* run_if) -> int {
+        select_candidates_kernel<<<dim3((unsigned)queries, (unsigned)groups), 256, 0, st>>>(lists.at + q0 * lists.cap, cnt + q0, lists.cap, best + (int64_t)q0 * topk,
+                                                                                            thr + q0, queries, topk, k2, mode, run_if);
         tq_count_launch();
         TQ_CUDA_TRY(cudaGetLastError());
         return TQ_OK;
     };
-    auto run_candidates = [&](const unsigned int* run_if) -> int {
-        TQ_STEP(init(sample_tiles * kTileKeys, run_if));
+    // `score`: one scoring launch or several over keys [key_off, key_off + key_cnt), every tile_stride-th tile of them, into the lists
+    auto run_candidates = [&](const Lists& lists, int q0, int queries, const unsigned int* run_if, auto score) -> int {
+        TQ_STEP(init(q0, (int64_t)groups * queries, sample_tiles * kTileKeys, run_if));
         for (int64_t c = 0; c < cp.nchunks; ++c) {
             const int64_t key_off = c * cp.chunk;
             int64_t key_cnt = keys_per_group - key_off;
             if (key_cnt > cp.chunk) key_cnt = cp.chunk;
             if (c == 0) {
-                TQ_STEP(score_passes(key_off, key_cnt, (int)kSampleEvery, nullptr, 0, run_if != nullptr, run_if));
-                TQ_STEP(select(1, run_if));
+                TQ_STEP(score(key_off, key_cnt, (int)kSampleEvery));
+                TQ_STEP(select(lists, q0, queries, 1, run_if));
             }
-            TQ_STEP(score_passes(key_off, key_cnt, 1, nullptr, 0, true, run_if));
-            TQ_STEP(select(0, run_if));
+            TQ_STEP(score(key_off, key_cnt, 1));
+            TQ_STEP(select(lists, q0, queries, 0, run_if));
         }
         return TQ_OK;
     };
     if (!filter) {
-        TQ_STEP(run_candidates(nullptr));
+        bool prepared = false;
+        TQ_STEP(run_candidates(all_lists, 0, qpg, nullptr, [&](int64_t key_off, int64_t key_cnt, int stride) {
+            const int rc = score_passes(key_off, key_cnt, stride, nullptr, 0, prepared);
+            prepared = true;
+            return rc;
+        }));
         return tq_merge_keys_launch(best, 1, qpg, groups, topk, idx_base, top_scores, top_idx, st);
     }
 
-    // Filtered search over one group.  A sample of the keys, spread over all of them, is scored in full and gives every query a
-    // first threshold; each round lists the keys of a larger sample (the last round: all keys) whose single-fp16 score plus
-    // bound reaches the threshold, gathers them, scores them in full and raises the thresholds; the last round's selection is
-    // the result.  With the sizes of the samples a geometric series, every round lists about ratio * topk keys per query.
-    // Data that lists more than a round has room for (long runs of equal scores, say) sets a flag on the device, upon which
-    // the rest of the rounds does nothing and the unfiltered procedure behind them, else skipped, does the work.
+    // Filtered search over one group, a pass of queries at a time.  A sample of the keys, spread over all of them, is scored in full
+    // and gives every query a first threshold; each round lists the keys of a larger sample (the last round: all keys) whose
+    // single-fp16 score plus bound reaches the threshold, gathers them, scores them in full and raises the thresholds; the last
+    // round's selection is the result.  With the sizes of the samples a geometric series, every round lists about ratio * topk keys
+    // per query.  Data that lists more than a round has room for (long runs of equal scores, say), and queries that the bound
+    // does not cover, set a flag on the device, upon which the rest of the rounds does nothing and the unfiltered procedure for
+    // this many keys, else skipped, does the pass.
     TqFilterPass f{};
     f.cap = kFilterRoom; f.room = kFilterRoom; f.beta_scale = p->beta_scale;
     f.fprep = sc + fp.off_prep;
-    f.bad = reinterpret_cast<unsigned int*>(sc + fp.off_bad);
+    f.bad = reinterpret_cast<unsigned int*>(sc + fp.off_words);
     f.gathered = f.bad + 1;
     f.rows = reinterpret_cast<unsigned int*>(sc + fp.off_rows);
     f.offsets = reinterpret_cast<unsigned int*>(sc + fp.off_offsets);
@@ -1289,39 +1329,49 @@ case B:                                                                         
     f.scores = reinterpret_cast<float*>(sc + fp.off_scores);
     const Keys gathered{f.g_codes, f.g_signs, f.g_rnorms, f.g_norms, kFilterRoom, f.gathered};
     const int64_t tiles = (keys_per_group + kTileKeys - 1) / kTileKeys;
-    const int stride0 = (int)((tiles + kFilterSample / kTileKeys - 1) / (kFilterSample / kTileKeys));
-    const int64_t first = (tiles + stride0 - 1) / stride0 * kTileKeys;
-    TQ_CUDA_TRY(cudaMemsetAsync(f.bad, 0, 2 * sizeof(unsigned int), st));
-    TQ_STEP(init(first, nullptr));
+    const int stride0 = (int)fp.stride0;
     for (int q0 = 0; q0 < qpg; q0 += pass) {
         const int nq = qpg - q0 < pass ? qpg - q0 : pass;
+        // (rows of the pass's own arrays, addressed as the scoring kernel does: by the number of the query in the call)
+        const Lists sample{reinterpret_cast<unsigned long long*>(sc + fp.off_sample) - q0 * fp.first, fp.first};
         f.nq = nq; f.qpad = pad_of(nq);
         f.thr = thr + q0; f.cnt = cnt + q0; f.best = best + (int64_t)q0 * topk;
+        TQ_CUDA_TRY(cudaMemsetAsync(f.bad, 0, 2 * sizeof(unsigned int), st));
+        TQ_STEP(init(q0, nq, fp.first, nullptr));
         TQ_STEP(prepare_pass(q0, nq));
-        TQ_STEP(score_pass(all_keys, q0, nq, 0, keys_per_group, stride0, nullptr, 0, nullptr));
+        TQ_STEP(score_pass(all_keys, q0, nq, 0, keys_per_group, stride0, nullptr, 0, sample, nullptr));
         TQ_STEP(tq_launch_filter_prep(p, prep, f.qpad, nq, p->c_max, p->beta_scale, f.fprep, f.bad, st));
-    }
-    TQ_STEP(tq_launch_sample_threshold(cand, cp.cand_cap, cnt, thr, qpg, topk, st));
-    for (int q0 = 0; q0 < qpg; q0 += pass) {
-        const int nq = qpg - q0 < pass ? qpg - q0 : pass;
-        f.nq = nq; f.qpad = pad_of(nq);
-        f.thr = thr + q0; f.cnt = cnt + q0; f.best = best + (int64_t)q0 * topk;
-        if (qpg > pass) {
-            TQ_STEP(prepare_pass(q0, nq));
-            TQ_STEP(tq_launch_filter_prep(p, prep, f.qpad, nq, p->c_max, p->beta_scale, f.fprep, f.bad, st));
-        }
+        TQ_STEP(tq_launch_sample_threshold(sample.at + q0 * fp.first, fp.first, f.cnt, f.thr, nq, topk, st));
         // rounds: the fewest whose ratio keeps the lists of all queries within two thirds of the room
-        const double span = (double)tiles / (double)(first / kTileKeys), most = 0.66 * kFilterRoom / ((double)nq * topk);
+        const double span = (double)tiles / (double)(fp.first / kTileKeys), most = 0.66 * kFilterRoom / ((double)nq * topk);
         int rounds = 1;
         while (pow(span, 1.0 / rounds) > most && rounds < 16) ++rounds;
         for (int r = 1; r <= rounds; ++r) {
             const int stride = r == rounds ? 1 : (int)std::max(1.0, stride0 / pow(span, (double)r / rounds));
             TQ_STEP(tq_launch_filter(p, f, codes, signs, rnorms, norms, keys_per_group, stride, st));
             TQ_STEP(tq_launch_filter_gather(p, f, codes, signs, rnorms, norms, st));
-            TQ_STEP(score_pass(gathered, q0, nq, 0, kFilterRoom, 1, f.scores - (int64_t)q0 * kFilterRoom, kFilterRoom, nullptr));
+            TQ_STEP(score_pass(gathered, q0, nq, 0, kFilterRoom, 1, f.scores - (int64_t)q0 * kFilterRoom, kFilterRoom, all_lists, nullptr));
             TQ_STEP(tq_launch_filter_select(f, topk, k2, r == rounds, st));
         }
+        float* pass_scores = top_scores + (int64_t)q0 * topk;
+        int64_t* pass_idx = top_idx + (int64_t)q0 * topk;
+        if (!fp.matrix) {
+            const Lists chunk{reinterpret_cast<unsigned long long*>(sc + fp.off_cand) - q0 * cp.cand_cap, cp.cand_cap};
+            TQ_STEP(run_candidates(chunk, q0, nq, f.bad, [&](int64_t key_off, int64_t key_cnt, int stride) {
+                return score_pass(all_keys, q0, nq, key_off, key_cnt, stride, nullptr, 0, chunk, f.bad);
+            }));
+        }
+        TQ_STEP(tq_merge_keys_launch(f.best, 1, nq, 1, topk, idx_base, pass_scores, pass_idx, st));
+        if (fp.matrix) {
+            float* mat = reinterpret_cast<float*>(sc + fp.off_matrix);
+            unsigned long long* part = reinterpret_cast<unsigned long long*>(sc + fp.off_part);
+            TQ_STEP(score_pass(all_keys, q0, nq, 0, keys_per_group, 1, mat - (int64_t)q0 * keys_per_group, keys_per_group, all_lists, f.bad));
+            topk_rows_kernel<<<dim3((unsigned)fp.segs, (unsigned)nq), kSelThreads, 0, st>>>(
+                mat, keys_per_group, (int64_t)nq * keys_per_group, nq, keys_per_group, kSegLen, group_rows, 0, topk, k2, (int)fp.segs, 0, part, f.bad);
+            tq_count_launch();
+            TQ_CUDA_TRY(cudaGetLastError());
+            TQ_STEP(tq_merge_keys_launch(part, (int)fp.segs, nq, 1, topk, idx_base, pass_scores, pass_idx, st, f.bad));
+        }
     }
-    TQ_STEP(run_candidates(f.bad));
-    return tq_merge_keys_launch(best, 1, qpg, groups, topk, idx_base, top_scores, top_idx, st);
+    return TQ_OK;
 }

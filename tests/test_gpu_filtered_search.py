@@ -32,11 +32,12 @@ def test_filtered_search_equals_the_sorted_matrix(lib_built, d, bits, n, nq, k):
     _check(prod, prod.quantize(x), q, k)
 
 
-def test_filtered_search_falls_back_when_its_lists_are_too_short(lib_built):
-    """Half the keys are one vector: more exact ties at the threshold than a round has room for."""
+@pytest.mark.parametrize("d,n,nq,k", [(128, (1 << 20) + 11, 32, 100), (64, (1 << 20) + 64, 70, 10), (256, (1 << 20) + 3, 33, 20), (64, (1 << 22) + 77, 70, 20)])
+def test_filtered_search_falls_back_when_its_lists_are_too_short(lib_built, d, n, nq, k):
+    """Half the keys are one vector: more exact ties at the threshold than a round has room for.  One pass of queries and several, with
+    the procedures of up to 4,194,304 keys and of more behind the first stage."""
     import torch
     import project_tensor_b200 as tg
-    d, n, nq, k = 128, (1 << 20) + 11, 32, 100
     gen = torch.Generator("cuda").manual_seed(5)
     x = torch.randn((n, d), device="cuda", generator=gen)
     x[1000:1000 + n // 2] = x[7]
@@ -45,6 +46,33 @@ def test_filtered_search_falls_back_when_its_lists_are_too_short(lib_built):
     q[4] = 0.0           # every score is zero
     prod = tg.TurboQuantProd(d, 4, seed=2026)
     _check(prod, prod.quantize(x), q, k)
+
+
+@pytest.mark.parametrize("n", [(1 << 20) + 5, 1 << 21])
+def test_filtered_search_for_queries_without_a_score(lib_built, n):
+    """NaN queries: every score is NaN, and the first rows are the best.  The other queries are unharmed."""
+    import torch
+    import project_tensor_b200 as tg
+    gen = torch.Generator("cuda").manual_seed(7)
+    prod = tg.TurboQuantProd(64, 4, seed=2026)
+    enc = prod.quantize(torch.randn((n, 64), device="cuda", generator=gen))
+    q = torch.randn((33, 64), device="cuda", generator=gen)
+    q[5, 3] = float("nan")
+    _check(prod, enc, q, 10, rows=[0, 4, 6, 32])
+    top_s, top_i = prod.attention_scores(q, enc, topk=10)
+    assert bool(top_s[5].isnan().all()) and top_i[5].tolist() == list(range(10))
+
+
+def test_scratch_of_a_search_is_that_of_one_score_matrix(lib_built):
+    import torch
+    import project_tensor_b200 as tg
+    from project_tensor_b200 import _native
+    handle = tg.TurboQuantProd(128, 4, seed=2026)._plans.handle(torch.device("cuda", 0))
+    for queries in (1, 16, 64, 1000, 10000):
+        for keys in (1 << 20, 1 << 21, 1 << 22):
+            got = _native.load().tq_topk_scratch_bytes(handle, 1, queries, keys, 20)
+            # a float per query and key; lists of every 65,536 keys, prepared queries and (few queries) gathered keys behind it
+            assert got <= queries * keys * 4 + queries * (keys >> 16) * 20 * 8 + (32 << 20), (queries, keys)
 
 
 def test_filtered_search_lists_keys_its_bound_does_not_cover(lib_built):
