@@ -31,4 +31,4 @@ int tq_launch_filter(const tq_plan* p, const TqFilterPass& f, const uint32_t* co
                      const float* norms, int64_t keys, int tile_stride, cudaStream_t st);
 int tq_launch_filter_gather(const tq_plan* p, const TqFilterPass& f, const uint32_t* codes, const uint32_t* signs, const float* rnorms,
                             const float* norms, cudaStream_t st);
-int tq_launch_filter_select(const TqFilterPass& f, int topk, int k2, bool final, cudaStream_t st);
+int tq_launch_filter_select(const TqFilterPass& f, int topk, int k2, bool final, bool keep_nan, cudaStream_t st);

@@ -532,8 +532,9 @@ gather_listed_kernel(const unsigned int* __restrict__ cnt, const unsigned int* _
 
 // First thresholds: the topk-th best of a query's sampled scores (list of sortable keys, empty slots 0), or a score just below it.
 // Bisection over the sortable bits of the scores, which the block keeps in registers; the lowest 8 bits stay open, so the
-// threshold is a lower bound.  NaN scores do not count.  One block per query.
+// threshold is a lower bound; at -inf it stays open altogether.  NaN scores do not count.  One block per query.
 constexpr int kSampleMax = 32768;
+constexpr uint32_t kOrderedMinusInf = 0x007fffffu;     // sortable bits
 __global__ void __launch_bounds__(1024)
 sample_threshold_kernel(const unsigned long long* __restrict__ cand, int64_t cap, unsigned int* __restrict__ cnt, float* __restrict__ thr, int topk) {
     __shared__ int total[24];
@@ -561,17 +562,18 @@ sample_threshold_kernel(const unsigned long long* __restrict__ cand, int64_t cap
         if (total[b] >= topk) prefix = trial;
     }
     if (threadIdx.x == 0) {
-        if (prefix != 0u) thr[q] = unordered_bits(prefix);
+        if (prefix > kOrderedMinusInf) thr[q] = unordered_bits(prefix);      // (the bits of -inf with some of them cleared are a NaN)
         cnt[q] = 0u;
     }
 }
 
 // One block per query: the k best of the gathered keys' scores.  final: they become the query's best list; otherwise only its
-// threshold is raised (the keys will be listed again).  The lists are empty afterwards.
+// threshold is raised (the keys will be listed again).  The lists are empty afterwards.  keep_nan: NaN scores rank by their
+// bits, as in a selection from a score matrix; else they are left out, as candidate mode does.
 __global__ void __launch_bounds__(256)
 select_gathered_kernel(const float* __restrict__ scores, int64_t row_stride, const unsigned int* __restrict__ g_rows,
                        const unsigned int* __restrict__ offsets, unsigned int* __restrict__ cnt, unsigned long long* __restrict__ best,
-                       float* __restrict__ thr, int topk, int k2, int final, const unsigned int* bad) {
+                       float* __restrict__ thr, int topk, int k2, int final, int keep_nan, const unsigned int* bad) {
     __shared__ __align__(16) unsigned long long a[kSelCap];
     __shared__ int hist[256];
     __shared__ int scratch[4];
@@ -607,7 +609,8 @@ select_gathered_kernel(const float* __restrict__ scores, int64_t row_stride, con
         }
 #pragma unroll
         for (int j = 0; j < (int)kBatch / 256; ++j) {
-            if (v[j] == v[j]) {
+            const bool have = base + j * 256 + threadIdx.x < end;
+            if (have && (keep_nan || v[j] == v[j])) {
                 const unsigned long long ck = make_key(v[j], r[j]);
                 if (ck > t) a[atomicAdd(&count, 1)] = ck;
             }
@@ -623,7 +626,9 @@ select_gathered_kernel(const float* __restrict__ scores, int64_t row_stride, con
     if (final)
         for (int i = threadIdx.x; i < topk; i += blockDim.x) best[(size_t)q * topk + i] = a[i];
     if (threadIdx.x == 0) {
-        if (keep == topk) thr[q] = unordered_bits((uint32_t)(a[topk - 1] >> 32));
+        // (a NaN above the others: only keys that are listed unseen can still come before it)
+        const uint32_t last = keep == topk ? (uint32_t)(a[topk - 1] >> 32) : 0u;
+        if (last >= kOrderedMinusInf) thr[q] = unordered_bits(last);
         cnt[q] = 0u;
     }
 }
@@ -699,8 +704,8 @@ int tq_launch_filter_gather(const tq_plan* p, const TqFilterPass& f, const uint3
     return TQ_OK;
 }
 
-int tq_launch_filter_select(const TqFilterPass& f, int topk, int k2, bool final, cudaStream_t st) {
-    select_gathered_kernel<<<f.nq, 256, 0, st>>>(f.scores, f.room, f.g_rows, f.offsets, f.cnt, f.best, f.thr, topk, k2, final ? 1 : 0, f.bad);
+int tq_launch_filter_select(const TqFilterPass& f, int topk, int k2, bool final, bool keep_nan, cudaStream_t st) {
+    select_gathered_kernel<<<f.nq, 256, 0, st>>>(f.scores, f.room, f.g_rows, f.offsets, f.cnt, f.best, f.thr, topk, k2, final ? 1 : 0, keep_nan ? 1 : 0, f.bad);
     tq_count_launch();
     TQ_CUDA_TRY(cudaGetLastError());
     return TQ_OK;

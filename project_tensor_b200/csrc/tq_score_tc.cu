@@ -1351,7 +1351,7 @@ case B:                                                                         
             TQ_STEP(tq_launch_filter(p, f, codes, signs, rnorms, norms, keys_per_group, stride, st));
             TQ_STEP(tq_launch_filter_gather(p, f, codes, signs, rnorms, norms, st));
             TQ_STEP(score_pass(gathered, q0, nq, 0, kFilterRoom, 1, f.scores - (int64_t)q0 * kFilterRoom, kFilterRoom, all_lists, nullptr));
-            TQ_STEP(tq_launch_filter_select(f, topk, k2, r == rounds, st));
+            TQ_STEP(tq_launch_filter_select(f, topk, k2, r == rounds, fp.matrix, st));
         }
         float* pass_scores = top_scores + (int64_t)q0 * topk;
         int64_t* pass_idx = top_idx + (int64_t)q0 * topk;

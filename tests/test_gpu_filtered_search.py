@@ -63,6 +63,46 @@ def test_filtered_search_for_queries_without_a_score(lib_built, n):
     assert bool(top_s[5].isnan().all()) and top_i[5].tolist() == list(range(10))
 
 
+@pytest.mark.parametrize("n", [(1 << 20) + 5, 1 << 22])
+def test_keys_without_a_score_rank_as_in_a_selection_from_the_matrix(lib_built, n):
+    """NaN norms: such scores come first up to 4,194,304 keys, the lowest rows first.  More of them than a query wants, and fewer."""
+    import torch
+    import project_tensor_b200 as tg
+    gen = torch.Generator("cuda").manual_seed(8)
+    prod = tg.TurboQuantProd(64, 4, seed=2026)
+    enc = prod.quantize(torch.randn((n, 64), device="cuda", generator=gen))
+    tg.packed_buffers(enc)["norms"][3::n // 16] = float("nan")
+    q = torch.randn((32, 64), device="cuda", generator=gen)
+    prod.set_kernel_path("tensor")
+    srt = torch.sort(prod.attention_scores(q, enc), dim=1, descending=True, stable=True)      # (NaN sorts as the greatest)
+    prod.set_kernel_path("auto")
+    for k in (10, 40):
+        top_s, top_i = prod.attention_scores(q, enc, topk=k)
+        assert torch.equal(top_i, srt.indices[:, :k])
+        assert torch.equal(top_s.nan_to_num(nan=7e30), srt.values[:, :k].nan_to_num(nan=7e30))
+
+
+def test_scores_that_are_nearly_all_minus_infinity(lib_built):
+    """Finite norms and products below the smallest float: some thirty scores of each query are finite, fewer than one in the sample."""
+    import torch
+    import project_tensor_b200 as tg
+    n, k = (1 << 20) + 5, 100
+    gen = torch.Generator("cuda").manual_seed(9)
+    prod = tg.TurboQuantProd(64, 4, seed=2026)
+    enc = prod.quantize(torch.randn((n, 64), device="cuda", generator=gen))
+    q = torch.randn((1, 64), device="cuda", generator=gen).expand(32, 64) * 1e6
+    packed = tg.packed_buffers(enc)
+    packed["residual_norms"][:] = 0.0
+    packed["norms"][:] = torch.where(prod.attention_score(q[0], enc) < 0, 1e37, -1e37)
+    prod.set_kernel_path("tensor")
+    mat = prod.attention_scores(q, enc)
+    prod.set_kernel_path("auto")
+    assert 5 <= int(torch.isfinite(mat[0]).sum()) < k
+    srt = torch.sort(mat, dim=1, descending=True, stable=True)
+    top_s, top_i = prod.attention_scores(q, enc, topk=k)
+    assert torch.equal(top_s, srt.values[:, :k]) and torch.equal(top_i, srt.indices[:, :k])
+
+
 def test_scratch_of_a_search_is_that_of_one_score_matrix(lib_built):
     import torch
     import project_tensor_b200 as tg
