@@ -16,6 +16,7 @@ struct TqFilterPass {
     unsigned int* offsets;       // [nq]
     unsigned int* bad;           // set: some list or the gathered arrays were too small, or a query is beyond the bound
     unsigned int* gathered;      // keys gathered
+    unsigned int* expected;      // [kFilterRounds] keys the rounds will list, by the sample
     uint32_t *g_codes, *g_signs;
     float *g_norms, *g_rnorms;
     unsigned int* g_rows;
@@ -26,7 +27,13 @@ struct TqFilterPass {
 size_t tq_filter_prep_bytes(int d, int qpad);
 int tq_launch_filter_prep(const tq_plan* p, const unsigned char* prep, int qpad, int nq, float c_max, float beta_scale, unsigned char* out,
                           unsigned int* bad, cudaStream_t st);
-int tq_launch_sample_threshold(const unsigned long long* cand, int64_t cap, unsigned int* cnt, float* thr, int queries, int topk, cudaStream_t st);
+// What the rounds multiply the sample by, so that the sample can tell how many keys each round will list.
+constexpr int kFilterRounds = 16;
+struct TqFilterRounds {
+    int rounds;
+    float keys[kFilterRounds];       // keys of round r over those of the sample
+};
+int tq_launch_sample_threshold(const TqFilterPass& f, const TqFilterRounds& rounds, const unsigned long long* cand, int64_t cap, int topk, cudaStream_t st);
 int tq_launch_filter(const tq_plan* p, const TqFilterPass& f, const uint32_t* codes, const uint32_t* signs, const float* rnorms,
                      const float* norms, int64_t keys, int tile_stride, cudaStream_t st);
 int tq_launch_filter_gather(const tq_plan* p, const TqFilterPass& f, const uint32_t* codes, const uint32_t* signs, const float* rnorms,

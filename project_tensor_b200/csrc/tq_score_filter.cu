@@ -535,13 +535,18 @@ gather_listed_kernel(const unsigned int* __restrict__ cnt, const unsigned int* _
 // threshold is a lower bound; at -inf it stays open altogether.  NaN scores do not count.  One block per query.
 constexpr int kSampleMax = 32768;
 constexpr uint32_t kOrderedMinusInf = 0x007fffffu;     // sortable bits
+//
+// The sample also tells when the lists will be too short, so that the first stage need not run into it: a query's round lists the
+// keys that reach its threshold, as many per key as in the sample, until the better ones among them are enough to raise the
+// threshold.  Without ties that is ratio * topk; with half of 4,194,304 keys equal the overflowing lists alone cost 1.3 ms.
 __global__ void __launch_bounds__(1024)
-sample_threshold_kernel(const unsigned long long* __restrict__ cand, int64_t cap, unsigned int* __restrict__ cnt, float* __restrict__ thr, int topk) {
-    __shared__ int total[24];
+sample_threshold_kernel(const unsigned long long* __restrict__ cand, int64_t cap, unsigned int* __restrict__ cnt, float* __restrict__ thr, int topk,
+                        const TqFilterRounds rounds, unsigned int* __restrict__ expected, int room, unsigned int* bad) {
+    __shared__ int total[26];
     const int q = blockIdx.x;
     const unsigned long long* list = cand + (size_t)q * cap;
     const int n = min((int)cnt[q], kSampleMax);
-    if (threadIdx.x < 24) total[threadIdx.x] = 0;
+    if (threadIdx.x < 26) total[threadIdx.x] = 0;
     uint32_t v[kSampleMax / 1024];
 #pragma unroll
     for (int j = 0; j < kSampleMax / 1024; ++j) {
@@ -550,20 +555,34 @@ sample_threshold_kernel(const unsigned long long* __restrict__ cand, int64_t cap
         if (v[j] > 0xff800000u) v[j] = 0u;
     }
     __syncthreads();
+    auto count = [&](uint32_t from, int slot) {       // sampled scores from `from` on
+        int c = 0;
+#pragma unroll
+        for (int j = 0; j < kSampleMax / 1024; ++j) c += v[j] >= from ? 1 : 0;
+        c = __reduce_add_sync(0xffffffffu, c);
+        if ((threadIdx.x & 31) == 0 && c) atomicAdd(&total[slot], c);
+        __syncthreads();
+        return total[slot];
+    };
     uint32_t prefix = 0u;
     for (int b = 0; b < 24; ++b) {
         const uint32_t trial = prefix | (0x80000000u >> b);
-        int c = 0;
-#pragma unroll
-        for (int j = 0; j < kSampleMax / 1024; ++j) c += v[j] >= trial ? 1 : 0;
-        c = __reduce_add_sync(0xffffffffu, c);
-        if ((threadIdx.x & 31) == 0 && c) atomicAdd(&total[b], c);
-        __syncthreads();
-        if (total[b] >= topk) prefix = trial;
+        if (count(trial, b) >= topk) prefix = trial;
     }
+    const bool open = prefix <= kOrderedMinusInf;       // (the bits of -inf with some of them cleared are a NaN)
+    const int reach = count(open ? 0u : prefix, 24), better = count(open ? 0xffffffffu : prefix + 256u, 25);
     if (threadIdx.x == 0) {
-        if (prefix > kOrderedMinusInf) thr[q] = unordered_bits(prefix);      // (the bits of -inf with some of them cleared are a NaN)
+        if (!open) thr[q] = unordered_bits(prefix);
         cnt[q] = 0u;
+        float before = 1.f;
+        bool tied = true;
+        for (int r = 0; r < rounds.rounds; ++r) {
+            tied = tied && (float)better * before < (float)topk;
+            const float mine = tied ? (float)reach * rounds.keys[r] : (float)topk * rounds.keys[r] / before;
+            before = rounds.keys[r];
+            const unsigned int add = (unsigned int)fminf(mine, 1.0e9f);
+            if (open || atomicAdd(expected + r, add) + add > (unsigned int)room) *bad = 1u;
+        }
     }
 }
 
@@ -663,8 +682,8 @@ int tq_launch_filter_prep(const tq_plan* p, const unsigned char* prep, int qpad,
     return TQ_OK;
 }
 
-int tq_launch_sample_threshold(const unsigned long long* cand, int64_t cap, unsigned int* cnt, float* thr, int queries, int topk, cudaStream_t st) {
-    sample_threshold_kernel<<<queries, 1024, 0, st>>>(cand, cap, cnt, thr, topk); tq_count_launch();
+int tq_launch_sample_threshold(const TqFilterPass& f, const TqFilterRounds& rounds, const unsigned long long* cand, int64_t cap, int topk, cudaStream_t st) {
+    sample_threshold_kernel<<<f.nq, 1024, 0, st>>>(cand, cap, f.cnt, f.thr, topk, rounds, f.expected, f.room, f.bad); tq_count_launch();
     TQ_CUDA_TRY(cudaGetLastError());
     return TQ_OK;
 }

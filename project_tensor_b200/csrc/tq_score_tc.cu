@@ -1041,13 +1041,15 @@ static bool use_candidates(const float* scores, int topk, int64_t keys_per_group
 // Its fixed part (a sample, two rounds, the skipped fallback: some 25 launches) costs about 80 us, what it saves grows with keys
 // and queries.  Search through an index, before / with it: 1,048,576 keys, 64 queries 300 / 249 us, 32 queries 210 / 198, 8 queries
 // 160 / 160; 2,097,152 keys, 8 queries 246 / 214, 1 query 219 / 183; 8,388,608 keys, 64 queries 1502 / 622, 1 query 1004 / 424.
+// Long lists want more keys too (they are gathered and sorted by query): 32 queries, top 1,000: 1,048,576 keys 304 / 388 us,
+// 1,500,000 keys 410 / 432, 2,097,152 keys 514 / 476.
 constexpr int64_t kFilterFrom = 1 << 21, kFilterFromMany = 1 << 20;      // keys from which on it pays; from 32 queries on
 constexpr int64_t kFilterSample = 1 << 15;     // keys of the first sample
 constexpr int kFilterRoom = 1 << 18;           // gathered keys of a round
 static bool use_filter(const tq_plan* p, const float* scores, int groups, int qpg, int topk, int64_t keys_per_group) {
     const int nq = qpg < 64 ? qpg : 64;
     return scores == nullptr && topk > 0 && groups == 1 && p->beta_scale > 0.f && keys_per_group >= (qpg >= 32 ? kFilterFromMany : kFilterFrom) &&
-           keys_per_group < (int64_t)1 << 31 && (int64_t)nq * topk * 6 <= kFilterRoom;
+           keys_per_group < (int64_t)1 << 31 && (int64_t)nq * topk * 6 <= kFilterRoom && (int64_t)nq * topk * 48 <= keys_per_group;
 }
 // The procedure that a filtered search falls back to takes the same passes of queries, one after the other, and works in the
 // memory that the pass's lists, scores and gathered keys have left: the whole is no larger than one pass of that procedure (64 queries x
@@ -1319,6 +1321,7 @@ case B:                                                                         
     f.fprep = sc + fp.off_prep;
     f.bad = reinterpret_cast<unsigned int*>(sc + fp.off_words);
     f.gathered = f.bad + 1;
+    f.expected = f.bad + 2;
     f.rows = reinterpret_cast<unsigned int*>(sc + fp.off_rows);
     f.offsets = reinterpret_cast<unsigned int*>(sc + fp.off_offsets);
     f.g_codes = reinterpret_cast<uint32_t*>(sc + fp.off_codes);
@@ -1336,22 +1339,27 @@ case B:                                                                         
         const Lists sample{reinterpret_cast<unsigned long long*>(sc + fp.off_sample) - q0 * fp.first, fp.first};
         f.nq = nq; f.qpad = pad_of(nq);
         f.thr = thr + q0; f.cnt = cnt + q0; f.best = best + (int64_t)q0 * topk;
-        TQ_CUDA_TRY(cudaMemsetAsync(f.bad, 0, 2 * sizeof(unsigned int), st));
+        TQ_CUDA_TRY(cudaMemsetAsync(f.bad, 0, (2 + kFilterRounds) * sizeof(unsigned int), st));
         TQ_STEP(init(q0, nq, fp.first, nullptr));
         TQ_STEP(prepare_pass(q0, nq));
         TQ_STEP(score_pass(all_keys, q0, nq, 0, keys_per_group, stride0, nullptr, 0, sample, nullptr));
         TQ_STEP(tq_launch_filter_prep(p, prep, f.qpad, nq, p->c_max, p->beta_scale, f.fprep, f.bad, st));
-        TQ_STEP(tq_launch_sample_threshold(sample.at + q0 * fp.first, fp.first, f.cnt, f.thr, nq, topk, st));
         // rounds: the fewest whose ratio keeps the lists of all queries within two thirds of the room
         const double span = (double)tiles / (double)(fp.first / kTileKeys), most = 0.66 * kFilterRoom / ((double)nq * topk);
-        int rounds = 1;
-        while (pow(span, 1.0 / rounds) > most && rounds < 16) ++rounds;
-        for (int r = 1; r <= rounds; ++r) {
-            const int stride = r == rounds ? 1 : (int)std::max(1.0, stride0 / pow(span, (double)r / rounds));
+        TqFilterRounds rounds{1, {}};
+        while (pow(span, 1.0 / rounds.rounds) > most && rounds.rounds < kFilterRounds) ++rounds.rounds;
+        int strides[kFilterRounds];
+        for (int r = 0; r < rounds.rounds; ++r) {
+            strides[r] = r + 1 == rounds.rounds ? 1 : (int)std::max(1.0, stride0 / pow(span, (double)(r + 1) / rounds.rounds));
+            rounds.keys[r] = (float)(((tiles + strides[r] - 1) / strides[r]) / (double)(fp.first / kTileKeys));
+        }
+        TQ_STEP(tq_launch_sample_threshold(f, rounds, sample.at + q0 * fp.first, fp.first, topk, st));
+        for (int r = 0; r < rounds.rounds; ++r) {
+            const int stride = strides[r];
             TQ_STEP(tq_launch_filter(p, f, codes, signs, rnorms, norms, keys_per_group, stride, st));
             TQ_STEP(tq_launch_filter_gather(p, f, codes, signs, rnorms, norms, st));
             TQ_STEP(score_pass(gathered, q0, nq, 0, kFilterRoom, 1, f.scores - (int64_t)q0 * kFilterRoom, kFilterRoom, all_lists, nullptr));
-            TQ_STEP(tq_launch_filter_select(f, topk, k2, r == rounds, fp.matrix, st));
+            TQ_STEP(tq_launch_filter_select(f, topk, k2, r + 1 == rounds.rounds, fp.matrix, st));
         }
         float* pass_scores = top_scores + (int64_t)q0 * topk;
         int64_t* pass_idx = top_idx + (int64_t)q0 * topk;
