@@ -6,6 +6,24 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
+def _fell_back(prod, enc, q, k):
+    """Whether a search over up to 4,194,304 keys went on to the score matrix: it lies over the lists of the first stage in the scratch
+    block and is larger than they are (32 queries and more), so that its end is written by nothing else."""
+    import torch
+    import project_tensor_b200 as tg
+    from project_tensor_b200 import _native
+    lib, packed, n = _native.load(), tg.packed_buffers(enc), enc.prefix_shape[0]
+    handle, nq = prod._plans.handle(q.device), q.shape[0]
+    need = lib.tq_topk_scratch_bytes(handle, 1, nq, n, k)
+    scratch = torch.full((need,), 0xA5, dtype=torch.uint8, device=q.device)
+    top_s, top_i = torch.empty((nq, k), device=q.device), torch.empty((nq, k), dtype=torch.int64, device=q.device)
+    _native.check(lib.tq_score_batched(handle, q.data_ptr(), 1, nq, packed["codes"].data_ptr(), packed["signs"].data_ptr(),
+                                       packed["residual_norms"].data_ptr(), packed["norms"].data_ptr(), n, None, k, top_s.data_ptr(),
+                                       top_i.data_ptr(), 0, scratch.data_ptr(), need, torch.cuda.current_stream().cuda_stream))
+    end = 4 * n * nq // 100 * 98
+    return not bool((scratch[end - (1 << 20):end] == 0xA5).all())
+
+
 def _check(prod, enc, q, k, rows=None):
     import torch
     prod.set_kernel_path("tensor")       # one to four queries would take a lookup-table kernel, with other last bits
@@ -45,7 +63,10 @@ def test_filtered_search_falls_back_when_its_lists_are_too_short(lib_built, d, n
     q[3] = x[7]
     q[4] = 0.0           # every score is zero
     prod = tg.TurboQuantProd(d, 4, seed=2026)
-    _check(prod, prod.quantize(x), q, k)
+    enc = prod.quantize(x)
+    _check(prod, enc, q, k)
+    if nq == 32:
+        assert _fell_back(prod, enc, q, k)
 
 
 @pytest.mark.parametrize("n", [(1 << 20) + 5, 1 << 21])
@@ -116,7 +137,8 @@ def test_scratch_of_a_search_is_that_of_one_score_matrix(lib_built):
 
 
 def test_filtered_search_lists_keys_its_bound_does_not_cover(lib_built):
-    """Hand-made norms: huge residual norms (the scaled sign operand leaves the fp16 range), huge and negative norms."""
+    """Hand-made norms: huge residual norms (the scaled sign operand leaves the fp16 range), huge and negative norms; few enough
+    for the lists, which a whole warp's keys enter beside a key of huge norm."""
     import torch
     import project_tensor_b200 as tg
     d, n, nq, k = 128, (1 << 20) + 3, 32, 100
@@ -124,8 +146,12 @@ def test_filtered_search_lists_keys_its_bound_does_not_cover(lib_built):
     prod = tg.TurboQuantProd(d, 4, seed=2026)
     enc = prod.quantize(torch.randn((n, d), device="cuda", generator=gen))
     packed = tg.packed_buffers(enc)
-    packed["residual_norms"][5:4000:37] = 1.0e7
-    packed["norms"][11:9000:41] *= -50.0
-    packed["norms"][13:9000:43] = 1.0e12
+    packed["residual_norms"][5::n // 40] = 1.0e7
+    packed["norms"][11::n // 50] *= -50.0
+    packed["norms"][1013::n // 20] = 1.0e12
     q = torch.randn((nq, d), device="cuda", generator=gen)
     _check(prod, enc, q, k)
+    top_s, top_i = prod.attention_scores(q, enc, topk=k)
+    for first, step in ((5, n // 40), (1013, n // 20)):       # they are among the best, and the first stage has seen to it
+        assert all(bool(((row - first) % step == 0).any()) for row in top_i)
+    assert not _fell_back(prod, enc, q, k)
