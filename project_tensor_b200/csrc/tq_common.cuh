@@ -236,9 +236,9 @@ int tq_launch_score_few(const tq_plan* p, const float* q, int groups, int qpg, c
                         const float* rnorms, const float* norms, int64_t keys_per_group, float* scores, cudaStream_t st,
                         int64_t group_rows = 0);
 
-// One query against many keys through tables of the query's products, where that is the faster way (tq_score_table.cu).
+// One query (or two) through tables of its products, where that is the faster way (tq_score_table.cu).
 bool tq_score_table_better(const tq_plan* p, int groups, int qpg, int64_t keys_per_group);
-int tq_launch_score_table(const tq_plan* p, const float* q, int groups, const uint32_t* codes, const uint32_t* signs, const float* rnorms,
+int tq_launch_score_table(const tq_plan* p, const float* q, int groups, int qpg, const uint32_t* codes, const uint32_t* signs, const float* rnorms,
                           const float* norms, int64_t keys_per_group, float* scores, cudaStream_t st, int64_t group_rows);
 
 // Scoring kernels.  `group_rows`: rows between the first keys of consecutive groups in the key arrays (0 = the

@@ -287,10 +287,12 @@ int launch_few(const tq_plan* p, const FewArgs& a, int groups, cudaStream_t st) 
     using P = FewPlan<KB, DR>;
     TQ_GRANT_SMEM((score_few_kernel<KB, DR>), P::total, p->device);
     const int passes = (a.qpg + NQ - 1) / NQ;
-    // a block per SM over all groups (its prologue costs some 4 us): every block of a group gets at least a tile per warp
-    int64_t blocks = (tq_sm_count(p->device) + (int64_t)passes * groups - 1) / ((int64_t)passes * groups);
+    // at most a block per SM over all groups, as many as run at once (the prologue costs 3 to 14 us: 64 groups in three blocks each
+    // took two rounds of it, 28 us for 64 x 4,096 keys of d = 128), and every block of a group gets at least a tile per warp
     const int64_t tiles = (a.keys_per_group + kTile - 1) / kTile, most = (tiles + 3) / 4;
+    int64_t blocks = tq_sm_count(p->device) / ((int64_t)passes * groups);
     if (blocks > most) blocks = most;
+    if (blocks < 1) blocks = 1;
     TQ_CUDA_TRY(tq_launch_dependent(score_few_kernel<KB, DR>, dim3((unsigned)blocks, (unsigned)passes, (unsigned)groups), dim3(kFewThreads),
                                     (size_t)P::total, st, p->dev, a));
     return TQ_OK;
@@ -312,7 +314,7 @@ int tq_launch_score_few(const tq_plan* p, const float* q, int groups, int qpg, c
     TqRange range("tq.score.few_queries");
     if (group_rows <= 0) group_rows = keys_per_group;
     if (tq_score_table_better(p, groups, qpg, keys_per_group))
-        return tq_launch_score_table(p, q, groups, codes, signs, rnorms, norms, keys_per_group, scores, st, group_rows);
+        return tq_launch_score_table(p, q, groups, qpg, codes, signs, rnorms, norms, keys_per_group, scores, st, group_rows);
     const FewArgs a{q, codes, signs, rnorms, norms, qpg, keys_per_group, group_rows, scores};
     const int d = p->dev.d;
     switch (p->dev.bits) {

@@ -1,4 +1,4 @@
-// attention_score for one query against many keys (_quant.py:334-358).
+// attention_score for one query (_quant.py:334-358) against very many keys, or in very many groups of few keys.
 //
 //   score(q, key) = norm * ( (R q) . codebook[codes]  +  alpha * rnorm * ((S q) . signs) )
 //
@@ -8,9 +8,9 @@
 //   byte table   [d/8 positions][256 entries]      sum over the 8 sign bits of the byte of +-(S q)[coordinate]
 //
 // and every thread walks the packed codes and sign words of one key: d/2 + d/8 lookups and additions, no unpacking.
-// score_few_kernel expands the keys for up to four queries at once; for one it pays its per-tile overhead at d = 64 (4,068,313
-// keys, 1 / 2 / 3 code bits: 76 / 79 / 83 us there, 54 / 58 / 66 here) and the expansion at d = 256 (2 / 3 bits: 225 / 316 us there, 197 /
-// 275 here).  Its prologue is the shorter one, so few keys are its own in either case.
+// score_few_kernel expands the keys for up to four queries at once; for one it pays that expansion alone (600,000 keys and more), and
+// it keeps an SM to itself for a prologue of 3 / 7 / 14 us at d = 64 / 128 / 256, where a block here takes 5 / 9 / 15 us but four to
+// eight run beside each other (hundreds of groups with a few keys each).  Anything between is its own.
 #include "tq_common.cuh"
 
 #include <stdint.h>
@@ -140,29 +140,37 @@ int launch_table(const tq_plan* p, const float* q, const uint32_t* codes, const 
 
 }  // namespace
 
-// The lines lie where the two kernels meet: the prologue is 1 to 6 us longer here, a thousand keys cost 13 against 19 ns at d = 64,
-// 30 against 31 at d = 128 (3-bit codes), 48 to 68 against 54 to 78 at d = 256 (2 and 3 bits).
+// The lines lie where the two kernels meet (kernel time in us, warp-level kernel / this one; 1, 2, 3 code bits):
+//   one group   d = 64     400,000 keys  - / 10.2:11.2 / -              1,048,576 keys  - / 21.2:16.2 / -        (4 bits 22.5:25.5)
+//               d = 128    400,000 keys  20.1:19.5 / 18.8:19.8 / 19.8:22.0    1,048,576 keys  40.7:28.2 / 36.7:29.2 / 40.0:38.1
+//                          4,000,000 keys  137:90 / 124:95 / 132:118 (4 bits 130:190)
+//               d = 256    400,000 keys  36.4:37.0 / 38.5:38.7 / 43.1:53.8    2,000,000 keys  127:104 / 143:116 / 171:165
+//   groups      d = 128    2,048 x 32 keys  100:36 / 104:37 / 106:42 (4 bits 104:72)    4,096 x 512  270:155 / 273:160 / 279:167 (280:341)
+//               d = 64, 256, 2 and 3 bits    4,096 x 32  83:32, 445:194    4,096 x 512  116:75, 587:468    512 x 1,008  22:21, 102:120
+//               (d = 64, 4 bits, 4,096 x 512  129:108)
 bool tq_score_table_better(const tq_plan* p, int groups, int qpg, int64_t keys_per_group) {
-    const int64_t keys = (int64_t)groups * keys_per_group;
     const int d = p->dev.d, bits = p->dev.bits;
-    if (!p->has_projection || qpg != 1) return false;
-    return (d == 64 && bits >= 1 && bits <= 4 && keys >= 1 << 18) || (d == 128 && (bits == 2 || bits == 3) && keys >= 3 << 20) ||
-           (d == 256 && (bits == 2 || bits == 3) && keys >= 1 << 20);
+    if (!p->has_projection || bits < 1 || bits > 4 || (d == 256 && bits == 4)) return false;
+    // more groups than the other kernel runs at once, and one or two blocks for each
+    const int64_t blocks = qpg * ((keys_per_group + kTableThreads - 1) / kTableThreads);
+    if (groups > tq_sm_count(p->device) && blocks <= (bits <= 3 || d == 64 ? 2 : 1)) return true;
+    if (qpg != 1 || bits == 4) return false;
+    return keys_per_group >= (bits <= 2 || d == 64 ? 1 << 19 : d == 128 ? 1 << 20 : 1 << 21);
 }
 
-// scores: [groups][keys_per_group]
-int tq_launch_score_table(const tq_plan* p, const float* q, int groups, const uint32_t* codes, const uint32_t* signs, const float* rnorms,
+// scores: [groups][qpg][keys_per_group]
+int tq_launch_score_table(const tq_plan* p, const float* q, int groups, int qpg, const uint32_t* codes, const uint32_t* signs, const float* rnorms,
                           const float* norms, int64_t keys_per_group, float* scores, cudaStream_t st, int64_t group_rows) {
     TqRange range("tq.score.one_query");
     if (group_rows <= 0) group_rows = keys_per_group;
-#define TQ_TABLE_ARGS p, q, codes, signs, rnorms, norms, keys_per_group, group_rows, groups, 1, scores, st
-    if (p->dev.d == 256) return p->dev.bits == 2 ? launch_table<2, 256>(TQ_TABLE_ARGS) : launch_table<3, 256>(TQ_TABLE_ARGS);
-    if (p->dev.d == 128) return p->dev.bits == 2 ? launch_table<2, 128>(TQ_TABLE_ARGS) : launch_table<3, 128>(TQ_TABLE_ARGS);
-#undef TQ_TABLE_ARGS
+    const int d = p->dev.d;
     switch (p->dev.bits) {
-#define TQ_TABLE(B) case B: return launch_table<B, 64>(p, q, codes, signs, rnorms, norms, keys_per_group, group_rows, groups, 1, scores, st);
-        TQ_TABLE(1) TQ_TABLE(2) TQ_TABLE(3) TQ_TABLE(4)
+#define TQ_TABLE(B, D) launch_table<B, D>(p, q, codes, signs, rnorms, norms, keys_per_group, group_rows, groups, qpg, scores, st)
+        case 1: return d == 256 ? TQ_TABLE(1, 256) : d == 128 ? TQ_TABLE(1, 128) : TQ_TABLE(1, 64);
+        case 2: return d == 256 ? TQ_TABLE(2, 256) : d == 128 ? TQ_TABLE(2, 128) : TQ_TABLE(2, 64);
+        case 3: return d == 256 ? TQ_TABLE(3, 256) : d == 128 ? TQ_TABLE(3, 128) : TQ_TABLE(3, 64);
+        case 4: if (d != 256) return d == 128 ? TQ_TABLE(4, 128) : TQ_TABLE(4, 64);
 #undef TQ_TABLE
     }
-    return tq_fail(TQ_ERR_UNSUPPORTED, "no one-query table kernel for d=%d bits=%d", p->dev.d, p->dev.bits);
+    return tq_fail(TQ_ERR_UNSUPPORTED, "no table kernel for d=%d bits=%d", d, p->dev.bits);
 }

@@ -14,7 +14,9 @@ def test_few_queries(d, bits):
     import torch
     quant = tg.TurboQuantProd(d, bits, seed=2026)
     gen = torch.Generator("cuda").manual_seed(d + bits)
-    many = ((1, 1, (1 << 20) + 33),) if d == 256 and bits in (3, 4) else ()      # where the table kernel takes over
+    # where the table kernel takes over: many keys, many groups of few keys
+    many = ((300, 1, 33), (151, 2, 256), (160, 1, 511), (150, 1, 256))
+    many += ((1, 1, ((1 << 19) if bits <= 3 else (1 << 20)) + 33),) if d < 256 or bits <= 3 else ()
     for groups, qpg, n in many + ((1, 1, 1), (1, 1, 15), (3, 1, 4097), (1, 2, 17), (2, 2, 2368), (1, 3, 37889), (4, 4, 530), (1, 1, 300001)):
         keys = torch.randn(groups * n, d, device="cuda", generator=gen)
         keys[n // 2] = 0
