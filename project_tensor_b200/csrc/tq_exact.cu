@@ -932,6 +932,21 @@ int launch_tile_rows(const RowsJob& a, const RowsJob* b, int64_t rows, int devic
                                     advance, shape));
     return TQ_OK;
 }
+// d > 256: a block has an SM to itself, so the time is that of a block times the rounds in which they run, and a block of 4, 8 or
+// 16 rows takes in proportion 68, 81 and 100 (d = 512, TurboQuantProd: 86 / 103 / 127 us; d = 768 191 / 228 / 291) or 55, 65 and 100 (d = 1,024:
+// 293 / 340 / 530 us).  The fewest rows win for single rows, the most for many; the shapes' columns fit d to a quarter.  (16 rows for every
+// call: one row of d = 1,024 took 573 us, d = 512 134.)
+int wide_block_rows(int d, int64_t rows, int64_t sms) {
+    static constexpr int kRows[3] = {4, 8, 16}, kCost[2][3] = {{68, 81, 100}, {55, 65, 100}};
+    int best = 0;
+    int64_t least = 0;
+    for (int i = 0; i < 3; ++i) {
+        const int64_t cost = ((rows + kRows[i] * sms - 1) / (kRows[i] * sms)) * kCost[d > 768][i];
+        if (i == 0 || cost < least) { least = cost; best = kRows[i]; }
+    }
+    return best;
+}
+
 // Rows per block: one while every row can have an SM to itself (d <= 128), then four, 16 (8 at d = 256) while larger blocks would leave
 // SMs idle, 64 or 32 from there on.
 int launch_rows(const RowsJob& a, const RowsJob* b, int64_t rows, int device, int advance, cudaStream_t st) {
@@ -939,7 +954,8 @@ int launch_rows(const RowsJob& a, const RowsJob* b, int64_t rows, int device, in
     const int64_t sms = tq_sm_count(device), total = b ? 2 * rows : rows;
     if (d <= 128 && total <= sms) return launch_few_rows<1>(a, b, rows, device, advance, st);
     if (d <= 128 && total <= sms * 4) return launch_few_rows<4>(a, b, rows, device, advance, st);
-    const bool many = total > sms * 32;
+    // (64-row blocks on half the SMs are slower than 16-row blocks on all of them: 4,737 rows of d = 96, TurboQuantMSE, 21.5 us against 10)
+    const bool many = total > sms * (d <= 96 ? 64 : d <= 128 ? 56 : 32);
     if (d <= 64) return many ? launch_tile_rows<16, 4, 8, 8>(a, b, rows, device, advance, st) : launch_tile_rows<4, 4, 32, 2>(a, b, rows, device, advance, st);
     if (d <= 96) return many ? launch_tile_rows<16, 4, 8, 12>(a, b, rows, device, advance, st) : launch_tile_rows<4, 4, 32, 3>(a, b, rows, device, advance, st);
     if (d <= 128) return many ? launch_tile_rows<8, 8, 16, 8>(a, b, rows, device, advance, st) : launch_tile_rows<4, 4, 32, 4>(a, b, rows, device, advance, st);
@@ -947,8 +963,16 @@ int launch_rows(const RowsJob& a, const RowsJob* b, int64_t rows, int device, in
         if (total <= sms * 8) return launch_tile_rows<2, 4, 64, 4>(a, b, rows, device, advance, st);
         return many ? launch_tile_rows<4, 8, 32, 8>(a, b, rows, device, advance, st) : launch_tile_rows<2, 8, 64, 4>(a, b, rows, device, advance, st);
     }
-    if (d <= 512) return launch_tile_rows<4, 4, 64, 8>(a, b, rows, device, advance, st);
-    return launch_tile_rows<4, 4, 64, 16>(a, b, rows, device, advance, st);
+    const int block = wide_block_rows(d, total, sms);
+#define TQ_WIDE(C4, T4, C8, T8, C16, T16)                                                                                              \
+    return block == 4   ? launch_tile_rows<1, 4, C4, T4>(a, b, rows, device, advance, st)                                              \
+           : block == 8 ? launch_tile_rows<1, 8, C8, T8>(a, b, rows, device, advance, st)                                              \
+                        : launch_tile_rows<2, 8, C16, T16>(a, b, rows, device, advance, st)
+    if (d <= 384) TQ_WIDE(128, 3, 128, 3, 128, 3);
+    if (d <= 512) TQ_WIDE(256, 2, 128, 4, 128, 4);
+    if (d <= 768) TQ_WIDE(256, 3, 128, 6, 128, 6);
+    TQ_WIDE(256, 4, 256, 4, 128, 8);
+#undef TQ_WIDE
 }
 RowsJob rows_job(const tq_plan* p, bool prod, const void* x, int xtype, int64_t n, uint32_t* codes, uint32_t* signs, float* rnorms,
                  float* norms, const TqRecheck* lists, unsigned long long* redo_counter, const TqRowMap* map) {
@@ -1023,14 +1047,30 @@ template <bool PROD>
 int launch_dequant_for(const tq_plan* p, const uint32_t* codes, const uint32_t* signs, const float* rnorms, const float* norms,
                        int64_t n, float* out, cudaStream_t st) {
     const int d = p->dev.d;
-    const bool many = n > (int64_t)tq_sm_count(p->device) * 32;
+    const int64_t sms = tq_sm_count(p->device);
+    // (64-row blocks on half the SMs are slower than 16-row blocks on all of them; d = 128, 8,000 rows: 20.6 / 24.3 us)
+    const bool many = n > sms * (d <= 96 ? 64 : d <= 128 ? 48 : 32);
 #define TQ_DQ(...) return launch_tile_dequant<PROD, __VA_ARGS__>(p, codes, signs, rnorms, norms, n, out, st)
     if (d <= 64) { if (many) TQ_DQ(16, 4, 8, 8); TQ_DQ(4, 4, 32, 2); }
     if (d <= 96) { if (many) TQ_DQ(16, 4, 8, 12); TQ_DQ(4, 4, 32, 3); }
     if (d <= 128) { if (many) TQ_DQ(16, 4, 16, 8); TQ_DQ(4, 4, 32, 4); }
-    if (d <= 256) { if (many) TQ_DQ(8, 4, 32, 8); TQ_DQ(2, 4, 64, 4); }
-    if (d <= 512) TQ_DQ(4, 4, 64, 8);
-    TQ_DQ(4, 4, 64, 16);
+    if (d <= 256) {
+        // blocks of 8 rows run two to an SM: where that leaves a last round of few blocks, 16 rows are faster (TurboQuantProd, d = 256:
+        // 2,000 rows 29 / 25 us, 3,000 rows 43 / 46, 4,736 rows 53 / 46)
+        if (many) TQ_DQ(8, 4, 32, 8);
+        if (n > 24 * sms || (n > 8 * sms && n <= 16 * sms)) TQ_DQ(4, 4, 64, 4);
+        TQ_DQ(2, 4, 64, 4);
+    }
+    const int block = wide_block_rows(d, n, sms);
+#define TQ_WIDE(C4, T4, C8, T8, C16, T16)      \
+    if (block == 4) TQ_DQ(1, 4, C4, T4);       \
+    if (block == 8) TQ_DQ(1, 8, C8, T8);       \
+    TQ_DQ(2, 8, C16, T16)
+    if (d <= 384) { TQ_WIDE(128, 3, 128, 3, 128, 3); }
+    if (d <= 512) { TQ_WIDE(256, 2, 128, 4, 128, 4); }
+    if (d <= 768) { TQ_WIDE(256, 3, 256, 3, 128, 6); }
+    TQ_WIDE(256, 4, 256, 4, 128, 8);
+#undef TQ_WIDE
 #undef TQ_DQ
 }
 }  // namespace

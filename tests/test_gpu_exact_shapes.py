@@ -73,3 +73,27 @@ def test_cache_step_in_one_launch_for_every_element_type(lib_built, d, groups, t
         assert torch.equal(have.view(groups, cap, -1)[:, :filled], want_k[name].view(groups, filled, -1)), name
     assert torch.equal(cache.value_codes.view(groups, cap, -1)[:, :filled], want_v["codes"].view(groups, filled, -1))
     assert torch.equal(cache.value_norms.view(groups, cap)[:, :filled], want_v["norms"].view(groups, filled))
+
+
+@pytest.mark.parametrize("d,bits,counts", [
+    (64, 6, (4737, 9473)), (96, 6, (4737, 9473)), (128, 6, (4737, 7105, 8289)), (200, 4, (1185, 2369, 3553, 4737)),
+    (300, 3, (592, 593, 1185, 2369)), (512, 4, (593, 1185, 2369)), (700, 3, (593, 1185)), (1024, 2, (593, 1185, 2369)),
+])
+def test_a_row_is_the_same_in_every_block_shape(lib_built, d, bits, counts):
+    """One chain of multiply-adds per output in every shape: the bytes of a row do not depend on the rows beside it."""
+    import torch
+    import project_tensor_b200 as tg
+    prod, mse = (make(d, bits, seed=2026, grid_size=4097, max_iter=64) for make in (tg.TurboQuantProd, tg.TurboQuantMSE))
+    x = torch.randn((max(counts), d), device="cuda", generator=torch.Generator("cuda").manual_seed(d))
+    for quant in (prod, mse):
+        quant.set_kernel_path("exact")
+        few = x[:3].contiguous(), x[-2:].contiguous()
+        want = [(tg.packed_buffers(e), quant.dequantize(e)) for e in map(quant.quantize, few)]
+        for n in counts:
+            batch = torch.cat([x[:3], x[:n - 5], x[-2:]])
+            enc = quant.quantize(batch)
+            restored, packed = quant.dequantize(enc), tg.packed_buffers(enc)
+            for part, (buffers, rows) in zip((slice(0, 3), slice(n - 2, n)), want):
+                assert torch.equal(restored[part], rows), (n, part)
+                for name, value in buffers.items():
+                    assert value is None or torch.equal(packed[name][part], value), (n, part, name)
