@@ -39,14 +39,11 @@ namespace {
 using namespace tqptx;
 
 constexpr int kTileRows = 128;
-// Warps: TMA, MMA, then the workers.  UNI (the kernels that run): 16 workers, four per row, each owning 32 columns of
-// its row through every phase of a tile -- conversion, first-accumulator epilogue and (TurboQuantProd) sign epilogue.
-// All workers walk the same code, so whichever phase the tensor pipe has finished finds warps to run it; with the
-// phases given to different warps (!UNI: converter warps and 8 epilogue warps, two per row; kept for comparison)
-// the issue slots were idle 44 % of the time although every warp had a backlog, because each role waited for the other.
-template <bool PROD, bool UNI> struct Threads {
-    static constexpr int kEpiPerRow = UNI ? 0 : 2;
-    static constexpr int kConvWarps = UNI ? 16 : (PROD ? 8 : 16);
+// Warps: TMA, MMA, then the workers: converter warps (TurboQuantProd: 8, which also run the sign epilogue; else 16) and 8 warps
+// for the first epilogue, two per row.
+template <bool PROD> struct Threads {
+    static constexpr int kEpiPerRow = 2;
+    static constexpr int kConvWarps = PROD ? 8 : 16;
     static constexpr int kFirstEpiWarp = 2 + kConvWarps;
     static constexpr int kThreads = (2 + kConvWarps + 4 * kEpiPerRow) * 32;
 };
@@ -101,7 +98,7 @@ __device__ __forceinline__ float2 widen_pair(uint32_t u, bool bf16) {
 // Shared-memory plan
 // ---------------------------------------------------------------------------------------------
 constexpr int kW = 128;   // width of the operand layouts in tensor and shared memory; d = 64 is zero-padded to it
-template <int D, bool PROD, bool UNI>
+template <int D, bool PROD>
 struct Smem {
     static constexpr int kBBytes = kW * kW * 2;                     // one fp16 operand matrix (padded)
     static constexpr int kNumB = PROD ? 4 : 2;
@@ -109,11 +106,11 @@ struct Smem {
     static constexpr int off_b = 0;
     static constexpr int off_ring = off_b + kNumB * kBBytes;
     static constexpr int off_misc = off_ring + kRingBoxes * kBoxBytes;  // sumsq exchange, force flags, barriers
-    static constexpr int kPendWarps = Threads<PROD, UNI>::kConvWarps + 4 * Threads<PROD, UNI>::kEpiPerRow;   // every worker warp
+    static constexpr int kPendWarps = Threads<PROD>::kConvWarps + 4 * Threads<PROD>::kEpiPerRow;   // every worker warp
                                                                 // stages entries: a 64-bit and a 32-bit list each
     static constexpr int kPendBytes = kPendWarps * kPendCap * (8 + 4);
-    static constexpr int kRsSlots = UNI ? 3 : 4;                 // tiles whose |rho|^2 partial sums are alive at once
-    static constexpr int kRsParts = UNI ? 4 : 2;                 // threads per row in the first epilogue
+    static constexpr int kRsSlots = 4;                 // tiles whose |rho|^2 partial sums are alive at once
+    static constexpr int kRsParts = 2;                 // threads per row in the first epilogue
     static constexpr int kRsBytes = kRsSlots * kRsParts * kTileRows * 4;
     static constexpr int kMiscBytes = 8 * kTileRows * 4 + 4 * kTileRows + 512 + kRsBytes + kCells * 16 + kPendBytes;
     static constexpr int total = off_misc + kMiscBytes + 1024;      // + slack to align the base to 1024
@@ -268,20 +265,20 @@ __device__ __noinline__ void pend_codes(const TqRecheck& l, WarpPending& w, uint
 }
 
 // HALF: rows of bf16 or fp16, widened (exactly) by the converters; a TMA box then holds 64 columns.
-template <int D, int BITS, bool PROD, bool UNI, bool HALF, bool MAPPED>
-__global__ void __launch_bounds__(Threads<PROD, UNI>::kThreads, 1)
+template <int D, int BITS, bool PROD, bool HALF, bool MAPPED>
+__global__ void __launch_bounds__(Threads<PROD>::kThreads, 1)
 tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorArgs a) {
     static_assert(D == 128 || D == 64, "this kernel is written for d = 128 and d = 64");
     // d = 64 runs in the layouts of d = 128 with the upper half of every row absent: the converter warps
     // and the epilogue warps of that half stay idle, the contractions stop after d / 16 k-blocks and cover
     // N = d output coordinates.
-    constexpr int kThreads = Threads<PROD, UNI>::kThreads;
-    constexpr int kFirstEpiWarp = Threads<PROD, UNI>::kFirstEpiWarp;
-    constexpr int kConvParts = Threads<PROD, UNI>::kConvWarps / 4;   // converter threads per row
+    constexpr int kThreads = Threads<PROD>::kThreads;
+    constexpr int kFirstEpiWarp = Threads<PROD>::kFirstEpiWarp;
+    constexpr int kConvParts = Threads<PROD>::kConvWarps / 4;   // converter threads per row
     constexpr int kXs = kW / kConvParts;                        // values a converter thread handles (64 or 32)
     constexpr int kActiveParts = D / kXs;                       // parts that have data (d = 64: half of them)
-    using L = Smem<D, PROD, UNI>;
-    constexpr int kEpiChunks = UNI ? 1 : 2;                     // 32-column chunks a thread owns in the first epilogue
+    using L = Smem<D, PROD>;
+    constexpr int kEpiChunks = 2;                     // 32-column chunks a thread owns in the first epilogue
     constexpr int kEpiParts = D / (32 * kEpiChunks);            // first-epilogue threads per row that have data
     constexpr int kSignChunks = kXs / 32;                       // chunks a thread owns in the sign epilogue
     constexpr int kBoxCols = HALF ? 64 : 32;                    // columns of a TMA box (128 bytes a row)
@@ -463,20 +460,18 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
         }
     } else {
         // ---- workers ------------------------------------------------------------------------------
-        // Roles of this warp: UNI: every role, on the 32 columns [32 * half, 32 * half + 32) of its rows; otherwise a
-        // converter warp (which also runs the sign epilogue of TurboQuantProd) or a first-epilogue warp.
-        const bool conv_role = UNI || warp < kFirstEpiWarp;
-        const bool epi_role = UNI || warp >= kFirstEpiWarp;
+        // A converter warp (which also runs the sign epilogue of TurboQuantProd) or a first-epilogue warp.
+        const bool conv_role = warp < kFirstEpiWarp;
         const int cw = warp - kFirstConvWarp;      // 0 .. workers-1
         const int half = cw >> 2;                  // converter: which kXs floats of the row
         const int quarter = warp & 3;              // TMEM lane quarter this warp may touch
         const int row = quarter * 32 + lane;
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
         constexpr int kCodeWords = D * BITS / 32;  // words per packed row
-        const int colgroup = UNI ? half : (warp - kFirstEpiWarp) >> 2;   // first epilogue: which kEpiChunks chunks of the row
+        const int colgroup = (warp - kFirstEpiWarp) >> 2;   // first epilogue: which kEpiChunks chunks of the row
         const int chunk0 = colgroup * kEpiChunks;
         const bool conv_active = conv_role && half < kActiveParts;      // d = 64: the warps of the absent columns idle
-        const bool epi_active = epi_role && colgroup < kEpiParts;
+        const bool epi_active = !conv_role && colgroup < kEpiParts;
         // lookup tables held in the lanes of the warp: per cell (boundary, boundaries below), per code (- centroid * 2^10)
         const float lut_bnd = cell_lut[lane].x;
         const int lut_base1 = __float_as_int(cell_lut[lane].y);   // boundaries below the cell = code of a value below its boundary
@@ -688,7 +683,7 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
             const uint32_t par2 = (uint32_t)((i >> 1) & 1);
             const int64_t grow = tile * kTileRows + row, orow = output_row<MAPPED>(a, grow);
             const bool live_row = grow < a.n;
-            TQ_PROF_CODE(const bool pr = a.prof && blockIdx.x == 0 && threadIdx.x == (UNI ? kFirstConvWarp : kFirstEpiWarp) * 32; long long c0 = clock64(), c1;)
+            TQ_PROF_CODE(const bool pr = a.prof && blockIdx.x == 0 && threadIdx.x == kFirstEpiWarp * 32; long long c0 = clock64(), c1;)
             const bool got = mbar_wait(BAR(BAR_ACC_FULL + b), par2, abort_flag);   // false: some role gave up, the
             const bool live = live_row && got;                                      // accumulator is not to be trusted
             tc_fence_after();
@@ -754,11 +749,9 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
                 TQ_PROF_CODE(if (pr) prof_acc[14] += clock64() - l0;)
                 // this thread's share of |rho|^2; summed in the sign epilogue of the same tile, which every worker reaches
                 // only after all of them have arrived on RHO_FULL below.  A slot is written again kRsSlots tiles later.
-                // !UNI, four slots: the warp of the other half may run ahead of this one (it needs MMA 1 of a later tile,
-                // not this warp's progress), but its first epilogue of tile i + 4 cannot start before every warp has
-                // finished the first epilogue of tile i + 2, which follows the sign epilogue of tile i.  UNI, three slots:
-                // the first epilogue of tile i + 3 follows the conversion of tile i + 4, which waits for the sign epilogue
-                // of tile i + 1 of every worker, and each worker runs that one after its sign epilogue of tile i.
+                // The warp of the other half may run ahead of this one (it needs MMA 1 of a later tile, not this warp's
+                // progress), but its first epilogue of tile i + 4 cannot start before every warp has finished the first
+                // epilogue of tile i + 2, which follows the sign epilogue of tile i.
                 rs_part[((int)(i % L::kRsSlots) * L::kRsParts + colgroup) * kTileRows + row] = rs;
             }
             tc_fence_before();
@@ -779,28 +772,7 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
             TQ_PROF_CODE(if (pr) prof_acc[17] += clock64() - c1;)
         };
 
-        if (UNI) {
-            // Per iteration: sign epilogue of tile it - 3, conversion of tile it, first epilogue of tile it - 1.  The tensor
-            // pipe runs the first contraction of tile it during the first epilogue of tile it - 1 and the second
-            // contraction of tile it - 1 during the next iteration's sign epilogue and conversion, so in steady state
-            // no phase finds its barrier unfinished.
-            const int64_t tiles = conv_active ? my_tiles : 0;
-            const int64_t iters = tiles > 0 ? tiles + (PROD ? 3 : 1) : 0;
-            for (int64_t it = 0; it < iters; ++it) {
-                if (PROD) {
-                    if (it >= 3) {
-                        sign_epilogue(it - 3);
-                    } else if (it == 2) {
-                        // A block 0 carries no second accumulator before tile 2 refills it; MMA 1 of tile 0 must have read it
-                        mbar_wait(BAR(BAR_ACC_FULL + 0), 0u, abort_flag);
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(BAR(BAR_A_EMPTY + 0));
-                    }
-                }
-                if (it < tiles) convert(it);
-                if (it >= 1 && it - 1 < tiles) epilogue1(it - 1);
-            }
-        } else if (conv_role) {
+        if (conv_role) {
             // TurboQuantProd: the converter warps also run the sign epilogue: they wait about half of every tile for a
             // free A block, while the epilogue warps are the longest chain of this variant.
             const int64_t conv_tiles = conv_active ? my_tiles : 0;
@@ -1451,18 +1423,11 @@ void tq_tensor_plan_free(tq_plan* p) {
     }
 }
 
-#ifndef TQ_UNI_PROD
-#define TQ_UNI_PROD false
-#endif
-#ifndef TQ_UNI_MSE
-#define TQ_UNI_MSE false
-#endif
 template <int D, int BITS, bool PROD, bool HALF, bool MAPPED>
 static int launch_type(const tq_plan* p, const CUtensorMap& map, const TensorArgs& args, int grid, cudaStream_t st) {
-    constexpr bool UNI = PROD ? TQ_UNI_PROD : TQ_UNI_MSE;
-    const int sm = Smem<D, PROD, UNI>::total;
-    TQ_GRANT_SMEM((tensor_quantize_kernel<D, BITS, PROD, UNI, HALF, MAPPED>), sm, p->device);
-    tensor_quantize_kernel<D, BITS, PROD, UNI, HALF, MAPPED><<<grid, Threads<PROD, UNI>::kThreads, sm, st>>>(map, args); tq_count_launch();
+    const int sm = Smem<D, PROD>::total;
+    TQ_GRANT_SMEM((tensor_quantize_kernel<D, BITS, PROD, HALF, MAPPED>), sm, p->device);
+    tensor_quantize_kernel<D, BITS, PROD, HALF, MAPPED><<<grid, Threads<PROD>::kThreads, sm, st>>>(map, args); tq_count_launch();
     TQ_CUDA_TRY(cudaGetLastError());
     return TQ_OK;
 }
