@@ -420,6 +420,10 @@ def packed_to_host(encoding, out: Optional[Dict[str, Any]] = None, wait: bool = 
     return host
 
 
+#: a last chunk of so few rows would be quantized by another kernel than the rest
+_SHORT_CHUNK_ROWS = 8192
+
+
 def quantize_to_host(quantizer, keys, chunk_rows: int = 131072, out: Optional[Dict[str, Any]] = None) -> Dict[str, Any]:
     """Quantize host-resident keys and leave the packed encoding in page-locked host tensors, for key sets
     that do not stay on the GPU (``quantizer`` is a TurboQuantMSE or TurboQuantProd, ``keys`` a NumPy
@@ -454,7 +458,8 @@ def quantize_to_host(quantizer, keys, chunk_rows: int = 131072, out: Optional[Di
     if n == 0:
         return host
     chunk_rows = max(1, min(int(chunk_rows), n))
-    chunk_rows = -(-n // -(-n // chunk_rows))    # chunks of one size: no short one at the end, which would take another kernel
+    if 0 < n % chunk_rows <= _SHORT_CHUNK_ROWS < chunk_rows:
+        chunk_rows = -(-n // -(-n // chunk_rows))    # chunks of one size
     with torch.cuda.device(device):
         s_in, s_run, s_out = torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.Stream()
         for s_ in (s_in, s_run, s_out):
