@@ -222,6 +222,24 @@ def run_reference(args):
     }))
 
 
+#: what the one line on stdout holds; everything else goes to stderr, so that a reader that keeps the end of the output gets it whole
+_LINE = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling", "vs_baseline", "dtype", "data",
+         "config", "attention_score", "search_ms", "roofline", "e2e", "gpu_launches", "clocks", "cpu_baseline")
+_PARTS = {"attention_score": ("value", "unit", "queries", "ms"), "roofline": ("bound", "achieved", "peak", "unit", "frac", "kernel_ms"),
+          "e2e": ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step"), "cpu_baseline": ("value", "unit", "cores", "kind")}
+
+
+def emit(line):
+    """The details on stderr as one JSON line, then the short line on stdout."""
+    sys.stderr.write("details " + json.dumps(line) + "\n")
+    sys.stderr.flush()
+    short = {k: line[k] for k in _LINE if k in line}
+    for name, keys in _PARTS.items():
+        if isinstance(short.get(name), dict):
+            short[name] = {k: short[name][k] for k in keys if k in short[name]}
+    print(json.dumps(short))
+
+
 def parity_report(quant, keys_dev, queries_dev, n):
     """Differences between the CUDA path and the NumPy oracle on the first `n` keys of this run: packed codes and QJL
     signs (counts, rate, how many lie outside the 1e-5 window of their decision point), norms, residual norms and
@@ -604,7 +622,7 @@ def run_gpu(args):
                 "attention_score_Gkeys_per_s": n_sample / (cs * N_QUERIES) / 1e9,
                 "sample": f"NumPy oracle, quantize {n_sample} of {N_KEYS} keys (best of 3); scoring 1 query x {n_sample} "
                           f"keys (best of 2) multiplied by {N_QUERIES} queries"}
-        print(json.dumps(line))
+        emit(line)
     if world > 1:
         dist.destroy_process_group()
 
@@ -823,7 +841,8 @@ def retrieval(tg, torch, dev, n_total, steps, warmup, peak, oracle_chunk):
         "search_Gpairs_per_s": n_total * n_q / (search_ms * 1e-3) / 1e9,
         "roofline": {"bound": "hbm", "achieved": search_gbs / world, "peak": peak, "unit": "GB/s", "frac": search_gbs / peak / world,
                      "bytes_per_key": kb, "traffic": None,
-                     "note": "per GPU; 64 queries cost 5 x 2 x 128 x 64 = 82 KFLOP of tensor work per 72-byte key, so the contractions bound this call, not HBM"},
+                     "note": "per GPU; the first stage costs 64 queries 2 x 2 x 128 x 64 = 33 KFLOP of tensor work per 72-byte key and some 1,400 cycles of "
+                             "expander instructions per 128 keys, which bound it"},
         "e2e": {"value": n_total / (e2e_ms * 1e-3) / 1e9, "unit": "Gkeys/s", "ms": e2e_ms,
                 "h2d_bytes_per_step": n_q * D * 4, "d2h_bytes_per_step": n_q * k * 12,
                 "what": "ShardedKeyIndex.search(NumPy queries) -> global top-100 copied to the host; packed keys resident"},
@@ -858,7 +877,7 @@ def run_retrieval(args):
             line["cpu_baseline"] = {"value": n_sample / (cs * 64) / 1e9, "unit": "Gkeys/s", "cores": host_threads(), "kind": "port",
                                     "quantize_Mvec_per_s": n_sample / cq / 1e6,
                                     "sample": f"NumPy oracle: one query x {n_sample} keys (best of 2) multiplied by 64 queries; no top-k pass"}
-        print(json.dumps(line))
+        emit(line)
     if world > 1:
         dist.destroy_process_group()
     if not all(v for v in res["checks"].values() if isinstance(v, bool)):
