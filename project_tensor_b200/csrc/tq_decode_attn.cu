@@ -38,7 +38,7 @@
 // over blocks; every block leaves (max, sum, accumulator) per query in scratch and decode_combine_kernel merges.
 //
 // The kernel this replaced scored from per-query lookup tables and accumulated values with one multiply-add per key,
-// coordinate and query: 64 groups x 4 queries x 32,768 keys (d = 128, 2 + 1 bit keys, 4-bit values) took 260 us, now 149.
+// coordinate and query: 64 groups x 4 queries x 32,768 keys (d = 128, 2 + 1 bit keys, 4-bit values) took 273 us, now 165.
 #include "tq_common.cuh"
 #include "tq_mma.cuh"
 

@@ -16,10 +16,9 @@
 // chain: 3 to 12 % more error than the multiply-adds of the table kernel, two: 10 to 40 % less).
 //
 // Bound: shared-memory lookups, 64 8-byte loads a key at d = 128 and 3-bit codes (2 cycles a warp and load, four lanes a key), and for
-// few keys the prologue.  Before -- one thread per key through tables of the query's own products, whose random rows met
-// in banks (another kernel for three or four queries) -- 2,000,000 keys of d = 128, 3-bit codes and one query took 71 us, now 66;
-// 262,147 keys 23, now 15.5.  (With signs as bits where they stand 1,048,576 keys took 35 us for one query and 36 for four, 40
-// and 84 before; +-1 costs some 8 % of that and gives a four times smaller error.)
+// few keys the prologue.  d = 128, 3-bit codes, one query: 262,144 keys 15.6 us (tables of the query's own products, a thread per
+// key: 19), 1,024 keys 7.0 (9.4); four queries x 1,048,576 keys 41 (84 in the table kernel for four queries that this one replaced).
+// Where tables are the faster way (very many keys, very many groups): tq_score_table.cu.
 #include "tq_common.cuh"
 #include "tq_mma.cuh"
 
