@@ -29,10 +29,6 @@ def _widen(staged):
     return staged
 
 
-def _off_boundary(staged) -> bool:
-    return staged is not None and staged.tensor.element_size() == 2 and staged.tensor.data_ptr() % 16 != 0
-
-
 class PackedKeyCache:
     """Packed TurboQuantProd keys of ``groups`` sequences, ``capacity`` rows each, all of one length."""
 
@@ -105,13 +101,14 @@ class PackedKeyCache:
         vstaged, vplans, vcodes, vnorms = values or (None, None, None, None)
         rows = self.groups * tokens
         bulk = rows > self.SMALL_APPEND_ROWS
+        x, v = staged.tensor.data_ptr(), vstaged.tensor.data_ptr() if values else None
         # 16-bit rows are widened first where the kernels do not take them as they are: the bulk kernel of d = 256 reads float32 only,
         # and the rows have to start on a 16-byte boundary (a view of a larger tensor need not)
-        if bulk and self.quantizer.dimension == 256 or any(_off_boundary(s) for s in (staged, vstaged)):
+        if (bulk and self.quantizer.dimension == 256) or ((x | (v or 0)) % 16 and staged.tensor.element_size() == 2):
             staged, vstaged = _widen(staged), _widen(vstaged) if values else None
+            x, v = staged.tensor.data_ptr(), vstaged.tensor.data_ptr() if values else None
         kh, vh = self._plans.handle(dev), vplans.handle(dev) if values else None
-        args = (kh, vh, staged.tensor.data_ptr(), vstaged.tensor.data_ptr() if values else None,
-                _tq._dtype_code(staged.tensor), self.groups, tokens, self.codes.data_ptr(), self.signs.data_ptr(),
+        args = (kh, vh, x, v, _tq._dtype_code(staged.tensor), self.groups, tokens, self.codes.data_ptr(), self.signs.data_ptr(),
                 self.residual_norms.data_ptr(), self.norms.data_ptr(), vcodes.data_ptr() if values else None,
                 vnorms.data_ptr() if values else None, self.capacity)
         if bulk:

@@ -372,11 +372,11 @@ def _row_shape(rows: int, prefix) -> Tuple[int, ...]:
     """Shape to allocate the results of ``rows`` rows in: ``prefix`` when it holds them as it stands, else flat -- the field
     ``prefix_shape`` can be edited, and ``reshape`` then says what it makes of it (a -1 in it, or no such shape)."""
     prefix = tuple(prefix)
-    return prefix if math.prod(prefix) == rows and min(prefix, default=0) >= 0 else (rows,)
+    return prefix if math.prod(prefix) == rows and (len(prefix) < 2 or min(prefix) >= 0) else (rows,)
 
 
 def _in_shape(result, shape):
-    return result if tuple(result.shape) == shape else result.reshape(shape)
+    return result if result.shape == shape else result.reshape(shape)
 
 
 def _encoding_from_packed(cls, pk: _Packed, prefix):
