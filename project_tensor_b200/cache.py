@@ -102,9 +102,9 @@ class PackedKeyCache:
         rows = self.groups * tokens
         bulk = rows > self.SMALL_APPEND_ROWS
         x, v = staged.tensor.data_ptr(), vstaged.tensor.data_ptr() if values else None
-        # 16-bit rows are widened first where the kernels do not take them as they are: the bulk kernel of d = 256 reads float32 only,
+        # 16-bit rows are widened first where the kernels do not take them as they are: the bulk kernels of d = 96 and 256 read float32 only,
         # and the rows have to start on a 16-byte boundary (a view of a larger tensor need not)
-        if (bulk and self.quantizer.dimension == 256) or ((x | (v or 0)) % 16 and staged.tensor.element_size() == 2):
+        if (bulk and self.quantizer.dimension in (96, 256)) or ((x | (v or 0)) % 16 and staged.tensor.element_size() == 2):
             staged, vstaged = _widen(staged), _widen(vstaged) if values else None
             x, v = staged.tensor.data_ptr(), vstaged.tensor.data_ptr() if values else None
         kh, vh = self._plans.handle(dev), vplans.handle(dev) if values else None

@@ -68,7 +68,7 @@ bool use_tensor(const tq_plan* p, int* err) {
         *err = tq_fail(TQ_ERR_UNSUPPORTED, "no tensor-core kernel for d=%d bits=%d", p->dev.d, p->dev.bits);
         return false;
     }
-    return p->tensor_ok;
+    return p->tensor_ok || p->path == TQ_PATH_AUTO && p->tensor;
 }
 }  // namespace
 
@@ -243,7 +243,8 @@ int tq_plan_create(int d, int bits_mse, const float* rotation, const float* code
     }
 
     p->tensor_ok = false;
-    if (tq_tensor_quantize_supported(d, bits_mse, projection != nullptr)) {
+    const bool wide = tq_tensor_wide_supported(d, bits_mse, projection != nullptr);
+    if (wide || tq_tensor_quantize_supported(d, bits_mse, projection != nullptr)) {
         const int r = tq_tensor_plan_init(p, rotation, codebook, projection);
         if (r != TQ_OK) {
             cudaFreeHost(word);
@@ -251,9 +252,9 @@ int tq_plan_create(int d, int bits_mse, const float* rotation, const float* code
             delete p;
             return r;
         }
-        p->tensor_ok = p->tensor != nullptr;
+        p->tensor_ok = p->tensor != nullptr && !wide;
     }
-    if (p->tensor_ok && tq_dequant_tc_supported(d, bits_mse, projection != nullptr)) {
+    if ((p->tensor || d == 96) && tq_dequant_tc_supported(d, bits_mse, projection != nullptr)) {
         const int r = tq_dequant_tc_plan_init(p, rotation, projection);
         if (r != TQ_OK) {
             tq_tensor_plan_free(p);
@@ -310,7 +311,16 @@ int64_t tq_topk_scratch_bytes(const tq_plan* p, int groups, int q_per_group, int
 // Up to 32 rows per SM the reference-order kernel alone is faster than the tensor-core kernel with its second stage
 // (four operations on the stream): TurboQuantProd, 2,048 rows: d = 64 10 against 28 us, d = 128 18 against 38, d = 256
 // 43 against 84; 8,192 rows: 23 / 34, 44 / 45, 121 / 84.
-static bool few_rows(const tq_plan* p, int64_t n) { return p->path == TQ_PATH_AUTO && n <= 32 * (int64_t)tq_sm_count(p->device); }
+// d = 96 and the codes of 5 and 6 bits, whose second stage has more to do: TurboQuantProd, 8,000 rows, 31 against 35 us (d = 96, 6
+// bits), 33 / 51 (d = 128), at d = 64 31 / 23 and from 12,000 rows on 27 / 31; TurboQuantMSE, 8,000 and 12,000 rows, 23 / 19 and 23 / 27
+// (d = 96, 4 bits), 27 / 27 and 29 / 39 (d = 128, 6 bits), 21 / 14 and 21 / 21 (d = 64).
+static bool few_rows(const tq_plan* p, bool prod, int64_t n) {
+    const int d = p->dev.d, per_sm = p->tensor_ok ? 32 : d == 64 ? 80 : d == 96 && !prod ? 64 : 48;
+    return p->path == TQ_PATH_AUTO && n <= per_sm * (int64_t)tq_sm_count(p->device);
+}
+// The reference-order dequantizer instead of the tensor-core one of the same plans, which takes 8 to 12 us however few the rows are
+// (4,700 rows: 6 to 8 against 8 to 10 us; 6,000 rows: equal).
+static bool few_restored(const tq_plan* p, int64_t n) { return !p->tensor_ok && n <= 36 * (int64_t)tq_sm_count(p->device); }
 
 // The lists of one call in the caller's scratch, behind its header.
 static unsigned char* place_lists(TqRecheck* l, TqRecheckHeader* hdr, unsigned char* at, int64_t n) {
@@ -339,7 +349,7 @@ static int quantize_common(const tq_plan* p, bool prod, const float* x, int64_t 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int err = TQ_OK;
     const TqQuantOut out{static_cast<uint32_t*>(codes), static_cast<uint32_t*>(signs), rnorms, norms, TqRowMap{}};
-    if (!few_rows(p, n) && use_tensor(p, &err)) {
+    if (!few_rows(p, prod, n) && use_tensor(p, &err)) {
         const int64_t need = tq_quantize_scratch_bytes(p, n);
         if (!scratch || (int64_t)scratch_bytes < need)
             return tq_fail(TQ_ERR_SCRATCH_TOO_SMALL, "quantize scratch: need %lld bytes, got %zu", (long long)need, scratch_bytes);
@@ -360,7 +370,7 @@ static int quantize_common(const tq_plan* p, bool prod, const float* x, int64_t 
     if (err != TQ_OK) return err;
     // (a plan with tensor-core kernels counts the rows of this kernel, all of them here)
     return tq_launch_exact_quantize(p, prod, x, TQ_F32, n, out.codes, out.signs, rnorms, norms,
-                                    p->path == TQ_PATH_AUTO && p->tensor_ok ? p->counters : nullptr, st);
+                                    p->path == TQ_PATH_AUTO && p->tensor ? p->counters : nullptr, st);
 }
 
 int tq_mse_quantize(const tq_plan* p, const float* x, int64_t n, void* codes, float* norms, void* scratch,
@@ -469,7 +479,7 @@ int tq_kv_prefill(const tq_plan* kp, const tq_plan* vp, const void* keys, const 
     for (int i = 0; i < njobs; ++i) {
         int err = TQ_OK;
         const tq_plan* p = jobs[i].plan;
-        whole[i] = few_rows(p, rows) || !use_tensor(p, &err) || !tq_tensor_input_supported(p->dev.d, dtype);
+        whole[i] = few_rows(p, jobs[i].prod, rows) || !use_tensor(p, &err) || !tq_tensor_input_supported(p->dev.d, dtype);
         if (err != TQ_OK) return err;
         if (!whole[i]) tensor[ntensor++] = jobs[i];
     }
@@ -533,7 +543,7 @@ int tq_mse_dequantize(const tq_plan* p, const void* codes, const float* norms, i
     DeviceScope scope(p->device);
     // the tensor-core kernel when the plan has one (within ~1e-7 relative of the reference arithmetic); the
     // exact kernel reproduces the reference bit for bit and serves every other geometry and the EXACT path
-    if (p->path != TQ_PATH_EXACT && p->dequant)
+    if (p->path != TQ_PATH_EXACT && p->dequant && !few_restored(p, n))
         return tq_launch_dequant_tc(p, false, static_cast<const uint32_t*>(codes), nullptr, nullptr, norms, n, out,
                                     static_cast<cudaStream_t>(stream));
     return tq_launch_exact_dequantize(p, false, static_cast<const uint32_t*>(codes), nullptr, nullptr, norms, n, out,
@@ -551,7 +561,7 @@ int tq_prod_dequantize(const tq_plan* p, const void* codes, const void* signs, c
     TQ_TRY(check_ptr(norms, "norms"));
     TQ_TRY(check_ptr(out, "out"));
     DeviceScope scope(p->device);
-    if (p->path != TQ_PATH_EXACT && p->dequant)
+    if (p->path != TQ_PATH_EXACT && p->dequant && !few_restored(p, n))
         return tq_launch_dequant_tc(p, true, static_cast<const uint32_t*>(codes), static_cast<const uint32_t*>(signs),
                                     residual_norms, norms, n, out, static_cast<cudaStream_t>(stream));
     return tq_launch_exact_dequantize(p, true, static_cast<const uint32_t*>(codes), static_cast<const uint32_t*>(signs),
@@ -586,7 +596,7 @@ int tq_score_pairwise(const tq_plan* p, const float* q, const void* codes, const
     DeviceScope scope(p->device);
     // q[i] . dequantize(key i) on the tensor-core dequantize kernel where the plan has one; the exact kernel
     // (reference order of operations) otherwise and on the EXACT path
-    if (p->path != TQ_PATH_EXACT && p->dequant && p->dev.d != 256)      // d = 256: no pair form of the streaming kernel
+    if (p->path != TQ_PATH_EXACT && p->dequant && p->tensor_ok && p->dev.d != 256)      // d = 256: no pair form of the streaming kernel
         return tq_launch_pairwise_tc(p, q, static_cast<const uint32_t*>(codes), static_cast<const uint32_t*>(signs),
                                      residual_norms, norms, n, scores, static_cast<cudaStream_t>(stream));
     return tq_launch_exact_pairwise(p, q, static_cast<const uint32_t*>(codes), static_cast<const uint32_t*>(signs),

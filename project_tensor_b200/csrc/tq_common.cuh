@@ -23,6 +23,11 @@ enum { TQ_INPUT_F32 = TQ_F32, TQ_INPUT_BF16 = TQ_BF16, TQ_INPUT_F16 = TQ_F16 };
 // Same idea for the QJL projection, whose sign is taken at zero.
 #define TQ_SIGN_GUARD 4.0e-6f
 
+// The tensor pipe truncates a sum to fp32 at every instruction, half a unit in the last place of it on average: a relative
+// 0.5 * 2^-23 * E[1 / mantissa] = 4.3e-8 (mantissas spread evenly over their logarithm: 1 / (2 ln 2)).  A term that is in the sum for
+// `steps` further instructions (a term of a chain of n on average for n / 2) loses this share; an operand is made that much larger.
+inline double tq_truncation_loss(double steps) { return steps * 4.3e-8; }
+
 // Work lists that the tensor-core quantizers leave in the caller's scratch buffer for the exact
 // second stage.  Layout of the scratch: this header (64 bytes), then `code_cap` 64-bit entries
 // (row << 8 | coordinate: a rotated coordinate inside the guard band of a boundary), then `row_cap`
@@ -107,7 +112,7 @@ struct tq_plan {
     int device;
     int path;
     bool has_projection;
-    bool tensor_ok;          // tensor-core kernels cover this (d, bits)
+    bool tensor_ok;          // tensor-core kernels cover this (d, bits); where `tensor` alone is set, the quantizers do (tq_tensor_wide_supported)
     void* slab;              // one device allocation holding every constant
     TensorConsts* tensor;    // host-side bookkeeping for the tensor-core kernels (may be null)
     DequantConsts* dequant;  // operand matrices of the tensor-core dequantize kernels (may be null)
@@ -214,6 +219,7 @@ int tq_launch_exact_pairwise(const tq_plan* p, const float* q, const uint32_t* c
 // Tensor-core (tcgen05) kernels.
 bool tq_tensor_supported(int d, int bits);
 bool tq_tensor_quantize_supported(int d, int bits, bool has_projection);
+bool tq_tensor_wide_supported(int d, int bits, bool has_projection);
 int tq_tensor_plan_init(tq_plan* p, const float* rotation, const float* codebook, const float* projection);
 void tq_tensor_plan_free(tq_plan* p);
 bool tq_tensor_input_supported(int d, int xtype);

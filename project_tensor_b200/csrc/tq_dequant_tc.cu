@@ -1,4 +1,4 @@
-// Tensor-core dequantize for d = 128 on B200: TurboQuantMSE.dequantize and TurboQuantProd.dequantize
+// Tensor-core dequantize on B200 (d = 64, 96 and 128; d = 256 below): TurboQuantMSE.dequantize and TurboQuantProd.dequantize
 // (_quant.py:238-242,251-254 and 317-332).
 //
 //   MSE :  x~ = norm * ( codebook[codes] . R )
@@ -13,12 +13,18 @@
 //   bulk copy (1 thread)   packed codes (and sign words) of 128 keys -> smem ring
 //   expanders (8 warps)    one thread per half key: codes -> (hi, lo) half2 pairs through a lane-replicated
 //                          pair lookup table, signs -> +-beta pairs; tcgen05.st into a ring of four
-//                          64-column operand slots in tensor memory (C_hi, C_lo [, B_hi, B_lo] of
-//                          successive tiles)
-//   MMA (1 thread)         operand by operand: C_hi x (Rt_hi, Rt_lo), C_lo x Rt_hi [, B_hi x (St_hi, St_lo),
-//                          B_lo x St_hi], N = 128, accumulators double-buffered
+//                          64-column operand slots in tensor memory (of successive tiles)
+//   MMA (1 thread)         N = d, accumulators double-buffered.  The tensor pipe truncates a sum at every instruction by a
+//                          share of what it holds, so the products with a lo part come first: [B_lo x St_hi,] C_lo x Rt_hi,
+//                          [B_hi x St_lo,] C_hi x Rt_lo, [B_hi x St_hi,] C_hi x Rt_hi.  TurboQuantProd of up to 3 code bits at
+//                          d = 64 and 128 goes operand by operand, centroids first: 1,048,576 keys at d = 128 184 against 234 us
 //   epilogue (8 warps)     two threads per key: tcgen05.ld, times norm * 2^-20, then through a staging block in
 //                          shared memory so that every global store instruction writes whole 128-byte lines
+//
+// What is left of the truncation is its mean, which the lo parts of the operands make up for (set_losses).  Reconstructions against
+// 64 bits (2-norm): TurboQuantMSE at 4 bits, d = 64 and 128, 0.9 and 1.3e-7 (3.0 and 6.2e-7 with every k-block's three products in
+// turn, 1.5 and 2.0e-7 in the reference's order); d = 96 1.2 to 1.4e-7 (reference order 1.8e-7), where 50,021 TurboQuantProd keys
+// of 5 code bits take 18 us instead of 70.
 //
 // Every wait is bounded; a wait that runs out sets the plan's status word and the kernel drains.
 #include "tq_common.cuh"
@@ -33,7 +39,7 @@ namespace {
 
 using namespace tqptx;
 
-constexpr int D = 128;   // width of the operand layouts; vectors of d = 64 use their lower half
+constexpr int D = 128;   // width of the operand layouts; vectors of d = 64 and 96 use their lower columns
 constexpr int kTileKeys = 128;
 constexpr int kFirstExpWarp = 2;
 constexpr int kFirstEpiWarp = 10;
@@ -54,6 +60,7 @@ struct DequantArgs {
     const unsigned char* bmat;   // [Rt_hi | Rt_lo | St_hi | St_lo], interleaved core-matrix layout
     const float* codebook;
     float alpha;
+    float c_loss, b_loss;        // what the truncation of the sums takes from the centroids' and the signs' part (tq_truncation_loss)
     int64_t n, ntiles;
     float* out;                  // reconstructions [n][d]; or, in pair mode, scores [n]
     const float* pair_q;         // pair mode: one query row per key, [n][d]
@@ -120,10 +127,22 @@ struct BlockStore {
 
 __device__ __forceinline__ void tmem_ld32_(uint32_t taddr, uint32_t (&v)[32]) { tmem_ld32(taddr, v); }
 
+// The operands of a tile in the order in which they pass through the slots.
+enum { C_HI, C_LO, B_HI, B_LO };
+template <bool PROD, bool SMALL_FIRST>
+constexpr __host__ __device__ int operand_at(int op) {
+    if (!PROD) return op == 0 ? C_LO : C_HI;
+    return SMALL_FIRST ? (op == 0 ? B_LO : op == 1 ? C_LO : op == 2 ? B_HI : C_HI) : (op == 0 ? C_HI : op == 1 ? C_LO : op == 2 ? B_HI : B_LO);
+}
+// TurboQuantProd goes operand by operand where the pair table serves it at d = 64 and 128.
+constexpr __host__ __device__ bool small_first(int d, int bits, bool prod) { return !prod || d == 96 || bits > 3; }
+
 template <int BITS, bool PROD, int DR>
 struct DqSmem {
-    static constexpr int kLutEntries = 1 << (2 * BITS);
-    static constexpr int kLutBytes = kLutEntries * 32 * 8;
+    // pairs of codes; one code at a time where that table would not fit beside the matrices
+    static constexpr bool kPairLut = BITS <= (PROD ? 3 : 4);
+    static constexpr int kLutEntries = 1 << (kPairLut ? 2 * BITS : BITS);
+    static constexpr int kLutBytes = kLutEntries * 32 * (kPairLut ? 8 : 4);
     static constexpr int kCodeRowBytes = DR * BITS / 8;
     static constexpr int kSignRowBytes = DR / 8;
     static constexpr int kRowExtra = PROD ? kSignRowBytes : 0;   // sign words
@@ -147,13 +166,16 @@ struct DqSmem {
 template <int BITS, bool PROD, int DR, bool PAIR>
 __global__ void __launch_bounds__(kThreads, 1)
 dequant_tc_kernel(const DequantArgs a) {
-    static_assert(DR == 128 || DR == 64, "written for d = 128 and d = 64");
-    // d = 64: the expander warps and the epilogue warps of the upper half idle, the contractions stop after
-    // DR / 16 k-blocks and cover N = DR output coordinates
-    constexpr int kHalves = DR / 64;
+    static_assert(DR == 128 || DR == 96 || DR == 64, "written for d = 64, 96 and 128");
+    static_assert(!PAIR || DR != 96, "no pair form at d = 96");
+    // d = 64 and 96: the expander warps and the epilogue warps of the upper half idle (d = 96: have 32 coordinates instead of
+    // 64), the contractions stop after DR / 16 k-blocks and cover N = DR output coordinates
+    constexpr int kHalves = (DR + 63) / 64;
+    constexpr bool kPartial = DR % 64 != 0;
     using L = DqSmem<BITS, PROD, DR>;
     constexpr int kStages = L::kStages;
-    constexpr int kOps = PROD ? 4 : 2;   // operands per tile: C_hi, C_lo [, B_hi, B_lo]
+    constexpr int kOps = PROD ? 4 : 2;   // operands per tile
+    constexpr bool kSmallFirst = small_first(DR, BITS, PROD);
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
     const uint32_t smem_base = smem_u32(smem);
@@ -174,16 +196,22 @@ dequant_tc_kernel(const DequantArgs a) {
     }
     {   // pair lookup table: entry e = (code0 | code1 << BITS) -> (half2 hi(c0), hi(c1)), (half2 lo(c0), lo(c1)),
         // one copy per lane so that the lookups of a warp never collide on a bank
+        // (one code at a time: hi in the low half of a word, lo in the high half)
         uint2* lut = reinterpret_cast<uint2*>(smem + L::off_lut);
         for (int i = threadIdx.x; i < L::kLutEntries * 32; i += kThreads) {
             const int e = i >> 5;
+            if (!L::kPairLut) {
+                const float c = __ldg(a.codebook + e) * kCentScale;
+                reinterpret_cast<uint32_t*>(lut)[i] = pack_half2(c, fmaf(c, a.c_loss, c - __half2float(__float2half_rn(c))));
+                continue;
+            }
             const float c0 = __ldg(a.codebook + (e & ((1 << BITS) - 1))) * kCentScale;
             const float c1 = __ldg(a.codebook + (e >> BITS)) * kCentScale;
             const __half2 h = __floats2half2_rn(c0, c1);
             const float2 hf = __half22float2(h);
             uint2 v;
             v.x = *reinterpret_cast<const uint32_t*>(&h);
-            v.y = pack_half2(c0 - hf.x, c1 - hf.y);
+            v.y = pack_half2(fmaf(c0, a.c_loss, c0 - hf.x), fmaf(c1, a.c_loss, c1 - hf.y));
             lut[i] = v;
         }
     }
@@ -261,25 +289,52 @@ dequant_tc_kernel(const DequantArgs a) {
                 if (!warp_wait(BAR(DB_D_EMPTY + b), par2 ^ 1u, abort_flag)) break;
                 const uint32_t acc = tm + kColD + b * D;
                 bool ok = true;
+                uint32_t held = 0;                                // B_hi, between its two products
+                (void)held;
 #pragma unroll
-                for (int op = 0; op < kOps; ++op) {              // 0: C_hi, 1: C_lo, 2: B_hi, 3: B_lo
+                for (int op = 0; op < kOps; ++op) {
                     const int64_t n = (int64_t)kOps * i + op;
                     const int slot = (int)(n & (kSlots - 1));
                     if (!warp_wait(BAR(DB_A_FULL + slot), (uint32_t)((n / kSlots) & 1), abort_flag)) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t aop = tm + slot * kSlotCols;
-                    const uint64_t bh = op < 2 ? d_rhi : d_shi, bl = op < 2 ? d_rlo : d_slo;
-                    if (elect_one()) {
-                        if (op == 0) mma_ts_first(acc, aop, bh, kIdesc); else mma_ts_acc(acc, aop, bh, kIdesc);
-                        if ((op & 1) == 0) mma_ts_acc(acc, aop, bl, kIdesc);   // hi operand also meets the lo matrix
-#pragma unroll 1
-                        for (int kb = 1; kb < DR / 16; ++kb) {
-                            // the start-address field counts 16-byte units: one k-block (two core matrices) further
-                            const uint64_t step = (uint64_t)(kb * 2 * lbo >> 4);
-                            mma_ts_acc(acc, aop + kb * 8, bh + step, kIdesc);
-                            if ((op & 1) == 0) mma_ts_acc(acc, aop + kb * 8, bl + step, kIdesc);
+                    // (the start-address field counts 16-byte units: a k-block is two core matrices)
+                    constexpr uint64_t kStep = 2 * 128 >> 4;
+                    if constexpr (kSmallFirst) {
+                        auto run = [&](uint32_t at, uint64_t mat, bool first) {
+                            if (first) mma_ts_first(acc, at, mat, kIdesc);
+#pragma unroll
+                            for (int kb = first ? 1 : 0; kb < DR / 16; ++kb) mma_ts_acc(acc, at + kb * 8, mat + kb * kStep, kIdesc);
+                        };
+                        if (elect_one()) {
+                            switch (operand_at<PROD, kSmallFirst>(op)) {
+                                case B_LO: run(aop, d_shi, true); break;
+                                case C_LO: run(aop, d_rhi, !PROD); break;
+                                case B_HI: run(aop, d_slo, false); break;
+                                default:
+                                    run(aop, d_rlo, false);
+                                    if (PROD) {
+                                        run(held, d_shi, false);
+                                        mma_commit(BAR(DB_A_EMPTY + (int)((n - 1) & (kSlots - 1))));
+                                    }
+                                    run(aop, d_rhi, false);
+                                    break;
+                            }
+                            if (operand_at<PROD, kSmallFirst>(op) != B_HI) mma_commit(BAR(DB_A_EMPTY + slot));
                         }
-                        mma_commit(BAR(DB_A_EMPTY + slot));
+                        held = aop;
+                    } else {
+                        const uint64_t bh = op < 2 ? d_rhi : d_shi, bl = op < 2 ? d_rlo : d_slo;
+                        if (elect_one()) {
+                            if (op == 0) mma_ts_first(acc, aop, bh, kIdesc); else mma_ts_acc(acc, aop, bh, kIdesc);
+                            if ((op & 1) == 0) mma_ts_acc(acc, aop, bl, kIdesc);   // hi operand also meets the lo matrix
+#pragma unroll 1
+                            for (int kb = 1; kb < DR / 16; ++kb) {
+                                mma_ts_acc(acc, aop + kb * 8, bh + kb * kStep, kIdesc);
+                                if ((op & 1) == 0) mma_ts_acc(acc, aop + kb * 8, bl + kb * kStep, kIdesc);
+                            }
+                            mma_commit(BAR(DB_A_EMPTY + slot));
+                        }
                     }
                     __syncwarp();
                 }
@@ -297,6 +352,8 @@ dequant_tc_kernel(const DequantArgs a) {
         const uint2* lut_lane = reinterpret_cast<const uint2*>(smem + L::off_lut) + lane;
         constexpr int kHalfWords = 2 * BITS;  // code words of 64 coordinates
         constexpr uint32_t kPairMask = (1u << (2 * BITS)) - 1u;
+        const uint32_t* one_lane = reinterpret_cast<const uint32_t*>(smem + L::off_lut) + lane;
+        const int blocks = kPartial && half == kHalves - 1 ? 1 : 2;      // blocks of 32 coordinates of this thread
         // residual norm of this thread's key, fetched a tile ahead of its use (Prod)
         float rn_next = 0.f;
         if (PROD && my_tiles > 0) {
@@ -316,37 +373,53 @@ dequant_tc_kernel(const DequantArgs a) {
                 const unsigned char* stage = smem + L::off_ring + s * L::kStageBytes;
                 const volatile uint32_t* cw = reinterpret_cast<const volatile uint32_t*>(stage + row * L::kCodeRowBytes) + half * kHalfWords;
 #pragma unroll
-                for (int k = 0; k < kHalfWords; ++k) w[k] = fail ? 0u : cw[k];
+                for (int k = 0; k < kHalfWords; ++k) w[k] = fail || (kPartial && k >= blocks * BITS) ? 0u : cw[k];
                 w[kHalfWords] = 0;
                 if (PROD) {
                     const volatile uint32_t* sg = reinterpret_cast<const volatile uint32_t*>(stage + kTileKeys * L::kCodeRowBytes + row * L::kSignRowBytes) + half * 2;
                     sw[0] = fail ? 0u : ~sg[0];   // a set bit now means a negative sign
-                    sw[1] = fail ? 0u : ~sg[1];
+                    sw[1] = fail || (kPartial && blocks == 1) ? 0u : ~sg[1];
                 }
             }
             __threadfence_block();   // every lane's loads from the stage are performed before the stage is released
             __syncwarp();
             if (lane == 0 && !fail) mbar_arrive(BAR(DB_K_EMPTY + s));
             uint32_t hi[2][16], lo[2][16];
+            auto look_up = [&]() {
 #pragma unroll
-            for (int sb = 0; sb < 2; ++sb)
+                for (int sb = 0; sb < 2; ++sb)
 #pragma unroll
-                for (int p = 0; p < 16; ++p) {
-                    const int pair = sb * 16 + p;
-                    const int bit = pair * 2 * BITS, wi = bit >> 5, sh = bit & 31;
-                    uint32_t e;
-                    if (sh + 2 * BITS <= 32) e = (w[wi] >> sh) & kPairMask;
-                    else e = __funnelshift_r(w[wi], w[wi + 1], sh) & kPairMask;
-                    const uint2 v = lut_lane[e * 32];
-                    hi[sb][p] = v.x;
-                    lo[sb][p] = v.y;
-                }
+                    for (int p = 0; p < 16; ++p) {
+                        const int pair = sb * 16 + p;
+                        if (kPartial && sb >= blocks) continue;
+                        if (!L::kPairLut) {
+                            uint32_t v[2];
+#pragma unroll
+                            for (int u = 0; u < 2; ++u) {
+                                const int bit = (2 * pair + u) * BITS, wi = bit >> 5, sh = bit & 31;
+                                const uint32_t c = sh + BITS <= 32 ? w[wi] >> sh : __funnelshift_r(w[wi], w[wi + 1], sh);
+                                v[u] = one_lane[(c & ((1u << BITS) - 1u)) * 32];
+                            }
+                            hi[sb][p] = __byte_perm(v[0], v[1], 0x5410);
+                            lo[sb][p] = __byte_perm(v[0], v[1], 0x7632);
+                            continue;
+                        }
+                        const int bit = pair * 2 * BITS, wi = bit >> 5, sh = bit & 31;
+                        uint32_t e;
+                        if (sh + 2 * BITS <= 32) e = (w[wi] >> sh) & kPairMask;
+                        else e = __funnelshift_r(w[wi], w[wi + 1], sh) & kPairMask;
+                        const uint2 v = lut_lane[e * 32];
+                        hi[sb][p] = v.x;
+                        lo[sb][p] = v.y;
+                    }
+            };
+            if (!PROD || !kSmallFirst) look_up();
             // beta = alpha * rnorm as fp16 hi + lo, both halves of a pair alike; the signs flip bit 15 / 31
             uint32_t bh2 = 0u, bl2 = 0u;
             if (PROD) {
                 const float beta = a.alpha * rn * kBetaScale;
                 const __half bh = __float2half_rn(beta);
-                const __half bl = __float2half_rn(beta - __half2float(bh));
+                const __half bl = __float2half_rn(fmaf(beta, a.b_loss, beta - __half2float(bh)));
                 const uint32_t bhu = (uint32_t)__half_as_ushort(bh), blu = (uint32_t)__half_as_ushort(bl);
                 bh2 = bhu | (bhu << 16);
                 bl2 = blu | (blu << 16);
@@ -358,14 +431,18 @@ dequant_tc_kernel(const DequantArgs a) {
                 if (!mbar_wait(BAR(DB_A_EMPTY + slot), (uint32_t)((n / kSlots) & 1) ^ 1u, abort_flag)) fail = true;
                 tc_fence_after();
                 const uint32_t abase = tmem + lane_addr + slot * kSlotCols + half * 32;
+                constexpr bool kLate = PROD && kSmallFirst;
+                const int kind = operand_at<PROD, kSmallFirst>(op);
+                if (kLate && op == 1) look_up();                 // (behind the first store, which needs none)
 #pragma unroll
                 for (int sb = 0; sb < 2; ++sb) {
-                    if (op == 0) tmem_st16(abase + sb * 16, hi[sb]);
-                    else if (op == 1) tmem_st16(abase + sb * 16, lo[sb]);
+                    if (kPartial && sb >= blocks) continue;
+                    if (kind == C_HI) tmem_st16(abase + sb * 16, hi[sb]);
+                    else if (kind == C_LO) tmem_st16(abase + sb * 16, lo[sb]);
                     else {
                         // sign word sb covers coordinates 32*sb .. 32*sb+31 of this half; pair p: bits p, 16+p
                         uint32_t sg[16];
-                        const uint32_t pat = op == 2 ? bh2 : bl2;
+                        const uint32_t pat = kind == B_HI ? bh2 : bl2;
 #pragma unroll
                         for (int p = 0; p < 16; ++p) sg[p] = pat ^ ((sw[sb] << (15 - p)) & 0x80008000u);
                         tmem_st16(abase + sb * 16, sg);
@@ -416,8 +493,9 @@ dequant_tc_kernel(const DequantArgs a) {
             tc_fence_after();
             const uint32_t acc = tmem + lane_addr + kColD + b * D + colhalf * 64;
             uint32_t va[32], vb[32];
+            const int chunks = kPartial && colhalf == kHalves - 1 ? 1 : 2;
             tmem_ld32_(acc, va);
-            tmem_ld32_(acc + 32, vb);
+            if (!kPartial || chunks == 2) tmem_ld32_(acc + 32, vb);
             tmem_wait_ld();
             tc_fence_before();
             __syncwarp();
@@ -460,6 +538,7 @@ dequant_tc_kernel(const DequantArgs a) {
             // whole 128-byte lines (four rows x 32 floats per instruction) instead of 16 bytes of 32 rows.
 #pragma unroll
             for (int ch = 0; ch < 2; ++ch) {
+                if (kPartial && ch >= chunks) continue;
                 float4* mine = reinterpret_cast<float4*>(stg + lane * L::kOutRowBytes);
 #pragma unroll
                 for (int m = 0; m < 8; ++m) {
@@ -574,7 +653,7 @@ dequant256_kernel(const __grid_constant__ CUtensorMap tmap_out, const DequantArg
             const float2 hf = __half22float2(h);
             uint2 v;
             v.x = *reinterpret_cast<const uint32_t*>(&h);
-            v.y = pack_half2(c0 - hf.x, c1 - hf.y);
+            v.y = pack_half2(fmaf(c0, a.c_loss, c0 - hf.x), fmaf(c1, a.c_loss, c1 - hf.y));
             lut[i] = v;
         }
     }
@@ -751,7 +830,7 @@ dequant256_kernel(const __grid_constant__ CUtensorMap tmap_out, const DequantArg
             if (PROD) {   // phase 1: +-beta, both halves of a pair alike; the signs flip bit 15 / 31
                 const float beta = a.alpha * rn * kBetaScale;
                 const __half bh = __float2half_rn(beta);
-                const __half bl = __float2half_rn(beta - __half2float(bh));
+                const __half bl = __float2half_rn(fmaf(beta, a.b_loss, beta - __half2float(bh)));
                 const uint32_t bhu = (uint32_t)__half_as_ushort(bh), blu = (uint32_t)__half_as_ushort(bl);
                 const uint32_t bh2 = bhu | (bhu << 16), bl2 = blu | (blu << 16);
                 if (!mbar_wait(BAR(A_EMPTY + (part >> 1)), (uint32_t)(phase_n & 1) ^ 1u, abort_flag)) fail = true;
@@ -907,13 +986,14 @@ struct DequantConsts {
 };
 
 bool tq_dequant_tc_supported(int d, int bits_mse, bool prod) {
-    // the pair lookup table of a 4-bit code and four operand matrices do not fit side by side
-    return (d == 128 || d == 64 || d == 256) && bits_mse >= 1 && bits_mse <= (prod ? 3 : 4);
+    // (the pair lookup table of a 4-bit code and four operand matrices do not fit side by side)
+    return ((d == 128 || d == 64 || d == 256) && bits_mse >= 1 && bits_mse <= (prod ? 3 : 4)) ||
+           (d == 96 && bits_mse >= 1 && bits_mse <= (prod ? 5 : 6)) || tq_tensor_wide_supported(d, bits_mse, prod);
 }
 
 int tq_dequant_tc_plan_init(tq_plan* p, const float* rotation, const float* projection) {
     const int d = p->dev.d;
-    if (d != 128 && d != 64 && d != 256) return TQ_OK;
+    if (d != 128 && d != 96 && d != 64 && d != 256) return TQ_OK;
     const size_t dd = (size_t)D * D;
     const int nmat = projection ? 4 : 2;
     std::vector<uint16_t> mats(d == 256 ? (size_t)d * d * nmat : dd * nmat, 0);
@@ -944,6 +1024,15 @@ void tq_dequant_tc_plan_free(tq_plan* p) {
     }
 }
 
+// Mean loss of the two parts to truncation.  Small products first: only the n = d / 16 hi products of the signs, then of the centroids,
+// meet a sum of size.  Otherwise three products per k-block, the centroids' before the signs'.
+static void set_losses(DequantArgs* a, int d, int bits, bool prod) {
+    const double n = d / 16.0;
+    const bool small = d != 256 && small_first(d, bits, prod);
+    a->c_loss = (float)tq_truncation_loss(small ? 0.5 * n : prod ? 4.5 * n : 1.5 * n);
+    a->b_loss = (float)tq_truncation_loss(1.5 * n);
+}
+
 int tq_launch_dequant_tc(const tq_plan* p, bool prod, const uint32_t* codes, const uint32_t* signs, const float* rnorms,
                          const float* norms, int64_t n, float* out, cudaStream_t st) {
     TqRange range("tq.dequantize.tensor_core");
@@ -954,6 +1043,7 @@ int tq_launch_dequant_tc(const tq_plan* p, bool prod, const uint32_t* codes, con
     a.bmat = static_cast<const unsigned char*>(p->dequant->dev);
     a.codebook = p->dev.codebook;
     a.alpha = p->dev.alpha;
+    set_losses(&a, p->dev.d, p->dev.bits, prod);
     a.n = n;
     a.ntiles = (n + kTileKeys - 1) / kTileKeys;
     a.out = out;
@@ -965,7 +1055,7 @@ int tq_launch_dequant_tc(const tq_plan* p, bool prod, const uint32_t* codes, con
     int r = TQ_ERR_UNSUPPORTED;
 #define TQ_DQ(B, P)                                                                                  \
     case B:                                                                                          \
-        r = p->dev.d == 64 ? launch_one<B, P, 64>(p, a, grid, st) : launch_one<B, P, 128>(p, a, grid, st); \
+        r = p->dev.d == 64 ? launch_one<B, P, 64>(p, a, grid, st) : p->dev.d == 96 ? launch_one<B, P, 96>(p, a, grid, st) : launch_one<B, P, 128>(p, a, grid, st); \
         break;
     if (p->dev.d == 256) {
         if (prod) {
@@ -985,9 +1075,13 @@ int tq_launch_dequant_tc(const tq_plan* p, bool prod, const uint32_t* codes, con
             }
         }
     } else if (prod) {
-        switch (bits) { TQ_DQ(1, true) TQ_DQ(2, true) TQ_DQ(3, true) default: break; }
+        switch (bits) {
+            TQ_DQ(1, true) TQ_DQ(2, true) TQ_DQ(3, true) TQ_DQ(5, true)
+            case 4: if (p->dev.d == 96) r = launch_one<4, true, 96>(p, a, grid, st); break;
+            default: break;
+        }
     } else {
-        switch (bits) { TQ_DQ(1, false) TQ_DQ(2, false) TQ_DQ(3, false) TQ_DQ(4, false) default: break; }
+        switch (bits) { TQ_DQ(1, false) TQ_DQ(2, false) TQ_DQ(3, false) TQ_DQ(4, false) TQ_DQ(5, false) TQ_DQ(6, false) default: break; }
     }
 #undef TQ_DQ
     if (r == TQ_ERR_UNSUPPORTED) return tq_fail(r, "no tensor-core dequantize kernel for bits=%d", bits);
@@ -1005,6 +1099,7 @@ int tq_launch_pairwise_tc(const tq_plan* p, const float* q, const uint32_t* code
     a.bmat = static_cast<const unsigned char*>(p->dequant->dev);
     a.codebook = p->dev.codebook;
     a.alpha = p->dev.alpha;
+    set_losses(&a, p->dev.d, p->dev.bits, true);
     a.n = n;
     a.ntiles = (n + kTileKeys - 1) / kTileKeys;
     a.out = scores;

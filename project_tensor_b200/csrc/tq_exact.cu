@@ -652,7 +652,7 @@ exact_code_check_kernel(const __grid_constant__ CheckJob first, const __grid_con
     constexpr int E = D > 128 ? 16 : 32, kLanes = 256 / E, kStep = E / (32 / kLanes);      // entries per block; lanes per entry
     constexpr int kStride = D + 1;                                                      // odd: a column is free of bank conflicts
     __shared__ float vt[E * kStride], mt[E * kStride];
-    __shared__ float bnd[16];
+    __shared__ float bnd[64];
     __shared__ unsigned long long entry[E];      // ~0: none
     __shared__ uint32_t stored[E];               // the code that stands in the packed row
     const bool one = (int)blockIdx.x < blocks0;
@@ -663,7 +663,7 @@ exact_code_check_kernel(const __grid_constant__ CheckJob first, const __grid_con
     // entries warp, warp + kStep, ... of the block: the lanes of different entries meet in different banks
     const int e = warp + kStep * (lane / kLanes), l = lane & (kLanes - 1);
     const TqRecheck& lists = job.lists;
-    if (t < p.levels - 1) bnd[t] = __ldg(p.boundaries + t);      // (at most 15: the tensor-core kernels take up to 4 bits)
+    if (t < p.levels - 1) bnd[t] = __ldg(p.boundaries + t);      // (at most 63: the tensor-core kernels take up to 6 bits)
     tq_grid_release();
     tq_grid_wait();
     // asked for before the header is known to allow it (the list's capacity bounds the index)
@@ -857,7 +857,8 @@ int tq_launch_exact_code_check(const TqSecondStage* a, const TqSecondStage* b, c
     // as many blocks as a list of typical length has entries for (about 1 in 48 rows of 128 coordinates at 4 bits, in
     // proportion to the coordinates); longer lists take more passes
     auto blocks = [&](const TqSecondStage* s) {
-        const int64_t w = (s->n * d / 128 / 48 + per_block - 1) / per_block;
+        // (a finer code has as many more boundaries)
+        const int64_t w = ((s->n * d / 128 << (s->plan->dev.bits > 4 ? s->plan->dev.bits - 4 : 0)) / 48 + per_block - 1) / per_block;
         return (int)(w < 4 ? 4 : w > most ? most : w);
     };
     auto job = [](const TqSecondStage* s) {
@@ -869,9 +870,10 @@ int tq_launch_exact_code_check(const TqSecondStage* a, const TqSecondStage* b, c
     const CheckJob first = job(a), second = b ? job(b) : first;
     const int b0 = blocks(a), grid = b0 + (b ? blocks(b) : 0);
     if (d == 128) TQ_CUDA_TRY(tq_launch_dependent(exact_code_check_kernel<128>, dim3(grid), dim3(256), 0, st, first, second, b0));
+    else if (d == 96) TQ_CUDA_TRY(tq_launch_dependent(exact_code_check_kernel<96>, dim3(grid), dim3(256), 0, st, first, second, b0));
     else if (d == 64) TQ_CUDA_TRY(tq_launch_dependent(exact_code_check_kernel<64>, dim3(grid), dim3(256), 0, st, first, second, b0));
     else if (d == 256) TQ_CUDA_TRY(tq_launch_dependent(exact_code_check_kernel<256>, dim3(grid), dim3(256), 0, st, first, second, b0));
-    else return tq_fail(TQ_ERR_UNSUPPORTED, "the coordinate re-check is written for d = 64, 128 and 256");
+    else return tq_fail(TQ_ERR_UNSUPPORTED, "the coordinate re-check is written for d = 64, 96, 128 and 256");
     return TQ_OK;
 }
 
@@ -1009,7 +1011,11 @@ int tq_launch_exact_listed(const TqSecondStage* a, const TqSecondStage* b, int a
     };
     // A listed pass does not know its size on the host.  About one row in 450 of a TurboQuantProd call at d = 128 is listed
     // (the coordinate re-check and the sign guard), hardly any of a TurboQuantMSE call; the blocks stride on where it is more.
-    auto rows = [](const TqSecondStage* s) { return s->prod ? s->n * s->plan->dev.d / 128 / 384 + 1 : s->n / 65536 + 1; };
+    // (a bit more halves the residual, whose projections are then twice as often near zero)
+    auto rows = [](const TqSecondStage* s) {
+        const int bits = s->plan->dev.bits;
+        return s->prod ? (s->n * s->plan->dev.d / 128 << (bits > 4 ? bits - 3 : 0)) / 384 + 1 : s->n / 65536 + 1;
+    };
     const RowsJob first = job(a), second = b ? job(b) : first;
     const int64_t ra = rows(a), rb = b ? rows(b) : 0;
     return launch_rows(first, b ? &second : nullptr, ra > rb ? ra : rb, a->plan->device, advance, st);

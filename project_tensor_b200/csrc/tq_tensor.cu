@@ -57,10 +57,14 @@ constexpr float kScaleM = 16.f;                 // R S^T -> second B operand
 constexpr int kCells = 32;
 constexpr int kPendCap = 32;               // second-stage entries staged per warp and list (a ballot adds up to 32)
 constexpr float kCellMul = 31.99998f;
+// 5- and 6-bit codes: a finer table in shared memory (Lloyd-Max boundaries of 6 bits are down to a 120th of their range apart)
+constexpr int kWideCells = 256;
+constexpr float kWideCellMul = 255.9998f;
+constexpr __host__ __device__ int table_cells(int bits) { return bits > 4 ? kWideCells : kCells; }
 
 struct TensorArgs {
     const __half* bmat;      // [R_hi | R_lo | M_hi | M_lo], each d*d halves in the interleaved layout
-    const float2* cell_lut;  // [32] per cell: boundary (x 2^20, +inf if none), boundaries below the cell (as int bits)
+    const float2* cell_lut;  // [table_cells(bits)] per cell: boundary (x 2^20, +inf if none), boundaries below the cell (as int bits)
     const float* code_ncent; // [32] entry l: -centroid(l mod levels) * 2^10
     float cell_scale, cell_offset;
     float code_guard, sign_guard;  // in accumulator units
@@ -98,7 +102,7 @@ __device__ __forceinline__ float2 widen_pair(uint32_t u, bool bf16) {
 // Shared-memory plan
 // ---------------------------------------------------------------------------------------------
 constexpr int kW = 128;   // width of the operand layouts in tensor and shared memory; d = 64 is zero-padded to it
-template <int D, bool PROD>
+template <int D, int BITS, bool PROD>
 struct Smem {
     static constexpr int kBBytes = kW * kW * 2;                     // one fp16 operand matrix (padded)
     static constexpr int kNumB = PROD ? 4 : 2;
@@ -112,7 +116,8 @@ struct Smem {
     static constexpr int kRsSlots = 4;                 // tiles whose |rho|^2 partial sums are alive at once
     static constexpr int kRsParts = 2;                 // threads per row in the first epilogue
     static constexpr int kRsBytes = kRsSlots * kRsParts * kTileRows * 4;
-    static constexpr int kMiscBytes = 8 * kTileRows * 4 + 4 * kTileRows + 512 + kRsBytes + kCells * 16 + kPendBytes;
+    static constexpr int kTableBytes = table_cells(BITS) * 8;
+    static constexpr int kMiscBytes = 8 * kTileRows * 4 + 4 * kTileRows + 512 + kRsBytes + kTableBytes + kPendBytes;
     static constexpr int total = off_misc + kMiscBytes + 1024;      // + slack to align the base to 1024
     static_assert(total <= 227 * 1024, "shared memory plan");
 };
@@ -178,14 +183,15 @@ __device__ __forceinline__ void pend_rows(const TqRecheck& l, WarpPending& w, bo
 // the lookup tables live in the lanes of the warp: lut_bnd / lut_base1 (boundaries below the cell) by cell, lut_ncent by code.
 // (One shuffle instead of two -- the count packed into the low mantissa bits of the boundary, taken apart with an AND --
 // was slower: 217 -> 226 us for TurboQuantProd, 162 -> 183 us for TurboQuantMSE; the integer pipe is the scarcer one.)
-template <int BITS, bool PROD>
+template <int BITS, bool PROD, int CHAINS = 2>
 __device__ __forceinline__ uint32_t process_chunk(const uint32_t (&v)[32], float lut_bnd, int lut_base1, float lut_ncent,
                                               float cell_scale, float cell_offset, float guard, uint32_t (&w)[BITS + 1],
-                                              uint32_t (&rhi)[16], uint32_t (&rlo)[16], float& rs) {
+                                              uint32_t (&rhi)[16], uint32_t (&rlo)[16], float& rs, const float2* table = nullptr) {
     // Elements go through the steps in groups of kGroup, step by step, so that the shuffles of a group
     // are in flight together instead of one element's chain after the other.
     constexpr int kGroup = 8;
     uint32_t nearmask = 0;  // bit e: element e lies inside the guard band of its boundary
+    float part[CHAINS] = {};      // the chunk's share of |rho|^2 in short chains
 #pragma unroll
     for (int k = 0; k <= BITS; ++k) w[k] = 0;
 #pragma unroll
@@ -197,10 +203,16 @@ __device__ __forceinline__ uint32_t process_chunk(const uint32_t (&v)[32], float
 #pragma unroll
         for (int t = 0; t < kGroup; ++t) {
             const float u = fma_sat(__uint_as_float(v[g + t]), cell_scale, cell_offset);
-            cell[t] = __float_as_int(fma_rm(u, kCellMul, 8388608.f));
+            cell[t] = __float_as_int(fma_rm(u, BITS > 4 ? kWideCellMul : kCellMul, 8388608.f));
         }
 #pragma unroll
         for (int t = 0; t < kGroup; ++t) {
+            if (BITS > 4) {
+                const float2 at = table[cell[t] & (kWideCells - 1)];
+                bnd[t] = at.x;
+                base1[t] = __float_as_int(at.y);
+                continue;
+            }
             bnd[t] = __shfl_sync(0xffffffffu, lut_bnd, cell[t]);
             base1[t] = __shfl_sync(0xffffffffu, lut_base1, cell[t]);
         }
@@ -234,14 +246,19 @@ __device__ __forceinline__ uint32_t process_chunk(const uint32_t (&v)[32], float
             // (packed fp32x2 arithmetic here made the kernel slower: the pairs have to be moved into adjacent registers)
 #pragma unroll
             for (int t = 0; t < kGroup; t += 2) {
-                rs = fmaf(r[t], r[t], rs);
-                rs = fmaf(r[t + 1], r[t + 1], rs);
+                part[t & (CHAINS - 2)] = fmaf(r[t], r[t], part[t & (CHAINS - 2)]);
+                part[(t & (CHAINS - 2)) + 1] = fmaf(r[t + 1], r[t + 1], part[(t & (CHAINS - 2)) + 1]);
                 const __half2 h = __floats2half2_rn(r[t], r[t + 1]);
                 const float2 hf = __half22float2(h);
                 rhi[(g + t) >> 1] = *reinterpret_cast<const uint32_t*>(&h);
                 rlo[(g + t) >> 1] = pack_half2(r[t] - hf.x, r[t + 1] - hf.y);
             }
         }
+    }
+    if (PROD) {
+#pragma unroll
+        for (int k = 2; k < CHAINS; ++k) part[k & 1] += part[k];
+        rs += part[0] + part[1];
     }
     return nearmask;
 }
@@ -268,18 +285,20 @@ __device__ __noinline__ void pend_codes(const TqRecheck& l, WarpPending& w, uint
 template <int D, int BITS, bool PROD, bool HALF, bool MAPPED>
 __global__ void __launch_bounds__(Threads<PROD>::kThreads, 1)
 tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorArgs a) {
-    static_assert(D == 128 || D == 64, "this kernel is written for d = 128 and d = 64");
-    // d = 64 runs in the layouts of d = 128 with the upper half of every row absent: the converter warps
-    // and the epilogue warps of that half stay idle, the contractions stop after d / 16 k-blocks and cover
-    // N = d output coordinates.
+    static_assert(D == 128 || D == 96 || D == 64, "this kernel is written for d = 64, 96 and 128");
+    static_assert(!HALF || D != 96, "16-bit rows come in boxes of 64 columns");
+    // d = 64 and 96 run in the layouts of d = 128 with the upper columns of every row absent: the converter warps
+    // and the epilogue warps of those columns stay idle (d = 96: or have one chunk of 32 instead of two), the
+    // contractions stop after d / 16 k-blocks and cover N = d output coordinates.
     constexpr int kThreads = Threads<PROD>::kThreads;
     constexpr int kFirstEpiWarp = Threads<PROD>::kFirstEpiWarp;
     constexpr int kConvParts = Threads<PROD>::kConvWarps / 4;   // converter threads per row
     constexpr int kXs = kW / kConvParts;                        // values a converter thread handles (64 or 32)
-    constexpr int kActiveParts = D / kXs;                       // parts that have data (d = 64: half of them)
-    using L = Smem<D, PROD>;
+    constexpr int kActiveParts = (D + kXs - 1) / kXs;           // parts that have data (d = 64: half of them)
+    using L = Smem<D, BITS, PROD>;
+    constexpr bool kPartial = D % 64 != 0;            // the last part of a row has one 32-column chunk, not two
     constexpr int kEpiChunks = 2;                     // 32-column chunks a thread owns in the first epilogue
-    constexpr int kEpiParts = D / (32 * kEpiChunks);            // first-epilogue threads per row that have data
+    constexpr int kEpiParts = (D + 32 * kEpiChunks - 1) / (32 * kEpiChunks);   // first-epilogue threads per row that have data
     constexpr int kSignChunks = kXs / 32;                       // chunks a thread owns in the sign epilogue
     constexpr int kBoxCols = HALF ? 64 : 32;                    // columns of a TMA box (128 bytes a row)
     constexpr int kBoxes = D / kBoxCols;                        // boxes of a tile
@@ -294,8 +313,8 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
     unsigned char* force = smem + L::off_misc + 8 * kTileRows * 4;                      // [4][128]
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::off_misc + 8 * kTileRows * 4 + 4 * kTileRows);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + BAR_COUNT);
-    float* rs_part = reinterpret_cast<float*>(smem + L::off_misc + L::kMiscBytes - L::kPendBytes - L::kRsBytes - kCells * 16);  // [kRsSlots][kRsParts][128]
-    float2* cell_lut = reinterpret_cast<float2*>(smem + L::off_misc + L::kMiscBytes - L::kPendBytes - kCells * 16);  // [32]
+    float* rs_part = reinterpret_cast<float*>(smem + L::off_misc + L::kMiscBytes - L::kPendBytes - L::kRsBytes - L::kTableBytes);  // [kRsSlots][kRsParts][128]
+    float2* cell_lut = reinterpret_cast<float2*>(smem + L::off_misc + L::kMiscBytes - L::kPendBytes - L::kTableBytes);  // [table_cells]
     unsigned char* pend_base = smem + L::off_misc + L::kMiscBytes - L::kPendBytes;
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const uint32_t bar0 = smem_u32(bars);
@@ -320,7 +339,8 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
         abort_flag[1] = a.wait_kcycles;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (threadIdx.x < kCells) cell_lut[threadIdx.x] = a.cell_lut[threadIdx.x];
+    if (threadIdx.x < table_cells(BITS)) cell_lut[threadIdx.x] = a.cell_lut[threadIdx.x];
+    static_assert(table_cells(BITS) <= kThreads, "a thread copies an entry");
     {   // operand matrices: global -> smem, once per CTA
         const uint4* src = reinterpret_cast<const uint4*>(a.bmat);
         uint4* dst = reinterpret_cast<uint4*>(smem + L::off_b);
@@ -340,6 +360,9 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
 
     const int64_t my_tiles = a.ntiles > (int64_t)blockIdx.x ? (a.ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
     constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(D >> 3) << 17) | ((uint32_t)(kTileRows >> 4) << 24);
+    // d = 96 and the finer codes: the products with a lo part come first.  The tensor pipe truncates a sum at every instruction by
+    // a share of what it holds (about 2.5e-8), so only the last D / 16 instructions count.
+    constexpr bool kSmallFirst = D == 96 || BITS > 4;
     constexpr int kABlock = kW / 2;  // TMEM columns of one fp16 A block (two halves per column)
     // TMEM column map
     auto A_COL = [&](int b) { return (uint32_t)(b * 2 * kABlock); };
@@ -403,16 +426,29 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
                     const uint32_t acc = tm + ACC_COL(b);
                     const uint32_t a_hi = tm + A_COL(b), a_lo = a_hi + kABlock;
                     if (elect_one()) {
-                        mma_ts_first(acc, a_hi, d_rhi, kIdesc);
-                        mma_ts_acc(acc, a_hi, d_rlo, kIdesc);
-                        mma_ts_acc(acc, a_lo, d_rhi, kIdesc);
+                        if constexpr (kSmallFirst) {
+                            mma_ts_first(acc, a_hi, d_rlo, kIdesc);
+                            mma_ts_acc(acc, a_lo, d_rhi, kIdesc);
 #pragma unroll 1
-                        for (int kb = 1; kb < D / 16; ++kb) {
-                            const uint64_t dh = d_rhi + (uint64_t)(kb * 2 * lbo >> 4);
-                            const uint64_t dl = d_rlo + (uint64_t)(kb * 2 * lbo >> 4);
-                            mma_ts_acc(acc, a_hi + kb * 8, dh, kIdesc);
-                            mma_ts_acc(acc, a_hi + kb * 8, dl, kIdesc);
-                            mma_ts_acc(acc, a_lo + kb * 8, dh, kIdesc);
+                            for (int kb = 1; kb < D / 16; ++kb) {
+                                mma_ts_acc(acc, a_hi + kb * 8, d_rlo + (uint64_t)(kb * 2 * lbo >> 4), kIdesc);
+                                mma_ts_acc(acc, a_lo + kb * 8, d_rhi + (uint64_t)(kb * 2 * lbo >> 4), kIdesc);
+                            }
+#pragma unroll
+                            for (int kb = 0; kb < D / 16; ++kb)
+                                mma_ts_acc(acc, a_hi + kb * 8, d_rhi + (uint64_t)(kb * 2 * lbo >> 4), kIdesc);
+                        } else {
+                            mma_ts_first(acc, a_hi, d_rhi, kIdesc);
+                            mma_ts_acc(acc, a_hi, d_rlo, kIdesc);
+                            mma_ts_acc(acc, a_lo, d_rhi, kIdesc);
+#pragma unroll 1
+                            for (int kb = 1; kb < D / 16; ++kb) {
+                                const uint64_t dh = d_rhi + (uint64_t)(kb * 2 * lbo >> 4);
+                                const uint64_t dl = d_rlo + (uint64_t)(kb * 2 * lbo >> 4);
+                                mma_ts_acc(acc, a_hi + kb * 8, dh, kIdesc);
+                                mma_ts_acc(acc, a_hi + kb * 8, dl, kIdesc);
+                                mma_ts_acc(acc, a_lo + kb * 8, dh, kIdesc);
+                            }
                         }
                         mma_commit(BAR(BAR_ACC_FULL + b));
                         if (!PROD) mma_commit(BAR(BAR_A_EMPTY + b));
@@ -472,6 +508,8 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
         const int chunk0 = colgroup * kEpiChunks;
         const bool conv_active = conv_role && half < kActiveParts;      // d = 64: the warps of the absent columns idle
         const bool epi_active = !conv_role && colgroup < kEpiParts;
+        const int epi_chunks = kPartial && chunk0 + 1 >= D / 32 ? 1 : kEpiChunks;            // chunks this thread has in the first epilogue
+        const int part_chunks = kPartial && half * (kXs / 32) + 1 >= D / 32 ? 1 : kXs / 32;   // ... as converter and in the sign epilogue
         // lookup tables held in the lanes of the warp: per cell (boundary, boundaries below), per code (- centroid * 2^10)
         const float lut_bnd = cell_lut[lane].x;
         const int lut_base1 = __float_as_int(cell_lut[lane].y);   // boundaries below the cell = code of a value below its boundary
@@ -508,7 +546,7 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
             uint32_t va[32];
             uint32_t sw0 = 0, sw1 = 0;
 #pragma unroll 1
-            for (int ch = 0; ch < kSignChunks; ++ch) {
+            for (int ch = 0; ch < (kPartial ? part_chunks : kSignChunks); ++ch) {
                 TQ_PROF_CODE(const long long l0 = clock64();)
                 tmem_ld32(acc2 + (sc0 + ch) * 32, va);
                 tmem_wait_ld();
@@ -543,7 +581,10 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
             __syncwarp();
             if (lane == 0) mbar_arrive(BAR(BAR_A_EMPTY + (b ^ 1)));  // that A block may be refilled
             if (live) {
-                if (kSignChunks == 2) *reinterpret_cast<uint2*>(a.signs + orow * (D / 32) + sc0) = make_uint2(sw0, sw1);
+                if (kPartial) {      // rows of three words
+                    a.signs[orow * (D / 32) + sc0] = sw0;
+                    if (part_chunks == 2) a.signs[orow * (D / 32) + sc0 + 1] = sw1;
+                } else if (kSignChunks == 2) *reinterpret_cast<uint2*>(a.signs + orow * (D / 32) + sc0) = make_uint2(sw0, sw1);
                 else a.signs[orow * (D / 32) + sc0] = sw0;
             }
             pend_rows(a.lists, pend, redo_row && live, grow, lane);
@@ -560,6 +601,11 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
             TQ_PROF_CODE(const bool pr = a.prof && blockIdx.x == 0 && threadIdx.x == kFirstConvWarp * 32; long long c0 = clock64(), c1;)
 #pragma unroll
             for (int bb = 0; bb < (HALF ? 1 : kXs / 32); ++bb) {
+                if (kPartial && bb >= part_chunks) {         // columns that are not there
+#pragma unroll
+                    for (int c = 0; c < 32; ++c) x[bb * 32 + c] = 0.f;
+                    continue;
+                }
                 const int64_t g = g_base + (HALF ? half / kBoxReaders : half * (kXs / 32) + bb);
                 const int slot = (int)(g % L::kRingBoxes);
                 const uint32_t par = (uint32_t)((g / L::kRingBoxes) & 1);
@@ -608,10 +654,15 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
                 }
                 ss = (s2[0].x + s2[0].y) + (s2[1].x + s2[1].y);
             } else {
-                float s4[4] = {0.f, 0.f, 0.f, 0.f};
+                constexpr int kChains = kSmallFirst ? 8 : 4;      // (as short as the reference's pairwise sum has them)
+                float s4[kChains] = {};
 #pragma unroll
-                for (int k = 0; k < kXs; ++k) s4[k & 3] = fmaf(x[k], x[k], s4[k & 3]);
-                ss = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+                for (int k = 0; k < kXs; ++k) s4[k & (kChains - 1)] = fmaf(x[k], x[k], s4[k & (kChains - 1)]);
+#pragma unroll
+                for (int w = kChains / 2; w > 0; w /= 2)
+#pragma unroll
+                    for (int k = 0; k < w; ++k) s4[k] += s4[k + w];
+                ss = s4[0];
             }
             // partial sums of a tile go to the buffer of its parity: a fast warp writes the next tile's sums
             // before the barrier of that tile, while a slow partner may still be reading this tile's
@@ -643,6 +694,7 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
             const uint32_t a_hi = tmem + lane_addr + A_COL(b) + half * (kXs / 2);
 #pragma unroll
             for (int s = 0; s < kXs / 32; ++s) {
+                if (kPartial && s >= part_chunks) continue;
                 uint32_t hi[16], lo[16];
 #pragma unroll
                 for (int p = 0; p < 16; ++p) {
@@ -708,15 +760,15 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
                 // instruction cache more than the loop overhead does
                 uint32_t nm0 = 0, nm1 = 0;
 #pragma unroll 1
-                for (int ch = 0; ch < kEpiChunks; ++ch) {
+                for (int ch = 0; ch < (kPartial ? epi_chunks : kEpiChunks); ++ch) {
                     uint32_t va[32];
                     TQ_PROF_CODE(const long long l0 = clock64();)
                     tmem_ld32(acc + (chunk0 + ch) * 32, va);
                     tmem_wait_ld();
                     TQ_PROF_CODE(if (pr) prof_acc[13] += clock64() - l0;)
                     uint32_t w[BITS + 1], rhi[16], rlo[16];
-                    const uint32_t m = process_chunk<BITS, PROD>(va, lut_bnd, lut_base1, lut_ncent, a.cell_scale, a.cell_offset,
-                                                                 a.code_guard, w, rhi, rlo, rs);
+                    const uint32_t m = process_chunk<BITS, PROD, kSmallFirst ? 4 : 2>(va, lut_bnd, lut_base1, lut_ncent, a.cell_scale, a.cell_offset,
+                                                                 a.code_guard, w, rhi, rlo, rs, cell_lut);
                     if (ch == 0) nm0 = m; else nm1 = m;
                     store_codes(ch, w);
                     // rho replaces the chunk it was computed from: 16 columns of hi pairs, 16 of lo pairs
@@ -731,14 +783,15 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
                 tmem_wait_ld();
 #pragma unroll
                 for (int ch = 0; ch < kEpiChunks; ++ch) {
+                    if (kPartial && ch >= epi_chunks) { nm[ch] = 0; continue; }
                     // fetch the next chunk while this one is processed
-                    if (ch + 1 < kEpiChunks) {
+                    if (ch + 1 < kEpiChunks && (!kPartial || ch + 1 < epi_chunks)) {
                         if (ch & 1) tmem_ld32(acc + (chunk0 + ch + 1) * 32, va); else tmem_ld32(acc + (chunk0 + ch + 1) * 32, vb);
                     }
                     uint32_t w[BITS + 1], rhi[16], rlo[16];
                     nm[ch] = (ch & 1)
-                        ? process_chunk<BITS, PROD>(vb, lut_bnd, lut_base1, lut_ncent, a.cell_scale, a.cell_offset, a.code_guard, w, rhi, rlo, rs)
-                        : process_chunk<BITS, PROD>(va, lut_bnd, lut_base1, lut_ncent, a.cell_scale, a.cell_offset, a.code_guard, w, rhi, rlo, rs);
+                        ? process_chunk<BITS, PROD>(vb, lut_bnd, lut_base1, lut_ncent, a.cell_scale, a.cell_offset, a.code_guard, w, rhi, rlo, rs, cell_lut)
+                        : process_chunk<BITS, PROD>(va, lut_bnd, lut_base1, lut_ncent, a.cell_scale, a.cell_offset, a.code_guard, w, rhi, rlo, rs, cell_lut);
                     store_codes(ch, w);
                     if (ch + 1 < kEpiChunks) tmem_wait_ld();
                 }
@@ -1242,9 +1295,9 @@ void split_operand(const std::vector<double>& m, int d, double scale, uint16_t* 
     const size_t sbo = (size_t)(kW / 8) * 128, lbo = 128;
     for (int n = 0; n < d; ++n)
         for (int k = 0; k < d; ++k) {
-            const float v = (float)(m[(size_t)n * d + k] * scale);
-            const uint16_t h = host_half_bits(v);
-            const uint16_t l = host_half_bits((float)((double)v - (double)host_half_value(h)));
+            const double v = m[(size_t)n * d + k] * scale;
+            const uint16_t h = host_half_bits((float)v);
+            const uint16_t l = host_half_bits((float)(v - (double)host_half_value(h)));
             const size_t off = ((size_t)(n / 8) * sbo + (size_t)(k / 8) * lbo + (size_t)(n % 8) * 16 + (size_t)(k % 8) * 2) / 2;
             hi[off] = h;
             lo[off] = l;
@@ -1257,9 +1310,9 @@ void split_operand_chunks(const double* m, double scale, uint16_t* out) {
     const int d = 256;
     for (int n = 0; n < d; ++n)
         for (int k = 0; k < d; ++k) {
-            const float v = (float)(m[(size_t)n * d + k] * scale);      // B[n][k]
-            const uint16_t h = host_half_bits(v);
-            const uint16_t l = host_half_bits((float)((double)v - (double)host_half_value(h)));
+            const double v = m[(size_t)n * d + k] * scale;      // B[n][k]
+            const uint16_t h = host_half_bits((float)v);
+            const uint16_t l = host_half_bits((float)(v - (double)host_half_value(h)));
             const int J = n / 128, I = k / 128, kb = (k % 128) / 16, nn = n % 128, kk = k % 16;
             const size_t chunk = (size_t)((J * 2 + I) * 8 + kb) * 8192;
             const size_t off = (size_t)(nn / 8) * 256 + (size_t)(kk / 8) * 128 + (size_t)(nn % 8) * 16 + (size_t)(kk % 8) * 2;
@@ -1268,16 +1321,16 @@ void split_operand_chunks(const double* m, double scale, uint16_t* out) {
         }
 }
 
-int host_cell(float v, float scale, float offset) {
+int host_cell(float v, float scale, float offset, int ncells) {
     float u = fmaf(v, scale, offset);
     u = u < 0.f ? 0.f : (u > 1.f ? 1.f : u);
     if (!(u == u)) u = 0.f;
-    return (int)floor((double)u * (double)kCellMul);
+    return (int)floor((double)u * (double)(ncells == kCells ? kCellMul : kWideCellMul));
 }
 
-// Find a 32-cell uniform grid over the (scaled) boundaries such that every cell holds at most one
+// Find a uniform grid of 32 (kWideCells) cells over the (scaled) boundaries such that every cell holds at most one
 // boundary and every boundary keeps its cell within +-margin.  Returns false if none is found.
-bool build_cell_lut(const float* bnd_scaled, int nb, float margin, float* scale, float* offset, float* lut_bnd,
+bool build_cell_lut(const float* bnd_scaled, int nb, int ncells, float margin, float* scale, float* offset, float* lut_bnd,
                     int* lut_base) {
     const float bmin = bnd_scaled[0], bmax = bnd_scaled[nb - 1];
     // cells must be much wider than the margin, also when there is a single boundary
@@ -1289,15 +1342,15 @@ bool build_cell_lut(const float* bnd_scaled, int nb, float margin, float* scale,
             int cells[256];
             bool ok = true;
             for (int k = 0; k < nb && ok; ++k) {
-                const int c = host_cell(bnd_scaled[k], sc, of);
-                if (host_cell(bnd_scaled[k] - margin, sc, of) != c || host_cell(bnd_scaled[k] + margin, sc, of) != c) ok = false;
-                if (c <= 0 || c >= kCells - 1) ok = false;  // keep the end cells free of boundaries
+                const int c = host_cell(bnd_scaled[k], sc, of, ncells);
+                if (host_cell(bnd_scaled[k] - margin, sc, of, ncells) != c || host_cell(bnd_scaled[k] + margin, sc, of, ncells) != c) ok = false;
+                if (c <= 0 || c >= ncells - 1) ok = false;  // keep the end cells free of boundaries
                 if (k > 0 && c == cells[k - 1]) ok = false;
                 cells[k] = c;
             }
             if (!ok) continue;
             int k = 0;
-            for (int c = 0; c < kCells; ++c) {
+            for (int c = 0; c < ncells; ++c) {
                 lut_base[c] = k;
                 if (k < nb && cells[k] == c) {
                     lut_bnd[c] = bnd_scaled[k];
@@ -1338,6 +1391,16 @@ bool tq_tensor_quantize_supported(int d, int bits, bool has_projection) {
     (void)has_projection;
     return tq_tensor_supported(d, bits) || (d == 256 && bits >= 1 && bits <= 4);
 }
+// Geometries that only the quantizers and dequantizers have on tensor cores: d = 96, and codes of 5 and, without a projection, 6 bits.
+// TurboQuantProd, 5 code bits, 50,021 rows of d = 96: 47 us with the second stage (135 in the reference's order); 65,536 rows of
+// d = 128: 62 (265).  Residual norms against 64 bits: 3.2e-7 at 5 code bits (the residual is a thirtieth of the vector), 1.0e-7 at 3;
+// in the reference's order 3.9 and 1.1e-7.
+bool tq_tensor_wide_supported(int d, int bits, bool has_projection) {
+    if (tq_tensor_supported(d, bits)) return false;
+    // (one code bit and a projection at d = 96: residual norms against 64 bits would be 6.0e-8 off, the reference order's are 5.6e-8)
+    if (d == 96 && bits == 1 && has_projection) return false;
+    return (d == 64 || d == 96 || d == 128) && bits >= 1 && bits <= (has_projection ? 5 : 6);
+}
 
 int tq_tensor_plan_init(tq_plan* p, const float* rotation, const float* codebook, const float* projection) {
     const int d = p->dev.d, levels = p->dev.levels, nb = levels - 1;
@@ -1352,12 +1415,13 @@ int tq_tensor_plan_init(tq_plan* p, const float* rotation, const float* codebook
         if (!(bnd_s[k] > bnd_s[k - 1])) return TQ_OK;  // degenerate codebook: leave tensor_ok false
     for (int k = 0; k < nb; ++k)
         if (!(fabsf(bnd[k]) < 4.f)) return TQ_OK;
-    float lut_bnd[kCells], lut_cent[kCells], cs = 0.f, co = 0.f;
-    int lut_base[kCells];
+    const int ncells = table_cells(p->dev.bits);
+    float lut_bnd[kWideCells], lut_cent[kCells], cs = 0.f, co = 0.f;
+    int lut_base[kWideCells];
     const float guard = TQ_CODE_GUARD * kAccScale;
-    if (!build_cell_lut(bnd_s.data(), nb, 4.f * guard, &cs, &co, lut_bnd, lut_base)) return TQ_OK;
-    float lut2[kCells * 2];
-    for (int c = 0; c < kCells; ++c) {
+    if (!build_cell_lut(bnd_s.data(), nb, ncells, 4.f * guard, &cs, &co, lut_bnd, lut_base)) return TQ_OK;
+    float lut2[kWideCells * 2];
+    for (int c = 0; c < ncells; ++c) {
         lut2[2 * c] = lut_bnd[c];
         memcpy(&lut2[2 * c + 1], &lut_base[c], 4);       // boundaries in lower cells = code of a value below this cell's boundary
     }
@@ -1367,12 +1431,14 @@ int tq_tensor_plan_init(tq_plan* p, const float* rotation, const float* codebook
     const int nmat = projection ? 4 : 2;
     std::vector<uint16_t> mats(d == 256 ? (size_t)d * d * nmat : dd * nmat, 0);
     std::vector<double> m((size_t)d * d);
+    // (the chain of the rotated coordinates: d / 16 instructions behind the small products, or three times as many in turn)
+    const double gain = 1.0 + tq_truncation_loss(d == 96 || p->dev.bits > 4 ? d / 32.0 : 1.5 * d / 16);
     if (d == 256) {
         for (size_t i = 0; i < (size_t)d * d; ++i) m[i] = rotation[i];  // B1[n=j][k] = R[j][k]
-        split_operand_chunks(m.data(), kScaleB, mats.data());
+        split_operand_chunks(m.data(), kScaleB * gain, mats.data());
     } else {
         for (size_t i = 0; i < (size_t)d * d; ++i) m[i] = rotation[i];  // B1[n=j][k] = R[j][k]
-        split_operand(m, d, kScaleB, mats.data(), mats.data() + dd);
+        split_operand(m, d, kScaleB * gain, mats.data(), mats.data() + dd);
     }
     if (projection) {
         // B2[n=j][k] = (R S^T)[k][j] = sum_i R[k][i] S[j][i]
@@ -1386,7 +1452,7 @@ int tq_tensor_plan_init(tq_plan* p, const float* rotation, const float* codebook
         else split_operand(m, d, kScaleM, mats.data() + 2 * dd, mats.data() + 3 * dd);
     }
     const size_t mat_bytes = mats.size() * 2;
-    const size_t total = mat_bytes + 5 * kCells * 4;
+    const size_t table_bytes = (size_t)ncells * 8, total = mat_bytes + table_bytes + kCells * 4;
     TensorConsts* t = new TensorConsts();
     cudaError_t e = cudaMalloc(&t->dev, total);
     if (e != cudaSuccess) {
@@ -1395,8 +1461,8 @@ int tq_tensor_plan_init(tq_plan* p, const float* rotation, const float* codebook
     }
     unsigned char* base = static_cast<unsigned char*>(t->dev);
     bool ok = cudaMemcpy(base, mats.data(), mat_bytes, cudaMemcpyHostToDevice) == cudaSuccess &&
-              cudaMemcpy(base + mat_bytes, lut2, sizeof(lut2), cudaMemcpyHostToDevice) == cudaSuccess &&
-              cudaMemcpy(base + mat_bytes + kCells * 16, lut_cent, kCells * 4, cudaMemcpyHostToDevice) == cudaSuccess;
+              cudaMemcpy(base + mat_bytes, lut2, table_bytes, cudaMemcpyHostToDevice) == cudaSuccess &&
+              cudaMemcpy(base + mat_bytes + table_bytes, lut_cent, kCells * 4, cudaMemcpyHostToDevice) == cudaSuccess;
     if (!ok || !tq_encode_tiled_fn()) {
         cudaFree(t->dev);
         delete t;
@@ -1404,14 +1470,13 @@ int tq_tensor_plan_init(tq_plan* p, const float* rotation, const float* codebook
     }
     t->args.bmat = reinterpret_cast<const __half*>(base);
     t->args.cell_lut = reinterpret_cast<const float2*>(base + mat_bytes);
-    t->args.code_ncent = reinterpret_cast<const float*>(base + mat_bytes + kCells * 16);
+    t->args.code_ncent = reinterpret_cast<const float*>(base + mat_bytes + table_bytes);
     t->args.cell_scale = cs;
     t->args.cell_offset = co;
     t->args.code_guard = guard;
     // accumulator 2 holds 2^10 * 16 * (residual . S row)
     t->args.sign_guard = TQ_SIGN_GUARD * 1024.f * kScaleM;
     p->tensor = t;
-    p->tensor_ok = true;
     return TQ_OK;
 }
 
@@ -1425,7 +1490,7 @@ void tq_tensor_plan_free(tq_plan* p) {
 
 template <int D, int BITS, bool PROD, bool HALF, bool MAPPED>
 static int launch_type(const tq_plan* p, const CUtensorMap& map, const TensorArgs& args, int grid, cudaStream_t st) {
-    const int sm = Smem<D, PROD>::total;
+    const int sm = Smem<D, BITS, PROD>::total;
     TQ_GRANT_SMEM((tensor_quantize_kernel<D, BITS, PROD, HALF, MAPPED>), sm, p->device);
     tensor_quantize_kernel<D, BITS, PROD, HALF, MAPPED><<<grid, Threads<PROD>::kThreads, sm, st>>>(map, args); tq_count_launch();
     TQ_CUDA_TRY(cudaGetLastError());
@@ -1435,7 +1500,9 @@ static int launch_type(const tq_plan* p, const CUtensorMap& map, const TensorArg
 template <int D, int BITS, bool PROD>
 static int launch_one(const tq_plan* p, const CUtensorMap& map, const TensorArgs& args, bool half, int grid, cudaStream_t st) {
     // (16-bit rows come from caches only)
-    if (half) return launch_type<D, BITS, PROD, true, true>(p, map, args, grid, st);
+    if constexpr (D != 96) {
+        if (half) return launch_type<D, BITS, PROD, true, true>(p, map, args, grid, st);
+    }
     return args.tokens ? launch_type<D, BITS, PROD, false, true>(p, map, args, grid, st) : launch_type<D, BITS, PROD, false, false>(p, map, args, grid, st);
 }
 
@@ -1453,7 +1520,7 @@ static int launch_256(const tq_plan* p, const CUtensorMap& map, const TensorArgs
 }
 
 // The kernels that read 16-bit rows are those for d = 64 and 128.
-bool tq_tensor_input_supported(int d, int xtype) { return xtype == TQ_INPUT_F32 || d != 256; }
+bool tq_tensor_input_supported(int d, int xtype) { return xtype == TQ_INPUT_F32 || d == 64 || d == 128; }
 
 int tq_launch_tensor_quantize(const tq_plan* p, bool prod, const void* x, int xtype, int64_t n, const TqQuantOut& out,
                               const TqRecheck* lists, cudaStream_t st) {
@@ -1509,7 +1576,8 @@ int tq_launch_tensor_quantize(const tq_plan* p, bool prod, const void* x, int xt
     }
 #define TQ_DISPATCH(B)                                                                                     \
     case B:                                                                                                \
-        if (d == 64) rc = prod ? launch_one<64, B, true>(p, map, args, half, grid, st) : launch_one<64, B, false>(p, map, args, half, grid, st); \
+        if (d == 96) rc = prod ? launch_one<96, B, true>(p, map, args, half, grid, st) : launch_one<96, B, false>(p, map, args, half, grid, st); \
+        else if (d == 64) rc = prod ? launch_one<64, B, true>(p, map, args, half, grid, st) : launch_one<64, B, false>(p, map, args, half, grid, st); \
         else rc = prod ? launch_one<128, B, true>(p, map, args, half, grid, st) : launch_one<128, B, false>(p, map, args, half, grid, st);      \
         break;
     switch (bits) {
@@ -1517,6 +1585,11 @@ int tq_launch_tensor_quantize(const tq_plan* p, bool prod, const void* x, int xt
         TQ_DISPATCH(2)
         TQ_DISPATCH(3)
         TQ_DISPATCH(4)
+        TQ_DISPATCH(5)
+        case 6:
+            if (!prod) rc = d == 96 ? launch_one<96, 6, false>(p, map, args, half, grid, st) : d == 64 ? launch_one<64, 6, false>(p, map, args, half, grid, st)
+                                                                                            : launch_one<128, 6, false>(p, map, args, half, grid, st);
+            break;
     }
 #undef TQ_DISPATCH
     tq_timer_mark(p, 0, 1, st);
