@@ -308,28 +308,45 @@ int64_t tq_topk_scratch_bytes(const tq_plan* p, int groups, int q_per_group, int
     return tq_score_topk_scratch(p, groups, q_per_group, keys_per_group, topk);
 }
 
-// Up to 32 rows per SM the reference-order kernel alone is faster than the tensor-core kernel with its second stage
-// (four operations on the stream): TurboQuantProd, 2,048 rows: d = 64 10 against 28 us, d = 128 18 against 38, d = 256
-// 43 against 84; 8,192 rows: 23 / 34, 44 / 45, 121 / 84.
-// d = 96 and the codes of 5 and 6 bits, whose second stage has more to do: TurboQuantProd, 8,000 rows, 31 against 35 us (d = 96, 6
-// bits), 33 / 51 (d = 128), at d = 64 31 / 23 and from 12,000 rows on 27 / 31; TurboQuantMSE, 8,000 and 12,000 rows, 23 / 19 and 23 / 27
-// (d = 96, 4 bits), 27 / 27 and 29 / 39 (d = 128, 6 bits), 21 / 14 and 21 / 21 (d = 64).
+// Up to 32 rows per SM (d = 64: 64, d = 96 and the 5- and 6-bit codes of TurboQuantMSE: 48) the reference-order kernel alone is as fast as the tensor-core kernel with its second
+// stage or faster.  TurboQuantProd, 4 bits, 3,600 rows of d = 128: 27 against 29 us, 4,800 rows 35 / 29; d = 64, 6,400 rows 15 / 23,
+// 9,600 rows 29 / 23; d = 96, 6 bits, 6,000 rows 25 / 28, 7,200 rows 33 / 29.  TurboQuantMSE, d = 128: 17 / 17 at 4,800 and 6,400 rows;
+// 6 bits 17 / 20 and 25 / 21 at 7,000 and 7,200 rows; d = 64, 6,400 and 9,600 rows 10 / 15 and 19 / 15.  d = 256, TurboQuantProd, 2,048 rows 43 / 84, 8,192 rows 121 / 84.
 static bool few_rows(const tq_plan* p, bool prod, int64_t n) {
-    const int d = p->dev.d, per_sm = p->tensor_ok ? 32 : d == 64 ? 80 : d == 96 && !prod ? 64 : 48;
+    const int d = p->dev.d, per_sm = d == 64 ? 64 : d == 96 || (!prod && !p->tensor_ok) ? 48 : 32;
     return p->path == TQ_PATH_AUTO && n <= per_sm * (int64_t)tq_sm_count(p->device);
 }
 // The reference-order dequantizer instead of the tensor-core one of the same plans, which takes 8 to 12 us however few the rows are
 // (4,700 rows: 6 to 8 against 8 to 10 us; 6,000 rows: equal).
 static bool few_restored(const tq_plan* p, int64_t n) { return !p->tensor_ok && n <= 36 * (int64_t)tq_sm_count(p->device); }
 
-// The lists of one call in the caller's scratch, behind its header.
-static unsigned char* place_lists(TqRecheck* l, TqRecheckHeader* hdr, unsigned char* at, int64_t n) {
+// The lists of one call in the caller's scratch, behind its header; those of the blocks and their lengths in the room of one pair.
+static unsigned char* place_lists(const tq_plan* p, TqRecheck* l, TqRecheckHeader* hdr, unsigned char* at, int64_t n) {
+    const size_t code_cap = tq_recheck_code_cap(n), row_cap = tq_recheck_row_cap(n);
+    const unsigned int blocks = p->dev.d == 256 ? 1 : (unsigned int)tq_tensor_quantize_blocks(p, n);
     l->hdr = hdr;
-    l->code_cap = tq_recheck_code_cap(n);
-    l->row_cap = tq_recheck_row_cap(n);
-    l->code_entries = reinterpret_cast<unsigned long long*>(at);
-    l->row_entries = reinterpret_cast<unsigned int*>(at + 8 * (size_t)l->code_cap);
-    return at + 8 * (size_t)l->code_cap + (4 * (size_t)l->row_cap + 15) / 16 * 16;
+    l->counts = p->dev.d == 256 ? nullptr : reinterpret_cast<unsigned int*>(at);
+    l->code_entries = reinterpret_cast<unsigned long long*>(at) + (l->counts ? blocks : 0);
+    l->code_cap = (unsigned int)((code_cap - (l->counts ? blocks : 0)) / blocks);
+    l->row_entries = reinterpret_cast<unsigned int*>(at + 8 * code_cap);
+    l->row_cap = (unsigned int)(row_cap / blocks);
+    return at + 8 * code_cap + (4 * row_cap + 15) / 16 * 16;
+}
+// The second stage of up to two jobs of one geometry.
+static int second_stage(const TqSecondStage* a, const TqSecondStage* b, int advance, cudaStream_t st) {
+    if (a->plan->dev.d != 256) {
+        tq_timer_mark(a->plan, 2, 0, st);
+        const int rc = tq_launch_second_stage(a, b, advance, st);
+        tq_timer_mark(a->plan, 2, 1, st);
+        return rc;
+    }
+    tq_timer_mark(a->plan, 2, 0, st);
+    TQ_TRY(tq_launch_exact_code_check(a, b, st));
+    tq_timer_mark(a->plan, 2, 1, st);
+    tq_timer_mark(a->plan, 3, 0, st);
+    const int rc = tq_launch_exact_listed(a, b, advance, st);
+    tq_timer_mark(a->plan, 3, 1, st);
+    return rc;
 }
 
 static int quantize_common(const tq_plan* p, bool prod, const float* x, int64_t n, void* codes, void* signs,
@@ -356,16 +373,10 @@ static int quantize_common(const tq_plan* p, bool prod, const float* x, int64_t 
         TQ_TRY(check_ptr(scratch, "scratch"));
         unsigned char* sc = static_cast<unsigned char*>(scratch);
         TqSecondStage second{p, prod, x, TQ_F32, n, out, {}};
-        place_lists(&second.lists, reinterpret_cast<TqRecheckHeader*>(sc), sc + sizeof(TqRecheckHeader), n);
-        TQ_CUDA_TRY(cudaMemsetAsync(second.lists.hdr, 0, sizeof(TqRecheckHeader), st));
+        place_lists(p, &second.lists, reinterpret_cast<TqRecheckHeader*>(sc), sc + sizeof(TqRecheckHeader), n);
+        if (p->dev.d == 256) TQ_CUDA_TRY(cudaMemsetAsync(second.lists.hdr, 0, sizeof(TqRecheckHeader), st));
         TQ_TRY(tq_launch_tensor_quantize(p, prod, x, TQ_F32, n, out, &second.lists, st));
-        tq_timer_mark(p, 2, 0, st);
-        TQ_TRY(tq_launch_exact_code_check(&second, nullptr, st));
-        tq_timer_mark(p, 2, 1, st);
-        tq_timer_mark(p, 3, 0, st);
-        const int rc = tq_launch_exact_listed(&second, nullptr, 0, st);
-        tq_timer_mark(p, 3, 1, st);
-        return rc;
+        return second_stage(&second, nullptr, 0, st);
     }
     if (err != TQ_OK) return err;
     // (a plan with tensor-core kernels counts the rows of this kernel, all of them here)
@@ -490,8 +501,8 @@ int tq_kv_prefill(const tq_plan* kp, const tq_plan* vp, const void* keys, const 
         TQ_TRY(check_ptr(scratch, "scratch"));
         TqRecheckHeader* hdr = static_cast<TqRecheckHeader*>(scratch);
         unsigned char* at = reinterpret_cast<unsigned char*>(hdr + ntensor);
-        for (int i = 0; i < ntensor; ++i) at = place_lists(&tensor[i].lists, hdr + i, at, rows);
-        TQ_CUDA_TRY(cudaMemsetAsync(hdr, 0, ntensor * sizeof(TqRecheckHeader), st));
+        for (int i = 0; i < ntensor; ++i) at = place_lists(tensor[i].plan, &tensor[i].lists, hdr + i, at, rows);
+        if (tensor[0].plan->dev.d == 256) TQ_CUDA_TRY(cudaMemsetAsync(hdr, 0, ntensor * sizeof(TqRecheckHeader), st));
     }
     for (int i = 0; i < ntensor; ++i)
         TQ_TRY(tq_launch_tensor_quantize(tensor[i].plan, tensor[i].prod, tensor[i].x, dtype, rows, tensor[i].out, &tensor[i].lists, st));
@@ -501,8 +512,7 @@ int tq_kv_prefill(const tq_plan* kp, const tq_plan* vp, const void* keys, const 
             TQ_TRY(tq_launch_exact_mapped(jobs[i].plan, jobs[i].prod, jobs[i].x, dtype, rows, jobs[i].out, --left == 0 && !ntensor ? 2 : 0, st));
     if (ntensor) {
         const TqSecondStage* second = ntensor == 2 ? &tensor[1] : nullptr;
-        TQ_TRY(tq_launch_exact_code_check(&tensor[0], second, st));
-        TQ_TRY(tq_launch_exact_listed(&tensor[0], second, 2, st));
+        TQ_TRY(second_stage(&tensor[0], second, 2, st));
     }
     return TQ_OK;
 }
@@ -528,8 +538,8 @@ int tq_mse_quantize_noalloc(const tq_plan* p, const float* x, int64_t n, void* c
         }
         scratch = g_noalloc_ptr[p->device];
     }
-    // quantize_common clears the list header at the start of every call (cudaMemsetAsync, no allocation);
-    // the entries behind it are only read up to the counts written by the same call.
+    // the entries of the lists are only read up to the lengths written by the same call (d = 256: quantize_common clears the header
+    // at the start of every call, cudaMemsetAsync, no allocation)
     return quantize_common(p, false, x, n, codes, nullptr, nullptr, norms, scratch, TQ_NOALLOC_SCRATCH_BYTES, stream);
 }
 

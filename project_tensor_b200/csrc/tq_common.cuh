@@ -28,21 +28,29 @@ enum { TQ_INPUT_F32 = TQ_F32, TQ_INPUT_BF16 = TQ_BF16, TQ_INPUT_F16 = TQ_F16 };
 // `steps` further instructions (a term of a chain of n on average for n / 2) loses this share; an operand is made that much larger.
 inline double tq_truncation_loss(double steps) { return steps * 4.3e-8; }
 
-// Work lists that the tensor-core quantizers leave in the caller's scratch buffer for the exact
-// second stage.  Layout of the scratch: this header (64 bytes), then `code_cap` 64-bit entries
-// (row << 8 | coordinate: a rotated coordinate inside the guard band of a boundary), then `row_cap`
-// 32-bit row numbers (rows to recompute completely).  If a list overflows, `overflow` is set and
-// the second stage recomputes every row instead.
+// Work lists that the tensor-core quantizers leave in the caller's scratch buffer for the exact second stage: entries
+// row << 8 | coordinate (64 bits: a rotated coordinate inside the guard band of a boundary) and row numbers (32 bits: rows to
+// recompute completely), behind this header (64 bytes).
+//
+// d <= 128: every block of the quantizer has lists of its own, code_cap and row_cap entries long, and leaves their lengths in
+// counts[2 * block] and counts[2 * block + 1] (a length above the list's says that the block's rows have to be done again, all of
+// them).  Nothing has to be cleared before a call, and block b of the second stage takes what block b left.
+// d = 256: one pair of lists, whose lengths the header counts; if one overflows, `overflow` is set and the second stage recomputes
+// every row.
+// Row numbers on the lists of d <= 128; the bit above: the row has no codes yet (its norm is outside the tensor-core kernel's range).
+constexpr unsigned int kRowNumber = 0x7fffffffu;
 struct TqRecheckHeader {
     unsigned int n_codes;    // entries appended to the coordinate list (may exceed code_cap)
-    unsigned int n_rows;     // entries appended to the row list (may exceed row_cap)
+    unsigned int n_rows;     // entries appended to the row list (may exceed row_cap); d <= 128: rows done again, over all blocks
     unsigned int overflow;
     unsigned int changed;    // diagnostic: codes the exact arithmetic decided differently
     unsigned int whole_rows; // non-zero: some listed rows have no codes yet (norms outside the tensor-core kernel's range)
-    unsigned int pad[11];
+    unsigned int done;       // d <= 128: blocks of the second stage that have finished
+    unsigned int pad[10];
 };
 struct TqRecheck {
     TqRecheckHeader* hdr;
+    unsigned int* counts;    // d <= 128
     unsigned long long* code_entries;
     unsigned int* row_entries;
     unsigned int code_cap, row_cap;
@@ -204,6 +212,9 @@ struct TqSecondStage {
     TqQuantOut out;
     TqRecheck lists;
 };
+// d <= 128, in one launch; it raises the length of the cache (advance != 0) and leaves the number of rows done again in the plans' counters.
+int tq_launch_second_stage(const TqSecondStage* a, const TqSecondStage* b, int advance, cudaStream_t st);
+// d = 256
 int tq_launch_exact_code_check(const TqSecondStage* a, const TqSecondStage* b, cudaStream_t st);
 int tq_launch_exact_listed(const TqSecondStage* a, const TqSecondStage* b, int advance, cudaStream_t st);
 // All rows of one call into the rows of a cache.
@@ -223,6 +234,8 @@ bool tq_tensor_wide_supported(int d, int bits, bool has_projection);
 int tq_tensor_plan_init(tq_plan* p, const float* rotation, const float* codebook, const float* projection);
 void tq_tensor_plan_free(tq_plan* p);
 bool tq_tensor_input_supported(int d, int xtype);
+// Blocks of the quantizer for n rows.
+int tq_tensor_quantize_blocks(const tq_plan* p, int64_t n);
 int tq_launch_tensor_quantize(const tq_plan* p, bool prod, const void* x, int xtype, int64_t n, const TqQuantOut& out,
                               const TqRecheck* lists, cudaStream_t st);
 

@@ -14,6 +14,7 @@
 // These kernels serve arbitrary (d <= 1024, bits <= 8), single tokens appended to a cache and small batches; they are
 // also the second stage of the tensor-core quantizers, which hand over lists of coordinates and rows to re-decide.
 #include "tq_common.cuh"
+#include "tq_ptx.cuh"
 
 namespace {
 
@@ -629,13 +630,416 @@ exact_quantize_tile_kernel(const __grid_constant__ RowsJob first, const __grid_c
     if (advance && t == 0) advance_length(job, rows.len0, advance);
 }
 
-// Listed coordinates (those inside the guard band of the tensor-core kernel) re-decided in the reference's order: norm, division and
-// the rotated coordinate as one FMA chain.  A wrong code is corrected in place and (TurboQuantProd) puts its row on the row
-// list.  Work is small -- 20,000 entries of 1,048,576 rows -- and every dependent access to global memory costs
-// about a microsecond, so the kernel is as long as its chain of such accesses: header and entry, then row, matrix row and
-// boundaries together.  Eight lanes fetch an entry's rows, normalise and leave both in shared memory; then a
-// lane per entry runs the chain, 32 entries side by side.  (One lane per entry for everything, 128 divisions in a row:
-// 18 us for the entries of 1,048,576 rows, now 8.7; 12.6 and 5.7 for 65,536.)
+// ------------------------------------------------------------------------------------------------
+// Second stage of the tensor-core quantizers, d <= 128: block b takes what block b of the quantizer left on its lists.  No list, counter
+// or matrix is shared with another block, so nothing is cleared before, and one launch does what a memset, a kernel for the
+// coordinates and a kernel for the rows did.  Work is small -- 70 coordinates and 16 rows a block of 1,048,576 TurboQuantProd keys at
+// d = 128 -- so the kernel is as long as its chain of dependent steps: while eight lanes a coordinate re-decide those (of the keys and
+// the values of a cache alike), eight warps fetch and normalise the listed rows, and the matrices come into shared memory; then
+// the products of all rows side by side, four rows x four columns a thread.  Listed rows keep their codes, which the first half settles.
+// 1,048,576 TurboQuantProd keys: 23 us behind the quantizer (37, and 6 in front of it, in three operations); 65,536 TurboQuantMSE
+// rows 7.5 (11 and 4).  Of 36 K cycles the coordinates take 11 K (entry, row and matrix row from L2 or HBM, 16 divisions, a chain of
+// 128), codes and matrices 7 K, a product 8 to 9 K: each piece of code runs once, and its instructions come from L2.
+// ------------------------------------------------------------------------------------------------
+struct StageJob {
+    RowsJob rows;            // lists, redo_counter and map among it
+    int blocks;              // blocks of its quantizer
+};
+constexpr int kStageThreads = 1024;
+constexpr int kStageRows = 32;                                  // rows side by side: 16 +- 4 a block in the case above
+constexpr int kProductRows = 4;                                 // rows x four columns of a product's thread (8: 11 to 16 K cycles a
+                                                                // product instead of 8, too few warps and registers)
+constexpr int kStageLoaders = kStageRows * 8;                   // threads that fetch rows, the last ones of the block
+constexpr int kStageCheckers = kStageThreads - kStageLoaders;   // the others: coordinates first
+constexpr int kStageExtra = 128;                                // rows whose codes the coordinates changed
+
+template <int D>
+struct StageSmem {
+    static constexpr int kRS = kStageRows + 4;                 // vectors lie transposed, [k][row]
+    static constexpr int kVec = D * kRS, kCodeRow = 128 + 8;
+    static constexpr int bytes(int matrices) { return (matrices * D * D + 2 * kVec) * 4 + kStageRows * kCodeRow; }
+};
+struct StageWait {           // of a plan: limit of a bounded wait, status word
+    int kcycles;
+    unsigned long long* status;
+};
+
+template <int D>
+__global__ void __launch_bounds__(kStageThreads, 1)
+second_stage_kernel(const __grid_constant__ StageJob first, const __grid_constant__ StageJob second, int njobs, int advance, const StageWait wait) {
+    using namespace tqptx;
+    using L = StageSmem<D>;
+    constexpr int RS = L::kRS, V = D / 8;
+    extern __shared__ __align__(16) float smem[];
+    float* vt = smem;                                          // [D][RS] unit vectors, later residuals
+    float* ct = vt + L::kVec;                                  // [D][RS] centroids
+    uint8_t* cs = reinterpret_cast<uint8_t*>(ct + L::kVec);    // [kStageRows][kCodeRow]
+    float* mats = reinterpret_cast<float*>(cs + kStageRows * L::kCodeRow);      // R (or Rt), St: [k][column]
+    __shared__ __align__(8) uint64_t arrived;                  // matrices
+    __shared__ int give_up[2];                                 // flag, limit of a wait
+    __shared__ float bnds[2][64], cbks[2][64];
+    __shared__ unsigned int extra[kStageExtra], n_extra;
+    __shared__ int64_t dst_row[kStageRows], src_row[kStageRows];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, l8 = t & 7, b = blockIdx.x;
+    // Matrices come in by bulk copies (cp.async of the whole block would stand before every other load of the SM: entries took 5 K
+    // cycles to arrive).  One thread asks, everybody waits.
+    uint32_t phase = 0;
+    // (in pieces, every block starting at another one: all of them read the same lines)
+    auto fetch_matrices = [&](const float* first_matrix, const float* second_matrix) {      // into the first place, and the second
+        if (warp != 0) return;
+        constexpr int kPieces = 16, kPiece = D * D / kPieces;
+        const int n = second_matrix ? 2 * kPieces : kPieces;
+        if (lane == 0) {
+            fence_async_smem();
+            mbar_arrive_expect_tx(smem_u32(&arrived), (uint32_t)(n * kPiece * 4));
+        }
+        __syncwarp();
+        if (lane < n) {
+            const int piece = (lane + b) % n;
+            const float* src = (piece < kPieces ? first_matrix : second_matrix) + (piece % kPieces) * kPiece;
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                         ::"r"(smem_u32(mats + piece * kPiece)), "l"(src), "r"(kPiece * 4), "r"(smem_u32(&arrived)) : "memory");
+        }
+    };
+    auto matrices_here = [&]() {                                     // (the whole block; false: the wait ran out)
+        const bool ok = mbar_wait(smem_u32(&arrived), phase, give_up);
+        phase ^= 1u;
+        return __syncthreads_and(ok) != 0;
+    };
+    if (t == 0) {
+        mbar_init(smem_u32(&arrived), 1);
+        give_up[0] = 0;
+        give_up[1] = wait.kcycles;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    bool pending = first.rows.prod != 0;                       // matrices asked for that nobody has waited for
+    if (pending) fetch_matrices(first.rows.p.R, first.rows.p.St);   // (a TurboQuantProd call leaves rows as a rule, a TurboQuantMSE call none)
+    for (int i = t; i < kStageRows * L::kCodeRow; i += kStageThreads) cs[i] = 0;
+    if (t < 128) {
+        const TqDev& p = t < 64 ? first.rows.p : second.rows.p;
+        const int i = t & 63;
+        if (i < p.levels) cbks[t >> 6][i] = __ldg(p.codebook + i);
+        if (i + 1 < p.levels) bnds[t >> 6][i] = __ldg(p.boundaries + i);
+    }
+    if (t == 0) n_extra = 0;
+    tq_grid_release();
+    tq_grid_wait();         // (only constants of the plans have been read so far)
+
+    // lengths of this block's lists; a list that overflowed says: all rows of the block's tiles
+    auto length_of = [&](const StageJob& j, int which) { return b < j.blocks ? j.rows.lists.counts[2 * b + which] : 0u; };
+    unsigned int nc[2] = {length_of(first, 0), 0u}, nr[2] = {length_of(first, 1), 0u};
+    if (njobs > 1) { nc[1] = length_of(second, 0); nr[1] = length_of(second, 1); }
+    bool whole[2];
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+        const TqRecheck& l = w == 0 ? first.rows.lists : second.rows.lists;
+        whole[w] = nc[w] > l.code_cap || nr[w] > l.row_cap;
+        if (whole[w]) nc[w] = nr[w] = 0;
+    }
+    auto source = [&](const RowsJob& job) {
+        RowSource rows;
+        rows.mapped = job.map.tokens > 0;
+        rows.len0 = rows.mapped ? job.map.base : 0;
+        return rows;
+    };
+    // eight lanes fetch row src_row[r] and divide it by its norm (whole warps; lanes without a row, `mine` false, keep the warp's
+    // shuffles company over its first row, which is there, and write nothing)
+    auto fetch_row = [&](const RowsJob& job, int r, bool mine) {
+        float* v = vt + (mine ? r : r & ~3);
+        if (mine) load_row(v, RS, D, l8, job.x, job.xtype, src_row[r]);
+        __syncwarp();
+        const float n2 = __fsqrt_rn(np_sumsq8<RS>(v, D, l8));
+        __syncwarp();
+        if (mine) divide_row(v, RS, D, l8, n2);
+        if (mine && l8 == 0 && dst_row[r] >= 0) job.norms[dst_row[r]] = n2;
+    };
+    __syncthreads();
+
+    // -- coordinates: norm, division and the rotated coordinate as one FMA chain that goes from lane to lane (lane l has the values
+    // [l V, + V) of the row); the first job's listed rows beside it
+    const unsigned int head = nr[0] < kStageRows ? nr[0] : kStageRows;       // rows of the first batch
+    if (t >= kStageCheckers) {
+        const int r = (t - kStageCheckers) >> 3;
+        const bool mine = r < (int)head;
+        if (l8 == 0 && mine) {
+            const int64_t row = (int64_t)(first.rows.lists.row_entries[(size_t)b * first.rows.lists.row_cap + r] & kRowNumber);
+            src_row[r] = row < first.rows.n ? row : -1;
+            dst_row[r] = source(first.rows).dst(first.rows, src_row[r]);
+        }
+        __syncwarp();
+        if ((r & ~3) < (int)head) fetch_row(first.rows, r, mine);
+    } else {
+        for (unsigned int base = 0; base < nc[0] + nc[1]; base += kStageCheckers / 8) {
+            const unsigned int at = base + (t >> 3);
+            const int w = at >= nc[0];
+            const RowsJob& job = w ? second.rows : first.rows;
+            const TqDev& p = job.p;
+            const bool given = at < nc[0] + nc[1];
+            const unsigned long long ent = given ? job.lists.code_entries[(size_t)b * job.lists.code_cap + (at - (w ? nc[0] : 0u))] : 0ull;
+            const int64_t row = (int64_t)(ent >> 8);
+            const int j = (int)(ent & 255u);
+            const bool valid = given && row < job.n && j < D;
+            if (!__any_sync(0xffffffffu, valid)) continue;
+            const int64_t to = source(job).dst(job, valid ? row : 0);
+            uint32_t* crow = job.codes + to * p.code_words;
+            const uint32_t old = valid && l8 == 7 ? tq_get_code(crow, j, p.bits) : 0u;
+            const int64_t first_value = (valid ? row : 0) * D;
+            float a[V], c[V];        // values l, l + 8, ... (NumPy's eight interleaved sums); values [l V, + V)
+            if (first.rows.xtype == TQ_INPUT_F32) {              // (the jobs of a call have one element type)
+                const float* x = static_cast<const float*>(job.x) + first_value;
+#pragma unroll
+                for (int i = 0; i < V; ++i) a[i] = __ldg(x + l8 + 8 * i);
+#pragma unroll
+                for (int i = 0; i < V; i += 4) *reinterpret_cast<float4*>(c + i) = __ldg(reinterpret_cast<const float4*>(x + l8 * V + i));
+            } else {
+                const uint16_t* x = static_cast<const uint16_t*>(job.x) + first_value;
+#pragma unroll
+                for (int i = 0; i < V; ++i) {
+                    a[i] = widen(__ldg(x + l8 + 8 * i), first.rows.xtype);
+                    c[i] = widen(__ldg(x + l8 * V + i), first.rows.xtype);
+                }
+            }
+            float sum = __fmul_rn(a[0], a[0]);
+#pragma unroll
+            for (int i = 1; i < V; ++i) sum = __fadd_rn(sum, __fmul_rn(a[i], a[i]));
+#pragma unroll
+            for (int s = 1; s < 8; s <<= 1) sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, s));
+            float m[V];
+#pragma unroll
+            for (int i = 0; i < V; i += 4) *reinterpret_cast<float4*>(m + i) = __ldg(reinterpret_cast<const float4*>(p.R + (size_t)(valid ? j : 0) * D + l8 * V + i));
+            const float n2 = __fsqrt_rn(sum);
+#pragma unroll
+            for (int i = 0; i < V; ++i) c[i] = n2 > 0.f ? __fdiv_rn(c[i], n2) : 0.f;
+            float acc = 0.f;
+#pragma unroll 1
+            for (int s = 0; s < 8; ++s) {
+                const float before = __shfl_sync(0xffffffffu, acc, (lane & 24) + (s > 0 ? s - 1 : 0));
+                acc = s > 0 ? before : 0.f;
+#pragma unroll
+                for (int i = 0; i < V; ++i) acc = __fmaf_rn(c[i], m[i], acc);
+            }
+            const uint32_t code = valid && l8 == 7 ? (uint32_t)count_below(bnds[w], p.levels - 1, acc) : 0u;
+            unsigned int slot = ~0u;
+            if (old != code) {
+                atomicAdd(&job.lists.hdr->changed, 1u);
+                const uint32_t delta = old ^ code;
+                const int bit = j * p.bits, word = bit >> 5, sh = bit & 31;
+                atomicXor(crow + word, delta << sh);
+                if (sh + p.bits > 32) atomicXor(crow + word + 1, delta >> (32 - sh));
+                if (job.prod) {          // the row's residual is another one: it joins the rows, as it stands here
+                    const unsigned int pos = atomicAdd(&n_extra, 1u);
+                    if (pos < kStageExtra) extra[pos] = (unsigned int)row;
+                    slot = head + pos;
+                }
+            }
+            slot = __shfl_sync(0xffffffffu, slot, lane | 7);
+            if (slot < kStageRows) {
+#pragma unroll
+                for (int i = 0; i < V; ++i) vt[(l8 * V + i) * RS + slot] = c[i];
+                if (l8 == 7) job.norms[to] = n2;
+            }
+        }
+    }
+    __threadfence_block();
+    __syncthreads();
+    const unsigned int extras = n_extra;
+    if (extras > kStageExtra) whole[0] = true;
+    unsigned int placed = kStageRows - head < extras ? kStageRows - head : extras;
+    if (t < (int)placed) {
+        const int64_t row = extra[t];
+        src_row[head + t] = row;
+        dst_row[head + t] = source(first.rows).dst(first.rows, row);
+    }
+
+    // -- rows in batches: the one that stands in shared memory, the rest of the lists, or all rows of the block's tiles
+    for (int which = 0; which < njobs; ++which) {
+        const StageJob& stage = which == 0 ? first : second;
+        const RowsJob& job = stage.rows;
+        const TqDev& p = job.p;
+        const bool prod = job.prod != 0;
+        const RowSource rows = source(job);
+        const float* bnd = bnds[which];
+        const float* cbk = cbks[which];
+        const uint32_t inv_bits = inverse_of_bits(p.bits);
+        const bool all = whole[which];
+        int64_t total = which == 0 ? (int64_t)nr[0] + extras : nr[1], next = 0;
+        int ready = which == 0 && !all ? (int)(head + placed) : 0;           // rows of this batch that stand in shared memory
+        if (all) {
+            const int64_t tiles = (job.n + 127) / 128;
+            total = b < tiles ? (tiles - b + stage.blocks - 1) / stage.blocks * 128 : 0;
+        }
+        bool ok = true;
+        if (total > 0 && which == 1) {
+            if (pending) ok = matrices_here();       // the first job had no rows: another copy may not meet its matrices
+            pending = false;
+            if (prod && ok) {
+                fetch_matrices(p.R, p.St);
+                pending = true;
+            }
+        }
+        for (next = 0; next < total && ok;) {
+            int count = ready;
+            if (ready == 0) {
+                count = (int)(total - next < kStageRows ? total - next : kStageRows);
+                __syncthreads();                                         // (the batch before is written out)
+                if (t < kStageRows) {
+                    const int64_t i = next + t;
+                    int64_t row = -1;
+                    if (t < count) {
+                        if (all) row = (b + i / 128 * stage.blocks) * 128 + i % 128;
+                        else if (which == 1) row = (int64_t)job.lists.row_entries[(size_t)b * job.lists.row_cap + i];
+                        else if (i - placed < nr[0]) row = (int64_t)job.lists.row_entries[(size_t)b * job.lists.row_cap + (i - placed)];
+                        else row = (int64_t)extra[i - nr[0]];
+                        row &= kRowNumber;
+                        if (row >= job.n) row = -1;
+                    }
+                    src_row[t] = row;
+                    dst_row[t] = rows.dst(job, row);
+                }
+                __syncthreads();
+                if (t >= kStageCheckers) fetch_row(job, (t - kStageCheckers) >> 3, true);
+            }
+            ready = 0;
+            next += count;
+            // A listed row has its codes, settled above, unless its norm was outside the tensor-core kernel's range (its number says so).
+            bool odd = false;
+            if (t < count && !all) {
+                const int64_t i = next - count + t;
+                const int64_t at = i < head ? i : i - placed;
+                if (which == 1) odd = true;
+                else if (i < head || (i >= head + placed && at < nr[0])) odd = (job.lists.row_entries[(size_t)b * job.lists.row_cap + at] & ~kRowNumber) != 0;
+            }
+            const bool full = __syncthreads_or(odd || all || !prod) != 0;
+
+            // acc[q][u] = sum_k vec[k][8 warp + q] * M[k][4 lane + u]: one FMA per k, k ascending
+            const int product_warps = (count + kProductRows - 1) / kProductRows;
+            const bool product_role = warp < product_warps, in_range = 4 * lane < D;
+            auto product = [&](int place, const float* vec, float (&acc)[kProductRows][4]) {
+                const float* m = mats + place * D * D + (in_range ? 4 * lane : 0);
+                const float* v = vec + kProductRows * warp;
+                float2 two[kProductRows / 2][4];        // pairs of rows: fma.rn.f32x2 rounds each half as fma.rn.f32 does
+#pragma unroll
+                for (int q = 0; q < kProductRows / 2; ++q)
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) two[q][u] = make_float2(0.f, 0.f);
+#pragma unroll 2
+                for (int k = 0; k < D; ++k) {
+                    float a[kProductRows];
+#pragma unroll
+                    for (int q = 0; q < kProductRows; q += 4) *reinterpret_cast<float4*>(a + q) = *reinterpret_cast<const float4*>(v + k * RS + q);
+                    const float4 bb = *reinterpret_cast<const float4*>(m + k * D);
+                    const float col[4] = {bb.x, bb.y, bb.z, bb.w};
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+#pragma unroll
+                        for (int q = 0; q < kProductRows / 2; ++q)
+                            two[q][u] = __ffma2_rn(make_float2(a[2 * q], a[2 * q + 1]), make_float2(col[u], col[u]), two[q][u]);
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                    for (int q = 0; q < kProductRows / 2; ++q) {
+                        acc[2 * q][u] = two[q][u].x;
+                        acc[2 * q + 1][u] = two[q][u].y;
+                    }
+            };
+            float acc[kProductRows][4];
+            if (full) {
+                if (pending && !matrices_here()) { ok = pending = false; break; }
+                pending = false;
+                fetch_matrices(p.Rt, nullptr);       // (for the one product, in the place of R)
+                if (!matrices_here()) { ok = false; break; }
+                if (product_role) {
+                    product(0, vt, acc);
+#pragma unroll
+                    for (int q = 0; q < kProductRows; ++q) {
+                        int code[4];
+                        codes_of<4>(bnd, p.levels, acc[q], code);
+                        const int r = kProductRows * warp + q;
+                        if (in_range) {
+                            *reinterpret_cast<uint32_t*>(cs + r * L::kCodeRow + 4 * lane) = (uint32_t)code[0] | (uint32_t)code[1] << 8 | (uint32_t)code[2] << 16 | (uint32_t)code[3] << 24;
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) ct[(4 * lane + u) * RS + r] = cbk[code[u]];
+                        }
+                    }
+                }
+                __syncthreads();
+                if (prod) fetch_matrices(p.R, nullptr);
+                for (int i = t; i < count * p.code_words; i += kStageThreads) {
+                    const int r = i / p.code_words, w = i - r * p.code_words;
+                    if (dst_row[r] >= 0) job.codes[dst_row[r] * p.code_words + w] = packed_code_word(cs + r * L::kCodeRow, p.bits, inv_bits, w);
+                }
+                if (!prod) continue;
+                if (!matrices_here()) { ok = false; break; }
+            } else {
+                // (through L2, where the corrections went)
+                for (int i = t; i < count * D; i += kStageThreads) {
+                    const int r = i / D, j = i % D, bit = j * p.bits, w = bit >> 5, sh = bit & 31;
+                    const uint32_t* row = job.codes + (dst_row[r] < 0 ? 0 : dst_row[r]) * p.code_words + w;
+                    uint32_t v = __ldcg(row) >> sh;
+                    if (sh + p.bits > 32) v |= __ldcg(row + 1) << (32 - sh);
+                    ct[j * RS + r] = cbk[v & ((1u << p.bits) - 1u)];
+                }
+                if (pending && !matrices_here()) { ok = pending = false; break; }
+                pending = false;
+                __syncthreads();
+            }
+            if (product_role) {          // residual = unit - centroids * R, in place (only this thread touches its elements)
+                product(0, ct, acc);
+                if (in_range) {
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+#pragma unroll
+                        for (int q = 0; q < kProductRows; q += 4) {
+                            float4* at = reinterpret_cast<float4*>(vt + (4 * lane + u) * RS + kProductRows * warp + q);
+                            const float4 unit = *at;
+                            *at = make_float4(__fsub_rn(unit.x, acc[q][u]), __fsub_rn(unit.y, acc[q + 1][u]), __fsub_rn(unit.z, acc[q + 2][u]), __fsub_rn(unit.w, acc[q + 3][u]));
+                        }
+                }
+            }
+            __syncthreads();
+            if (t >= kStageCheckers) {
+                const int r = (t - kStageCheckers) >> 3;
+                const float rn = __fsqrt_rn(np_sumsq8<RS>(vt + r, D, l8));
+                if (l8 == 0 && r < count && dst_row[r] >= 0) job.rnorms[dst_row[r]] = rn;
+            } else if (product_role) {
+                product(1, vt, acc);
+#pragma unroll
+                for (int q = 0; q < kProductRows; ++q) {
+                    uint32_t word = 0;           // the signs of 32 columns from eight lanes
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) word |= (acc[q][u] >= 0.f ? 1u : 0u) << (4 * l8 + u);
+#pragma unroll
+                    for (int s = 1; s < 8; s <<= 1) word |= __shfl_xor_sync(0xffffffffu, word, s);
+                    const int r = kProductRows * warp + q;
+                    if (l8 == 0 && in_range && r < count && dst_row[r] >= 0) job.signs[dst_row[r] * p.sign_words + (lane >> 3)] = tq_sign_word_from_natural(word);
+                }
+            }
+        }
+        if (!ok) break;
+        if (t == 0 && total > 0) atomicAdd(&job.lists.hdr->n_rows, (unsigned int)total);
+    }
+    if (pending) matrices_here();        // (nothing may land in shared memory that the block has left)
+    if (t == 0) {
+        if (give_up[0]) {
+            report_status(wait.status, 1ull);
+            mbar_drain(smem_u32(&arrived), phase ^ 1u);
+        }
+        __threadfence();
+        if (atomicAdd(&first.rows.lists.hdr->done, 1u) == gridDim.x - 1) {        // the last block has every block's sum
+            __threadfence();
+            if (first.rows.redo_counter) *first.rows.redo_counter = atomicAdd(&first.rows.lists.hdr->n_rows, 0u);
+            if (njobs > 1 && second.rows.redo_counter) *second.rows.redo_counter = atomicAdd(&second.rows.lists.hdr->n_rows, 0u);
+        }
+        if (advance) advance_length(first.rows, 0, advance);
+    }
+}
+
+// d = 256, listed coordinates (those inside the guard band of the tensor-core kernel) re-decided in the reference's order: norm, division
+// and the rotated coordinate as one FMA chain.  A wrong code is corrected in place and (TurboQuantProd) puts its row on the row
+// list.  Every dependent access to global memory costs about a microsecond, so the kernel is as long as its chain of such accesses:
+// header and entry, then row, matrix row and boundaries together.  Sixteen lanes fetch an entry's rows, normalise and leave both in
+// shared memory; then a lane per entry runs the chain, 16 entries side by side.
 struct CheckJob {
     TqDev p;
     const void* x;
@@ -646,13 +1050,12 @@ struct CheckJob {
     TqRowMap map;
 };
 
-template <int D>
 __global__ void __launch_bounds__(256)
 exact_code_check_kernel(const __grid_constant__ CheckJob first, const __grid_constant__ CheckJob second, int blocks0) {
-    constexpr int E = D > 128 ? 16 : 32, kLanes = 256 / E, kStep = E / (32 / kLanes);      // entries per block; lanes per entry
+    constexpr int D = 256, E = 16, kLanes = 256 / E, kStep = E / (32 / kLanes);      // entries per block; lanes per entry
     constexpr int kStride = D + 1;                                                      // odd: a column is free of bank conflicts
     __shared__ float vt[E * kStride], mt[E * kStride];
-    __shared__ float bnd[64];
+    __shared__ float bnd[16];
     __shared__ unsigned long long entry[E];      // ~0: none
     __shared__ uint32_t stored[E];               // the code that stands in the packed row
     const bool one = (int)blockIdx.x < blocks0;
@@ -663,7 +1066,7 @@ exact_code_check_kernel(const __grid_constant__ CheckJob first, const __grid_con
     // entries warp, warp + kStep, ... of the block: the lanes of different entries meet in different banks
     const int e = warp + kStep * (lane / kLanes), l = lane & (kLanes - 1);
     const TqRecheck& lists = job.lists;
-    if (t < p.levels - 1) bnd[t] = __ldg(p.boundaries + t);      // (at most 63: the tensor-core kernels take up to 6 bits)
+    if (t < p.levels - 1) bnd[t] = __ldg(p.boundaries + t);      // (at most 15: the kernel at d = 256 takes up to 4 bits)
     tq_grid_release();
     tq_grid_wait();
     // asked for before the header is known to allow it (the list's capacity bounds the index)
@@ -689,7 +1092,6 @@ exact_code_check_kernel(const __grid_constant__ CheckJob first, const __grid_con
         }
         if (l < 8) {
             load_row(v, 1, D, l, job.x, job.xtype, valid ? row : -1);
-            if (kLanes == 8) load_row(m, 1, D, l, p.R, TQ_INPUT_F32, valid ? j : -1);
         } else {
             load_row(m, 1, D, l - 8, p.R, TQ_INPUT_F32, valid ? j : -1);
         }
@@ -853,12 +1255,12 @@ int grid_for(int64_t work_items, int per_block) {
 int tq_launch_exact_code_check(const TqSecondStage* a, const TqSecondStage* b, cudaStream_t st) {
     TqRange range("tq.quantize.recheck_coordinates");
     const int d = a->plan->dev.d;
-    const int64_t per_block = d > 128 ? 16 : 32, most = tq_sm_count(a->plan->device) * (int64_t)(b ? 3 : 6);
+    if (d != 256) return tq_fail(TQ_ERR_UNSUPPORTED, "the coordinate re-check alone is written for d = 256");
+    const int64_t per_block = 16, most = tq_sm_count(a->plan->device) * (int64_t)(b ? 3 : 6);
     // as many blocks as a list of typical length has entries for (about 1 in 48 rows of 128 coordinates at 4 bits, in
     // proportion to the coordinates); longer lists take more passes
     auto blocks = [&](const TqSecondStage* s) {
-        // (a finer code has as many more boundaries)
-        const int64_t w = ((s->n * d / 128 << (s->plan->dev.bits > 4 ? s->plan->dev.bits - 4 : 0)) / 48 + per_block - 1) / per_block;
+        const int64_t w = (s->n * d / 128 / 48 + per_block - 1) / per_block;
         return (int)(w < 4 ? 4 : w > most ? most : w);
     };
     auto job = [](const TqSecondStage* s) {
@@ -869,11 +1271,7 @@ int tq_launch_exact_code_check(const TqSecondStage* a, const TqSecondStage* b, c
     };
     const CheckJob first = job(a), second = b ? job(b) : first;
     const int b0 = blocks(a), grid = b0 + (b ? blocks(b) : 0);
-    if (d == 128) TQ_CUDA_TRY(tq_launch_dependent(exact_code_check_kernel<128>, dim3(grid), dim3(256), 0, st, first, second, b0));
-    else if (d == 96) TQ_CUDA_TRY(tq_launch_dependent(exact_code_check_kernel<96>, dim3(grid), dim3(256), 0, st, first, second, b0));
-    else if (d == 64) TQ_CUDA_TRY(tq_launch_dependent(exact_code_check_kernel<64>, dim3(grid), dim3(256), 0, st, first, second, b0));
-    else if (d == 256) TQ_CUDA_TRY(tq_launch_dependent(exact_code_check_kernel<256>, dim3(grid), dim3(256), 0, st, first, second, b0));
-    else return tq_fail(TQ_ERR_UNSUPPORTED, "the coordinate re-check is written for d = 64, 96, 128 and 256");
+    TQ_CUDA_TRY(tq_launch_dependent(exact_code_check_kernel, dim3(grid), dim3(256), 0, st, first, second, b0));
     return TQ_OK;
 }
 
@@ -1011,14 +1409,38 @@ int tq_launch_exact_listed(const TqSecondStage* a, const TqSecondStage* b, int a
     };
     // A listed pass does not know its size on the host.  About one row in 450 of a TurboQuantProd call at d = 128 is listed
     // (the coordinate re-check and the sign guard), hardly any of a TurboQuantMSE call; the blocks stride on where it is more.
-    // (a bit more halves the residual, whose projections are then twice as often near zero)
-    auto rows = [](const TqSecondStage* s) {
-        const int bits = s->plan->dev.bits;
-        return s->prod ? (s->n * s->plan->dev.d / 128 << (bits > 4 ? bits - 3 : 0)) / 384 + 1 : s->n / 65536 + 1;
-    };
+    auto rows = [](const TqSecondStage* s) { return s->prod ? s->n * s->plan->dev.d / 128 / 384 + 1 : s->n / 65536 + 1; };
     const RowsJob first = job(a), second = b ? job(b) : first;
     const int64_t ra = rows(a), rb = b ? rows(b) : 0;
     return launch_rows(first, b ? &second : nullptr, ra > rb ? ra : rb, a->plan->device, advance, st);
+}
+
+template <int D>
+static int launch_stage(const StageJob& a, const StageJob* b, const tq_plan* plan, int advance, cudaStream_t st) {
+    const int device = plan->device;
+    const int bytes = StageSmem<D>::bytes(a.rows.prod || (b && b->rows.prod) ? 2 : 1), grid = b && b->blocks > a.blocks ? b->blocks : a.blocks;
+    TQ_GRANT_SMEM((second_stage_kernel<D>), bytes, device);
+    TQ_CUDA_TRY(tq_launch_dependent(second_stage_kernel<D>, dim3(grid), dim3(kStageThreads), (size_t)bytes, st, a, b ? *b : a, b ? 2 : 1, advance,
+                                    StageWait{plan->wait_kcycles, plan->status_dev}));
+    return TQ_OK;
+}
+
+int tq_launch_second_stage(const TqSecondStage* a, const TqSecondStage* b, int advance, cudaStream_t st) {
+    TqRange range("tq.quantize.second_stage");
+    auto job = [](const TqSecondStage* s) {
+        StageJob j;
+        j.rows = rows_job(s->plan, s->prod, s->x, s->xtype, s->n, s->out.codes, s->out.signs, s->out.rnorms, s->out.norms, &s->lists,
+                          s->plan->counters, &s->out.map);
+        j.blocks = tq_tensor_quantize_blocks(s->plan, s->n);
+        return j;
+    };
+    const StageJob first = job(a), second = b ? job(b) : first;
+    switch (a->plan->dev.d) {
+        case 64: return launch_stage<64>(first, b ? &second : nullptr, a->plan, advance, st);
+        case 96: return launch_stage<96>(first, b ? &second : nullptr, a->plan, advance, st);
+        case 128: return launch_stage<128>(first, b ? &second : nullptr, a->plan, advance, st);
+    }
+    return tq_fail(TQ_ERR_UNSUPPORTED, "the second stage in one launch is written for d = 64, 96 and 128");
 }
 
 // One step of a cache: the keys of `kp` (TurboQuantProd), the values of `vp` (TurboQuantMSE), or both (either plan may be

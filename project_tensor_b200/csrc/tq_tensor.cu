@@ -55,7 +55,6 @@ constexpr float kAccScale = kScaleA * kScaleB;  // accumulator = 2^20 * rotated 
 constexpr float kScaleRho = 1.f / 1024.f;       // accumulator units -> 2^10 * rho for the second A operand
 constexpr float kScaleM = 16.f;                 // R S^T -> second B operand
 constexpr int kCells = 32;
-constexpr int kPendCap = 32;               // second-stage entries staged per warp and list (a ballot adds up to 32)
 constexpr float kCellMul = 31.99998f;
 // 5- and 6-bit codes: a finer table in shared memory (Lloyd-Max boundaries of 6 bits are down to a 120th of their range apart)
 constexpr int kWideCells = 256;
@@ -110,14 +109,11 @@ struct Smem {
     static constexpr int off_b = 0;
     static constexpr int off_ring = off_b + kNumB * kBBytes;
     static constexpr int off_misc = off_ring + kRingBoxes * kBoxBytes;  // sumsq exchange, force flags, barriers
-    static constexpr int kPendWarps = Threads<PROD>::kConvWarps + 4 * Threads<PROD>::kEpiPerRow;   // every worker warp
-                                                                // stages entries: a 64-bit and a 32-bit list each
-    static constexpr int kPendBytes = kPendWarps * kPendCap * (8 + 4);
     static constexpr int kRsSlots = 4;                 // tiles whose |rho|^2 partial sums are alive at once
     static constexpr int kRsParts = 2;                 // threads per row in the first epilogue
     static constexpr int kRsBytes = kRsSlots * kRsParts * kTileRows * 4;
     static constexpr int kTableBytes = table_cells(BITS) * 8;
-    static constexpr int kMiscBytes = 8 * kTileRows * 4 + 4 * kTileRows + 512 + kRsBytes + kTableBytes + kPendBytes;
+    static constexpr int kMiscBytes = 8 * kTileRows * 4 + 4 * kTileRows + 512 + kRsBytes + kTableBytes;
     static constexpr int total = off_misc + kMiscBytes + 1024;      // + slack to align the base to 1024
     static_assert(total <= 227 * 1024, "shared memory plan");
 };
@@ -134,49 +130,6 @@ enum {
     BAR_ACC2_FULL = 26,           // [2]
     BAR_COUNT = 28
 };
-
-// Work for the exact second stage is rare (about one row in a hundred), but a global atomic per entry
-// would stall the epilogue warp for a memory round trip each time.  Every epilogue warp therefore
-// collects its entries in a private shared-memory buffer and reserves space in the global lists
-// once per batch.
-struct WarpPending {
-    unsigned long long* codes;  // [kPendCap]
-    unsigned int* rows;         // [kPendCap]
-    int n_codes, n_rows;        // warp-uniform
-};
-
-__device__ __noinline__ void flush_pending_codes(const TqRecheck& l, WarpPending& w, int lane) {
-    __syncwarp();
-    unsigned int base = 0;
-    if (lane == 0) base = atomicAdd(&l.hdr->n_codes, (unsigned int)w.n_codes);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    for (int i = lane; i < w.n_codes; i += 32) {
-        if (base + i < l.code_cap) l.code_entries[base + i] = w.codes[i];
-        else l.hdr->overflow = 1u;
-    }
-    __syncwarp();
-    w.n_codes = 0;
-}
-__device__ __noinline__ void flush_pending_rows(const TqRecheck& l, WarpPending& w, int lane) {
-    __syncwarp();
-    unsigned int base = 0;
-    if (lane == 0) base = atomicAdd(&l.hdr->n_rows, (unsigned int)w.n_rows);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    for (int i = lane; i < w.n_rows; i += 32) {
-        if (base + i < l.row_cap) l.row_entries[base + i] = w.rows[i];
-        else l.hdr->overflow = 1u;
-    }
-    __syncwarp();
-    w.n_rows = 0;
-}
-// Whole warp: every lane with `want` appends its row.
-__device__ __forceinline__ void pend_rows(const TqRecheck& l, WarpPending& w, bool want, int64_t row, int lane) {
-    const uint32_t votes = __ballot_sync(0xffffffffu, want);
-    if (votes == 0u) return;
-    if (w.n_rows + __popc(votes) > kPendCap) flush_pending_rows(l, w, lane);
-    if (want) w.rows[w.n_rows + __popc(votes & ((1u << lane) - 1u))] = (unsigned int)row;
-    w.n_rows += __popc(votes);
-}
 
 // One 32-column chunk of the first accumulator for one row: codes (packed into w), guard-band test,
 // and for TurboQuantProd the scaled residual split into fp16 hi/lo pairs;
@@ -263,24 +216,6 @@ __device__ __forceinline__ uint32_t process_chunk(const uint32_t (&v)[32], float
     return nearmask;
 }
 
-// Whole warp: every lane appends one (row, coordinate) entry per bit of its mask.  Called after the
-// accumulator has been handed back, so it never delays the tensor pipe.
-__device__ __noinline__ void pend_codes(const TqRecheck& l, WarpPending& w, uint32_t mask, int64_t row, int first_coord,
-                                        int lane) {
-    for (;;) {
-        const uint32_t votes = __ballot_sync(0xffffffffu, mask != 0u);
-        if (votes == 0u) break;
-        if (w.n_codes + __popc(votes) > kPendCap) flush_pending_codes(l, w, lane);
-        if (mask != 0u) {
-            const int e = __ffs(mask) - 1;
-            mask &= mask - 1;
-            w.codes[w.n_codes + __popc(votes & ((1u << lane) - 1u))] =
-                ((unsigned long long)row << 8) | (unsigned long long)(first_coord + e);
-        }
-        w.n_codes += __popc(votes);
-    }
-}
-
 // HALF: rows of bf16 or fp16, widened (exactly) by the converters; a TMA box then holds 64 columns.
 template <int D, int BITS, bool PROD, bool HALF, bool MAPPED>
 __global__ void __launch_bounds__(Threads<PROD>::kThreads, 1)
@@ -313,10 +248,10 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
     unsigned char* force = smem + L::off_misc + 8 * kTileRows * 4;                      // [4][128]
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::off_misc + 8 * kTileRows * 4 + 4 * kTileRows);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + BAR_COUNT);
-    float* rs_part = reinterpret_cast<float*>(smem + L::off_misc + L::kMiscBytes - L::kPendBytes - L::kRsBytes - L::kTableBytes);  // [kRsSlots][kRsParts][128]
-    float2* cell_lut = reinterpret_cast<float2*>(smem + L::off_misc + L::kMiscBytes - L::kPendBytes - L::kTableBytes);  // [table_cells]
-    unsigned char* pend_base = smem + L::off_misc + L::kMiscBytes - L::kPendBytes;
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    float* rs_part = reinterpret_cast<float*>(smem + L::off_misc + L::kMiscBytes - L::kRsBytes - L::kTableBytes);  // [kRsSlots][kRsParts][128]
+    float2* cell_lut = reinterpret_cast<float2*>(smem + L::off_misc + L::kMiscBytes - L::kTableBytes);  // [table_cells]
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);     // and the limit of a wait
+    unsigned int* listed = tmem_slot + 3;                                          // entries on the block's two lists
     const uint32_t bar0 = smem_u32(bars);
     auto BAR = [&](int i) { return bar0 + 8u * (uint32_t)i; };
 
@@ -337,6 +272,8 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
         mbar_init(BAR(BAR_ACC2_FULL + 1), 1);
         abort_flag[0] = 0;
         abort_flag[1] = a.wait_kcycles;
+        listed[0] = listed[1] = 0;
+        if (blockIdx.x == 0) { a.lists.hdr->n_rows = 0; a.lists.hdr->changed = 0; a.lists.hdr->done = 0; }      // sums of the second stage
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (threadIdx.x < table_cells(BITS)) cell_lut[threadIdx.x] = a.cell_lut[threadIdx.x];
@@ -514,11 +451,21 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
         const float lut_bnd = cell_lut[lane].x;
         const int lut_base1 = __float_as_int(cell_lut[lane].y);   // boundaries below the cell = code of a value below its boundary
         const float lut_ncent = a.code_ncent[lane];
-        WarpPending pend;
-        pend.codes = reinterpret_cast<unsigned long long*>(pend_base) + cw * kPendCap;
-        pend.rows = reinterpret_cast<unsigned int*>(pend_base + L::kPendWarps * kPendCap * 8) + cw * kPendCap;
-        pend.n_codes = 0;
-        pend.n_rows = 0;
+        // Work for the exact second stage: about one row in fifty has an entry, so every lane puts its own on the block's lists.  (Entries
+        // staged per warp, with a ballot per 32 columns and a global atomic per batch: 226 us per 1,048,576 TurboQuantProd rows of
+        // d = 128 instead of 205, 31 instead of 21 for 50,021 of d = 96.)
+        auto list_codes = [&](uint32_t mask, int64_t at_row, int first_coord) {
+            for (; mask != 0u; mask &= mask - 1u) {
+                const unsigned int pos = atomicAdd(listed, 1u);
+                if (pos < a.lists.code_cap)
+                    a.lists.code_entries[(size_t)blockIdx.x * a.lists.code_cap + pos] =
+                        ((unsigned long long)at_row << 8) | (unsigned long long)(first_coord + __ffs(mask) - 1);
+            }
+        };
+        auto list_row = [&](int64_t at_row, bool no_codes) {
+            const unsigned int pos = atomicAdd(listed + 1, 1u);
+            if (pos < a.lists.row_cap) a.lists.row_entries[(size_t)blockIdx.x * a.lists.row_cap + pos] = (unsigned int)at_row | (no_codes ? ~kRowNumber : 0u);
+        };
         int64_t g_base = 0;
 
         // -- sign epilogue of tile j (TurboQuantProd): second accumulator -> sign bits, residual norm, rows for the exact
@@ -531,8 +478,9 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
             const uint32_t par2 = (uint32_t)((j >> 1) & 1);
             const int64_t grow = tile * kTileRows + row, orow = output_row<MAPPED>(a, grow);
             TQ_PROF_CODE(const bool pr = a.prof && blockIdx.x == 0 && threadIdx.x == kFirstConvWarp * 32; long long c0 = clock64(), c1;)
-            bool redo_row = sc0 == 0 && force[(j & 3) * kTileRows + row] != 0;
+            bool redo_row = false;
             const bool live = mbar_wait(BAR(BAR_ACC2_FULL + b), par2, abort_flag) && grow < a.n;   // no stores after a give-up
+            const bool forced = force[(j & 3) * kTileRows + row] != 0;     // (listed once, by its first thread)
             tc_fence_after();
             TQ_PROF_CODE(c1 = clock64(); if (pr) prof_acc[18] += c1 - c0;)
             const uint32_t acc2 = tmem + lane_addr + A_COL(b ^ 1);
@@ -587,7 +535,7 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
                 } else if (kSignChunks == 2) *reinterpret_cast<uint2*>(a.signs + orow * (D / 32) + sc0) = make_uint2(sw0, sw1);
                 else a.signs[orow * (D / 32) + sc0] = sw0;
             }
-            pend_rows(a.lists, pend, redo_row && live, grow, lane);
+            if (live && (forced ? sc0 == 0 : redo_row)) list_row(grow, forced);
             TQ_PROF_CODE(if (pr) prof_acc[19] += clock64() - c1;)
         };
 
@@ -811,17 +759,11 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
             __syncwarp();
             if (lane == 0) mbar_arrive(BAR(PROD ? BAR_RHO_FULL + b : BAR_ACC_EMPTY + b));
             // second-stage work is recorded after the accumulator went back to the tensor pipe
-            uint32_t any_nm = 0;
+            if (live && !redo_row) {
 #pragma unroll
-            for (int ch = 0; ch < kEpiChunks; ++ch) {
-                if (!live || redo_row) nm[ch] = 0;
-                any_nm |= nm[ch];
+                for (int ch = 0; ch < kEpiChunks; ++ch) list_codes(nm[ch], grow, (chunk0 + ch) * 32);
             }
-            if (__any_sync(0xffffffffu, any_nm != 0u)) {
-#pragma unroll
-                for (int ch = 0; ch < kEpiChunks; ++ch) pend_codes(a.lists, pend, nm[ch], grow, (chunk0 + ch) * 32, lane);
-            }
-            if (!PROD) pend_rows(a.lists, pend, redo_row && live && chunk0 == 0, grow, lane);
+            if (!PROD && redo_row && live && chunk0 == 0) list_row(grow, true);
             TQ_PROF_CODE(if (pr) prof_acc[17] += clock64() - c1;)
         };
 
@@ -847,14 +789,13 @@ tensor_quantize_kernel(const __grid_constant__ CUtensorMap tmap_x, const TensorA
             const int64_t epi_tiles = epi_active ? my_tiles : 0;
             for (int64_t i = 0; i < epi_tiles; ++i) epilogue1(i);
         }
-        if (pend.n_codes > 0) flush_pending_codes(a.lists, pend, lane);
-        if (pend.n_rows > 0) flush_pending_rows(a.lists, pend, lane);
     }
 
     // ---- teardown -----------------------------------------------------------------------------------
     if (*abort_flag) __nanosleep(20000);   // tensor instructions issued before the give-up may still be running
     tc_fence_before();
     __syncthreads();
+    if (threadIdx.x < 2) a.lists.counts[2 * blockIdx.x + threadIdx.x] = listed[threadIdx.x];
     if (threadIdx.x == 0 && *abort_flag) report_status(a.status, 1ull);
 #ifdef TQ_PROF
     if (a.prof && blockIdx.x == 0) {
@@ -915,8 +856,9 @@ constexpr int off_bars = off_force + 4 * kTileRows;
 enum { X_FULL = 0, X_EMPTY = 8, B_FULL = 16, B_EMPTY = 24, A_FULL = 32, A_EMPTY = 34, ACC_FULL = 35, ACC_EMPTY = 37, RHO_FULL = 39, ACC2_FULL = 41, N_BARS = 43 };
 constexpr int off_lut = off_bars + 512;                          // barriers, tensor-memory slot, give-up flag; then the cell table
 constexpr int off_rs = off_lut + 512;                            // |rho|^2 partial sums [4 parts][128] (TurboQuantProd)
-constexpr int off_pend = off_rs + 4 * kTileRows * 4;
-constexpr int total = off_pend + kWorkers * kPendCap * (8 + 4) + 1024;
+constexpr int kListCap = 512;                                     // second-stage entries a block collects before they go to the lists
+constexpr int off_list = off_rs + 4 * kTileRows * 4;
+constexpr int total = off_list + kListCap * (8 + 4) + 1024;
 static_assert(total <= 227 * 1024, "shared memory plan");
 }  // namespace d256
 
@@ -934,7 +876,9 @@ tensor_quantize256_kernel(const __grid_constant__ CUtensorMap tmap_x, const Tens
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     float2* cell_lut = reinterpret_cast<float2*>(smem + off_lut);
     float* rs_part = reinterpret_cast<float*>(smem + off_rs);
-    unsigned char* pend_base = smem + off_pend;
+    unsigned long long* list_codes = reinterpret_cast<unsigned long long*>(smem + off_list);
+    unsigned int* list_rows = reinterpret_cast<unsigned int*>(list_codes + kListCap);
+    unsigned int* listed = tmem_slot + 3;                            // entries collected: coordinates, rows; then their places in the lists
     const uint32_t bar0 = smem_u32(bars);
     auto BAR = [&](int i) { return bar0 + 8u * (uint32_t)i; };
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -952,6 +896,7 @@ tensor_quantize256_kernel(const __grid_constant__ CUtensorMap tmap_x, const Tens
         }
         abort_flag[0] = 0;
         abort_flag[1] = a.wait_kcycles;
+        listed[0] = listed[1] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (threadIdx.x < kCells) cell_lut[threadIdx.x] = a.cell_lut[threadIdx.x];
@@ -1084,11 +1029,25 @@ tensor_quantize256_kernel(const __grid_constant__ CUtensorMap tmap_x, const Tens
         const float lut_bnd = cell_lut[lane].x;
         const int lut_base1 = __float_as_int(cell_lut[lane].y);
         const float lut_ncent = PROD ? a.code_ncent[lane] : 0.f;
-        WarpPending pend;
-        pend.codes = reinterpret_cast<unsigned long long*>(pend_base) + cw * kPendCap;
-        pend.rows = reinterpret_cast<unsigned int*>(pend_base + kWorkers * kPendCap * 8) + cw * kPendCap;
-        pend.n_codes = 0;
-        pend.n_rows = 0;
+        // Work for the exact second stage is rare (about one row in twenty has an entry): every lane puts its own into shared memory, or
+        // on the lists at once where that is full.
+        auto list_codes_of = [&](uint32_t mask, int64_t at_row, int first_coord) {
+            for (; mask != 0u; mask &= mask - 1u) {
+                const unsigned long long entry = ((unsigned long long)at_row << 8) | (unsigned long long)(first_coord + __ffs(mask) - 1);
+                unsigned int pos = atomicAdd(listed, 1u);
+                if (pos < kListCap) { list_codes[pos] = entry; continue; }
+                pos = atomicAdd(&a.lists.hdr->n_codes, 1u);
+                if (pos < a.lists.code_cap) a.lists.code_entries[pos] = entry;
+                else a.lists.hdr->overflow = 1u;
+            }
+        };
+        auto list_row = [&](int64_t at_row) {
+            unsigned int pos = atomicAdd(listed + 1, 1u);
+            if (pos < kListCap) { list_rows[pos] = (unsigned int)at_row; return; }
+            pos = atomicAdd(&a.lists.hdr->n_rows, 1u);
+            if (pos < a.lists.row_cap) a.lists.row_entries[pos] = (unsigned int)at_row;
+            else a.lists.hdr->overflow = 1u;
+        };
         bool fail = false;
         float scale = 0.f;          // of the tile whose norm was computed last
         // 64 columns [64 part, + 64) of the row: boxes 2 part and 2 part + 1, in the slots of the same numbers
@@ -1196,9 +1155,8 @@ tensor_quantize256_kernel(const __grid_constant__ CUtensorMap tmap_x, const Tens
                     for (int k = 0; k < BITS; ++k) dst[k] = w[k];
                 }
             }
-            if (!live || redo_row) nm = 0;
-            if (__any_sync(0xffffffffu, nm != 0u)) pend_codes(a.lists, pend, nm, grow, j * 128 + part * 32, lane);
-            if (!PROD && j == 0) pend_rows(a.lists, pend, redo_row && live && part == 0, grow, lane);
+            if (live && !redo_row) list_codes_of(nm, grow, j * 128 + part * 32);
+            if (!PROD && j == 0 && redo_row && live && part == 0) list_row(grow);
         };
         // -- TurboQuantProd: second accumulator of output half part >> 1 -> two sign words of the row, from the cells that this
         // thread fills again for the next tile (columns [32 h, + 32) and [64 + 32 h, + 32) with h = part & 1)
@@ -1236,7 +1194,7 @@ tensor_quantize256_kernel(const __grid_constant__ CUtensorMap tmap_x, const Tens
                 if (live) a.signs[orow * (kD / 32) + j * 4 + 2 * ch + hcol] = word;
             }
             tc_fence_before();
-            pend_rows(a.lists, pend, redo_row && live, grow, lane);
+            if (redo_row && live) list_row(grow);
         };
 
         if (my_tiles > 0) norm(0);
@@ -1259,14 +1217,26 @@ tensor_quantize256_kernel(const __grid_constant__ CUtensorMap tmap_x, const Tens
                 }
             }
         }
-        if (pend.n_codes > 0) flush_pending_codes(a.lists, pend, lane);
-        if (pend.n_rows > 0) flush_pending_rows(a.lists, pend, lane);
     }
 
     if (*abort_flag) __nanosleep(20000);   // tensor instructions issued before the give-up may still be running
     tc_fence_before();
     __syncthreads();
     if (threadIdx.x == 0 && *abort_flag) report_status(a.status, 1ull);
+    {   // what the block collected goes to the lists
+        const unsigned int nc = min(listed[0], (unsigned int)kListCap), nr = min(listed[1], (unsigned int)kListCap);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            listed[0] = nc ? atomicAdd(&a.lists.hdr->n_codes, nc) : 0u;
+            listed[1] = nr ? atomicAdd(&a.lists.hdr->n_rows, nr) : 0u;
+            if (listed[0] + nc > a.lists.code_cap || listed[1] + nr > a.lists.row_cap) a.lists.hdr->overflow = 1u;
+        }
+        __syncthreads();
+        for (unsigned int i = threadIdx.x; i < nc; i += kThreads)
+            if (listed[0] + i < a.lists.code_cap) a.lists.code_entries[listed[0] + i] = list_codes[i];
+        for (unsigned int i = threadIdx.x; i < nr; i += kThreads)
+            if (listed[1] + i < a.lists.row_cap) a.lists.row_entries[listed[1] + i] = list_rows[i];
+    }
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem, 512);
@@ -1392,8 +1362,8 @@ bool tq_tensor_quantize_supported(int d, int bits, bool has_projection) {
     return tq_tensor_supported(d, bits) || (d == 256 && bits >= 1 && bits <= 4);
 }
 // Geometries that only the quantizers and dequantizers have on tensor cores: d = 96, and codes of 5 and, without a projection, 6 bits.
-// TurboQuantProd, 5 code bits, 50,021 rows of d = 96: 47 us with the second stage (135 in the reference's order); 65,536 rows of
-// d = 128: 62 (265).  Residual norms against 64 bits: 3.2e-7 at 5 code bits (the residual is a thirtieth of the vector), 1.0e-7 at 3;
+// TurboQuantProd, 5 code bits, 50,021 rows of d = 96: 37 us with the second stage (135 in the reference's order); 65,536 rows of
+// d = 128: 50 (265).  Residual norms against 64 bits: 3.2e-7 at 5 code bits (the residual is a thirtieth of the vector), 1.0e-7 at 3;
 // in the reference's order 3.9 and 1.1e-7.
 bool tq_tensor_wide_supported(int d, int bits, bool has_projection) {
     if (tq_tensor_supported(d, bits)) return false;
@@ -1520,6 +1490,10 @@ static int launch_256(const tq_plan* p, const CUtensorMap& map, const TensorArgs
 }
 
 // The kernels that read 16-bit rows are those for d = 64 and 128.
+int tq_tensor_quantize_blocks(const tq_plan* p, int64_t n) {
+    const int64_t tiles = (n + kTileRows - 1) / kTileRows, sms = tq_sm_count(p->device);
+    return (int)(tiles < sms ? tiles : sms);
+}
 bool tq_tensor_input_supported(int d, int xtype) { return xtype == TQ_INPUT_F32 || d == 64 || d == 128; }
 
 int tq_launch_tensor_quantize(const tq_plan* p, bool prod, const void* x, int xtype, int64_t n, const TqQuantOut& out,
@@ -1558,8 +1532,7 @@ int tq_launch_tensor_quantize(const tq_plan* p, bool prod, const void* x, int xt
                                          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return tq_fail(TQ_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d", (int)r);
 
-    const int sms = tq_sm_count(p->device);
-    const int grid = (int)(args.ntiles < sms ? args.ntiles : sms);
+    const int grid = tq_tensor_quantize_blocks(p, n);
     const int bits = p->dev.bits;
     tq_timer_mark(p, 0, 0, st);
     int rc = TQ_ERR_UNSUPPORTED;
