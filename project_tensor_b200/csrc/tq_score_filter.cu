@@ -185,43 +185,56 @@ score_filter_kernel(const FilterArgs a) {
     const int64_t t0 = a.tiles * (int64_t)blockIdx.x / gridDim.x, t1 = a.tiles * (int64_t)(blockIdx.x + 1) / gridDim.x;
 
     if (warp == 0) {
-        if (lane == 0) {
+        // The whole warp walks the tiles and waits, one elected lane issues: a copy costs the lane of a diverged warp some 300 cycles,
+        // and there are four a tile (16,777,216 keys x 64 queries: 740 us with one lane walking, now 708).
+        if (elect_one()) {
             mbar_arrive_expect_tx(BAR(FB_B_FULL), L::kBBytes);
             bulk_load(smem_base + L::off_b, a.prep, L::kBBytes, BAR(FB_B_FULL));
-            int64_t issued = 0;
-            for (int64_t t = t0; t < t1; ++t) {
-                const int64_t i = t - t0;
-                const int s = (int)(i % kStages);
-                if (!mbar_wait(BAR(FB_K_EMPTY + s), (uint32_t)((i / kStages) & 1) ^ 1u, abort_flag)) break;
-                const int64_t row0 = t * a.tile_stride * kTileKeys;
-                int64_t valid = a.key_cnt - row0;
-                if (valid > kTileKeys) valid = kTileKeys;
-                const uint32_t cb = (uint32_t)valid * L::kCodeRow, sb = (uint32_t)valid * L::kSignRow, nb = (uint32_t)valid * 4u;
-                unsigned char* stage = smem + L::off_ring + s * L::kStage;
-                const uint32_t dst = smem_base + L::off_ring + s * L::kStage;
-                const unsigned char* src[4] = {a.codes + row0 * L::kCodeRow, a.signs + row0 * L::kSignRow,
-                                               reinterpret_cast<const unsigned char*>(a.norms + row0),
-                                               reinterpret_cast<const unsigned char*>(a.rnorms + row0)};
-                const uint32_t off[4] = {0u, (uint32_t)(kTileKeys * L::kCodeRow), (uint32_t)L::kNormOff, (uint32_t)(L::kNormOff + kTileKeys * 4)};
-                const uint32_t len[4] = {cb, sb, nb, nb};
-                uint32_t tx = 0;
+        }
+        __syncwarp();
+        int64_t issued = 0;
+        for (int64_t t = t0; t < t1; ++t) {
+            const int64_t i = t - t0;
+            const int s = (int)(i % kStages);
+            if (!warp_wait(BAR(FB_K_EMPTY + s), (uint32_t)((i / kStages) & 1) ^ 1u, abort_flag)) break;
+            const int64_t row0 = t * a.tile_stride * kTileKeys;
+            const uint32_t dst = smem_base + L::off_ring + s * L::kStage;
+            const unsigned char* src[4] = {a.codes + row0 * L::kCodeRow, a.signs + row0 * L::kSignRow,
+                                           reinterpret_cast<const unsigned char*>(a.norms + row0),
+                                           reinterpret_cast<const unsigned char*>(a.rnorms + row0)};
+            constexpr uint32_t off[4] = {0u, (uint32_t)(kTileKeys * L::kCodeRow), (uint32_t)L::kNormOff, (uint32_t)(L::kNormOff + kTileKeys * 4)};
+            if (a.key_cnt - row0 >= kTileKeys) {
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(BAR(FB_K_FULL + s), (uint32_t)L::kStage);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    copy_tail_words(stage + off[k], src[k], len[k]);
-                    tx += len[k] & ~15u;
+                    for (int k = 0; k < 4; ++k) bulk_load(dst + off[k], src[k], (k < 3 ? off[k < 3 ? k + 1 : 3] : (uint32_t)L::kStage) - off[k], BAR(FB_K_FULL + s));
                 }
-                mbar_arrive_expect_tx(BAR(FB_K_FULL + s), tx);
+            } else {         // the last tile: what is left of a row of bytes behind a multiple of 16 goes by plain loads
+                const uint32_t valid = (uint32_t)(a.key_cnt - row0);
+                const uint32_t len[4] = {valid * L::kCodeRow, valid * L::kSignRow, valid * 4u, valid * 4u};
+                if (lane == 0) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (len[k] & ~15u) bulk_load(dst + off[k], src[k], len[k] & ~15u, BAR(FB_K_FULL + s));
-                issued = i + 1;
+                    for (int k = 0; k < 4; ++k) copy_tail_words(smem + L::off_ring + s * L::kStage + off[k], src[k], len[k]);
+                }
+                __syncwarp();
+                if (elect_one()) {
+                    uint32_t tx = 0;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) tx += len[k] & ~15u;
+                    mbar_arrive_expect_tx(BAR(FB_K_FULL + s), tx);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (len[k] & ~15u) bulk_load(dst + off[k], src[k], len[k] & ~15u, BAR(FB_K_FULL + s));
+                }
             }
-            if (*abort_flag) {
-                // copies armed above may still be on their way into this block's shared memory
-                mbar_drain(BAR(FB_B_FULL), 0u);
-                for (int64_t ii = issued > kStages ? issued - kStages : 0; ii < issued; ++ii)
-                    mbar_drain(BAR(FB_K_FULL + (int)(ii % kStages)), (uint32_t)((ii / kStages) & 1));
-            }
+            __syncwarp();
+            issued = i + 1;
+        }
+        if (lane == 0 && *abort_flag) {
+            // copies armed above may still be on their way into this block's shared memory
+            mbar_drain(BAR(FB_B_FULL), 0u);
+            for (int64_t ii = issued > kStages ? issued - kStages : 0; ii < issued; ++ii)
+                mbar_drain(BAR(FB_K_FULL + (int)(ii % kStages)), (uint32_t)((ii / kStages) & 1));
         }
     } else if (warp == 1) {
         // The whole warp walks the tiles and waits; one elected lane issues, every operand from warp-uniform values.
