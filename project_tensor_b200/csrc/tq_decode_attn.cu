@@ -97,8 +97,8 @@ struct Plan {
     static constexpr int kLuts = kTables > kMerge ? kTables : kMerge;
     static constexpr int off_frag = kLuts;                               // two query operands
     static constexpr int off_slice = off_frag + (NQ == 8 ? 2 * kFragBytes : 0);   // [kSlices][2][NQ][DR] partial sums
-    static constexpr int off_vec = off_slice + kSlices * 2 * NQ * DR * 4;         // [2][NQ][DR] rotated, projected queries
-    static constexpr int off_qin = off_vec + 2 * NQ * DR * 4;            // [DR][NQ]
+    static constexpr int off_ops = off_slice + kSlices * 2 * NQ * DR * 4;         // four queries: [2][NQ][hi, lo][operand_row(DR)] fp16
+    static constexpr int off_qin = off_ops + (NQ == 4 ? (2 * NQ * 2 * operand_row(DR) * 2 + 15) / 16 * 16 : 0);   // [DR][NQ]
     static constexpr int off_small = off_qin + NQ * DR * 4;              // [2][NQ] scales, [kWarps][NQ] max, sum, factor
     static constexpr int total = off_small + (2 * NQ + 3 * kWarps * NQ) * 4;
 };
@@ -116,7 +116,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 decode_partial_kernel(TqDev kp, DecodeArgs a) {
     using P = Plan<KB, VB, DR, NQ>;
     extern __shared__ __align__(128) unsigned char smem[];
-    float* vec = reinterpret_cast<float*>(smem + P::off_vec);
+    __half* ops = reinterpret_cast<__half*>(smem + P::off_ops);
+    (void)ops;
     float* qin = reinterpret_cast<float*>(smem + P::off_qin);
     int* scl = reinterpret_cast<int*>(smem + P::off_small);                   // exponents of the queries' scales
     float* wm = reinterpret_cast<float*>(smem + P::off_small) + 2 * NQ;                                                    // [kWarps][NQ]
@@ -216,72 +217,73 @@ decode_partial_kernel(TqDev kp, DecodeArgs a) {
     // rotated[j] = sum_k q[k] R[j][k], projected[j] = sum_k q[k] S[j][k] in 32-bit arithmetic
     float* slice = reinterpret_cast<float*>(smem + P::off_slice);
     {
-        float4 sum[NQ];
 #pragma unroll
-        for (int qq = 0; qq < NQ; ++qq) sum[qq] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int qq = 0; qq < NQ; ++qq) {
+            float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (q0 + qq < a.qpg) {
 #pragma unroll
-        for (int u = 0; u < P::kSliceLen; ++u) {
-            const float* qk = qin + min(xk + u, DR - 1) * NQ;       // (meets a matrix element of zero behind the end)
-#pragma unroll
-            for (int qq = 0; qq < NQ; ++qq) {
-                const float v = qk[qq];
-                sum[qq].x = fmaf(v, mat[u].x, sum[qq].x);
-                sum[qq].y = fmaf(v, mat[u].y, sum[qq].y);
-                sum[qq].z = fmaf(v, mat[u].z, sum[qq].z);
-                sum[qq].w = fmaf(v, mat[u].w, sum[qq].w);
-            }
-        }
-#pragma unroll
-        for (int qq = 0; qq < NQ; ++qq) *reinterpret_cast<float4*>(slice + ((xs * 2 + xm) * NQ + qq) * DR + xj) = sum[qq];
-    }
-    __syncthreads();
-    for (int i = tid; i < 2 * NQ * DR; i += kThreads) {
-        float v = slice[i];
-#pragma unroll
-        for (int u = 1; u < P::kSlices; ++u) v += slice[u * 2 * NQ * DR + i];
-        vec[i] = v;
-    }
-    __syncthreads();
-    for (int v = warp; v < 2 * NQ; v += kWarps) {
-        float m = 0.f;
-        for (int k = lane; k < DR; k += 32) {
-            m = fmaxf(m, fabsf(vec[v * DR + k]));
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        }
-        if (lane == 0) {
-            scl[v] = scale_exp(m);
-        }
-    }
-    __syncthreads();
-    // Query operands.  Up to 4 queries: in registers, column r is hi (r < 4) or lo (r >= 4) of query r & 3.  Up to 8: in
-    // shared memory, (hi b0, hi b1, lo b0, lo b1) of query r per lane and step.
-    constexpr int kRegSteps = NQ == 4 ? P::kSteps : 1;
-    uint32_t qf[2][kRegSteps][2];
-    {
-        const int qq = NQ == 4 ? r & 3 : r;
-#pragma unroll
-        for (int m = 0; m < 2; ++m) {
-            const float* x = vec + (m * NQ + qq) * DR + t * (DR / 4);
-            const float sc = pow2i(scl[m * NQ + qq]);
-#pragma unroll
-            for (int s = 0; s < P::kSteps; ++s) {
-                if (NQ == 8 && s % kWarps != warp) continue;      // (each warp stores some of the steps)
-                uint32_t h0, l0, h1, l1;
-                split_pair(x[4 * s] * sc, x[4 * s + 1] * sc, h0, l0);
-                split_pair(x[4 * s + 2] * sc, x[4 * s + 3] * sc, h1, l1);
-                if constexpr (NQ == 4) {
-                    qf[m][s][0] = r < 4 ? h0 : l0;
-                    qf[m][s][1] = r < 4 ? h1 : l1;
-                } else {
-                    *reinterpret_cast<uint4*>(smem + P::off_frag + m * P::kFragBytes + (s * 32 + lane) * 16) = make_uint4(h0, h1, l0, l1);
+                for (int u = 0; u < P::kSliceLen; ++u) {
+                    const float v = qin[min(xk + u, DR - 1) * NQ + qq];       // (meets a matrix element of zero behind the end)
+                    sum.x = fmaf(v, mat[u].x, sum.x);
+                    sum.y = fmaf(v, mat[u].y, sum.y);
+                    sum.z = fmaf(v, mat[u].z, sum.z);
+                    sum.w = fmaf(v, mat[u].w, sum.w);
                 }
             }
+            *reinterpret_cast<float4*>(slice + ((xs * 2 + xm) * NQ + qq) * DR + xj) = sum;
         }
     }
-    if constexpr (NQ == 8) __syncthreads();
+    __syncthreads();
+    // A warp per vector: slices added up, scale, fp16 hi and lo parts where the operands are read.  Up to 4 queries: rows of parts, from
+    // which lane t of a quad takes the coordinates [t DR / 4, + DR / 4), four a step.  Up to 8: (hi b0, hi b1, lo b0, lo b1) of query r
+    // per lane and step.
+    for (int v = warp; v < 2 * NQ; v += kWarps) {
+        float x[DR / 32], m = 0.f;
+#pragma unroll
+        for (int i = 0; i < DR / 32; ++i) {
+            const int k = lane + 32 * i;
+            x[i] = slice[v * DR + k];
+#pragma unroll
+            for (int u = 1; u < P::kSlices; ++u) x[i] += slice[(u * 2 * NQ + v) * DR + k];
+            m = fmaxf(m, fabsf(x[i]));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        const int e = scale_exp(m);
+        const float sc = pow2i(e);
+        if (lane == 0) scl[v] = e;
+#pragma unroll
+        for (int i = 0; i < DR / 32; ++i) {
+            const int k = lane + 32 * i;
+            const float y = x[i] * sc;
+            const __half hi = __float2half_rn(y), lo = __float2half_rn(y - __half2float(hi));
+            if constexpr (NQ == 4) {
+                ops[(v * 2) * operand_row(DR) + k] = hi;
+                ops[(v * 2 + 1) * operand_row(DR) + k] = lo;
+            } else {
+                const int step = k % (DR / 4) / 4, to = v % NQ * 4 + k / (DR / 4);
+                __half* at = reinterpret_cast<__half*>(smem + P::off_frag + v / NQ * P::kFragBytes + (step * 32 + to) * 16) + k % 4;
+                at[0] = hi;
+                at[4] = lo;
+            }
+        }
+    }
+    __syncthreads();
+    // Query operands of up to 4 queries: column r is hi (r < 4) or lo (r >= 4) of query r & 3.
+    constexpr int kRegSteps = NQ == 4 ? P::kSteps : 1;
+    uint32_t qf[2][kRegSteps][2];
+    if constexpr (NQ == 4) {
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+            const uint2* x = reinterpret_cast<const uint2*>(ops + ((m * NQ + (r & 3)) * 2 + (r >> 2)) * operand_row(DR) + t * (DR / 4));
+#pragma unroll
+            for (int s = 0; s < P::kSteps; ++s) {
+                const uint2 w = x[s];
+                qf[m][s][0] = w.x;
+                qf[m][s][1] = w.y;
+            }
+        }
+    }
     // The two queries of this lane's score columns: descaling factors, softmax state.
     float ds1[2], ds2[2], mref[2], lsum[2];
     float wsc[2];                     // power of two that scales the weights

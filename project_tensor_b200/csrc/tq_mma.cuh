@@ -46,6 +46,10 @@ __device__ __forceinline__ int scale_exp(float m) {
     return min(max(13 - (int)((__float_as_uint(m) >> 23) - 127), -115), 100);      // (the largest float needs -114)
 }
 
+// Halves from one row of fp16 query operands to the next: eight rows (hi and lo of four queries) times four lanes of a quad, which
+// start d / 4 halves apart, read 8 bytes each from different banks.
+constexpr __host__ __device__ int operand_row(int d) { return d + 4; }
+
 // f(0), f(1), ... f(N - 1) with compile-time arguments
 template <int N, class F, int I = 0>
 __device__ __forceinline__ void for_steps(F&& f) {

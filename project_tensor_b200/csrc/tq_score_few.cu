@@ -16,8 +16,8 @@
 // chain: 3 to 12 % more error than the multiply-adds of the table kernel, two: 10 to 40 % less).
 //
 // Bound: shared-memory lookups, 64 8-byte loads a key at d = 128 and 3-bit codes (2 cycles a warp and load, four lanes a key), and for
-// few keys the prologue.  d = 128, 3-bit codes, one query: 262,144 keys 15.6 us (tables of the query's own products, a thread per
-// key: 19), 1,024 keys 7.0 (9.4); four queries x 1,048,576 keys 41 (84 in the table kernel for four queries that this one replaced).
+// few keys the prologue.  Kernel alone, 3-bit codes, one query, 256 / 262,147 keys: d = 64 2.7 / 8.1 us, d = 128 3.5 / 12.4,
+// d = 256 8.1 / 26.1 (4.1 / 9.5, 8.1 / 16.7, 16.5 / 35.2 with every lane splitting the queries for itself).
 // Where tables are the faster way (very many keys, very many groups): tq_score_table.cu.
 #include "tq_common.cuh"
 #include "tq_mma.cuh"
@@ -31,7 +31,7 @@ using namespace tqmma;
 constexpr int kFewThreads = 512;
 constexpr int kFewWarps = kFewThreads / 32;
 constexpr int kTile = 16;           // keys a warp takes at a time
-constexpr int NQ = 4;               // queries of a pass
+constexpr int kMaxQ = 4;            // queries of a pass
 
 struct FewArgs {
     const float* q;              // [groups][qpg][d]
@@ -44,32 +44,43 @@ struct FewArgs {
     float* scores;               // [groups][qpg][keys_per_group]
 };
 
-template <int KB, int DR>
+// NQ: queries whose vectors the prologue computes, one or four.
+template <int KB, int DR, int NQ>
 struct FewPlan {
     static constexpr int kSteps = DR / 16;
     static constexpr int kSlices = kFewThreads / (DR / 2), kSliceLen = DR / kSlices;   // four outputs of one matrix and a slice of the sum per thread
     static constexpr int off_slice = table_rows(KB) * kRowBytes;                     // [kSlices][2][NQ][DR] partial sums
-    static constexpr int off_vec = off_slice + kSlices * 2 * NQ * DR * 4;            // [2][NQ][DR] rotated, projected queries
-    static constexpr int off_qin = off_vec + 2 * NQ * DR * 4;                        // [DR][NQ]
+    static constexpr int off_ops = off_slice + kSlices * 2 * NQ * DR * 4;            // [2][NQ][hi, lo][operand_row(DR)] fp16: rotated, projected queries
+    static constexpr int off_qin = off_ops + (2 * NQ * 2 * operand_row(DR) * 2 + 15) / 16 * 16;     // [DR][NQ]
     static constexpr int off_small = off_qin + NQ * DR * 4;                          // [2][NQ] scales, [2][NQ] sums of the vectors
     static constexpr int total = off_small + 4 * NQ * 4;
     static_assert(total <= 227 * 1024, "shared memory plan");
 };
 
+// Where coordinate k of a query lies among the operands: lane t of a quad takes the coordinates [t DR / 4, + DR / 4), four a step; 1-bit
+// codes: coordinates that lie half a word apart make a pair.
+template <int DR, bool HALF_APART>
+__device__ __forceinline__ int operand_place(int k) {
+    if (!HALF_APART) return k;
+    constexpr int kHalf = DR == 64 ? 8 : 16;
+    const int lane_first = k / (DR / 4) * (DR / 4), rel = k % (DR / 4), i = rel % kHalf;
+    return lane_first + 4 * (rel / (2 * kHalf) * (kHalf / 2) + i / 2) + (i & 1) * 2 + (rel % (2 * kHalf) >= kHalf ? 1 : 0);
+}
+
 // grid (blocks over the keys, passes over the queries of a group, groups)
-template <int KB, int DR>
+template <int KB, int DR, int NQ>
 __global__ void __launch_bounds__(kFewThreads, 1)
 score_few_kernel(const TqDev p, const FewArgs a) {
-    using P = FewPlan<KB, DR>;
+    using P = FewPlan<KB, DR, NQ>;
     using W = KeyWords<KB, DR>;
     extern __shared__ __align__(128) unsigned char smem[];
-    float* vec = reinterpret_cast<float*>(smem + P::off_vec);
+    __half* ops = reinterpret_cast<__half*>(smem + P::off_ops);
     float* qin = reinterpret_cast<float*>(smem + P::off_qin);
     float* slice = reinterpret_cast<float*>(smem + P::off_slice);
     int* scl = reinterpret_cast<int*>(smem + P::off_small);                   // exponents of the queries' scales
     float* psum = reinterpret_cast<float*>(smem + P::off_small) + 2 * NQ;
 
-    const int g = blockIdx.z, q0 = blockIdx.y * NQ;
+    const int g = blockIdx.z, q0 = blockIdx.y * kMaxQ;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int t = lane & 3, r = lane >> 2;      // position in the quad, row of the fragments
     const uint32_t keys = (uint32_t)a.keys_per_group;            // rows of all groups together stay below 2^32
@@ -157,62 +168,61 @@ score_few_kernel(const TqDev p, const FewArgs a) {
         for (int qq = 0; qq < NQ; ++qq) *reinterpret_cast<float4*>(slice + ((tid / (DR / 2) * 2 + xm) * NQ + qq) * DR + xj) = sum[qq];
     }
     __syncthreads();
-    for (int v = warp; v < 2 * NQ; v += kFewWarps) {      // a warp per vector: slices added up, largest value, sum
-        float m = 0.f, sum = 0.f;
+    for (int v = warp; v < 2 * NQ; v += kFewWarps) {      // a warp per vector: slices added up, largest value, sum, fp16 parts
+        float m = 0.f, sum = 0.f, x[DR / 32];
 #pragma unroll
-        for (int k = lane; k < DR; k += 32) {
-            float x = slice[v * DR + k];
+        for (int i = 0; i < DR / 32; ++i) {
+            const int k = lane + 32 * i;
+            x[i] = slice[v * DR + k];
 #pragma unroll
-            for (int u = 1; u < P::kSlices; ++u) x += slice[(u * 2 * NQ + v) * DR + k];
-            vec[v * DR + k] = x;
-            m = fmaxf(m, fabsf(x));
-            sum += x;
+            for (int u = 1; u < P::kSlices; ++u) x[i] += slice[(u * 2 * NQ + v) * DR + k];
+            m = fmaxf(m, fabsf(x[i]));
+            sum += x[i];
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
             sum += __shfl_xor_sync(0xffffffffu, sum, o);
         }
+        const int e = scale_exp(m);
+        const float sc = pow2i(e);
+#pragma unroll
+        for (int i = 0; i < DR / 32; ++i) {
+            const int k = lane + 32 * i, at = KB == 1 && v < NQ ? operand_place<DR, true>(k) : operand_place<DR, false>(k);
+            const float y = x[i] * sc;
+            const __half h = __float2half_rn(y);
+            ops[(v * 2) * operand_row(DR) + at] = h;
+            ops[(v * 2 + 1) * operand_row(DR) + at] = __float2half_rn(y - __half2float(h));
+        }
         if (lane == 0) {
-            scl[v] = scale_exp(m);
+            scl[v] = e;
             psum[v] = sum;
         }
     }
     __syncthreads();
-    // Query operands: column r is hi (r < 4) or lo (r >= 4) of query r & 3.
+    // Query operands: column r is hi (r < 4) or lo (r >= 4) of query r & 3.  (Split once, by the warp that has the vector: every lane
+    // splitting what it needs, from rows whose words all lay in the same banks, took more than half of the prologue.)
     uint32_t qf[2][P::kSteps][2];
 #pragma unroll
     for (int m = 0; m < 2; ++m) {
-        const float* x = vec + (m * NQ + (r & 3)) * DR + t * (DR / 4);
-        const float sc = pow2i(scl[m * NQ + (r & 3)]);
+        const uint2* x = reinterpret_cast<const uint2*>(ops + ((m * NQ + (r & (NQ - 1))) * 2 + (r >> 2)) * operand_row(DR) + t * (DR / 4));
 #pragma unroll
         for (int s = 0; s < P::kSteps; ++s) {
-            uint32_t h0, l0, h1, l1;
-            float4 f;
-            if (KB == 1 && m == 0) {
-                // 1-bit codes: coordinates that lie half a word apart make a pair
-                constexpr int kHalf = DR == 64 ? 8 : 16;
-                const int at = 2 * s / kHalf * 32 + 2 * s % kHalf;
-                f = make_float4(x[at], x[at + kHalf], x[at + 1], x[at + 1 + kHalf]);
-            } else {
-                f = *reinterpret_cast<const float4*>(x + 4 * s);
-            }
-            split_pair(f.x * sc, f.y * sc, h0, l0);
-            split_pair(f.z * sc, f.w * sc, h1, l1);
-            qf[m][s][0] = r < 4 ? h0 : l0;
-            qf[m][s][1] = r < 4 ? h1 : l1;
+            const uint2 w = (r & 3) < NQ ? x[s] : make_uint2(0u, 0u);
+            qf[m][s][0] = w.x;
+            qf[m][s][1] = w.y;
         }
     }
     // the two queries of this lane's score columns
     float ds1[2], ds2[2], dbase[2] = {0.f, 0.f};
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
-        const int qq = (2 * t + c) & (NQ - 1);
+        const int qq = (2 * t + c) & (NQ - 1);         // (columns without a query: any)
         ds1[c] = pow2i(-scl[qq]) * p.cent_unit;
         if constexpr (KB == 1) {
             const float c0 = __ldg(p.codebook), c1 = __ldg(p.codebook + 1);
             ds1[c] = pow2i(-scl[qq]) * (0.5f * (c1 - c0));
-            dbase[c] = 2 * t < NQ ? 0.5f * (c0 + c1) * psum[qq] : 0.f;
+            dbase[c] = 2 * t < kMaxQ ? 0.5f * (c0 + c1) * psum[qq] : 0.f;
         }
         ds2[c] = pow2i(-scl[NQ + qq]) * p.alpha;
     }
@@ -281,20 +291,25 @@ score_few_kernel(const TqDev p, const FewArgs a) {
     }
 }
 
-template <int KB, int DR>
-int launch_few(const tq_plan* p, const FewArgs& a, int groups, cudaStream_t st) {
-    using P = FewPlan<KB, DR>;
-    TQ_GRANT_SMEM((score_few_kernel<KB, DR>), P::total, p->device);
-    const int passes = (a.qpg + NQ - 1) / NQ;
+template <int KB, int DR, int NQ>
+int launch_few_queries(const tq_plan* p, const FewArgs& a, int groups, cudaStream_t st) {
+    using P = FewPlan<KB, DR, NQ>;
+    TQ_GRANT_SMEM((score_few_kernel<KB, DR, NQ>), P::total, p->device);
+    const int passes = (a.qpg + kMaxQ - 1) / kMaxQ;
     // at most a block per SM over all groups, as many as run at once (the prologue costs 3 to 14 us: 64 groups in three blocks each
     // took two rounds of it, 28 us for 64 x 4,096 keys of d = 128), and every block of a group gets at least a tile per warp
     const int64_t tiles = (a.keys_per_group + kTile - 1) / kTile, most = (tiles + 3) / 4;
     int64_t blocks = tq_sm_count(p->device) / ((int64_t)passes * groups);
     if (blocks > most) blocks = most;
     if (blocks < 1) blocks = 1;
-    TQ_CUDA_TRY(tq_launch_dependent(score_few_kernel<KB, DR>, dim3((unsigned)blocks, (unsigned)passes, (unsigned)groups), dim3(kFewThreads),
+    TQ_CUDA_TRY(tq_launch_dependent(score_few_kernel<KB, DR, NQ>, dim3((unsigned)blocks, (unsigned)passes, (unsigned)groups), dim3(kFewThreads),
                                     (size_t)P::total, st, p->dev, a));
     return TQ_OK;
+}
+// One query: a quarter of the prologue's products.
+template <int KB, int DR>
+int launch_few(const tq_plan* p, const FewArgs& a, int groups, cudaStream_t st) {
+    return a.qpg == 1 ? launch_few_queries<KB, DR, 1>(p, a, groups, st) : launch_few_queries<KB, DR, 4>(p, a, groups, st);
 }
 }  // namespace
 

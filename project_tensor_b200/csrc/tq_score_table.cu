@@ -8,9 +8,9 @@
 //   byte table   [d/8 positions][256 entries]      sum over the 8 sign bits of the byte of +-(S q)[coordinate]
 //
 // and every thread walks the packed codes and sign words of one key: d/2 + d/8 lookups and additions, no unpacking.
-// score_few_kernel expands the keys for up to four queries at once; for one it pays that expansion alone (600,000 keys and more), and
-// it keeps an SM to itself for a prologue of 3 / 7 / 14 us at d = 64 / 128 / 256, where a block here takes 5 / 9 / 15 us but four to
-// eight run beside each other (hundreds of groups with a few keys each).  Anything between is its own.
+// score_few_kernel expands the keys for up to four queries at once; for one it pays that expansion alone (half a million to four million
+// keys), and it keeps an SM to itself for a prologue of 2 / 2 / 6 us at d = 64 / 128 / 256, where a block here takes 5 / 9 / 15 us but four to
+// eight run beside each other (a thousand groups with a few keys each).  Anything between is its own.
 #include "tq_common.cuh"
 
 #include <stdint.h>
@@ -140,22 +140,28 @@ int launch_table(const tq_plan* p, const float* q, const uint32_t* codes, const 
 
 }  // namespace
 
-// The lines lie where the two kernels meet (kernel time in us, warp-level kernel / this one; 1, 2, 3 code bits):
-//   one group   d = 64     400,000 keys  - / 10.2:11.2 / -              1,048,576 keys  - / 21.2:16.2 / -        (4 bits 22.5:25.5)
-//               d = 128    400,000 keys  20.1:19.5 / 18.8:19.8 / 19.8:22.0    1,048,576 keys  40.7:28.2 / 36.7:29.2 / 40.0:38.1
-//                          4,000,000 keys  137:90 / 124:95 / 132:118 (4 bits 130:190)
-//               d = 256    400,000 keys  36.4:37.0 / 38.5:38.7 / 43.1:53.8    2,000,000 keys  127:104 / 143:116 / 171:165
-//   groups      d = 128    2,048 x 32 keys  100:36 / 104:37 / 106:42 (4 bits 104:72)    4,096 x 512  270:155 / 273:160 / 279:167 (280:341)
-//               d = 64, 256, 2 and 3 bits    4,096 x 32  83:32, 445:194    4,096 x 512  116:75, 587:468    512 x 1,008  22:21, 102:120
-//               (d = 64, 4 bits, 4,096 x 512  129:108)
+// The lines lie where the two kernels meet (us, warp-level kernel / this one; 1, 2, 3 code bits):
+//   one group   d = 64     524,288 keys  14.6:13.0 / 14.3:14.7 / 14.9:14.9      1,048,576 keys  23:18 / 23:19 / 25:21      (4 bits 23:27)
+//               d = 128    524,288 keys  21:23 / 21:23 / 21:27                  800,000 keys  29:27 / 27:27 / 29:33
+//                          4,000,000 keys  119:90 / 111:95 / 122:117  (2,097,152 keys, 3 bits 68:74; 4 bits 118:189)
+//               d = 256    800,000 keys  51:50 / 54:62 / 69:82                  2,097,152 keys  117:107 / 124:120 / 157:171
+//   groups      d = 64     512 x 512  14.2:14.8 / 13.4:14.7 / 14.7:14.8         2,048 x 32  25:20 / 25:21 / 25:21     4,096 x 512  78:76 / 78:78 / 91:85
+//               d = 128    512 x 512  21:25 / 21:25 / 23:29                     2,048 x 32  39:39 / 35:40 / 35:46     2,048 x 256  50:45 / 52:45 / 55:50
+//                          4,096 x 512  136:157 / 142:164 / 150:170
+//               d = 256    512 x 512  44:50 / 45:52 / 51:68                     2,048 x 32  103:76 / 88:79 / 93:105   2,048 x 256  122:89 / 124:95 / 141:123
+//               4 bits, any d: 2,048 x 256  d = 64 33:31, d = 128 54:86
 bool tq_score_table_better(const tq_plan* p, int groups, int qpg, int64_t keys_per_group) {
     const int d = p->dev.d, bits = p->dev.bits;
-    if (!p->has_projection || bits < 1 || bits > 4 || (d == 256 && bits == 4)) return false;
-    // more groups than the other kernel runs at once, and one or two blocks for each
+    if (!p->has_projection || bits < 1 || bits > 3) return false;
+    // many more groups than the other kernel runs at once, and a block for each (d = 64: or two)
     const int64_t blocks = qpg * ((keys_per_group + kTableThreads - 1) / kTableThreads);
-    if (groups > tq_sm_count(p->device) && blocks <= (bits <= 3 || d == 64 ? 2 : 1)) return true;
-    if (qpg != 1 || bits == 4) return false;
-    return keys_per_group >= (bits <= 2 || d == 64 ? 1 << 19 : d == 128 ? 1 << 20 : 1 << 21);
+    if (groups > 6 * tq_sm_count(p->device)) {
+        if (d == 64 ? blocks <= 2 : blocks == 1 && ((d == 256 && bits <= 2) || keys_per_group > kTableThreads / 2)) return true;
+    }
+    if (qpg != 1) return false;
+    if (d == 64) return keys_per_group >= 1 << 19;
+    if (bits == 1 || (bits == 2 && d == 128)) return keys_per_group >= 3 << 18;
+    return keys_per_group >= (bits == 2 ? 1 << 21 : d == 128 ? 7 << 19 : 1 << 22);
 }
 
 // scores: [groups][qpg][keys_per_group]
@@ -169,7 +175,6 @@ int tq_launch_score_table(const tq_plan* p, const float* q, int groups, int qpg,
         case 1: return d == 256 ? TQ_TABLE(1, 256) : d == 128 ? TQ_TABLE(1, 128) : TQ_TABLE(1, 64);
         case 2: return d == 256 ? TQ_TABLE(2, 256) : d == 128 ? TQ_TABLE(2, 128) : TQ_TABLE(2, 64);
         case 3: return d == 256 ? TQ_TABLE(3, 256) : d == 128 ? TQ_TABLE(3, 128) : TQ_TABLE(3, 64);
-        case 4: if (d != 256) return d == 128 ? TQ_TABLE(4, 128) : TQ_TABLE(4, 64);
 #undef TQ_TABLE
     }
     return tq_fail(TQ_ERR_UNSUPPORTED, "no table kernel for d=%d bits=%d", d, p->dev.bits);

@@ -44,3 +44,24 @@ def test_queries_near_the_largest_float(d, bits):
     for scale in (2.0 ** 116, 2.0 ** 121):       # (S q itself is near the largest float)
         got = quant.attention_scores(queries * scale, enc) * (1.0 / scale)
         assert float((got - want).abs().max()) <= 1e-6 * float(want.abs().max()), scale
+
+
+@pytest.mark.parametrize("d,bits", [(64, 2), (64, 4), (128, 2), (128, 4), (256, 2), (256, 4)])
+def test_one_query_on_both_sides_of_the_table_kernels_lines(d, bits):
+    """Many groups with one or two blocks of keys each, and one group at the lowest count that takes tables."""
+    import torch
+    quant = tg.TurboQuantProd(d, bits, seed=2026)
+    gen = torch.Generator("cuda").manual_seed(d + bits)
+    for groups, qpg, n in ((888, 1, 33), (900, 1, 33), (900, 1, 128), (900, 1, 129), (900, 1, 256), (900, 1, 257), (900, 2, 250), (1, 1, (3 << 18) + 33)):
+        if groups * n * d > 1 << 27:
+            continue
+        keys = torch.randn(groups * n, d, device="cuda", generator=gen)
+        queries = torch.randn(groups * qpg, d, device="cuda", generator=gen) * 100
+        enc = quant.quantize(keys)
+        got = quant.attention_scores(queries, enc, groups=groups)
+        want = torch.einsum("gqd,gnd->gqn", queries.view(groups, qpg, d).double(),
+                            quant.dequantize(enc).double().view(groups, n, d)).reshape(groups * qpg, n)
+        knorm = keys.norm(dim=1).view(groups, 1, n).expand(groups, qpg, n).reshape(groups * qpg, n)
+        err = float(((got.double() - want).abs() / (queries.norm(dim=1)[:, None] * knorm)).max())
+        # (the reconstruction and the score are each within a few 1e-6 of the product of the norms)
+        assert err <= 1e-5, (groups, qpg, n, err)
