@@ -152,6 +152,16 @@ int tq_score_broadcast(const tq_plan* plan, const float* q, const void* codes, c
                        const float* residual_norms, const float* norms, int64_t n, float* scores,
                        void* stream);
 
+/*
+ * tq_score_broadcast for a caller whose query and scores are ordinary host memory (d and n floats, n at most TQ_HOST_SCORES): the
+ * query goes through a page-locked block of the plan, which the kernels read and write where it lies; the call waits for the
+ * stream and returns the scores in place.  *status: as of tq_plan_status, read and cleared behind the wait; scores
+ * of a call that leaves it non-zero may be incomplete.  Calls on several threads and streams each take a block of their own.
+ */
+#define TQ_HOST_SCORES 16384
+int tq_score_host(const tq_plan* plan, const float* q, const void* codes, const void* signs, const float* residual_norms,
+                  const float* norms, int64_t n, float* scores, int64_t* status, void* stream);
+
 /* Same formula with one query row per key (_quant.py:342-358).  q: float32[n*d]. */
 int tq_score_pairwise(const tq_plan* plan, const float* q, const void* codes, const void* signs,
                       const float* residual_norms, const float* norms, int64_t n, float* scores,

@@ -14,6 +14,7 @@ LIB_NAME = "libtq_sm100.so"
 
 TQ_OK = 0
 TQ_F32, TQ_BF16, TQ_F16 = 0, 1, 2
+TQ_HOST_SCORES = 16384
 TQ_PATH_AUTO, TQ_PATH_EXACT, TQ_PATH_TENSOR = 0, 1, 2
 
 # name -> (restype, argtypes); mirrors include/tq_b200.h one to one
@@ -38,6 +39,8 @@ SIGNATURES = {
     "tq_prod_dequantize": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p]),
     "tq_score_broadcast": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64,
                                    c_void_p, c_void_p]),
+    "tq_score_host": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, POINTER(c_int64),
+                              c_void_p]),
     "tq_score_pairwise": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64,
                                   c_void_p, c_void_p]),
     "tq_score_batched": (c_int, [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,

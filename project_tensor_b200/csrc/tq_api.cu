@@ -42,6 +42,50 @@ struct DeviceScope {
     }
 };
 
+// A page-locked block for one call on host memory: a query of up to TQ_MAX_DIM values, then up to TQ_HOST_SCORES scores.  A plan keeps the
+// blocks of calls that are over, as many as have run at a time but at most kIdleBlocks, until it is destroyed.
+constexpr int kIdleBlocks = 8;
+}  // namespace
+struct TqHostBlocks {
+    std::mutex lock;
+    float* idle[kIdleBlocks];
+    int count = 0;
+};
+namespace {
+std::mutex g_host_blocks_lock;       // makes a plan's first
+struct TqHostBlock {
+    TqHostBlocks* pool = nullptr;
+    float* at = nullptr;
+    explicit TqHostBlock(const tq_plan* plan) {
+        {
+            std::lock_guard<std::mutex> hold(g_host_blocks_lock);
+            tq_plan* p = const_cast<tq_plan*>(plan);
+            if (!p->host_blocks) p->host_blocks = new (std::nothrow) TqHostBlocks();
+            pool = p->host_blocks;
+        }
+        if (!pool) return;
+        {
+            std::lock_guard<std::mutex> hold(pool->lock);
+            if (pool->count > 0) at = pool->idle[--pool->count];
+        }
+        void* block = at;
+        if (!at && cudaHostAlloc(&block, sizeof(float) * (TQ_MAX_DIM + TQ_HOST_SCORES), cudaHostAllocPortable) == cudaSuccess) at = static_cast<float*>(block);
+    }
+    ~TqHostBlock() {
+        if (!at) return;
+        {
+            std::lock_guard<std::mutex> hold(pool->lock);
+            if (pool->count < kIdleBlocks) {
+                pool->idle[pool->count++] = at;
+                return;
+            }
+        }
+        cudaFreeHost(at);
+    }
+    TqHostBlock(const TqHostBlock&) = delete;
+    TqHostBlock& operator=(const TqHostBlock&) = delete;
+};
+
 int check_plan(const tq_plan* p, bool need_proj) {
     if (!p) return tq_fail(TQ_ERR_INVALID_ARGUMENT, "plan is null");
     if (need_proj && !p->has_projection)
@@ -271,6 +315,10 @@ int tq_plan_create(int d, int bits_mse, const float* rotation, const float* code
 void tq_plan_destroy(tq_plan* p) {
     if (!p) return;
     DeviceScope scope(p->device);
+    if (p->host_blocks) {
+        for (int i = 0; i < p->host_blocks->count; ++i) cudaFreeHost(p->host_blocks->idle[i]);
+        delete p->host_blocks;
+    }
     if (p->timer) {
         for (int k = 0; k < kTimerKinds; ++k)
             for (int i = 0; i < kTimerSlots; ++i) { cudaEventDestroy(p->timer->ev[k][i][0]); cudaEventDestroy(p->timer->ev[k][i][1]); }
@@ -593,6 +641,28 @@ int tq_score_broadcast(const tq_plan* p, const float* q, const void* codes, cons
     return tq_launch_score_general(p, q, 1, 1, static_cast<const uint32_t*>(codes), static_cast<const uint32_t*>(signs),
                                    residual_norms, norms, n, scores, 0, nullptr, nullptr, 0, nullptr, 0,
                                    static_cast<cudaStream_t>(stream));
+}
+
+int tq_score_host(const tq_plan* p, const float* q, const void* codes, const void* signs, const float* residual_norms, const float* norms,
+                  int64_t n, float* scores, int64_t* status, void* stream) {
+    TQ_TRY(check_plan(p, true));
+    if (!q || !scores || !status) return tq_fail(TQ_ERR_INVALID_ARGUMENT, "q, scores or status is null");
+    if (n < 0 || n > TQ_HOST_SCORES) return tq_fail(TQ_ERR_INVALID_ARGUMENT, "n outside [0, %d]", TQ_HOST_SCORES);
+    *status = 0;
+    if (n == 0) return TQ_OK;
+    DeviceScope scope(p->device);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    TqHostBlock block(p);
+    if (!block.at) return tq_fail(TQ_ERR_CUDA, "cudaHostAlloc of a block for a call on host memory failed");
+    float* out = block.at + TQ_MAX_DIM;
+    memcpy(block.at, q, sizeof(float) * (size_t)p->dev.d);
+    TQ_TRY(tq_score_broadcast(p, block.at, codes, signs, residual_norms, norms, n, out, stream));
+    TQ_CUDA_TRY(cudaStreamSynchronize(st));
+    const unsigned long long v = *p->status_host;
+    if (v != 0) *p->status_host = 0ull;   // reported once
+    *status = (int64_t)v;
+    memcpy(scores, out, sizeof(float) * (size_t)n);
+    return TQ_OK;
 }
 
 int tq_score_pairwise(const tq_plan* p, const float* q, const void* codes, const void* signs,

@@ -132,6 +132,7 @@ struct tq_plan {
     int wait_kcycles;              // limit of a bounded wait inside the tensor-core kernels, in units of 1024 cycles
     float c_max, beta_scale;       // first stage of long searches (tq_score_filter.cu): largest |centroid| and the power of two
                                    // that scales its sign operand; beta_scale 0: these constants do not fit fp16
+    struct TqHostBlocks* host_blocks;   // page-locked blocks of calls on host memory (tq_score_host)
     struct TqKernelTimer* timer;   // event pairs around the main kernels while tq_plan_time_kernels is on (else null)
 };
 

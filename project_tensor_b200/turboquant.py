@@ -265,10 +265,14 @@ class _PlanSet:
         status = ctypes.c_int64(0)
         _native.check(_native.load().tq_plan_status(h, _stream_ptr(device), ctypes.byref(status)))
         if status.value:
-            what = {1: "quantize", 2: "scoring", 3: "dequantize"}.get(status.value, "tensor-core")
-            raise _native.TurboQuantNativeError(
-                f"a {what} kernel gave up on a bounded wait (status {status.value}); the results of the calls "
-                f"since the last check are incomplete")
+            self.refuse(status.value)
+
+    @staticmethod
+    def refuse(status: int) -> None:
+        what = {1: "quantize", 2: "scoring", 3: "dequantize"}.get(status, "tensor-core")
+        raise _native.TurboQuantNativeError(
+            f"a {what} kernel gave up on a bounded wait (status {status}); the results of the calls "
+            f"since the last check are incomplete")
 
     def set_wait_limit(self, cycles: int) -> None:
         """Limit of one bounded wait inside the tensor-core kernels, in GPU cycles, for plans that exist already."""
@@ -669,6 +673,9 @@ class TurboQuantProd:
     def attention_score(self, query: Any, encoding: TurboQuantProdEncoding):
         """One query row broadcast over all keys, or one query row per key (_quant.py:334-358)."""
         pk = _as_packed(encoding, self._plans, need_signs=True)
+        if (type(query) is np.ndarray and query.size == self.dimension and query.shape[-1:] == (self.dimension,) and query.dtype.kind in "fiub"
+                and 1 < pk.n <= _native.TQ_HOST_SCORES and self._plans._path == _native.TQ_PATH_AUTO):
+            return self._score_on_host(query, pk, tuple(encoding.prefix_shape))
         staged = _stage_query(query, self.dimension, pk.device)
         q = staged.tensor
         num_codes = pk.n
@@ -681,7 +688,7 @@ class TurboQuantProd:
                 f"query batch size {staged.n} does not match encoding batch size {num_codes}"
             )
         lib = _native.load()
-        # a short row of scores for a NumPy caller is written straight to page-locked memory
+        # a short row of scores for a NumPy caller is written straight to page-locked memory (one query: _score_on_host)
         to_host = staged.kind == "numpy" and 4 * num_codes <= _MAPPED_BYTES
         rows = _row_shape(num_codes, q_prefix)
         scores = _torch().empty(rows, dtype=_torch().float32, device="cpu", pin_memory=True) if to_host else pk.norms.new_empty(rows)
@@ -707,6 +714,20 @@ class TurboQuantProd:
             self._plans.check_status(pk.device)      # waits for the stream
             return _in_shape(scores.clone().numpy(), q_prefix)
         return _in_shape(_deliver(scores, staged.kind, self._plans), q_prefix)
+
+    def _score_on_host(self, query: np.ndarray, pk: _Packed, shape):
+        """One NumPy query against a few thousand keys: one call into the library takes the query, waits and returns the scores
+        (the same through page-locked torch tensors and a call to wait took 31 us instead of 21, the kernel 3 of them)."""
+        q = np.ascontiguousarray(query, dtype=np.float32)
+        scores = np.empty(pk.n, dtype=np.float32)
+        status = ctypes.c_int64(0)
+        _native.check(_native.load().tq_score_host(
+            self._plans.handle(pk.device), q.__array_interface__["data"][0], pk.codes.data_ptr(), pk.signs.data_ptr(),
+            pk.residual_norms.data_ptr(), pk.norms.data_ptr(), pk.n, scores.__array_interface__["data"][0], ctypes.byref(status),
+            _stream_ptr(pk.device)))
+        if status.value:
+            _PlanSet.refuse(status.value)
+        return _in_shape(scores, shape)
 
     def attention_scores(self, queries: Any, encoding: TurboQuantProdEncoding, *, topk: Optional[int] = None,
                          groups: int = 1, return_matrix: Optional[bool] = None, index_base: int = 0,
