@@ -54,7 +54,7 @@ constexpr int kPendKeys = 64;                     // survivors a warp stages in 
 constexpr int kMaxStages = 8;
 constexpr float kCentScale = 1024.f;
 constexpr int kRowBytesB = D * 2;  // one query row of one fp16 operand matrix
-constexpr int kPrepSmemBytes = 2 * D * D * 4;  // rotation and projection matrices staged by the preparation kernel
+constexpr int kPrepSmemBytes = D * D * 4;  // the matrix that a block of the preparation kernel stages
 constexpr int kEpiBarrier = 1;     // named barriers of the epilogue groups: this one and the next
 
 // Prepared queries of one group: per half of the coordinates (two halves of 128 for d = 256, one otherwise) the four
@@ -637,142 +637,113 @@ score_tc_kernel(const __grid_constant__ CUtensorMap tmap_out, const __grid_const
     }
 }
 
-// Rotate / project the queries of one pass and lay them out as fp16 hi/lo B operands.
-// grid (QPAD, groups), block 128 (thread = coordinate).
+// Rotate (z = 0) / project (z = 1) the queries of one pass and lay them out as fp16 hi/lo B operands.
+// grid (QPAD, groups, 2), block 128 (thread = coordinate).  A block per matrix: 32 queries at d = 128 4.4 us, 5.1 with both matrices
+// in one block.
 __global__ void __launch_bounds__(128)
 score_prep_kernel(TqDev p, const float* __restrict__ q, int qpg, int q0, int nq, int qpad, unsigned char* __restrict__ prep) {
     tq_grid_release();      // the scoring kernel sets itself up meanwhile
     __shared__ float qs[D];
-    __shared__ float red[2][4];
-    const int slot = blockIdx.x, g = blockIdx.y, j = threadIdx.x;
+    __shared__ float red[4];
+    const int slot = blockIdx.x, g = blockIdx.y, which = blockIdx.z, j = threadIdx.x;
     unsigned char* base = prep + (size_t)g * prep_group_bytes(qpad);
     const size_t off = (size_t)(slot / 8) * ((D / 8) * 128) + (size_t)(j / 8) * 128 + (size_t)(slot % 8) * 16 + (size_t)(j % 8) * 2;
-    __half* m0 = reinterpret_cast<__half*>(base + 0 * (size_t)qpad * kRowBytesB + off);
-    __half* m1 = reinterpret_cast<__half*>(base + 1 * (size_t)qpad * kRowBytesB + off);
-    __half* m2 = reinterpret_cast<__half*>(base + 2 * (size_t)qpad * kRowBytesB + off);
-    __half* m3 = reinterpret_cast<__half*>(base + 3 * (size_t)qpad * kRowBytesB + off);
-    float* ds = reinterpret_cast<float*>(base + 4 * (size_t)qpad * kRowBytesB) + (slot >> 1) * 4 + (slot & 1);   // pairs of queries: two 1 / scales of q, two of p
+    __half* hi = reinterpret_cast<__half*>(base + (2 * which) * (size_t)qpad * kRowBytesB + off);
+    __half* lo = reinterpret_cast<__half*>(base + (2 * which + 1) * (size_t)qpad * kRowBytesB + off);
+    // pairs of queries: two 1 / scales of q, two of p
+    float* ds = reinterpret_cast<float*>(base + 4 * (size_t)qpad * kRowBytesB) + (slot >> 1) * 4 + (slot & 1) + 2 * which;
     if (slot >= nq) {
-        *m0 = *m1 = *m2 = *m3 = __float2half_rn(0.f);
-        if (j == 0) ds[0] = ds[2] = 0.f;
+        *hi = *lo = __float2half_rn(0.f);
+        if (j == 0) *ds = 0.f;
         return;
     }
     const int d = p.d;   // 128, or 64 with the upper half of every operand row left unused
     qs[j] = j < d ? q[((size_t)g * qpg + q0 + slot) * d + j] : 0.f;
     __syncthreads();
-    float r = 0.f, s = 0.f;
     // The matrices are usually cold (the keys streamed through L2 since the last call), so the time would
-    // go into memory latency if the loads trickled in between the arithmetic: bring both matrices into
-    // shared memory with all copies in flight at once, then run the two chains in order from there.
-    extern __shared__ __align__(16) float mats[];   // [2][D][D]: R^T, S^T
+    // go into memory latency if the loads trickled in between the arithmetic: bring the matrix into
+    // shared memory with all copies in flight at once, then run the chain in order from there.
+    extern __shared__ __align__(16) float mat[];   // [D][D]: R^T or S^T
     {
-        const uint32_t dst0 = (uint32_t)__cvta_generic_to_shared(mats);
-        const int kChunks = d * d / 4;              // 16-byte chunks per matrix
-        for (int c = j; c < kChunks; c += 128) {
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst0 + c * 16), "l"(p.Rt + (size_t)c * 4) : "memory");
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst0 + (kChunks + c) * 16), "l"(p.St + (size_t)c * 4) : "memory");
-        }
+        const uint32_t dst0 = (uint32_t)__cvta_generic_to_shared(mat);
+        const float* src = which ? p.St : p.Rt;
+#pragma unroll 8
+        for (int c = j; c < d * d / 4; c += 128)        // 16-byte chunks
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst0 + c * 16), "l"(src + (size_t)c * 4) : "memory");
         asm volatile("cp.async.commit_group;" ::: "memory");
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
     }
-    const float* Rs = mats;
-    const float* Ss = mats + d * d;
+    float r = 0.f;
     if (j < d) {
 #pragma unroll 16
-        for (int k = 0; k < d; ++k) {
-            r = fmaf(qs[k], Rs[k * d + j], r);
-            s = fmaf(qs[k], Ss[k * d + j], s);
-        }
+        for (int k = 0; k < d; ++k) r = fmaf(qs[k], mat[k * d + j], r);
     }
-    float mr = fabsf(r), ms = fabsf(s);
-    for (int o = 16; o > 0; o >>= 1) {
-        mr = fmaxf(mr, __shfl_xor_sync(0xffffffffu, mr, o));
-        ms = fmaxf(ms, __shfl_xor_sync(0xffffffffu, ms, o));
-    }
-    if ((j & 31) == 0) { red[0][j >> 5] = mr; red[1][j >> 5] = ms; }
+    float m = fabsf(r);
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((j & 31) == 0) red[j >> 5] = m;
     __syncthreads();
-    mr = fmaxf(fmaxf(red[0][0], red[0][1]), fmaxf(red[0][2], red[0][3]));
-    ms = fmaxf(fmaxf(red[1][0], red[1][1]), fmaxf(red[1][2], red[1][3]));
-    // power-of-two scales that bring the largest magnitude into [512, 1024): safe in fp16, exact to undo
-    const bool okr = mr > 0.f && mr < 3.0e38f, oks = ms > 0.f && ms < 3.0e38f;
-    const float e1 = okr ? ldexpf(1.f, 9 - ilogbf(mr)) : 1.f;
-    const float e2 = oks ? ldexpf(1.f, 9 - ilogbf(ms)) : 1.f;
-    const float rs = r * e1, ss = s * e2;
-    const __half rh = __float2half_rn(rs), sh = __float2half_rn(ss);
-    *m0 = rh;
-    *m1 = __float2half_rn(rs - __half2float(rh));
-    *m2 = sh;
-    *m3 = __float2half_rn(ss - __half2float(sh));
-    if (j == 0) { ds[0] = 1.f / (e1 * kCentScale); ds[2] = 1.f / e2; }
+    m = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
+    // a power-of-two scale that brings the largest magnitude into [512, 1024): safe in fp16, exact to undo
+    const float e = m > 0.f && m < 3.0e38f ? ldexpf(1.f, 9 - ilogbf(m)) : 1.f;
+    const float rs = r * e;
+    const __half h = __float2half_rn(rs);
+    *hi = h;
+    *lo = __float2half_rn(rs - __half2float(h));
+    if (j == 0) *ds = 1.f / (which ? e : e * kCentScale);
 }
 
 // The same for d = 256: the matrices do not fit shared memory and are read from global memory (usually cold), so the
-// kernel lives on the number of loads in flight: block 1024, thread = (coordinate, quarter of the sum), 16 loads per
-// matrix in flight per thread (39 us with 256 threads and four: a third of the scoring of 1,048,576 keys it precedes).
+// kernel lives on the number of loads in flight: block 1024, thread = (coordinate, quarter of the sum), 32 loads
+// in flight per thread; a block per matrix (16 queries: 10 us, 17 with both matrices in one block).
 // The operands are written as two halves of 128 coordinates, each in the layout of d = 128.
 __global__ void __launch_bounds__(1024)
 score_prep256_kernel(TqDev p, const float* __restrict__ q, int qpg, int q0, int nq, int qpad, unsigned char* __restrict__ prep) {
     constexpr int kD = 256, kParts = 4, kSteps = kD / kParts;
     __shared__ float qs[kD];
-    __shared__ float part[2][kParts][kD];
-    __shared__ float red[2][8];
-    const int slot = blockIdx.x, g = blockIdx.y, j = threadIdx.x & (kD - 1), kq = threadIdx.x >> 8;
+    __shared__ float part[kParts][kD];
+    __shared__ float red[8];
+    const int slot = blockIdx.x, g = blockIdx.y, which = blockIdx.z, j = threadIdx.x & (kD - 1), kq = threadIdx.x >> 8;
     unsigned char* base = prep + (size_t)g * prep_group_bytes(qpad, 2);
     const int jh = j & 127;
     const size_t off = (size_t)(j >> 7) * (4 * (size_t)qpad * kRowBytesB) + (size_t)(slot / 8) * ((D / 8) * 128) +
                        (size_t)(jh / 8) * 128 + (size_t)(slot % 8) * 16 + (size_t)(jh % 8) * 2;
-    __half* m0 = reinterpret_cast<__half*>(base + 0 * (size_t)qpad * kRowBytesB + off);
-    __half* m1 = reinterpret_cast<__half*>(base + 1 * (size_t)qpad * kRowBytesB + off);
-    __half* m2 = reinterpret_cast<__half*>(base + 2 * (size_t)qpad * kRowBytesB + off);
-    __half* m3 = reinterpret_cast<__half*>(base + 3 * (size_t)qpad * kRowBytesB + off);
-    float* ds = reinterpret_cast<float*>(base + 8 * (size_t)qpad * kRowBytesB) + (slot >> 1) * 4 + (slot & 1);
+    __half* hi = reinterpret_cast<__half*>(base + (2 * which) * (size_t)qpad * kRowBytesB + off);
+    __half* lo = reinterpret_cast<__half*>(base + (2 * which + 1) * (size_t)qpad * kRowBytesB + off);
+    float* ds = reinterpret_cast<float*>(base + 8 * (size_t)qpad * kRowBytesB) + (slot >> 1) * 4 + (slot & 1) + 2 * which;
     tq_grid_release();      // the scoring kernel sets itself up meanwhile
     if (slot >= nq) {
         if (kq == 0) {
-            *m0 = *m1 = *m2 = *m3 = __float2half_rn(0.f);
-            if (j == 0) ds[0] = ds[2] = 0.f;
+            *hi = *lo = __float2half_rn(0.f);
+            if (j == 0) *ds = 0.f;
         }
         return;
     }
+    // four independent chains; the order of the sums differs from the general kernel's, which the fp32
+    // tolerance of the scores covers
+    const float* M = (which ? p.St : p.Rt) + (size_t)kq * kSteps * kD + j;
+    float r[4] = {0.f, 0.f, 0.f, 0.f};
     if (kq == 0) qs[j] = q[((size_t)g * qpg + q0 + slot) * kD + j];
     __syncthreads();
-    // four independent chains per matrix; the order of the sums differs from the general kernel's, which the fp32
-    // tolerance of the scores covers
-    float r[4] = {0.f, 0.f, 0.f, 0.f}, s[4] = {0.f, 0.f, 0.f, 0.f};
-    const float* Rt = p.Rt + (size_t)kq * kSteps * kD + j;
-    const float* St = p.St + (size_t)kq * kSteps * kD + j;
     const float* qk = qs + kq * kSteps;
-#pragma unroll 16
-    for (int k = 0; k < kSteps; ++k) {
-        r[k & 3] = fmaf(qk[k], __ldg(Rt + (size_t)k * kD), r[k & 3]);
-        s[k & 3] = fmaf(qk[k], __ldg(St + (size_t)k * kD), s[k & 3]);
-    }
-    part[0][kq][j] = (r[0] + r[1]) + (r[2] + r[3]);
-    part[1][kq][j] = (s[0] + s[1]) + (s[2] + s[3]);
+#pragma unroll 32
+    for (int k = 0; k < kSteps; ++k) r[k & 3] = fmaf(qk[k], __ldg(M + (size_t)k * kD), r[k & 3]);
+    part[kq][j] = (r[0] + r[1]) + (r[2] + r[3]);
     __syncthreads();
     if (kq != 0) return;      // threads 0..255 (warps 0..7) finish the coordinate
-    const float rr = (part[0][0][j] + part[0][1][j]) + (part[0][2][j] + part[0][3][j]);
-    const float sv = (part[1][0][j] + part[1][1][j]) + (part[1][2][j] + part[1][3][j]);
-    float mr = fabsf(rr), ms = fabsf(sv);
-    for (int o = 16; o > 0; o >>= 1) {
-        mr = fmaxf(mr, __shfl_xor_sync(0xffffffffu, mr, o));
-        ms = fmaxf(ms, __shfl_xor_sync(0xffffffffu, ms, o));
-    }
-    if ((j & 31) == 0) { red[0][j >> 5] = mr; red[1][j >> 5] = ms; }
+    const float rr = (part[0][j] + part[1][j]) + (part[2][j] + part[3][j]);
+    float m = fabsf(rr);
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((j & 31) == 0) red[j >> 5] = m;
     asm volatile("bar.sync 1, 256;" ::: "memory");      // the 256 threads that are left
-    mr = ms = 0.f;
-    for (int w = 0; w < 8; ++w) { mr = fmaxf(mr, red[0][w]); ms = fmaxf(ms, red[1][w]); }
-    const bool okr = mr > 0.f && mr < 3.0e38f, oks = ms > 0.f && ms < 3.0e38f;
-    const float e1 = okr ? ldexpf(1.f, 9 - ilogbf(mr)) : 1.f;
-    const float e2 = oks ? ldexpf(1.f, 9 - ilogbf(ms)) : 1.f;
-    const float rs = rr * e1, ss = sv * e2;
-    const __half rh = __float2half_rn(rs), sh = __float2half_rn(ss);
-    *m0 = rh;
-    *m1 = __float2half_rn(rs - __half2float(rh));
-    *m2 = sh;
-    *m3 = __float2half_rn(ss - __half2float(sh));
-    if (j == 0) { ds[0] = 1.f / (e1 * kCentScale); ds[2] = 1.f / e2; }
+    m = 0.f;
+    for (int w = 0; w < 8; ++w) m = fmaxf(m, red[w]);
+    const float e = m > 0.f && m < 3.0e38f ? ldexpf(1.f, 9 - ilogbf(m)) : 1.f;
+    const float rs = rr * e;
+    const __half h = __float2half_rn(rs);
+    *hi = h;
+    *lo = __float2half_rn(rs - __half2float(h));
+    if (j == 0) *ds = 1.f / (which ? e : e * kCentScale);
 }
 
 // grid (segments, rows): block scans scores[row][seg*seg_len ...) and writes its k best as sortable keys
@@ -1146,10 +1117,10 @@ int tq_launch_score_tc(const tq_plan* p, const float* q, int groups, int qpg, co
     auto prepare_pass = [&](int q0, int nq) -> int {
         const int qpad = pad_of(nq);
         if (p->dev.d == 256) {
-            score_prep256_kernel<<<dim3(qpad, groups), 1024, 0, st>>>(p->dev, q, qpg, q0, nq, qpad, prep); tq_count_launch();
+            score_prep256_kernel<<<dim3(qpad, groups, 2), 1024, 0, st>>>(p->dev, q, qpg, q0, nq, qpad, prep); tq_count_launch();
         } else {
             TQ_GRANT_SMEM((score_prep_kernel), kPrepSmemBytes, p->device);
-            score_prep_kernel<<<dim3(qpad, groups), 128, kPrepSmemBytes, st>>>(p->dev, q, qpg, q0, nq, qpad, prep); tq_count_launch();
+            score_prep_kernel<<<dim3(qpad, groups, 2), 128, kPrepSmemBytes, st>>>(p->dev, q, qpg, q0, nq, qpad, prep); tq_count_launch();
         }
         TQ_CUDA_TRY(cudaGetLastError());
         return TQ_OK;
