@@ -1035,11 +1035,11 @@ second_stage_kernel(const __grid_constant__ StageJob first, const __grid_constan
     }
 }
 
-// d = 256, listed coordinates (those inside the guard band of the tensor-core kernel) re-decided in the reference's order: norm, division
-// and the rotated coordinate as one FMA chain.  A wrong code is corrected in place and (TurboQuantProd) puts its row on the row
-// list.  Every dependent access to global memory costs about a microsecond, so the kernel is as long as its chain of such accesses:
-// header and entry, then row, matrix row and boundaries together.  Sixteen lanes fetch an entry's rows, normalise and leave both in
-// shared memory; then a lane per entry runs the chain, 16 entries side by side.
+// d = 256, listed coordinates (those inside the guard band of the tensor-core kernel) re-decided in the reference's order, eight lanes
+// each: norm, division, and the rotated coordinate as one FMA chain that goes from lane to lane (lane l has the values [32 l, + 32)).
+// A wrong code is corrected in place and (TurboQuantProd) puts its row on the row list.  Every dependent access to global memory
+// costs about a microsecond, so what counts is how many entries are on their way side by side: 64 an SM, in registers.  524,309
+// TurboQuantProd rows (22,000 entries): 23 us behind the quantizer, 41 with sixteen lanes an entry and the rows in shared memory.
 struct CheckJob {
     TqDev p;
     const void* x;
@@ -1049,85 +1049,97 @@ struct CheckJob {
     TqRecheck lists;
     TqRowMap map;
 };
+constexpr int kCheckEntries = 32;        // of a block at a time
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kCheckEntries * 8, 2)
 exact_code_check_kernel(const __grid_constant__ CheckJob first, const __grid_constant__ CheckJob second, int blocks0) {
-    constexpr int D = 256, E = 16, kLanes = 256 / E, kStep = E / (32 / kLanes);      // entries per block; lanes per entry
-    constexpr int kStride = D + 1;                                                      // odd: a column is free of bank conflicts
-    __shared__ float vt[E * kStride], mt[E * kStride];
+    constexpr int D = 256, V = D / 8;
     __shared__ float bnd[16];
-    __shared__ unsigned long long entry[E];      // ~0: none
-    __shared__ uint32_t stored[E];               // the code that stands in the packed row
     const bool one = (int)blockIdx.x < blocks0;
     const CheckJob& job = one ? first : second;
     const TqDev& p = job.p;
     const unsigned int block = one ? blockIdx.x : blockIdx.x - blocks0, nblocks = one ? blocks0 : gridDim.x - blocks0;
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    // entries warp, warp + kStep, ... of the block: the lanes of different entries meet in different banks
-    const int e = warp + kStep * (lane / kLanes), l = lane & (kLanes - 1);
+    const int t = threadIdx.x, lane = t & 31, l = t & 7;
     const TqRecheck& lists = job.lists;
     if (t < p.levels - 1) bnd[t] = __ldg(p.boundaries + t);      // (at most 15: the kernel at d = 256 takes up to 4 bits)
+    __syncthreads();
     tq_grid_release();
     tq_grid_wait();
     // asked for before the header is known to allow it (the list's capacity bounds the index)
-    unsigned int at = block * E + e;
+    unsigned int at = block * kCheckEntries + (t >> 3);
     unsigned long long ent = at < lists.code_cap ? lists.code_entries[at] : 0ull;
     if (lists.hdr->overflow) return;  // the row pass will redo everything
     const unsigned int count = min(lists.hdr->n_codes, lists.code_cap);
-    for (unsigned int at0 = block * E; at0 < count; at0 += nblocks * E) {
-        const unsigned int mine = at0 + e;
-        if (mine != at && mine < count) ent = lists.code_entries[mine];
-        at = mine;
+    for (; at - (t >> 3) < count; at += nblocks * kCheckEntries) {
+        if (at != block * kCheckEntries + (t >> 3)) ent = at < count ? lists.code_entries[at] : 0ull;
         const int64_t row = (int64_t)(ent >> 8);
         const int j = (int)(ent & 255u);
-        const bool valid = mine < count && row < job.n && j < D;
-        float* v = vt + e * kStride;
-        float* m = mt + e * kStride;
-        auto packed_row = [&](int64_t r) {
-            return job.codes + (job.map.tokens > 0 ? r / job.map.tokens * job.map.capacity + job.map.base + r % job.map.tokens : r) * p.code_words;
-        };
-        if (l == 0) {
-            entry[e] = valid ? ent : ~0ull;
-            if (valid) stored[e] = tq_get_code(packed_row(row), j, p.bits);
+        const bool valid = at < count && row < job.n;
+        if (!__any_sync(0xffffffffu, valid)) continue;
+        uint32_t* crow = job.codes + (!valid ? 0 : job.map.tokens > 0 ? row / job.map.tokens * job.map.capacity + job.map.base + row % job.map.tokens : row) * p.code_words;
+        const uint32_t old = valid && l == 7 ? tq_get_code(crow, j, p.bits) : 0u;
+        const int64_t x0 = (valid ? row : 0) * D;
+        float c[V], m[V];
+        {
+            const float4* src = reinterpret_cast<const float4*>(p.R + (size_t)(valid ? j : 0) * D + l * V);
+#pragma unroll
+            for (int i = 0; i < V / 4; ++i) *reinterpret_cast<float4*>(m + 4 * i) = __ldg(src + i);
         }
-        if (l < 8) {
-            load_row(v, 1, D, l, job.x, job.xtype, valid ? row : -1);
-        } else {
-            load_row(m, 1, D, l - 8, p.R, TQ_INPUT_F32, valid ? j : -1);
-        }
-        __syncwarp();
-        const float nr = __fsqrt_rn(np_sumsq8<1>(v, D, l & 7));
-        __syncwarp();
-        if (l < 8) divide_row(v, 1, D, l, nr);
-        __syncthreads();
-        // lane i of the first warp takes the chain of entry i
-        if (warp == 0) {
-            if (lane < E && entry[lane] != ~0ull) {
-                const int64_t r = (int64_t)(entry[lane] >> 8);
-                const int c = (int)(entry[lane] & 255u);
-                const uint32_t old = stored[lane];
-                const float* ve = vt + lane * kStride;
-                const float* me = mt + lane * kStride;
-                float acc = 0.f;
-#pragma unroll 32
-                for (int k = 0; k < D; ++k) acc = __fmaf_rn(ve[k], me[k], acc);
-                const uint32_t code = (uint32_t)count_below(bnd, p.levels - 1, acc);
-                if (old != code) {
-                    if (job.prod) {        // the row's residual is another one
-                        const unsigned int pos = atomicAdd(&lists.hdr->n_rows, 1u);
-                        if (pos < lists.row_cap) lists.row_entries[pos] = (unsigned int)r;
-                        else lists.hdr->overflow = 1u;
-                    }
-                    uint32_t* crow = packed_row(r);
-                    const uint32_t delta = old ^ code;
-                    const int bit = c * p.bits, w = bit >> 5, sh = bit & 31;
-                    atomicXor(crow + w, delta << sh);
-                    if (sh + p.bits > 32) atomicXor(crow + w + 1, delta >> (32 - sh));
-                    atomicAdd(&lists.hdr->changed, 1u);
+        float half[2];       // NumPy's pairwise sum: eight interleaved sums for each 128 values
+        {
+            float a[V];
+            if (job.xtype == TQ_INPUT_F32) {
+                const float* x = static_cast<const float*>(job.x) + x0;
+#pragma unroll
+                for (int i = 0; i < V; ++i) a[i] = __ldg(x + l + 8 * i);
+#pragma unroll
+                for (int i = 0; i < V; i += 4) *reinterpret_cast<float4*>(c + i) = __ldg(reinterpret_cast<const float4*>(x + l * V + i));
+            } else {
+                const uint16_t* x = static_cast<const uint16_t*>(job.x) + x0;
+#pragma unroll
+                for (int i = 0; i < V; ++i) {
+                    a[i] = widen(__ldg(x + l + 8 * i), job.xtype);
+                    c[i] = widen(__ldg(x + l * V + i), job.xtype);
                 }
             }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                half[h] = __fmul_rn(a[h * 16], a[h * 16]);
+#pragma unroll
+                for (int i = 1; i < 16; ++i) half[h] = __fadd_rn(half[h], __fmul_rn(a[h * 16 + i], a[h * 16 + i]));
+            }
         }
-        __syncthreads();
+#pragma unroll
+        for (int s = 1; s < 8; s <<= 1) {
+            half[0] = __fadd_rn(half[0], __shfl_xor_sync(0xffffffffu, half[0], s));
+            half[1] = __fadd_rn(half[1], __shfl_xor_sync(0xffffffffu, half[1], s));
+        }
+        const float nr = __fsqrt_rn(__fadd_rn(half[0], half[1]));
+#pragma unroll
+        for (int i = 0; i < V; ++i) c[i] = nr > 0.f ? __fdiv_rn(c[i], nr) : 0.f;
+        float acc = 0.f;
+#pragma unroll 1
+        for (int s = 0; s < 8; ++s) {
+            const float before = __shfl_sync(0xffffffffu, acc, (lane & 24) + (s > 0 ? s - 1 : 0));
+            acc = s > 0 ? before : 0.f;
+#pragma unroll
+            for (int i = 0; i < V; ++i) acc = __fmaf_rn(c[i], m[i], acc);
+        }
+        if (valid && l == 7) {
+            const uint32_t code = (uint32_t)count_below(bnd, p.levels - 1, acc);
+            if (old != code) {
+                if (job.prod) {        // the row's residual is another one
+                    const unsigned int pos = atomicAdd(&lists.hdr->n_rows, 1u);
+                    if (pos < lists.row_cap) lists.row_entries[pos] = (unsigned int)row;
+                    else lists.hdr->overflow = 1u;
+                }
+                const uint32_t delta = old ^ code;
+                const int bit = j * p.bits, w = bit >> 5, sh = bit & 31;
+                atomicXor(crow + w, delta << sh);
+                if (sh + p.bits > 32) atomicXor(crow + w + 1, delta >> (32 - sh));
+                atomicAdd(&lists.hdr->changed, 1u);
+            }
+        }
     }
 }
 
@@ -1256,7 +1268,7 @@ int tq_launch_exact_code_check(const TqSecondStage* a, const TqSecondStage* b, c
     TqRange range("tq.quantize.recheck_coordinates");
     const int d = a->plan->dev.d;
     if (d != 256) return tq_fail(TQ_ERR_UNSUPPORTED, "the coordinate re-check alone is written for d = 256");
-    const int64_t per_block = 16, most = tq_sm_count(a->plan->device) * (int64_t)(b ? 3 : 6);
+    const int64_t per_block = kCheckEntries, most = tq_sm_count(a->plan->device) * (int64_t)(b ? 1 : 2);
     // as many blocks as a list of typical length has entries for (about 1 in 48 rows of 128 coordinates at 4 bits, in
     // proportion to the coordinates); longer lists take more passes
     auto blocks = [&](const TqSecondStage* s) {
@@ -1271,7 +1283,7 @@ int tq_launch_exact_code_check(const TqSecondStage* a, const TqSecondStage* b, c
     };
     const CheckJob first = job(a), second = b ? job(b) : first;
     const int b0 = blocks(a), grid = b0 + (b ? blocks(b) : 0);
-    TQ_CUDA_TRY(tq_launch_dependent(exact_code_check_kernel, dim3(grid), dim3(256), 0, st, first, second, b0));
+    TQ_CUDA_TRY(tq_launch_dependent(exact_code_check_kernel, dim3(grid), dim3(kCheckEntries * 8), 0, st, first, second, b0));
     return TQ_OK;
 }
 
