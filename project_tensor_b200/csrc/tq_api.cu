@@ -414,9 +414,11 @@ static int quantize_common(const tq_plan* p, bool prod, const float* x, int64_t 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int err = TQ_OK;
     const TqQuantOut out{static_cast<uint32_t*>(codes), static_cast<uint32_t*>(signs), rnorms, norms, TqRowMap{}};
-    if (!few_rows(p, prod, n) && use_tensor(p, &err)) {
-        const int64_t need = tq_quantize_scratch_bytes(p, n);
-        if (!scratch || (int64_t)scratch_bytes < need)
+    const int64_t need = tq_quantize_scratch_bytes(p, n);
+    const bool room = scratch && (int64_t)scratch_bytes >= need;
+    // (plans whose other calls have no tensor-core kernel go without one where there is no room for its lists)
+    if (!few_rows(p, prod, n) && (room || p->tensor_ok) && use_tensor(p, &err)) {
+        if (!room)
             return tq_fail(TQ_ERR_SCRATCH_TOO_SMALL, "quantize scratch: need %lld bytes, got %zu", (long long)need, scratch_bytes);
         TQ_TRY(check_ptr(scratch, "scratch"));
         unsigned char* sc = static_cast<unsigned char*>(scratch);
@@ -534,17 +536,18 @@ int tq_kv_prefill(const tq_plan* kp, const tq_plan* vp, const void* keys, const 
     int njobs = 0, ntensor = 0;
     if (kp) jobs[njobs++] = TqSecondStage{kp, true, keys, dtype, rows, {static_cast<uint32_t*>(k_codes), static_cast<uint32_t*>(k_signs), k_residual_norms, k_norms, map}, {}};
     if (vp) jobs[njobs++] = TqSecondStage{vp, false, values, dtype, rows, {static_cast<uint32_t*>(v_codes), nullptr, nullptr, v_norms, map}, {}};
+    const int64_t need = tq_kv_prefill_scratch_bytes(kp, vp, rows);
+    const bool room = scratch && (int64_t)scratch_bytes >= need;
     bool whole[2] = {false, false};      // jobs for the reference-order kernel alone
     for (int i = 0; i < njobs; ++i) {
         int err = TQ_OK;
         const tq_plan* p = jobs[i].plan;
-        whole[i] = few_rows(p, jobs[i].prod, rows) || !use_tensor(p, &err) || !tq_tensor_input_supported(p->dev.d, dtype);
+        whole[i] = few_rows(p, jobs[i].prod, rows) || (!room && !p->tensor_ok) || !use_tensor(p, &err) || !tq_tensor_input_supported(p->dev.d, dtype);
         if (err != TQ_OK) return err;
         if (!whole[i]) tensor[ntensor++] = jobs[i];
     }
     if (ntensor) {
-        const int64_t need = tq_kv_prefill_scratch_bytes(kp, vp, rows);
-        if (!scratch || (int64_t)scratch_bytes < need)
+        if (!room)
             return tq_fail(TQ_ERR_SCRATCH_TOO_SMALL, "prefill scratch: need %lld bytes, got %zu", (long long)need, scratch_bytes);
         TQ_TRY(check_ptr(scratch, "scratch"));
         TqRecheckHeader* hdr = static_cast<TqRecheckHeader*>(scratch);

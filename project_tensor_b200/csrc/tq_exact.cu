@@ -250,14 +250,14 @@ __device__ __forceinline__ void advance_length(const RowsJob& job, int64_t len0,
 // Few rows, d <= 128 (a decode step's tokens, a handful of vectors): RB rows per block, the three matrices copied whole into
 // shared memory (64 bytes a cycle and SM from L2: 1.6 us for the 192 KB of d = 128) while the rows are normalised; one thread
 // per output, so that a product is a 128-long FMA chain with its loads running ahead.  64 keys and 64 values of d = 128 with the
-// length: 10.8 us in one launch (18.6 + 10.6 + 1.2 us in three before).
+// length: 9.8 us in one launch.
 template <int RB>
 __global__ void __launch_bounds__(128 * RB)
 exact_quantize_few_kernel(const __grid_constant__ RowsJob first, const __grid_constant__ RowsJob second, int blocks0, int advance) {
     extern __shared__ __align__(16) float smem[];
     __shared__ __align__(16) float vt[RB][128], ct[RB][128];   // unit vector, later residual; centroids
     __shared__ uint8_t cs[RB][128 + 8];
-    __shared__ float bnd[256], cbk[256];
+    __shared__ float bnd[256], cbk[256], row_norm;
     const bool one = (int)blockIdx.x < blocks0;
     const RowsJob& job = one ? first : second;
     const int block = one ? blockIdx.x : blockIdx.x - blocks0, nblocks = one ? blocks0 : gridDim.x - blocks0;
@@ -275,12 +275,18 @@ exact_quantize_few_kernel(const __grid_constant__ RowsJob first, const __grid_co
     };
     auto product = [&](int which, const float* vec) {
         const float* m = smem + which * dd4 * 4 + (j < d ? j : 0);
-        float acc = 0.f;
+        float acc = 0.f, b[16];
         int k = 0;
-        for (; k + 16 <= d; k += 16) {
-            float b[16];
+        constexpr bool kAhead = RB == 1;      // the next piece on its way while one runs (more rows: other warps fill the time)
+        auto fetch = [&](float (&to)[16], int from) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) b[i] = m[(k + i) * d];
+            for (int i = 0; i < 16; ++i) to[i] = m[(from + i) * d];
+        };
+        if (kAhead && d >= 16) fetch(b, 0);
+        for (; k + 16 <= d; k += 16) {
+            float next[16];
+            if constexpr (kAhead) fetch(next, k + 32 <= d ? k + 16 : k);      // (behind the end: the last piece again)
+            else fetch(b, k);
 #pragma unroll
             for (int i = 0; i < 16; i += 4) {
                 const float4 v = *reinterpret_cast<const float4*>(vec + k + i);
@@ -289,16 +295,24 @@ exact_quantize_few_kernel(const __grid_constant__ RowsJob first, const __grid_co
                 acc = __fmaf_rn(v.z, b[i + 2], acc);
                 acc = __fmaf_rn(v.w, b[i + 3], acc);
             }
+            if constexpr (kAhead) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) b[i] = next[i];
+            }
         }
         for (; k < d; ++k) acc = __fmaf_rn(vec[k], m[k * d], acc);
         return acc;
     };
-    copy(0, p.Rt);
-    if (prod) { copy(1, p.R); copy(2, p.St); }
     for (int i = t; i < levels; i += kThreads) {
         cbk[i] = __ldg(p.codebook + i);
         if (i + 1 < levels) bnd[i] = __ldg(p.boundaries + i);
     }
+    copy(0, p.Rt);
+    // One row: the other two matrices are asked for behind it, or it would have to wait for all 192 KB.  (With that, a thread per value and
+    // the products' loads a piece ahead, 100 TurboQuantProd rows of d = 128 take 8.4 us instead of 9.9, 64 keys and 64 values 9.8
+    // instead of 10.8.  Four rows a block are slower that way, 500 rows 14.7 against 13.0.)
+    bool later = prod && RB == 1;
+    if (prod && !later) { copy(1, p.R); copy(2, p.St); }
     if (j < 8) cs[r][128 + j] = 0;
     const uint32_t inv_bits = inverse_of_bits(p.bits);
     tq_grid_release();
@@ -308,16 +322,38 @@ exact_quantize_few_kernel(const __grid_constant__ RowsJob first, const __grid_co
     for (int64_t g0 = (int64_t)block * RB; g0 < rows.limit; g0 += (int64_t)nblocks * RB) {
         const int64_t row = rows.src(job, g0 + r), to = rows.dst(job, row);
         __syncthreads();
-        if (j < 8) {     // eight lanes per row: load, sum of squares, divide
-            // (the other lanes of the warp wait here; with 16 values per lane the row is in flight at once)
-            load_row(vt[r], 1, d, j, job.x, job.xtype, row);
-        }
-        if (j < 32) {
-            __syncwarp();
-            const float nr = __fsqrt_rn(np_sumsq8<1>(vt[r], d, lane & 7));
-            __syncwarp();
-            if (j < 8) divide_row(vt[r], 1, d, j, nr);
-            if (j == 0 && to >= 0) job.norms[to] = nr;
+        if constexpr (RB == 1) {         // a thread per value; the sum of squares by eight lanes
+            float value = 0.f;
+            if (row >= 0 && j < d)
+                value = job.xtype == TQ_INPUT_F32 ? __ldg(static_cast<const float*>(job.x) + row * d + j) : widen(__ldg(static_cast<const uint16_t*>(job.x) + row * d + j), job.xtype);
+            if (later) {
+                copy(1, p.R);
+                copy(2, p.St);
+                later = false;
+            }
+            vt[r][j] = value;
+            __syncthreads();
+            if (j < 32) {
+                const float nr = __fsqrt_rn(np_sumsq8<1>(vt[r], d, lane & 7));
+                if (j == 0) {
+                    row_norm = nr;
+                    if (to >= 0) job.norms[to] = nr;
+                }
+            }
+            __syncthreads();
+            vt[r][j] = row_norm > 0.f ? __fdiv_rn(value, row_norm) : 0.f;
+        } else {
+            if (j < 8) {     // eight lanes per row: load, sum of squares, divide
+                // (the other lanes of the warp wait here; with 16 values per lane the row is in flight at once)
+                load_row(vt[r], 1, d, j, job.x, job.xtype, row);
+            }
+            if (j < 32) {
+                __syncwarp();
+                const float nr = __fsqrt_rn(np_sumsq8<1>(vt[r], d, lane & 7));
+                __syncwarp();
+                if (j < 8) divide_row(vt[r], 1, d, j, nr);
+                if (j == 0 && to >= 0) job.norms[to] = nr;
+            }
         }
         if (prod) asm volatile("cp.async.wait_group 2;" ::: "memory");
         else asm volatile("cp.async.wait_group 0;" ::: "memory");

@@ -78,3 +78,24 @@ def test_rows_of_a_cache(lib_built, d, kbits, vbits, dtype):
     want = tg.packed_buffers(vq.quantize(values.float().reshape(-1, d)))
     assert torch.equal(cache.value_codes.view(groups, tokens + 5, -1)[:, :tokens].reshape(groups * tokens, -1),
                        want["codes"].reshape(groups * tokens, -1))
+
+
+@pytest.mark.parametrize("kind,d,bits", [("mse", 96, 4), ("prod", 128, 6), ("mse", 64, 6)])
+def test_without_scratch_the_reference_order_kernels_serve(lib_built, kind, d, bits):
+    """A C caller that passes no scratch block for such a plan, which needed none before there was a kernel with lists."""
+    import torch
+    from project_tensor_b200 import _native
+    lib, n = _native.load(), 12001
+    quant = _quantizer(kind, d, bits)
+    x = torch.randn(n, d, device="cuda", generator=torch.Generator("cuda").manual_seed(d))
+    want = tg.packed_buffers(quant.quantize(x))
+    plan, stream = quant._plans.handle(x.device), torch.cuda.current_stream().cuda_stream
+    got = {k: torch.zeros_like(v) for k, v in want.items() if v is not None}
+    if kind == "mse":
+        _native.check(lib.tq_mse_quantize(plan, x.data_ptr(), n, got["codes"].data_ptr(), got["norms"].data_ptr(), None, 0, stream))
+    else:
+        _native.check(lib.tq_prod_quantize(plan, x.data_ptr(), n, got["codes"].data_ptr(), got["signs"].data_ptr(),
+                                           got["residual_norms"].data_ptr(), got["norms"].data_ptr(), None, 0, stream))
+    assert torch.equal(got["codes"], want["codes"])
+    if kind == "prod":
+        assert torch.equal(got["signs"], want["signs"])
