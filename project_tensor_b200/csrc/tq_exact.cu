@@ -250,14 +250,14 @@ __device__ __forceinline__ void advance_length(const RowsJob& job, int64_t len0,
 // Few rows, d <= 128 (a decode step's tokens, a handful of vectors): RB rows per block, the three matrices copied whole into
 // shared memory (64 bytes a cycle and SM from L2: 1.6 us for the 192 KB of d = 128) while the rows are normalised; one thread
 // per output, so that a product is a 128-long FMA chain with its loads running ahead.  64 keys and 64 values of d = 128 with the
-// length: 9.8 us in one launch.
+// length: 9.8 us in one launch, 120 and 120 with two rows a block 9.6.
 template <int RB>
 __global__ void __launch_bounds__(128 * RB)
 exact_quantize_few_kernel(const __grid_constant__ RowsJob first, const __grid_constant__ RowsJob second, int blocks0, int advance) {
     extern __shared__ __align__(16) float smem[];
     __shared__ __align__(16) float vt[RB][128], ct[RB][128];   // unit vector, later residual; centroids
     __shared__ uint8_t cs[RB][128 + 8];
-    __shared__ float bnd[256], cbk[256], row_norm;
+    __shared__ float bnd[256], cbk[256], row_norm[RB];
     const bool one = (int)blockIdx.x < blocks0;
     const RowsJob& job = one ? first : second;
     const int block = one ? blockIdx.x : blockIdx.x - blocks0, nblocks = one ? blocks0 : gridDim.x - blocks0;
@@ -277,7 +277,7 @@ exact_quantize_few_kernel(const __grid_constant__ RowsJob first, const __grid_co
         const float* m = smem + which * dd4 * 4 + (j < d ? j : 0);
         float acc = 0.f, b[16];
         int k = 0;
-        constexpr bool kAhead = RB == 1;      // the next piece on its way while one runs (more rows: other warps fill the time)
+        constexpr bool kAhead = RB <= 2;      // the next piece on its way while one runs (four rows: other warps fill the time)
         auto fetch = [&](float (&to)[16], int from) {
 #pragma unroll
             for (int i = 0; i < 16; ++i) to[i] = m[(from + i) * d];
@@ -308,10 +308,11 @@ exact_quantize_few_kernel(const __grid_constant__ RowsJob first, const __grid_co
         if (i + 1 < levels) bnd[i] = __ldg(p.boundaries + i);
     }
     copy(0, p.Rt);
-    // One row: the other two matrices are asked for behind it, or it would have to wait for all 192 KB.  (With that, a thread per value and
-    // the products' loads a piece ahead, 100 TurboQuantProd rows of d = 128 take 8.4 us instead of 9.9, 64 keys and 64 values 9.8
-    // instead of 10.8.  Four rows a block are slower that way, 500 rows 14.7 against 13.0.)
-    bool later = prod && RB == 1;
+    // One or two rows: the other two matrices are asked for behind them, or they would have to wait for all 192 KB.  (With that, a thread per
+    // value and the products' loads a piece ahead, 100 TurboQuantProd rows of d = 128 take 8.4 us instead of 9.9, 64 keys and 64 values
+    // 9.8 instead of 10.8.  Four rows a block are slower that way, 500 rows 14.7 against 13.0; also with two columns of all four rows a
+    // thread, which halves the shared-memory traffic and leaves too few warps: 14.7 with the old loading, 15.6 with the new.)
+    bool later = prod && RB <= 2;
     if (prod && !later) { copy(1, p.R); copy(2, p.St); }
     if (j < 8) cs[r][128 + j] = 0;
     const uint32_t inv_bits = inverse_of_bits(p.bits);
@@ -322,7 +323,7 @@ exact_quantize_few_kernel(const __grid_constant__ RowsJob first, const __grid_co
     for (int64_t g0 = (int64_t)block * RB; g0 < rows.limit; g0 += (int64_t)nblocks * RB) {
         const int64_t row = rows.src(job, g0 + r), to = rows.dst(job, row);
         __syncthreads();
-        if constexpr (RB == 1) {         // a thread per value; the sum of squares by eight lanes
+        if constexpr (RB <= 2) {         // a thread per value; a row's sum of squares by eight lanes
             float value = 0.f;
             if (row >= 0 && j < d)
                 value = job.xtype == TQ_INPUT_F32 ? __ldg(static_cast<const float*>(job.x) + row * d + j) : widen(__ldg(static_cast<const uint16_t*>(job.x) + row * d + j), job.xtype);
@@ -336,12 +337,12 @@ exact_quantize_few_kernel(const __grid_constant__ RowsJob first, const __grid_co
             if (j < 32) {
                 const float nr = __fsqrt_rn(np_sumsq8<1>(vt[r], d, lane & 7));
                 if (j == 0) {
-                    row_norm = nr;
+                    row_norm[r] = nr;
                     if (to >= 0) job.norms[to] = nr;
                 }
             }
             __syncthreads();
-            vt[r][j] = row_norm > 0.f ? __fdiv_rn(value, row_norm) : 0.f;
+            vt[r][j] = row_norm[r] > 0.f ? __fdiv_rn(value, row_norm[r]) : 0.f;
         } else {
             if (j < 8) {     // eight lanes per row: load, sum of squares, divide
                 // (the other lanes of the warp wait here; with 16 values per lane the row is in flight at once)
@@ -1395,12 +1396,15 @@ int wide_block_rows(int d, int64_t rows, int64_t sms) {
     return best;
 }
 
-// Rows per block: one while every row can have an SM to itself (d <= 128), then four, 16 (8 at d = 256) while larger blocks would leave
-// SMs idle, 64 or 32 from there on.
+// Rows per block: one while every row can have an SM to itself (d <= 128), two while every two can, then four, 16 (8 at d = 256) while
+// larger blocks would leave SMs idle, 64 or 32 from there on.  (Two against four, us: 120 keys and 120 values of d = 64 / 96 / 128
+// 7.5:10.4 / 8.7:12.6 / 9.6:15.0; 296 rows of d = 128, TurboQuantProd 8.9:12.5, TurboQuantMSE 5.2:7.3; two blocks an SM of one or two rows
+// each, 400 rows of d = 64, Prod, 12.9 and 11.8 against 8.8 with four.)
 int launch_rows(const RowsJob& a, const RowsJob* b, int64_t rows, int device, int advance, cudaStream_t st) {
     const int d = a.p.d;
     const int64_t sms = tq_sm_count(device), total = b ? 2 * rows : rows;
     if (d <= 128 && total <= sms) return launch_few_rows<1>(a, b, rows, device, advance, st);
+    if (d <= 128 && total <= sms * 2) return launch_few_rows<2>(a, b, rows, device, advance, st);
     if (d <= 128 && total <= sms * 4) return launch_few_rows<4>(a, b, rows, device, advance, st);
     // (64-row blocks on half the SMs are slower than 16-row blocks on all of them: 4,737 rows of d = 96, TurboQuantMSE, 21.5 us against 10)
     const bool many = total > sms * (d <= 96 ? 64 : d <= 128 ? 56 : 32);

@@ -97,3 +97,30 @@ def test_a_row_is_the_same_in_every_block_shape(lib_built, d, bits, counts):
                 assert torch.equal(restored[part], rows), (n, part)
                 for name, value in buffers.items():
                     assert value is None or torch.equal(packed[name][part], value), (n, part, name)
+
+
+@pytest.mark.parametrize("d", [33, 64, 100, 128])
+def test_two_rows_a_block_equal_one(lib_built, d):
+    """More rows than SMs, up to two an SM, share blocks in pairs: the same bytes as in calls of at most 100 rows, an odd last row, zero
+    rows on either side of a pair and the keys and values of a cache step included."""
+    import torch
+    import project_tensor_b200 as tg
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    prod, mse = (make(d, 4, seed=2026, grid_size=4097, max_iter=64) for make in (tg.TurboQuantProd, tg.TurboQuantMSE))
+    x = torch.randn((2 * sms + 1, d), device="cuda", generator=torch.Generator("cuda").manual_seed(d)).bfloat16()
+    x[4] = x[9] = 0
+    ones = {}
+    for quant in (prod, mse):
+        parts = [tg.packed_buffers(quant.quantize(p.float())) for p in x.split(min(100, sms))]
+        ones[quant] = {k: torch.cat([p[k] for p in parts]) for k, v in parts[0].items() if v is not None}
+        for n in (sms + 1, 2 * sms - 1, 2 * sms, 2 * sms + 1):
+            packed = tg.packed_buffers(quant.quantize(x[:n].float()))
+            for name, want in ones[quant].items():
+                assert torch.equal(packed[name], want[:n]), (n, name)
+    for groups in (sms // 2 + 1, sms - 1, sms):
+        cache = tg.PackedKVCache(prod, mse, groups, 1)
+        cache.append(x[:groups], x[groups:2 * groups])
+        for name in ("codes", "signs", "norms", "residual_norms"):
+            assert torch.equal(getattr(cache.keys, name), ones[prod][name][:groups]), (groups, name)
+        assert torch.equal(cache.value_codes, ones[mse]["codes"][groups:2 * groups])
+        assert torch.equal(cache.value_norms, ones[mse]["norms"][groups:2 * groups]) and cache.sync_length() == 1
